@@ -33,6 +33,29 @@ inline int check_launch() {
 // ranked on the device collide and order exactly as they do on the host.
 __device__ __forceinline__ float exp_as_host(float x) { return (float)exp((double)x); }
 
+// f16 of an activation: a finite value beyond the f16 range saturates to +-65504 instead of becoming an infinity
+// (which the f32 accumulation would turn into NaN on the first cancellation), the rule of the reference's f16
+// activation stores (src/hip/krk_hip.hpp:141-202). Infinities and NaNs pass through unchanged.
+__device__ __forceinline__ __half half_sat(float v) {
+    return __float2half_rn(fabsf(v) <= 3.4028234e38f ? fminf(fmaxf(v, -65504.0f), 65504.0f) : v);
+}
+
+// A launch that may overlap the tail of the kernel before it in the stream (the kernel waits for that grid itself).
+template <class... KArgs, class... Args>
+cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 // ---- geometry (src/quant.cpp:1805-1900) ----------------------------------------------
 
 __host__ __device__ constexpr int block_size(int wt) {
@@ -208,22 +231,6 @@ __device__ __forceinline__ float decode_value<KRK_CUDA_IQ4_NL>(const uint8_t *ro
     default: break;                                                                     \
     }
 
-// The formats the tensor-core GEMM stages: every one whose 256-value segment is a whole number of 8-byte
-// granules (Q2_K's 84 and Q3_K's 110 bytes are not: those take the row-batch rung).
-#define KRK_DISPATCH_WT_GEMM(wt, ...)                                                   \
-    switch (wt) {                                                                       \
-    case KRK_CUDA_Q8_0: { constexpr int WT = KRK_CUDA_Q8_0; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q4_0: { constexpr int WT = KRK_CUDA_Q4_0; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q4_K: { constexpr int WT = KRK_CUDA_Q4_K; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q6_K: { constexpr int WT = KRK_CUDA_Q6_K; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q5_0: { constexpr int WT = KRK_CUDA_Q5_0; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q5_1: { constexpr int WT = KRK_CUDA_Q5_1; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q5_K: { constexpr int WT = KRK_CUDA_Q5_K; __VA_ARGS__; } break;       \
-    case KRK_CUDA_IQ4_NL: { constexpr int WT = KRK_CUDA_IQ4_NL; __VA_ARGS__; } break;   \
-    case KRK_CUDA_Q2_K: { constexpr int WT = KRK_CUDA_Q2_K; __VA_ARGS__; } break;       \
-    case KRK_CUDA_Q3_K: { constexpr int WT = KRK_CUDA_Q3_K; __VA_ARGS__; } break;       \
-    default: break;                                                                     \
-    }
 // (every format this library decodes has a tensor-core prefill arm; the row-batch rung remains for K % 256 != 0)
 __host__ __device__ constexpr bool gemm_tc_takes(int wt) { return block_size(wt) != 0; }
 
@@ -317,6 +324,11 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
                            cudaStream_t st, const float *logits = nullptr, int n_expert = 0);
 
 // Prefill GEMM on tcgen05 (krk_gemm_tc.cu).
+int launch_f32_to_f16(__half *out, const float *in, int64_t n, cudaStream_t st);
+// A group of up to tile_m tokens of one expert: its first weight row in the bank, its first X / output row, its tokens.
+struct GemmGroup {
+    int w_row, x_row, m;
+};
 size_t gemm_workspace_bytes(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows);
 int launch_gemm_tc(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out,
                    int64_t n_in, int64_t rows, void *workspace, cudaStream_t st);

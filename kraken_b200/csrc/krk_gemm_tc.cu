@@ -14,18 +14,26 @@
 // bytes, which leaves its bandwidth to the one operand the MMA still reads from it.
 //
 // One persistent CTA per SM, warp-specialised, everything connected by mbarriers:
-//   warps 0..7   decode: two threads per weight row, 32 values each per 64-value K step. The raw blocks of
+//   warps 0..15  decode, two groups of eight that fill alternate A stages: two threads per weight row, 32 values
+//                each per 64-value K step. The raw blocks of
 //                128 rows x 256 values (Q8_0: 128 values) arrive in shared memory by TMA: a 2-D tensor map
-//                over the raw byte matrix for Q4_K / Q4_0 / Q5_K / Q8_0, eight maps (rows 8 apart) for
-//                Q6_K, whose rows do not start on 16-byte boundaries; a thread takes its row's bytes into
-//                registers and decodes with packed half2 arithmetic. Q5_0 / Q5_1 are staged by the decode
-//                warps themselves and decoded element by element. 16 x 32-bit TMEM columns per thread and step;
-//   warps 8..11  epilogue: tcgen05.ld of the accumulator (warp w%4 owns TMEM lanes 32*(w%4)..), 32 tokens
+//                over the raw byte matrix where a row's 256-value segments start on 16-byte boundaries, eight
+//                maps (rows 8 apart) for Q6_K, Q3_K and Q2_K, whose rows do not; a thread takes its row's bytes
+//                into registers and decodes them four values at a time. 16 x 32-bit TMEM columns per thread and step;
+//   warps 16..19 epilogue: tcgen05.ld of the accumulator (warp w%4 owns TMEM lanes 32*(w%4)..), 32 tokens
 //                at a time into a [token][weight row] staging buffer in shared memory, TMA stores of Y;
-//   warp 12      TMA producer of X tiles (cp.async.bulk.tensor.2d, each CTA loads its own copy);
-//   warp 13      TMA producer of the raw block columns;
-//   warp 14      TMEM allocation and the single thread that issues tcgen05.mma / tcgen05.commit.
-// Tensor memory: columns 0..255 the accumulator, 256..511 four A stages of 64 columns (two K steps each).
+//   warp 20      TMA producer of X tiles (cp.async.bulk.tensor.2d, each CTA loads its own copy);
+//   warp 21      TMA producer of the raw block columns;
+//   warp 22      TMEM allocation and issue of tcgen05.mma / tcgen05.commit.
+// Tensor memory: columns 0..255 the accumulator (two of 128 columns when a tile has at most 128 tokens, so that
+// one is read out while the next tile is multiplied), 256..511 four A stages of 64 columns (two K steps each).
+//
+// Ring depths are chosen per launch from the tile: what bounds a narrow tile is the latency of the copies, not
+// HBM (a four-deep X ring and three raw stages cost 330 ns per K step at every M <= 128 and in every format,
+// against 104 ns of HBM time for Q4_K), so the shared memory that a small X tile leaves goes into more stages.
+//
+// Few tiles (a short prompt, a narrow matrix): the CTAs of a cluster share one tile, each taking a piece of K; the
+// accumulators meet over distributed shared memory and are added in K order, the same on every run.
 //
 // Same contract as gemm_wmma_kernel of the reference (src/hip/kernels/gemm.hpp:621-970): f16
 // staged operands, f32 accumulation; here the output stays f32.
@@ -34,7 +42,6 @@
 // runs to its end without waiting again and frees its tensor memory.
 #include <cuda.h>
 
-#include <cstdlib>
 #include <mutex>
 
 #include "krk_common.cuh"
@@ -46,67 +53,84 @@ namespace {
 constexpr int kTileN = 128;            // weight rows per tile (MMA M)
 constexpr int kMaxTileM = 256;         // tokens per tile (MMA N)
 constexpr int kBK = 64;                // K values per step: one 128-byte swizzle row of f16 X, 32 TMEM columns of A
-constexpr int kBStages = 4;            // X tiles in shared memory
+constexpr int kMaxB = 16, kMinB = 4;   // X tiles in shared memory
 constexpr int kAStages = 4;            // decoded weight tiles in tensor memory, two K steps (64 columns) each
-constexpr int kRawStages = 3;          // raw block columns (256 values x 128 rows) in shared memory, at most
-constexpr int kRawBytes = kTileN * 144;
-// Formats whose 256-value row segment is a multiple of 16 bytes arrive by TMA: Q4_K (144), Q4_0 (8 x 18 = 144),
-// Q5_K (176, two stages in the same area). Q8_0 arrives 128 values at a time: four 34-byte blocks = 136 bytes,
-// which start 0 or 8 bytes after a 16-byte boundary, so a 144-byte box that starts on the boundary covers them.
+constexpr int kMaxRaw = 8, kMinRaw = 2;   // raw block columns (256 values x 128 rows) in shared memory
+// Formats whose 256-value row segment is a multiple of 16 bytes arrive as one box per stage: Q4_K (144), Q4_0 and
+// IQ4_NL (8 x 18 = 144), Q5_K (176), Q5_0 (8 x 22 = 176), Q5_1 (8 x 24 = 192). Q8_0 arrives 128 values at a time:
+// four 34-byte blocks = 136 bytes, which start 0 or 8 bytes after a 16-byte boundary, so a 144-byte box that starts
+// on the boundary covers them.
 
-// Q6_K's 210-byte blocks start on even addresses only, but eight rows on, the address is the same modulo 16
-// (row lengths are even): the rows r = c (mod 8) of the matrix, seen from the 16-byte boundary at or before row
-// c, are a tensor with a 16-byte-multiple pitch. One map per c; a stage is eight boxes of 16 rows x 224 bytes
-// (the 16-byte granules that hold a block), and the 128 staged rows are in the order (c, k) <-> row c + 8k.
-__host__ __device__ constexpr bool row_phased(int wt) { return wt == KRK_CUDA_Q6_K; }
+// The 210-, 110- and 84-byte blocks of Q6_K, Q3_K and Q2_K start on even addresses only, but eight rows on, the
+// address is the same modulo 16 (row lengths are even): the rows r = c (mod 8) of the matrix, seen from the 16-byte
+// boundary at or before row c, are a tensor with a 16-byte-multiple pitch. One map per c; a stage is eight boxes of
+// 16 rows (the 16-byte granules that hold a block), and the 128 staged rows are in the order (c, k) <-> row c + 8k.
+// Slot pitches: 224 holds a Q6_K block at any lead; 144 (Q3_K) and 112 (Q2_K) keep the eight rows of a 16-byte load
+// phase on different banks.
+__host__ __device__ constexpr bool row_phased(int wt) { return wt == KRK_CUDA_Q6_K || wt == KRK_CUDA_Q3_K || wt == KRK_CUDA_Q2_K; }
 constexpr int kPhases = 8;
-__host__ __device__ constexpr bool tma_staged(int wt) {
-    return wt == KRK_CUDA_Q4_K || wt == KRK_CUDA_Q4_0 || wt == KRK_CUDA_Q5_K || wt == KRK_CUDA_Q8_0 || wt == KRK_CUDA_Q5_0 ||
-           wt == KRK_CUDA_Q5_1 || row_phased(wt);
-}
-// (Q5_0: eight 22-byte blocks = 176 bytes; Q5_1: eight 24-byte blocks = 192)
 __host__ __device__ constexpr int raw_seg(int wt) {
-    return (wt == KRK_CUDA_Q5_K || wt == KRK_CUDA_Q5_0) ? 176 : wt == KRK_CUDA_Q5_1 ? 192 : wt == KRK_CUDA_Q6_K ? 224 : 144;
+    return (wt == KRK_CUDA_Q5_K || wt == KRK_CUDA_Q5_0) ? 176 : wt == KRK_CUDA_Q5_1 ? 192 : wt == KRK_CUDA_Q6_K ? 224
+           : wt == KRK_CUDA_Q2_K ? 112 : 144;
 }
-// Which staged row and which weight row of the tile the decode thread of TMEM lane t works on. Phased formats:
-// a warp's 32 lanes take the rows 32w .. 32w + 31 of the tile (so the read-out writes 32 different banks) in
-// an order whose neighbouring lanes read staged rows on different banks.
-__host__ __device__ constexpr int tile_row(int wt, int t) { return row_phased(wt) ? ((t & 31) >> 2) + 8 * (4 * (t >> 5) + (t & 3)) : t; }
-__host__ __device__ constexpr int tile_slot(int wt, int t) { return row_phased(wt) ? 16 * ((t & 31) >> 2) + 4 * (t >> 5) + (t & 3) : t; }
+
+// What a launch computes. kDense: Y = X . W^T. The other two serve the routed experts, whose tiles come from a
+// device-side list of (expert, token group) entries: kGateUp takes 64 gate rows and the 64 up rows of the same
+// outputs as one weight tile and leaves f16 silu(gate) * up, kDown leaves f32 rows.
+enum GemmKind { kDense = 0, kGateUp = 1, kDown = 2 };
+
+// Which staged row and which weight row the decode thread of TMEM lane t works on. A weight tile is one run of 128
+// rows, or (kGateUp) 64 of each matrix. Phased formats: a warp's 32 lanes take 32 neighbouring rows (so the read-out
+// writes 32 different banks) in an order whose neighbouring lanes read staged rows on different banks.
+template <int WT, int KIND>
+__host__ __device__ constexpr int tile_row(int t) {   // row inside the tile; kGateUp: inside the matrix's half, up rows + 64
+    if (!row_phased(WT)) return t;
+    const int w = t >> 5, half = KIND == kGateUp ? w >> 1 : 0, wh = KIND == kGateUp ? w & 1 : w;
+    return 64 * half + ((t & 31) >> 2) + 8 * (4 * wh + (t & 3));
+}
+template <int WT, int KIND>
+__host__ __device__ constexpr int tile_slot(int t) {
+    if (!row_phased(WT)) return t;
+    const int w = t >> 5, half = KIND == kGateUp ? w >> 1 : 0, wh = KIND == kGateUp ? w & 1 : w;
+    return 64 * half + (KIND == kGateUp ? 8 : 16) * ((t & 31) >> 2) + 4 * wh + (t & 3);
+}
+template <int KIND>
 struct WMaps {
-    CUtensorMap m[kPhases];   // m[0] alone for the formats staged as one box
+    CUtensorMap m[KIND == kGateUp ? 2 * kPhases : kPhases];   // m[0] (kGateUp: m[0] gate, m[1] up) alone for the formats staged as one box
 };
-__host__ __device__ constexpr int raw_stages(int wt) { return raw_seg(wt) > 144 ? 2 : 3; }
-constexpr int kRawArea = 2 * kTileN * 224;
-static_assert(2 * kTileN * 192 <= kRawArea && kRawStages * kRawBytes <= kRawArea, "every format's stages fit the raw area");
-constexpr int kDecodeThreads = 256, kEpilogueThreads = 128;   // two decode threads per weight row
-constexpr int kThreads = kDecodeThreads + kEpilogueThreads + 96;
+constexpr int kDecodeGroups = 2, kGroupThreads = 256;   // two decode threads per weight row in each group
+constexpr int kDecodeThreads = kDecodeGroups * kGroupThreads, kEpilogueThreads = 128;
+constexpr int kDecodeWarps = kDecodeThreads / 32, kEpilogueWarps = kEpilogueThreads / 32;
+constexpr int kXWarp = kDecodeWarps + kEpilogueWarps, kRawWarp = kXWarp + 1, kMmaWarp = kXWarp + 2;
+constexpr int kThreads = 32 * (kMmaWarp + 1);
 constexpr int kTmemCols = 512, kTmemA = 256;
 constexpr int kYChunk = 32;            // tokens per TMA store of the read-out
-constexpr int kMaxPieces = 4;          // a cut tile has about this many pieces at most
+constexpr int kGroupBox = 32;          // tokens per X box of the expert kinds
+constexpr int kMaxSplit = 8;           // CTAs of a cluster that share a tile
 constexpr long long kWaitCycles = 4000000000LL;
+constexpr int kSmemMax = 227 * 1024;
 
 struct GemmParams {
-    const uint8_t *w;
     float *y;
+    __half *h;           // kGateUp: output [x rows][n_out] f16
     int64_t n_out, n_in, rows;
     int tile_m;          // tokens per tile: multiple of 16, <= 256
     int n_tiles_n, n_tiles_m;
     int row_bytes;
+    int n_b, n_raw;      // ring depths
+    int raw_off, y_off, bar_off;   // where the raw ring, the read-out buffers and the barriers start (the X ring starts at 0)
+    int split;           // CTAs per cluster, each with a piece of K (1: no cluster)
+    int y_tma;           // 1: tiles leave through shared memory and TMA stores (y 16-byte aligned, n_out % 4 == 0)
     int *status;
-    int split_tail;        // 1: cut the tiles left after the last whole wave over the CTAs along K (needs y_tma and the counters)
-    unsigned *tail_count;  // per tail tile: how many of its pieces (in K order) are in Y; zero at launch
-    int y_tma;             // 1: whole tiles leave through shared memory and TMA stores (y 16-byte aligned, n_out % 4 == 0)
+    const GemmGroup *groups;   // kGateUp, kDown: token groups, and how many
+    const int *n_groups;
 };
 
-struct __align__(1024) GemmSmem {
-    uint8_t b[kBStages][kMaxTileM * 128];      // X tiles, [tokens][64 f16], 128B swizzle (TMA)
-    uint8_t raw[kRawArea];                     // raw block bytes, stages of [128 rows][144, 176 or 224] (TMA), or the decode warps' own staging
-    float ystage[2][kYChunk][kTileN];          // accumulator read-out on its way to Y: [tokens][weight rows] (TMA store)
-    unsigned long long b_full[kBStages], b_empty[kBStages];
+struct GemmBars {
+    unsigned long long b_full[kMaxB], b_empty[kMaxB];
     unsigned long long a_full[kAStages], a_empty[kAStages];
-    unsigned long long raw_full[kRawStages], raw_empty[kRawStages];
-    unsigned long long d_full, d_empty;
+    unsigned long long raw_full[kMaxRaw], raw_empty[kMaxRaw];
+    unsigned long long d_full[2], d_empty[2];
     uint32_t tmem_base;
     int gave_up;
 };
@@ -157,10 +181,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int 
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
                  ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
 }
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap *map, int x, int y, uint32_t src) {
-    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
-                 ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
-}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
@@ -173,14 +193,26 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+// One K step: four MMAs over 16 K values each, A from tensor memory (lane = row, 32-bit column = two consecutive K
+// values, so 8 columns per MMA), B from shared memory (32 bytes of every row per MMA). `first`: the first MMA starts a
+// new sum. Executed by a whole converged warp whose operands are all warp-uniform, issued by the lane `elected` picks:
+// with the operands in uniform registers a step issues in 80 cycles; from a one-lane branch the operands go through
+// per-lane registers first and a step takes 470-510 cycles whatever N is (608 at N = 256 against the pipe's 512).
+__device__ __forceinline__ void umma_f16_ts_step(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t first, uint32_t elected) {
+    asm volatile("{\n .reg .pred p, q, t;\n .reg .b64 b1, b2, b3;\n .reg .b32 a1, a2, a3;\n"
+                 " setp.eq.b32 p, %4, 0;\n setp.ne.b32 q, %6, 0;\n setp.eq.b32 t, 0, 0;\n"
+                 " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
+                 " add.s32 a1, %1, 8;\n add.s32 a2, %1, 16;\n add.s32 a3, %1, 24;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, {%5, %5, %5, %5}, t;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, {%5, %5, %5, %5}, t;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, {%5, %5, %5, %5}, t;\n}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(first), "r"(0u), "r"(elected) : "memory");
 }
-// A from tensor memory (lane = row, 32-bit column = two consecutive K values), B from shared memory.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e;
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -188,8 +220,9 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
                    "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t elected) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+                 ::"r"(bar), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -221,252 +254,235 @@ __host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Cluster plumbing of the split-K form: barriers over all threads of the cluster's CTAs, and loads from another CTA's
+// shared memory.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_peer(uint32_t addr, int rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+
 // ---- decode of half a weight row's K step (32 values) to f16 ---------------------------------------
-// A decode thread first LOADS the raw bytes it needs (Raw), ahead of time, and later CONVERTS
-// them: out[j] holds values 2j, 2j+1 (low, high half) of its 32. f16 arithmetic runs on exact
-// small integers; the scale products are formed in f32 as the host decoder forms them and rounded
-// to f16 once.
+// A 256-value block column is four K steps. Decode group `grp` takes K steps 2 grp and 2 grp + 1 of it; a thread
+// (half h of its row) first LOADS the raw bytes it needs for both, then CONVERTS one step at a time: out[j] holds
+// values 2j, 2j+1 (low, high half) of its 32 (`half` is a template argument: it fixes shift distances). f16 arithmetic runs on exact small integers; the scale products are
+// formed in f32 as the host decoder forms them and rounded to f16 once. (A Q8_0 stage is two K steps: each group takes
+// one. Groups that took turns over whole stages would meet a ring slot only every other lap where the ring has an odd
+// number of slots, and a parity wait cannot tell a lap from the one two before it.)
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+// Byte i of t as an exact float plus 2^23: the byte under the exponent of 2^23.
+__device__ __forceinline__ float byte_plus_2_23(uint32_t t, int i) { return __uint_as_float(prmt(t, 0x4B000000u, 0x7650u + i)); }
+// Four quant bytes to two half2: (bytes 0, 1) and (bytes 2, 3), each under a 0x64 high byte, i.e. 1024 + q.
+__device__ __forceinline__ __half2 halves_lo(uint32_t t) { return bits_h2(__byte_perm(t, 0x64646464u, 0x4140)); }
+__device__ __forceinline__ __half2 halves_hi(uint32_t t) { return bits_h2(__byte_perm(t, 0x64646464u, 0x4342)); }
+// out[0..1] = (q - bias) * d, or (q - bias) * d + m, of the four quant bytes in t
+__device__ __forceinline__ void scale4(uint32_t t, __half2 bias, __half2 d, uint32_t *out) {
+    out[0] = h2_bits(__hmul2(__hsub2(halves_lo(t), bias), d));
+    out[1] = h2_bits(__hmul2(__hsub2(halves_hi(t), bias), d));
+}
+__device__ __forceinline__ void scale4(uint32_t t, __half2 bias, __half2 d, __half2 m, uint32_t *out) {
+    out[0] = h2_bits(__hfma2(__hsub2(halves_lo(t), bias), d, m));
+    out[1] = h2_bits(__hfma2(__hsub2(halves_hi(t), bias), d, m));
+}
+__device__ __forceinline__ __half2 half2_of_bits(uint32_t h) { return __half2half2(__ushort_as_half((unsigned short)h)); }
+__device__ __forceinline__ float float_of_half_bits(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
+template <int N>
+__device__ __forceinline__ void load_quads(const uint8_t *src, uint32_t *w) {   // N 16-byte loads
+    const uint4 *b = reinterpret_cast<const uint4 *>(src);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const uint4 v = b[i];
+        w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+    }
+}
+// Half of a block column whose halves are 8 bytes past a multiple of 16 long (72 or 88 bytes): `QUADS` 16-byte loads
+// and one of 8 bytes, before them in the second half.
+template <int QUADS>
+__device__ __forceinline__ void load_half_column(const uint8_t *column, int grp, uint32_t (&w)[4 * QUADS + 2]) {
+    if (grp == 0) {
+        load_quads<QUADS>(column, w);
+        const uint2 v = *reinterpret_cast<const uint2 *>(column + 16 * QUADS);
+        w[4 * QUADS] = v.x, w[4 * QUADS + 1] = v.y;
+    } else {
+        const uint2 v = *reinterpret_cast<const uint2 *>(column + 16 * QUADS + 8);
+        w[0] = v.x, w[1] = v.y;
+        load_quads<QUADS>(column + 16 * QUADS + 16, w + 2);
+    }
+}
 
 template <int WT>
-struct Raw {   // formats without a packed decoder (IQ4_NL, Q2_K, Q3_K): raw bytes staged in shared memory, decoded element by element
-    static constexpr int kSteps = 4;                                                       // K steps per stage
-    static constexpr int kRowSeg = kSteps * kBK / block_size(WT) * block_bytes(WT);       // bytes of one row per stage
-    static constexpr int kStageBytes = kTileN * kRowSeg;
-    // Staging granule: with K a multiple of 256 the rows and the segments start on a multiple of it (144-byte
-    // segments: 8 bytes; Q2_K's 84: 4; Q3_K's 110: 2).
-    static constexpr int kGran = kRowSeg % 8 == 0 ? 8 : kRowSeg % 4 == 0 ? 4 : 2;
-    static constexpr int kUnits = kStageBytes / kGran;
-    static constexpr int kPer = (kUnits + kDecodeThreads - 1) / kDecodeThreads;            // loads per thread
-    static constexpr int kWords = kGran == 8 ? 2 : 1;
-    static_assert(kStageBytes <= kRawStages * kRawBytes / 2, "two stages must fit the raw staging area");
-    uint32_t pre[kWords * kPer];   // this thread's share of the NEXT stage, on its way from global memory
-    const uint8_t *stage;     // the stage being decoded, [128 rows][kRowSeg]
-    // Loads of stage `ks` (K steps ks .. ks + kSteps of weight rows n0 ..): neighbouring threads take
-    // neighbouring granules of a row. Rows past n_out read as zero blocks.
-    __device__ __forceinline__ void fetch(const uint8_t *w, int64_t n0, int64_t n_out, int row_bytes, int ks, int tid) {
-        const size_t seg = (size_t)(ks * kBK / block_size(WT)) * block_bytes(WT);
+struct Raw;
+
+// The eight words that start `o` bytes (even) into a slot.
+__device__ __forceinline__ void window(const uint8_t *slot, int o, uint32_t (&y)[8]) {
+    uint32_t x[12];
+    load_quads<3>(slot + (o & ~15), x);
+    const bool by2 = (o & 8) != 0, by1 = (o & 4) != 0;
 #pragma unroll
-        for (int j = 0; j < kPer; j++) {
-            const int i = tid + j * kDecodeThreads;
-            const int rr = i / (kRowSeg / kGran), col = i - rr * (kRowSeg / kGran);
-            const bool ok = i < kUnits && n0 + rr < n_out;
-            const uint8_t *src = w + (size_t)(n0 + rr) * row_bytes + seg + (size_t)col * kGran;
-            if constexpr (kGran == 8) {
-                uint2 v = make_uint2(0u, 0u);
-                if (ok) v = __ldg(reinterpret_cast<const uint2 *>(src));
-                pre[2 * j] = v.x;
-                pre[2 * j + 1] = v.y;
-            } else if constexpr (kGran == 4) {
-                pre[j] = ok ? __ldg(reinterpret_cast<const uint32_t *>(src)) : 0u;
-            } else {
-                pre[j] = ok ? (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(src)) : 0u;
-            }
-        }
-    }
-    __device__ __forceinline__ void stash(uint8_t *dst, int tid) {
+    for (int i = 0; i < 10; i++) x[i] = by2 ? x[i + 2] : x[i];
 #pragma unroll
-        for (int j = 0; j < kPer; j++) {
-            const int i = tid + j * kDecodeThreads;
-            if (i < kUnits) {
-                if constexpr (kGran == 8) reinterpret_cast<uint2 *>(dst)[i] = make_uint2(pre[2 * j], pre[2 * j + 1]);
-                else if constexpr (kGran == 4) reinterpret_cast<uint32_t *>(dst)[i] = pre[j];
-                else reinterpret_cast<unsigned short *>(dst)[i] = (unsigned short)pre[j];
-            }
-        }
-        stage = dst;
-    }
-    __device__ __forceinline__ void convert(int j, int half, int r, uint32_t (&out)[16]) const {
-        const uint8_t *row = stage + (size_t)r * kRowSeg;
+    for (int i = 0; i < 9; i++) x[i] = by1 ? x[i + 1] : x[i];
+    const int sh = 8 * (o & 2);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int64_t k = (int64_t)j * kBK + 32 * half + 2 * i;   // relative to the stage: stages start on block boundaries
-            out[i] = h2_bits(__floats2half2_rn(decode_value<WT>(row, k), decode_value<WT>(row, k + 1)));
-        }
-    }
-};
+    for (int i = 0; i < 8; i++) y[i] = __funnelshift_r(x[i], x[i + 1], sh);
+}
 
 // Q6_K: the staged slot of a row holds its 210-byte block (src/quant.cpp:491-512) `lead` bytes (even, 0..14)
-// after the slot's 16-byte-aligned start. A thread (half h of its row) takes what its four chunks need into
-// registers at once: for each 128-value half hf the 32 ql bytes at 64 hf + 32 h and the 32 qh bytes at
-// 128 + 32 hf, each read as three 128-bit words and moved down by lead's word and half-word parts; its four
-// scale pairs; d. Chunk c = 2j + h then is quad = c & 3 of half hf = j >> 1: the low (quad < 2) or high nibbles
-// of those ql bytes and bit pair `quad` of the qh bytes, four quants per step.
+// after the slot's 16-byte-aligned start. Group grp takes 128-value half grp: its thread half h the 32 ql bytes at
+// 64 grp + 32 h, the 32 qh bytes at 128 + 32 grp, two scale pairs and d. Step j's chunk is quad 2j + h: the low (j = 0)
+// or high nibbles of those ql bytes and bit pair 2j + h of the qh bytes, four quants per operation.
 template <>
 struct Raw<KRK_CUDA_Q6_K> {
     static constexpr int kSteps = 4;
-    uint32_t ql[2][8], qh[2][8], sc[4], dbits;
+    uint32_t ql[8], qh[8], sc[2], dbits;
     int lead = 0;
-    // the eight words that start `o` bytes (even) into the slot
-    __device__ __forceinline__ static void window(const uint8_t *slot, int o, uint32_t (&y)[8]) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(slot + (o & ~15));
-        const uint4 v0 = b[0], v1 = b[1], v2 = b[2];
-        uint32_t x[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
-        const bool by2 = (o & 8) != 0, by1 = (o & 4) != 0;
+    __device__ __forceinline__ void load_block(const uint8_t *slot, int half, int, int grp) {
+        window(slot, lead + 64 * grp + 32 * half, ql);
+        window(slot, lead + 128 + 32 * grp, qh);
 #pragma unroll
-        for (int i = 0; i < 10; i++) x[i] = by2 ? x[i + 2] : x[i];
-#pragma unroll
-        for (int i = 0; i < 9; i++) x[i] = by1 ? x[i + 1] : x[i];
-        const int sh = 8 * (o & 2);
-#pragma unroll
-        for (int i = 0; i < 8; i++) y[i] = __funnelshift_r(x[i], x[i + 1], sh);
-    }
-    __device__ __forceinline__ void load_block(const uint8_t *slot, int half, int) {
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            window(slot, lead + 64 * hf + 32 * half, ql[hf]);
-            window(slot, lead + 128 + 32 * hf, qh[hf]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            sc[j] = *reinterpret_cast<const unsigned short *>(slot + lead + 192 + 8 * (j >> 1) + 4 * (j & 1) + 2 * half);
+        for (int j = 0; j < 2; j++) sc[j] = *reinterpret_cast<const unsigned short *>(slot + lead + 192 + 8 * grp + 4 * j + 2 * half);
         dbits = *reinterpret_cast<const unsigned short *>(slot + lead + 208);
     }
     // f16(d * scale) is formed in f32 as the host decoder forms d * scale.
-    __device__ __forceinline__ void convert(int j, int half, int, uint32_t (&out)[16]) const {
-        const int hf = j >> 1, nib = (j & 1) ? 4 : 0, hs = 4 * (j & 1) + 2 * half;
-        const float d = __half2float(__ushort_as_half((unsigned short)dbits));
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const float d = float_of_half_bits(dbits);
         const __half2 dl0 = __float2half2_rn(__fmul_rn(d, (float)(int8_t)(sc[j] & 0xFF)));
         const __half2 dl1 = __float2half2_rn(__fmul_rn(d, (float)(int8_t)(sc[j] >> 8)));
-        const __half2 bias = __float2half2_rn(1056.0f);   // 0x6400 | q is the half 1024 + q; the quant is q - 32
+        const __half2 bias = __float2half2_rn(1056.0f);   // 1024 + q; the quant is q - 32
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t t = ((ql[hf][i] >> nib) & 0x0F0F0F0Fu) | (((qh[hf][i] >> hs) & 0x03030303u) << 4);
-            const __half2 dl = i < 4 ? dl0 : dl1;
-            out[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(t, 0x64646464u, 0x5140)), bias), dl));
-            out[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(t, 0x64646464u, 0x7362)), bias), dl));
+            const int up = 4 - (4 * j + 2 * half);   // bit pair 2j + half of every qh byte to bits 4 and 5
+            const uint32_t hi = (up >= 0 ? qh[i] << up : qh[i] >> -up) & 0x30303030u;
+            const uint32_t t = ((ql[i] >> (4 * j)) & 0x0F0F0F0Fu) | hi;
+            scale4(t, bias, i < 4 ? dl0 : dl1, out + 2 * i);
         }
     }
 };
 
-// Q4_K: one load() takes a whole 144-byte super-block = four K steps (from the TMA-staged tile in
-// shared memory). K step p of the block covers chunks 2p, 2p+1: the low and the high nibbles of the
+// The 6-bit scales and mins of chunks 4 grp .. 4 grp + 3 of a Q4_K / Q5_K header, a byte each (src/quant.cpp:427-435).
+__device__ __forceinline__ void k_scales(const uint4 &hdr, int grp, uint32_t &sc, uint32_t &mn) {
+    if (grp == 0) {
+        sc = hdr.y & 0x3F3F3F3Fu;
+        mn = hdr.z & 0x3F3F3F3Fu;
+    } else {
+        sc = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+        mn = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+    }
+}
+
+// Q4_K: K step p of the 144-byte block covers chunks 2p, 2p+1: the low and the high nibbles of the
 // same 32 bytes (src/quant.cpp:437-460). Thread half h converts chunk 2p+h.
 template <>
 struct Raw<KRK_CUDA_Q4_K> {
     static constexpr int kSteps = 4;
-    uint4 hdr, q[8];
-    __device__ __forceinline__ void load_block(const uint8_t *block, int, int) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(block);
-        hdr = b[0];
-#pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = b[1 + i];
+    uint32_t q[16], sc, mn, dd;
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) {
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(block);
+        load_quads<4>(block + 16 + 64 * grp, q);
+        k_scales(hdr, grp, sc, mn);
+        dd = hdr.x;
     }
-    __device__ __forceinline__ void convert(int p, int half, int, uint32_t (&out)[16]) const {
-        // 6-bit scale / min of chunk c = 2p + half out of the 12 packed bytes in hdr.y, hdr.z, hdr.w
-        // (src/quant.cpp:427-435)
-        const int c = 2 * p + half;
-        int sc, mn;
-        if (c < 4) {
-            sc = (hdr.y >> (8 * c)) & 63;
-            mn = (hdr.z >> (8 * c)) & 63;
-        } else {
-            const int sh = 8 * (c - 4);
-            sc = ((hdr.w >> sh) & 0xF) | (((hdr.y >> (sh + 6)) & 3) << 4);
-            mn = ((hdr.w >> (sh + 4)) & 0xF) | (((hdr.z >> (sh + 6)) & 3) << 4);
-        }
-        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xFFFF)));
-        const float dm = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        const __half2 dl = __float2half2_rn(__fmul_rn(d, (float)sc)), ml = __float2half2_rn(-__fmul_rn(dm, (float)mn));
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const int k = 2 * j + half;
+        const float s = byte_plus_2_23(sc, k) - 8388608.0f, m = byte_plus_2_23(mn, k) - 8388608.0f;
+        const __half2 dl = __float2half2_rn(__fmul_rn(float_of_half_bits(dd & 0xFFFF), s));
+        const __half2 ml = __float2half2_rn(-__fmul_rn(float_of_half_bits(dd >> 16), m));
         const __half2 k1024 = __float2half2_rn(1024.0f);
-        const uint32_t qw[8] = {q[2 * p].x, q[2 * p].y, q[2 * p].z, q[2 * p].w, q[2 * p + 1].x, q[2 * p + 1].y, q[2 * p + 1].z, q[2 * p + 1].w};
-        const int shift = 4 * half;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            // bytes 4i..4i+3 hold values 4i..4i+3 of the chunk; 0x6400 | q is the half 1024 + q
-            const uint32_t t = (qw[i] >> shift) & 0x0F0F0F0Fu;
-            const uint32_t v01 = __byte_perm(t, 0x64646464u, 0x5140), v23 = __byte_perm(t, 0x64646464u, 0x7362);
-            out[2 * i] = h2_bits(__hfma2(__hsub2(bits_h2(v01), k1024), dl, ml));
-            out[2 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(v23), k1024), dl, ml));
-        }
-    }
-};
-
-// Q4_0: eight 18-byte blocks per 256 values = the same 144-byte column as Q4_K. K step p covers blocks 2p
-// (thread half 0) and 2p + 1 (half 1): block 2p starts on a word of the 144 bytes, block 2p + 1 half a word
-// later, so its 16 quant bytes are whole words (src/quant.cpp:331-339).
-template <>
-struct Raw<KRK_CUDA_Q4_0> {
-    static constexpr int kSteps = 4;
-    uint32_t w[36];
-    __device__ __forceinline__ void load_block(const uint8_t *block, int, int) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(block);
-#pragma unroll
-        for (int i = 0; i < 9; i++) {
-            const uint4 v = b[i];
-            w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
-        }
-    }
-    __device__ __forceinline__ void convert(int p, int half, int, uint32_t (&out)[16]) const {
-        uint32_t q[4], dbits;
-        if (half == 0) {
-            dbits = w[9 * p] & 0xFFFFu;
-#pragma unroll
-            for (int i = 0; i < 4; i++) q[i] = __funnelshift_r(w[9 * p + i], w[9 * p + i + 1], 16);
-        } else {
-            dbits = w[9 * p + 4] >> 16;
-#pragma unroll
-            for (int i = 0; i < 4; i++) q[i] = w[9 * p + 5 + i];
-        }
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits));
-        const __half2 bias = __float2half2_rn(1032.0f);   // 0x6400 | q is the half 1024 + q; the quant is q - 8
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            // byte b of the block: value b in its low nibble, value 16 + b in its high one
-            const uint32_t lo = q[i] & 0x0F0F0F0Fu, hi = (q[i] >> 4) & 0x0F0F0F0Fu;
-            out[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x5140)), bias), d2));
-            out[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x7362)), bias), d2));
-            out[8 + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x5140)), bias), d2));
-            out[8 + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x7362)), bias), d2));
-        }
+        for (int i = 0; i < 8; i++) scale4((q[8 * j + i] >> (4 * half)) & 0x0F0F0F0Fu, k1024, dl, ml, out + 2 * i);
     }
 };
 
 // Q5_K: the 176-byte super-block (src/quant.cpp:462-489) is Q4_K's header and nibbles plus 32 mask bytes whose
-// bit c is the fifth quant bit of chunk c. K step p covers chunks 2p, 2p + 1; thread half h converts 2p + h.
+// bit c is the fifth quant bit of chunk c.
 template <>
 struct Raw<KRK_CUDA_Q5_K> {
     static constexpr int kSteps = 4;
-    uint4 hdr;
-    uint32_t qh[8], q[32];
-    __device__ __forceinline__ void load_block(const uint8_t *block, int, int) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(block);
-        hdr = b[0];
+    uint32_t q[16], qh[8], sc, mn, dd;
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) {
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(block);
+        load_quads<2>(block + 16, qh);
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const uint4 v = b[1 + i];
-            qh[4 * i] = v.x, qh[4 * i + 1] = v.y, qh[4 * i + 2] = v.z, qh[4 * i + 3] = v.w;
-        }
+        for (int i = 0; i < 8; i++) qh[i] >>= 4 * grp;
+        load_quads<4>(block + 48 + 64 * grp, q);
+        k_scales(hdr, grp, sc, mn);
+        dd = hdr.x;
+    }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const int k = 2 * j + half, up = 4 - k;   // (the masks were moved down by the group's 4 bits when loaded)
+        const float s = byte_plus_2_23(sc, k) - 8388608.0f, m = byte_plus_2_23(mn, k) - 8388608.0f;
+        const __half2 dl = __float2half2_rn(__fmul_rn(float_of_half_bits(dd & 0xFFFF), s));
+        const __half2 ml = __float2half2_rn(-__fmul_rn(float_of_half_bits(dd >> 16), m));
+        const __half2 k1024 = __float2half2_rn(1024.0f);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint4 v = b[3 + i];
-            q[4 * i] = v.x, q[4 * i + 1] = v.y, q[4 * i + 2] = v.z, q[4 * i + 3] = v.w;
+        for (int i = 0; i < 8; i++)
+            scale4(((q[8 * j + i] >> (4 * half)) & 0x0F0F0F0Fu) | ((qh[i] << up) & 0x10101010u), k1024, dl, ml, out + 2 * i);
+    }
+};
+
+// Q4_0: eight 18-byte blocks per 256 values = the same 144-byte column as Q4_K. K step p covers blocks 2p
+// (thread half 0) and 2p + 1 (half 1): block 2p starts on a word of the column, block 2p + 1 half a word
+// later, so its 16 quant bytes are whole words (src/quant.cpp:331-339). (Both candidates with constant indices, then a
+// select: `half` in the index would put w[] in local memory.)
+template <>
+struct Raw<KRK_CUDA_Q4_0> {
+    static constexpr int kSteps = 4;
+    uint32_t w[18];
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<4>(block, grp, w); }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const __half2 d2 = half2_of_bits(half ? (w[9 * j + 4] >> 16) : (w[9 * j] & 0xFFFFu));
+        const __half2 bias = __float2half2_rn(1032.0f);   // 1024 + q; the quant is q - 8
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            // byte b of the block: value b in its low nibble, value 16 + b in its high one
+            const uint32_t q = half ? w[9 * j + 5 + i] : __funnelshift_r(w[9 * j + i], w[9 * j + i + 1], 16);
+            scale4(q & 0x0F0F0F0Fu, bias, d2, out + 2 * i);
+            scale4((q >> 4) & 0x0F0F0F0Fu, bias, d2, out + 8 + 2 * i);
         }
     }
-    __device__ __forceinline__ void convert(int p, int half, int, uint32_t (&out)[16]) const {
-        const int c = 2 * p + half;
-        int sc, mn;
-        if (c < 4) {
-            sc = (hdr.y >> (8 * c)) & 63;
-            mn = (hdr.z >> (8 * c)) & 63;
-        } else {
-            const int sh = 8 * (c - 4);
-            sc = ((hdr.w >> sh) & 0xF) | (((hdr.y >> (sh + 6)) & 3) << 4);
-            mn = ((hdr.w >> (sh + 4)) & 0xF) | (((hdr.z >> (sh + 6)) & 3) << 4);
-        }
-        const float d = __half2float(__ushort_as_half((unsigned short)(hdr.x & 0xFFFF)));
-        const float dm = __half2float(__ushort_as_half((unsigned short)(hdr.x >> 16)));
-        const __half2 dl = __float2half2_rn(__fmul_rn(d, (float)sc)), ml = __float2half2_rn(-__fmul_rn(dm, (float)mn));
-        const __half2 k1024 = __float2half2_rn(1024.0f);
-        const int shift = 4 * half;
+};
+
+// IQ4_NL: Q4_0's block with indices into a grid of 16 signed bytes (src/quant.cpp:88-91, 566-575). The grid lies in
+// four words, biased by 128; a byte permute looks four indices up in half of it at a time and another permute in its
+// sign-replicating mode makes the mask that picks between the halves by the index's top bit. d is an f16 and the
+// grid value an exact one, so the product is rounded once.
+template <>
+struct Raw<KRK_CUDA_IQ4_NL> {
+    static constexpr int kSteps = 4;
+    uint32_t w[18];
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<4>(block, grp, w); }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        constexpr uint32_t kG0 = 0x3F2D1801u, kG1 = 0x766A5D4Fu, kG2 = 0xA6998D81u, kG3 = 0xF1D9C5B5u;   // grid + 128
+        const __half2 d2 = half2_of_bits(half ? (w[9 * j + 4] >> 16) : (w[9 * j] & 0xFFFFu));
+        const __half2 bias = __float2half2_rn(1152.0f);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t t = ((q[8 * p + i] >> shift) & 0x0F0F0F0Fu) | (((qh[i] >> c) & 0x01010101u) << 4);
-            const uint32_t v01 = __byte_perm(t, 0x64646464u, 0x5140), v23 = __byte_perm(t, 0x64646464u, 0x7362);
-            out[2 * i] = h2_bits(__hfma2(__hsub2(bits_h2(v01), k1024), dl, ml));
-            out[2 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(v23), k1024), dl, ml));
+        for (int i = 0; i < 4; i++) {
+            const uint32_t q = half ? w[9 * j + 5 + i] : __funnelshift_r(w[9 * j + i], w[9 * j + i + 1], 16);
+            const uint32_t s = q & 0x77777777u, s2 = s >> 16, y = q << 4;
+            const uint32_t m01 = prmt(y, q, 0xD9C8u), m23 = prmt(y, q, 0xFBEAu);   // 0xFF where the index is 8..15
+            const uint32_t r01 = (prmt(kG0, kG1, s) & ~m01) | (prmt(kG2, kG3, s) & m01);     // [low 0, high 0, low 1, high 1]
+            const uint32_t r23 = (prmt(kG0, kG1, s2) & ~m23) | (prmt(kG2, kG3, s2) & m23);
+            out[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(r01, 0x64646464u, 0x4240)), bias), d2));
+            out[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(r23, 0x64646464u, 0x4240)), bias), d2));
+            out[8 + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(r01, 0x64646464u, 0x4341)), bias), d2));
+            out[8 + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(r23, 0x64646464u, 0x4341)), bias), d2));
         }
     }
 };
@@ -476,38 +492,24 @@ __device__ __forceinline__ uint32_t spread_fifth(uint32_t b) { return (((b & 0xF
 
 // Q5_0: eight 22-byte blocks per 256 values (src/quant.cpp:351-364): f16 d, 32 fifth bits, 16 bytes whose low nibbles
 // are quants 0..15 and whose high nibbles are quants 16..31; value = d * (q - 16). K step p covers blocks 2p (thread
-// half 0: the block starts on a word of the 176 bytes) and 2p + 1 (half 1: half a word later, so its bit word and its
+// half 0: the block starts on a word of the column) and 2p + 1 (half 1: half a word later, so its bit word and its
 // quant bytes are whole words).
 template <>
 struct Raw<KRK_CUDA_Q5_0> {
     static constexpr int kSteps = 4;
-    uint32_t w[44];
-    __device__ __forceinline__ void load_block(const uint8_t *block, int, int) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(block);
-#pragma unroll
-        for (int i = 0; i < 11; i++) {
-            const uint4 v = b[i];
-            w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
-        }
-    }
-    __device__ __forceinline__ void convert(int p, int half, int, uint32_t (&out)[16]) const {
-        // (both candidates with constant indices, then a select: a branch on `half` would index w[] dynamically)
-        const int W = 11 * p;
-        uint32_t q[4];
-        const uint32_t dbits = half ? (w[W + 5] >> 16) : (w[W] & 0xFFFFu);
+    uint32_t w[22];
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<5>(block, grp, w); }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const int W = 11 * j;
+        const __half2 d2 = half2_of_bits(half ? (w[W + 5] >> 16) : (w[W] & 0xFFFFu));
         const uint32_t qh = half ? w[W + 6] : __funnelshift_r(w[W], w[W + 1], 16);
-#pragma unroll
-        for (int i = 0; i < 4; i++) q[i] = half ? w[W + 7 + i] : __funnelshift_r(w[W + 1 + i], w[W + 2 + i], 16);
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits));
-        const __half2 bias = __float2half2_rn(1040.0f);   // 0x6400 | q is the half 1024 + q; the quant is q - 16
+        const __half2 bias = __float2half2_rn(1040.0f);   // 1024 + q; the quant is q - 16
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t lo = (q[i] & 0x0F0F0F0Fu) | spread_fifth(qh >> (4 * i));
-            const uint32_t hi = ((q[i] >> 4) & 0x0F0F0F0Fu) | spread_fifth(qh >> (16 + 4 * i));
-            out[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x5140)), bias), d2));
-            out[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x7362)), bias), d2));
-            out[8 + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x5140)), bias), d2));
-            out[8 + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x7362)), bias), d2));
+            const uint32_t q = half ? w[W + 7 + i] : __funnelshift_r(w[W + 1 + i], w[W + 2 + i], 16);
+            scale4((q & 0x0F0F0F0Fu) | spread_fifth(qh >> (4 * i)), bias, d2, out + 2 * i);
+            scale4(((q >> 4) & 0x0F0F0F0Fu) | spread_fifth(qh >> (16 + 4 * i)), bias, d2, out + 8 + 2 * i);
         }
     }
 };
@@ -517,406 +519,419 @@ struct Raw<KRK_CUDA_Q5_0> {
 template <>
 struct Raw<KRK_CUDA_Q5_1> {
     static constexpr int kSteps = 4;
-    uint32_t w[48];
-    __device__ __forceinline__ void load_block(const uint8_t *block, int, int) {
-        const uint4 *b = reinterpret_cast<const uint4 *>(block);
-#pragma unroll
-        for (int i = 0; i < 12; i++) {
-            const uint4 v = b[i];
-            w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
-        }
-    }
-    __device__ __forceinline__ void convert(int p, int half, int, uint32_t (&out)[16]) const {
-        // (the block's six words picked with constant indices and a select: `half` in the index would put w[] in
-        // local memory)
+    uint32_t w[24];
+    __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_quads<6>(block + 96 * grp, w); }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         uint32_t b[6];
 #pragma unroll
-        for (int i = 0; i < 6; i++) b[i] = half ? w[12 * p + 6 + i] : w[12 * p + i];
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)(b[0] & 0xFFFFu)));
-        const __half2 m2 = __half2half2(__ushort_as_half((unsigned short)(b[0] >> 16)));
+        for (int i = 0; i < 6; i++) b[i] = half ? w[12 * j + 6 + i] : w[12 * j + i];
+        const __half2 d2 = half2_of_bits(b[0] & 0xFFFFu), m2 = half2_of_bits(b[0] >> 16);
         const uint32_t qh = b[1];
         const __half2 k1024 = __float2half2_rn(1024.0f);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t qw = b[2 + i];
-            const uint32_t lo = (qw & 0x0F0F0F0Fu) | spread_fifth(qh >> (4 * i));
-            const uint32_t hi = ((qw >> 4) & 0x0F0F0F0Fu) | spread_fifth(qh >> (16 + 4 * i));
-            out[2 * i] = h2_bits(__hfma2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x5140)), k1024), d2, m2));
-            out[2 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(__byte_perm(lo, 0x64646464u, 0x7362)), k1024), d2, m2));
-            out[8 + 2 * i] = h2_bits(__hfma2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x5140)), k1024), d2, m2));
-            out[8 + 2 * i + 1] = h2_bits(__hfma2(__hsub2(bits_h2(__byte_perm(hi, 0x64646464u, 0x7362)), k1024), d2, m2));
+            const uint32_t q = b[2 + i];
+            scale4((q & 0x0F0F0F0Fu) | spread_fifth(qh >> (4 * i)), k1024, d2, m2, out + 2 * i);
+            scale4(((q >> 4) & 0x0F0F0F0Fu) | spread_fifth(qh >> (16 + 4 * i)), k1024, d2, m2, out + 8 + 2 * i);
         }
     }
 };
 
 // Q8_0: a stage is 128 values = four 34-byte blocks (f16 d, 32 int8; src/quant.cpp:381-387) inside a 144-byte
-// box that starts 0 (even stage) or 8 (odd stage) bytes before them. K step p covers blocks 2p (thread half 0)
-// and 2p + 1 (half 1); a thread takes only its own two blocks, as nine words each: block 2p starts on a word,
+// box that starts 0 (even stage) or 8 (odd stage) bytes before them. K step p = grp covers blocks 2p (thread half 0)
+// and 2p + 1 (half 1); a thread takes only its own block, as nine words: block 2p starts on a word,
 // block 2p + 1 half a word later, so its quants are whole words.
 template <>
 struct Raw<KRK_CUDA_Q8_0> {
     static constexpr int kSteps = 2;
-    uint32_t w[2][9];
-    int odd;
-    __device__ __forceinline__ void load_block(const uint8_t *box, int half, int ks) {
-        odd = half;
-        const uint32_t *b = reinterpret_cast<const uint32_t *>(box + 8 * ((ks >> 1) & 1) + 32 * half);
+    uint32_t w[9];
+    __device__ __forceinline__ void load_block(const uint8_t *box, int half, int ks, int grp) {
+        const uint32_t *b = reinterpret_cast<const uint32_t *>(box + 8 * ((ks >> 1) & 1) + 32 * half + 68 * grp);
 #pragma unroll
-        for (int p = 0; p < 2; p++)
-#pragma unroll
-            for (int i = 0; i < 9; i++) w[p][i] = b[17 * p + i];
+        for (int i = 0; i < 9; i++) w[i] = b[i];
     }
-    __device__ __forceinline__ void convert(int p, int, int, uint32_t (&out)[16]) const {
-        uint32_t q[8], dbits;
-        if (odd == 0) {
-            dbits = w[p][0] & 0xFFFFu;
-#pragma unroll
-            for (int i = 0; i < 8; i++) q[i] = __funnelshift_r(w[p][i], w[p][i + 1], 16);
-        } else {
-            dbits = w[p][0] >> 16;
-#pragma unroll
-            for (int i = 0; i < 8; i++) q[i] = w[p][1 + i];
-        }
-        const __half2 d2 = __half2half2(__ushort_as_half((unsigned short)dbits));
+    template <int half>
+    __device__ __forceinline__ void convert(int, uint32_t (&out)[16]) const {
+        const __half2 d2 = half2_of_bits(half ? (w[0] >> 16) : (w[0] & 0xFFFFu));
         const __half2 bias = __float2half2_rn(1152.0f);   // q ^ 0x80 under a 0x64 high byte is the half 1024 + 128 + q
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t t = q[i] ^ 0x80808080u;
-            out[2 * i] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(t, 0x64646464u, 0x5140)), bias), d2));
-            out[2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(__byte_perm(t, 0x64646464u, 0x7362)), bias), d2));
+            const uint32_t q = half ? w[1 + i] : __funnelshift_r(w[i], w[i + 1], 16);
+            scale4(q ^ 0x80808080u, bias, d2, out + 2 * i);
+        }
+    }
+};
+
+// Q2_K (84-byte super-blocks, src/quant.cpp:398-424) and Q3_K (110, src/quant.cpp:514-553). Step j of group grp covers
+// 2-bit fields 2j + h (thread half h) of the 32 quant bytes of 128-value half grp, two scales of 16 values each.
+// Their scale products need more than 11 bits, so a value is formed in f32 exactly as the host decoder forms it
+// and rounded to f16 once (single-precision arithmetic also issues at twice the rate of the packed f16 kind).
+template <>
+struct Raw<KRK_CUDA_Q2_K> {
+    static constexpr int kSteps = 4;
+    uint32_t q[8], sc[2], dm;
+    int lead = 0;
+    __device__ __forceinline__ void load_block(const uint8_t *slot, int, int, int grp) {
+        window(slot, lead + 16 + 32 * grp, q);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(slot + lead);   // 84-byte blocks: word aligned
+        sc[0] = w[2 * grp];
+        sc[1] = w[2 * grp + 1];
+        dm = w[20];
+    }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const float d = float_of_half_bits(dm & 0xFFFF), dmin = float_of_half_bits(dm >> 16);
+        const uint32_t lo = sc[j] & 0x0F0F0F0Fu, hi = (sc[j] >> 4) & 0x0F0F0F0Fu;   // scales, minimums: bytes 2h, 2h + 1 are this chunk's
+        const float dl0 = __fmul_rn(d, byte_plus_2_23(lo, 2 * half) - 8388608.0f), dl1 = __fmul_rn(d, byte_plus_2_23(lo, 2 * half + 1) - 8388608.0f);
+        const float ml0 = -__fmul_rn(dmin, byte_plus_2_23(hi, 2 * half) - 8388608.0f), ml1 = -__fmul_rn(dmin, byte_plus_2_23(hi, 2 * half + 1) - 8388608.0f);
+        const int shift = 4 * j + 2 * half;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t t = (q[i] >> shift) & 0x03030303u;
+            const float dl = i < 4 ? dl0 : dl1, ml = i < 4 ? ml0 : ml1;
+            const float v0 = fmaf(dl, byte_plus_2_23(t, 0) - 8388608.0f, ml), v1 = fmaf(dl, byte_plus_2_23(t, 1) - 8388608.0f, ml);
+            const float v2 = fmaf(dl, byte_plus_2_23(t, 2) - 8388608.0f, ml), v3 = fmaf(dl, byte_plus_2_23(t, 3) - 8388608.0f, ml);
+            out[2 * i] = h2_bits(__floats2half2_rn(v0, v1));
+            out[2 * i + 1] = h2_bits(__floats2half2_rn(v2, v3));
+        }
+    }
+};
+template <>
+struct Raw<KRK_CUDA_Q3_K> {
+    static constexpr int kSteps = 4;
+    uint32_t q[8], hm[8], sc[2];
+    float d;
+    int lead = 0;
+    __device__ __forceinline__ void load_block(const uint8_t *slot, int, int, int grp) {
+        window(slot, lead, hm);
+#pragma unroll
+        for (int i = 0; i < 8; i++) hm[i] >>= 4 * grp;   // mask bit 4 grp + f to bit f
+        window(slot, lead + 32 + 32 * grp, q);
+        const unsigned short *u = reinterpret_cast<const unsigned short *>(slot + lead + 96);
+        const uint32_t a0 = u[0] | ((uint32_t)u[1] << 16), a1 = u[2] | ((uint32_t)u[3] << 16), a2 = u[4] | ((uint32_t)u[5] << 16);
+        d = float_of_half_bits(u[6]);
+        // scale i: low four bits in the nibbles of bytes 0..7, high two in byte 8 + i % 4 at bits 2 * (i / 4)
+        sc[0] = ((a0 >> (4 * grp)) & 0x0F0F0F0Fu) | (((a2 >> (4 * grp)) << 4) & 0x30303030u);
+        sc[1] = ((a1 >> (4 * grp)) & 0x0F0F0F0Fu) | (((a2 >> (4 * grp)) << 2) & 0x30303030u);
+    }
+    template <int half>
+    __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
+        const float dl0 = __fmul_rn(d, byte_plus_2_23(sc[j], 2 * half) - 8388640.0f);   // d * (scale - 32)
+        const float dl1 = __fmul_rn(d, byte_plus_2_23(sc[j], 2 * half + 1) - 8388640.0f);
+        const int f = 2 * j + half;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int up = 2 - f;
+            const uint32_t t = ((q[i] >> (2 * f)) & 0x03030303u) | ((up >= 0 ? hm[i] << up : hm[i] >> -up) & 0x04040404u);
+            const float dl = i < 4 ? dl0 : dl1;
+            const float v0 = dl * (byte_plus_2_23(t, 0) - 8388612.0f), v1 = dl * (byte_plus_2_23(t, 1) - 8388612.0f);   // q - 4 without the mask bit
+            const float v2 = dl * (byte_plus_2_23(t, 2) - 8388612.0f), v3 = dl * (byte_plus_2_23(t, 3) - 8388612.0f);
+            out[2 * i] = h2_bits(__floats2half2_rn(v0, v1));
+            out[2 * i + 1] = h2_bits(__floats2half2_rn(v2, v3));
         }
     }
 };
 
 // ---- the kernel ------------------------------------------------------------------------------------
 
-// ---- work items ---------------------------------------------------------------------------------------
-// Tiles are dealt to the persistent CTAs in whole waves. With split_tail set (off by default) the tiles left
-// over after the last whole wave, which would keep only some SMs busy, have their K range cut into equal
-// pieces over ALL CTAs instead (in units of four K steps = one super-block). The pieces of a cut tile meet in
-// Y itself: piece 0 stores, piece k waits (bounded) until the tile's count says that pieces 0..k-1 are in Y and
-// then adds with a TMA reduction, so the additions happen in K order and the result is the same on every run.
-struct Item {
-    int tile;      // tile index
-    int k0, nk;    // K steps [k0, k0 + nk)
-    int partial;   // 1: a piece of a cut tile (accumulate into Y), 0: the whole tile (store)
+// One tile of work. Tiles are dealt to the CTAs (clusters) in whole waves; an expert launch's tiles come from its
+// device-side list, weight tiles of one token group in a row so that the CTAs at work share the group's X in L2.
+struct Tile {
+    int w_row;      // first weight row (of the matrix, or of the expert bank)
+    int n0;         // first output column
+    int x_row;      // first X row
+    int m;          // valid tokens
 };
-
-struct ItemIter {
-    int next_full, n_full, stride;   // whole tiles: next_full, next_full + stride, ... < n_full
-    int b, e, k_blocks, tail0;       // tail pieces in units of 4 K steps: [b, e) of the tail's block range
-    int tail_grid;                   // CTAs that share the tail (at most kMaxPieces per tile, so the last piece's
-                                     // additions stay short)
-    __device__ __forceinline__ void init(int cta, int grid, int n_tiles, int k_steps, int split_tail) {
-        n_full = split_tail ? (n_tiles / grid) * grid : n_tiles;
-        next_full = cta;
-        stride = grid;
-        k_blocks = k_steps / 4;
-        tail0 = n_full;
-        const int tail_tiles = n_tiles - n_full;
-        tail_grid = min(grid, tail_tiles * kMaxPieces);
-        const long long total = (long long)tail_tiles * k_blocks;
-        b = e = 0;
-        if (cta < tail_grid) {
-            b = (int)(total * cta / tail_grid);
-            e = (int)(total * (cta + 1) / tail_grid);
-        }
+template <int KIND>
+struct TileIter {
+    int i, n, stride;
+    __device__ __forceinline__ void init(const GemmParams &p) {
+        i = (int)blockIdx.x / p.split;
+        stride = (int)gridDim.x / p.split;
+        n = KIND == kDense ? p.n_tiles_n * p.n_tiles_m : *p.n_groups * p.n_tiles_n;
     }
-    __device__ __forceinline__ bool next(Item &it) {
-        if (next_full < n_full) {
-            it.tile = next_full;
-            it.k0 = 0;
-            it.nk = k_blocks * 4;
-            it.partial = 0;
-            next_full += stride;
-            return true;
+    __device__ __forceinline__ bool next(const GemmParams &p, Tile &t) {
+        if (i >= n) return false;
+        if (KIND == kDense) {
+            const int nt = i / p.n_tiles_m, mt = i - nt * p.n_tiles_m;
+            t.w_row = t.n0 = nt * kTileN;
+            t.x_row = mt * p.tile_m;
+            t.m = p.tile_m;
+        } else {
+            const int g = i / p.n_tiles_n, nt = i - g * p.n_tiles_n;
+            const GemmGroup gr = p.groups[g];
+            t.n0 = nt * (KIND == kGateUp ? kTileN / 2 : kTileN);
+            t.w_row = gr.w_row + t.n0;
+            t.x_row = gr.x_row;
+            t.m = gr.m;
         }
-        if (b < e) {
-            // A share that runs from the middle of one tile into the next gives its piece of the LATER tile
-            // first: that piece starts the tile's sum and waits for nobody, so the chain of pieces waiting
-            // for their predecessor in K order never gets longer than one tile's pieces.
-            const int t_b = b / k_blocks, t_e = (e - 1) / k_blocks;
-            int from = b, to = e;
-            if (t_e > t_b) from = t_e * k_blocks;
-            const int t = from / k_blocks, kb = from - t * k_blocks;
-            const int n = to - from;
-            it.tile = tail0 + t;
-            it.k0 = kb * 4;
-            it.nk = n * 4;
-            it.partial = n != k_blocks;
-            e = from;   // what is left is the earlier tile's piece (or nothing)
-            return true;
-        }
-        return false;
+        i += stride;
+        return true;
     }
 };
+// Tokens the MMA of a tile covers: all of tile_m, or (expert kinds) the group's own rounded up to 16.
+template <int KIND>
+__device__ __forceinline__ int tile_tokens(const GemmParams &p, const Tile &t) {
+    return KIND == kDense ? p.tile_m : (t.m + 15) & ~15;
+}
 
-template <int WT>
+template <int WT, int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap x_map,
-               const __grid_constant__ WMaps w_maps, const __grid_constant__ CUtensorMap y_map) {
-    constexpr bool kStagedRaw = tma_staged(WT);
-    constexpr int kSeg = raw_seg(WT), kNRaw = raw_stages(WT);
+               const __grid_constant__ WMaps<KIND> w_maps, const __grid_constant__ CUtensorMap y_map) {
+    constexpr int kSeg = raw_seg(WT), kStageBytes = kTileN * kSeg;
+    constexpr bool kOwnStages = Raw<WT>::kSteps == 4;   // a decode group fills A stages of its own (else both fill every one)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    GemmSmem *sm = reinterpret_cast<GemmSmem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (the offset to the next 1024-byte boundary is the same in every CTA of a cluster: same kernel, same layout)
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *raw_ring = smem + p.raw_off;
+    float *ystage = reinterpret_cast<float *>(smem + p.y_off);   // [2][kYChunk][kTileN]: accumulator read-out on its way to Y
+    GemmBars *sm = reinterpret_cast<GemmBars *>(smem + p.bar_off);
+    const int b_bytes = p.tile_m * 128;                          // an X tile: [tokens][64 f16], 128-byte swizzle
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);   // warp-uniform to the compiler too
     volatile int *gave_up = &sm->gave_up;
 
     if (tid == 0) {
-        for (int s = 0; s < kBStages; s++) {
+        for (int s = 0; s < p.n_b; s++) {
             mbar_init(smem_u32(&sm->b_full[s]), 1);
             mbar_init(smem_u32(&sm->b_empty[s]), 1);
         }
         for (int s = 0; s < kAStages; s++) {
-            mbar_init(smem_u32(&sm->a_full[s]), kDecodeThreads / 32);
+            mbar_init(smem_u32(&sm->a_full[s]), kOwnStages ? kDecodeWarps / kDecodeGroups : kDecodeWarps);
             mbar_init(smem_u32(&sm->a_empty[s]), 1);
         }
-        for (int s = 0; s < kRawStages; s++) {
+        for (int s = 0; s < p.n_raw; s++) {
             mbar_init(smem_u32(&sm->raw_full[s]), 1);
-            mbar_init(smem_u32(&sm->raw_empty[s]), kDecodeThreads / 32);
+            mbar_init(smem_u32(&sm->raw_empty[s]), kDecodeWarps);
         }
-        mbar_init(smem_u32(&sm->d_full), 1);
-        mbar_init(smem_u32(&sm->d_empty), kEpilogueThreads / 32);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(&sm->d_full[s]), 1);
+            mbar_init(smem_u32(&sm->d_empty[s]), kEpilogueThreads / 32);
+        }
         sm->gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 14) {
+    if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(&sm->tmem_base), kTmemCols);
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // The kernel may start while the one before it in the stream drains: weights are never written by a kernel in
+    // flight, so their copies go ahead (dense form); X, the expert list and Y wait for that grid.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (KIND != kDense) asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tmem_base = sm->tmem_base;
+    const int n_acc = p.tile_m <= kMaxTileM / 2 ? 2 : 1;   // accumulators in tensor memory
 
-    const int n_tiles = p.n_tiles_n * p.n_tiles_m;
-    const int k_steps = (int)(p.n_in / kBK);
-    ItemIter iter;
-    iter.init((int)blockIdx.x, (int)gridDim.x, n_tiles, k_steps, p.split_tail);
-    Item it;
+    // this CTA's K steps: all, or its cluster rank's share in whole super-blocks
+    const int k_blocks = (int)(p.n_in / 256), rank = (int)blockIdx.x % p.split;
+    const int kb0 = k_blocks * rank / p.split, kb1 = k_blocks * (rank + 1) / p.split;
+    const int ks0 = kb0 * 4, ks1 = kb1 * 4;
+    TileIter<KIND> iter;
+    iter.init(p);
+    Tile it;
 
-    if (warp < 8) {
-        // ===== decode warps: threads r and r + 128 <-> weight row r = TMEM lane r, 32 values each =====
-        const int r = tid & 127, half = tid >> 7;
-        const int trow = tile_row(WT, r), tslot = tile_slot(WT, r);
+    if (warp < kDecodeWarps) {
+        // ===== decode warps: threads r and r + 128 of a group <-> weight row r = TMEM lane r, 32 values each. The groups
+        // fill alternate A stages: four warps a scheduler hide each other's latencies =====
+        const int r = tid & 127, half = (warp >> 2) & 1, grp = warp / (kDecodeWarps / kDecodeGroups);
+        const int trow = tile_row<WT, KIND>(r) & (KIND == kGateUp ? 63 : 127), tslot = tile_slot<WT, KIND>(r);
+        // how far the row's first byte lies off a 16-byte boundary (a tile starts a multiple of 8 rows into its matrix)
+        const int row_lead = row_phased(WT) ? (int)(((size_t)trow * p.row_bytes) & 15) : 0;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + kTmemA + 16 * half;
-        int sa = 0, sr = 0;
+        int sa = kOwnStages ? grp : 0, sr = 0;
         uint32_t pa = 0, pr = 0;
-        while (iter.next(it)) {
-            const int64_t n0 = (int64_t)(it.tile / p.n_tiles_m) * kTileN;
+        while (iter.next(p, it)) {
             // Rows past n_out need no care here: their staged bytes are zero (the tensor maps fill what lies
-            // outside the matrix with zeros, and fetch() does the same), and a zero block decodes to zeros.
+            // outside the matrix with zeros), and a zero block decodes to zeros.
             Raw<WT> cur;
-            if constexpr (!kStagedRaw) cur.fetch(p.w, n0, p.n_out, p.row_bytes, it.k0, tid);
-            for (int ks0 = it.k0; ks0 < it.k0 + it.nk; ks0 += Raw<WT>::kSteps) {
-                if constexpr (kStagedRaw) {
-                    wait_phase(smem_u32(&sm->raw_full[sr]), pr, gave_up, p.status);
-                    if constexpr (row_phased(WT))
-                        cur.lead = (int)(((size_t)trow * p.row_bytes + (size_t)(ks0 >> 2) * 210) & 15);   // n0 rows are a multiple of 16 bytes
-                    cur.load_block(sm->raw + (size_t)sr * (kTileN * kSeg) + tslot * kSeg, half, ks0);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]));   // the bytes are in registers now
-                    if (++sr == kNRaw) {
-                        sr = 0;
-                        pr ^= 1;
-                    }
-                } else {
-                    // The bytes fetched a stage ago go to the buffer nobody reads any more (the one before
-                    // last); one barrier of the decode warps makes them visible, and the next stage's loads
-                    // fly while this one is decoded.
-                    cur.stash(sm->raw + (size_t)(sr & 1) * (kRawStages * kRawBytes / 2), tid);
-                    sr++;
-                    asm volatile("bar.sync 1, %0;" ::"n"(kDecodeThreads) : "memory");
-                    if (ks0 + Raw<WT>::kSteps < it.k0 + it.nk)
-                        cur.fetch(p.w, n0, p.n_out, p.row_bytes, ks0 + Raw<WT>::kSteps, tid);
+            for (int ks = ks0; ks < ks1; ks += Raw<WT>::kSteps) {
+                wait_phase(smem_u32(&sm->raw_full[sr]), pr, gave_up, p.status);
+                if constexpr (row_phased(WT)) cur.lead = (row_lead + (ks >> 2) * block_bytes(WT)) & 15;
+                cur.load_block(raw_ring + (size_t)sr * kStageBytes + tslot * kSeg, half, ks, grp);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]));   // the bytes are in registers now
+                if (++sr == p.n_raw) {
+                    sr = 0;
+                    pr ^= 1;
                 }
-                // Two K steps share one tensor-memory stage and one hand-over to the MMA thread; the next K step
-                // is converted while this one's store is in flight.
-                uint32_t v[2][16];
-                cur.convert(0, half, r, v[0]);
-#pragma unroll
-                for (int j = 0; j < Raw<WT>::kSteps; j++) {
-                    if ((j & 1) == 0) {
-                        wait_phase(smem_u32(&sm->a_empty[sa]), pa ^ 1, gave_up, p.status);
-                        tc_fence_after();
-                    }
-                    tmem_st16(lane_addr + 64 * sa + 32 * (j & 1), v[j & 1]);
-                    if (j + 1 < Raw<WT>::kSteps) cur.convert(j + 1, half, r, v[(j + 1) & 1]);
-                    if (j & 1) {
-                        tmem_st_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&sm->a_full[sa]));
-                        if (++sa == kAStages) {
-                            sa = 0;
-                            pa ^= 1;
-                        }
-                    }
+                // The group's two K steps fill one tensor-memory stage (Q8_0: its one step half of it); the second is
+                // converted while the first's store is in flight.
+                uint32_t v[16];
+                if (half) cur.template convert<1>(0, v);
+                else cur.template convert<0>(0, v);
+                wait_phase(smem_u32(&sm->a_empty[sa]), pa ^ 1, gave_up, p.status);
+                tc_fence_after();
+                tmem_st16(lane_addr + 64 * sa + (kOwnStages ? 0 : 32 * grp), v);
+                if constexpr (kOwnStages) {
+                    uint32_t u[16];
+                    if (half) cur.template convert<1>(1, u);
+                    else cur.template convert<0>(1, u);
+                    tmem_st16(lane_addr + 64 * sa + 32, u);
+                }
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sm->a_full[sa]));
+                if ((sa += kOwnStages ? kDecodeGroups : 1) >= kAStages) {
+                    sa -= kAStages;
+                    pa ^= 1;
                 }
             }
         }
-    } else if (warp < 12) {
+    } else if (warp < kDecodeWarps + kEpilogueWarps) {
         // ===== epilogue warps: TMEM lane = weight row, column = token =====
-        // Whole tiles and cut tiles leave the same way: the accumulator is read 32 tokens at a time, written to
-        // shared memory as [token][weight row] and stored by TMA, so the accumulator is free again as soon as
-        // it has been read (this read-out is not hidden behind MMAs: its length counts). Rows past the end of
-        // Y are clipped by the tensor map.
-        const int ew = warp - 8, et = tid - kDecodeThreads;
-        const int tgrid = iter.tail_grid;
-        const long long tail_total = (long long)(n_tiles - iter.n_full) * iter.k_blocks;
-        const uint32_t d_addr = tmem_base + ((uint32_t)(32 * ew) << 16);
-        int ybuf = 0;
+        // The accumulator is read 32 tokens at a time, written to shared memory as [token][weight row] and stored
+        // from there, so it is free again as soon as it has been read.
+        const int ew = warp - kDecodeWarps, et = tid - kDecodeThreads;
+        const uint32_t lane_d = tmem_base + ((uint32_t)(32 * ew) << 16);
+        const int my_row = tile_row<WT, KIND>(32 * ew + lane);
+        int ybuf = 0, da = 0;
         uint32_t ph = 0;
-        // one chunk: registers -> staging buffer -> TMA store through `map` at (x, y)
-        auto ship = [&](const uint32_t (&v)[32], const CUtensorMap *map, int x, int y, bool add) {
-            if (et == 0) tma_store_wait_read<1>();   // the store that read this buffer two chunks ago is done with it
-            asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueThreads) : "memory");
-            float *dst = &sm->ystage[ybuf][0][tile_row(WT, 32 * ew + lane)];
-#pragma unroll
-            for (int j = 0; j < 32; j++) dst[j * kTileN] = __uint_as_float(v[j]);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueThreads) : "memory");
-            if (et == 0) {
-                if (add) tma_reduce_add_2d(map, x, y, smem_u32(sm->ystage[ybuf]));
-                else tma_store_2d(map, x, y, smem_u32(sm->ystage[ybuf]));
-                tma_store_commit();
-            }
-            ybuf ^= 1;
-        };
-        // one chunk straight to Y (a Y the tensor map cannot describe)
-        auto put = [&](const uint32_t (&v)[32], int64_t n, int64_t m_first) {
-            if (n < p.n_out) {
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const int64_t m = m_first + j;
-                    if (m < p.rows) p.y[m * p.n_out + n] = __uint_as_float(v[j]);
-                }
-            }
-        };
-        while (iter.next(it)) {
-            const int64_t n0 = (int64_t)(it.tile / p.n_tiles_m) * kTileN, m0 = (int64_t)(it.tile % p.n_tiles_m) * p.tile_m;
-            wait_phase(smem_u32(&sm->d_full), ph, gave_up, p.status);
-            ph ^= 1;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        while (iter.next(p, it)) {
+            wait_phase(smem_u32(&sm->d_full[da]), ph, gave_up, p.status);
             tc_fence_after();
-            const int64_t n = n0 + tile_row(WT, 32 * ew + lane);
-            if (!it.partial) {
-                for (int c0 = 0; c0 < p.tile_m; c0 += kYChunk) {
+            const uint32_t d_addr = lane_d + 128 * da;
+            const int tokens = tile_tokens<KIND>(p, it);
+            if (KIND == kDense && p.split > 1) {
+                // a piece of K: the whole accumulator goes to shared memory over the drained X ring (every MMA that
+                // read it is done); the cluster adds the pieces up below
+                float *part = reinterpret_cast<float *>(smem);
+                for (int c0 = 0; c0 < tokens; c0 += kYChunk) {
                     uint32_t v[32];
                     tmem_ld32(d_addr + (uint32_t)c0, v);
                     tmem_ld_wait();
-                    if (p.y_tma) ship(v, &y_map, (int)n0, (int)(m0 + c0), false);
-                    else put(v, n, m0 + c0);
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (c0 + j < tokens) part[(c0 + j) * kTileN + my_row] = __uint_as_float(v[j]);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->d_empty));   // the accumulator is free again
-                continue;
+                break;   // one tile per cluster
             }
-            // ---- a piece of a cut tile: added into Y in K order ----
-            // Piece k of the tile (k = how many CTAs hold earlier blocks of it) waits, bounded, until the
-            // tile's count says that pieces 0..k-1 are in Y; piece 0 stores, the others add (TMA reduction in
-            // L2); then the count goes up. The order of the additions is the K order whoever finishes first.
-            const int t = it.tile - iter.tail0;
-            const long long lo = (long long)t * iter.k_blocks, hi = lo + iter.k_blocks;
-            int c_lo = (int)(lo * tgrid / tail_total);
-            c_lo = max(c_lo - 1, 0);
-            int k_piece = 0;
-            for (int c = c_lo; c < (int)blockIdx.x; c++) {
-                const long long sb = tail_total * c / tgrid, se = tail_total * (c + 1) / tgrid;
-                k_piece += (max(sb, lo) < min(se, hi)) ? 1 : 0;
-            }
-            if (k_piece > 0) {
-                if (et == 0) {
-                    const long long t0 = clock64();
-                    while (*reinterpret_cast<volatile unsigned *>(p.tail_count + t) < (unsigned)k_piece) {
-                        __nanosleep(64);
-                        if (clock64() - t0 > kWaitCycles) {
-                            atomicExch(p.status, KRK_CUDA_ETIMEOUT);
-                            break;
-                        }
-                    }
-                    __threadfence();
-                }
-                asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueThreads) : "memory");
-            }
-            for (int c0 = 0; c0 < p.tile_m; c0 += kYChunk) {
+            for (int c0 = 0; c0 < tokens; c0 += kYChunk) {
                 uint32_t v[32];
                 tmem_ld32(d_addr + (uint32_t)c0, v);
                 tmem_ld_wait();
-                ship(v, &y_map, (int)n0, (int)(m0 + c0), k_piece > 0);
+                if (KIND == kDense && !p.y_tma) {   // a Y the tensor map cannot describe: straight out
+                    const int64_t n = it.n0 + my_row, m_first = it.x_row + c0;
+                    if (n < p.n_out) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (m_first + j < p.rows) p.y[(m_first + j) * p.n_out + n] = __uint_as_float(v[j]);
+                    }
+                    continue;
+                }
+                if (KIND == kDense && et == 0) tma_store_wait_read<1>();   // the store that read this buffer two chunks ago is done with it
+                asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueThreads) : "memory");
+                float *buf = ystage + ybuf * (kYChunk * kTileN);
+#pragma unroll
+                for (int j = 0; j < 32; j++) buf[j * kTileN + my_row] = __uint_as_float(v[j]);
+                if (KIND == kDense) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("bar.sync 2, %0;" ::"n"(kEpilogueThreads) : "memory");
+                if (KIND == kDense) {
+                    if (et == 0) {   // rows past the end of Y are clipped by the tensor map
+                        tma_store_2d(&y_map, it.n0, it.x_row + c0, smem_u32(buf));
+                        tma_store_commit();
+                    }
+                } else if (KIND == kGateUp) {
+                    // four threads a token, 16 outputs each: columns 0..63 of the buffer are gates, 64..127 ups. The
+                    // result is rounded to f16 as the GEMM that reads it would round it (finite values saturate).
+                    const int tok = et >> 2, col = 16 * (et & 3);
+                    if (c0 + tok < it.m) {
+                        uint32_t o[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            const float2 g = *reinterpret_cast<const float2 *>(buf + tok * kTileN + col + 2 * i);
+                            const float2 u = *reinterpret_cast<const float2 *>(buf + tok * kTileN + 64 + col + 2 * i);
+                            o[i] = h2_bits(__halves2half2(half_sat(g.x / (1.0f + expf(-g.x)) * u.x), half_sat(g.y / (1.0f + expf(-g.y)) * u.y)));
+                        }
+                        uint4 *dst = reinterpret_cast<uint4 *>(p.h + (int64_t)(it.x_row + c0 + tok) * p.n_out + it.n0 + col);
+                        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kYChunk / 4; i++) {
+                        const int tok = 4 * i + ew;   // a warp per token: 512 contiguous bytes
+                        if (c0 + tok < it.m)
+                            *reinterpret_cast<float4 *>(p.y + (int64_t)(it.x_row + c0 + tok) * p.n_out + it.n0 + 4 * lane) =
+                                *reinterpret_cast<const float4 *>(buf + tok * kTileN + 4 * lane);
+                    }
+                }
+                ybuf ^= 1;
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm->d_empty));
-            if (et == 0) {
-                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // this piece is in Y
-                asm volatile("fence.proxy.async;" ::: "memory");
-                __threadfence();
-                atomicAdd(p.tail_count + t, 1u);
+            if (lane == 0) mbar_arrive(smem_u32(&sm->d_empty[da]));   // the accumulator is free again
+            if (++da == n_acc) {
+                da = 0;
+                ph ^= 1;
             }
         }
         // the staging buffers must outlive the stores that read them
-        if (et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    } else if (warp == 12) {
+        if (KIND == kDense && et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    } else if (warp == kXWarp) {
         // ===== TMA producer of X tiles =====
         if (lane == 0) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             int sb = 0;
             uint32_t pb = 0;
-            while (iter.next(it)) {
-                const int m0 = (it.tile % p.n_tiles_m) * p.tile_m;
-                for (int ks = it.k0; ks < it.k0 + it.nk; ks++) {
+            while (iter.next(p, it)) {
+                const int boxes = (tile_tokens<KIND>(p, it) + kGroupBox - 1) / kGroupBox;
+                for (int ks = ks0; ks < ks1; ks++) {
                     wait_phase(smem_u32(&sm->b_empty[sb]), pb ^ 1, gave_up, p.status);
-                    const uint32_t bar = smem_u32(&sm->b_full[sb]);
-                    mbar_arrive_expect_tx(bar, (uint32_t)p.tile_m * 128u);
-                    tma_load_2d(smem_u32(sm->b[sb]), &x_map, ks * kBK, m0, bar);
-                    if (++sb == kBStages) {
+                    const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem + (size_t)sb * b_bytes);
+                    if (KIND == kDense) {
+                        mbar_arrive_expect_tx(bar, (uint32_t)b_bytes);
+                        tma_load_2d(dst, &x_map, ks * kBK, it.x_row, bar);
+                    } else {   // only the boxes that hold tokens of the group
+                        mbar_arrive_expect_tx(bar, (uint32_t)(boxes * kGroupBox * 128));
+                        for (int b = 0; b < boxes; b++) tma_load_2d(dst + b * kGroupBox * 128, &x_map, ks * kBK, it.x_row + b * kGroupBox, bar);
+                    }
+                    if (++sb == p.n_b) {
                         sb = 0;
                         pb ^= 1;
                     }
                 }
             }
         }
-    } else if (warp == 13) {
-        // ===== producer of raw block columns: one TMA box of 128 rows per stage, or one bulk copy per row =====
-        if constexpr (row_phased(WT)) {
-            if (lane == 0) {
-                int sr = 0;
-                uint32_t pr = 0;
-                while (iter.next(it)) {
-                    const int n0 = (it.tile / p.n_tiles_m) * kTileN;
-                    for (int blk = it.k0 / 4; blk < (it.k0 + it.nk) / 4; blk++) {
-                        wait_phase(smem_u32(&sm->raw_empty[sr]), pr ^ 1, gave_up, p.status);
-                        const uint32_t bar = smem_u32(&sm->raw_full[sr]);
-                        mbar_arrive_expect_tx(bar, (uint32_t)(kTileN * kSeg));
-                        const uint32_t stage = smem_u32(sm->raw + (size_t)sr * (kTileN * kSeg));
-                        for (int c = 0; c < kPhases; c++) {
-                            // map c starts (c * row_bytes) % 16 bytes before row c; the block's granules from there
-                            const int x0 = (int)((((size_t)c * p.row_bytes) & 15) + (size_t)blk * 210) & ~15;
-                            // a matrix of fewer than eight rows has no row c: read outside the map, which fills zeros
-                            const int y0 = c < p.n_out ? n0 / kPhases : (1 << 24);
-                            tma_load_2d(stage + c * (kTileN / kPhases) * kSeg, &w_maps.m[c], x0, y0, bar);
-                        }
-                        if (++sr == kNRaw) {
-                            sr = 0;
-                            pr ^= 1;
-                        }
-                    }
-                }
-            }
-        } else if (kStagedRaw && lane == 0) {
+    } else if (warp == kRawWarp) {
+        // ===== TMA producer of raw block columns =====
+        if (lane == 0) {
+            constexpr int kHalves = KIND == kGateUp ? 2 : 1;   // matrices in a weight tile
             int sr = 0;
             uint32_t pr = 0;
-            while (iter.next(it)) {
-                const int n0 = (it.tile / p.n_tiles_m) * kTileN;
+            while (iter.next(p, it)) {
                 constexpr int kPer = Raw<WT>::kSteps;   // K steps per stage
-                for (int blk = it.k0 / kPer; blk < (it.k0 + it.nk) / kPer; blk++) {
+                for (int blk = ks0 / kPer; blk < ks1 / kPer; blk++) {
                     wait_phase(smem_u32(&sm->raw_empty[sr]), pr ^ 1, gave_up, p.status);
                     const uint32_t bar = smem_u32(&sm->raw_full[sr]);
-                    mbar_arrive_expect_tx(bar, (uint32_t)(kTileN * kSeg));
-                    const int x0 = WT == KRK_CUDA_Q8_0 ? 136 * blk - 8 * (blk & 1) : blk * kSeg;   // a multiple of 16
-                    tma_load_2d(smem_u32(sm->raw + (size_t)sr * (kTileN * kSeg)), &w_maps.m[0], x0, n0, bar);
-                    if (++sr == kNRaw) {
+                    const uint32_t stage = smem_u32(raw_ring + (size_t)sr * kStageBytes);
+                    mbar_arrive_expect_tx(bar, (uint32_t)kStageBytes);
+                    if constexpr (row_phased(WT)) {
+                        constexpr int kBoxRows = kTileN / kPhases / kHalves;
+#pragma unroll
+                        for (int c = 0; c < kPhases; c++) {
+                            // map c starts (c * row_bytes) % 16 bytes before row c; the block's granules from there
+                            const int x0 = ((int)(((size_t)c * p.row_bytes) & 15) + blk * block_bytes(WT)) & ~15;
+                            // a matrix of fewer than eight rows has no row c: read outside the map, which fills zeros
+                            const int y0 = (KIND != kDense || c < p.n_out) ? it.w_row / kPhases : (1 << 24);
+#pragma unroll
+                            for (int hf = 0; hf < kHalves; hf++)
+                                tma_load_2d(stage + (hf * (kTileN / 2) + c * kBoxRows) * kSeg, &w_maps.m[hf * kPhases + c], x0, y0, bar);
+                        }
+                    } else {
+                        const int x0 = WT == KRK_CUDA_Q8_0 ? 136 * blk - 8 * (blk & 1) : blk * kSeg;   // a multiple of 16
+#pragma unroll
+                        for (int hf = 0; hf < kHalves; hf++)
+                            tma_load_2d(stage + hf * (kTileN / 2) * kSeg, &w_maps.m[hf], x0, it.w_row, bar);
+                    }
+                    if (++sr == p.n_raw) {
                         sr = 0;
                         pr ^= 1;
                     }
@@ -924,57 +939,86 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             }
         }
     } else {
-        // ===== MMA issuer =====
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(kTileN, p.tile_m);
-            int sa = 0, sb = 0;
-            uint32_t pa = 0, pb = 0, pd = 0;
-            while (iter.next(it)) {
-                wait_phase(smem_u32(&sm->d_empty), pd ^ 1, gave_up, p.status);   // the epilogue has drained the accumulator
-                pd ^= 1;
+        // ===== MMA issuer: the whole warp walks the loop, one elected lane issues (see umma_f16_ts_step) =====
+        const uint32_t elected = elect_one();
+        const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+        iter.n = __shfl_sync(0xFFFFFFFFu, iter.n, 0);
+        int sa = 0, sb = 0, da = 0;
+        uint32_t pa = 0, pb = 0, pd = 0;
+        while (iter.next(p, it)) {
+            const uint32_t idesc = instr_desc(kTileN, __shfl_sync(0xFFFFFFFFu, tile_tokens<KIND>(p, it), 0));
+            wait_phase(smem_u32(&sm->d_empty[da]), pd ^ 1, gave_up, p.status);   // the epilogue has drained the accumulator
+            tc_fence_after();
+            for (int ks = ks0; ks < ks1; ks++) {   // an even number: a stage of decoded A holds two K steps
+                wait_phase(smem_u32(&sm->b_full[sb]), pb, gave_up, p.status);
+                if ((ks & 1) == 0) wait_phase(smem_u32(&sm->a_full[sa]), pa, gave_up, p.status);
                 tc_fence_after();
-                for (int ks = 0; ks < it.nk; ks++) {   // nk is even: a stage of decoded A holds two K steps
-                    wait_phase(smem_u32(&sm->b_full[sb]), pb, gave_up, p.status);
-                    if ((ks & 1) == 0) wait_phase(smem_u32(&sm->a_full[sa]), pa, gave_up, p.status);
-                    tc_fence_after();
-                    const uint64_t bdesc = smem_desc(smem_u32(sm->b[sb]));
-                    const uint32_t a_tmem = tmem_base + kTmemA + 64 * sa + 32 * (ks & 1);
-#pragma unroll
-                    for (int kk = 0; kk < kBK / 16; kk++)   // 16 K values = 8 TMEM columns of A, 32 bytes of every B row
-                        umma_f16_ts(tmem_base, a_tmem + 8 * kk, bdesc + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
-                    umma_commit(smem_u32(&sm->b_empty[sb]));   // a stage is free once the MMAs that read it are done
-                    if (ks & 1) {
-                        umma_commit(smem_u32(&sm->a_empty[sa]));
-                        if (++sa == kAStages) {
-                            sa = 0;
-                            pa ^= 1;
-                        }
-                    }
-                    if (++sb == kBStages) {
-                        sb = 0;
-                        pb ^= 1;
+                umma_f16_ts_step(tmem + 128 * da, tmem + kTmemA + 64 * sa + 32 * (ks & 1), smem_desc(smem_u32(smem) + (uint32_t)(sb * b_bytes)),
+                                 idesc, ks == ks0 ? 1u : 0u, elected);
+                umma_commit(smem_u32(&sm->b_empty[sb]), elected);   // a stage is free once the MMAs that read it are done
+                if (ks & 1) {
+                    umma_commit(smem_u32(&sm->a_empty[sa]), elected);
+                    if (++sa == kAStages) {
+                        sa = 0;
+                        pa ^= 1;
                     }
                 }
-                umma_commit(smem_u32(&sm->d_full));
+                if (++sb == p.n_b) {
+                    sb = 0;
+                    pb ^= 1;
+                }
+            }
+            umma_commit(smem_u32(&sm->d_full[da]), elected);
+            if (++da == n_acc) {
+                da = 0;
+                pd ^= 1;
             }
         }
     }
 
     tc_fence_before();
     __syncthreads();
-    if (warp == 14) {
+    if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
+        __syncwarp();
+    }
+    if (KIND == kDense && p.split > 1) {
+        // ---- the pieces of a tile meet: CTA `rank` adds its share of the tokens over all CTAs of the cluster, in K order ----
+        cluster_sync();
+        const int nt = ((int)blockIdx.x / p.split) / p.n_tiles_m, mt = ((int)blockIdx.x / p.split) % p.n_tiles_m;
+        const int t0 = p.tile_m * rank / p.split, t1 = p.tile_m * (rank + 1) / p.split;
+        for (int i = tid; i < (t1 - t0) * (kTileN / 4); i += kThreads) {
+            const int tok = t0 + i / (kTileN / 4), col = 4 * (i % (kTileN / 4));
+            const int64_t m = (int64_t)mt * p.tile_m + tok, n = (int64_t)nt * kTileN + col;
+            if (m >= p.rows || n >= p.n_out) continue;
+            const uint32_t at = smem_u32(smem) + (uint32_t)(tok * kTileN + col) * 4u;
+            float4 s = ld_peer(at, 0);
+            for (int q = 1; q < p.split; q++) {
+                const float4 v = ld_peer(at, q);
+                s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+            }
+            float *y = p.y + m * p.n_out + n;
+            if (p.y_tma) {   // 16-byte aligned, n_out a multiple of four
+                *reinterpret_cast<float4 *>(y) = s;
+            } else {
+                y[0] = s.x;
+                if (n + 1 < p.n_out) y[1] = s.y;
+                if (n + 2 < p.n_out) y[2] = s.z;
+                if (n + 3 < p.n_out) y[3] = s.w;
+            }
+        }
+        cluster_sync();   // nobody leaves while its shared memory is being read
     }
 }
 
-__global__ void __launch_bounds__(256) f32_to_f16_kernel(__half *__restrict__ out, const float *__restrict__ in, int64_t n) {
-    // A finite activation beyond the f16 range saturates to +-65504 instead of becoming an infinity (which the
-    // f32 accumulation would turn into NaN on the first cancellation): the rule of the reference's f16
-    // activation stores (src/hip/krk_hip.hpp:141-202). Infinities and NaNs pass through unchanged.
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float v = in[i];
-        out[i] = __float2half_rn(fabsf(v) <= 3.4028234e38f ? fminf(fmaxf(v, -65504.0f), 65504.0f) : v);
+__global__ void __launch_bounds__(256) f32_to_f16_kernel(__half *__restrict__ out, const float *__restrict__ in, int64_t n4) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 v = reinterpret_cast<const float4 *>(in)[i];
+        reinterpret_cast<uint2 *>(out)[i] = make_uint2(h2_bits(__halves2half2(half_sat(v.x), half_sat(v.y))),
+                                                       h2_bits(__halves2half2(half_sat(v.z), half_sat(v.w))));
     }
 }
 
@@ -983,171 +1027,180 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
+    static EncodeTiledFn fn = [] {
         void *ptr = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            ptr = nullptr;
+        return reinterpret_cast<EncodeTiledFn>(ptr);
+    }();
     return fn;
 }
 
-// Tensor map over the raw weight bytes as a [n_out][row_bytes] byte matrix, box = one Q4_K super-block
-// (144 bytes) x 128 rows. For the formats that are not staged this way a 16-byte-wide box of the same
-// matrix is encoded so that the kernel always receives a valid map.
-bool encode_w_map(CUtensorMap *map, const uint8_t *w, int wt, int64_t n_out, int row_bytes) {
+// A row-major matrix as a 2-d tensor map (no fill but zeros outside it).
+bool encode_2d(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t cols, int64_t rows, size_t pitch, int box_cols,
+               int box_rows, CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return false;
-    const bool staged = tma_staged(wt) && !row_phased(wt);   // phased formats: encode_phase_maps
-    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)n_out};
-    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-    const cuuint32_t box[2] = {staged ? (cuuint32_t)raw_seg(wt) : 16u, staged ? (cuuint32_t)kTileN : 1u};
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    if (!staged && (row_bytes % 16) != 0) {
-        // never used by the kernel; describe a 16-byte row of the same buffer so that encoding succeeds
-        const cuuint64_t d2[2] = {16, 1};
-        const cuuint64_t s2[1] = {16};
-        return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(w), d2, s2, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promo,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Phased formats: map c covers the rows c, c + 8, c + 16, ... of the matrix from the 16-byte boundary at or before
-// row c: inner extent = the lead bytes + one row (so nothing past a row's own end is ever read, and what the box
-// holds beyond it is zero fill), pitch = eight rows, box = 224 bytes x 16 rows. A c with no row at all (fewer than
-// eight rows in the matrix) repeats map 0; its staged rows are never used.
-bool encode_phase_maps(WMaps *maps, const uint8_t *w, int64_t n_out, int row_bytes) {
-    EncodeTiledFn encode = encode_tiled();
-    if (!encode) return false;
-    const cuuint32_t box[2] = {224u, (cuuint32_t)(kTileN / kPhases)};
-    const cuuint32_t estr[2] = {1, 1};
-    for (int c = 0; c < kPhases; c++) {
-        const int cc = c < n_out ? c : 0;
-        const size_t start = (size_t)cc * row_bytes, lead = start & 15;
-        const cuuint64_t dims[2] = {(cuuint64_t)(lead + row_bytes), (cuuint64_t)((n_out - cc + kPhases - 1) / kPhases)};
-        const cuuint64_t strides[1] = {(cuuint64_t)kPhases * row_bytes};
-        if (encode(&maps->m[c], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(w + (start - lead)), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
-    return true;
-}
-
-// Tensor map over Y as a [rows][n_out] f32 matrix, box = 128 weight rows x kYChunk tokens, for the TMA stores
-// of the read-out. A Y that is not 16-byte aligned with 16-byte-multiple rows cannot be described: then a
-// dummy map over the first 16 bytes of the weights is encoded (never used) and the kernel stores directly.
-bool encode_y_map(CUtensorMap *map, float *y, const uint8_t *w, int64_t n_out, int64_t rows, bool usable) {
-    EncodeTiledFn encode = encode_tiled();
-    if (!encode) return false;
-    const cuuint32_t estr[2] = {1, 1};
-    if (!usable) {
-        const cuuint64_t d2[2] = {16, 1};
-        const cuuint64_t s2[1] = {16};
-        const cuuint32_t b2[2] = {16, 1};
-        return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(w), d2, s2, b2, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
-    const cuuint64_t dims[2] = {(cuuint64_t)n_out, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)n_out * sizeof(float)};
-    const cuuint32_t box[2] = {(cuuint32_t)kTileN, (cuuint32_t)kYChunk};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
+// The maps over the raw weight bytes of one matrix ([n_out][row_bytes] bytes), for boxes that bring `tile_rows` rows.
+// Formats staged as one box: box = one stage's bytes of a row x the rows. Phased formats: map c covers the rows c,
+// c + 8, c + 16, ... from the 16-byte boundary at or before row c: inner extent = the lead bytes + one row (so nothing
+// past a row's own end is ever read, and what the box holds beyond it is zero fill), pitch = eight rows. A c with no
+// row at all (fewer than eight rows in the matrix) repeats map 0; its staged rows are never used.
 template <int WT>
-int launch_wt(const GemmParams &p, const CUtensorMap &map, int grid, cudaStream_t st) {
-    WMaps w_maps;
-    CUtensorMap y_map;
-    if (!encode_w_map(&w_maps.m[0], p.w, WT, p.n_out, p.row_bytes)) return KRK_CUDA_ELAUNCH;
-    for (int c = 1; c < kPhases; c++) w_maps.m[c] = w_maps.m[0];
-    if (row_phased(WT) && !encode_phase_maps(&w_maps, p.w, p.n_out, p.row_bytes)) return KRK_CUDA_ELAUNCH;
-    if (!encode_y_map(&y_map, p.y, p.w, p.n_out, p.rows, p.y_tma != 0)) return KRK_CUDA_ELAUNCH;
+bool encode_w_maps(CUtensorMap *maps, const uint8_t *w, int64_t n_out, int row_bytes, int tile_rows) {
+    if constexpr (!row_phased(WT)) {
+        return encode_2d(maps, CU_TENSOR_MAP_DATA_TYPE_UINT8, w, row_bytes, n_out, row_bytes, raw_seg(WT), tile_rows,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    } else {
+        for (int c = 0; c < kPhases; c++) {
+            const int cc = c < n_out ? c : 0;
+            const size_t start = (size_t)cc * row_bytes, lead = start & 15;
+            if (!encode_2d(&maps[c], CU_TENSOR_MAP_DATA_TYPE_UINT8, w + (start - lead), (int64_t)(lead + row_bytes), (n_out - cc + kPhases - 1) / kPhases,
+                           (size_t)kPhases * row_bytes, raw_seg(WT), tile_rows / kPhases, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+                return false;
+        }
+        return true;
+    }
+}
+
+// Ring depths and the shared-memory map of a launch. The raw ring wants as many K steps in flight as the X ring;
+// both grow in turn while they fit.
+template <int WT>
+size_t layout(GemmParams &p) {
+    const int stage = kTileN * raw_seg(WT), steps = Raw<WT>::kSteps, xb = p.tile_m * 128;
+    const int y_bytes = 2 * kYChunk * kTileN * (int)sizeof(float);
+    const int room = kSmemMax - 1024 - y_bytes - (int)sizeof(GemmBars);
+    p.n_b = kMinB;
+    p.n_raw = kMinRaw;
+    for (;;) {
+        const int left = room - p.n_b * xb - p.n_raw * stage;
+        const bool want_b = p.n_b < kMaxB && p.n_b < steps * p.n_raw;
+        if (want_b && left >= xb) p.n_b++;
+        else if (p.n_raw < kMaxRaw && left >= stage) p.n_raw++;
+        else if (p.n_b < kMaxB && left >= xb) p.n_b++;
+        else break;
+    }
+    p.raw_off = p.n_b * xb;
+    p.y_off = p.raw_off + p.n_raw * stage;
+    p.bar_off = p.y_off + y_bytes;
+    return (size_t)p.bar_off + sizeof(GemmBars) + 1024;
+}
+
+template <int WT, int KIND>
+int launch_kernel(const GemmParams &p, const CUtensorMap &x_map, const WMaps<KIND> &w_maps, const CUtensorMap &y_map, int grid, size_t smem,
+                  cudaStream_t st) {
     static bool configured[64] = {};
-    auto kernel = gemm_tc_kernel<WT>;
-    const size_t smem = sizeof(GemmSmem) + 1024;
+    auto kernel = gemm_tc_kernel<WT, KIND>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
         if (e != cudaSuccess) {
             note_cuda_error(e);
             return KRK_CUDA_ELAUNCH;
         }
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    kernel<<<grid, kThreads, smem, st>>>(p, map, w_maps, y_map);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.split;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.split > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p, x_map, w_maps, y_map);
     note_launch(1, KRK_CUDA_FAMILY_GEMM_TC);
-    return check_launch();
+    if (e != cudaSuccess) {
+        note_cuda_error(e);
+        (void)cudaGetLastError();
+        return KRK_CUDA_ELAUNCH;
+    }
+    return KRK_CUDA_OK;
 }
 
-} // namespace
-
-namespace {
-
+// How a dense product is cut. One tile is 128 weight rows x tile_m tokens, `split` CTAs share it along K, and the
+// model below (clocks; fitted to single tiles on all SMs, Q4_K, K = 16384: a K step took 206 / 218 / 290 / 466 ns at
+// 16 / 64 / 128 / 256 tokens, every other format within a fifth of that or slower at the narrow end) picks the pair
+// that ends first: narrow tiles are bound by the decode, wide ones by MMA and power, a tile costs some fixed clocks
+// for its pipeline fill and read-out, and a cluster some more to add its pieces.
 struct GemmPlan {
-    int tile_m, n_tiles_n, n_tiles_m, grid, tail;   // tail: tiles left after the last whole wave (0 = none)
-    size_t x_bytes, count_bytes;
+    int tile_m, n_tiles_n, n_tiles_m, split, grid;
+    size_t x_bytes;
 };
+constexpr double kStepMin = 400.0, kStepBase = 200.0, kStepToken = 2.7;
+constexpr int kFixedCycles = 4000;
 
-int grid_bound() {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-        return sms;
-    (void)cudaGetLastError();
-    return 148;
-}
-
-GemmPlan plan_gemm(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows) {
+GemmPlan plan_gemm(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows, int sms) {
     GemmPlan g;
-    g.tile_m = rows >= kMaxTileM ? kMaxTileM : (int)((rows + 15) / 16 * 16);
     g.n_tiles_n = (int)((n_out + kTileN - 1) / kTileN);
-    g.n_tiles_m = (int)((rows + g.tile_m - 1) / g.tile_m);
-    const int tiles = g.n_tiles_n * g.n_tiles_m, sms = grid_bound();
-    g.grid = tiles < sms ? tiles : sms;
-    // Cutting the left-over tiles along K is opt-in (KRK_CUDA_GEMM_SPLIT=1, read once, in the style of the
-    // reference's KRK_* A/B switches): the pieces meet in Y through ordered TMA reductions, without scratch,
-    // but every extra piece pays a pipeline fill and a read-out, and measured on config 3 that eats what the
-    // better balance gains (M = 512: 65.1 vs 64.9 us), so whole tiles are the default.
-    static const bool split_on = [] {
-        const char *e = std::getenv("KRK_CUDA_GEMM_SPLIT");
-        return e && e[0] == '1';
-    }();
-    g.tail = (split_on && tiles >= sms) ? tiles % sms : 0;
+    const int k_blocks = (int)(n_in / 256), m_max = (int)(rows >= kMaxTileM ? kMaxTileM : (rows + 15) / 16 * 16);
+    double best = 0.0;
+    g.tile_m = 0;
+    for (int tm = m_max; tm >= 16; tm -= 16) {
+        const int nm = (int)((rows + tm - 1) / tm);
+        if (nm > 1 && (tm & (kYChunk - 1)) != 0) continue;   // whole chunks: a store must not reach into the next tile's tokens
+        const long long tiles = (long long)g.n_tiles_n * nm;
+        const double wide = kStepBase + kStepToken * tm, step = wide > kStepMin ? wide : kStepMin;
+        for (int s = 1; s <= kMaxSplit; s *= 2) {
+            if (s > 1 && (s > k_blocks || tiles * s > sms * 15 / 16)) break;   // one wave of clusters only
+            const long long waves = (tiles * s + sms - 1) / sms;
+            const double t = waves * (4.0 * ((k_blocks + s - 1) / s) * step + tm * 12.0) + kFixedCycles + (s > 1 ? 1500.0 + tm * 8.0 : 0.0);
+            if (g.tile_m == 0 || t < best * 0.98) {   // a smaller tile or more pieces have to pay
+                best = t;
+                g.tile_m = tm;
+                g.n_tiles_m = nm;
+                g.split = s;
+            }
+        }
+    }
+    const long long ctas = (long long)g.n_tiles_n * g.n_tiles_m * g.split;
+    g.grid = (int)(ctas < sms ? ctas : sms);
     g.x_bytes = x_dtype == KRK_CUDA_X_F32 ? (((size_t)rows * (size_t)n_in * sizeof(__half) + 255) & ~(size_t)255) : 0;
-    g.count_bytes = g.tail ? (((size_t)g.tail * sizeof(unsigned) + 255) & ~(size_t)255) : 0;
     return g;
 }
 
-} // namespace
-
-size_t gemm_workspace_bytes(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows) {
-    const GemmPlan g = plan_gemm(x_dtype, n_out, n_in, rows);
-    return g.x_bytes + g.count_bytes;
+template <int WT>
+int launch_dense(GemmParams &p, const GemmPlan &g, const uint8_t *w, const __half *xh, cudaStream_t st, const float *x_f32) {
+    CUtensorMap x_map, y_map;
+    WMaps<kDense> w_maps;
+    const size_t smem = layout<WT>(p);
+    if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.n_in, p.rows, (size_t)p.n_in * sizeof(__half), kBK, p.tile_m,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !encode_w_maps<WT>(w_maps.m, w, p.n_out, p.row_bytes, kTileN))
+        return KRK_CUDA_ELAUNCH;
+    // Y as a [rows][n_out] f32 matrix, box = 128 weight rows x kYChunk tokens, for the stores of the read-out. A Y that
+    // is not 16-byte aligned with 16-byte-multiple rows cannot be described: the kernel then stores directly.
+    if (p.y_tma && !encode_2d(&y_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.y, p.n_out, p.rows, (size_t)p.n_out * sizeof(float), kTileN, kYChunk,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE))
+        return KRK_CUDA_ELAUNCH;
+    if (!p.y_tma) y_map = x_map;   // never used
+    // every map is encoded: from here on only a launch can fail
+    if (x_f32) {
+        const int rc = launch_f32_to_f16(const_cast<__half *>(xh), x_f32, p.rows * p.n_in, st);
+        if (rc != KRK_CUDA_OK) return rc;
+    }
+    return launch_kernel<WT, kDense>(p, x_map, w_maps, y_map, g.grid, smem, st);
 }
 
-int launch_gemm_tc(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out, int64_t n_in,
-                   int64_t rows, void *workspace, cudaStream_t st) {
-    if (rows > (1 << 24) || n_out > (1 << 30) || n_in > (1 << 24)) return KRK_CUDA_ESHAPE;
-    const GemmPlan g = plan_gemm(x_dtype, n_out, n_in, rows);
-    uint8_t *ws = static_cast<uint8_t *>(workspace);
-    const __half *xh = static_cast<const __half *>(x);
-    if (x_dtype == KRK_CUDA_X_F32) {
-        const int64_t n = rows * n_in;
-        const int64_t want = (n + 255) / 256;
-        const int cgrid = (int)(want < (int64_t)sm_count() * 8 ? want : (int64_t)sm_count() * 8);
-        f32_to_f16_kernel<<<cgrid, 256, 0, st>>>(reinterpret_cast<__half *>(ws), static_cast<const float *>(x), n);
-        note_launch();
-        const int rc = check_launch();
-        if (rc != KRK_CUDA_OK) return rc;
-        xh = reinterpret_cast<const __half *>(ws);
-    }
+int run_dense(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out, int64_t n_in, int64_t rows, __half *x_copy,
+              int *status, int sms, cudaStream_t st) {
+    const GemmPlan g = plan_gemm(x_dtype, n_out, n_in, rows, sms);
     GemmParams p{};
-    p.w = w;
     p.y = y;
     p.n_out = n_out;
     p.n_in = n_in;
@@ -1155,35 +1208,43 @@ int launch_gemm_tc(float *y, const void *x, int x_dtype, const uint8_t *w, int w
     p.tile_m = g.tile_m;
     p.n_tiles_n = g.n_tiles_n;
     p.n_tiles_m = g.n_tiles_m;
+    p.split = g.split;
     p.row_bytes = (int)row_bytes(wt, n_in);
     p.y_tma = ((reinterpret_cast<uintptr_t>(y) & 15) == 0 && (n_out % 4) == 0) ? 1 : 0;
-    p.split_tail = (g.tail && p.y_tma) ? 1 : 0;   // the pieces of a cut tile meet in Y through TMA reductions
-    p.tail_count = reinterpret_cast<unsigned *>(ws + g.x_bytes);
-    p.status = device_status_word();
-    if (!p.status) return KRK_CUDA_EDEVICE;
-    if (g.tail) {
-        const cudaError_t e = cudaMemsetAsync(p.tail_count, 0, g.count_bytes, st);
-        if (e != cudaSuccess) {
-            note_cuda_error(e);
-            return KRK_CUDA_ELAUNCH;
-        }
-    }
-
-    EncodeTiledFn encode = encode_tiled();
-    if (!encode) return KRK_CUDA_EDEVICE;
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)n_in, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)n_in * sizeof(__half)};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)p.tile_m};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims, strides, box, estr,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return KRK_CUDA_ELAUNCH;
-
+    p.status = status;
+    const bool f32 = x_dtype == KRK_CUDA_X_F32;
+    const __half *xh = f32 ? x_copy : static_cast<const __half *>(x);
     int rc = KRK_CUDA_EDTYPE;
-    KRK_DISPATCH_WT_GEMM(wt, rc = launch_wt<WT>(p, map, g.grid, st));
+    KRK_DISPATCH_WT(wt, rc = launch_dense<WT>(p, g, w, xh, st, f32 ? static_cast<const float *>(x) : nullptr));
     return rc;
+}
+
+} // namespace
+
+// f16 copy of n activations (n a multiple of 4), finite values beyond the f16 range saturated (half_sat).
+int launch_f32_to_f16(__half *out, const float *in, int64_t n, cudaStream_t st) {
+    const int64_t want = (n / 4 + 255) / 256;
+    const int grid = (int)(want < (int64_t)sm_count() * 8 ? want : (int64_t)sm_count() * 8);
+    const cudaError_t e = launch_overlapped(f32_to_f16_kernel, dim3((unsigned)grid), dim3(256), st, out, in, n / 4);
+    note_launch();
+    if (e != cudaSuccess) {
+        note_cuda_error(e);
+        (void)cudaGetLastError();
+        return KRK_CUDA_ELAUNCH;
+    }
+    return KRK_CUDA_OK;
+}
+
+size_t gemm_workspace_bytes(int x_dtype, int64_t, int64_t n_in, int64_t rows) {
+    return x_dtype == KRK_CUDA_X_F32 ? (((size_t)rows * (size_t)n_in * sizeof(__half) + 255) & ~(size_t)255) : 0;
+}
+
+int launch_gemm_tc(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out, int64_t n_in,
+                   int64_t rows, void *workspace, cudaStream_t st) {
+    if (rows > (1 << 24) || n_out > (1 << 30) || n_in > (1 << 24)) return KRK_CUDA_ESHAPE;
+    int *status = device_status_word();
+    if (!status) return KRK_CUDA_EDEVICE;
+    return run_dense(y, x, x_dtype, w, wt, n_out, n_in, rows, static_cast<__half *>(workspace), status, sm_count(), st);
 }
 
 // ---- prefill GEMM for callers that must not allocate --------------------------------------------------
@@ -1239,56 +1300,11 @@ extern "C" int krk_cuda_gemm_f32_static(void *y_f32, const void *x_f32, const vo
         scratch = g_static_addr[dev];
         sms = g_static_sms[dev];
     }
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    __half *xh = reinterpret_cast<__half *>(scratch);
-    int *status = reinterpret_cast<int *>(scratch + kStaticHalves * 2);
-
-    // Everything that can fail on the host comes before the first launch.
-    GemmParams p{};
-    p.w = static_cast<const uint8_t *>(w);
-    p.y = static_cast<float *>(y_f32);
-    p.n_out = n_out;
-    p.n_in = n_in;
-    p.rows = rows;
-    p.tile_m = rows >= kMaxTileM ? kMaxTileM : (int)((rows + 15) / 16 * 16);
-    p.n_tiles_n = (int)((n_out + kTileN - 1) / kTileN);
-    p.n_tiles_m = (int)((rows + p.tile_m - 1) / p.tile_m);
-    p.row_bytes = (int)row_bytes(wt, n_in);
-    // Y leaves by tensor stores only where a tensor map can describe it; otherwise element by element
-    p.y_tma = ((reinterpret_cast<uintptr_t>(y_f32) & 15) == 0 && (n_out % 4) == 0) ? 1 : 0;
-    p.split_tail = 0;   // cutting tiles needs counters in a workspace; this entry keeps whole tiles
-    p.tail_count = nullptr;
-    p.status = status;
-    EncodeTiledFn encode = encode_tiled();
-    if (!encode) return KRK_CUDA_EDEVICE;
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)n_in, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)n_in * sizeof(__half)};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)p.tile_m};
-    const cuuint32_t estr[2] = {1, 1};
-    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return KRK_CUDA_ELAUNCH;
-    {
-        CUtensorMap probe_map;   // the maps launch_wt will encode: refuse now rather than after the first kernel
-        if (!encode_w_map(&probe_map, p.w, wt, n_out, p.row_bytes) || !encode_y_map(&probe_map, p.y, p.w, n_out, rows, p.y_tma != 0))
-            return KRK_CUDA_ELAUNCH;
-    }
-
-    // Every call overwrites the part of the array it uses before reading it (the conversion kernel
-    // below), so nothing of the previous call's contents is ever consumed.
-    const int64_t n = rows * n_in;
-    const int64_t want = (n + 255) / 256;
-    const int cgrid = (int)(want < (int64_t)sms * 8 ? want : (int64_t)sms * 8);
-    f32_to_f16_kernel<<<cgrid, 256, 0, st>>>(xh, static_cast<const float *>(x_f32), n);
-    note_launch();
-    int rc = check_launch();
-    if (rc != KRK_CUDA_OK) return rc;
-    const int tiles = p.n_tiles_n * p.n_tiles_m;
-    const int grid = tiles < sms ? tiles : sms;
-    rc = KRK_CUDA_EDTYPE;
-    KRK_DISPATCH_WT_GEMM(wt, rc = launch_wt<WT>(p, map, grid, st));
-    return rc;
+    // Every call overwrites the part of the array it uses before reading it (the conversion kernel), so nothing of
+    // the previous call's contents is ever consumed.
+    return run_dense(static_cast<float *>(y_f32), x_f32, KRK_CUDA_X_F32, static_cast<const uint8_t *>(w), wt, n_out, n_in, rows,
+                     reinterpret_cast<__half *>(scratch), reinterpret_cast<int *>(scratch + kStaticHalves * 2), sms,
+                     static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int krk_cuda_gemm_f32_static_status(void) {

@@ -390,22 +390,6 @@ moe_plan_kernel(const __grid_constant__ MoeParams p, StreamTable *gate_up, Strea
     }
 }
 
-// A launch that may overlap the tail of the kernel before it in the stream (the kernel waits for that grid itself).
-template <class... KArgs, class... Args>
-cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-
 } // namespace
 
 int launch_route(int32_t *ids, float *wts, const float *logits, int64_t n_tok, int n_expert, int k,

@@ -136,3 +136,18 @@ np.save(sys.argv[1], y1.cpu().numpy())
     ref = oracle.gemm(x, w[sel], synth.Q4_K, len(sel), n_in, rows=rows, threads=8)
     ok, worst = bound_ok(y[:, sel], ref, oracle.dequant_rows(w[sel], synth.Q4_K, len(sel), n_in), x, GEMM_TOL)
     assert ok, worst
+
+
+@pytest.mark.parametrize("wt", [synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q5_1, synth.Q2_K, synth.Q3_K, synth.IQ4_NL])
+def test_gemm_split_k_clusters(cuda, oracle, wt):
+    """Few tiles: the CTAs of a cluster share a tile along K. Pieces of unequal length (an odd number of super-blocks),
+    outputs that float4 stores cannot describe (n_out % 4 != 0), fewer super-blocks than CTAs would like, weight rows
+    past the end of the matrix, and matrices of fewer rows than a phased tensor map has phases."""
+    for n_out, n_in, rows in ((130, 2304, 17), (64, 5376, 9), (7, 1280, 48), (257, 768, 250), (1001, 4352, 100)):
+        run_gemm(cuda, oracle, wt, n_out, n_in, rows, SEED + 110 + rows)
+
+
+@pytest.mark.parametrize("rows", [129, 288, 400])
+def test_gemm_token_tiles_narrower_than_the_rows(cuda, oracle, rows):
+    """More than one token tile of less than 256 tokens: a tile's last store must not reach into the next one's rows."""
+    run_gemm(cuda, oracle, synth.Q4_0, 2300, 512, rows, SEED + 120 + rows)
