@@ -4,6 +4,7 @@
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "krk_cuda.h"
@@ -248,16 +249,14 @@ struct GemvMat {
     int wt;
 };
 
-// A list of single-row GEMVs in device memory, for launches whose matrices are chosen on the device
-// (the routed experts). Entries are matrices, or gate/up pairs (2 matrices per entry); gran_begin is
-// the running count of row granules (see stream_gran) before each entry.
-constexpr int kStreamTableEntries = 64;
+// A list of GEMVs in device memory, for launches whose matrices are chosen on the device (the routed experts). Entries
+// are matrices, or gate/up pairs (2 matrices per entry), all of one shape.
 struct StreamTable {
-    GemvMat mat[2 * kStreamTableEntries];
-    int gran_begin[kStreamTableEntries + 1];
     int n_entries;
-    int total_gran;
+    int pad[3];
+    GemvMat mat[1];   // n_entries, or 2 * n_entries of them
 };
+inline size_t stream_table_bytes(size_t mats) { return (offsetof(StreamTable, mat) + mats * sizeof(GemvMat) + 255) & ~(size_t)255; }
 
 // Reference-shaped kernel (one warp per output row): takes every legal shape.
 int launch_gemv_generic(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate,
@@ -289,15 +288,13 @@ struct StreamBanks {
     const uint8_t *base[2];
     int64_t rows;
 };
-// Rows per granule the streaming kernel splits matrices of this type and width by (1, 8, or a whole tile when the
-// launch will use the banks' tensor maps), or 0 when it does not address the shape (then the shape-agnostic kernels
-// serve it).
-int stream_gran(int wt, int64_t n_in, bool banks = false);
-// The streaming kernel over a device-side table (one activation row per matrix; all matrices of type
-// wt and width n_in; built with the granule of stream_gran(wt, n_in, banks != nullptr)). Returns 1 when launched, 0
-// when the shape is not addressed, < 0 on error.
-int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_in, int silu_pair, const StreamBanks *banks,
-                             cudaStream_t st);
+// Does the streaming kernel address matrices of this type and width at this many activation rows? (Else the
+// shape-agnostic kernels serve them.)
+bool stream_takes(int wt, int64_t n_in, int rows);
+// The streaming kernel over a device-side table (`rows` activation rows per matrix; all matrices of type wt and shape
+// n_out x n_in). Returns 1 when launched, 0 when the shape is not addressed, < 0 on error.
+int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
+                             const StreamBanks *banks, cudaStream_t st);
 
 int launch_silu_mul(float *out, const float *gate, const float *up, int64_t n, cudaStream_t st);
 int launch_gather_rows(float *dst, const float *src, const int32_t *rows, int64_t n_rows, int64_t n, cudaStream_t st);
@@ -325,10 +322,27 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
 
 // Prefill GEMM on tcgen05 (krk_gemm_tc.cu).
 int launch_f32_to_f16(__half *out, const float *in, int64_t n, cudaStream_t st);
-// A group of up to tile_m tokens of one expert: its first weight row in the bank, its first X / output row, its tokens.
+// A group of up to tile_m tokens of one expert: the expert's place in the bank, its first X / output row, its tokens.
 struct GemmGroup {
-    int w_row, x_row, m;
+    int expert, x_row, m;
 };
+// The tensor-core products of routed experts: every group's X rows times its expert's weights. The groups and their
+// number lie in device memory; n_in and n_out are multiples of 256. gate_up: h = f16(silu(gate) * up), one row per
+// X row; down: y = f32 rows.
+struct ExpertGemm {
+    const __half *x;
+    int64_t x_rows;            // rows of x (and of the output) in all
+    const uint8_t *w, *w_up;   // the bank (gate_up: the gate bank and the up bank)
+    int64_t bank_rows;         // weight rows in a bank
+    int wt;
+    int64_t n_out, n_in;
+    int tile_m;                // tokens per group at most: a multiple of 32, <= 256
+    const GemmGroup *groups;
+    const int *n_groups;
+    int max_groups;
+};
+int launch_gemm_experts_gate_up(__half *h, const ExpertGemm &e, cudaStream_t st);
+int launch_gemm_experts_down(float *y, const ExpertGemm &e, cudaStream_t st);
 size_t gemm_workspace_bytes(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows);
 int launch_gemm_tc(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out,
                    int64_t n_in, int64_t rows, void *workspace, cudaStream_t st);

@@ -662,7 +662,7 @@ struct TileIter {
             const int g = i / p.n_tiles_n, nt = i - g * p.n_tiles_n;
             const GemmGroup gr = p.groups[g];
             t.n0 = nt * (KIND == kGateUp ? kTileN / 2 : kTileN);
-            t.w_row = gr.w_row + t.n0;
+            t.w_row = gr.expert * (int)p.n_out + t.n0;   // an expert holds n_out rows of (each) bank
             t.x_row = gr.x_row;
             t.m = gr.m;
         }
@@ -1219,7 +1219,53 @@ int run_dense(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, in
     return rc;
 }
 
+template <int WT, int KIND>
+int launch_experts(GemmParams &p, const ExpertGemm &e, cudaStream_t st) {
+    CUtensorMap x_map;
+    WMaps<KIND> w_maps;
+    constexpr int kRows = KIND == kGateUp ? kTileN / 2 : kTileN;   // rows of one matrix in a weight tile
+    p.row_bytes = (int)row_bytes(WT, e.n_in);
+    const size_t smem = layout<WT>(p);
+    if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, e.x, e.n_in, e.x_rows, (size_t)e.n_in * sizeof(__half), kBK, kGroupBox,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+        !encode_w_maps<WT>(w_maps.m, e.w, e.bank_rows, p.row_bytes, kRows) ||
+        (KIND == kGateUp && !encode_w_maps<WT>(w_maps.m + (row_phased(WT) ? kPhases : 1), e.w_up, e.bank_rows, p.row_bytes, kRows)))
+        return KRK_CUDA_ELAUNCH;
+    const long long tiles = (long long)e.max_groups * p.n_tiles_n;
+    const int sms = sm_count();
+    return launch_kernel<WT, KIND>(p, x_map, w_maps, x_map, (int)(tiles < sms ? tiles : sms), smem, st);
+}
+
+template <int KIND>
+int run_experts(GemmParams &p, const ExpertGemm &e, cudaStream_t st) {
+    p.n_out = e.n_out;
+    p.n_in = e.n_in;
+    p.rows = e.x_rows;
+    p.tile_m = e.tile_m;
+    p.n_tiles_n = (int)(e.n_out / (KIND == kGateUp ? kTileN / 2 : kTileN));
+    p.n_tiles_m = 1;
+    p.split = 1;
+    p.groups = e.groups;
+    p.n_groups = e.n_groups;
+    p.status = device_status_word();
+    if (!p.status) return KRK_CUDA_EDEVICE;
+    int rc = KRK_CUDA_EDTYPE;
+    KRK_DISPATCH_WT(e.wt, rc = (launch_experts<WT, KIND>(p, e, st)));
+    return rc;
+}
+
 } // namespace
+
+int launch_gemm_experts_gate_up(__half *h, const ExpertGemm &e, cudaStream_t st) {
+    GemmParams p{};
+    p.h = h;
+    return run_experts<kGateUp>(p, e, st);
+}
+int launch_gemm_experts_down(float *y, const ExpertGemm &e, cudaStream_t st) {
+    GemmParams p{};
+    p.y = y;
+    return run_experts<kDown>(p, e, st);
+}
 
 // f16 copy of n activations (n a multiple of 4), finite values beyond the f16 range saturated (half_sat).
 int launch_f32_to_f16(__half *out, const float *in, int64_t n, cudaStream_t st) {

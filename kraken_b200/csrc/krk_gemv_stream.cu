@@ -115,7 +115,8 @@ struct StreamParams {
     int n_stages;
     int total_gran;
     int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
-    const StreamTable *dev_table;   // when set, matrices and granule prefix come from device memory
+    const StreamTable *dev_table;   // when set, the matrices come from device memory
+    int entry_gran;       // table launches: granules of every entry (all have one shape)
     // Table launches with tensor copies: every matrix of the table lies inside one of two stacked banks (the gate
     // and the up bank of an expert set), each described by ONE tensor map (wmap[0], wmap[1]) over all of its
     // rows; a matrix is then a row offset into its bank.
@@ -306,23 +307,28 @@ struct StageInfo {
 // expert ids that never leave the device).
 struct TableView {
     const GemvMat *mat;
-    const int *gran_begin;
+    const int *gran_begin;   // host-built launches
+    int entry_gran;          // tables: granules per entry (0: host-built)
     int n_entries;
     int gran_q, gran_r;
+    __device__ __forceinline__ int begin(int e) const { return entry_gran ? e * entry_gran : gran_begin[e]; }
+    __device__ __forceinline__ int first(int g) const { return entry_gran ? g / entry_gran : 0; }   // no entry before it holds granule g
 };
 
 __device__ __forceinline__ TableView table_view(const StreamParams &p) {
     TableView tv;
     if (p.dev_table) {
         tv.mat = p.dev_table->mat;
-        tv.gran_begin = p.dev_table->gran_begin;
+        tv.gran_begin = nullptr;
+        tv.entry_gran = p.entry_gran;
         tv.n_entries = p.dev_table->n_entries;
-        const int total = p.dev_table->total_gran;
+        const int total = tv.n_entries * tv.entry_gran;
         tv.gran_q = total / (int)gridDim.x;
         tv.gran_r = total % (int)gridDim.x;
     } else {
         tv.mat = p.mat;
         tv.gran_begin = p.gran_begin;
+        tv.entry_gran = 0;
         tv.n_entries = p.n_entries;
         tv.gran_q = p.gran_q;
         tv.gran_r = p.gran_r;
@@ -338,12 +344,13 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
     const int g1 = g0 + tv.gran_q + (c < tv.gran_r ? 1 : 0);
     const int ku_max = p.whole_tiles ? p.units : kConsumerWarps;
     int slot = 0, phase = 0;
-    for (int e = 0; e < tv.n_entries; e++) {
-        const int lo = max(g0, tv.gran_begin[e]), hi = min(g1, tv.gran_begin[e + 1]);
+    for (int e = tv.first(g0); e < tv.n_entries; e++) {
+        const int lo = max(g0, tv.begin(e)), hi = min(g1, tv.begin(e + 1));
+        if (tv.begin(e) >= g1) break;
         if (lo >= hi) continue;
         const int n_out = (int)tv.mat[e * p.step].n_out;
-        const int r0 = (lo - tv.gran_begin[e]) * p.gran;
-        const int r1 = min(n_out, (hi - tv.gran_begin[e]) * p.gran);
+        const int r0 = (lo - tv.begin(e)) * p.gran;
+        const int r1 = min(n_out, (hi - tv.begin(e)) * p.gran);
         on_segment(e * p.step);
         const int stage_rows = kTileRows * tps;
         for (int tr = r0; tr < r1; tr += stage_rows) {
@@ -1485,12 +1492,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const uint32_t full0 = smem_u32(&sm->full[0]), empty0 = smem_u32(&sm->empty[0]);
     int slot = 0;
     uint32_t phase = 0;
-    for (int e = 0; e < tv.n_entries; e++) {
-        const int lo = max(g0, tv.gran_begin[e]), hi = min(g1, tv.gran_begin[e + 1]);
+    for (int e = tv.first(g0); e < tv.n_entries; e++) {
+        const int lo = max(g0, tv.begin(e)), hi = min(g1, tv.begin(e + 1));
+        if (tv.begin(e) >= g1) break;
         if (lo >= hi) continue;
         const int m = e * p.step;
-        const int r0 = (lo - tv.gran_begin[e]) * p.gran;
-        const int r1 = min((int)tv.mat[m].n_out, (hi - tv.gran_begin[e]) * p.gran);
+        const int r0 = (lo - tv.begin(e)) * p.gran;
+        const int r1 = min((int)tv.mat[m].n_out, (hi - tv.begin(e)) * p.gran);
         if (tv.mat[m].x != prepared) {
             // x may be the output of the kernel before this one (and y its input): wait for that grid to
             // complete. Weights are never written by a kernel in flight, so the producer warp does not wait.
@@ -1719,6 +1727,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.ragged = 0;
     p.gran = 1;
     p.dev_table = nullptr;
+    p.entry_gran = 0;
     p.n_peers = 0;
     p.my_rank = p.epoch = 0;
     p.peer_row_stride = p.peer_offset = 0;
@@ -1969,23 +1978,13 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
 }
 
 template <int WT>
-int gran_fmt(int64_t n_in, bool banks) {
+int launch_table_fmt(const StreamTable *table, int64_t n_out, int64_t n_in, int rows, int silu_pair, const StreamBanks *banks, cudaStream_t st) {
     StreamParams p;
     size_t smem = 0;
-    static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
-    if (banks && Fmt<WT>::tma == 1 && !no_tma && setup_format<WT>(p, n_in, 1, 0, &smem, true) && p.use_tma == 1) return p.gran;
-    return setup_format<WT>(p, n_in, 1, 0, &smem) ? p.gran : 0;
-}
-
-template <int WT>
-int launch_table_fmt(const StreamTable *table, int64_t n_in, int silu_pair, const StreamBanks *banks, cudaStream_t st) {
-    StreamParams p;
-    size_t smem = 0;
-    // With the banks known, a stage arrives as one tensor copy out of the bank's map (the table must then have been
-    // built with the granule of stream_gran(..., true): rows split at tile boundaries).
+    // With the banks known, a stage arrives as one tensor copy out of the bank's map.
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     bool tma = false;
-    if (banks && Fmt<WT>::tma == 1 && !no_tma && setup_format<WT>(p, n_in, 1, silu_pair, &smem, true) && p.use_tma == 1) {
+    if (banks && Fmt<WT>::tma == 1 && !no_tma && setup_format<WT>(p, n_in, rows, silu_pair, &smem, true) && p.use_tma == 1) {
         tma = true;
         const int ku_max = p.units < kConsumerWarps ? p.units : kConsumerWarps;
         for (int b = 0; b < p.step && tma; b++) {
@@ -1994,13 +1993,12 @@ int launch_table_fmt(const StreamTable *table, int64_t n_in, int silu_pair, cons
                   weight_map(&p.wmap[b], banks->base[b], banks->rows, p.row_bytes, Fmt<WT>::unit_bytes, kTileRows * p.tps, ku_max, 1);
         }
     }
-    if (!tma && !setup_format<WT>(p, n_in, 1, silu_pair, &smem)) return 0;
-    // the table was built with this granule whichever way the stages arrive (row copies take any granule)
-    if (banks) p.gran = gran_fmt<WT>(n_in, true);
+    if (!tma && !setup_format<WT>(p, n_in, rows, silu_pair, &smem)) return 0;
     p.n_entries = 0;
     p.total_gran = 0;
     p.gran_q = p.gran_r = 0;
     p.dev_table = table;
+    p.entry_gran = (int)((n_out + p.gran - 1) / p.gran);
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
     const int rc = launch_rows<WT>(p, sm_count() * ctas_per_sm<WT>(smem, p.rows), smem, st);
@@ -2079,21 +2077,11 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
     }
 }
 
-int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_in, int silu_pair, const StreamBanks *banks,
-                             cudaStream_t st) {
-    switch (wt) {
-    case KRK_CUDA_Q4_K: return launch_table_fmt<KRK_CUDA_Q4_K>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q6_K: return launch_table_fmt<KRK_CUDA_Q6_K>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q8_0: return launch_table_fmt<KRK_CUDA_Q8_0>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q4_0: return launch_table_fmt<KRK_CUDA_Q4_0>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q5_K: return launch_table_fmt<KRK_CUDA_Q5_K>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q2_K: return launch_table_fmt<KRK_CUDA_Q2_K>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q3_K: return launch_table_fmt<KRK_CUDA_Q3_K>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_IQ4_NL: return launch_table_fmt<KRK_CUDA_IQ4_NL>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q5_0: return launch_table_fmt<KRK_CUDA_Q5_0>(table, n_in, silu_pair, banks, st);
-    case KRK_CUDA_Q5_1: return launch_table_fmt<KRK_CUDA_Q5_1>(table, n_in, silu_pair, banks, st);
-    default: return 0;
-    }
+int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
+                             const StreamBanks *banks, cudaStream_t st) {
+    int rc = 0;
+    KRK_DISPATCH_WT(wt, rc = launch_table_fmt<WT>(table, n_out, n_in, rows, silu_pair, banks, st));
+    return rc;
 }
 
 int launch_gemv_stream_peers(const GemvMat &mat, int64_t n_in, int rows, const PeerScatter &ps, cudaStream_t st) {
@@ -2120,20 +2108,12 @@ int launch_flag_wait(const int *flags, int n, int epoch, cudaStream_t st) {
     return check_launch();
 }
 
-int stream_gran(int wt, int64_t n_in, bool banks) {
-    switch (wt) {
-    case KRK_CUDA_Q4_K: return gran_fmt<KRK_CUDA_Q4_K>(n_in, banks);
-    case KRK_CUDA_Q6_K: return gran_fmt<KRK_CUDA_Q6_K>(n_in, banks);
-    case KRK_CUDA_Q8_0: return gran_fmt<KRK_CUDA_Q8_0>(n_in, banks);
-    case KRK_CUDA_Q4_0: return gran_fmt<KRK_CUDA_Q4_0>(n_in, banks);
-    case KRK_CUDA_Q5_K: return gran_fmt<KRK_CUDA_Q5_K>(n_in, banks);
-    case KRK_CUDA_Q2_K: return gran_fmt<KRK_CUDA_Q2_K>(n_in, banks);
-    case KRK_CUDA_Q3_K: return gran_fmt<KRK_CUDA_Q3_K>(n_in, banks);
-    case KRK_CUDA_IQ4_NL: return gran_fmt<KRK_CUDA_IQ4_NL>(n_in, banks);
-    case KRK_CUDA_Q5_0: return gran_fmt<KRK_CUDA_Q5_0>(n_in, banks);
-    case KRK_CUDA_Q5_1: return gran_fmt<KRK_CUDA_Q5_1>(n_in, banks);
-    default: return 0;
-    }
+bool stream_takes(int wt, int64_t n_in, int rows) {
+    StreamParams p;
+    size_t smem = 0;
+    bool ok = false;
+    KRK_DISPATCH_WT(wt, ok = setup_format<WT>(p, n_in, rows, 0, &smem));
+    return ok;
 }
 
 } // namespace krk_cuda

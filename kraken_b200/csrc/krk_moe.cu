@@ -220,6 +220,8 @@ struct MoeParams {
     float *y;              // [n_tok][n_embd]
     int64_t n_embd, n_ff;
     int n_local, expert_base, k, n_tok;
+    const int32_t *pos;    // row of d that holds a pick (null: the pick's own number)
+    int vec;               // y takes float4 stores
 };
 
 __device__ __forceinline__ int local_expert(const MoeParams &p, int pick) {
@@ -273,9 +275,10 @@ moe_down_kernel(const __grid_constant__ MoeParams p) {
 // y[t][j] = sum over the picks of token t held here, ascending expert id, of w * d[pick][j]
 // starting from zero: the order and the arithmetic of the reference's per-expert
 // scatter_axpy_rows chain (src/engine.cpp:12353-, src/backend_cpu.cpp:3193-3220).
-__global__ void __launch_bounds__(256)
+constexpr int kCombineThreads = 128;
+__global__ void __launch_bounds__(kCombineThreads)
 moe_combine_kernel(const __grid_constant__ MoeParams p) {
-    __shared__ int s_pick[kMaxK];
+    __shared__ int s_row[kMaxK];
     __shared__ float s_w[kMaxK];
     __shared__ int s_n;
     // programmatic dependent launch: this grid may start while the one before it drains (it reads nothing before
@@ -300,40 +303,49 @@ moe_combine_kernel(const __grid_constant__ MoeParams p) {
             }
         }
         if (e >= 0) {
-            s_pick[rank] = t * p.k + s;
+            s_row[rank] = p.pos ? p.pos[t * p.k + s] : t * p.k + s;
             s_w[rank] = p.wts[t * p.k + s];
         }
         if (s == 0) s_n = n;
     }
     __syncthreads();
     const int n = s_n;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < p.n_embd;
-         j += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t n4 = p.n_embd >> 2;   // rows are whole 32-value blocks
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n4; j += (int64_t)gridDim.x * blockDim.x) {
         // the loads of a batch of eight go out together; the additions keep their order
-        float acc = 0.0f;
+        float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         for (int i0 = 0; i0 < n; i0 += 8) {
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = i0 + i < n ? p.d[(int64_t)s_pick[i0 + i] * p.n_embd + j] : 0.0f;
+            float4 v[8];
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                if (i0 + i < n) acc = __fadd_rn(acc, __fmul_rn(s_w[i0 + i], v[i]));
+                v[i] = i0 + i < n ? reinterpret_cast<const float4 *>(p.d + (int64_t)s_row[i0 + i] * p.n_embd)[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (i0 + i < n) {
+                    const float w = s_w[i0 + i];
+                    acc.x = __fadd_rn(acc.x, __fmul_rn(w, v[i].x));
+                    acc.y = __fadd_rn(acc.y, __fmul_rn(w, v[i].y));
+                    acc.z = __fadd_rn(acc.z, __fmul_rn(w, v[i].z));
+                    acc.w = __fadd_rn(acc.w, __fmul_rn(w, v[i].w));
+                }
         }
-        p.y[(int64_t)t * p.n_embd + j] = acc;
+        float *y = p.y + (int64_t)t * p.n_embd + 4 * j;
+        if (p.vec) *reinterpret_cast<float4 *>(y) = acc;
+        else y[0] = acc.x, y[1] = acc.y, y[2] = acc.z, y[3] = acc.w;
     }
 }
 
 // Builds the two device-side matrix tables of the streaming path from the routed expert ids: one
 // gate/up pair and one down matrix per pick this bank holds, ordered by expert id so that an expert
 // picked by several tokens is streamed by neighbouring CTAs at about the same time (its second read
-// comes from L2). One block; picks <= kStreamTableEntries.
+// comes from L2). One block; picks <= kPlanThreads.
 // With `logits` the routing itself runs first, one warp per token (n_tok <= 8), writing p.ids / p.wts.
 constexpr int kPlanThreads = 256;
 constexpr int kPlanRouteExperts = 1024;   // experts the fused routing holds in shared memory, per token
 __global__ void __launch_bounds__(kPlanThreads)
 moe_plan_kernel(const __grid_constant__ MoeParams p, StreamTable *gate_up, StreamTable *down, int wt_gate_up, int wt_down,
-                size_t rb_gate_up, size_t rb_down, int gran_gate_up, int gran_down, const float *logits, int n_expert) {
-    __shared__ int key[kStreamTableEntries];
+                size_t rb_gate_up, size_t rb_down, const float *logits, int n_expert) {
+    __shared__ int key[kPlanThreads];
     __shared__ float prob[KRK_CUDA_MAX_ROWS][kPlanRouteExperts];
     __shared__ int sid[KRK_CUDA_MAX_ROWS][kMaxK];   // the ids the fused routing picked, for the plan below
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (see moe_combine_kernel)
@@ -353,8 +365,8 @@ moe_plan_kernel(const __grid_constant__ MoeParams p, StreamTable *gate_up, Strea
         const int le = id - p.expert_base;
         e = (le >= 0 && le < p.n_local) ? le : -1;
     }
-    if (pick < kStreamTableEntries) key[pick] = e >= 0 ? e * kStreamTableEntries + pick : 0x7FFFFFFF;
-    __syncthreads();
+    key[pick] = e >= 0 ? e * kPlanThreads + pick : 0x7FFFFFFF;
+    const int n = __syncthreads_count(e >= 0);
     if (e >= 0) {
         int rank = 0;
         for (int j = 0; j < n_pick; j++) rank += key[j] < key[pick];
@@ -376,17 +388,156 @@ moe_plan_kernel(const __grid_constant__ MoeParams p, StreamTable *gate_up, Strea
         gate_up->mat[2 * rank + 1] = u;
         down->mat[rank] = d;
     }
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int j = 0; j < n_pick; j++) n += key[j] != 0x7FFFFFFF;
-        const int gu = (int)((p.n_ff + gran_gate_up - 1) / gran_gate_up), dn = (int)((p.n_embd + gran_down - 1) / gran_down);
-        for (int i = 0; i <= n; i++) {
-            gate_up->gran_begin[i] = i * gu;
-            down->gran_begin[i] = i * dn;
+    if (threadIdx.x == 0) gate_up->n_entries = down->n_entries = n;
+}
+
+// ---- more than eight tokens ----------------------------------------------------------------------------------
+// Expert-major (the reference's grouped form, src/engine.cpp:12353-12690), planned and run on the device without the
+// host ever seeing the counts. Experts that more than kFewRows tokens picked run on the tensor cores: their tokens'
+// rows are gathered into one f16 block, groups of up to tile_m rows of it are the token tiles of the expert GEMMs.
+// Experts with fewer rows keep f32 activations on the streaming kernel: one table per capacity class (rows are
+// padded to the class, so that one launch serves all experts of a class). A launch over an empty list or table ends
+// at once; the host picks the classes from the expected rows per expert, so that few of them are empty.
+constexpr int kFewRows = KRK_CUDA_MAX_ROWS;
+constexpr int kMaxClasses = 4;
+struct GroupedParams {
+    const uint8_t *gate, *up, *down;
+    size_t rb_gate_up, rb_down;
+    int wt_gate_up, wt_down;
+    const float *x;        // [n_tok][n_embd]
+    const int32_t *ids;    // [n_tok][k]
+    int64_t n_embd, n_ff;
+    int n_local, expert_base, k, n_tok, tile_m;
+    int n_class, cap[kMaxClasses];        // rows per expert of each class, ascending, the last kFewRows
+    int *n_groups;
+    GemmGroup *groups;
+    StreamTable *table_gu[kMaxClasses], *table_dn[kMaxClasses];
+    __half *xg;            // [picks][n_embd]: gathered rows of the tensor-core experts
+    float *xs, *hs;        // [rows][n_embd], [rows][n_ff]: the few-row experts' activations
+    float *d;              // [picks + rows][n_embd]: down projections, tensor-core rows first
+    int32_t *pos;          // [n_tok][k]: a pick's row of d (-1: held elsewhere)
+};
+
+// Exclusive sum over the block's 1024 threads; `total` is the sum of all.
+__device__ __forceinline__ int block_scan(int v, int *warp_sums, int &total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    __syncthreads();   // the sums of the scan before are read
+    if (lane == 31) warp_sums[warp] = inc;
+    __syncthreads();
+    const int w = warp_sums[lane];
+    int winc = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xFFFFFFFFu, winc, o);
+        if (lane >= o) winc += u;
+    }
+    total = __shfl_sync(0xFFFFFFFFu, winc, 31);
+    return inc - v + __shfl_sync(0xFFFFFFFFu, winc - w, warp);
+}
+
+// One block; thread e looks after expert e. Picks take places in their expert's rows through shared-memory counters;
+// the few-row experts' picks are then put in token order (a row's place decides which limb columns it rides in, and
+// with them the rounding order of its sums; a tensor-core row's place changes nothing).
+__global__ void __launch_bounds__(kMaxExperts)
+moe_group_plan_kernel(const __grid_constant__ GroupedParams p) {
+    __shared__ int cnt[kMaxExperts], base[kMaxExperts], list[kMaxExperts * kFewRows], warp_sums[32];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int e = threadIdx.x, n_pick = p.n_tok * p.k;
+    cnt[e] = 0;
+    __syncthreads();
+    for (int i = e; i < n_pick; i += kMaxExperts) {
+        const int le = p.ids[i] - p.expert_base;
+        if (le >= 0 && le < p.n_local) atomicAdd(&cnt[le], 1);
+    }
+    __syncthreads();
+    const int m = cnt[e];
+    const bool few = m > 0 && m <= kFewRows, many = m > kFewRows;
+    int cls = 0;
+    while (cls + 1 < p.n_class && p.cap[cls] < m) cls++;
+    int total;
+    const int many_off = block_scan(many ? m : 0, warp_sums, total);
+    const int group_off = block_scan(many ? (m + p.tile_m - 1) / p.tile_m : 0, warp_sums, total);
+    if (e == 0) *p.n_groups = total;
+    const int few_off = block_scan(few ? p.cap[cls] : 0, warp_sums, total);
+    for (int c = 0; c < p.n_class; c++) {
+        const int at = block_scan(few && cls == c, warp_sums, total);
+        if (e == 0) p.table_gu[c]->n_entries = p.table_dn[c]->n_entries = total;
+        if (few && cls == c) {
+            GemvMat g, u, d;
+            g.w = p.gate + (size_t)e * p.n_ff * p.rb_gate_up;
+            u.w = p.up + (size_t)e * p.n_ff * p.rb_gate_up;
+            g.x = u.x = p.xs + (int64_t)few_off * p.n_embd;
+            g.y = u.y = p.hs + (int64_t)few_off * p.n_ff;   // the pair's fold writes silu(gate) * up through the gate's pointer
+            g.n_out = u.n_out = p.n_ff;
+            g.wt = u.wt = p.wt_gate_up;
+            d.w = p.down + (size_t)e * p.n_embd * p.rb_down;
+            d.x = g.y;
+            d.y = p.d + (int64_t)(n_pick + few_off) * p.n_embd;
+            d.n_out = p.n_embd;
+            d.wt = p.wt_down;
+            p.table_gu[c]->mat[2 * at] = g;
+            p.table_gu[c]->mat[2 * at + 1] = u;
+            p.table_dn[c]->mat[at] = d;
         }
-        gate_up->n_entries = down->n_entries = n;
-        gate_up->total_gran = n * gu;
-        down->total_gran = n * dn;
+    }
+    if (many)
+        for (int g = 0; g * p.tile_m < m; g++) p.groups[group_off + g] = GemmGroup{e, many_off + g * p.tile_m, min(p.tile_m, m - g * p.tile_m)};
+    base[e] = many ? many_off : n_pick + few_off;
+    cnt[e] = 0;
+    __syncthreads();
+    for (int i = e; i < n_pick; i += kMaxExperts) {
+        const int le = p.ids[i] - p.expert_base;
+        if (le < 0 || le >= p.n_local) {
+            p.pos[i] = -1;
+            continue;
+        }
+        const int slot = atomicAdd(&cnt[le], 1), b = base[le];
+        if (b < n_pick) p.pos[i] = b + slot;
+        else list[le * kFewRows + slot] = i;
+    }
+    __syncthreads();
+    if (few) {
+        int *mine = list + e * kFewRows;
+        for (int i = 1; i < m; i++) {
+            const int v = mine[i];
+            int j = i;
+            for (; j > 0 && mine[j - 1] > v; j--) mine[j] = mine[j - 1];
+            mine[j] = v;
+        }
+        for (int i = 0; i < m; i++) p.pos[mine[i]] = base[e] + i;
+    }
+}
+
+// Every pick's activation row to its place: f16 for the tensor-core experts (rounded as the dense GEMM rounds f32
+// activations), f32 for the others. One block per pick; a token's row comes out of L2 for all picks but the first.
+constexpr int kGatherThreads = 128;
+__global__ void __launch_bounds__(kGatherThreads)
+moe_gather_kernel(const __grid_constant__ GroupedParams p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int pick = blockIdx.x, row = p.pos[pick], n_pick = p.n_tok * p.k;
+    if (row < 0) return;
+    const float4 *src = reinterpret_cast<const float4 *>(p.x + (int64_t)(pick / p.k) * p.n_embd);
+    const int n4 = (int)(p.n_embd >> 2);
+    if (row < n_pick) {
+        uint2 *dst = reinterpret_cast<uint2 *>(p.xg + (int64_t)row * p.n_embd);
+#pragma unroll 4
+        for (int j = threadIdx.x; j < n4; j += kGatherThreads) {
+            const float4 v = src[j];
+            const __half2 a = __halves2half2(half_sat(v.x), half_sat(v.y)), b = __halves2half2(half_sat(v.z), half_sat(v.w));
+            dst[j] = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        }
+    } else {
+        float4 *dst = reinterpret_cast<float4 *>(p.xs + (int64_t)(row - n_pick) * p.n_embd);
+#pragma unroll 4
+        for (int j = threadIdx.x; j < n4; j += kGatherThreads) dst[j] = src[j];
     }
 }
 
@@ -428,52 +579,222 @@ int launch_moe_plan_build(const int32_t *ids, int64_t n_rows, int k, int n_exper
     return check_launch();
 }
 
+static size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// n_tok <= 8: per-pick h and d rows, then the two matrix tables of the streaming path
 static size_t moe_float_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
-    const size_t b = sizeof(float) * (size_t)(n_tok * k) * (size_t)(bank->n_ff + bank->n_embd);
-    return (b + 255) & ~(size_t)255;
+    return up256(sizeof(float) * (size_t)(n_tok * k) * (size_t)(bank->n_ff + bank->n_embd));
 }
 
-// ---- more than eight tokens: expert-major, the tokens of an expert as one matrix (the reference's grouped form,
-// src/engine.cpp:12353-12690: gather the expert's rows, gate / up as a GEMM each, silu_mul, down, scatter-add).
+// More than eight tokens, shapes that the tensor-core and the streaming kernels address: the workspace of
+// launch_moe_ffn_grouped. Calls of many tokens go in chunks, so that it stays bounded.
+constexpr int64_t kChunkPicks = 65536;
 struct GroupedLayout {
-    size_t off, rows, wt, xg, g, u, dg, gemm, total;
-    size_t gemm_bytes;
+    size_t head, groups, pos, tables[kMaxClasses], xg, h, xs, hs, d, total;
+    int64_t chunk;   // tokens per chunk
+    int max_groups, max_few;
 };
-static size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
-// rung for a [m x n_in] . W^T product by row count: streaming / shape-agnostic GEMV up to 8 rows, tensor cores above
-static size_t grouped_gemm_bytes(const krk_cuda_expert_bank *bank, int64_t n_tok) {
-    size_t a = 0, b = 0;
-    if (bank->n_embd % 256 == 0 && gemm_tc_takes(bank->wt_gate_up)) a = gemm_workspace_bytes(KRK_CUDA_X_F32, bank->n_ff, bank->n_embd, n_tok);
-    if (bank->n_ff % 256 == 0 && gemm_tc_takes(bank->wt_down)) b = gemm_workspace_bytes(KRK_CUDA_X_F32, bank->n_embd, bank->n_ff, n_tok);
-    return up256(a > b ? a : b);
-}
+constexpr int kMinTileM = 32;
 static GroupedLayout grouped_layout(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
     GroupedLayout L;
+    L.chunk = kChunkPicks / k < n_tok ? kChunkPicks / k : n_tok;
+    const size_t picks = (size_t)(L.chunk * k);
+    L.max_few = (int)((int64_t)picks < bank->n_local ? (int64_t)picks : bank->n_local);
+    L.max_groups = (int)(picks / kMinTileM) + bank->n_local;
+    const size_t few_rows = (size_t)L.max_few * kFewRows;
+    size_t at = 0;
+    auto take = [&at](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
+    L.head = take(sizeof(int));
+    L.groups = take(sizeof(GemmGroup) * (size_t)L.max_groups);
+    L.pos = take(sizeof(int32_t) * picks);
+    for (int c = 0; c < kMaxClasses; c++)
+        L.tables[c] = take(stream_table_bytes(2 * (size_t)L.max_few) + stream_table_bytes((size_t)L.max_few));
+    L.xg = take(sizeof(__half) * picks * bank->n_embd);
+    L.h = take(sizeof(__half) * picks * bank->n_ff);
+    L.xs = take(sizeof(float) * few_rows * bank->n_embd);
+    L.hs = take(sizeof(float) * few_rows * bank->n_ff);
+    L.d = take(sizeof(float) * (picks + few_rows) * bank->n_embd);
+    L.total = at;
+    return L;
+}
+static bool grouped_takes(const krk_cuda_expert_bank *bank) {
+    return bank->n_embd % 256 == 0 && bank->n_ff % 256 == 0 && stream_takes(bank->wt_gate_up, bank->n_embd, kFewRows) &&
+           stream_takes(bank->wt_down, bank->n_ff, kFewRows);
+}
+
+// The other shapes: one expert after the other, the tokens of an expert as one matrix.
+struct LoopLayout {
+    size_t off, rows, wt, xg, g, u, dg, gemm, total;
+};
+// rung for a [m x n_in] . W^T product by row count: streaming / shape-agnostic GEMV up to 8 rows, tensor cores above
+static size_t loop_gemm_bytes(const krk_cuda_expert_bank *bank, int64_t n_tok) {
+    size_t a = 0, b = 0;
+    if (bank->n_embd % 256 == 0) a = gemm_workspace_bytes(KRK_CUDA_X_F32, bank->n_ff, bank->n_embd, n_tok);
+    if (bank->n_ff % 256 == 0) b = gemm_workspace_bytes(KRK_CUDA_X_F32, bank->n_embd, bank->n_ff, n_tok);
+    return a > b ? a : b;
+}
+static LoopLayout loop_layout(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
+    LoopLayout L;
     const size_t picks = (size_t)(n_tok * k);
     size_t at = 0;
-    L.off = at; at += up256(sizeof(int32_t) * (kMaxExperts + 1));
-    L.rows = at; at += up256(sizeof(int32_t) * picks);
-    L.wt = at; at += up256(sizeof(float) * picks);
-    L.xg = at; at += up256(sizeof(float) * (size_t)n_tok * bank->n_embd);
-    L.g = at; at += up256(sizeof(float) * (size_t)n_tok * bank->n_ff);
-    L.u = at; at += up256(sizeof(float) * (size_t)n_tok * bank->n_ff);
-    L.dg = at; at += up256(sizeof(float) * (size_t)n_tok * bank->n_embd);
-    L.gemm = at;
-    L.gemm_bytes = grouped_gemm_bytes(bank, n_tok);
-    at += L.gemm_bytes;
+    auto take = [&at](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
+    L.off = take(sizeof(int32_t) * (kMaxExperts + 1));
+    L.rows = take(sizeof(int32_t) * picks);
+    L.wt = take(sizeof(float) * picks);
+    L.xg = take(sizeof(float) * (size_t)n_tok * bank->n_embd);
+    L.g = take(sizeof(float) * (size_t)n_tok * bank->n_ff);
+    L.u = take(sizeof(float) * (size_t)n_tok * bank->n_ff);
+    L.dg = take(sizeof(float) * (size_t)n_tok * bank->n_embd);
+    L.gemm = take(loop_gemm_bytes(bank, n_tok));
     L.total = at;
     return L;
 }
 
 size_t moe_workspace_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
-    if (n_tok > KRK_CUDA_MAX_ROWS) return grouped_layout(bank, k, n_tok).total;
-    // per-pick h and d rows, then the two matrix tables of the streaming path
-    return moe_float_bytes(bank, k, n_tok) + 2 * ((sizeof(StreamTable) + 255) & ~(size_t)255);
+    if (n_tok > KRK_CUDA_MAX_ROWS) return grouped_takes(bank) ? grouped_layout(bank, k, n_tok).total : loop_layout(bank, k, n_tok).total;
+    const size_t picks = (size_t)(n_tok * k);
+    return moe_float_bytes(bank, k, n_tok) + stream_table_bytes(2 * picks) + stream_table_bytes(picks);
+}
+
+static int launched(cudaError_t e) {
+    note_launch();
+    if (e != cudaSuccess) {
+        note_cuda_error(e);
+        (void)cudaGetLastError();
+        return KRK_CUDA_ELAUNCH;
+    }
+    return KRK_CUDA_OK;
+}
+
+static int launch_combine(const MoeParams &p, cudaStream_t st) {
+    const int64_t n4 = p.n_embd / 4;
+    return launched(launch_overlapped(moe_combine_kernel, dim3((unsigned)((n4 + kCombineThreads - 1) / kCombineThreads), (unsigned)p.n_tok),
+                                      dim3(kCombineThreads), st, p));
+}
+
+static MoeParams moe_params(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
+    MoeParams p;
+    p.gate = static_cast<const uint8_t *>(bank->gate);
+    p.up = static_cast<const uint8_t *>(bank->up);
+    p.down = static_cast<const uint8_t *>(bank->down);
+    p.x = x;
+    p.ids = ids;
+    p.wts = wts;
+    p.h = p.d = nullptr;
+    p.y = y;
+    p.n_embd = bank->n_embd;
+    p.n_ff = bank->n_ff;
+    p.n_local = bank->n_local;
+    p.expert_base = bank->expert_base;
+    p.k = k;
+    p.n_tok = (int)n_tok;
+    p.pos = nullptr;
+    p.vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+    return p;
+}
+
+static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const float *x, const int32_t *ids, const float *wts,
+                         const krk_cuda_expert_bank *bank, int k, int64_t n_tok, int n_expert, cudaStream_t st) {
+    GroupedParams p;
+    p.gate = static_cast<const uint8_t *>(bank->gate);
+    p.up = static_cast<const uint8_t *>(bank->up);
+    p.down = static_cast<const uint8_t *>(bank->down);
+    p.rb_gate_up = row_bytes(bank->wt_gate_up, bank->n_embd);
+    p.rb_down = row_bytes(bank->wt_down, bank->n_ff);
+    p.wt_gate_up = bank->wt_gate_up;
+    p.wt_down = bank->wt_down;
+    p.x = x;
+    p.ids = ids;
+    p.n_embd = bank->n_embd;
+    p.n_ff = bank->n_ff;
+    p.n_local = bank->n_local;
+    p.expert_base = bank->expert_base;
+    p.k = k;
+    p.n_tok = (int)n_tok;
+    // From the rows an expert can expect: the token tile (an expert's rows should fit one, since every further tile
+    // decodes its weights again; up to 128 tokens two accumulators alternate), and the classes of the few-row experts.
+    const int64_t picks = n_tok * k, mean = picks / n_expert;
+    p.tile_m = mean <= 44 ? 64 : mean <= 100 ? 128 : 256;
+    static const int kCaps[4][kMaxClasses] = {{1, 2, 4, 8}, {2, 4, 8, 8}, {4, 8, 8, 8}, {8, 8, 8, 8}};
+    const int pick_caps = 2 * picks < 3 * n_expert ? 0 : picks < 6 * n_expert ? 1 : picks < 14 * n_expert ? 2 : 3;
+    p.n_class = kMaxClasses - pick_caps;
+    for (int c = 0; c < kMaxClasses; c++) p.cap[c] = kCaps[pick_caps][c];
+    p.n_groups = reinterpret_cast<int *>(ws + L.head);
+    p.groups = reinterpret_cast<GemmGroup *>(ws + L.groups);
+    p.pos = reinterpret_cast<int32_t *>(ws + L.pos);
+    for (int c = 0; c < kMaxClasses; c++) {
+        p.table_gu[c] = reinterpret_cast<StreamTable *>(ws + L.tables[c]);
+        p.table_dn[c] = reinterpret_cast<StreamTable *>(ws + L.tables[c] + stream_table_bytes(2 * (size_t)L.max_few));
+    }
+    p.xg = reinterpret_cast<__half *>(ws + L.xg);
+    p.xs = reinterpret_cast<float *>(ws + L.xs);
+    p.hs = reinterpret_cast<float *>(ws + L.hs);
+    p.d = reinterpret_cast<float *>(ws + L.d);
+    __half *h = reinterpret_cast<__half *>(ws + L.h);
+
+    int rc = launched(launch_overlapped(moe_group_plan_kernel, dim3(1), dim3(kMaxExperts), st, p));
+    if (rc != KRK_CUDA_OK) return rc;
+    if ((rc = launched(launch_overlapped(moe_gather_kernel, dim3((unsigned)picks), dim3(kGatherThreads), st, p))) != KRK_CUDA_OK) return rc;
+
+    ExpertGemm gu, dn;
+    gu.x = p.xg;
+    gu.x_rows = dn.x_rows = picks;
+    gu.w = p.gate;
+    gu.w_up = p.up;
+    gu.bank_rows = (int64_t)bank->n_local * bank->n_ff;
+    gu.wt = bank->wt_gate_up;
+    gu.n_out = bank->n_ff;
+    gu.n_in = bank->n_embd;
+    dn.x = h;
+    dn.w = p.down;
+    dn.w_up = nullptr;
+    dn.bank_rows = (int64_t)bank->n_local * bank->n_embd;
+    dn.wt = bank->wt_down;
+    dn.n_out = bank->n_embd;
+    dn.n_in = bank->n_ff;
+    gu.tile_m = dn.tile_m = p.tile_m;
+    gu.groups = dn.groups = p.groups;
+    gu.n_groups = dn.n_groups = p.n_groups;
+    gu.max_groups = dn.max_groups = L.max_groups;
+    StreamBanks gu_banks, dn_banks;
+    gu_banks.base[0] = p.gate;
+    gu_banks.base[1] = p.up;
+    gu_banks.rows = gu.bank_rows;
+    dn_banks.base[0] = p.down;
+    dn_banks.base[1] = nullptr;
+    dn_banks.rows = dn.bank_rows;
+    if ((rc = launch_gemm_experts_gate_up(h, gu, st)) != KRK_CUDA_OK) return rc;
+    for (int c = 0; c < p.n_class; c++)
+        if ((rc = launch_gemv_stream_table(p.table_gu[c], bank->wt_gate_up, bank->n_ff, bank->n_embd, p.cap[c], 1, &gu_banks, st)) < 0) return rc;
+    if ((rc = launch_gemm_experts_down(p.d, dn, st)) != KRK_CUDA_OK) return rc;
+    for (int c = 0; c < p.n_class; c++)
+        if ((rc = launch_gemv_stream_table(p.table_dn[c], bank->wt_down, bank->n_embd, bank->n_ff, p.cap[c], 0, &dn_banks, st)) < 0) return rc;
+
+    MoeParams cp = moe_params(y, x, ids, wts, bank, k, n_tok);
+    cp.d = p.d;
+    cp.pos = p.pos;
+    return launch_combine(cp, st);
+}
+
+static int launch_moe_ffn_grouped(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank,
+                                  int k, int64_t n_tok, int n_expert, void *workspace, cudaStream_t st) {
+    const int last = bank->expert_base + bank->n_local;   // ids at or above this are held elsewhere
+    if (last > kMaxExperts) return KRK_CUDA_EARG;
+    if (n_expert < last) n_expert = last;
+    if (n_expert < 1) n_expert = 1;
+    const GroupedLayout L = grouped_layout(bank, k, n_tok);
+    for (int64_t t0 = 0; t0 < n_tok; t0 += L.chunk) {
+        const int64_t n = n_tok - t0 < L.chunk ? n_tok - t0 : L.chunk;
+        const int rc = moe_ffn_chunk(L, static_cast<uint8_t *>(workspace), y + t0 * bank->n_embd, x + t0 * bank->n_embd, ids + t0 * k,
+                                     wts + t0 * k, bank, k, n, n_expert, st);
+        if (rc != KRK_CUDA_OK) return rc;
+    }
+    return KRK_CUDA_OK;
 }
 
 static int grouped_matmul(float *y, const float *x, const uint8_t *w, int wt, int64_t n_out, int64_t n_in, int64_t m, void *ws,
                           cudaStream_t st) {
-    if (m > KRK_CUDA_MAX_ROWS && n_in % 256 == 0 && gemm_tc_takes(wt))
+    if (m > KRK_CUDA_MAX_ROWS && n_in % 256 == 0)
         return launch_gemm_tc(y, x, KRK_CUDA_X_F32, w, wt, n_out, n_in, m, ws, st);
     for (int64_t r0 = 0; r0 < m; r0 += KRK_CUDA_MAX_ROWS) {
         const int64_t nr = m - r0 < KRK_CUDA_MAX_ROWS ? m - r0 : KRK_CUDA_MAX_ROWS;
@@ -494,11 +815,11 @@ static int grouped_matmul(float *y, const float *x, const uint8_t *w, int wt, in
 // y[n_tok][n_embd] = sum over the picks this bank holds, experts in ascending id, of w * down(silu(gate x) * up x).
 // One device-to-host copy of the plan's offsets (a stream synchronisation) tells the host how many rows each
 // expert has, as the reference's host plan does.
-static int launch_moe_ffn_grouped(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank,
-                                  int k, int64_t n_tok, void *workspace, cudaStream_t st) {
+static int launch_moe_ffn_loop(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank,
+                               int k, int64_t n_tok, void *workspace, cudaStream_t st) {
     const int n_expert = bank->expert_base + bank->n_local;   // ids at or above this are held elsewhere
     if (n_expert > kMaxExperts) return KRK_CUDA_EARG;
-    const GroupedLayout L = grouped_layout(bank, k, n_tok);
+    const LoopLayout L = loop_layout(bank, k, n_tok);
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     int32_t *off = reinterpret_cast<int32_t *>(ws + L.off), *rows = reinterpret_cast<int32_t *>(ws + L.rows);
     float *wt = reinterpret_cast<float *>(ws + L.wt), *xg = reinterpret_cast<float *>(ws + L.xg);
@@ -544,24 +865,12 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
             const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);
             if (rc != KRK_CUDA_OK) return rc;
         }
-        return launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, workspace, st);
+        return grouped_takes(bank) ? launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, n_expert, workspace, st)
+                                   : launch_moe_ffn_loop(y, x, ids, wts, bank, k, n_tok, workspace, st);
     }
-    MoeParams p;
-    p.gate = static_cast<const uint8_t *>(bank->gate);
-    p.up = static_cast<const uint8_t *>(bank->up);
-    p.down = static_cast<const uint8_t *>(bank->down);
-    p.x = x;
-    p.ids = ids;
-    p.wts = wts;
+    MoeParams p = moe_params(y, x, ids, wts, bank, k, n_tok);
     p.h = static_cast<float *>(workspace);
     p.d = p.h + (size_t)(n_tok * k) * bank->n_ff;
-    p.y = y;
-    p.n_embd = bank->n_embd;
-    p.n_ff = bank->n_ff;
-    p.n_local = bank->n_local;
-    p.expert_base = bank->expert_base;
-    p.k = k;
-    p.n_tok = (int)n_tok;
     const int picks = (int)(n_tok * k);
     // Streaming path: the same kernel as the dense decode GEMV, fed from device-side tables.
     // gate and up experts are rows of two stacked banks: their table launch stages weights out of one tensor map each
@@ -569,42 +878,24 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
     gu_banks.base[0] = p.gate;
     gu_banks.base[1] = p.up;
     gu_banks.rows = (int64_t)bank->n_local * bank->n_ff;
-    const int gran_gu = stream_gran(bank->wt_gate_up, bank->n_embd, true), gran_dn = stream_gran(bank->wt_down, bank->n_ff);
-    if (gran_gu > 0 && gran_dn > 0 && picks <= kStreamTableEntries) {
+    if (picks <= kPlanThreads && stream_takes(bank->wt_gate_up, bank->n_embd, 1) && stream_takes(bank->wt_down, bank->n_ff, 1)) {
         const bool fuse_route = !routed && n_expert <= kPlanRouteExperts && n_tok * 32 <= kPlanThreads;
         if (!routed && !fuse_route) {
             const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);
             if (rc != KRK_CUDA_OK) return rc;
         }
-        routed = true;
         uint8_t *tables = static_cast<uint8_t *>(workspace) + moe_float_bytes(bank, k, n_tok);
         StreamTable *ta = reinterpret_cast<StreamTable *>(tables);
-        StreamTable *tb = reinterpret_cast<StreamTable *>(tables + ((sizeof(StreamTable) + 255) & ~(size_t)255));
-        cudaError_t le = launch_overlapped(moe_plan_kernel, dim3(1), dim3(kPlanThreads), st, p, ta, tb, bank->wt_gate_up,
-                                           bank->wt_down, row_bytes(bank->wt_gate_up, bank->n_embd),
-                                           row_bytes(bank->wt_down, bank->n_ff), gran_gu, gran_dn,
-                                           fuse_route ? logits : (const float *)nullptr, n_expert);
-        note_launch();
-        if (le != cudaSuccess) {
-            note_cuda_error(le);
-            (void)cudaGetLastError();
-            return KRK_CUDA_ELAUNCH;
-        }
-        int rc = check_launch();
+        StreamTable *tb = reinterpret_cast<StreamTable *>(tables + stream_table_bytes(2 * (size_t)picks));
+        int rc = launched(launch_overlapped(moe_plan_kernel, dim3(1), dim3(kPlanThreads), st, p, ta, tb, bank->wt_gate_up, bank->wt_down,
+                                            row_bytes(bank->wt_gate_up, bank->n_embd), row_bytes(bank->wt_down, bank->n_ff),
+                                            fuse_route ? logits : (const float *)nullptr, n_expert));
         if (rc != KRK_CUDA_OK) return rc;
-        rc = launch_gemv_stream_table(ta, bank->wt_gate_up, bank->n_embd, 1, &gu_banks, st);
+        rc = launch_gemv_stream_table(ta, bank->wt_gate_up, bank->n_ff, bank->n_embd, 1, 1, &gu_banks, st);
         if (rc < 0) return rc;
-        rc = launch_gemv_stream_table(tb, bank->wt_down, bank->n_ff, 0, nullptr, st);
+        rc = launch_gemv_stream_table(tb, bank->wt_down, bank->n_embd, bank->n_ff, 1, 0, nullptr, st);
         if (rc < 0) return rc;
-        dim3 grid((unsigned)((bank->n_embd + 255) / 256), (unsigned)n_tok);
-        le = launch_overlapped(moe_combine_kernel, grid, dim3(256), st, p);
-        note_launch();
-        if (le != cudaSuccess) {
-            note_cuda_error(le);
-            (void)cudaGetLastError();
-            return KRK_CUDA_ELAUNCH;
-        }
-        return check_launch();
+        return launch_combine(p, st);
     }
     if (!routed) {
         const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);
@@ -624,12 +915,7 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
         const int rc = check_launch();
         if (rc != KRK_CUDA_OK) return rc;
     }
-    {
-        dim3 grid((unsigned)((bank->n_embd + 255) / 256), (unsigned)n_tok);
-        moe_combine_kernel<<<grid, 256, 0, st>>>(p);
-        note_launch();
-        return check_launch();
-    }
+    return launch_combine(p, st);
 }
 
 } // namespace krk_cuda
