@@ -144,8 +144,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes, uint32_t elected) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n"
+                 ::"r"(bar), "r"(bytes), "r"(elected) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -173,9 +174,11 @@ __device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volati
     if (*gave_up) return;
     wait_slow(bar, parity, gave_up, status);
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+// Issued by the elected lane of a converged warp (see umma_f16_ts_step: operands in uniform registers).
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar, uint32_t elected) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+                 " @q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y, uint32_t src) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
@@ -876,65 +879,68 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         // the staging buffers must outlive the stores that read them
         if (KIND == kDense && et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp == kXWarp) {
-        // ===== TMA producer of X tiles =====
-        if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            int sb = 0;
-            uint32_t pb = 0;
-            while (iter.next(p, it)) {
-                const int boxes = (tile_tokens<KIND>(p, it) + kGroupBox - 1) / kGroupBox;
-                for (int ks = ks0; ks < ks1; ks++) {
-                    wait_phase(smem_u32(&sm->b_empty[sb]), pb ^ 1, gave_up, p.status);
-                    const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem + (size_t)sb * b_bytes);
-                    if (KIND == kDense) {
-                        mbar_arrive_expect_tx(bar, (uint32_t)b_bytes);
-                        tma_load_2d(dst, &x_map, ks * kBK, it.x_row, bar);
-                    } else {   // only the boxes that hold tokens of the group
-                        mbar_arrive_expect_tx(bar, (uint32_t)(boxes * kGroupBox * 128));
-                        for (int b = 0; b < boxes; b++) tma_load_2d(dst + b * kGroupBox * 128, &x_map, ks * kBK, it.x_row + b * kGroupBox, bar);
-                    }
-                    if (++sb == p.n_b) {
-                        sb = 0;
-                        pb ^= 1;
-                    }
+        // ===== TMA producer of X tiles: like the MMA issuer a whole warp, one elected lane issues (from a one-lane branch
+        // a copy took some 250 clocks to issue, which bound the formats staged as eight boxes) =====
+        const uint32_t elected = elect_one();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        iter.n = __shfl_sync(0xFFFFFFFFu, iter.n, 0);
+        int sb = 0;
+        uint32_t pb = 0;
+        while (iter.next(p, it)) {
+            const int boxes = __shfl_sync(0xFFFFFFFFu, (tile_tokens<KIND>(p, it) + kGroupBox - 1) / kGroupBox, 0);
+            const int x_row = __shfl_sync(0xFFFFFFFFu, it.x_row, 0);
+            for (int ks = ks0; ks < ks1; ks++) {
+                wait_phase(smem_u32(&sm->b_empty[sb]), pb ^ 1, gave_up, p.status);
+                const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem) + (uint32_t)(sb * b_bytes);
+                if (KIND == kDense) {
+                    mbar_arrive_expect_tx(bar, (uint32_t)b_bytes, elected);
+                    tma_load_2d(dst, &x_map, ks * kBK, x_row, bar, elected);
+                } else {   // only the boxes that hold tokens of the group
+                    mbar_arrive_expect_tx(bar, (uint32_t)(boxes * kGroupBox * 128), elected);
+                    for (int b = 0; b < boxes; b++) tma_load_2d(dst + b * kGroupBox * 128, &x_map, ks * kBK, x_row + b * kGroupBox, bar, elected);
+                }
+                if (++sb == p.n_b) {
+                    sb = 0;
+                    pb ^= 1;
                 }
             }
         }
     } else if (warp == kRawWarp) {
         // ===== TMA producer of raw block columns =====
-        if (lane == 0) {
-            constexpr int kHalves = KIND == kGateUp ? 2 : 1;   // matrices in a weight tile
-            int sr = 0;
-            uint32_t pr = 0;
-            while (iter.next(p, it)) {
-                constexpr int kPer = Raw<WT>::kSteps;   // K steps per stage
-                for (int blk = ks0 / kPer; blk < ks1 / kPer; blk++) {
-                    wait_phase(smem_u32(&sm->raw_empty[sr]), pr ^ 1, gave_up, p.status);
-                    const uint32_t bar = smem_u32(&sm->raw_full[sr]);
-                    const uint32_t stage = smem_u32(raw_ring + (size_t)sr * kStageBytes);
-                    mbar_arrive_expect_tx(bar, (uint32_t)kStageBytes);
-                    if constexpr (row_phased(WT)) {
-                        constexpr int kBoxRows = kTileN / kPhases / kHalves;
+        constexpr int kHalves = KIND == kGateUp ? 2 : 1;   // matrices in a weight tile
+        constexpr int kPer = Raw<WT>::kSteps;              // K steps per stage
+        const uint32_t elected = elect_one();
+        iter.n = __shfl_sync(0xFFFFFFFFu, iter.n, 0);
+        int sr = 0;
+        uint32_t pr = 0;
+        while (iter.next(p, it)) {
+            const int w_row = __shfl_sync(0xFFFFFFFFu, it.w_row, 0);
+            for (int blk = ks0 / kPer; blk < ks1 / kPer; blk++) {
+                wait_phase(smem_u32(&sm->raw_empty[sr]), pr ^ 1, gave_up, p.status);
+                const uint32_t bar = smem_u32(&sm->raw_full[sr]);
+                const uint32_t stage = smem_u32(raw_ring) + (uint32_t)(sr * kStageBytes);
+                mbar_arrive_expect_tx(bar, (uint32_t)kStageBytes, elected);
+                if constexpr (row_phased(WT)) {
+                    constexpr int kBoxRows = kTileN / kPhases / kHalves;
 #pragma unroll
-                        for (int c = 0; c < kPhases; c++) {
-                            // map c starts (c * row_bytes) % 16 bytes before row c; the block's granules from there
-                            const int x0 = ((int)(((size_t)c * p.row_bytes) & 15) + blk * block_bytes(WT)) & ~15;
-                            // a matrix of fewer than eight rows has no row c: read outside the map, which fills zeros
-                            const int y0 = (KIND != kDense || c < p.n_out) ? it.w_row / kPhases : (1 << 24);
-#pragma unroll
-                            for (int hf = 0; hf < kHalves; hf++)
-                                tma_load_2d(stage + (hf * (kTileN / 2) + c * kBoxRows) * kSeg, &w_maps.m[hf * kPhases + c], x0, y0, bar);
-                        }
-                    } else {
-                        const int x0 = WT == KRK_CUDA_Q8_0 ? 136 * blk - 8 * (blk & 1) : blk * kSeg;   // a multiple of 16
+                    for (int c = 0; c < kPhases; c++) {
+                        // map c starts (c * row_bytes) % 16 bytes before row c; the block's granules from there
+                        const int x0 = (((c * p.row_bytes) & 15) + blk * block_bytes(WT)) & ~15;
+                        // a matrix of fewer than eight rows has no row c: read outside the map, which fills zeros
+                        const int y0 = (KIND != kDense || c < p.n_out) ? w_row / kPhases : (1 << 24);
 #pragma unroll
                         for (int hf = 0; hf < kHalves; hf++)
-                            tma_load_2d(stage + hf * (kTileN / 2) * kSeg, &w_maps.m[hf], x0, it.w_row, bar);
+                            tma_load_2d(stage + (hf * (kTileN / 2) + c * kBoxRows) * kSeg, &w_maps.m[hf * kPhases + c], x0, y0, bar, elected);
                     }
-                    if (++sr == p.n_raw) {
-                        sr = 0;
-                        pr ^= 1;
-                    }
+                } else {
+                    const int x0 = WT == KRK_CUDA_Q8_0 ? 136 * blk - 8 * (blk & 1) : blk * kSeg;   // a multiple of 16
+#pragma unroll
+                    for (int hf = 0; hf < kHalves; hf++)
+                        tma_load_2d(stage + hf * (kTileN / 2) * kSeg, &w_maps.m[hf], x0, w_row, bar, elected);
+                }
+                if (++sr == p.n_raw) {
+                    sr = 0;
+                    pr ^= 1;
                 }
             }
         }
