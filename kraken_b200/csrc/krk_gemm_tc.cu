@@ -117,7 +117,8 @@ struct GemmParams {
     int tile_m;          // tokens per tile: multiple of 16, <= 256
     int n_tiles_n, n_tiles_m;
     int row_bytes;
-    int n_b, n_raw;      // ring depths
+    int xk;              // K steps per X stage: 4, 2 or 1
+    int n_b, n_raw;      // ring depths (stages)
     int raw_off, y_off, bar_off;   // where the raw ring, the read-out buffers and the barriers start (the X ring starts at 0)
     int split;           // CTAs per cluster, each with a piece of K (1: no cluster)
     int y_tma;           // 1: tiles leave through shared memory and TMA stores (y 16-byte aligned, n_out % 4 == 0)
@@ -691,7 +692,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     uint8_t *raw_ring = smem + p.raw_off;
     float *ystage = reinterpret_cast<float *>(smem + p.y_off);   // [2][kYChunk][kTileN]: accumulator read-out on its way to Y
     GemmBars *sm = reinterpret_cast<GemmBars *>(smem + p.bar_off);
-    const int b_bytes = p.tile_m * 128;                          // an X tile: [tokens][64 f16], 128-byte swizzle
+    const int b_bytes = p.tile_m * 128;                          // X of a K step: [tokens][64 f16], 128-byte swizzle
+    const int b_stage = b_bytes * p.xk;
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);   // warp-uniform to the compiler too
     volatile int *gave_up = &sm->gave_up;
@@ -889,15 +891,18 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         while (iter.next(p, it)) {
             const int boxes = __shfl_sync(0xFFFFFFFFu, (tile_tokens<KIND>(p, it) + kGroupBox - 1) / kGroupBox, 0);
             const int x_row = __shfl_sync(0xFFFFFFFFu, it.x_row, 0);
-            for (int ks = ks0; ks < ks1; ks++) {
+            for (int ks = ks0; ks < ks1; ks += p.xk) {
                 wait_phase(smem_u32(&sm->b_empty[sb]), pb ^ 1, gave_up, p.status);
-                const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem) + (uint32_t)(sb * b_bytes);
-                if (KIND == kDense) {
-                    mbar_arrive_expect_tx(bar, (uint32_t)b_bytes, elected);
-                    tma_load_2d(dst, &x_map, ks * kBK, x_row, bar, elected);
-                } else {   // only the boxes that hold tokens of the group
-                    mbar_arrive_expect_tx(bar, (uint32_t)(boxes * kGroupBox * 128), elected);
-                    for (int b = 0; b < boxes; b++) tma_load_2d(dst + b * kGroupBox * 128, &x_map, ks * kBK, x_row + b * kGroupBox, bar, elected);
+                const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem) + (uint32_t)(sb * b_stage);
+                // (dense: one box per K step; else only the boxes that hold tokens of the group)
+                mbar_arrive_expect_tx(bar, (uint32_t)(p.xk * (KIND == kDense ? b_bytes : boxes * kGroupBox * 128)), elected);
+                for (int j = 0; j < p.xk; j++) {
+                    if (KIND == kDense) {
+                        tma_load_2d(dst + j * b_bytes, &x_map, (ks + j) * kBK, x_row, bar, elected);
+                    } else {
+                        for (int b = 0; b < boxes; b++)
+                            tma_load_2d(dst + j * b_bytes + b * kGroupBox * 128, &x_map, (ks + j) * kBK, x_row + b * kGroupBox, bar, elected);
+                    }
                 }
                 if (++sb == p.n_b) {
                     sb = 0;
@@ -955,23 +960,42 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             const uint32_t idesc = instr_desc(kTileN, __shfl_sync(0xFFFFFFFFu, tile_tokens<KIND>(p, it), 0));
             wait_phase(smem_u32(&sm->d_empty[da]), pd ^ 1, gave_up, p.status);   // the epilogue has drained the accumulator
             tc_fence_after();
-            for (int ks = ks0; ks < ks1; ks++) {   // an even number: a stage of decoded A holds two K steps
-                wait_phase(smem_u32(&sm->b_full[sb]), pb, gave_up, p.status);
-                if ((ks & 1) == 0) wait_phase(smem_u32(&sm->a_full[sa]), pa, gave_up, p.status);
-                tc_fence_after();
-                umma_f16_ts_step(tmem + 128 * da, tmem + kTmemA + 64 * sa + 32 * (ks & 1), smem_desc(smem_u32(smem) + (uint32_t)(sb * b_bytes)),
-                                 idesc, ks == ks0 ? 1u : 0u, elected);
-                umma_commit(smem_u32(&sm->b_empty[sb]), elected);   // a stage is free once the MMAs that read it are done
-                if (ks & 1) {
-                    umma_commit(smem_u32(&sm->a_empty[sa]), elected);
-                    if (++sa == kAStages) {
-                        sa = 0;
-                        pa ^= 1;
+            // A super-block at a time. This loop shares its scheduler with decode warps and is the critical path of narrow
+            // tiles: one X stage and one A stage are waited for and committed per several MMAs, both waits in flight
+            // together.
+            const int xmask = p.xk - 1;
+            for (int ks = ks0; ks < ks1; ks += 4) {
+                uint64_t bdesc = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const bool new_b = (j & xmask) == 0, new_a = (j & 1) == 0;
+                    const uint32_t b_bar = smem_u32(&sm->b_full[sb]), a_bar = smem_u32(&sm->a_full[sa]);
+                    if (new_b) {
+                        const bool okb = mbar_try_wait(b_bar, pb), oka = !new_a || mbar_try_wait(a_bar, pa);
+                        if (!okb) wait_phase(b_bar, pb, gave_up, p.status);
+                        if (!oka) wait_phase(a_bar, pa, gave_up, p.status);
+                        tc_fence_after();
+                        bdesc = smem_desc(smem_u32(smem) + (uint32_t)(sb * b_stage));
+                    } else if (new_a) {
+                        wait_phase(a_bar, pa, gave_up, p.status);
+                        tc_fence_after();
                     }
-                }
-                if (++sb == p.n_b) {
-                    sb = 0;
-                    pb ^= 1;
+                    umma_f16_ts_step(tmem + 128 * da, tmem + kTmemA + 64 * sa + 32 * (j & 1), bdesc, idesc, (j == 0 && ks == ks0) ? 1u : 0u, elected);
+                    bdesc += (uint32_t)b_bytes >> 4;
+                    if (((j + 1) & xmask) == 0) {
+                        umma_commit(smem_u32(&sm->b_empty[sb]), elected);   // a stage is free once the MMAs that read it are done
+                        if (++sb == p.n_b) {
+                            sb = 0;
+                            pb ^= 1;
+                        }
+                    }
+                    if (j & 1) {
+                        umma_commit(smem_u32(&sm->a_empty[sa]), elected);
+                        if (++sa == kAStages) {
+                            sa = 0;
+                            pa ^= 1;
+                        }
+                    }
                 }
             }
             umma_commit(smem_u32(&sm->d_full[da]), elected);
@@ -1082,14 +1106,16 @@ bool encode_w_maps(CUtensorMap *maps, const uint8_t *w, int64_t n_out, int row_b
 // both grow in turn while they fit.
 template <int WT>
 size_t layout(GemmParams &p) {
-    const int stage = kTileN * raw_seg(WT), steps = Raw<WT>::kSteps, xb = p.tile_m * 128;
+    const int stage = kTileN * raw_seg(WT), steps = Raw<WT>::kSteps;
+    p.xk = p.tile_m <= 64 ? 4 : p.tile_m <= 128 ? 2 : 1;   // X stages of at most 32 KB
+    const int xb = p.tile_m * 128 * p.xk;
     const int y_bytes = 2 * kYChunk * kTileN * (int)sizeof(float);
     const int room = kSmemMax - 1024 - y_bytes - (int)sizeof(GemmBars);
-    p.n_b = kMinB;
+    p.n_b = kMinB / p.xk > 2 ? kMinB / p.xk : 2;
     p.n_raw = kMinRaw;
     for (;;) {
         const int left = room - p.n_b * xb - p.n_raw * stage;
-        const bool want_b = p.n_b < kMaxB && p.n_b < steps * p.n_raw;
+        const bool want_b = p.n_b < kMaxB && p.n_b * p.xk < steps * p.n_raw;
         if (want_b && left >= xb) p.n_b++;
         else if (p.n_raw < kMaxRaw && left >= stage) p.n_raw++;
         else if (p.n_b < kMaxB && left >= xb) p.n_b++;
