@@ -1,4 +1,5 @@
-"""Builds kraken_b200/libkrk_cuda.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds kraken_b200/libkrk_cuda.so (the C-ABI library) in-tree with nvcc for sm_100a, and the CPython extension
+over it (_fastcall) that kraken_b200.capi calls.
 
     python -m kraken_b200.build [--force] [--verbose]
 
@@ -19,6 +20,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libkrk_cuda.so")
+FASTCALL_SRC = os.path.join(CSRC, "py", "krk_fastcall.cpp")
+FASTCALL = os.path.join(HERE, "_fastcall.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
@@ -48,6 +51,30 @@ def _digest(path: str, flags) -> str:
             if f.endswith((".cuh", ".h", ".hpp")):
                 h.update(open(os.path.join(dep_dir, f), "rb").read())
     return h.hexdigest()[:16]
+
+
+def build_fastcall(force: bool = False) -> str:
+    """The CPython extension: torch tensors in, C ABI calls out. Needs the library's file only at link time."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    inc = cpp_extension.include_paths() + [sysconfig.get_path("include"), os.path.join(ROOT, "include"), "/usr/local/cuda/include"]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    stamp = os.path.join(OBJ, f"fastcall.{_digest(FASTCALL_SRC, flags + [torch.__version__, sys.version])}.stamp")
+    if not force and os.path.exists(stamp) and os.path.exists(FASTCALL):
+        return FASTCALL
+    libdirs = cpp_extension.library_paths()
+    cmd = (["g++"] + flags + [a for i in inc for a in ("-I", i)] + [FASTCALL_SRC, "-o", FASTCALL, "-L", HERE, "-l:libkrk_cuda.so", "-Wl,-rpath,$ORIGIN"] +
+           [a for d in libdirs for a in ("-L", d)] + ["-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling krk_fastcall.cpp failed:\n{r.stdout}\n{r.stderr}")
+    for f in os.listdir(OBJ):
+        if f.startswith("fastcall."):
+            os.remove(os.path.join(OBJ, f))
+    open(stamp, "w").close()
+    return FASTCALL
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -90,6 +117,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"linking libkrk_cuda.so failed:\n{r.stdout}\n{r.stderr}")
+    build_fastcall(force)
     return LIB
 
 

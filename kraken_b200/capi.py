@@ -1,14 +1,17 @@
-"""ctypes binding of libkrk_cuda.so: one Python function per entry of include/krk_cuda.h.
+"""Python binding of libkrk_cuda.so: one function per entry of include/krk_cuda.h.
 
 This is glue, not a second implementation: every function checks nothing and computes
 nothing itself, it passes device pointers (``tensor.data_ptr()``) and sizes to the C ABI
 and raises ``KrkCudaError`` on a non-zero status. torch supplies device memory and streams.
-If the library has not been built, importing this module raises: there is no fallback.
+The calls of a decode loop go through the CPython extension ``_fastcall`` (csrc/py/), the
+others through ctypes. If either has not been built, importing this module raises: there is no fallback.
 """
 from __future__ import annotations
 
 import ctypes as C
 import os
+
+import torch   # before the extension, which links its libraries
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libkrk_cuda.so")
@@ -32,6 +35,7 @@ if not os.path.exists(LIB_PATH):
                       "(this package has no fallback path)")
 
 lib = C.CDLL(LIB_PATH)
+from . import _fastcall as _fc   # noqa: E402
 
 _vp, _i64, _int, _sz = C.c_void_p, C.c_int64, C.c_int, C.c_size_t
 
@@ -149,9 +153,15 @@ def _check(rc: int, where: str) -> None:
         raise KrkCudaError(rc, where)
 
 
+def _raise(rc: int, where: str) -> None:
+    raise KrkCudaError(rc, where)
+
+
+_fc.set_raise(_raise)
+
+
 def _stream_ptr(stream=None):
     """cudaStream_t of a torch stream (None = torch's current stream)."""
-    import torch
     s = torch.cuda.current_stream() if stream is None else stream
     return C.c_void_p(s.cuda_stream)
 
@@ -173,7 +183,6 @@ def gemm_k_ok(wt: int, k: int) -> bool:
 # ---- device-pointer entries ----------------------------------------------------------------
 
 def dequant_rows(w, wt: int, n_rows: int, n_in: int, stream=None):
-    import torch
     out = torch.empty((n_rows, n_in), dtype=torch.float32, device=w.device)
     _check(lib.krk_cuda_dequant_rows(_ptr(out), _ptr(w), wt, n_rows, n_in, _stream_ptr(stream)), "dequant_rows")
     return out
@@ -181,31 +190,12 @@ def dequant_rows(w, wt: int, n_rows: int, n_in: int, stream=None):
 
 def gemv(x, w, wt: int, n_out: int, n_in: int, out=None, accumulate: bool = False, stream=None):
     """y[rows][n_out] (+)= x[rows][n_in] . W^T; x is f32 [rows, n_in] or [n_in]."""
-    import torch
-    rows = 1 if x.dim() == 1 else x.shape[0]
-    if out is None:
-        if accumulate:
-            raise ValueError("accumulate needs an existing output")
-        out = torch.empty((rows, n_out), dtype=torch.float32, device=x.device)
-    _check(lib.krk_cuda_gemv(_ptr(out), _ptr(x), _ptr(w), wt, n_out, n_in, rows, int(accumulate),
-                             _stream_ptr(stream)), "gemv")
-    return out
+    return _fc.gemv(x, w, wt, n_out, n_in, out, accumulate, stream)
 
 
 def gemv_group(xs, ws, wts, n_outs, n_in: int, outs=None, fuse_silu_pair: bool = False, stream=None):
     """One launch for up to 16 single-row GEMVs. xs/ws/outs are lists of tensors."""
-    import torch
-    n = len(ws)
-    if outs is None:
-        outs = [torch.empty((n_outs[m],), dtype=torch.float32, device=ws[m].device) for m in range(n)]
-    ya = (_vp * n)(*[t.data_ptr() for t in outs])
-    xa = (_vp * n)(*[t.data_ptr() for t in xs])
-    wa = (_vp * n)(*[t.data_ptr() for t in ws])
-    ta = (_int * n)(*wts)
-    na = (_i64 * n)(*n_outs)
-    _check(lib.krk_cuda_gemv_group(ya, xa, wa, ta, na, n_in, n, int(fuse_silu_pair), _stream_ptr(stream)),
-           "gemv_group")
-    return outs
+    return _fc.gemv_group(xs, ws, wts, n_outs, n_in, outs, fuse_silu_pair, stream)
 
 
 def gemm_workspace_bytes(x_dtype: int, n_out: int, n_in: int, rows: int) -> int:
@@ -214,22 +204,11 @@ def gemm_workspace_bytes(x_dtype: int, n_out: int, n_in: int, rows: int) -> int:
 
 def gemm(x, w, wt: int, n_out: int, n_in: int, out=None, workspace=None, stream=None):
     """Prefill GEMM: x is f16 or f32 [rows, n_in]; returns f32 [rows, n_out]."""
-    import torch
-    rows = x.shape[0]
-    x_dtype = X_F16 if x.dtype == torch.float16 else X_F32
-    need = gemm_workspace_bytes(x_dtype, n_out, n_in, rows)
-    if workspace is None and need:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-    if out is None:
-        out = torch.empty((rows, n_out), dtype=torch.float32, device=x.device)
-    _check(lib.krk_cuda_gemm(_ptr(out), _ptr(x), x_dtype, _ptr(w), wt, n_out, n_in, rows, _ptr(workspace),
-                             workspace.numel() if workspace is not None else 0, _stream_ptr(stream)), "gemm")
-    return out
+    return _fc.gemm(x, w, wt, n_out, n_in, out, workspace, stream)
 
 
 def gemm_f32_static(x, w, wt: int, n_out: int, n_in: int, out=None, stream=None):
     """krk_cuda_gemm_f32_static: f32 x [rows, n_in] -> f32 [rows, n_out], scratch inside the library."""
-    import torch
     rows = x.shape[0]
     if out is None:
         out = torch.empty((rows, n_out), dtype=torch.float32, device=x.device)
@@ -243,7 +222,6 @@ def gemm_f32_static_status() -> int:
 
 
 def route(logits, k: int, stream=None):
-    import torch
     n_tok, n_expert = logits.shape
     ids = torch.empty((n_tok, k), dtype=torch.int32, device=logits.device)
     wts = torch.empty((n_tok, k), dtype=torch.float32, device=logits.device)
@@ -252,7 +230,6 @@ def route(logits, k: int, stream=None):
 
 
 def router_softmax(logits, stream=None):
-    import torch
     probs = torch.empty_like(logits)
     _check(lib.krk_cuda_router_softmax(_ptr(probs), _ptr(logits), logits.shape[0], logits.shape[1], _stream_ptr(stream)),
            "router_softmax")
@@ -260,7 +237,6 @@ def router_softmax(logits, stream=None):
 
 
 def router_topk(probs, k: int, normalize: bool = True, scale: float = 1.0, stream=None):
-    import torch
     n_rows, n_expert = probs.shape
     ids = torch.empty((n_rows, k), dtype=torch.int32, device=probs.device)
     wts = torch.empty((n_rows, k), dtype=torch.float32, device=probs.device)
@@ -271,7 +247,6 @@ def router_topk(probs, k: int, normalize: bool = True, scale: float = 1.0, strea
 
 def moe_plan_build(ids, wts, n_expert: int, stream=None):
     """Expert-major plan of a layer: (off int32 [n_expert + 1], rows int32 [n * k], wt f32 [n * k])."""
-    import torch
     n_rows, k = ids.shape
     off = torch.empty(n_expert + 1, dtype=torch.int32, device=ids.device)
     rows = torch.full((n_rows * k,), -1, dtype=torch.int32, device=ids.device)
@@ -317,40 +292,16 @@ def make_bank(gate, up, down, wt_gate_up: int, wt_down: int, n_local: int, exper
 
 
 def moe_ffn(x, ids, wts, bank: ExpertBank, out=None, workspace=None, stream=None):
-    import torch
-    n_tok, k = ids.shape
-    need = lib.krk_cuda_moe_workspace_bytes(C.byref(bank), k, n_tok)
-    if workspace is None:
-        workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    if out is None:
-        out = torch.empty((n_tok, bank.n_embd), dtype=torch.float32, device=x.device)
-    _check(lib.krk_cuda_moe_ffn(_ptr(out), _ptr(x), _ptr(ids), _ptr(wts), C.byref(bank), k, n_tok, _ptr(workspace),
-                                workspace.numel(), _stream_ptr(stream)), "moe_ffn")
-    return out
+    return _fc.moe_ffn(x, ids, wts, bank, out, workspace, stream)
 
 
 def moe_ffn_routed(x, logits, k: int, bank: ExpertBank, out=None, workspace=None, stream=None):
     """Routing + routed-expert FFN in one call. Returns (y, ids, wts); ids / wts are what route() gives."""
-    import torch
-    n_tok, n_expert = logits.shape
-    ids = torch.empty((n_tok, k), dtype=torch.int32, device=x.device)
-    wts = torch.empty((n_tok, k), dtype=torch.float32, device=x.device)
-    need = lib.krk_cuda_moe_workspace_bytes(C.byref(bank), k, n_tok)
-    if workspace is None:
-        workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
-    if out is None:
-        out = torch.empty((n_tok, bank.n_embd), dtype=torch.float32, device=x.device)
-    _check(lib.krk_cuda_moe_ffn_routed(_ptr(out), _ptr(x), _ptr(logits), n_expert, _ptr(ids), _ptr(wts), C.byref(bank), k,
-                                       n_tok, _ptr(workspace), workspace.numel(), _stream_ptr(stream)), "moe_ffn_routed")
-    return out, ids, wts
+    return _fc.moe_ffn_routed(x, logits, k, bank, out, workspace, stream)
 
 
 def silu_mul(gate, up, out=None, stream=None):
-    import torch
-    if out is None:
-        out = torch.empty_like(gate)
-    _check(lib.krk_cuda_silu_mul(_ptr(out), _ptr(gate), _ptr(up), gate.numel(), _stream_ptr(stream)), "silu_mul")
-    return out
+    return _fc.silu_mul(gate, up, out, stream)
 
 
 def gather_rows(dst, src, rows, stream=None):
@@ -367,7 +318,6 @@ def scatter_axpy_rows(dst, src, rows, alpha, stream=None):
 
 
 def sum_parts(parts, out=None, stream=None):
-    import torch
     n_parts = parts.shape[0]
     n = parts[0].numel()
     if out is None:
@@ -393,29 +343,13 @@ def wait_flags(flags, n_peers: int, epoch: int, stream=None):
 
 def embed(table, wt: int, n_vocab: int, n_embd: int, tokens, out=None, stream=None):
     """Rows of a quantized embedding table by token id (device int32 tensor) as f32; bad ids give zero rows."""
-    import torch
-    n_tok = tokens.numel()
-    if out is None:
-        out = torch.empty((n_tok, n_embd), dtype=torch.float32, device=table.device)
-    _check(lib.krk_cuda_embed(_ptr(out), _ptr(table), wt, n_vocab, n_embd, _ptr(tokens), n_tok, _stream_ptr(stream)), "embed")
-    return out
+    return _fc.embed(table, wt, n_vocab, n_embd, tokens, out, stream)
 
 
 def logits_topk(logits, k: int, pen_mask=None, rep_pen: float = 1.0, softcap: float = 0.0, temp: float = 1.0,
                 want_mass: bool = True, workspace=None, stream=None):
     """Device top-k of one f32 logits row: (ids int32 [k], vals f32 [k], mass f32 [1] or None)."""
-    import torch
-    n = logits.numel()
-    ids = torch.empty(k, dtype=torch.int32, device=logits.device)
-    vals = torch.empty(k, dtype=torch.float32, device=logits.device)
-    mass = torch.empty(1, dtype=torch.float32, device=logits.device) if want_mass else None
-    need = lib.krk_cuda_logits_topk_workspace_bytes(n, k)
-    if workspace is None:
-        workspace = torch.empty(max(need, 16), dtype=torch.uint8, device=logits.device)
-    _check(lib.krk_cuda_logits_topk(_ptr(logits), n, k, _ptr(pen_mask) if pen_mask is not None else None, rep_pen, softcap,
-                                    temp, _ptr(ids), _ptr(vals), _ptr(mass) if mass is not None else None, _ptr(workspace),
-                                    workspace.numel(), _stream_ptr(stream)), "logits_topk")
-    return ids, vals, mass
+    return _fc.logits_topk(logits, k, pen_mask, rep_pen, softcap, temp, want_mass, workspace, stream)
 
 
 def allgather_sum(gather_peer_ptrs, flag_peer_ptrs, my_rank: int, slot_stride: int, part, out, stream=None):
@@ -448,7 +382,6 @@ class PeerBuffer:
 
     def tensor(self, shape, dtype):
         """The buffer as a tensor of the current device (own buffers only)."""
-        import torch
         if not self.owned:
             raise ValueError("a mapped peer buffer is only addressed by kernels of this library")
         itemsize = torch.empty(0, dtype=dtype).element_size()
@@ -531,10 +464,10 @@ class Backend:
         lib.krk_cuda_backend_release(self.h, p)
 
     def upload(self, dst: int, host_ptr: int, nbytes: int, off: int = 0) -> None:
-        lib.krk_cuda_backend_upload(self.h, dst, host_ptr, nbytes, off)
+        _fc.backend_upload(self.h, dst, host_ptr, nbytes, off)
 
     def download(self, host_ptr: int, src: int, nbytes: int, off: int = 0) -> None:
-        lib.krk_cuda_backend_download(self.h, host_ptr, src, nbytes, off)
+        _fc.backend_download(self.h, host_ptr, src, nbytes, off)
 
     def router_softmax(self, probs: int, logits: int, n_rows: int, n_expert: int) -> None:
         lib.krk_cuda_backend_router_softmax(self.h, probs, logits, n_rows, n_expert)
@@ -556,25 +489,15 @@ class Backend:
         return bool(lib.krk_cuda_backend_gemm_k_ok(self.h, wt, k))
 
     def gemm(self, out: int, x: int, w: int, wt: int, n_out: int, n_in: int, rows: int) -> None:
-        lib.krk_cuda_backend_gemm(self.h, out, x, w, wt, n_out, n_in, rows)
+        _fc.backend_gemm(self.h, out, x, w, wt, n_out, n_in, rows)
 
     def gemm_accumulate(self, dst: int, x: int, w: int, wt: int, n_out: int, n_in: int, rows: int) -> bool:
-        return bool(lib.krk_cuda_backend_gemm_accumulate(self.h, dst, x, w, wt, n_out, n_in, rows))
+        return _fc.backend_gemm_accumulate(self.h, dst, x, w, wt, n_out, n_in, rows)
 
     def gemm_group(self, outs, x: int, ws, wt: int, n_outs, n_in: int, rows: int = 1, silu: bool = False,
                    wts=None, xs=None):
         """Backend::gemm_group; wts / xs are its optional per-matrix weight types and activations."""
-        n = len(ws)
-        fused = _int(0)
-        if wts is None and xs is None:
-            ran = lib.krk_cuda_backend_gemm_group(self.h, (_vp * n)(*outs), x, (_vp * n)(*ws), wt, (_i64 * n)(*n_outs),
-                                                  n_in, n, rows, int(silu), C.byref(fused))
-        else:
-            ran = lib.krk_cuda_backend_gemm_group_ex(self.h, (_vp * n)(*outs), x, (_vp * n)(*ws), wt, (_i64 * n)(*n_outs),
-                                                     n_in, n, rows, int(silu), C.byref(fused),
-                                                     (_int * n)(*wts) if wts is not None else None,
-                                                     (_vp * n)(*xs) if xs is not None else None)
-        return bool(ran), bool(fused.value)
+        return _fc.backend_gemm_group(self.h, outs, x, ws, wt, n_outs, n_in, rows, silu, wts, xs)
 
 
 class Gguf:
