@@ -185,8 +185,8 @@ int krk_cuda_gemm(void *y_f32, const void *x, int x_dtype, const void *w, int wt
     if (rc != KRK_CUDA_OK) return rc;
     if (n_in % 256 != 0 || !gemm_tc_takes(wt)) {
         // The fallback rung (the place of gemm_simt_kernel, src/hip/kernels/gemm.hpp:1013-1134): 32-value
-        // block formats whose K is a whole number of blocks but not of 256. Correct, not fast: the
-        // shape-agnostic GEMV over batches of KRK_CUDA_MAX_ROWS activation rows. f32 activations only.
+        // block formats whose K is a whole number of blocks but not of 256, at f32 precision: the
+        // decode GEMV over batches of KRK_CUDA_MAX_ROWS activation rows. f32 activations only.
         if (x_dtype != KRK_CUDA_X_F32) return KRK_CUDA_ESHAPE;
         if (n_out == 0 || rows == 0) return KRK_CUDA_OK;
         if (!device_state()) return KRK_CUDA_EDEVICE;
@@ -198,8 +198,9 @@ int krk_cuda_gemm(void *y_f32, const void *x, int x_dtype, const void *w, int wt
             m.y = static_cast<float *>(y_f32) + r0 * n_out;
             m.n_out = n_out;
             m.wt = wt;
-            const int grc = launch_gemv_generic(&m, 1, n_in, (int)nr, 0, 0, static_cast<cudaStream_t>(stream));
-            if (grc != KRK_CUDA_OK) return grc;
+            int grc = launch_gemv_stream(&m, 1, n_in, (int)nr, 0, 0, static_cast<cudaStream_t>(stream));
+            if (grc == 0) grc = launch_gemv_generic(&m, 1, n_in, (int)nr, 0, 0, static_cast<cudaStream_t>(stream));
+            if (grc < 0) return grc;
         }
         return KRK_CUDA_OK;
     }

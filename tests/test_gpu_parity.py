@@ -566,3 +566,19 @@ def test_backend_gemm_fallback_rung_k_not_multiple_of_256(cuda, oracle, wt, n_in
     for p in (d_w, d_x, d_y):
         be.release(p)
     be.close()
+
+
+@pytest.mark.parametrize("wt", [synth.Q8_0, synth.Q4_0, synth.Q5_0, synth.Q5_1, synth.IQ4_NL])
+def test_gemv_stream_whole_blocks_not_super_blocks(cuda, oracle, wt):
+    """K whole 32-value blocks but not a multiple of 256: rows start at every even offset, the last unit of a row is
+    short (one block up to all but one), few units are stacked, and one stage ends inside a unit."""
+    for i, (n_out, n_in, rows) in enumerate(((50, 288, 1), (333, 416, 2), (129, 1056, 1), (1001, 2080, 1), (77, 4128, 3), (40, 5600, 4),
+                                             (100, 2272, 8), (17, 480, 5), (4099, 2976, 1), (64, 384, 1), (33, 1152, 6))):
+        run_gemv(cuda, oracle, wt, n_out, n_in, rows, SEED + 300 + 20 * wt + i, random_payload=i % 2 == 1, expect_stream=True)
+    run_gemv(cuda, oracle, wt, 300, 2080, 1, SEED + 320, accumulate=True, expect_stream=True)
+    x = synth.activations(1, 1056, SEED + 321)
+    ws = [synth.weights(wt, n, 1056, SEED + 321, stream=500 + i) for i, n in enumerate((200, 200))]
+    y, _ = cuda.gemv_group([dev(x)] * 2, [dev(w) for w in ws], [wt] * 2, [200, 200], 1056, fuse_silu_pair=True)
+    g, u = (oracle.gemm(x, w, wt, 200, 1056) for w in ws)
+    want = g.astype(np.float64) / (1.0 + np.exp(-g.astype(np.float64))) * u
+    assert np.abs(y.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
