@@ -39,6 +39,7 @@
 #include <cfloat>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "krk_common.cuh"
@@ -51,15 +52,19 @@ namespace stream {
 
 constexpr int kConsumerWarps = 8;
 constexpr int kConsumerThreads = kConsumerWarps * 32;
-constexpr int kThreads = kConsumerThreads + 64;   // warp 0: producer, warps 1..8: consumers, warp 9: epilogue
-constexpr int kEpilogueWarp = kConsumerWarps + 1;
+// One or two groups of consumer warps per CTA. One or two activation rows: one group in half an SM. More rows: two
+// groups in a whole SM that share one prepared activation and take tiles in turn (one group per SM, all that its
+// registers allowed before the accumulators were folded, left the schedulers waiting half of the time).
+__host__ __device__ constexpr int consumer_groups(int ng) { return ng == 1 ? 1 : 2; }
+__host__ __device__ constexpr int cta_threads(int groups) { return groups * kConsumerThreads + 64; }   // warp 0: producer, then the consumers, then the epilogue
 // Tiles whose partial sums may wait for the epilogue warp (fewer when more activation rows make a slot larger).
-__host__ __device__ constexpr int red_slots(int ng) { return ng == 1 ? 4 : ng == 2 ? 2 : 1; }
+__host__ __device__ constexpr int red_slots(int ng) { return ng == 1 ? 4 : ng == 2 ? 2 : 1; }   // of each consumer group
 constexpr int kMaxRedSlots = 4;
 constexpr int kMaxStack = 4;      // 16-row tiles per stage at most
 constexpr int kTileRows = 16;                     // the M of the MMA
-constexpr int kMaxStages = 4;                    // measured: four stages in flight per CTA stream a large Q4_K matrix at 0.89 of the
-                                                  // copy bandwidth, five (all that fit) at 0.86, three at 0.86
+constexpr int kMaxStages = 8;                    // of a whole-SM CTA
+constexpr int kMaxHalfStages = 4;                // of a half-SM one. Measured: four stages in flight per CTA stream a large Q4_K matrix at
+                                                 // 0.89 of the copy bandwidth, five (all that fit) at 0.86, three at 0.86
 constexpr int kSmemLimit = 113 * 1024;           // two CTAs per SM (228 KB, 1 KB reserved per CTA)
 constexpr int kSmemWhole = 227 * 1024;
 constexpr int kPlanePad = 32;                     // bytes between limb planes beyond n_in: spreads the B-fragment loads over the banks
@@ -274,7 +279,8 @@ struct Smem {
     int pad[3];
     float gate[kMaxStack][NG][32];   // epilogue warp: the gate tile(s) of a gate/up pair, until the up tile arrives
     // per consumer warp, column group and row pair (g, g+8): {row g x even activation row, g x odd, g+8 x even, g+8 x odd}
-    float4 red[red_slots(NG)][kConsumerWarps][NG][8];
+    float4 red[consumer_groups(NG) * red_slots(NG)][kConsumerWarps][NG][8];
+    float scale[NG == 1 ? 1 : kConsumerWarps][2 * NG];   // two groups: each prepared half of the activation rows, these are the scales
 };
 
 __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / a * a; }
@@ -560,49 +566,99 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
 // A fragments of rows g and g+8, column g of the B fragment (limb g%3 of activation row g/3 of
 // the column group), and accumulator columns 2t, 2t+1.
 
-// Column groups that go through the MMAs. One or two groups carry two activation rows each in columns 0..5. The
+// Column groups that go through the MMAs (32-value block formats; the super-block formats multiply all NG, two rows of
+// four columns each). One or two groups carry two activation rows each in columns 0..5. The
 // form for five to eight rows has four groups of outputs but multiplies only three: rows 0..5 sit in columns 0..5
 // of groups 0..2 and rows 6 and 7 in the spare columns 6 and 7, limb mg of the row in group mg, so that 24 columns
 // carry 8 rows x 3 limbs with none to spare.
 template <int NG>
 constexpr int kMmaGroups = NG == 4 ? 3 : NG;
 
+// The 32-value block formats.
 template <int NG>
 struct Accum {
     float f[NG][4];   // [group][(row g | g+8) x (col 2t | 2t+1)], already times the block scale d
-    float m[NG][4];   // Q4_K: the same for dmin * sum(min_c * sum_X_c), columns = 4 limbs x 2 activation rows
 };
-
+// The super-block formats. A lane holds two neighbouring columns of every column group, and the columns are dealt so that
+// all it holds belongs to its own activation rows: a unit's integer sums, their limb weights and the minimum term then fold
+// into one number per weight row and activation row (a quarter of the registers of a sum per limb).
+//   Three and more rows: lane t looks after rows t and t + 4. Group 0 carries limbs 0 and 1 of row t in columns 2t and
+//   2t + 1, group 1 (five and more rows) the same of row t + 4, the last group limb 2 of both: 24 limb columns in
+//   three groups, and nothing is left to add between lanes at the end of a tile.
+//   One or two rows: one group, row 0 in columns 0..3 and row 1 in 4..7 (the fourth column of each unused).
+// The minimum term's chunk sums (four limbs) lie the same way: limbs 0, 1 then 2, 3 of row t, then of row t + 4; with one
+// or two rows the four limbs of a row in its four columns.
+template <int NG>
+constexpr int kFoldGroups = NG == 4 ? 3 : NG;
+template <int NG>
+constexpr int kFoldRows = NG == 4 ? 2 : 1;   // activation rows a lane looks after
+template <int NG>
+struct AccumFold {
+    float a[kFoldRows<NG>][2];   // [row t, t + 4][weight row g, g + 8]
+};
+// acc += d * (limb sums of a unit), dA and dB the scales of weight rows g and g + 8
+template <int NG>
+__device__ __forceinline__ void fold(AccumFold<NG> &acc, float dA, float dB, const int (&I)[NG][4], int t) {
+    if constexpr (NG == 1) {
+        const float w0 = t & 1 ? 1.0f : 65536.0f, w1 = t & 1 ? 0.0f : 256.0f;
+        acc.a[0][0] = fmaf(dA, fmaf(w0, (float)I[0][0], w1 * (float)I[0][1]), acc.a[0][0]);
+        acc.a[0][1] = fmaf(dB, fmaf(w0, (float)I[0][2], w1 * (float)I[0][3]), acc.a[0][1]);
+    } else {
+#pragma unroll
+        for (int h = 0; h < kFoldRows<NG>; h++) {
+            constexpr int L = kFoldGroups<NG> - 1;
+            acc.a[h][0] = fmaf(dA, fmaf(65536.0f, (float)I[h][0], fmaf(256.0f, (float)I[h][1], (float)I[L][h])), acc.a[h][0]);
+            acc.a[h][1] = fmaf(dB, fmaf(65536.0f, (float)I[h][2], fmaf(256.0f, (float)I[h][3], (float)I[L][2 + h])), acc.a[h][1]);
+        }
+    }
+}
+// acc -= dmin * (minimums times group mg of the chunk sums)
+template <int NG>
+__device__ __forceinline__ void fold_min(AccumFold<NG> &acc, float nA, float nB, const int (&c)[4], int mg, int t) {
+    const bool low = NG == 1 ? (t & 1) : (mg & 1);   // limbs 2 and 3 (weights 2^8, 1), else 0 and 1 (2^24, 2^16)
+    const float w0 = low ? -256.0f : -16777216.0f, w1 = low ? -1.0f : -65536.0f;
+    const int h = NG == 4 ? mg >> 1 : 0;
+    acc.a[h][0] = fmaf(nA, fmaf(w0, (float)c[0], w1 * (float)c[1]), acc.a[h][0]);
+    acc.a[h][1] = fmaf(nB, fmaf(w0, (float)c[2], w1 * (float)c[3]), acc.a[h][1]);
+}
 template <int NG>
 __device__ __forceinline__ void accum_zero(Accum<NG> &a) {
 #pragma unroll
     for (int i = 0; i < NG; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) a.f[i][j] = 0.0f;
+}
+template <int NG>
+__device__ __forceinline__ void accum_zero(AccumFold<NG> &a) {
 #pragma unroll
-    for (int i = 0; i < NG; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) a.m[i][j] = 0.0f;
+    for (int i = 0; i < kFoldRows<NG>; i++) a.a[i][0] = a.a[i][1] = 0.0f;
 }
 
 // Byte planes this lane reads its B fragments from, one per column group. A lane whose column
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
 // accumulator columns are never looked at, so what it multiplies does not matter.
-template <int NG>
+template <int NG, bool FOLD>
 __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int n_in, int n_sums, int rows, int g,
                                             const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         int r = 2 * mg + (g % 6) / 3, limb = g % 3;
-        if (NG == 4 && g >= 6) {   // the spare columns: limb mg of activation row 6 or 7 (group 3 multiplies nothing)
+        int rs = 2 * mg + g / 4, ls = g % 4;   // chunk sums
+        if (FOLD && NG == 1) {
+            r = g >> 2;
+            limb = min(g & 3, 2);
+        } else if (FOLD) {   // see AccumFold
+            const bool last = mg >= kFoldGroups<NG> - 1;
+            r = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
+            limb = last ? 2 : g & 1;
+            rs = (g >> 1) + 4 * (mg >> 1);
+            ls = 2 * (mg & 1) + (g & 1);
+        } else if (NG == 4 && g >= 6) {   // the spare columns: limb mg of activation row 6 or 7 (group 3 multiplies nothing)
             r = g;
             limb = mg % 3;
         }
-        r = min(r, rows - 1);
-        bp[mg] = planes + (size_t)(r * 3 + limb) * plane_stride(n_in);
-        // chunk sums: column c = limb c%4 of activation row c/4 of the group
-        const int rs = min(2 * mg + g / 4, rows - 1);
-        sp[mg] = chunk_sum + (size_t)(rs * 4 + g % 4) * n_sums;
+        bp[mg] = planes + (size_t)(min(r, rows - 1) * 3 + limb) * plane_stride(n_in);
+        sp[mg] = chunk_sum + (size_t)(min(rs, rows - 1) * 4 + ls) * n_sums;
     }
 }
 
@@ -610,7 +666,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
 // same position; the nibbles follow them.
 template <int NG, bool FIFTH>
 __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, Accum<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, AccumFold<NG> &acc) {
     constexpr int kQs = FIFTH ? 48 : 16;
     const uint4 hA = *reinterpret_cast<const uint4 *>(rowA);
     const uint4 hB = *reinterpret_cast<const uint4 *>(rowB);
@@ -626,7 +682,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
     const uint32_t mnB[2] = {hB.z & 0x3F3F3F3Fu, ((hB.w >> 4) & 0x0F0F0F0Fu) | ((hB.z >> 2) & 0x30303030u)};
     int I[NG][4];
 #pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++)
+    for (int mg = 0; mg < kFoldGroups<NG>; mg++)
 #pragma unroll
         for (int j = 0; j < 4; j++) I[mg][j] = 0;
 #pragma unroll
@@ -646,7 +702,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
             }
             const int sa = (scA[c >> 2] >> (8 * (c & 3))) & 0xFF, sb = (scB[c >> 2] >> (8 * (c & 3))) & 0xFF;
 #pragma unroll
-            for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+            for (int mg = 0; mg < kFoldGroups<NG>; mg++) {
                 const uint2 b = *reinterpret_cast<const uint2 *>(bp[mg] + kbase + 32 * c + 8 * t);
                 int cc[4];
                 mma_s8_k32(cc, a0, a1, a2, a3, b.x, b.y);
@@ -658,13 +714,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
         }
     }
     const float dA = half_lo(hA.x), dB = half_lo(hB.x);
-#pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
-        acc.f[mg][0] = fmaf(dA, (float)I[mg][0], acc.f[mg][0]);
-        acc.f[mg][1] = fmaf(dA, (float)I[mg][1], acc.f[mg][1]);
-        acc.f[mg][2] = fmaf(dB, (float)I[mg][2], acc.f[mg][2]);
-        acc.f[mg][3] = fmaf(dB, (float)I[mg][3], acc.f[mg][3]);
-    }
+    fold<NG>(acc, dA, dB, I, t);
     // min term, also exact: one k16 MMA of the 8 mins of the super-block (k slots 0..7) against the
     // per-chunk sums of X, held as 4 limbs x 2 activation rows in the 8 columns
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
@@ -674,10 +724,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 5) + 4 * (t & 1));
         int cc[4];
         mma_s8_k16(cc, a0, a1, b0);
-        acc.m[mg][0] = fmaf(nA, (float)cc[0], acc.m[mg][0]);
-        acc.m[mg][1] = fmaf(nA, (float)cc[1], acc.m[mg][1]);
-        acc.m[mg][2] = fmaf(nB, (float)cc[2], acc.m[mg][2]);
-        acc.m[mg][3] = fmaf(nB, (float)cc[3], acc.m[mg][3]);
+        fold_min<NG>(acc, nA, nB, cc, mg, t);
     }
 }
 
@@ -1094,10 +1141,10 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
 
 template <int NG, int ODD>
 __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, Accum<NG> &acc) {
+                                          int t, AccumFold<NG> &acc) {
     int I[NG][4];
 #pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++)
+    for (int mg = 0; mg < kFoldGroups<NG>; mg++)
 #pragma unroll
         for (int j = 0; j < 4; j++) I[mg][j] = 0;
 #pragma unroll
@@ -1130,7 +1177,7 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
             const uint32_t a1 = (lowB & 0x3C3C3C3Cu) | (hiB & 0xC0C0C0C0u);
             const int sa = sext_byte(scA[G >> 2], G & 3), sb = sext_byte(scB[G >> 2], G & 3);
 #pragma unroll
-            for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+            for (int mg = 0; mg < kFoldGroups<NG>; mg++) {
                 const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 128 * h + 16 * G + 4 * t);
                 int cc[4];
                 mma_s8_k16(cc, a0, a1, b0);
@@ -1143,13 +1190,7 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
     }
     const float dA = 0.25f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkA + 208)));
     const float dB = 0.25f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkB + 208)));
-#pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
-        acc.f[mg][0] = fmaf(dA, (float)I[mg][0], acc.f[mg][0]);
-        acc.f[mg][1] = fmaf(dA, (float)I[mg][1], acc.f[mg][1]);
-        acc.f[mg][2] = fmaf(dB, (float)I[mg][2], acc.f[mg][2]);
-        acc.f[mg][3] = fmaf(dB, (float)I[mg][3], acc.f[mg][3]);
-    }
+    fold<NG>(acc, dA, dB, I, t);
 }
 
 // A Q2_K super-block (src/quant.cpp:398-424): 16 bytes of (scale | min << 4), 64 bytes of 2-bit quants, d, dmin;
@@ -1159,7 +1200,7 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
 // sums of X (acc.m, as for Q4_K).
 template <int NG>
 __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, Accum<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, AccumFold<NG> &acc) {
     const uint32_t *wa = reinterpret_cast<const uint32_t *>(blkA), *wb = reinterpret_cast<const uint32_t *>(blkB);
     uint32_t scA[4], scB[4];
 #pragma unroll
@@ -1169,7 +1210,7 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
     }
     int I[NG][4];
 #pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++)
+    for (int mg = 0; mg < kFoldGroups<NG>; mg++)
 #pragma unroll
         for (int j = 0; j < 4; j++) I[mg][j] = 0;
 #pragma unroll
@@ -1181,7 +1222,7 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
             const uint32_t a0 = (qA[s] >> (2 * j)) & 0x03030303u, a1 = (qB[s] >> (2 * j)) & 0x03030303u;
             const int sa = (scA[G >> 2] >> (8 * (G & 3))) & 0xF, sb = (scB[G >> 2] >> (8 * (G & 3))) & 0xF;
 #pragma unroll
-            for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+            for (int mg = 0; mg < kFoldGroups<NG>; mg++) {
                 const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 16 * G + 4 * t);
                 int cc[4];
                 mma_s8_k16(cc, a0, a1, b0);
@@ -1195,22 +1236,13 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
     const uint32_t hA = wa[20], hB = wb[20];
     const float dA = half_lo(hA), dB = half_lo(hB), nA = half_hi(hA), nB = half_hi(hB);
     const uint32_t m0 = (wa[t] >> 4) & 0x0F0F0F0Fu, m1 = (wb[t] >> 4) & 0x0F0F0F0Fu;   // k slot j = group j: lane t brings 4t..4t+3
-#pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
-        acc.f[mg][0] = fmaf(dA, (float)I[mg][0], acc.f[mg][0]);
-        acc.f[mg][1] = fmaf(dA, (float)I[mg][1], acc.f[mg][1]);
-        acc.f[mg][2] = fmaf(dB, (float)I[mg][2], acc.f[mg][2]);
-        acc.f[mg][3] = fmaf(dB, (float)I[mg][3], acc.f[mg][3]);
-    }
+    fold<NG>(acc, dA, dB, I, t);
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 4) + 4 * t);
         int cc[4];
         mma_s8_k16(cc, m0, m1, b0);
-        acc.m[mg][0] = fmaf(nA, (float)cc[0], acc.m[mg][0]);
-        acc.m[mg][1] = fmaf(nA, (float)cc[1], acc.m[mg][1]);
-        acc.m[mg][2] = fmaf(nB, (float)cc[2], acc.m[mg][2]);
-        acc.m[mg][3] = fmaf(nB, (float)cc[3], acc.m[mg][3]);
+        fold_min<NG>(acc, nA, nB, cc, mg, t);
     }
 }
 
@@ -1221,7 +1253,7 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
 // 2 bytes off a word boundary (MODE as for Q6_K).
 template <int NG, int MODE>
 __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, Accum<NG> &acc) {
+                                          int t, AccumFold<NG> &acc) {
     uint32_t SA[4], SB[4];
     {
         const uint32_t a0 = ld_q6<MODE>(blkA, 96), a1 = ld_q6<MODE>(blkA, 100), a2 = ld_q6<MODE>(blkA, 104);
@@ -1245,7 +1277,7 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
     const uint32_t hmB[2] = {~ld_q6<MODE>(blkB, 4 * t), ~ld_q6<MODE>(blkB, 16 + 4 * t)};
     int I[NG][4];
 #pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++)
+    for (int mg = 0; mg < kFoldGroups<NG>; mg++)
 #pragma unroll
         for (int j = 0; j < 4; j++) I[mg][j] = 0;
 #pragma unroll
@@ -1260,7 +1292,7 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
             const uint32_t a1 = (qb & 0x60606060u) | ((hmB[s] << (7 - hb)) & 0x80808080u);
             const int sa = sext_byte(SA[G >> 2], G & 3), sb = sext_byte(SB[G >> 2], G & 3);
 #pragma unroll
-            for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+            for (int mg = 0; mg < kFoldGroups<NG>; mg++) {
                 const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 16 * G + 4 * t);
                 int cc[4];
                 mma_s8_k16(cc, a0, a1, b0);
@@ -1273,13 +1305,7 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
     }
     const float dA = 0.03125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkA + 108)));
     const float dB = 0.03125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkB + 108)));
-#pragma unroll
-    for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
-        acc.f[mg][0] = fmaf(dA, (float)I[mg][0], acc.f[mg][0]);
-        acc.f[mg][1] = fmaf(dA, (float)I[mg][1], acc.f[mg][1]);
-        acc.f[mg][2] = fmaf(dB, (float)I[mg][2], acc.f[mg][2]);
-        acc.f[mg][3] = fmaf(dB, (float)I[mg][3], acc.f[mg][3]);
-    }
+    fold<NG>(acc, dA, dB, I, t);
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------
@@ -1295,12 +1321,8 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
 
 // SINGLE: 0 the general form; 1 Q4_K with one activation row (unit_q4_k_single); 2 the same with the B
 // fragments of the warp's (at most two) K units held in registers, for rows of at most 16 units.
-// Two CTAs per SM (96 registers per thread) or one (up to 192). One or two activation rows always fit in 96.
-// Three or four rows (two column groups) of Q8_0 also do, and two half-SM CTAs are then 1.1-1.5x faster than one
-// at every size. Q4_0 fits too but gains only on very tall matrices (+14 % at 131072 rows, -3 to -9 % at layer
-// sizes); the K-quant forms spill at 96 registers and are faster alone on an SM at layer sizes.
-template <int WT, int NG>
-constexpr bool kTwoPerSm = NG == 1 || (NG == 2 && WT == KRK_CUDA_Q8_0);
+// Either way an SM runs sixteen consumer warps of up to 96 registers: two half-SM CTAs for one or two activation rows,
+// one CTA of two consumer groups for more (see consumer_groups).
 
 // RAG: the form for ragged rows of Q6_K and Q3_K and of the 32-value block formats (K not a multiple of 256), whose units
 // find each word's alignment from its address; compiled apart so that the usual form does not carry another copy of
@@ -1310,12 +1332,14 @@ constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_si
 template <int WT>
 constexpr bool kMayRag = kRagForm<WT> || WT == KRK_CUDA_Q2_K;
 template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false>
-__global__ void __launch_bounds__(kThreads, kTwoPerSm<WT, NG> ? 2 : 1)
+__global__ void __launch_bounds__(cta_threads(consumer_groups(NG)), NG == 1 ? 2 : 1)
 gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // STACK: several 16-row tiles per stage (p.tps of them); compiled apart so that the usual one-tile
     // form carries none of its index arithmetic.
     static_assert(!SINGLE || ((WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q4_0) && NG == 1), "the single-row forms are Q4_K and Q4_0");
     const int tps = STACK ? p.tps : 1;
+    constexpr int kGroups = consumer_groups(NG), kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
+    constexpr bool kFold = block_size(WT) == 256 && !SINGLE;   // AccumFold
     using F = Fmt<WT>;
     using SmemT = Smem<NG>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1340,9 +1364,9 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         if (lane == 0) {
             for (int s = 0; s < p.n_stages; s++) {
                 mbar_init(smem_u32(&sm->full[s]), 1);
-                mbar_init(smem_u32(&sm->empty[s]), kConsumerWarps);
+                mbar_init(smem_u32(&sm->empty[s]), kGroups * kConsumerWarps);
             }
-            for (int s = 0; s < red_slots(NG); s++) {
+            for (int s = 0; s < kGroups * red_slots(NG); s++) {
                 mbar_init(smem_u32(&sm->red_full[s]), n_warps);
                 mbar_init(smem_u32(&sm->red_empty[s]), 1);
             }
@@ -1428,8 +1452,9 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         int tile_it = 0;
         walk(p, tv, tps, [](int) {}, [&](const StageInfo &s) {
             if (!s.last) return;
-            const int slot = tile_it % kSlots;
-            wait_phase(smem_u32(&sm->red_full[slot]), (tile_it / kSlots) & 1, gave_up, p.status);
+            // (two groups take the tiles in turn, each through slots of its own)
+            const int nth = tile_it / kGroups, slot = (tile_it % kGroups) * kSlots + nth % kSlots;
+            wait_phase(smem_u32(&sm->red_full[slot]), (nth / kSlots) & 1, gave_up, p.status);
             tile_it++;
 #pragma unroll
             for (int sub = 0; sub < (STACK ? kMaxStack : 1); sub++) {
@@ -1511,12 +1536,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     }
 
     // ===== consumer warps =====
-    const int wid = warp - 1, g = lane >> 2, t = lane & 3;
+    const int grp = kGroups == 1 ? 0 : (warp - 1) / kConsumerWarps;   // consumer group: takes tiles grp, grp + 2, ...
+    const int wid = warp - 1 - grp * kConsumerWarps, g = lane >> 2, t = lane & 3;
     const float *prepared = nullptr;
     const int8_t *bp[NG], *sp[NG];
     const float *fe[NG], *fo[NG];   // Q5_1: per-block sums of the even / odd activation row of each column group
-    float xs[2 * NG];   // this warp's scale of each activation row
-    Accum<NG> acc;
+    float xs[2 * NG];   // this warp's scale of each activation row (kFold: of its own rows, xs[0] and xs[1])
+    std::conditional_t<kFold, AccumFold<NG>, Accum<NG>> acc;
     AccumSingle acs;
     accum_zero(acc);
     acs.f[0] = acs.f[1] = acs.m[0] = acs.m[1] = acs.m[2] = acs.m[3] = 0.0f;
@@ -1559,17 +1585,35 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                 asm volatile("griddepcontrol.wait;" ::: "memory");
                 if (p.tune & 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             }
-            prepared = tv.mat[m].x;
+            const float *x = tv.mat[m].x;
+            // (stacked tiles: every sub-tile prepares its own copy)
+            auto prepare = [&](int r) {
+                return prepare_x_row<WT, RAG && block_size(WT) == 32>(x + (size_t)r * p.n_in, p, planes + (size_t)(r * 3) * plane_stride(p.n_in),
+                                                                      chunk_sum + (size_t)(r * 4) * (p.n_in >> kSumShift<WT>),
+                                                                      stacked_idle ? p.units : my_unit, lane);
+            };
+            if (kGroups == 1) {
 #pragma unroll
-            for (int r = 0; r < 2 * NG; r++)
-                // (stacked tiles: every sub-tile prepares its own copy)
-                xs[r] = r < p.rows ? prepare_x_row<WT, RAG && block_size(WT) == 32>(prepared + (size_t)r * p.n_in, p,
-                                                       planes + (size_t)(r * 3) * plane_stride(p.n_in),
-                                                       chunk_sum + (size_t)(r * 4) * (p.n_in >> kSumShift<WT>),
-                                                       stacked_idle ? kConsumerWarps : my_unit, lane)
-                                   : 0.0f;
-            __syncwarp();
-            if (!SINGLE) lane_planes<NG>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
+                for (int r = 0; r < 2 * NG; r++) xs[r] = r < p.rows ? prepare(r) : 0.0f;
+                __syncwarp();
+            } else {
+                // each group prepares every other row; nobody may still read the activation before this one
+                if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
+#pragma unroll 1
+                for (int r = grp; r < p.rows; r += kGroups) {
+                    const float sc = prepare(r);
+                    if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = sc;
+                }
+                asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
+#pragma unroll
+                for (int r = 0; r < (kFold ? kFoldRows<NG> : 2 * NG); r++) {
+                    const int row = kFold ? t + 4 * r : r;
+                    xs[r] = row < p.rows ? sm->scale[NG == 1 ? 0 : wid][row] : 0.0f;
+                }
+            }
+            if (kFold && NG == 1) xs[0] = t < 2 ? xs[0] : xs[1];
+            prepared = x;
+            if (!SINGLE) lane_planes<NG, kFold>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -1588,6 +1632,21 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         const int stage_rows = kTileRows * tps;
         const int n_tiles = ((r1 - r0 + stage_rows - 1) / stage_rows) * p.step;
         for (int tile = 0; tile < n_tiles; tile++) {
+            if (kGroups > 1 && tile_it % kGroups != grp) {
+                // the other group's tile: its stages are seen to land (a ring slot's parity only tells two laps apart for a
+                // warp that looks at every lap) and given back
+                tile_it++;
+                for (int ck = 0; ck < n_chunks; ck++) {
+                    wait_phase(full0 + 8 * slot, phase, gave_up, p.status);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty0 + 8 * slot);
+                    if (++slot == p.n_stages) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
+                continue;
+            }
             // ragged rows: how far this lane's two rows sit into their slots of a stage
             uint32_t ragA = 0, ragB = 0;
             if (RAG || (WT == KRK_CUDA_Q2_K && p.ragged)) {
@@ -1608,29 +1667,29 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         const int unit = ck * kConsumerWarps + su;
                         const int kbase = unit * F::unit_values;
                         const int nb = (p.n_in - kbase) >> 5;   // 32-value blocks of the unit (short rows: fewer than a full unit's)
-                        if (WT == KRK_CUDA_Q4_0 && !SINGLE) {
+                        if constexpr (WT == KRK_CUDA_Q4_0 && !SINGLE) {
                             unit_q4_0_rows<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
-                        } else if (WT == KRK_CUDA_Q4_0) {
+                        } else if constexpr (WT == KRK_CUDA_Q4_0) {
                             unit_q4_0(rowA, rowB, bq + kbase, reinterpret_cast<const float *>(chunk_sum) + (kbase >> 5), t, acs);
-                        } else if (SINGLE == 2) {
+                        } else if constexpr (SINGLE == 2) {
                             unit_q4_k_single(rowA, rowB, bf, t, acs);
-                        } else if (SINGLE == 1) {
+                        } else if constexpr (SINGLE == 1) {
                             unit_q4_k_single(rowA, rowB, load_bfrag(bq + kbase, sq + (kbase >> 5), t), t, acs);
-                        } else if (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K) {
+                        } else if constexpr (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K) {
                             unit_q4_k<NG, WT == KRK_CUDA_Q5_K>(rowA, rowB, kbase, bp, sp, t, acc);
-                        } else if (WT == KRK_CUDA_Q8_0) {
+                        } else if constexpr (WT == KRK_CUDA_Q8_0) {
                             unit_q8_0<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
-                        } else if (WT == KRK_CUDA_Q5_0) {
+                        } else if constexpr (WT == KRK_CUDA_Q5_0) {
                             unit_q5_0<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
-                        } else if (WT == KRK_CUDA_IQ4_NL) {
+                        } else if constexpr (WT == KRK_CUDA_IQ4_NL) {
                             unit_iq4_nl<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
-                        } else if (WT == KRK_CUDA_Q2_K) {
+                        } else if constexpr (WT == KRK_CUDA_Q2_K) {
                             unit_q2_k<NG>(rowA, rowB, kbase, bp, sp, t, acc);
-                        } else if (WT == KRK_CUDA_Q3_K) {
+                        } else if constexpr (WT == KRK_CUDA_Q3_K) {
                             if (RAG) unit_q3_k<NG, 2>(rowA, rowB, kbase, bp, t, acc);
                             else if (unit & 1) unit_q3_k<NG, 1>(rowA, rowB, kbase, bp, t, acc);
                             else unit_q3_k<NG, 0>(rowA, rowB, kbase, bp, t, acc);
-                        } else if (WT == KRK_CUDA_Q5_1) {
+                        } else if constexpr (WT == KRK_CUDA_Q5_1) {
                             unit_q5_1<NG, RAG>(rowA, rowB, kbase, bp, fe, fo, t, acc, nb);
                         } else {
                             if (RAG) unit_q6_k<NG, 2>(rowA, rowB, kbase, bp, t, acc);
@@ -1653,74 +1712,89 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                 for (int ck = 0; ck < n_chunks; ck++) stage(ck, held[0]);
             }
             {
-             // ---- end of the tile: the four lanes of a row group add their weighted shares, lane t = 0 leaves them ----
+             // ---- end of the tile: the lanes of a row group add their weighted shares ----
              constexpr int kSlots = red_slots(NG);
-             const int rslot = tile_it % kSlots;
-             const uint32_t rphase = (tile_it / kSlots) & 1;
+             const int nth = tile_it / kGroups, rslot = grp * kSlots + nth % kSlots;
+             const uint32_t rphase = (nth / kSlots) & 1;
              tile_it++;
              if (wid >= n_warps) continue;
-             // min columns: limb c%4 (weights 2^24, 2^16, 2^8, 1) of activation row c/4
-             const float me0 = t == 0 ? 16777216.0f : (t == 1 ? 256.0f : 0.0f), me1 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f);
-             const float mo0 = t == 2 ? 16777216.0f : (t == 3 ? 256.0f : 0.0f), mo1 = t == 2 ? 65536.0f : (t == 3 ? 1.0f : 0.0f);
-             float4 o[NG];
-             if (SINGLE) {
-                 // lane t holds limb t (weights 65536, 256, 1) of rows g and g+8, times 16
-                 // (Q4_0: lane t = 3 holds d * sum of X per block, the -8 of every quant)
-                 const float wl = t == 0 ? 4096.0f : (t == 1 ? 16.0f : (t == 2 ? 0.0625f : (WT == KRK_CUDA_Q4_0 ? -8.0f : 0.0f)));
-                 o[0].x = (wl * acs.f[0] - fmaf(me0, acs.m[0], me1 * acs.m[1])) * xs[0];
-                 o[0].z = (wl * acs.f[1] - fmaf(me0, acs.m[2], me1 * acs.m[3])) * xs[0];
-                 o[0].y = o[0].w = 0.0f;
-                 acs.f[0] = acs.f[1] = acs.m[0] = acs.m[1] = acs.m[2] = acs.m[3] = 0.0f;
+             if constexpr (kFold) {
+                 float o[kFoldRows<NG>][2];
+#pragma unroll
+                 for (int h = 0; h < kFoldRows<NG>; h++)
+#pragma unroll
+                     for (int b = 0; b < 2; b++) {
+                         o[h][b] = acc.a[h][b] * xs[h];
+                         if (NG == 1) o[h][b] += __shfl_xor_sync(0xFFFFFFFFu, o[h][b], 1);   // lanes 0, 1: row 0; 2, 3: row 1
+                     }
+                 accum_zero(acc);
+                 wait_phase(smem_u32(&sm->red_empty[rslot]), rphase ^ 1, gave_up, p.status);
+                 if (NG > 1 || (t & 1) == 0) {
+#pragma unroll
+                     for (int h = 0; h < kFoldRows<NG>; h++) {
+                         const int r = NG == 1 ? t >> 1 : t + 4 * h;
+                         float *dst = reinterpret_cast<float *>(&sm->red[rslot][wid][r >> 1][g]) + (r & 1);
+                         dst[0] = o[h][0];   // weight row g
+                         dst[2] = o[h][1];   // g + 8
+                     }
+                 }
              } else {
-                 // Column c of a group carries limb c%3 (weights 65536, 256, 1) of activation row c/3; this lane
-                 // holds columns 2t and 2t+1, so its accumulators enter the even activation row with (we0, we1)
-                 // and the odd one with (wo0, wo1). The Q4_K min term is already a per-lane partial sum.
-                 const float we0 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f), we1 = t == 0 ? 256.0f : 0.0f;
-                 const float wo0 = t == 2 ? 256.0f : 0.0f, wo1 = t == 1 ? 65536.0f : (t == 2 ? 1.0f : 0.0f);
+                 float4 o[NG];
+                 if constexpr (SINGLE != 0) {
+                     // lane t holds limb t (weights 65536, 256, 1) of rows g and g+8, times 16
+                     // (Q4_0: lane t = 3 holds d * sum of X per block, the -8 of every quant); Q4_K's minimum columns: two
+                     // of four limbs (weights 2^24 .. 1) in lanes 0 and 1
+                     const float me0 = t == 0 ? 16777216.0f : (t == 1 ? 256.0f : 0.0f), me1 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f);
+                     const float wl = t == 0 ? 4096.0f : (t == 1 ? 16.0f : (t == 2 ? 0.0625f : (WT == KRK_CUDA_Q4_0 ? -8.0f : 0.0f)));
+                     o[0].x = (wl * acs.f[0] - fmaf(me0, acs.m[0], me1 * acs.m[1])) * xs[0];
+                     o[0].z = (wl * acs.f[1] - fmaf(me0, acs.m[2], me1 * acs.m[3])) * xs[0];
+                     o[0].y = o[0].w = 0.0f;
+                     acs.f[0] = acs.f[1] = acs.m[0] = acs.m[1] = acs.m[2] = acs.m[3] = 0.0f;
+                 } else {
+                     // Column c of a group carries limb c%3 (weights 65536, 256, 1) of activation row c/3; this lane
+                     // holds columns 2t and 2t+1, so its accumulators enter the even activation row with (we0, we1)
+                     // and the odd one with (wo0, wo1).
+                     const float we0 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f), we1 = t == 0 ? 256.0f : 0.0f;
+                     const float wo0 = t == 2 ? 256.0f : 0.0f, wo1 = t == 1 ? 65536.0f : (t == 2 ? 1.0f : 0.0f);
+#pragma unroll
+                     for (int mg = 0; mg < NG; mg++) {
+                         if (NG == 4 && mg == 3) {
+                             // activation rows 6 and 7 rode in columns 6 and 7 (lane t = 3) of groups 0..2, limb mg in group mg
+                             const float w0 = t == 3 ? 65536.0f : 0.0f, w1 = t == 3 ? 256.0f : 0.0f, w2 = t == 3 ? 1.0f : 0.0f;
+                             o[mg].x = fmaf(w0, acc.f[0][0], fmaf(w1, acc.f[1 % NG][0], w2 * acc.f[2 % NG][0]));
+                             o[mg].y = fmaf(w0, acc.f[0][1], fmaf(w1, acc.f[1 % NG][1], w2 * acc.f[2 % NG][1]));
+                             o[mg].z = fmaf(w0, acc.f[0][2], fmaf(w1, acc.f[1 % NG][2], w2 * acc.f[2 % NG][2]));
+                             o[mg].w = fmaf(w0, acc.f[0][3], fmaf(w1, acc.f[1 % NG][3], w2 * acc.f[2 % NG][3]));
+                         } else {
+                             o[mg].x = fmaf(we0, acc.f[mg][0], we1 * acc.f[mg][1]);   // row g,   even activation row
+                             o[mg].y = fmaf(wo0, acc.f[mg][0], wo1 * acc.f[mg][1]);   // row g,   odd
+                             o[mg].z = fmaf(we0, acc.f[mg][2], we1 * acc.f[mg][3]);   // row g+8, even
+                             o[mg].w = fmaf(wo0, acc.f[mg][2], wo1 * acc.f[mg][3]);   // row g+8, odd
+                         }
+                         o[mg].x *= xs[2 * mg];
+                         o[mg].y *= xs[2 * mg + 1];
+                         o[mg].z *= xs[2 * mg];
+                         o[mg].w *= xs[2 * mg + 1];
+                     }
+                     accum_zero(acc);
+                 }
 #pragma unroll
                  for (int mg = 0; mg < NG; mg++) {
-                     if (NG == 4 && mg == 3) {
-                         // activation rows 6 and 7 rode in columns 6 and 7 (lane t = 3) of groups 0..2, limb mg in group mg
-                         const float w0 = t == 3 ? 65536.0f : 0.0f, w1 = t == 3 ? 256.0f : 0.0f, w2 = t == 3 ? 1.0f : 0.0f;
-                         o[mg].x = fmaf(w0, acc.f[0][0], fmaf(w1, acc.f[1][0], w2 * acc.f[2][0]));
-                         o[mg].y = fmaf(w0, acc.f[0][1], fmaf(w1, acc.f[1][1], w2 * acc.f[2][1]));
-                         o[mg].z = fmaf(w0, acc.f[0][2], fmaf(w1, acc.f[1][2], w2 * acc.f[2][2]));
-                         o[mg].w = fmaf(w0, acc.f[0][3], fmaf(w1, acc.f[1][3], w2 * acc.f[2][3]));
-                     } else {
-                         o[mg].x = fmaf(we0, acc.f[mg][0], we1 * acc.f[mg][1]);   // row g,   even activation row
-                         o[mg].y = fmaf(wo0, acc.f[mg][0], wo1 * acc.f[mg][1]);   // row g,   odd
-                         o[mg].z = fmaf(we0, acc.f[mg][2], we1 * acc.f[mg][3]);   // row g+8, even
-                         o[mg].w = fmaf(wo0, acc.f[mg][2], wo1 * acc.f[mg][3]);   // row g+8, odd
-                     }
-                     if (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K) {
-                         o[mg].x -= fmaf(me0, acc.m[mg][0], me1 * acc.m[mg][1]);
-                         o[mg].y -= fmaf(mo0, acc.m[mg][0], mo1 * acc.m[mg][1]);
-                         o[mg].z -= fmaf(me0, acc.m[mg][2], me1 * acc.m[mg][3]);
-                         o[mg].w -= fmaf(mo0, acc.m[mg][2], mo1 * acc.m[mg][3]);
-                     }
-                     o[mg].x *= xs[2 * mg];
-                     o[mg].y *= xs[2 * mg + 1];
-                     o[mg].z *= xs[2 * mg];
-                     o[mg].w *= xs[2 * mg + 1];
-                 }
-                 accum_zero(acc);
-             }
 #pragma unroll
-             for (int mg = 0; mg < NG; mg++) {
-#pragma unroll
-                 for (int d = 1; d <= 2; d <<= 1) {   // (t0 + t1) + (t2 + t3): a fixed order
-                     o[mg].x += __shfl_xor_sync(0xFFFFFFFFu, o[mg].x, d);
-                     o[mg].z += __shfl_xor_sync(0xFFFFFFFFu, o[mg].z, d);
-                     if (!SINGLE) {
-                         o[mg].y += __shfl_xor_sync(0xFFFFFFFFu, o[mg].y, d);
-                         o[mg].w += __shfl_xor_sync(0xFFFFFFFFu, o[mg].w, d);
+                     for (int d = 1; d <= 2; d <<= 1) {   // (t0 + t1) + (t2 + t3): a fixed order
+                         o[mg].x += __shfl_xor_sync(0xFFFFFFFFu, o[mg].x, d);
+                         o[mg].z += __shfl_xor_sync(0xFFFFFFFFu, o[mg].z, d);
+                         if (!SINGLE) {
+                             o[mg].y += __shfl_xor_sync(0xFFFFFFFFu, o[mg].y, d);
+                             o[mg].w += __shfl_xor_sync(0xFFFFFFFFu, o[mg].w, d);
+                         }
                      }
                  }
-             }
-             wait_phase(smem_u32(&sm->red_empty[rslot]), rphase ^ 1, gave_up, p.status);
-             if (t == 0) {
+                 wait_phase(smem_u32(&sm->red_empty[rslot]), rphase ^ 1, gave_up, p.status);
+                 if (t == 0) {
 #pragma unroll
-                 for (int mg = 0; mg < NG; mg++) sm->red[rslot][wid][mg][g] = o[mg];
+                     for (int mg = 0; mg < NG; mg++) sm->red[rslot][wid][mg][g] = o[mg];
+                 }
              }
              __syncwarp();
              if (lane == 0) mbar_arrive(smem_u32(&sm->red_full[rslot]));
@@ -1747,7 +1821,7 @@ int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(cta_threads(consumer_groups(NG)));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1844,13 +1918,13 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     }
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
     const int fixed = align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows));
-    // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most
-    // kMaxStages. Wide activations (large K) leave too little of a half, and the forms compiled for one CTA
-    // per SM (more registers; see kTwoPerSm) take the whole SM.
-    const bool halves = rows <= 2 || (rows <= 4 && kTwoPerSm<WT, 2>);
+    // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
+    // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
+    const bool halves = rows <= 2;
     int max_fit = halves ? (kSmemLimit - fixed) / p.stage_bytes : 0;
     if (max_fit < 3) max_fit = (kSmemWhole - fixed) / p.stage_bytes;
-    p.n_stages = max_fit < kMaxStages ? max_fit : kMaxStages;
+    const int most = halves ? kMaxHalfStages : kMaxStages;
+    p.n_stages = max_fit < most ? max_fit : most;
     if (p.n_stages < 2) return false;
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
     return true;
@@ -1896,8 +1970,7 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
 // (KRK_CUDA_GEMV_CTAS_PER_SM=1): the other half is left to the next launch in the stream, which becomes
 // resident early, sets itself up and fills its ring while this one streams; measured on the layer-sized
 // matrices of a decode step the slower streaming of eight warps costs more than the overlap saves.
-// The forms compiled for one CTA per SM (kTwoPerSm) get one whatever their shared memory: a grid of two per
-// SM would run as two waves and prepare the activation twice.
+// The forms of two consumer groups get one whatever their shared memory.
 template <int WT>
 int ctas_per_sm(size_t smem, int rows) {
     static const int want = [] {
@@ -1905,8 +1978,7 @@ int ctas_per_sm(size_t smem, int rows) {
         const int v = e ? std::atoi(e) : 0;
         return v == 1 ? 1 : 2;
     }();
-    const bool halves = rows <= 2 || (rows <= 4 && kTwoPerSm<WT, 2>);
-    return halves && smem <= (size_t)kSmemLimit ? want : 1;
+    return rows <= 2 && smem <= (size_t)kSmemLimit ? want : 1;
 }
 
 // Tensor maps are encoded on the host (a driver call of a microsecond or two) and kept per (matrix, box):
