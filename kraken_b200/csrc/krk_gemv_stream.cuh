@@ -95,9 +95,8 @@ template <> struct Fmt<KRK_CUDA_Q3_K> { static constexpr int unit_values = 256, 
 template <> struct Fmt<KRK_CUDA_IQ4_NL> { static constexpr int unit_values = 256, unit_bytes = 144, stride_mod = 16, tma = 1; };
 template <> struct Fmt<KRK_CUDA_Q5_1> { static constexpr int unit_values = 256, unit_bytes = 192, stride_mod = 16, tma = 0; };
 
+// What every warp reads before its first load stands first: parameters arrive cold in every launch, a cache line at a time.
 struct StreamParams {
-    GemvMat mat[KRK_CUDA_MAX_GROUP];
-    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
     int n_entries;        // matrices, or gate/up pairs when silu_pair
     int step;             // matrices per entry (2 for gate/up pairs)
     int rows;             // activation rows
@@ -118,14 +117,15 @@ struct StreamParams {
     int use_tma;          // 1: a stage arrives as one tiled tensor copy, laid out [unit][row][unit_bytes]; 2: [row][units]
     int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this
     int box_bytes;        // bytes one tensor copy signals (the whole box, also where the matrix clips it)
-    int tune;             // experiment bits: 1 = weights are not prefetched before the dependency wait; 2 = the dependent
-                          // launch is released after this grid's own dependency wait instead of at its start
     int stage_bytes;
     int n_stages;
     int total_gran;
     int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
     const StreamTable *dev_table;   // when set, the matrices come from device memory
     int entry_gran;       // table launches: granules of every entry (all have one shape)
+    int *status;
+    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
+    GemvMat mat[KRK_CUDA_MAX_GROUP];
     // Table launches with tensor copies: every matrix of the table lies inside one of two stacked banks (the gate
     // and the up bank of an expert set), each described by ONE tensor map (wmap[0], wmap[1]) over all of its
     // rows; a matrix is then a row offset into its bank.
@@ -136,7 +136,6 @@ struct StreamParams {
     int *peer_flag[KRK_CUDA_MAX_PEERS];   // peer_flag[q][my_rank] <- epoch once every CTA here has stored
     int n_peers, my_rank, epoch, wait_peers;
     long long peer_row_stride, peer_offset;
-    int *status;
     // per matrix: the weights as a 3-d tensor {unit_bytes, n_out rows, units per row}; box = {unit_bytes,
     // rows of a stage, units of a stage}
     CUtensorMap wmap[KRK_CUDA_MAX_GROUP];
@@ -315,36 +314,32 @@ struct StageInfo {
 // Where the list of matrices lives: the kernel parameters (host-built launches) or a table in
 // device memory written by an earlier kernel (the routed-expert launches, whose matrices depend on
 // expert ids that never leave the device).
+// (Parameters are read as parameters, never through a pointer that may also be a table's: such a generic load of the
+// parameter space misses to level 2, and four of them in a row kept a launch of 5.7 us waiting for 0.8 us.)
 struct TableView {
-    const GemvMat *mat;
-    const int *gran_begin;   // host-built launches
-    int entry_gran;          // tables: granules per entry (0: host-built)
+    const StreamParams &p;
+    const StreamTable *dev;
     int n_entries;
     int gran_q, gran_r;
-    __device__ __forceinline__ int begin(int e) const { return entry_gran ? e * entry_gran : gran_begin[e]; }
-    __device__ __forceinline__ int first(int g) const { return entry_gran ? g / entry_gran : 0; }   // no entry before it holds granule g
-};
-
-__device__ __forceinline__ TableView table_view(const StreamParams &p) {
-    TableView tv;
-    if (p.dev_table) {
-        tv.mat = p.dev_table->mat;
-        tv.gran_begin = nullptr;
-        tv.entry_gran = p.entry_gran;
-        tv.n_entries = p.dev_table->n_entries;
-        const int total = tv.n_entries * tv.entry_gran;
-        tv.gran_q = total / (int)gridDim.x;
-        tv.gran_r = total % (int)gridDim.x;
-    } else {
-        tv.mat = p.mat;
-        tv.gran_begin = p.gran_begin;
-        tv.entry_gran = 0;
-        tv.n_entries = p.n_entries;
-        tv.gran_q = p.gran_q;
-        tv.gran_r = p.gran_r;
+    __device__ __forceinline__ explicit TableView(const StreamParams &params) : p(params), dev(params.dev_table) {
+        if (dev) {
+            n_entries = dev->n_entries;
+            const int total = n_entries * p.entry_gran;
+            gran_q = total / (int)gridDim.x;
+            gran_r = total % (int)gridDim.x;
+        } else {
+            n_entries = p.n_entries;
+            gran_q = p.gran_q;
+            gran_r = p.gran_r;
+        }
     }
-    return tv;
-}
+    __device__ __forceinline__ int begin(int e) const { return dev ? e * p.entry_gran : p.gran_begin[e]; }
+    __device__ __forceinline__ int first(int g) const { return dev ? g / p.entry_gran : 0; }   // no entry before it holds granule g
+    __device__ __forceinline__ const uint8_t *w(int m) const { return dev ? dev->mat[m].w : p.mat[m].w; }
+    __device__ __forceinline__ const float *x(int m) const { return dev ? dev->mat[m].x : p.mat[m].x; }
+    __device__ __forceinline__ float *y(int m) const { return dev ? dev->mat[m].y : p.mat[m].y; }
+    __device__ __forceinline__ int n_out(int m) const { return (int)(dev ? dev->mat[m].n_out : p.mat[m].n_out); }
+};
 
 template <class SegmentFn, class StageFn>
 __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv, int tps, SegmentFn &&on_segment, StageFn &&on_stage) {
@@ -358,7 +353,7 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
         const int lo = max(g0, tv.begin(e)), hi = min(g1, tv.begin(e + 1));
         if (tv.begin(e) >= g1) break;
         if (lo >= hi) continue;
-        const int n_out = (int)tv.mat[e * p.step].n_out;
+        const int n_out = tv.n_out(e * p.step);
         const int r0 = (lo - tv.begin(e)) * p.gran;
         const int r1 = min(n_out, (hi - tv.begin(e)) * p.gran);
         on_segment(e * p.step);
@@ -413,16 +408,18 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
     int total = 0;
 #pragma unroll
     for (int j4 = 0; j4 < PER; j4 += 4) {
+        // The bits of x * inv + 1.5 * 2^23 are those of 1.5 * 2^23 plus X (|X| <= 2^22); adding 0x00808080 less that
+        // constant makes the limb bytes l + 128, whose sign bits are flipped back once they are packed.
         uint32_t z[4];   // byte 0: limb 2 (weight 1), byte 1: limb 1 (256), byte 2: limb 0 (65536)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int X = __float_as_int(fmaf(f[j4 + j], inv, kMagic)) - 0x4B400000;   // |x * inv| < 2^22
-            total += X;
-            z[j] = limbs3(X);
+            const int bits = __float_as_int(fmaf(f[j4 + j], inv, kMagic));
+            total += bits;
+            z[j] = (uint32_t)(bits + (0x00808080 - 0x4B400000));
         }
         const uint32_t lo01 = __byte_perm(z[0], z[1], 0x5140), lo23 = __byte_perm(z[2], z[3], 0x5140);   // l2a l2b l1a l1b
-        const uint32_t w2 = __byte_perm(lo01, lo23, 0x5410), w1 = __byte_perm(lo01, lo23, 0x7632);
-        const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], 0x0062), __byte_perm(z[2], z[3], 0x0062), 0x5410);
+        const uint32_t w2 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u, w1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
+        const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], 0x0062), __byte_perm(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
         const int i = k0 + j4;
         if (NATURAL) {
             if (live) {
@@ -482,6 +479,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
             *reinterpret_cast<uint32_t *>(p2 + i) = w2;
         }
     }
+    total -= (int)((unsigned)PER * 0x4B400000u);   // the sum of X
     if (WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_Q5_1) {
         // the sum of X over each 32-value block, as a float: the -8 of every quant leaves -8 * d * sum per block
         // (Q5_1: the block's offset m enters as m * sum)
@@ -542,11 +540,22 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
         float f[PER];
         load_slice<WT>(xr, at(u), f, mxb, live(u));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mxb = max(mxb, __shfl_xor_sync(0xFFFFFFFFu, mxb, o));
-    const bool bad = mxb > 0x7F7FFFFFu;
+    mxb = __reduce_max_sync(0xFFFFFFFFu, mxb);
+    // inv = kFixedOne / max and its counterpart s, each within a unit in the last place (|x * inv| <= 2^22 then); a maximum
+    // too small for that quotient is scaled by a power of two instead, and a non-finite activation makes the output NaN as
+    // it would in f32
     const float mx = __uint_as_float(mxb);
-    const float inv = (mx > 0.0f && !bad) ? __fdiv_rn(kFixedOne, mx) : 0.0f;
+    float rcp;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(mx));
+    float inv = fmaf(rcp, fmaf(-mx, rcp, 1.0f), rcp) * kFixedOne, s = mx * (1.0f / kFixedOne);
+    if (mx < 1e-30f) {
+        inv = 2.658455991569832e36f;    // 2^121
+        s = 3.7615819226313200e-37f;    // 2^-121
+    }
+    if (mxb > 0x7F7FFFFFu) {
+        inv = 0.0f;
+        s = __int_as_float(0x7FC00000);
+    }
 #pragma unroll
     for (int j = 0; j < kHeld; j++) {
         const int u = wid + j * kConsumerWarps;
@@ -558,7 +567,7 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
         load_slice<WT>(xr, at(u), f, m2, live(u));
         quantize_slice<WT, SHORT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane, live(u));
     }
-    return bad ? __int_as_float(0x7FC00000) : __fdiv_rn(mx, kFixedOne);
+    return s;
 }
 
 // ---- per-format unit kernels -------------------------------------------------------------------------
@@ -1356,7 +1365,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // Programmatic dependent launch: the next kernel in the stream may become resident beside this one
     // (a CTA takes half an SM) as soon as every CTA here has passed this point; it prefetches weights
     // and waits for this grid to complete before touching activations or outputs.
-    if (!(p.tune & 2)) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     volatile int *gave_up = &sm->gave_up;
 
     if (warp == 0) {
@@ -1379,14 +1388,14 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         // the other warps wait here for the barriers (they arrive as they start); this warp does not wait
         asm volatile("bar.arrive 1, %0;" ::"r"(kThreads) : "memory");
         // A device-side table is the output of the kernel before this one: wait for that grid.
-        if (p.dev_table || (p.tune & 1)) asm volatile("griddepcontrol.wait;" ::: "memory");
-        const TableView tv = table_view(p);
+        if (p.dev_table) asm volatile("griddepcontrol.wait;" ::: "memory");
+        const TableView tv(p);
         walk(p, tv, tps, [](int) {}, [&](const StageInfo &s) {
             const int slot = s.slot;
             const uint32_t full = smem_u32(&sm->full[slot]), empty = smem_u32(&sm->empty[slot]);
             wait_phase(empty, s.phase ^ 1, gave_up, p.status);
             uint8_t *dst = stages + (size_t)slot * p.stage_bytes;
-            const uint8_t *src = tv.mat[s.mat].w + (size_t)s.row0 * p.row_bytes;
+            const uint8_t *src = tv.w(s.mat) + (size_t)s.row0 * p.row_bytes;
             if (p.use_tma) {
                 // the box is clipped where the matrix ends (rows past n_out, units past the row) and
                 // still signals its full size
@@ -1395,7 +1404,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     if (p.dev_table) {
                         // (a 64-bit division per stage, by the one lane that issues a copy per stage)
                         const int bank = s.mat % p.step;
-                        const int row_off = (int)((size_t)(tv.mat[s.mat].w - p.bank_base[bank]) / (size_t)p.row_bytes);
+                        const int row_off = (int)((size_t)(tv.w(s.mat) - p.bank_base[bank]) / (size_t)p.row_bytes);
                         tma_box(smem_u32(dst), &p.wmap[bank], row_off + s.row0, s.unit0 / p.tma_unit_div, full);
                     } else {
                         tma_box(smem_u32(dst), &p.wmap[s.mat], s.row0, s.unit0 / p.tma_unit_div, full);
@@ -1441,7 +1450,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     }
     asm volatile("bar.sync 1, %0;" ::"r"(kThreads) : "memory");
     if (p.dev_table) asm volatile("griddepcontrol.wait;" ::: "memory");
-    const TableView tv = table_view(p);
+    const TableView tv(p);
 
     if (warp == kEpilogueWarp) {
         // ===== epilogue warp =====
@@ -1481,8 +1490,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                                 const long long at = (long long)r * p.peer_row_stride + p.peer_offset + s.row0 + srow;
                                 for (int q = 0; q < p.n_peers; q++) p.peer_y[q][at] = v;
                             } else {
-                                const GemvMat &mat = tv.mat[p.step == 2 ? s.mat - 1 : s.mat];
-                                float *y = mat.y + (size_t)r * mat.n_out + s.row0 + srow;
+                                const int om = p.step == 2 ? s.mat - 1 : s.mat;
+                                float *y = tv.y(om) + (size_t)r * tv.n_out(om) + s.row0 + srow;
                                 const float gt = STACK ? sm->gate[sub][i][lane] : gate_reg[i];
                                 if (p.step == 2) v = __fmul_rn(__fdiv_rn(gt, __fadd_rn(1.0f, exp_as_host(-gt))), v);
                                 *y = p.accumulate ? __fadd_rn(*y, v) : v;
@@ -1577,15 +1586,18 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         if (lo >= hi) continue;
         const int m = e * p.step;
         const int r0 = (lo - tv.begin(e)) * p.gran;
-        const int r1 = min((int)tv.mat[m].n_out, (hi - tv.begin(e)) * p.gran);
-        if (tv.mat[m].x != prepared) {
+        const int r1 = min(tv.n_out(m), (hi - tv.begin(e)) * p.gran);
+        const float *x = tv.x(m);
+        if (x != prepared) {
             // x may be the output of the kernel before this one (and y its input): wait for that grid to
             // complete. Weights are never written by a kernel in flight, so the producer warp does not wait.
             if (prepared == nullptr) {
+                // (x to level 2 meanwhile, where it is coherent whoever still writes it)
+                for (int u = my_unit; u < p.units; u += kConsumerWarps)
+                    if (u * F::unit_values + lane * (F::unit_values / 32) < p.n_in)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(x + u * F::unit_values + lane * (F::unit_values / 32)));
                 asm volatile("griddepcontrol.wait;" ::: "memory");
-                if (p.tune & 2) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             }
-            const float *x = tv.mat[m].x;
             // (stacked tiles: every sub-tile prepares its own copy)
             auto prepare = [&](int r) {
                 return prepare_x_row<WT, RAG && block_size(WT) == 32>(x + (size_t)r * p.n_in, p, planes + (size_t)(r * 3) * plane_stride(p.n_in),
@@ -1651,7 +1663,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             uint32_t ragA = 0, ragB = 0;
             if (RAG || (WT == KRK_CUDA_Q2_K && p.ragged)) {
                 const int row = r0 + (tile / p.step) * stage_rows + kTileRows * my_sub + g;
-                const uintptr_t base = reinterpret_cast<uintptr_t>(tv.mat[m + tile % p.step].w);
+                const uintptr_t base = reinterpret_cast<uintptr_t>(tv.w(m + tile % p.step));
                 ragA = (uint32_t)((base + (size_t)row * p.row_bytes) & 15);
                 ragB = (uint32_t)((base + (size_t)(row + 8) * p.row_bytes) & 15);
             }
@@ -1881,11 +1893,6 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.tps = p.tps < 1 ? 1 : (p.tps > kMaxStack ? kMaxStack : p.tps);
     p.use_tma = 0;
     p.box_bytes = 0;
-    static const int tune = [] {
-        const char *e = std::getenv("KRK_CUDA_GEMV_TUNE");
-        return e ? std::atoi(e) : 0;
-    }();
-    p.tune = tune;
     p.unit_stride = F::unit_bytes;
     p.tma_unit_div = 1;
     if (want_tma && F::tma == 1 && !p.whole_tiles && !p.ragged) {
@@ -2086,12 +2093,13 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     if (!setup_launch<WT>(p, mats, n_mat, n_in, rows, silu_pair, &smem)) return 0;
     p.accumulate = accumulate;
     p.n_entries = 0;
-    int total = 0;
+    int total = 0, tiles = 0;
     for (int m = 0; m < n_mat; m += p.step) {
         if (mats[m].n_out > (1 << 30)) return 0;
         for (int j = 0; j < p.step; j++) p.mat[p.n_entries * p.step + j] = mats[m + j];
         p.gran_begin[p.n_entries] = total;
         total += (int)((mats[m].n_out + p.gran - 1) / p.gran);
+        tiles += (int)((mats[m].n_out + kTileRows * p.tps - 1) / (kTileRows * p.tps));
         p.n_entries++;
     }
     p.gran_begin[p.n_entries] = total;
@@ -2099,7 +2107,11 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     if (total == 0) return 1;
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
-    const int sms = sm_count() * ctas_per_sm<WT>(smem, p.rows);
+    // A launch whose tiles fit one to an SM takes one CTA per SM: a second would only cut tiles in two (both halves still
+    // cost a whole tile of MMAs), and the other half of the SM lets the next launch start early (Q8_0 2048x2048 3.92 ->
+    // 3.42 us, Q6_K 2048x6656 10.5 -> 8.1 us).
+    const int per_sm = tiles <= sm_count() ? 1 : ctas_per_sm<WT>(smem, p.rows);
+    const int sms = sm_count() * per_sm;
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
     p.gran_r = total % grid;
