@@ -12,6 +12,10 @@
 
 namespace krk_cuda {
 
+// krk_cuda_gemv_group for 1..8 activation rows per matrix ([rows][n_in] and [rows][n_out] each); krk_cuda_abi.cu.
+int gemv_group_rows(void *const host_y[], const void *const host_x[], const void *const host_w[], const int host_wt[],
+                    const int64_t host_n_out[], int64_t n_in, int n_mat, int rows, int fuse_silu_pair, void *stream);
+
 namespace {
 
 // The reference routes every HIP call through KRK_HIP(expr) -> hip_check, which logs and
@@ -150,20 +154,17 @@ bool CudaBackend::gemm_group(void *const out[], const void *x, const void *const
     if (silu_fused) *silu_fused = false;
     const bool fold = silu && n_mat >= 2 && n_out[0] == n_out[1] && !xs &&
                       (!wts || wts[0] == wts[1]);
-    if (rows == 1 && n_mat >= 1 && n_mat <= KRK_CUDA_MAX_GROUP) {
+    // (decode batches too: rows of a group share the launch, and with it its fixed cost, as one row does)
+    if (rows >= 1 && rows <= KRK_CUDA_MAX_ROWS && n_mat >= 1 && n_mat <= KRK_CUDA_MAX_GROUP) {
         const void *xv[KRK_CUDA_MAX_GROUP];
         int wtv[KRK_CUDA_MAX_GROUP];
         for (int m = 0; m < n_mat; m++) {
             xv[m] = xs ? xs[m] : x;
             wtv[m] = (int)(wts ? wts[m] : wt);
         }
-        int rc;
-        if (fold && n_mat == 2) {
-            rc = krk_cuda_gemv_group(out, xv, w, wtv, n_out, n_in, 2, 1, stream_);
-            if (rc == KRK_CUDA_OK && silu_fused) *silu_fused = true;
-        } else {
-            rc = krk_cuda_gemv_group(out, xv, w, wtv, n_out, n_in, n_mat, 0, stream_);
-        }
+        const bool pair = fold && n_mat == 2;
+        const int rc = gemv_group_rows(out, xv, w, wtv, n_out, n_in, n_mat, (int)rows, pair ? 1 : 0, stream_);
+        if (rc == KRK_CUDA_OK && pair && silu_fused) *silu_fused = true;
         if (rc != KRK_CUDA_OK) die("gemm_group", rc, n_out[0], n_in, rows, wtv[0]);
         return true;
     }

@@ -57,6 +57,17 @@ cudaError_t launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// The status of such a launch, counted.
+inline int launched(cudaError_t e) {
+    note_launch();
+    if (e != cudaSuccess) {
+        note_cuda_error(e);
+        (void)cudaGetLastError();
+        return KRK_CUDA_ELAUNCH;
+    }
+    return KRK_CUDA_OK;
+}
+
 // ---- geometry (src/quant.cpp:1805-1900) ----------------------------------------------
 
 __host__ __device__ constexpr int block_size(int wt) {

@@ -69,6 +69,43 @@ static int check_matmul_args(const void *y, const void *x, const void *w, int wt
     return KRK_CUDA_OK;
 }
 
+int gemv_group_rows(void *const host_y[], const void *const host_x[], const void *const host_w[], const int host_wt[],
+                    const int64_t host_n_out[], int64_t n_in, int n_mat, int rows, int fuse_silu_pair, void *stream) {
+    if (n_mat < 0 || n_mat > KRK_CUDA_MAX_GROUP || rows < 1 || rows > KRK_CUDA_MAX_ROWS) return KRK_CUDA_EARG;
+    if (n_mat == 0) return KRK_CUDA_OK;
+    if (!host_y || !host_x || !host_w || !host_wt || !host_n_out) return KRK_CUDA_ENULL;
+    if (fuse_silu_pair && (n_mat & 1)) return KRK_CUDA_EARG;
+    GemvMat mats[KRK_CUDA_MAX_GROUP];
+    for (int m = 0; m < n_mat; m++) {
+        const int rc = check_matmul_args(host_y[m], host_x[m], host_w[m], host_wt[m], host_n_out[m], n_in, rows);
+        if (rc != KRK_CUDA_OK) return rc;
+        if (fuse_silu_pair && (m & 1) &&
+            (host_n_out[m] != host_n_out[m - 1] || host_wt[m] != host_wt[m - 1] || host_x[m] != host_x[m - 1]))
+            return KRK_CUDA_EARG;
+        mats[m].w = static_cast<const uint8_t *>(host_w[m]);
+        mats[m].x = static_cast<const float *>(host_x[m]);
+        mats[m].y = static_cast<float *>(host_y[m]);
+        mats[m].n_out = host_n_out[m];
+        mats[m].wt = host_wt[m];
+    }
+    if (!device_state()) return KRK_CUDA_EDEVICE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // One launch per run of equal weight types (a pair of the silu fold never straddles two runs: its types are
+    // equal), each on the streaming kernel where it addresses the shape.
+    for (int first = 0; first < n_mat;) {
+        int last = first + 1;
+        while (last < n_mat && mats[last].wt == mats[first].wt) last++;
+        int rc = launch_gemv_stream(mats + first, last - first, n_in, rows, 0, fuse_silu_pair, st);
+        if (rc < 0) return rc;
+        if (rc == 0) {
+            rc = launch_gemv_generic(mats + first, last - first, n_in, rows, 0, fuse_silu_pair, st);
+            if (rc != KRK_CUDA_OK) return rc;
+        }
+        first = last;
+    }
+    return KRK_CUDA_OK;
+}
+
 } // namespace krk_cuda
 
 using namespace krk_cuda;
@@ -137,39 +174,7 @@ int krk_cuda_gemv(void *y_f32, const void *x_f32, const void *w, int wt, int64_t
 int krk_cuda_gemv_group(void *const host_y[], const void *const host_x[], const void *const host_w[],
                         const int host_wt[], const int64_t host_n_out[], int64_t n_in, int n_mat,
                         int fuse_silu_pair, void *stream) {
-    if (n_mat < 0 || n_mat > KRK_CUDA_MAX_GROUP) return KRK_CUDA_EARG;
-    if (n_mat == 0) return KRK_CUDA_OK;
-    if (!host_y || !host_x || !host_w || !host_wt || !host_n_out) return KRK_CUDA_ENULL;
-    if (fuse_silu_pair && (n_mat & 1)) return KRK_CUDA_EARG;
-    GemvMat mats[KRK_CUDA_MAX_GROUP];
-    for (int m = 0; m < n_mat; m++) {
-        const int rc = check_matmul_args(host_y[m], host_x[m], host_w[m], host_wt[m], host_n_out[m], n_in, 1);
-        if (rc != KRK_CUDA_OK) return rc;
-        if (fuse_silu_pair && (m & 1) &&
-            (host_n_out[m] != host_n_out[m - 1] || host_wt[m] != host_wt[m - 1] || host_x[m] != host_x[m - 1]))
-            return KRK_CUDA_EARG;
-        mats[m].w = static_cast<const uint8_t *>(host_w[m]);
-        mats[m].x = static_cast<const float *>(host_x[m]);
-        mats[m].y = static_cast<float *>(host_y[m]);
-        mats[m].n_out = host_n_out[m];
-        mats[m].wt = host_wt[m];
-    }
-    if (!device_state()) return KRK_CUDA_EDEVICE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // One launch per run of equal weight types (a pair of the silu fold never straddles two runs: its types are
-    // equal), each on the streaming kernel where it addresses the shape.
-    for (int first = 0; first < n_mat;) {
-        int last = first + 1;
-        while (last < n_mat && mats[last].wt == mats[first].wt) last++;
-        int rc = launch_gemv_stream(mats + first, last - first, n_in, 1, 0, fuse_silu_pair, st);
-        if (rc < 0) return rc;
-        if (rc == 0) {
-            rc = launch_gemv_generic(mats + first, last - first, n_in, 1, 0, fuse_silu_pair, st);
-            if (rc != KRK_CUDA_OK) return rc;
-        }
-        first = last;
-    }
-    return KRK_CUDA_OK;
+    return gemv_group_rows(host_y, host_x, host_w, host_wt, host_n_out, n_in, n_mat, 1, fuse_silu_pair, stream);
 }
 
 size_t krk_cuda_gemm_workspace_bytes(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows) {

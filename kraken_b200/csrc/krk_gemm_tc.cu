@@ -1303,14 +1303,7 @@ int launch_gemm_experts_down(float *y, const ExpertGemm &e, cudaStream_t st) {
 int launch_f32_to_f16(__half *out, const float *in, int64_t n, cudaStream_t st) {
     const int64_t want = (n / 4 + 255) / 256;
     const int grid = (int)(want < (int64_t)sm_count() * 8 ? want : (int64_t)sm_count() * 8);
-    const cudaError_t e = launch_overlapped(f32_to_f16_kernel, dim3((unsigned)grid), dim3(256), st, out, in, n / 4);
-    note_launch();
-    if (e != cudaSuccess) {
-        note_cuda_error(e);
-        (void)cudaGetLastError();
-        return KRK_CUDA_ELAUNCH;
-    }
-    return KRK_CUDA_OK;
+    return launched(launch_overlapped(f32_to_f16_kernel, dim3((unsigned)grid), dim3(256), st, out, in, n / 4));
 }
 
 size_t gemm_workspace_bytes(int x_dtype, int64_t, int64_t n_in, int64_t rows) {

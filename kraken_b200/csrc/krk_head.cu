@@ -9,11 +9,12 @@
 // key(i) = logits[i], clamped to +-softcap when softcap > 0, then divided (positive) or multiplied
 // (negative) by rep_pen where the token's bit is set in pen_mask; the k largest keys in descending order,
 // ties toward the lower id; ids past the row's length are -1 / -FLT_MAX; mass = sum over the whole row of
-// exp((key - max) / temp). Two kernels. Every block takes a 2048-key slice of the row: each of its 32 warps
-// pulls the k best of its own 64 keys out of registers (k rounds of a shuffle arg-max), one warp merges the
-// 32 sorted lists into the block's k best, and the slice's (max, sum of exp) is left beside them. One warp of
-// the second kernel merges the blocks' lists the same way and the sums are folded. No block-wide barrier
-// sits inside a round.
+// exp((key - max) / temp). Two kernels, both a radix select: four passes over 8-bit digits of the order-preserving
+// integer form of the keys find the k-th largest, everything above it (and the lowest ids among its equals) is
+// collected. Every block of the first kernel selects from its 2048-key slice of the row and leaves the slice's (max, sum
+// of exp); the one block of the second selects from the slices' candidates, ranks the k of them against each other and
+// folds the sums. What bounds it is latency: about a dozen barriers and two passes through level 2. (Pulling the k best
+// out one at a time, by warp arg-max and list merges, took 52 us at k = 40 on 128,256 logits.)
 #include "krk_common.cuh"
 
 #include <cfloat>
@@ -26,6 +27,8 @@ template <int WT>
 __global__ void __launch_bounds__(256)
 embed_kernel(float *__restrict__ out, const uint8_t *__restrict__ table, const int32_t *__restrict__ tokens,
              int64_t n_vocab, int64_t n_embd, int64_t n_tok, size_t rb) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t total = n_tok * n_embd;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t t = i / n_embd, k = i - t * n_embd;
@@ -34,9 +37,12 @@ embed_kernel(float *__restrict__ out, const uint8_t *__restrict__ table, const i
     }
 }
 
-constexpr int kTopkThreads = 1024;
+constexpr int kTopkThreads = 512;
 constexpr int kTopkMaxK = 64;
-constexpr int kTopkSlice = 2048;   // keys a block holds in shared memory
+constexpr int kTopkSlice = 2048;        // keys of a block of the first kernel
+constexpr int kTopkPer = kTopkSlice / kTopkThreads;
+constexpr int kMergeThreads = 1024;
+constexpr int kMergeHeld = 8192;        // candidates the second kernel keeps in shared memory
 
 struct TopkParams {
     const float *logits;
@@ -46,180 +52,253 @@ struct TopkParams {
     int k;
 };
 
+// A NaN key ranks last, as -infinity does.
 __device__ __forceinline__ float topk_key(const TopkParams &p, int64_t i) {
     float v = p.logits[i];
     if (p.softcap > 0.0f) v = v > p.softcap ? p.softcap : (v < -p.softcap ? -p.softcap : v);
     if (p.pen_mask && p.rep_pen > 0.0f && p.rep_pen != 1.0f && ((p.pen_mask[(uint32_t)i >> 5] >> ((uint32_t)i & 31)) & 1u))
         v = v > 0.0f ? __fdiv_rn(v, p.rep_pen) : __fmul_rn(v, p.rep_pen);
-    return v;
+    return v == v ? v : -INFINITY;
+}
+// Order-preserving unsigned form (both zeros alike); 0 is "nothing" and loses to every key, -infinity included.
+__device__ __forceinline__ uint32_t order(float v) {
+    const uint32_t b = __float_as_uint(v + 0.0f);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
 }
 
-// (value, id) order of the reference: larger value first, then lower id. "Nothing" is (-inf, INT_MAX): it
-// loses to every real element, a real -inf key included.
 constexpr int kNone = 0x7FFFFFFF;
-__device__ __forceinline__ bool better(float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); }
 
-__device__ __forceinline__ void warp_best(float &v, int &i) {
+// By a whole block: the k-th largest of the keys that `each(f)` hands to f (each thread its own; zeros are ignored), and
+// how many of its equals belong to the k largest. Fewer than k keys: threshold 0, nothing taken from its equals.
+template <class Each>
+__device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &threshold, int &of_equals) {
+    __shared__ int hist[256];
+    __shared__ uint32_t s_prefix;
+    __shared__ int s_left;
+    uint32_t prefix = 0u, mask = 0u;
+    int left = k;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
+        __syncthreads();
+        each([&](uint32_t u) {
+            if (u != 0u && (u & mask) == prefix) atomicAdd(&hist[(u >> shift) & 255u], 1);
+        });
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            // lane l holds bins 255 - 8l .. 248 - 8l, descending; the digit is where the running count reaches `left`
+            const int lane = threadIdx.x;
+            int c[8], sum = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        const int oi = __shfl_xor_sync(0xFFFFFFFFu, i, o);
-        if (better(ov, oi, v, i)) {
-            v = ov;
-            i = oi;
-        }
-    }
-}
-
-// One warp merges `n_lists` lists of `k` (value, id) pairs, each best first, into the k best overall, best
-// first: lane l looks after lists l, l + 32, ...; a round takes the best list head and advances that list.
-// head[] (one int per list) is scratch in shared memory.
-__device__ __forceinline__ void merge_lists(const float *lv, const int *li, int n_lists, int k, int *head, float *out_v,
-                                            int *out_i, int lane) {
-    for (int l = lane; l < n_lists; l += 32) head[l] = 0;
-    __syncwarp();
-    for (int r = 0; r < k; r++) {
-        float v = -INFINITY;
-        int i = kNone, from = -1;
-        for (int l = lane; l < n_lists; l += 32) {
-            const int h = head[l];
-            if (h < k) {
-                const float cv = lv[l * k + h];
-                const int ci = li[l * k + h];
-                if (better(cv, ci, v, i)) {
-                    v = cv;
-                    i = ci;
-                    from = l;
-                }
+            for (int j = 0; j < 8; j++) sum += c[j] = hist[255 - 8 * lane - j];
+            int above = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xFFFFFFFFu, above, o);
+                if (lane >= o) above += v;
+            }
+            const int total = __shfl_sync(0xFFFFFFFFu, above, 31);
+            above -= sum;
+            if (total < left) {   // (only in the first pass: fewer keys than k)
+                if (lane == 0) s_left = -1;
+            } else if (above < left && above + sum >= left) {
+                int j = 0;
+#pragma unroll
+                for (int q = 0; q < 7; q++)
+                    if (j == q && above + c[q] < left) {
+                        above += c[q];
+                        j++;
+                    }
+                s_prefix = prefix | ((uint32_t)(255 - 8 * lane - j) << shift);
+                s_left = left - above;
             }
         }
-        float bv = v;
-        int bi = i;
-        warp_best(bv, bi);
-        if (from >= 0 && i == bi && bi != kNone) head[from]++;   // ids are distinct: exactly one lane advances
-        if (lane == 0) {
-            out_v[r] = bv;
-            out_i[r] = bi;
+        __syncthreads();
+        left = s_left;
+        if (left < 0) {
+            threshold = 0u;
+            of_equals = 0;
+            return;
         }
-        __syncwarp();
+        prefix = s_prefix;
+        mask |= 255u << shift;
     }
+    threshold = prefix;
+    of_equals = left;
 }
 
-// cand_v / cand_i: [blocks][k] best first; part: [blocks][2] = (slice max, slice sum of exp((key - slice max) * inv_temp))
+// The selected of a block in shared memory, in no order: keys above the threshold, and of its equals the lowest ids.
+struct Selected {
+    uint32_t u[kTopkMaxK];
+    int id[kTopkMaxK];
+    int n, n_equal;
+};
+
+// cand_u / cand_i: [blocks][k] in no order; part: [blocks][2] = (slice max, slice sum of exp((key - slice max) * inv_temp))
 __global__ void __launch_bounds__(kTopkThreads)
-topk_slices_kernel(const __grid_constant__ TopkParams p, float *__restrict__ cand_v, int *__restrict__ cand_i,
+topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ cand_u, int *__restrict__ cand_i,
                    float *__restrict__ part) {
-    constexpr int kWarps = kTopkThreads / 32, kPerLane = kTopkSlice / kTopkThreads;
-    __shared__ float wl_v[kWarps * kTopkMaxK];   // every warp's k best of its 64 keys, best first
-    __shared__ int wl_i[kWarps * kTopkMaxK];
+    constexpr int kWarps = kTopkThreads / 32;
+    __shared__ Selected sel;
+    __shared__ int equal[kTopkSlice];
     __shared__ float red[kWarps];
-    __shared__ int head[kWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t per = (p.n + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = (int64_t)blockIdx.x * per, hi = min(p.n, lo + per);
-    const int cnt = (int)max((int64_t)0, hi - lo);
-    float v[kPerLane];
-    int id[kPerLane];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) sel.n = sel.n_equal = 0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t lo = (int64_t)blockIdx.x * kTopkSlice;
+    const int cnt = (int)min((int64_t)kTopkSlice, p.n - lo);
+    float v[kTopkPer];
+    uint32_t u[kTopkPer];
+#pragma unroll
+    for (int j = 0; j < kTopkPer; j++) {
+        const int i = j * kTopkThreads + tid;
+        v[j] = i < cnt ? topk_key(p, lo + i) : -INFINITY;
+        u[j] = i < cnt ? order(v[j]) : 0u;
+    }
     float mx = -FLT_MAX;
 #pragma unroll
-    for (int u = 0; u < kPerLane; u++) {
-        const int j = warp * (32 * kPerLane) + 32 * u + lane;
-        v[u] = -INFINITY;
-        id[u] = kNone;
-        if (j < cnt) {
-            float key = topk_key(p, lo + j);
-            if (!(key == key)) key = -INFINITY;   // a NaN key ranks last
-            v[u] = key;
-            id[u] = (int)(lo + j);
-            mx = fmaxf(mx, key);
-        }
-    }
-    // slice max and sum of exponentials for the mass
+    for (int j = 0; j < kTopkPer; j++) mx = fmaxf(mx, v[j]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
     if (lane == 0) red[warp] = mx;
-    __syncthreads();
+    uint32_t threshold;
+    int of_equals;
+    radix_select([&](auto &&f) {
+#pragma unroll
+        for (int j = 0; j < kTopkPer; j++) f(u[j]);
+    }, p.k, threshold, of_equals);   // (its barriers publish red[])
+    float sum = 0.0f;
     mx = red[0];
     for (int w = 1; w < kWarps; w++) mx = fmaxf(mx, red[w]);
     __syncthreads();
-    float sum = 0.0f;
 #pragma unroll
-    for (int u = 0; u < kPerLane; u++)
-        if (id[u] != kNone) sum += expf((v[u] - mx) * p.inv_temp);
+    for (int j = 0; j < kTopkPer; j++)
+        if (u[j] != 0u) sum += expf((v[j] - mx) * p.inv_temp);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
     if (lane == 0) red[warp] = sum;
+#pragma unroll
+    for (int j = 0; j < kTopkPer; j++) {
+        const int i = j * kTopkThreads + tid;
+        if (u[j] > threshold) {
+            const int at = atomicAdd(&sel.n, 1);
+            sel.u[at] = u[j];
+            sel.id[at] = (int)(lo + i);
+        } else if (u[j] == threshold && of_equals > 0) {
+            equal[atomicAdd(&sel.n_equal, 1)] = (int)(lo + i);
+        }
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    const int n_above = sel.n, n_equal = sel.n_equal;
+    for (int i = tid; i < n_equal; i += kTopkThreads) {
+        const int id = equal[i];
+        int rank = i;
+        if (n_equal > of_equals) {
+            rank = 0;
+            for (int q = 0; q < n_equal; q++) rank += equal[q] < id;
+        }
+        if (rank < of_equals) {
+            sel.u[n_above + rank] = threshold;
+            sel.id[n_above + rank] = id;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < p.k; i += kTopkThreads) {
+        const bool ok = i < n_above + of_equals;
+        cand_u[(size_t)blockIdx.x * p.k + i] = ok ? sel.u[i] : 0u;
+        cand_i[(size_t)blockIdx.x * p.k + i] = ok ? sel.id[i] : kNone;
+    }
+    if (tid == 0) {
         float s = 0.0f;
         for (int w = 0; w < kWarps; w++) s += red[w];
         part[2 * blockIdx.x] = mx;
-        part[2 * blockIdx.x + 1] = cnt > 0 ? s : 0.0f;
+        part[2 * blockIdx.x + 1] = s;
     }
-    // every warp: k rounds over its own keys (registers and shuffles only)
-    for (int r = 0; r < p.k; r++) {
-        float bv = -INFINITY;
-        int bi = kNone;
-#pragma unroll
-        for (int u = 0; u < kPerLane; u++)
-            if (better(v[u], id[u], bv, bi)) {
-                bv = v[u];
-                bi = id[u];
-            }
-        warp_best(bv, bi);
-#pragma unroll
-        for (int u = 0; u < kPerLane; u++)
-            if (id[u] == bi && bi != kNone) {   // struck
-                v[u] = -INFINITY;
-                id[u] = kNone;
-            }
-        if (lane == 0) {
-            wl_v[warp * p.k + r] = bv;
-            wl_i[warp * p.k + r] = bi;
-        }
-    }
-    __syncthreads();
-    // warp 0: the block's k best out of the warps' lists
-    if (warp == 0)
-        merge_lists(wl_v, wl_i, kWarps, p.k, head, cand_v + (size_t)blockIdx.x * p.k, cand_i + (size_t)blockIdx.x * p.k, lane);
 }
 
-__global__ void __launch_bounds__(256)
-topk_merge_kernel(const float *__restrict__ cand_v, const int *__restrict__ cand_i, const float *__restrict__ part,
-                  int n_blocks, int k, float inv_temp, int32_t *__restrict__ ids, float *__restrict__ vals,
+__global__ void __launch_bounds__(kMergeThreads)
+topk_merge_kernel(const __grid_constant__ TopkParams p, const uint32_t *__restrict__ cand_u, const int *__restrict__ cand_i,
+                  const float *__restrict__ part, int n_blocks, int32_t *__restrict__ ids, float *__restrict__ vals,
                   float *__restrict__ mass_out) {
-    extern __shared__ float sm_v[];                       // [n_blocks * k], then the ids, then one head per list
-    int *sm_i = reinterpret_cast<int *>(sm_v + (size_t)n_blocks * k);
-    int *head = sm_i + (size_t)n_blocks * k;
-    __shared__ float out_v[kTopkMaxK];
-    __shared__ int out_i[kTopkMaxK];
-    const int total = n_blocks * k;
-    for (int j = threadIdx.x; j < total; j += blockDim.x) {
-        sm_v[j] = cand_v[j];
-        sm_i[j] = cand_i[j];
+    __shared__ uint32_t held[kMergeHeld];
+    __shared__ Selected sel;
+    const int tid = threadIdx.x, lane = tid & 31, k = p.k;
+    if (tid == 0) sel.n = 0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t total = (int64_t)n_blocks * k;
+    const bool in_smem = total <= kMergeHeld;
+    if (in_smem)
+        for (int i = tid; i < (int)total; i += kMergeThreads) held[i] = cand_u[i];
+    if (mass_out && tid >= kMergeThreads - 32) {   // the last warp: the slices' sums
+        float mx = -FLT_MAX;
+        for (int b = lane; b < n_blocks; b += 32) mx = fmaxf(mx, part[2 * b]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        float m = 0.0f;
+        for (int b = lane; b < n_blocks; b += 32)
+            if (part[2 * b + 1] > 0.0f) m += part[2 * b + 1] * expf((part[2 * b] - mx) * p.inv_temp);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xFFFFFFFFu, m, o);
+        if (lane == 0) *mass_out = m;
     }
     __syncthreads();
-    if (threadIdx.x < 32) {
-        merge_lists(sm_v, sm_i, n_blocks, k, head, out_v, out_i, threadIdx.x);
-        for (int r = threadIdx.x; r < k; r += 32) {
-            const bool ok = out_i[r] != kNone;
-            ids[r] = ok ? out_i[r] : -1;
-            vals[r] = ok ? out_v[r] : -FLT_MAX;
+    auto each_at = [&](auto &&f) {
+        for (int64_t i = tid; i < total; i += kMergeThreads) f(in_smem ? held[i] : cand_u[i], i);
+    };
+    uint32_t threshold;
+    int of_equals;
+    radix_select([&](auto &&f) { each_at([&](uint32_t u, int64_t) { f(u); }); }, k, threshold, of_equals);
+    each_at([&](uint32_t u, int64_t i) {
+        if (u > threshold) {
+            const int at = atomicAdd(&sel.n, 1);
+            sel.u[at] = u;
+            sel.id[at] = cand_i[i];
         }
-    } else if (mass_out && threadIdx.x == 32) {
-        float mx = -FLT_MAX;
-        for (int b = 0; b < n_blocks; b++) mx = fmaxf(mx, part[2 * b]);
-        float m = 0.0f;
-        for (int b = 0; b < n_blocks; b++)
-            if (part[2 * b + 1] > 0.0f) m += part[2 * b + 1] * expf((part[2 * b] - mx) * inv_temp);
-        *mass_out = m;
+    });
+    __syncthreads();
+    int n_sel = sel.n;
+    // the equals of the threshold, lowest ids first: one at a time, each above the one before (rarely more than one)
+    int last = -1;
+    for (int q = 0; q < of_equals; q++) {
+        __shared__ int s_min;
+        if (tid == 0) s_min = kNone;
+        __syncthreads();
+        int best = kNone;
+        each_at([&](uint32_t u, int64_t i) {
+            if (u == threshold) {
+                const int id = cand_i[i];
+                if (id > last) best = min(best, id);
+            }
+        });
+        best = __reduce_min_sync(0xFFFFFFFFu, best);
+        if (lane == 0 && best != kNone) atomicMin(&s_min, best);
+        __syncthreads();
+        last = s_min;
+        if (tid == 0) {
+            sel.u[n_sel] = threshold;
+            sel.id[n_sel] = last;
+        }
+        n_sel++;
+        __syncthreads();
+    }
+    __syncthreads();
+    if (tid < k) {
+        if (tid < n_sel) {
+            const uint32_t u = sel.u[tid];
+            const int id = sel.id[tid];
+            int rank = 0;
+            for (int q = 0; q < n_sel; q++) rank += sel.u[q] > u || (sel.u[q] == u && sel.id[q] < id);
+            ids[rank] = id;
+            vals[rank] = topk_key(p, id);
+        } else {
+            ids[tid] = -1;
+            vals[tid] = -FLT_MAX;
+        }
     }
 }
 
-int topk_blocks(int64_t n) {
-    const int64_t need = (n + kTopkSlice - 1) / kTopkSlice;   // a slice must fit the block's shared memory
-    return (int)(need < 1 ? 1 : need);
-}
+int topk_blocks(int64_t n) { return (int)((n + kTopkSlice - 1) / kTopkSlice); }
 
 } // namespace
 
@@ -230,9 +309,9 @@ int launch_embed(float *out, const uint8_t *table, int wt, int64_t n_vocab, int6
     const int64_t want = (total + 255) / 256;
     const int grid = (int)(want < (int64_t)sm_count() * 16 ? want : (int64_t)sm_count() * 16);
     const size_t rb = row_bytes(wt, n_embd);
-    KRK_DISPATCH_WT(wt, embed_kernel<WT><<<grid, 256, 0, st>>>(out, table, tokens, n_vocab, n_embd, n_tok, rb));
-    note_launch();
-    return check_launch();
+    int rc = KRK_CUDA_EDTYPE;
+    KRK_DISPATCH_WT(wt, rc = launched(launch_overlapped(embed_kernel<WT>, dim3((unsigned)grid), dim3(256), st, out, table, tokens, n_vocab, n_embd, n_tok, rb)));
+    return rc;
 }
 
 size_t logits_topk_workspace_bytes(int64_t n, int k) {
@@ -243,10 +322,10 @@ size_t logits_topk_workspace_bytes(int64_t n, int k) {
 int launch_logits_topk(const float *logits, int64_t n, int k, const uint32_t *pen_mask, float rep_pen, float softcap,
                        float temp, int32_t *ids, float *vals, float *mass_out, void *workspace, cudaStream_t st) {
     if (k < 1 || k > kTopkMaxK || n < 1) return KRK_CUDA_EARG;
+    if (n > INT32_MAX) return KRK_CUDA_ESHAPE;   // ids are 32-bit
     const int blocks = topk_blocks(n);
-    if ((size_t)blocks * k * 8 + (size_t)blocks * 4 > 200 * 1024) return KRK_CUDA_ESHAPE;   // the merge holds every candidate in shared memory
-    float *cand_v = static_cast<float *>(workspace);
-    int *cand_i = reinterpret_cast<int *>(cand_v + (size_t)blocks * k);
+    uint32_t *cand_u = static_cast<uint32_t *>(workspace);
+    int *cand_i = reinterpret_cast<int *>(cand_u + (size_t)blocks * k);
     float *part = reinterpret_cast<float *>(cand_i + (size_t)blocks * k);
     TopkParams p;
     p.logits = logits;
@@ -256,22 +335,9 @@ int launch_logits_topk(const float *logits, int64_t n, int k, const uint32_t *pe
     p.inv_temp = temp > 0.0f ? 1.0f / temp : 1.0f;
     p.n = n;
     p.k = k;
-    topk_slices_kernel<<<blocks, kTopkThreads, 0, st>>>(p, cand_v, cand_i, part);
-    note_launch();
-    int rc = check_launch();
+    int rc = launched(launch_overlapped(topk_slices_kernel, dim3((unsigned)blocks), dim3(kTopkThreads), st, p, cand_u, cand_i, part));
     if (rc != KRK_CUDA_OK) return rc;
-    const size_t smem = (size_t)blocks * k * 8 + (size_t)blocks * 4;
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || !configured[dev])) {
-        if (cudaFuncSetAttribute(topk_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-            return KRK_CUDA_ELAUNCH;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    topk_merge_kernel<<<1, 256, smem, st>>>(cand_v, cand_i, part, blocks, k, p.inv_temp, ids, vals, mass_out);
-    note_launch();
-    return check_launch();
+    return launched(launch_overlapped(topk_merge_kernel, dim3(1), dim3(kMergeThreads), st, p, cand_u, cand_i, part, blocks, ids, vals, mass_out));
 }
 
 } // namespace krk_cuda

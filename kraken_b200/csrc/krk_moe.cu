@@ -656,16 +656,6 @@ size_t moe_workspace_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n_to
     return moe_float_bytes(bank, k, n_tok) + stream_table_bytes(2 * picks) + stream_table_bytes(picks);
 }
 
-static int launched(cudaError_t e) {
-    note_launch();
-    if (e != cudaSuccess) {
-        note_cuda_error(e);
-        (void)cudaGetLastError();
-        return KRK_CUDA_ELAUNCH;
-    }
-    return KRK_CUDA_OK;
-}
-
 static int launch_combine(const MoeParams &p, cudaStream_t st) {
     const int64_t n4 = p.n_embd / 4;
     return launched(launch_overlapped(moe_combine_kernel, dim3((unsigned)((n4 + kCombineThreads - 1) / kCombineThreads), (unsigned)p.n_tok),

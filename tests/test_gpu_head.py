@@ -122,3 +122,15 @@ def test_head_refusals(cuda):
                                   ws.data_ptr(), 8, None) == -6
     assert L.krk_cuda_embed(vals.data_ptr(), ws.data_ptr(), 99, 10, 256, ids.data_ptr(), 1, None) == -1
     assert L.krk_cuda_embed(vals.data_ptr(), ws.data_ptr(), synth.Q4_K, 10, 100, ids.data_ptr(), 1, None) == -2
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (63, 64), (2048, 64), (2049, 40), (4095, 2), (16385, 33), (300000, 64)])
+def test_topk_slice_edges(cuda, oracle, n, k):
+    """Rows around the slice size, candidates beyond what the merge holds in shared memory (300,000 at k = 64), both
+    zeros tied, runs of equals across a slice boundary and at the k-th place."""
+    lg = synth.normal(n, SEED, 60 + k) * 2.0
+    lg[::5] = np.float32(0.5)
+    lg[1::97] = -0.0
+    lg[2::97] = 0.0
+    check_topk(cuda, oracle, lg, k)
+    check_topk(cuda, oracle, np.minimum(lg, np.float32(0.25)), k)   # the top is one run of equals

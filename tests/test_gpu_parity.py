@@ -582,3 +582,36 @@ def test_gemv_stream_whole_blocks_not_super_blocks(cuda, oracle, wt):
     g, u = (oracle.gemm(x, w, wt, 200, 1056) for w in ws)
     want = g.astype(np.float64) / (1.0 + np.exp(-g.astype(np.float64))) * u
     assert np.abs(y.cpu().numpy() - want).max() <= 1e-4 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("wt,n_in", [(synth.Q4_K, 2048), (synth.Q6_K, 1280), (synth.Q8_0, 1056), (synth.Q8_0, 96)])
+@pytest.mark.parametrize("rows", [2, 3, 8])
+def test_backend_gemm_group_decode_batches(cuda, oracle, wt, n_in, rows):
+    """gemm_group over 2..8 activation rows: one launch per group, the gate/up fold per row (the warp-per-row kernel's
+    separate fold at K = 96)."""
+    be = cuda.Backend(0)
+    n_outs = (150, 150, 64)
+    ws = [synth.weights(wt, n, n_in, SEED + 400, stream=600 + i) for i, n in enumerate(n_outs)]
+    x = synth.activations(rows, n_in, SEED + 400)
+    d_x, d_w, d_y = be.alloc(x.nbytes), [be.alloc(w.nbytes) for w in ws], [be.alloc(rows * n * 4) for n in n_outs]
+    be.upload(d_x, x.ctypes.data, x.nbytes)
+    for d, w in zip(d_w, ws):
+        be.upload(d, w.ctypes.data, w.nbytes)
+    ref = [oracle.gemm(x, w, wt, w.shape[0], n_in, rows=rows, threads=4) for w in ws]
+    ran, fused = be.gemm_group(d_y, d_x, d_w, wt, list(n_outs), n_in, rows=rows)
+    assert ran and not fused
+    for i, n in enumerate(n_outs):
+        y = np.empty((rows, n), np.float32)
+        be.download(y.ctypes.data, d_y[i], y.nbytes)
+        ok, worst = bound_ok(y, ref[i], oracle.dequant_rows(ws[i], wt, n, n_in), x, GEMV_TOL)
+        assert ok, (i, worst)
+    ran, fused = be.gemm_group(d_y[:2], d_x, d_w[:2], wt, list(n_outs[:2]), n_in, rows=rows, silu=True)
+    assert ran and fused
+    h = np.empty((rows, n_outs[0]), np.float32)
+    be.download(h.ctypes.data, d_y[0], h.nbytes)
+    g = ref[0].astype(np.float64)
+    want = g / (1.0 + np.exp(-g)) * ref[1]
+    assert np.abs(h - want).max() <= 2e-4 * np.abs(want).max()   # the bound of the single-row fold
+    for p in [d_x] + d_w + d_y:
+        be.release(p)
+    be.close()
