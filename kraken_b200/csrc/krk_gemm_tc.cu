@@ -24,7 +24,7 @@
 //                at a time into a [token][weight row] staging buffer in shared memory, TMA stores of Y;
 //   warp 20      TMA producer of X tiles (cp.async.bulk.tensor.2d, each CTA loads its own copy);
 //   warp 21      TMA producer of the raw block columns;
-//   warp 22      TMEM allocation and issue of tcgen05.mma / tcgen05.commit.
+//   warps 22, 23 TMEM allocation and issue of tcgen05.mma / tcgen05.commit.
 // Tensor memory: columns 0..255 the accumulator (two of 128 columns when a tile has at most 128 tokens, so that
 // one is read out while the next tile is multiplied), 256..511 four A stages of 64 columns (two K steps each).
 //
@@ -101,8 +101,8 @@ struct WMaps {
 constexpr int kDecodeGroups = 2, kGroupThreads = 256;   // two decode threads per weight row in each group
 constexpr int kDecodeThreads = kDecodeGroups * kGroupThreads, kEpilogueThreads = 128;
 constexpr int kDecodeWarps = kDecodeThreads / 32, kEpilogueWarps = kEpilogueThreads / 32;
-constexpr int kXWarp = kDecodeWarps + kEpilogueWarps, kRawWarp = kXWarp + 1, kMmaWarp = kXWarp + 2;
-constexpr int kThreads = 32 * (kMmaWarp + 1);
+constexpr int kXWarp = kDecodeWarps + kEpilogueWarps, kRawWarp = kXWarp + 1, kMmaWarp = kXWarp + 2;   // two MMA warps
+constexpr int kThreads = 32 * (kMmaWarp + 2);
 constexpr int kTmemCols = 512, kTmemA = 256;
 constexpr int kYChunk = 32;            // tokens per TMA store of the read-out
 constexpr int kGroupBox = 32;          // tokens per X box of the expert kinds
@@ -118,6 +118,7 @@ struct GemmParams {
     int n_tiles_n, n_tiles_m;
     int row_bytes;
     int xk;              // K steps per X stage: 4, 2 or 1
+    int dual;            // 1: both MMA warps issue, super-blocks in turn, into an accumulator each
     int n_b, n_raw;      // ring depths (stages)
     int raw_off, y_off, bar_off;   // where the raw ring, the read-out buffers and the barriers start (the X ring starts at 0)
     int split;           // CTAs per cluster, each with a piece of K (1: no cluster)
@@ -202,16 +203,19 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 // new sum. Executed by a whole converged warp whose operands are all warp-uniform, issued by the lane `elected` picks:
 // with the operands in uniform registers a step issues in 80 cycles; from a one-lane branch the operands go through
 // per-lane registers first and a step takes 470-510 cycles whatever N is (608 at N = 256 against the pipe's 512).
-__device__ __forceinline__ void umma_f16_ts_step(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t first, uint32_t elected) {
-    asm volatile("{\n .reg .pred p, q, t;\n .reg .b64 b1, b2, b3;\n .reg .b32 a1, a2, a3;\n"
+// `b_lo` is the low half of the descriptor (16 K values are 2 units of its address field; the field cannot carry out of
+// it), `hi` the constant other half.
+__device__ __forceinline__ void umma_f16_ts_step(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t first, uint32_t elected) {
+    asm volatile("{\n .reg .pred p, q, t;\n .reg .b64 b0, b1, b2, b3;\n .reg .b32 a1, a2, a3, l1, l2, l3;\n"
                  " setp.eq.b32 p, %4, 0;\n setp.ne.b32 q, %6, 0;\n setp.eq.b32 t, 0, 0;\n"
-                 " add.s64 b1, %2, 2;\n add.s64 b2, %2, 4;\n add.s64 b3, %2, 6;\n"
+                 " add.s32 l1, %2, 2;\n add.s32 l2, %2, 4;\n add.s32 l3, %2, 6;\n"
+                 " mov.b64 b0, {%2, %7};\n mov.b64 b1, {l1, %7};\n mov.b64 b2, {l2, %7};\n mov.b64 b3, {l3, %7};\n"
                  " add.s32 a1, %1, 8;\n add.s32 a2, %1, 16;\n add.s32 a3, %1, 24;\n"
-                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %3, {%5, %5, %5, %5}, p;\n"
                  " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, {%5, %5, %5, %5}, t;\n"
                  " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, {%5, %5, %5, %5}, t;\n"
                  " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, {%5, %5, %5, %5}, t;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(first), "r"(0u), "r"(elected) : "memory");
+                 ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(first), "r"(0u), "r"(elected), "r"(hi) : "memory");
 }
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t e;
@@ -248,10 +252,9 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // start address >> 4 in bits 0-13, leading byte offset (unused for this layout) 1 in bits 16-29,
 // stride byte offset 1024 >> 4 (eight rows) in bits 32-45, descriptor version 1 in bits 46-47,
 // layout type 2 (SWIZZLE_128B) in bits 61-63.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+constexpr uint32_t kSmemDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+
 // Instruction descriptor, kind::f16: D f32 (bits 4-5 = 1), A and B f16 (0), both K-major (0),
 // N >> 3 in bits 17-22, M >> 4 in bits 24-28.
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
@@ -712,7 +715,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             mbar_init(smem_u32(&sm->raw_empty[s]), kDecodeWarps);
         }
         for (int s = 0; s < 2; s++) {
-            mbar_init(smem_u32(&sm->d_full[s]), 1);
+            mbar_init(smem_u32(&sm->d_full[s]), p.dual ? 2 : 1);
             mbar_init(smem_u32(&sm->d_empty[s]), kEpilogueThreads / 32);
         }
         sm->gave_up = 0;
@@ -731,7 +734,9 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (KIND != kDense) asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tmem_base = sm->tmem_base;
-    const int n_acc = p.tile_m <= kMaxTileM / 2 ? 2 : 1;   // accumulators in tensor memory
+    // Accumulators in tensor memory: a tile has one, or one per MMA warp; narrow tiles alternate between two sets.
+    const int n_acc = p.tile_m <= kMaxTileM / (p.dual ? 4 : 2) ? 2 : 1;
+    const int d_other = p.tile_m <= kMaxTileM / 4 ? 64 : 128;   // second accumulator of a tile, columns on from the first
 
     // this CTA's K steps: all, or its cluster rank's share in whole super-blocks
     const int k_blocks = (int)(p.n_in / 256), rank = (int)blockIdx.x % p.split;
@@ -796,8 +801,24 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         const int ew = warp - kDecodeWarps, et = tid - kDecodeThreads;
         const uint32_t lane_d = tmem_base + ((uint32_t)(32 * ew) << 16);
         const int my_row = tile_row<WT, KIND>(32 * ew + lane);
-        int ybuf = 0, da = 0;
+        int ybuf = 0, da = 0, first = 0;   // first: as in the MMA warps
         uint32_t ph = 0;
+        const int n_blk = kb1 - kb0;
+        // 32 tokens of the accumulator; of both, where two MMA warps shared the tile's super-blocks (of a single one, only one
+        // did anything)
+        auto read = [&](uint32_t addr, uint32_t (&v)[32]) {
+            if (!p.dual || n_blk == 1) {
+                tmem_ld32(addr + (p.dual && (first & 1) ? (uint32_t)d_other : 0u), v);
+                tmem_ld_wait();
+                return;
+            }
+            uint32_t w[32];
+            tmem_ld32(addr, v);
+            tmem_ld32(addr + (uint32_t)d_other, w);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+        };
         asm volatile("griddepcontrol.wait;" ::: "memory");
         while (iter.next(p, it)) {
             wait_phase(smem_u32(&sm->d_full[da]), ph, gave_up, p.status);
@@ -810,8 +831,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                 float *part = reinterpret_cast<float *>(smem);
                 for (int c0 = 0; c0 < tokens; c0 += kYChunk) {
                     uint32_t v[32];
-                    tmem_ld32(d_addr + (uint32_t)c0, v);
-                    tmem_ld_wait();
+                    read(d_addr + (uint32_t)c0, v);
 #pragma unroll
                     for (int j = 0; j < 32; j++)
                         if (c0 + j < tokens) part[(c0 + j) * kTileN + my_row] = __uint_as_float(v[j]);
@@ -820,8 +840,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             }
             for (int c0 = 0; c0 < tokens; c0 += kYChunk) {
                 uint32_t v[32];
-                tmem_ld32(d_addr + (uint32_t)c0, v);
-                tmem_ld_wait();
+                read(d_addr + (uint32_t)c0, v);
                 if (KIND == kDense && !p.y_tma) {   // a Y the tensor map cannot describe: straight out
                     const int64_t n = it.n0 + my_row, m_first = it.x_row + c0;
                     if (n < p.n_out) {
@@ -870,6 +889,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                 }
                 ybuf ^= 1;
             }
+            first += n_blk;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sm->d_empty[da]));   // the accumulator is free again
@@ -950,39 +970,45 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             }
         }
     } else {
-        // ===== MMA issuer: the whole warp walks the loop, one elected lane issues (see umma_f16_ts_step) =====
+        // ===== MMA issuers: the whole warp walks the loop, one elected lane issues (see umma_f16_ts_step). Their loop shares
+        // a scheduler with decode warps, and for narrow tiles its chain of waits, address arithmetic and commits is what
+        // a super-block takes (290 clocks a K step against 126 alone). So two warps take super-blocks in turn, each into
+        // an accumulator of its own, which the read-out adds. Every ring holds an even number of super-blocks (the A ring
+        // two), so that a warp meets each of its slots on every lap and a parity cannot be taken for that of the lap before. =====
+        const int who = warp - kMmaWarp, step = p.dual ? 2 : 1;
         const uint32_t elected = elect_one();
-        const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+        constexpr uint32_t tmem = 0;   // an allocation of all 512 columns starts at the first
         iter.n = __shfl_sync(0xFFFFFFFFu, iter.n, 0);
-        int sa = 0, sb = 0, da = 0;
+        const int per_blk = 4 / p.xk, n_blk = kb1 - kb0;   // X stages per super-block
+        int blk = who;                    // this warp's next super-block of the CTA's sequence
+        int first = 0;                    // the sequence number of the tile's first super-block
+        int sb = (who * per_blk) % p.n_b, sa = 2 * who, da = 0;
         uint32_t pa = 0, pb = 0, pd = 0;
-        while (iter.next(p, it)) {
+        while ((who == 0 || p.dual) && iter.next(p, it)) {
             const uint32_t idesc = instr_desc(kTileN, __shfl_sync(0xFFFFFFFFu, tile_tokens<KIND>(p, it), 0));
             wait_phase(smem_u32(&sm->d_empty[da]), pd ^ 1, gave_up, p.status);   // the epilogue has drained the accumulator
             tc_fence_after();
-            // A super-block at a time. This loop shares its scheduler with decode warps and is the critical path of narrow
-            // tiles: one X stage and one A stage are waited for and committed per several MMAs, both waits in flight
-            // together.
-            const int xmask = p.xk - 1;
-            for (int ks = ks0; ks < ks1; ks += 4) {
-                uint64_t bdesc = 0;
+            const uint32_t d_tmem = tmem + 128 * da + (who ? d_other : 0);
+            uint32_t fresh = 1u;
+            for (; blk < first + n_blk; blk += step) {
+                uint32_t b_lo = 0;
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const bool new_b = (j & xmask) == 0, new_a = (j & 1) == 0;
+                    const bool new_b = (j & (p.xk - 1)) == 0, new_a = (j & 1) == 0;
                     const uint32_t b_bar = smem_u32(&sm->b_full[sb]), a_bar = smem_u32(&sm->a_full[sa]);
-                    if (new_b) {
+                    if (new_b) {   // both waits in flight together
                         const bool okb = mbar_try_wait(b_bar, pb), oka = !new_a || mbar_try_wait(a_bar, pa);
                         if (!okb) wait_phase(b_bar, pb, gave_up, p.status);
                         if (!oka) wait_phase(a_bar, pa, gave_up, p.status);
                         tc_fence_after();
-                        bdesc = smem_desc(smem_u32(smem) + (uint32_t)(sb * b_stage));
+                        b_lo = smem_desc_lo(smem_u32(smem) + (uint32_t)(sb * b_stage));
                     } else if (new_a) {
                         wait_phase(a_bar, pa, gave_up, p.status);
                         tc_fence_after();
                     }
-                    umma_f16_ts_step(tmem + 128 * da, tmem + kTmemA + 64 * sa + 32 * (j & 1), bdesc, idesc, (j == 0 && ks == ks0) ? 1u : 0u, elected);
-                    bdesc += (uint32_t)b_bytes >> 4;
-                    if (((j + 1) & xmask) == 0) {
+                    umma_f16_ts_step(d_tmem, tmem + kTmemA + 64 * sa + 32 * (j & 1), b_lo, kSmemDescHi, idesc, j == 0 ? fresh : 0u, elected);
+                    b_lo += (uint32_t)b_bytes >> 4;
+                    if (((j + 1) & (p.xk - 1)) == 0) {
                         umma_commit(smem_u32(&sm->b_empty[sb]), elected);   // a stage is free once the MMAs that read it are done
                         if (++sb == p.n_b) {
                             sb = 0;
@@ -997,7 +1023,21 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                         }
                     }
                 }
+                fresh = 0u;
+                if (p.dual) {   // past the other warp's super-block
+                    sb += per_blk;
+                    if (sb >= p.n_b) {
+                        sb -= p.n_b;
+                        pb ^= 1;
+                    }
+                    sa += 2;
+                    if (sa >= kAStages) {
+                        sa -= kAStages;
+                        pa ^= 1;
+                    }
+                }
             }
+            first += n_blk;
             umma_commit(smem_u32(&sm->d_full[da]), elected);
             if (++da == n_acc) {
                 da = 0;
@@ -1111,14 +1151,16 @@ size_t layout(GemmParams &p) {
     const int xb = p.tile_m * 128 * p.xk;
     const int y_bytes = 2 * kYChunk * kTileN * (int)sizeof(float);
     const int room = kSmemMax - 1024 - y_bytes - (int)sizeof(GemmBars);
-    p.n_b = kMinB / p.xk > 2 ? kMinB / p.xk : 2;
+    p.dual = p.tile_m <= kMaxTileM / 2;
+    const int unit_b = p.dual ? 2 * (4 / p.xk) : 1;   // the X ring grows by this many stages (see the MMA warps)
+    p.n_b = p.dual ? unit_b : kMinB;
     p.n_raw = kMinRaw;
     for (;;) {
         const int left = room - p.n_b * xb - p.n_raw * stage;
-        const bool want_b = p.n_b < kMaxB && p.n_b * p.xk < steps * p.n_raw;
-        if (want_b && left >= xb) p.n_b++;
+        const bool want_b = p.n_b + unit_b <= kMaxB && p.n_b * p.xk < steps * p.n_raw;
+        if (want_b && left >= unit_b * xb) p.n_b += unit_b;
         else if (p.n_raw < kMaxRaw && left >= stage) p.n_raw++;
-        else if (p.n_b < kMaxB && left >= xb) p.n_b++;
+        else if (p.n_b + unit_b <= kMaxB && left >= unit_b * xb) p.n_b += unit_b;
         else break;
     }
     p.raw_off = p.n_b * xb;
