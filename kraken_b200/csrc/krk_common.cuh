@@ -303,8 +303,9 @@ struct StreamBanks {
 // shape-agnostic kernels serve them.)
 bool stream_takes(int wt, int64_t n_in, int rows);
 // The streaming kernel over a device-side table (`rows` activation rows per matrix; all matrices of type wt and shape
-// n_out x n_in). Returns 1 when launched, 0 when the shape is not addressed, < 0 on error.
-int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
+// n_out x n_in). x_rows (device memory, [entries][rows], or null): which rows of its x are an entry's activation rows, else
+// the first ones. Returns 1 when launched, 0 when the shape is not addressed, < 0 on error.
+int launch_gemv_stream_table(const StreamTable *table, const int32_t *x_rows, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
                              const StreamBanks *banks, cudaStream_t st);
 
 int launch_silu_mul(float *out, const float *gate, const float *up, int64_t n, cudaStream_t st);

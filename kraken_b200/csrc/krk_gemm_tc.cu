@@ -1145,13 +1145,15 @@ bool encode_w_maps(CUtensorMap *maps, const uint8_t *w, int64_t n_out, int row_b
 // Ring depths and the shared-memory map of a launch. The raw ring wants as many K steps in flight as the X ring;
 // both grow in turn while they fit.
 template <int WT>
-size_t layout(GemmParams &p) {
+size_t layout(GemmParams &p, bool one_tile) {   // one_tile: no CTA has a second one
     const int stage = kTileN * raw_seg(WT), steps = Raw<WT>::kSteps;
     p.xk = p.tile_m <= 64 ? 4 : p.tile_m <= 128 ? 2 : 1;   // X stages of at most 32 KB
     const int xb = p.tile_m * 128 * p.xk;
     const int y_bytes = 2 * kYChunk * kTileN * (int)sizeof(float);
     const int room = kSmemMax - 1024 - y_bytes - (int)sizeof(GemmBars);
-    p.dual = p.tile_m <= kMaxTileM / 2;
+    // Tiles of 65..128 tokens have room for two accumulators only: for two MMA warps, or for the read-out beside the next
+    // tile, which is worth more where a CTA has several tiles of short K (Q8_0 experts of K = 2048: 34.7 against 40.8 us).
+    p.dual = p.tile_m <= kMaxTileM / 4 || (p.tile_m <= kMaxTileM / 2 && p.n_in >= (one_tile ? 2048 : 4096));
     const int unit_b = p.dual ? 2 * (4 / p.xk) : 1;   // the X ring grows by this many stages (see the MMA warps)
     p.n_b = p.dual ? unit_b : kMinB;
     p.n_raw = kMinRaw;
@@ -1252,7 +1254,7 @@ template <int WT>
 int launch_dense(GemmParams &p, const GemmPlan &g, const uint8_t *w, const __half *xh, cudaStream_t st, const float *x_f32) {
     CUtensorMap x_map, y_map;
     WMaps<kDense> w_maps;
-    const size_t smem = layout<WT>(p);
+    const size_t smem = layout<WT>(p, (long long)g.n_tiles_n * g.n_tiles_m * g.split <= g.grid);
     if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.n_in, p.rows, (size_t)p.n_in * sizeof(__half), kBK, p.tile_m,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !encode_w_maps<WT>(w_maps.m, w, p.n_out, p.row_bytes, kTileN))
@@ -1299,7 +1301,7 @@ int launch_experts(GemmParams &p, const ExpertGemm &e, cudaStream_t st) {
     WMaps<KIND> w_maps;
     constexpr int kRows = KIND == kGateUp ? kTileN / 2 : kTileN;   // rows of one matrix in a weight tile
     p.row_bytes = (int)row_bytes(WT, e.n_in);
-    const size_t smem = layout<WT>(p);
+    const size_t smem = layout<WT>(p, false);
     if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, e.x, e.n_in, e.x_rows, (size_t)e.n_in * sizeof(__half), kBK, kGroupBox,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !encode_w_maps<WT>(w_maps.m, e.w, e.bank_rows, p.row_bytes, kRows) ||

@@ -44,10 +44,10 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
     return rc;
 }
 
-int launch_gemv_stream_table(const StreamTable *table, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
+int launch_gemv_stream_table(const StreamTable *table, const int32_t *x_rows, int wt, int64_t n_out, int64_t n_in, int rows, int silu_pair,
                              const StreamBanks *banks, cudaStream_t st) {
     int rc = 0;
-    KRK_DISPATCH_WT(wt, rc = stream::launch_table_fmt<WT>(table, n_out, n_in, rows, silu_pair, banks, st));
+    KRK_DISPATCH_WT(wt, rc = stream::launch_table_fmt<WT>(table, x_rows, n_out, n_in, rows, silu_pair, banks, st));
     return rc;
 }
 

@@ -122,6 +122,7 @@ struct StreamParams {
     int total_gran;
     int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
     const StreamTable *dev_table;   // when set, the matrices come from device memory
+    const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
     int entry_gran;       // table launches: granules of every entry (all have one shape)
     int *status;
     int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
@@ -1548,6 +1549,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const int grp = kGroups == 1 ? 0 : (warp - 1) / kConsumerWarps;   // consumer group: takes tiles grp, grp + 2, ...
     const int wid = warp - 1 - grp * kConsumerWarps, g = lane >> 2, t = lane & 3;
     const float *prepared = nullptr;
+    int prepared_row = 0;
     const int8_t *bp[NG], *sp[NG];
     const float *fe[NG], *fo[NG];   // Q5_1: per-block sums of the even / odd activation row of each column group
     float xs[2 * NG];   // this warp's scale of each activation row (kFold: of its own rows, xs[0] and xs[1])
@@ -1588,7 +1590,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         const int r0 = (lo - tv.begin(e)) * p.gran;
         const int r1 = min(tv.n_out(m), (hi - tv.begin(e)) * p.gran);
         const float *x = tv.x(m);
-        if (x != prepared) {
+        // lane r: which row of x is activation row r
+        const bool picked = !SINGLE && p.table_rows;
+        const int my_row = picked && lane < p.rows ? p.table_rows[e * p.rows + lane] : lane;
+        if (x != prepared || (picked && __any_sync(0xFFFFFFFFu, my_row != prepared_row))) {
             // x may be the output of the kernel before this one (and y its input): wait for that grid to
             // complete. Weights are never written by a kernel in flight, so the producer warp does not wait.
             if (prepared == nullptr) {
@@ -1600,7 +1605,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             // (stacked tiles: every sub-tile prepares its own copy)
             auto prepare = [&](int r) {
-                return prepare_x_row<WT, RAG && block_size(WT) == 32>(x + (size_t)r * p.n_in, p, planes + (size_t)(r * 3) * plane_stride(p.n_in),
+                return prepare_x_row<WT, RAG && block_size(WT) == 32>(x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in), p, planes + (size_t)(r * 3) * plane_stride(p.n_in),
                                                                       chunk_sum + (size_t)(r * 4) * (p.n_in >> kSumShift<WT>),
                                                                       stacked_idle ? p.units : my_unit, lane);
             };
@@ -1625,6 +1630,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             if (kFold && NG == 1) xs[0] = t < 2 ? xs[0] : xs[1];
             prepared = x;
+            prepared_row = my_row;
             if (!SINGLE) lane_planes<NG, kFold>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
@@ -1870,6 +1876,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.ragged = 0;
     p.gran = 1;
     p.dev_table = nullptr;
+    p.table_rows = nullptr;
     p.entry_gran = 0;
     p.n_peers = 0;
     p.my_rank = p.epoch = 0;
@@ -2120,7 +2127,7 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
 }
 
 template <int WT>
-int launch_table_fmt(const StreamTable *table, int64_t n_out, int64_t n_in, int rows, int silu_pair, const StreamBanks *banks, cudaStream_t st) {
+int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_out, int64_t n_in, int rows, int silu_pair, const StreamBanks *banks, cudaStream_t st) {
     StreamParams p;
     size_t smem = 0;
     // With the banks known, a stage arrives as one tensor copy out of the bank's map.
@@ -2140,6 +2147,7 @@ int launch_table_fmt(const StreamTable *table, int64_t n_out, int64_t n_in, int 
     p.total_gran = 0;
     p.gran_q = p.gran_r = 0;
     p.dev_table = table;
+    p.table_rows = x_rows;
     p.entry_gran = (int)((n_out + p.gran - 1) / p.gran);
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
@@ -2189,7 +2197,7 @@ bool takes_fmt(int64_t n_in, int rows) {
 
 #define KRK_STREAM_FORMAT(LINKAGE, WT)                                                                                                  \
     LINKAGE template int launch_fmt<WT>(const GemvMat *, int, int64_t, int, int, int, cudaStream_t);                                    \
-    LINKAGE template int launch_table_fmt<WT>(const StreamTable *, int64_t, int64_t, int, int, const StreamBanks *, cudaStream_t);      \
+    LINKAGE template int launch_table_fmt<WT>(const StreamTable *, const int32_t *, int64_t, int64_t, int, int, const StreamBanks *, cudaStream_t); \
     LINKAGE template int launch_peers_fmt<WT>(const GemvMat &, int64_t, int, const PeerScatter &, cudaStream_t);                        \
     LINKAGE template bool takes_fmt<WT>(int64_t, int);
 

@@ -1,4 +1,4 @@
-// Router and routed-expert FFN for decode batches (1..8 tokens).
+// Router and routed-expert FFN: one token, decode batches and prefill.
 //
 // The routing result stays on the device: expert ids are read by the kernels themselves,
 // so no logits or ids cross PCIe (the reference downloads the logits and routes on the
@@ -391,34 +391,37 @@ moe_plan_kernel(const __grid_constant__ MoeParams p, StreamTable *gate_up, Strea
     if (threadIdx.x == 0) gate_up->n_entries = down->n_entries = n;
 }
 
-// ---- more than eight tokens ----------------------------------------------------------------------------------
+// ---- more than one token ------------------------------------------------------------------------------------
 // Expert-major (the reference's grouped form, src/engine.cpp:12353-12690), planned and run on the device without the
 // host ever seeing the counts. Experts that more than kFewRows tokens picked run on the tensor cores: their tokens'
 // rows are gathered into one f16 block, groups of up to tile_m rows of it are the token tiles of the expert GEMMs.
-// Experts with fewer rows keep f32 activations on the streaming kernel: one table per capacity class (rows are
-// padded to the class, so that one launch serves all experts of a class). A launch over an empty list or table ends
-// at once; the host picks the classes from the expected rows per expert, so that few of them are empty.
+// Experts with fewer rows keep f32 activations on the streaming kernel, `cap` rows of an expert per table entry, so
+// that an expert's weights are streamed once per `cap` of its tokens (entries of one expert are neighbours: a second
+// read comes from level 2). One table, one launch: the host picks `cap` from the expected rows per expert.
 constexpr int kFewRows = KRK_CUDA_MAX_ROWS;
-constexpr int kMaxClasses = 4;
+constexpr int kRouteFloats = kMaxExperts * kFewRows;   // router probabilities that fit beside the plan
 struct GroupedParams {
     const uint8_t *gate, *up, *down;
     size_t rb_gate_up, rb_down;
     int wt_gate_up, wt_down;
     const float *x;        // [n_tok][n_embd]
     const int32_t *ids;    // [n_tok][k]
+    const float *wts;      // [n_tok][k]
+    const float *logits;   // set: the routing runs first and writes ids and wts ([n_tok][n_expert], at most kRouteFloats)
+    int n_expert;
     int64_t n_embd, n_ff;
-    int n_local, expert_base, k, n_tok, tile_m;
-    int n_class, cap[kMaxClasses];        // rows per expert of each class, ascending, the last kFewRows
-    int *n_groups;
+    int n_local, expert_base, k, n_tok, tile_m, cap, cap_log2;
+    int *n_groups;         // null (no tensor-core experts): at most kFewRows tokens
     GemmGroup *groups;
-    StreamTable *table_gu[kMaxClasses], *table_dn[kMaxClasses];
+    StreamTable *table_gu, *table_dn;
+    int32_t *x_rows;       // [entries][cap]: the tokens of an entry (cap 1: the entry's own x pointer says it)
     __half *xg;            // [picks][n_embd]: gathered rows of the tensor-core experts
-    float *xs, *hs;        // [rows][n_embd], [rows][n_ff]: the few-row experts' activations
-    float *d;              // [picks + rows][n_embd]: down projections, tensor-core rows first
+    float *hs;             // [entries * cap][n_ff]
+    float *d;              // [picks + entries * cap][n_embd]: down projections, tensor-core rows first
     int32_t *pos;          // [n_tok][k]: a pick's row of d (-1: held elsewhere)
 };
 
-// Exclusive sum over the block's 1024 threads; `total` is the sum of all.
+// Exclusive sum over the block's threads (whole warps); `total` is the sum of all.
 __device__ __forceinline__ int block_scan(int v, int *warp_sums, int &total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int inc = v;
@@ -430,7 +433,7 @@ __device__ __forceinline__ int block_scan(int v, int *warp_sums, int &total) {
     __syncthreads();   // the sums of the scan before are read
     if (lane == 31) warp_sums[warp] = inc;
     __syncthreads();
-    const int w = warp_sums[lane];
+    const int w = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0;
     int winc = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -441,103 +444,117 @@ __device__ __forceinline__ int block_scan(int v, int *warp_sums, int &total) {
     return inc - v + __shfl_sync(0xFFFFFFFFu, winc - w, warp);
 }
 
-// One block; thread e looks after expert e. Picks take places in their expert's rows through shared-memory counters;
-// the few-row experts' picks are then put in token order (a row's place decides which limb columns it rides in, and
-// with them the rounding order of its sums; a tensor-core row's place changes nothing).
+// One block of at least n_local threads; thread e looks after expert e, and after the picks e, e + blockDim, ... Picks
+// take places in their expert's rows through shared-memory counters; a few-row expert's picks are then put in token order
+// (a row's place decides which limb columns it rides in, and with them the rounding order of its sums; a tensor-core
+// row's place changes nothing). What a call of few tokens costs here is latency, so nothing is read back from global
+// memory: the ids come out of the routing's shared copy, a thread's first pick stays in registers.
+constexpr int kPlanIds = 1024;
 __global__ void __launch_bounds__(kMaxExperts)
 moe_group_plan_kernel(const __grid_constant__ GroupedParams p) {
-    __shared__ int cnt[kMaxExperts], base[kMaxExperts], list[kMaxExperts * kFewRows], warp_sums[32];
+    __shared__ int cnt[kMaxExperts], base[kMaxExperts], sid[kPlanIds], warp_sums[32];
+    __shared__ union {
+        float prob[kRouteFloats];
+        int list[kMaxExperts * kFewRows];
+    } u;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int e = threadIdx.x, n_pick = p.n_tok * p.k;
     cnt[e] = 0;
+    if (p.logits) {   // a warp per token (n_pick <= kPlanIds: up to 32 tokens of up to 32 picks)
+        for (int t = e >> 5; t < p.n_tok; t += blockDim.x >> 5)
+            route_token(const_cast<int32_t *>(p.ids) + t * p.k, const_cast<float *>(p.wts) + t * p.k, p.logits + (int64_t)t * p.n_expert,
+                        p.n_expert, p.k, u.prob + t * p.n_expert, sid + t * p.k, e & 31);
+    }
     __syncthreads();
-    for (int i = e; i < n_pick; i += kMaxExperts) {
-        const int le = p.ids[i] - p.expert_base;
-        if (le >= 0 && le < p.n_local) atomicAdd(&cnt[le], 1);
+    auto local = [&](int i) {   // pick i's expert in the bank, or -1
+        const int le = (p.logits ? sid[i] : p.ids[i]) - p.expert_base;
+        return le >= 0 && le < p.n_local ? le : -1;
+    };
+    const int le0 = e < n_pick ? local(e) : -1;
+    const int slot0 = le0 >= 0 ? atomicAdd(&cnt[le0], 1) : 0;
+    for (int i = e + blockDim.x; i < n_pick; i += blockDim.x) {
+        const int le = local(i);
+        if (le >= 0) p.pos[i] = atomicAdd(&cnt[le], 1);   // its place, until the pass below
     }
     __syncthreads();
     const int m = cnt[e];
-    const bool few = m > 0 && m <= kFewRows, many = m > kFewRows;
-    int cls = 0;
-    while (cls + 1 < p.n_class && p.cap[cls] < m) cls++;
-    int total;
-    const int many_off = block_scan(many ? m : 0, warp_sums, total);
-    const int group_off = block_scan(many ? (m + p.tile_m - 1) / p.tile_m : 0, warp_sums, total);
-    if (e == 0) *p.n_groups = total;
-    const int few_off = block_scan(few ? p.cap[cls] : 0, warp_sums, total);
-    for (int c = 0; c < p.n_class; c++) {
-        const int at = block_scan(few && cls == c, warp_sums, total);
-        if (e == 0) p.table_gu[c]->n_entries = p.table_dn[c]->n_entries = total;
-        if (few && cls == c) {
-            GemvMat g, u, d;
-            g.w = p.gate + (size_t)e * p.n_ff * p.rb_gate_up;
-            u.w = p.up + (size_t)e * p.n_ff * p.rb_gate_up;
-            g.x = u.x = p.xs + (int64_t)few_off * p.n_embd;
-            g.y = u.y = p.hs + (int64_t)few_off * p.n_ff;   // the pair's fold writes silu(gate) * up through the gate's pointer
-            g.n_out = u.n_out = p.n_ff;
-            g.wt = u.wt = p.wt_gate_up;
-            d.w = p.down + (size_t)e * p.n_embd * p.rb_down;
-            d.x = g.y;
-            d.y = p.d + (int64_t)(n_pick + few_off) * p.n_embd;
-            d.n_out = p.n_embd;
-            d.wt = p.wt_down;
-            p.table_gu[c]->mat[2 * at] = g;
-            p.table_gu[c]->mat[2 * at + 1] = u;
-            p.table_dn[c]->mat[at] = d;
-        }
+    const bool many = p.n_groups && m > kFewRows, few = m > 0 && !many;   // (ids of the caller may repeat within a token)
+    const int n_ent = few ? (m + p.cap - 1) >> p.cap_log2 : 0;
+    int total, many_off = 0;
+    if (p.n_groups) {
+        many_off = block_scan(many ? m : 0, warp_sums, total);
+        const int group_off = block_scan(many ? (m + p.tile_m - 1) / p.tile_m : 0, warp_sums, total);
+        if (e == 0) *p.n_groups = total;
+        if (many)
+            for (int g = 0; g * p.tile_m < m; g++) p.groups[group_off + g] = GemmGroup{e, many_off + g * p.tile_m, min(p.tile_m, m - g * p.tile_m)};
     }
-    if (many)
-        for (int g = 0; g * p.tile_m < m; g++) p.groups[group_off + g] = GemmGroup{e, many_off + g * p.tile_m, min(p.tile_m, m - g * p.tile_m)};
-    base[e] = many ? many_off : n_pick + few_off;
-    cnt[e] = 0;
+    const int ent0 = block_scan(n_ent, warp_sums, total);
+    if (e == 0) p.table_gu->n_entries = p.table_dn->n_entries = total;
+    base[e] = many ? many_off : n_pick + ent0 * p.cap;
     __syncthreads();
-    for (int i = e; i < n_pick; i += kMaxExperts) {
-        const int le = p.ids[i] - p.expert_base;
-        if (le < 0 || le >= p.n_local) {
+    for (int i = e; i < n_pick; i += blockDim.x) {
+        const int le = i == e ? le0 : local(i);
+        if (le < 0) {
             p.pos[i] = -1;
             continue;
         }
-        const int slot = atomicAdd(&cnt[le], 1), b = base[le];
+        const int slot = i == e ? slot0 : p.pos[i], b = base[le];
         if (b < n_pick) p.pos[i] = b + slot;
-        else list[le * kFewRows + slot] = i;
+        else u.list[b - n_pick + slot] = i;
     }
     __syncthreads();
-    if (few) {
-        int *mine = list + e * kFewRows;
-        for (int i = 1; i < m; i++) {
-            const int v = mine[i];
-            int j = i;
-            for (; j > 0 && mine[j - 1] > v; j--) mine[j] = mine[j - 1];
-            mine[j] = v;
+    for (int i = e; i < n_pick; i += blockDim.x) {
+        const int le = i == e ? le0 : local(i);
+        if (le < 0 || base[le] < n_pick) continue;
+        const int row0 = base[le] - n_pick, n = cnt[le], token = i / p.k;
+        int rank = 0;
+        for (int q = 0; q < n; q++) rank += u.list[row0 + q] < i;
+        const int row = row0 + rank;
+        p.pos[i] = n_pick + row;
+        if (p.cap > 1) {   // (rows past the expert's last repeat it; nobody reads what they give)
+            p.x_rows[row] = token;
+            if (rank == n - 1)
+                for (int q = row + 1; q & (p.cap - 1); q++) p.x_rows[q] = token;
         }
-        for (int i = 0; i < m; i++) p.pos[mine[i]] = base[e] + i;
+        if ((rank & (p.cap - 1)) == 0) {   // the first pick of an entry writes it
+            const int ent = row >> p.cap_log2;
+            GemvMat g, up, d;
+            g.w = p.gate + (size_t)le * p.n_ff * p.rb_gate_up;
+            up.w = p.up + (size_t)le * p.n_ff * p.rb_gate_up;
+            g.x = up.x = p.x + (p.cap > 1 ? 0 : (int64_t)token * p.n_embd);
+            g.y = up.y = p.hs + (int64_t)row * p.n_ff;   // the pair's fold writes silu(gate) * up through the gate's pointer
+            g.n_out = up.n_out = p.n_ff;
+            g.wt = up.wt = p.wt_gate_up;
+            d.w = p.down + (size_t)le * p.n_embd * p.rb_down;
+            d.x = g.y;
+            d.y = p.d + (int64_t)(n_pick + row) * p.n_embd;
+            d.n_out = p.n_embd;
+            d.wt = p.wt_down;
+            p.table_gu->mat[2 * ent] = g;
+            p.table_gu->mat[2 * ent + 1] = up;
+            p.table_dn->mat[ent] = d;
+        }
     }
 }
 
-// Every pick's activation row to its place: f16 for the tensor-core experts (rounded as the dense GEMM rounds f32
-// activations), f32 for the others. One block per pick; a token's row comes out of L2 for all picks but the first.
+// The activation rows of the tensor-core experts' picks to their places as f16, rounded as the dense GEMM rounds f32
+// activations. One block per pick; a token's row comes out of L2 for all picks but the first.
 constexpr int kGatherThreads = 128;
 __global__ void __launch_bounds__(kGatherThreads)
 moe_gather_kernel(const __grid_constant__ GroupedParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int pick = blockIdx.x, row = p.pos[pick], n_pick = p.n_tok * p.k;
-    if (row < 0) return;
+    if (row < 0 || row >= n_pick) return;
     const float4 *src = reinterpret_cast<const float4 *>(p.x + (int64_t)(pick / p.k) * p.n_embd);
     const int n4 = (int)(p.n_embd >> 2);
-    if (row < n_pick) {
-        uint2 *dst = reinterpret_cast<uint2 *>(p.xg + (int64_t)row * p.n_embd);
+    uint2 *dst = reinterpret_cast<uint2 *>(p.xg + (int64_t)row * p.n_embd);
 #pragma unroll 4
-        for (int j = threadIdx.x; j < n4; j += kGatherThreads) {
-            const float4 v = src[j];
-            const __half2 a = __halves2half2(half_sat(v.x), half_sat(v.y)), b = __halves2half2(half_sat(v.z), half_sat(v.w));
-            dst[j] = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
-        }
-    } else {
-        float4 *dst = reinterpret_cast<float4 *>(p.xs + (int64_t)(row - n_pick) * p.n_embd);
-#pragma unroll 4
-        for (int j = threadIdx.x; j < n4; j += kGatherThreads) dst[j] = src[j];
+    for (int j = threadIdx.x; j < n4; j += kGatherThreads) {
+        const float4 v = src[j];
+        const __half2 a = __halves2half2(half_sat(v.x), half_sat(v.y)), b = __halves2half2(half_sat(v.z), half_sat(v.w));
+        dst[j] = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
     }
 }
 
@@ -586,40 +603,48 @@ static size_t moe_float_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n
     return up256(sizeof(float) * (size_t)(n_tok * k) * (size_t)(bank->n_ff + bank->n_embd));
 }
 
-// More than eight tokens, shapes that the tensor-core and the streaming kernels address: the workspace of
-// launch_moe_ffn_grouped. Calls of many tokens go in chunks, so that it stays bounded.
+// More than one token, shapes that the streaming kernel (and above eight tokens the tensor-core kernel) addresses: the
+// workspace of launch_moe_ffn_grouped. Calls of many tokens go in chunks, so that it stays bounded.
 constexpr int64_t kChunkPicks = 65536;
 struct GroupedLayout {
-    size_t head, groups, pos, tables[kMaxClasses], xg, h, xs, hs, d, total;
+    size_t head, groups, pos, table_gu, table_dn, x_rows, xg, h, hs, d, total;
     int64_t chunk;   // tokens per chunk
-    int max_groups, max_few;
+    int max_groups;
 };
 constexpr int kMinTileM = 32;
 static GroupedLayout grouped_layout(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
     GroupedLayout L;
     L.chunk = kChunkPicks / k < n_tok ? kChunkPicks / k : n_tok;
     const size_t picks = (size_t)(L.chunk * k);
-    L.max_few = (int)((int64_t)picks < bank->n_local ? (int64_t)picks : bank->n_local);
-    L.max_groups = (int)(picks / kMinTileM) + bank->n_local;
-    const size_t few_rows = (size_t)L.max_few * kFewRows;
+    const bool many = n_tok > kFewRows;
+    // entries and their rows, whichever rows per entry are chosen: no entry is empty, and beside tensor-core experts an
+    // expert has at most kFewRows
+    size_t entries = 0, rows = 0;
+    for (size_t cap = 1; cap <= kFewRows; cap *= 2) {
+        const size_t most = (size_t)bank->n_local * (kFewRows / cap), n = many && most < picks ? most : picks;
+        entries = n > entries ? n : entries;
+        rows = n * cap > rows ? n * cap : rows;
+    }
+    L.max_groups = many ? (int)(picks / kMinTileM) + bank->n_local : 0;
     size_t at = 0;
     auto take = [&at](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
     L.head = take(sizeof(int));
     L.groups = take(sizeof(GemmGroup) * (size_t)L.max_groups);
     L.pos = take(sizeof(int32_t) * picks);
-    for (int c = 0; c < kMaxClasses; c++)
-        L.tables[c] = take(stream_table_bytes(2 * (size_t)L.max_few) + stream_table_bytes((size_t)L.max_few));
-    L.xg = take(sizeof(__half) * picks * bank->n_embd);
-    L.h = take(sizeof(__half) * picks * bank->n_ff);
-    L.xs = take(sizeof(float) * few_rows * bank->n_embd);
-    L.hs = take(sizeof(float) * few_rows * bank->n_ff);
-    L.d = take(sizeof(float) * (picks + few_rows) * bank->n_embd);
+    L.table_gu = take(stream_table_bytes(2 * entries));
+    L.table_dn = take(stream_table_bytes(entries));
+    L.x_rows = take(sizeof(int32_t) * rows);
+    L.xg = take(many ? sizeof(__half) * picks * bank->n_embd : 0);
+    L.h = take(many ? sizeof(__half) * picks * bank->n_ff : 0);
+    L.hs = take(sizeof(float) * rows * bank->n_ff);
+    L.d = take(sizeof(float) * ((many ? picks : 0) + rows) * bank->n_embd);
     L.total = at;
     return L;
 }
-static bool grouped_takes(const krk_cuda_expert_bank *bank) {
-    return bank->n_embd % 256 == 0 && bank->n_ff % 256 == 0 && stream_takes(bank->wt_gate_up, bank->n_embd, kFewRows) &&
-           stream_takes(bank->wt_down, bank->n_ff, kFewRows);
+static bool grouped_takes(const krk_cuda_expert_bank *bank, int64_t n_tok) {
+    if (n_tok <= kFewRows && bank->n_local > kMaxExperts) return false;   // more than the plan has threads
+    return n_tok > 1 && (n_tok <= kFewRows || (bank->n_embd % 256 == 0 && bank->n_ff % 256 == 0)) &&
+           stream_takes(bank->wt_gate_up, bank->n_embd, kFewRows) && stream_takes(bank->wt_down, bank->n_ff, kFewRows);
 }
 
 // The other shapes: one expert after the other, the tokens of an expert as one matrix.
@@ -651,9 +676,11 @@ static LoopLayout loop_layout(const krk_cuda_expert_bank *bank, int k, int64_t n
 }
 
 size_t moe_workspace_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {
-    if (n_tok > KRK_CUDA_MAX_ROWS) return grouped_takes(bank) ? grouped_layout(bank, k, n_tok).total : loop_layout(bank, k, n_tok).total;
+    const size_t grouped = grouped_takes(bank, n_tok) ? grouped_layout(bank, k, n_tok).total : 0;
+    if (n_tok > KRK_CUDA_MAX_ROWS) return grouped ? grouped : loop_layout(bank, k, n_tok).total;
     const size_t picks = (size_t)(n_tok * k);
-    return moe_float_bytes(bank, k, n_tok) + stream_table_bytes(2 * picks) + stream_table_bytes(picks);
+    const size_t by_pick = moe_float_bytes(bank, k, n_tok) + stream_table_bytes(2 * picks) + stream_table_bytes(picks);
+    return grouped > by_pick ? grouped : by_pick;
 }
 
 static int launch_combine(const MoeParams &p, cudaStream_t st) {
@@ -683,8 +710,15 @@ static MoeParams moe_params(float *y, const float *x, const int32_t *ids, const 
     return p;
 }
 
+// Rows per entry of the few-row experts, from the rows an expert can expect: two cost what one does, four and eight 1.5
+// and 2.2 times.
+static int entry_rows_log2(int64_t picks, int n_expert) {
+    return 5 * picks < 2 * n_expert ? 0 : picks < 2 * n_expert ? 1 : picks < 5 * n_expert ? 2 : 3;
+}
+
 static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const float *x, const int32_t *ids, const float *wts,
-                         const krk_cuda_expert_bank *bank, int k, int64_t n_tok, int n_expert, cudaStream_t st) {
+                         const krk_cuda_expert_bank *bank, int k, int64_t n_tok, const float *logits, int n_expert, cudaStream_t st) {
+    const bool many = L.max_groups > 0;   // some expert may go to the tensor cores
     GroupedParams p;
     p.gate = static_cast<const uint8_t *>(bank->gate);
     p.up = static_cast<const uint8_t *>(bank->up);
@@ -695,6 +729,9 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
     p.wt_down = bank->wt_down;
     p.x = x;
     p.ids = ids;
+    p.wts = wts;
+    p.logits = logits;
+    p.n_expert = n_expert;
     p.n_embd = bank->n_embd;
     p.n_ff = bank->n_ff;
     p.n_local = bank->n_local;
@@ -702,30 +739,29 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
     p.k = k;
     p.n_tok = (int)n_tok;
     // From the rows an expert can expect: the token tile (an expert's rows should fit one, since every further tile
-    // decodes its weights again; up to 128 tokens two accumulators alternate), and the classes of the few-row experts.
+    // decodes its weights again; up to 64 tokens two accumulators alternate), and the rows per entry of the few-row experts.
     const int64_t picks = n_tok * k, mean = picks / n_expert;
     p.tile_m = mean <= 44 ? 64 : mean <= 100 ? 128 : 256;
-    static const int kCaps[4][kMaxClasses] = {{1, 2, 4, 8}, {2, 4, 8, 8}, {4, 8, 8, 8}, {8, 8, 8, 8}};
-    const int pick_caps = 2 * picks < 3 * n_expert ? 0 : picks < 6 * n_expert ? 1 : picks < 14 * n_expert ? 2 : 3;
-    p.n_class = kMaxClasses - pick_caps;
-    for (int c = 0; c < kMaxClasses; c++) p.cap[c] = kCaps[pick_caps][c];
-    p.n_groups = reinterpret_cast<int *>(ws + L.head);
+    p.cap_log2 = entry_rows_log2(picks, n_expert);
+    p.cap = 1 << p.cap_log2;
+    p.n_groups = many ? reinterpret_cast<int *>(ws + L.head) : nullptr;
     p.groups = reinterpret_cast<GemmGroup *>(ws + L.groups);
     p.pos = reinterpret_cast<int32_t *>(ws + L.pos);
-    for (int c = 0; c < kMaxClasses; c++) {
-        p.table_gu[c] = reinterpret_cast<StreamTable *>(ws + L.tables[c]);
-        p.table_dn[c] = reinterpret_cast<StreamTable *>(ws + L.tables[c] + stream_table_bytes(2 * (size_t)L.max_few));
-    }
+    p.table_gu = reinterpret_cast<StreamTable *>(ws + L.table_gu);
+    p.table_dn = reinterpret_cast<StreamTable *>(ws + L.table_dn);
+    p.x_rows = reinterpret_cast<int32_t *>(ws + L.x_rows);
     p.xg = reinterpret_cast<__half *>(ws + L.xg);
-    p.xs = reinterpret_cast<float *>(ws + L.xs);
     p.hs = reinterpret_cast<float *>(ws + L.hs);
     p.d = reinterpret_cast<float *>(ws + L.d);
+    if (!many) p.d -= picks * p.n_embd;   // rows of d count from the picks on
     __half *h = reinterpret_cast<__half *>(ws + L.h);
 
-    int rc = launched(launch_overlapped(moe_group_plan_kernel, dim3(1), dim3(kMaxExperts), st, p));
+    // threads: one per expert, a warp per token to route, one per pick
+    int64_t threads = bank->n_local > picks ? bank->n_local : picks;
+    if (logits && 32 * n_tok > threads) threads = 32 * n_tok;
+    threads = threads < kMaxExperts ? (threads + 31) / 32 * 32 : kMaxExperts;
+    int rc = launched(launch_overlapped(moe_group_plan_kernel, dim3(1), dim3((unsigned)threads), st, p));
     if (rc != KRK_CUDA_OK) return rc;
-    if ((rc = launched(launch_overlapped(moe_gather_kernel, dim3((unsigned)picks), dim3(kGatherThreads), st, p))) != KRK_CUDA_OK) return rc;
-
     ExpertGemm gu, dn;
     gu.x = p.xg;
     gu.x_rows = dn.x_rows = picks;
@@ -753,12 +789,13 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
     dn_banks.base[0] = p.down;
     dn_banks.base[1] = nullptr;
     dn_banks.rows = dn.bank_rows;
-    if ((rc = launch_gemm_experts_gate_up(h, gu, st)) != KRK_CUDA_OK) return rc;
-    for (int c = 0; c < p.n_class; c++)
-        if ((rc = launch_gemv_stream_table(p.table_gu[c], bank->wt_gate_up, bank->n_ff, bank->n_embd, p.cap[c], 1, &gu_banks, st)) < 0) return rc;
-    if ((rc = launch_gemm_experts_down(p.d, dn, st)) != KRK_CUDA_OK) return rc;
-    for (int c = 0; c < p.n_class; c++)
-        if ((rc = launch_gemv_stream_table(p.table_dn[c], bank->wt_down, bank->n_embd, bank->n_ff, p.cap[c], 0, &dn_banks, st)) < 0) return rc;
+    if (many) {
+        if ((rc = launched(launch_overlapped(moe_gather_kernel, dim3((unsigned)picks), dim3(kGatherThreads), st, p))) != KRK_CUDA_OK) return rc;
+        if ((rc = launch_gemm_experts_gate_up(h, gu, st)) != KRK_CUDA_OK) return rc;
+    }
+    if ((rc = launch_gemv_stream_table(p.table_gu, p.cap > 1 ? p.x_rows : nullptr, bank->wt_gate_up, bank->n_ff, bank->n_embd, p.cap, 1, &gu_banks, st)) < 0) return rc;
+    if (many && (rc = launch_gemm_experts_down(p.d, dn, st)) != KRK_CUDA_OK) return rc;
+    if ((rc = launch_gemv_stream_table(p.table_dn, nullptr, bank->wt_down, bank->n_embd, bank->n_ff, p.cap, 0, &dn_banks, st)) < 0) return rc;
 
     MoeParams cp = moe_params(y, x, ids, wts, bank, k, n_tok);
     cp.d = p.d;
@@ -767,16 +804,22 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
 }
 
 static int launch_moe_ffn_grouped(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank,
-                                  int k, int64_t n_tok, int n_expert, void *workspace, cudaStream_t st) {
+                                  int k, int64_t n_tok, const float *logits, int n_expert, void *workspace, cudaStream_t st) {
     const int last = bank->expert_base + bank->n_local;   // ids at or above this are held elsewhere
-    if (last > kMaxExperts) return KRK_CUDA_EARG;
+    if (n_tok > kFewRows && last > kMaxExperts) return KRK_CUDA_EARG;
+    const GroupedLayout L = grouped_layout(bank, k, n_tok);
+    // up to a router row per warp of its block: the plan kernel routes them itself
+    if (logits && (n_tok > kMaxExperts / 32 || n_tok * n_expert > kRouteFloats || n_tok * k > kPlanIds)) {
+        const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);
+        if (rc != KRK_CUDA_OK) return rc;
+        logits = nullptr;
+    }
     if (n_expert < last) n_expert = last;
     if (n_expert < 1) n_expert = 1;
-    const GroupedLayout L = grouped_layout(bank, k, n_tok);
     for (int64_t t0 = 0; t0 < n_tok; t0 += L.chunk) {
         const int64_t n = n_tok - t0 < L.chunk ? n_tok - t0 : L.chunk;
         const int rc = moe_ffn_chunk(L, static_cast<uint8_t *>(workspace), y + t0 * bank->n_embd, x + t0 * bank->n_embd, ids + t0 * k,
-                                     wts + t0 * k, bank, k, n, n_expert, st);
+                                     wts + t0 * k, bank, k, n, logits, n_expert, st);
         if (rc != KRK_CUDA_OK) return rc;
     }
     return KRK_CUDA_OK;
@@ -849,14 +892,17 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
                            cudaStream_t st, const float *logits, int n_expert) {
     // `logits` set: route first (ids / wts are outputs). The streaming path folds the routing into its plan
     // kernel; every other path runs the routing kernel on its own.
+    // (few picks, or so thinly spread that entries would hold one row each: an entry per pick, and the shorter plan)
+    const int last = bank->expert_base + bank->n_local;
+    const bool by_pick = n_tok <= KRK_CUDA_MAX_ROWS && (n_tok * k <= 8 || entry_rows_log2(n_tok * k, n_expert > last ? n_expert : last) == 0);
+    if (!by_pick && grouped_takes(bank, n_tok)) return launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, logits, n_expert, workspace, st);
     bool routed = logits == nullptr;
     if (n_tok > KRK_CUDA_MAX_ROWS) {
         if (!routed) {
             const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);
             if (rc != KRK_CUDA_OK) return rc;
         }
-        return grouped_takes(bank) ? launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, n_expert, workspace, st)
-                                   : launch_moe_ffn_loop(y, x, ids, wts, bank, k, n_tok, workspace, st);
+        return launch_moe_ffn_loop(y, x, ids, wts, bank, k, n_tok, workspace, st);
     }
     MoeParams p = moe_params(y, x, ids, wts, bank, k, n_tok);
     p.h = static_cast<float *>(workspace);
@@ -881,9 +927,9 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
                                             row_bytes(bank->wt_gate_up, bank->n_embd), row_bytes(bank->wt_down, bank->n_ff),
                                             fuse_route ? logits : (const float *)nullptr, n_expert));
         if (rc != KRK_CUDA_OK) return rc;
-        rc = launch_gemv_stream_table(ta, bank->wt_gate_up, bank->n_ff, bank->n_embd, 1, 1, &gu_banks, st);
+        rc = launch_gemv_stream_table(ta, nullptr, bank->wt_gate_up, bank->n_ff, bank->n_embd, 1, 1, &gu_banks, st);
         if (rc < 0) return rc;
-        rc = launch_gemv_stream_table(tb, bank->wt_down, bank->n_embd, bank->n_ff, 1, 0, nullptr, st);
+        rc = launch_gemv_stream_table(tb, nullptr, bank->wt_down, bank->n_embd, bank->n_ff, 1, 0, nullptr, st);
         if (rc < 0) return rc;
         return launch_combine(p, st);
     }

@@ -615,3 +615,32 @@ def test_backend_gemm_group_decode_batches(cuda, oracle, wt, n_in, rows):
     for p in [d_x] + d_w + d_y:
         be.release(p)
     be.close()
+
+
+@pytest.mark.parametrize("n_exp,k,n_tok,local", [(4, 4, 8, None), (4, 2, 5, (1, 3)), (16, 4, 6, None), (16, 4, 13, None), (64, 3, 7, (20, 64)),
+                                                 (64, 6, 12, None), (64, 6, 31, (32, 64))])
+def test_moe_entries_of_several_tokens(cuda, oracle, n_exp, k, n_tok, local):
+    """Few-row experts share a streaming entry between 1, 2, 4 or 8 tokens (by the rows an expert can expect); beyond eight
+    rows they go to the tensor cores (f16 operands: the prefill bound)."""
+    for wt_gu, wt_dn in ((synth.Q4_K, synth.Q6_K), (synth.Q8_0, synth.Q5_0)):
+        y, y_ref, _ = moe_case(cuda, oracle, 512, 768, n_exp, k, n_tok, SEED + 500 + n_exp + n_tok, local=local, wt_gu=wt_gu, wt_dn=wt_dn)
+        assert np.linalg.norm(y - y_ref) <= (2e-4 if n_tok <= 8 else 2e-3) * np.linalg.norm(y_ref)
+
+
+def test_moe_repeated_ids_in_a_decode_batch(cuda, oracle):
+    """Ids of the caller's own may name one expert several times for a token: more rows of an expert than tokens."""
+    n_embd, n_ff, n_exp, k, n_tok = 512, 512, 4, 6, 8
+    seed = SEED + 560
+    gate, up, down = (synth.weights(wt, n_exp * r, c, seed, stream=700 + i) for i, (wt, r, c) in
+                      enumerate(((synth.Q4_K, n_ff, n_embd), (synth.Q4_K, n_ff, n_embd), (synth.Q6_K, n_embd, n_ff))))
+    x = synth.activations(n_tok, n_embd, seed)
+    ids = np.array([[(t + s // 3) % n_exp for s in range(k)] for t in range(n_tok)], np.int32)
+    wts = np.full((n_tok, k), 1.0 / k, np.float32)
+    bank = cuda.make_bank(dev(gate), dev(up), dev(down), synth.Q4_K, synth.Q6_K, n_exp, 0, n_embd, n_ff)
+    got = cuda.moe_ffn(dev(x), dev(ids), dev(wts), bank).cpu().numpy()
+    want = np.zeros((n_tok, n_embd))
+    for t in range(n_tok):
+        for e in ids[t]:
+            g, u = (oracle.gemm(x[t:t + 1], m.reshape(n_exp, n_ff, -1)[e], synth.Q4_K, n_ff, n_embd) for m in (gate, up))
+            want[t] += oracle.gemm(oracle.silu_mul(g[0], u[0])[None], down.reshape(n_exp, n_embd, -1)[e], synth.Q6_K, n_embd, n_ff)[0].astype(np.float64) / k
+    assert np.linalg.norm(got - want) <= 2e-4 * np.linalg.norm(want)
