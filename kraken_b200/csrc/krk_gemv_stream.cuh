@@ -276,7 +276,7 @@ struct Smem {
     unsigned long long red_full[kMaxRedSlots];  // every consumer warp has written its partial sums of a tile
     unsigned long long red_empty[kMaxRedSlots]; // the epilogue warp has consumed them
     int gave_up;
-    int pad[3];
+    int touched[11];   // where the parameter fetches of the first instructions end (never read)
     float gate[kMaxStack][NG][32];   // epilogue warp: the gate tile(s) of a gate/up pair, until the up tile arrives
     // per consumer warp, column group and row pair (g, g+8): {row g x even activation row, g x odd, g+8 x even, g+8 x odd}
     float4 red[consumer_groups(NG) * red_slots(NG)][kConsumerWarps][NG][8];
@@ -1368,6 +1368,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // and waits for this grid to complete before touching activations or outputs.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     volatile int *gave_up = &sm->gave_up;
+    // Parameters arrive cold in every launch, and a miss holds its warp for some 700 clocks, one line after the other:
+    // warps 1..8 fetch a 64-byte line each, side by side (the scalars and the first seven entries). Q4_K 4096 x 4096
+    // 5.09 -> 4.95 us in a chain of launches, 1536 x 1536 3.37 -> 3.25. Only the single-row forms: the others have the
+    // longer start anyway and gain nothing (Q6_K 5.22 -> 5.18, Q8_0 5.94 -> 6.03, Q3_K 5.49 -> 5.65).
+    static_assert(kGroups * kConsumerWarps >= 8 && sizeof(StreamParams) >= 8 * 64, "a warp for each of eight lines");
+    if (SINGLE && warp >= 1 && warp <= 8 && lane == 0)
+        sm->touched[warp] = reinterpret_cast<const int *>(&p)[16 * (warp - 1)];
 
     if (warp == 0) {
         // ===== producer warp: weights only, so it can run ahead of everything else =====
