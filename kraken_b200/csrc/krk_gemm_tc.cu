@@ -117,6 +117,7 @@ struct GemmParams {
     int tile_m;          // tokens per tile: multiple of 16, <= 256
     int n_tiles_n, n_tiles_m;
     int row_bytes;
+    uint32_t zero;       // always 0, which the compiler does not know (see the decode warps)
     int xk;              // K steps per X stage: 4, 2 or 1
     int dual;            // 1: both MMA warps issue, super-blocks in turn, into an accumulator each
     int n_b, n_raw;      // ring depths (stages)
@@ -329,6 +330,7 @@ __device__ __forceinline__ void load_half_column(const uint8_t *column, int grp,
     }
 }
 
+// loaded(): a word that depends on every load of load_block.
 template <int WT>
 struct Raw;
 
@@ -363,6 +365,7 @@ struct Raw<KRK_CUDA_Q6_K> {
         dbits = *reinterpret_cast<const unsigned short *>(slot + lead + 208);
     }
     // f16(d * scale) is formed in f32 as the host decoder forms d * scale.
+    __device__ __forceinline__ uint32_t loaded() const { return ql[0] ^ ql[7] ^ qh[0] ^ qh[7] ^ sc[0] ^ sc[1] ^ dbits; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const float d = float_of_half_bits(dbits);
@@ -402,6 +405,7 @@ struct Raw<KRK_CUDA_Q4_K> {
         k_scales(hdr, grp, sc, mn);
         dd = hdr.x;
     }
+    __device__ __forceinline__ uint32_t loaded() const { return q[0] ^ q[4] ^ q[8] ^ q[12] ^ dd; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const int k = 2 * j + half;
@@ -429,6 +433,7 @@ struct Raw<KRK_CUDA_Q5_K> {
         k_scales(hdr, grp, sc, mn);
         dd = hdr.x;
     }
+    __device__ __forceinline__ uint32_t loaded() const { return q[0] ^ q[4] ^ q[8] ^ q[12] ^ qh[0] ^ qh[4] ^ dd; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const int k = 2 * j + half, up = 4 - k;   // (the masks were moved down by the group's 4 bits when loaded)
@@ -451,6 +456,7 @@ struct Raw<KRK_CUDA_Q4_0> {
     static constexpr int kSteps = 4;
     uint32_t w[18];
     __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<4>(block, grp, w); }
+    __device__ __forceinline__ uint32_t loaded() const { return w[0] ^ w[2] ^ w[4] ^ w[8] ^ w[12] ^ w[14] ^ w[16]; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const __half2 d2 = half2_of_bits(half ? (w[9 * j + 4] >> 16) : (w[9 * j] & 0xFFFFu));
@@ -474,6 +480,7 @@ struct Raw<KRK_CUDA_IQ4_NL> {
     static constexpr int kSteps = 4;
     uint32_t w[18];
     __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<4>(block, grp, w); }
+    __device__ __forceinline__ uint32_t loaded() const { return w[0] ^ w[2] ^ w[4] ^ w[8] ^ w[12] ^ w[14] ^ w[16]; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         constexpr uint32_t kG0 = 0x3F2D1801u, kG1 = 0x766A5D4Fu, kG2 = 0xA6998D81u, kG3 = 0xF1D9C5B5u;   // grid + 128
@@ -506,6 +513,7 @@ struct Raw<KRK_CUDA_Q5_0> {
     static constexpr int kSteps = 4;
     uint32_t w[22];
     __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_half_column<5>(block, grp, w); }
+    __device__ __forceinline__ uint32_t loaded() const { return w[0] ^ w[2] ^ w[4] ^ w[8] ^ w[12] ^ w[16] ^ w[18] ^ w[20]; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const int W = 11 * j;
@@ -528,6 +536,7 @@ struct Raw<KRK_CUDA_Q5_1> {
     static constexpr int kSteps = 4;
     uint32_t w[24];
     __device__ __forceinline__ void load_block(const uint8_t *block, int, int, int grp) { load_quads<6>(block + 96 * grp, w); }
+    __device__ __forceinline__ uint32_t loaded() const { return w[0] ^ w[4] ^ w[8] ^ w[12] ^ w[16] ^ w[20]; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         uint32_t b[6];
@@ -558,6 +567,7 @@ struct Raw<KRK_CUDA_Q8_0> {
 #pragma unroll
         for (int i = 0; i < 9; i++) w[i] = b[i];
     }
+    __device__ __forceinline__ uint32_t loaded() const { return w[0] ^ w[1] ^ w[2] ^ w[3] ^ w[4] ^ w[5] ^ w[6] ^ w[7] ^ w[8]; }
     template <int half>
     __device__ __forceinline__ void convert(int, uint32_t (&out)[16]) const {
         const __half2 d2 = half2_of_bits(half ? (w[0] >> 16) : (w[0] & 0xFFFFu));
@@ -586,6 +596,7 @@ struct Raw<KRK_CUDA_Q2_K> {
         sc[1] = w[2 * grp + 1];
         dm = w[20];
     }
+    __device__ __forceinline__ uint32_t loaded() const { return q[0] ^ q[7] ^ sc[0] ^ sc[1] ^ dm; }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const float d = float_of_half_bits(dm & 0xFFFF), dmin = float_of_half_bits(dm >> 16);
@@ -622,6 +633,7 @@ struct Raw<KRK_CUDA_Q3_K> {
         sc[0] = ((a0 >> (4 * grp)) & 0x0F0F0F0Fu) | (((a2 >> (4 * grp)) << 4) & 0x30303030u);
         sc[1] = ((a1 >> (4 * grp)) & 0x0F0F0F0Fu) | (((a2 >> (4 * grp)) << 2) & 0x30303030u);
     }
+    __device__ __forceinline__ uint32_t loaded() const { return hm[0] ^ hm[7] ^ q[0] ^ q[7] ^ sc[0] ^ sc[1] ^ __float_as_uint(d); }
     template <int half>
     __device__ __forceinline__ void convert(int j, uint32_t (&out)[16]) const {
         const float dl0 = __fmul_rn(d, byte_plus_2_23(sc[j], 2 * half) - 8388640.0f);   // d * (scale - 32)
@@ -764,17 +776,20 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                 wait_phase(smem_u32(&sm->raw_full[sr]), pr, gave_up, p.status);
                 if constexpr (row_phased(WT)) cur.lead = (row_lead + (ks >> 2) * block_bytes(WT)) & 15;
                 cur.load_block(raw_ring + (size_t)sr * kStageBytes + tslot * kSeg, half, ks, grp);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]));   // the bytes are in registers now
-                if (++sr == p.n_raw) {
-                    sr = 0;
-                    pr ^= 1;
-                }
                 // The group's two K steps fill one tensor-memory stage (Q8_0: its one step half of it); the second is
                 // converted while the first's store is in flight.
                 uint32_t v[16];
                 if (half) cur.template convert<1>(0, v);
                 else cur.template convert<0>(0, v);
+                // The stage is given back when its bytes ARE in registers: an arrival does not wait for loads in flight, and
+                // while the MMAs and the copies of X keep shared memory busy those took longer than a refill (Q8_0, tiles of
+                // 96 tokens and more: rows of a later stage in the first ones). Hence the address that needs them.
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]) + (cur.loaded() & p.zero));
+                if (++sr == p.n_raw) {
+                    sr = 0;
+                    pr ^= 1;
+                }
                 wait_phase(smem_u32(&sm->a_empty[sa]), pa ^ 1, gave_up, p.status);
                 tc_fence_after();
                 tmem_st16(lane_addr + 64 * sa + (kOwnStages ? 0 : 32 * grp), v);

@@ -151,3 +151,22 @@ def test_gemm_split_k_clusters(cuda, oracle, wt):
 def test_gemm_token_tiles_narrower_than_the_rows(cuda, oracle, rows):
     """More than one token tile of less than 256 tokens: a tile's last store must not reach into the next one's rows."""
     run_gemm(cuda, oracle, synth.Q4_0, 2300, 512, rows, SEED + 120 + rows)
+
+
+@pytest.mark.parametrize("wt", [synth.Q8_0, synth.Q4_K, synth.Q6_K, synth.Q5_1, synth.Q2_K, synth.IQ4_NL])
+def test_gemm_stages_are_not_refilled_while_being_read(cuda, oracle, wt):
+    """Wide tiles keep shared memory busy, so the decode warps' loads are slow while the ring of raw stages turns over
+    many times: every call has the same bits, and the first rows of a stage (a refill's first) are right."""
+    n_out, n_in = 128 * 157, 1536
+    w = synth.weights(wt, n_out, n_in, SEED + 130, stream=wt)
+    sel = np.concatenate([np.arange(t, t + 32) for t in range(0, n_out, 128 * 20)])
+    for rows in (96, 257):
+        x16 = synth.activations_f16(rows, n_in, SEED + 131)
+        xd, wd = dev(x16), dev(w)
+        y = [cuda.gemm(xd, wd, wt, n_out, n_in).cpu().numpy() for _ in range(5)]
+        assert cuda.device_status() == 0
+        assert all(np.array_equal(y[0], o) for o in y[1:])
+        x = x16.astype(np.float32)
+        y_ref = oracle.gemm(x, w[sel], wt, len(sel), n_in, rows=rows, threads=8)
+        ok, worst = bound_ok(y[0][:, sel], y_ref, oracle.dequant_rows(w[sel], wt, len(sel), n_in), x, GEMM_TOL)
+        assert ok, worst
