@@ -32,8 +32,9 @@
 // HBM (a four-deep X ring and three raw stages cost 330 ns per K step at every M <= 128 and in every format,
 // against 104 ns of HBM time for Q4_K), so the shared memory that a small X tile leaves goes into more stages.
 //
-// Few tiles (a short prompt, a narrow matrix): the CTAs of a cluster share one tile, each taking a piece of K; the
-// accumulators meet over distributed shared memory and are added in K order, the same on every run.
+// Tiles come in whole waves, and the CTAs of a cluster share each of the tiles left over (all of them, for a short prompt
+// or a narrow matrix), a piece of K each; the accumulators meet over distributed shared memory and are added in K
+// order, the same on every run.
 //
 // Same contract as gemm_wmma_kernel of the reference (src/hip/kernels/gemm.hpp:621-970): f16
 // staged operands, f32 accumulation; here the output stays f32.
@@ -42,6 +43,7 @@
 // runs to its end without waiting again and frees its tensor memory.
 #include <cuda.h>
 
+#include <cstddef>
 #include <mutex>
 
 #include "krk_common.cuh"
@@ -116,13 +118,18 @@ struct GemmParams {
     int64_t n_out, n_in, rows;
     int tile_m;          // tokens per tile: multiple of 16, <= 256
     int n_tiles_n, n_tiles_m;
+    int group;           // tiles in a row that share a weight tile (dense: n_tiles_m) or a token group (expert kinds: n_tiles_n)
+    uint32_t per_group;  // ceil(2^32 / group) where the high half of a product with it divides every tile's number exactly, else 0
+    int k_blocks, kb_each, kb_more;   // super-blocks of K; a piece has kb_each of them, the first kb_more pieces one more
+    int sum_tokens;      // tokens of a shared tile that one CTA of the cluster adds up
     int row_bytes;
     uint32_t zero;       // always 0, which the compiler does not know (see the decode warps)
     int xk;              // K steps per X stage: 4, 2 or 1
     int dual;            // 1: both MMA warps issue, super-blocks in turn, into an accumulator each
     int n_b, n_raw;      // ring depths (stages)
     int raw_off, y_off, bar_off;   // where the raw ring, the read-out buffers and the barriers start (the X ring starts at 0)
-    int split;           // CTAs per cluster, each with a piece of K (1: no cluster)
+    int split;           // CTAs per cluster (1: no cluster)
+    int n_full;          // tiles that one CTA computes alone; the clusters share the rest, at most one each
     int y_tma;           // 1: tiles leave through shared memory and TMA stores (y 16-byte aligned, n_out % 4 == 0)
     int *status;
     const GemmGroup *groups;   // kGateUp, kDown: token groups, and how many
@@ -266,6 +273,16 @@ __host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
 // shared memory.
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int cluster_rank() {
+    int v;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v));
+    return v;
+}
+__device__ __forceinline__ int cluster_id() {
+    int v;
+    asm("mov.u32 %0, %%clusterid.x;" : "=r"(v));
+    return v;
 }
 __device__ __forceinline__ float4 ld_peer(uint32_t addr, int rank) {
     uint32_t a;
@@ -661,24 +678,42 @@ struct Tile {
     int n0;         // first output column
     int x_row;      // first X row
     int m;          // valid tokens
+    int kb0, kb1;   // super-blocks of K
+    bool piece;     // of a tile that the cluster shares (a CTA's last)
 };
+// at / p.group. (A division here is 100 clocks and more of every warp's way to its first work, and of a shared tile's end.)
+__device__ __forceinline__ int tile_group(const GemmParams &p, int at) {
+    return p.group == 1 ? at : p.per_group ? (int)__umulhi((uint32_t)at, p.per_group) : at / p.group;
+}
 template <int KIND>
 struct TileIter {
-    int i, n, stride;
+    int i, n, stride, shared;   // shared: the cluster's shared tile, -1: none (any more)
     __device__ __forceinline__ void init(const GemmParams &p) {
-        i = (int)blockIdx.x / p.split;
-        stride = (int)gridDim.x / p.split;
-        n = KIND == kDense ? p.n_tiles_n * p.n_tiles_m : *p.n_groups * p.n_tiles_n;
+        i = (int)blockIdx.x;
+        stride = (int)gridDim.x;
+        n = KIND == kDense ? p.n_full : *p.n_groups * p.n_tiles_n;
+        shared = -1;
+        if (KIND == kDense && p.split > 1) {
+            const int at = p.n_full + cluster_id();
+            if (at < p.n_tiles_n * p.n_tiles_m) shared = at;
+        }
     }
     __device__ __forceinline__ bool next(const GemmParams &p, Tile &t) {
-        if (i >= n) return false;
+        int at = i;
+        t.kb0 = 0, t.kb1 = p.k_blocks, t.piece = false;
+        if (i >= n) {
+            if (KIND != kDense || shared < 0) return false;
+            const int rank = cluster_rank();
+            at = shared, shared = -1;
+            t.kb0 = rank * p.kb_each + min(rank, p.kb_more), t.kb1 = t.kb0 + p.kb_each + (rank < p.kb_more ? 1 : 0), t.piece = true;
+        }
         if (KIND == kDense) {
-            const int nt = i / p.n_tiles_m, mt = i - nt * p.n_tiles_m;
+            const int nt = tile_group(p, at), mt = at - nt * p.n_tiles_m;
             t.w_row = t.n0 = nt * kTileN;
             t.x_row = mt * p.tile_m;
             t.m = p.tile_m;
         } else {
-            const int g = i / p.n_tiles_n, nt = i - g * p.n_tiles_n;
+            const int g = tile_group(p, at), nt = at - g * p.n_tiles_n;
             const GemmGroup gr = p.groups[g];
             t.n0 = nt * (KIND == kGateUp ? kTileN / 2 : kTileN);
             t.w_row = gr.expert * (int)p.n_out + t.n0;   // an expert holds n_out rows of (each) bank
@@ -713,27 +748,27 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);   // warp-uniform to the compiler too
     volatile int *gave_up = &sm->gave_up;
 
-    if (tid == 0) {
-        for (int s = 0; s < p.n_b; s++) {
-            mbar_init(smem_u32(&sm->b_full[s]), 1);
-            mbar_init(smem_u32(&sm->b_empty[s]), 1);
+    // Barriers, two per lane: by one thread they took longer than all else before the first copy. The maps are fetched
+    // meanwhile.
+    if (warp == 0) {
+        constexpr int kBars = 2 * (kMaxB + kAStages + kMaxRaw + 2);
+        static_assert(offsetof(GemmBars, tmem_base) == 8 * kBars, "barriers come first, in this order");
+        for (int b = lane; b < kBars; b += 32) {
+            const int a = b - 2 * kMaxB, w = a - 2 * kAStages, d = w - 2 * kMaxRaw;
+            const int count = a < 0 ? 1 : w < 0 ? (a >= kAStages ? 1 : kOwnStages ? kDecodeWarps / kDecodeGroups : kDecodeWarps)
+                              : d < 0 ? (w >= kMaxRaw ? kDecodeWarps : 1) : d >= 2 ? kEpilogueThreads / 32 : p.dual ? 2 : 1;
+            mbar_init(smem_u32(sm) + 8 * b, count);
         }
-        for (int s = 0; s < kAStages; s++) {
-            mbar_init(smem_u32(&sm->a_full[s]), kOwnStages ? kDecodeWarps / kDecodeGroups : kDecodeWarps);
-            mbar_init(smem_u32(&sm->a_empty[s]), 1);
-        }
-        for (int s = 0; s < p.n_raw; s++) {
-            mbar_init(smem_u32(&sm->raw_full[s]), 1);
-            mbar_init(smem_u32(&sm->raw_empty[s]), kDecodeWarps);
-        }
-        for (int s = 0; s < 2; s++) {
-            mbar_init(smem_u32(&sm->d_full[s]), p.dual ? 2 : 1);
-            mbar_init(smem_u32(&sm->d_empty[s]), kEpilogueThreads / 32);
-        }
-        sm->gave_up = 0;
+        if (lane == 0) sm->gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    } else if (warp == kXWarp && lane == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&x_map) : "memory");
+    } else if (warp == kRawWarp && lane < (row_phased(WT) ? (KIND == kGateUp ? 2 * kPhases : kPhases) : KIND == kGateUp ? 2 : 1)) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&w_maps.m[lane]) : "memory");
     }
+    TileIter<KIND> iter;
+    if (KIND == kDense) iter.init(p);   // (its parameters arrive cold, so before the barrier, which waits for some anyway)
     if (warp == kMmaWarp) {
         tmem_alloc(smem_u32(&sm->tmem_base), kTmemCols);
         tmem_relinquish();
@@ -750,12 +785,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
     const int n_acc = p.tile_m <= kMaxTileM / (p.dual ? 4 : 2) ? 2 : 1;
     const int d_other = p.tile_m <= kMaxTileM / 4 ? 64 : 128;   // second accumulator of a tile, columns on from the first
 
-    // this CTA's K steps: all, or its cluster rank's share in whole super-blocks
-    const int k_blocks = (int)(p.n_in / 256), rank = (int)blockIdx.x % p.split;
-    const int kb0 = k_blocks * rank / p.split, kb1 = k_blocks * (rank + 1) / p.split;
-    const int ks0 = kb0 * 4, ks1 = kb1 * 4;
-    TileIter<KIND> iter;
-    iter.init(p);
+    if (KIND != kDense) iter.init(p);
     Tile it;
 
     if (warp < kDecodeWarps) {
@@ -772,7 +802,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             // Rows past n_out need no care here: their staged bytes are zero (the tensor maps fill what lies
             // outside the matrix with zeros), and a zero block decodes to zeros.
             Raw<WT> cur;
-            for (int ks = ks0; ks < ks1; ks += Raw<WT>::kSteps) {
+            for (int ks = 4 * it.kb0; ks < 4 * it.kb1; ks += Raw<WT>::kSteps) {
                 wait_phase(smem_u32(&sm->raw_full[sr]), pr, gave_up, p.status);
                 if constexpr (row_phased(WT)) cur.lead = (row_lead + (ks >> 2) * block_bytes(WT)) & 15;
                 cur.load_block(raw_ring + (size_t)sr * kStageBytes + tslot * kSeg, half, ks, grp);
@@ -818,7 +848,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         const int my_row = tile_row<WT, KIND>(32 * ew + lane);
         int ybuf = 0, da = 0, first = 0;   // first: as in the MMA warps
         uint32_t ph = 0;
-        const int n_blk = kb1 - kb0;
+        int n_blk = 0;
         // 32 tokens of the accumulator; of both, where two MMA warps shared the tile's super-blocks (of a single one, only one
         // did anything)
         auto read = [&](uint32_t addr, uint32_t (&v)[32]) {
@@ -840,7 +870,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             tc_fence_after();
             const uint32_t d_addr = lane_d + 128 * da;
             const int tokens = tile_tokens<KIND>(p, it);
-            if (KIND == kDense && p.split > 1) {
+            n_blk = it.kb1 - it.kb0;
+            if (KIND == kDense && it.piece) {
                 // a piece of K: the whole accumulator goes to shared memory over the drained X ring (every MMA that
                 // read it is done); the cluster adds the pieces up below
                 float *part = reinterpret_cast<float *>(smem);
@@ -851,7 +882,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                     for (int j = 0; j < 32; j++)
                         if (c0 + j < tokens) part[(c0 + j) * kTileN + my_row] = __uint_as_float(v[j]);
                 }
-                break;   // one tile per cluster
+                break;   // the last
             }
             for (int c0 = 0; c0 < tokens; c0 += kYChunk) {
                 uint32_t v[32];
@@ -926,7 +957,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         while (iter.next(p, it)) {
             const int boxes = __shfl_sync(0xFFFFFFFFu, (tile_tokens<KIND>(p, it) + kGroupBox - 1) / kGroupBox, 0);
             const int x_row = __shfl_sync(0xFFFFFFFFu, it.x_row, 0);
-            for (int ks = ks0; ks < ks1; ks += p.xk) {
+            for (int ks = 4 * it.kb0; ks < 4 * it.kb1; ks += p.xk) {
                 wait_phase(smem_u32(&sm->b_empty[sb]), pb ^ 1, gave_up, p.status);
                 const uint32_t bar = smem_u32(&sm->b_full[sb]), dst = smem_u32(smem) + (uint32_t)(sb * b_stage);
                 // (dense: one box per K step; else only the boxes that hold tokens of the group)
@@ -955,7 +986,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         uint32_t pr = 0;
         while (iter.next(p, it)) {
             const int w_row = __shfl_sync(0xFFFFFFFFu, it.w_row, 0);
-            for (int blk = ks0 / kPer; blk < ks1 / kPer; blk++) {
+            for (int blk = 4 * it.kb0 / kPer; blk < 4 * it.kb1 / kPer; blk++) {
                 wait_phase(smem_u32(&sm->raw_empty[sr]), pr ^ 1, gave_up, p.status);
                 const uint32_t bar = smem_u32(&sm->raw_full[sr]);
                 const uint32_t stage = smem_u32(raw_ring) + (uint32_t)(sr * kStageBytes);
@@ -994,7 +1025,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         const uint32_t elected = elect_one();
         constexpr uint32_t tmem = 0;   // an allocation of all 512 columns starts at the first
         iter.n = __shfl_sync(0xFFFFFFFFu, iter.n, 0);
-        const int per_blk = 4 / p.xk, n_blk = kb1 - kb0;   // X stages per super-block
+        const int per_blk = 4 / p.xk;     // X stages per super-block
         int blk = who;                    // this warp's next super-block of the CTA's sequence
         int first = 0;                    // the sequence number of the tile's first super-block
         int sb = (who * per_blk) % p.n_b, sa = 2 * who, da = 0;
@@ -1004,6 +1035,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
             wait_phase(smem_u32(&sm->d_empty[da]), pd ^ 1, gave_up, p.status);   // the epilogue has drained the accumulator
             tc_fence_after();
             const uint32_t d_tmem = tmem + 128 * da + (who ? d_other : 0);
+            const int n_blk = it.kb1 - it.kb0;
             uint32_t fresh = 1u;
             for (; blk < first + n_blk; blk += step) {
                 uint32_t b_lo = 0;
@@ -1061,6 +1093,19 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         }
     }
 
+    // A shared tile's pieces meet: CTA `rank` adds its share of the tokens over all CTAs of the cluster, in K order. The
+    // decode warps do that, who have the time to work out where while the last super-blocks are multiplied.
+    const bool sums = KIND == kDense && p.split > 1 && warp < kDecodeWarps;
+    int tok = 0, tok_end = 0, col = 0;
+    int64_t m = 0, n = 0;
+    if (sums) {
+        const int rank = cluster_rank(), at = p.n_full + cluster_id();
+        const int nt = tile_group(p, at), mt = at - nt * p.n_tiles_m;
+        tok = rank * p.sum_tokens + tid / (kTileN / 4), col = 4 * (tid % (kTileN / 4));
+        m = (int64_t)mt * p.tile_m + tok, n = (int64_t)nt * kTileN + col;
+        tok_end = nt < p.n_tiles_n && n < p.n_out ? min((rank + 1) * p.sum_tokens, p.tile_m) : 0;   // (not: a cluster without a tile)
+        tok_end = (int)min((int64_t)tok_end, tok + p.rows - m);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -1069,31 +1114,32 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
         __syncwarp();
     }
     if (KIND == kDense && p.split > 1) {
-        // ---- the pieces of a tile meet: CTA `rank` adds its share of the tokens over all CTAs of the cluster, in K order ----
         cluster_sync();
-        const int nt = ((int)blockIdx.x / p.split) / p.n_tiles_m, mt = ((int)blockIdx.x / p.split) % p.n_tiles_m;
-        const int t0 = p.tile_m * rank / p.split, t1 = p.tile_m * (rank + 1) / p.split;
-        for (int i = tid; i < (t1 - t0) * (kTileN / 4); i += kThreads) {
-            const int tok = t0 + i / (kTileN / 4), col = 4 * (i % (kTileN / 4));
-            const int64_t m = (int64_t)mt * p.tile_m + tok, n = (int64_t)nt * kTileN + col;
-            if (m >= p.rows || n >= p.n_out) continue;
-            const uint32_t at = smem_u32(smem) + (uint32_t)(tok * kTileN + col) * 4u;
-            float4 s = ld_peer(at, 0);
-            for (int q = 1; q < p.split; q++) {
-                const float4 v = ld_peer(at, q);
-                s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
-            }
+        if (sums) {
             float *y = p.y + m * p.n_out + n;
-            if (p.y_tma) {   // 16-byte aligned, n_out a multiple of four
-                *reinterpret_cast<float4 *>(y) = s;
-            } else {
-                y[0] = s.x;
-                if (n + 1 < p.n_out) y[1] = s.y;
-                if (n + 2 < p.n_out) y[2] = s.z;
-                if (n + 3 < p.n_out) y[3] = s.w;
+            for (; tok < tok_end; tok += kDecodeThreads / (kTileN / 4), y += (kDecodeThreads / (kTileN / 4)) * p.n_out) {
+                const uint32_t at = smem_u32(smem) + (uint32_t)(tok * kTileN + col) * 4u;
+                float4 v[kMaxSplit];   // all in flight together: one after the other they took some 250 ns each
+#pragma unroll
+                for (int q = 0; q < kMaxSplit; q++)
+                    if (q < p.split) v[q] = ld_peer(at, q);
+                float4 s = v[0];
+#pragma unroll
+                for (int q = 1; q < kMaxSplit; q++)
+                    if (q < p.split) s.x += v[q].x, s.y += v[q].y, s.z += v[q].z, s.w += v[q].w;
+                if (p.y_tma) {   // 16-byte aligned, n_out a multiple of four
+                    *reinterpret_cast<float4 *>(y) = s;
+                } else {
+                    y[0] = s.x;
+                    if (n + 1 < p.n_out) y[1] = s.y;
+                    if (n + 2 < p.n_out) y[2] = s.z;
+                    if (n + 3 < p.n_out) y[3] = s.w;
+                }
             }
         }
-        cluster_sync();   // nobody leaves while its shared memory is being read
+        // Nobody leaves while its shared memory is being read. Relaxed: what was read has been used by the stores above, and a
+        // release would wait for those (700 ns).
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
     }
 }
 
@@ -1133,6 +1179,18 @@ bool encode_2d(CUtensorMap *map, CUtensorMapDataType type, const void *base, int
     const cuuint32_t estr[2] = {1, 1};
     return encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promo,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The division-free parameters of GemmParams.
+void set_divisions(GemmParams &p, int group, int64_t tiles) {
+    const uint64_t most = (uint64_t)tiles + 256, m = (uint64_t)group;   // (clusters without a tile look past the last)
+    p.group = group;
+    // at * per is at / m * 2^32 and less than at more: the quotient is exact while at * m < 2^32
+    p.per_group = m > 1 && most * m < (1ull << 32) ? (uint32_t)(((1ull << 32) + m - 1) / m) : 0u;
+    p.k_blocks = (int)(p.n_in / 256);
+    p.kb_each = p.k_blocks / p.split;
+    p.kb_more = p.k_blocks % p.split;
+    p.sum_tokens = (p.tile_m + p.split - 1) / p.split;
 }
 
 // The maps over the raw weight bytes of one matrix ([n_out][row_bytes] bytes), for boxes that bring `tile_rows` rows.
@@ -1224,19 +1282,19 @@ int launch_kernel(const GemmParams &p, const CUtensorMap &x_map, const WMaps<KIN
     return KRK_CUDA_OK;
 }
 
-// How a dense product is cut. One tile is 128 weight rows x tile_m tokens, `split` CTAs share it along K, and the
-// model below (clocks; fitted to single tiles on all SMs, Q4_K, K = 16384: a K step took 206 / 218 / 290 / 466 ns at
-// 16 / 64 / 128 / 256 tokens, every other format within a fifth of that or slower at the narrow end) picks the pair
+// How a dense product is cut. One tile is 128 weight rows x tile_m tokens; whole waves of tiles go to the CTAs one by
+// one, and clusters of `split` CTAs share what is left of them, if that is at most one tile for every cluster (Q3_K
+// 11008 x 4096, M = 300: 172 tiles of 160 tokens are a wave of 148 and 24 more; 53 -> 43 us). The model below (clocks; fitted to single tiles on all SMs, Q4_K, K = 16384: a K step took 206 / 218 / 290 / 466 ns at
+// 16 / 64 / 128 / 256 tokens, every other format within a fifth of that or slower at the narrow end) picks the pair of both
 // that ends first: narrow tiles are bound by the decode, wide ones by MMA and power, a tile costs some fixed clocks
 // for its pipeline fill and read-out, and a cluster some more to add its pieces.
 struct GemmPlan {
-    int tile_m, n_tiles_n, n_tiles_m, split, grid;
-    size_t x_bytes;
+    int tile_m, n_tiles_n, n_tiles_m, split, n_full, grid;
 };
 constexpr double kStepMin = 400.0, kStepBase = 200.0, kStepToken = 2.7;
 constexpr int kFixedCycles = 4000;
 
-GemmPlan plan_gemm(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows, int sms) {
+GemmPlan plan_gemm(int64_t n_out, int64_t n_in, int64_t rows, int sms, const int *clusters) {
     GemmPlan g;
     g.n_tiles_n = (int)((n_out + kTileN - 1) / kTileN);
     const int k_blocks = (int)(n_in / 256), m_max = (int)(rows >= kMaxTileM ? kMaxTileM : (rows + 15) / 16 * 16);
@@ -1247,29 +1305,60 @@ GemmPlan plan_gemm(int x_dtype, int64_t n_out, int64_t n_in, int64_t rows, int s
         if (nm > 1 && (tm & (kYChunk - 1)) != 0) continue;   // whole chunks: a store must not reach into the next tile's tokens
         const long long tiles = (long long)g.n_tiles_n * nm;
         const double wide = kStepBase + kStepToken * tm, step = wide > kStepMin ? wide : kStepMin;
-        for (int s = 1; s <= kMaxSplit; s *= 2) {
-            if (s > 1 && (s > k_blocks || tiles * s > sms * 15 / 16)) break;   // one wave of clusters only
-            const long long waves = (tiles * s + sms - 1) / sms;
-            const double t = waves * (4.0 * ((k_blocks + s - 1) / s) * step + tm * 12.0) + kFixedCycles + (s > 1 ? 1500.0 + tm * 8.0 : 0.0);
+        for (int s = 1; s <= kMaxSplit && s <= k_blocks; s++) {
+            const long long ctas = s > 1 ? (long long)s * clusters[s] : sms, waves = tiles / ctas, left = tiles - waves * ctas;
+            if (s > 1 && (left == 0 || left > clusters[s])) continue;
+            double t = waves * (4.0 * k_blocks * step + tm * 12.0) + kFixedCycles;
+            if (left > 0) t += 4.0 * ((k_blocks + s - 1) / s) * step + tm * 12.0 + (s > 1 ? 1500.0 + tm * 8.0 : 0.0);
             if (g.tile_m == 0 || t < best * 0.98) {   // a smaller tile or more pieces have to pay
                 best = t;
                 g.tile_m = tm;
                 g.n_tiles_m = nm;
                 g.split = s;
+                g.n_full = (int)(s > 1 ? waves * ctas : tiles);
+                g.grid = (int)(waves > 0 ? ctas : left * s);
             }
         }
     }
-    const long long ctas = (long long)g.n_tiles_n * g.n_tiles_m * g.split;
-    g.grid = (int)(ctas < sms ? ctas : sms);
-    g.x_bytes = x_dtype == KRK_CUDA_X_F32 ? (((size_t)rows * (size_t)n_in * sizeof(__half) + 255) & ~(size_t)255) : 0;
     return g;
+}
+
+// How many clusters of 1..kMaxSplit CTAs (one per SM) the current device holds at a time; looked up once per device.
+const int *cluster_counts(int sms) {
+    static std::mutex mu;
+    static int counts[64][kMaxSplit + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    std::lock_guard<std::mutex> lk(mu);
+    int *c = counts[dev];
+    if (c[1] == 0) {
+        auto kernel = gemm_tc_kernel<KRK_CUDA_Q4_K, kDense>;   // every dense form fills an SM alike
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+        for (int s = 2; s <= kMaxSplit; s++) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(sms / s * s));
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = kSmemMax;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)s;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&c[s], kernel, &cfg) != cudaSuccess) c[s] = 0;   // none: tiles are not shared
+        }
+        (void)cudaGetLastError();
+        c[1] = sms;
+    }
+    return c;
 }
 
 template <int WT>
 int launch_dense(GemmParams &p, const GemmPlan &g, const uint8_t *w, const __half *xh, cudaStream_t st, const float *x_f32) {
     CUtensorMap x_map, y_map;
     WMaps<kDense> w_maps;
-    const size_t smem = layout<WT>(p, (long long)g.n_tiles_n * g.n_tiles_m * g.split <= g.grid);
+    set_divisions(p, g.n_tiles_m, (int64_t)g.n_tiles_n * g.n_tiles_m);
+    const size_t smem = layout<WT>(p, g.n_full == 0 || (g.n_full <= g.grid && g.split == 1));
     if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.n_in, p.rows, (size_t)p.n_in * sizeof(__half), kBK, p.tile_m,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !encode_w_maps<WT>(w_maps.m, w, p.n_out, p.row_bytes, kTileN))
@@ -1290,7 +1379,7 @@ int launch_dense(GemmParams &p, const GemmPlan &g, const uint8_t *w, const __hal
 
 int run_dense(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, int64_t n_out, int64_t n_in, int64_t rows, __half *x_copy,
               int *status, int sms, cudaStream_t st) {
-    const GemmPlan g = plan_gemm(x_dtype, n_out, n_in, rows, sms);
+    const GemmPlan g = plan_gemm(n_out, n_in, rows, sms, cluster_counts(sms));
     GemmParams p{};
     p.y = y;
     p.n_out = n_out;
@@ -1300,6 +1389,7 @@ int run_dense(float *y, const void *x, int x_dtype, const uint8_t *w, int wt, in
     p.n_tiles_n = g.n_tiles_n;
     p.n_tiles_m = g.n_tiles_m;
     p.split = g.split;
+    p.n_full = g.n_full;
     p.row_bytes = (int)row_bytes(wt, n_in);
     p.y_tma = ((reinterpret_cast<uintptr_t>(y) & 15) == 0 && (n_out % 4) == 0) ? 1 : 0;
     p.status = status;
@@ -1316,6 +1406,7 @@ int launch_experts(GemmParams &p, const ExpertGemm &e, cudaStream_t st) {
     WMaps<KIND> w_maps;
     constexpr int kRows = KIND == kGateUp ? kTileN / 2 : kTileN;   // rows of one matrix in a weight tile
     p.row_bytes = (int)row_bytes(WT, e.n_in);
+    set_divisions(p, p.n_tiles_n, (int64_t)e.max_groups * p.n_tiles_n);
     const size_t smem = layout<WT>(p, false);
     if (!encode_2d(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, e.x, e.n_in, e.x_rows, (size_t)e.n_in * sizeof(__half), kBK, kGroupBox,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||

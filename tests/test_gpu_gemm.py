@@ -170,3 +170,11 @@ def test_gemm_stages_are_not_refilled_while_being_read(cuda, oracle, wt):
         y_ref = oracle.gemm(x, w[sel], wt, len(sel), n_in, rows=rows, threads=8)
         ok, worst = bound_ok(y[0][:, sel], y_ref, oracle.dequant_rows(w[sel], wt, len(sel), n_in), x, GEMM_TOL)
         assert ok, worst
+
+
+@pytest.mark.parametrize("wt", [synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q3_K])
+def test_gemm_left_over_tiles_are_shared(cuda, oracle, wt):
+    """A few tiles more than whole waves: clusters share the tiles left over (one CTA each for the rest), with pieces of
+    unequal length, clusters without a tile, a last weight tile of one row and outputs that float4 stores cannot describe."""
+    for n_out, n_in, rows in ((19200, 2304, 40), (19201, 1280, 40), (11008, 1024, 300), (128 * 149, 2048, 256)):
+        run_gemm(cuda, oracle, wt, n_out, n_in, rows, SEED + 140 + rows, check_rows=np.unique(np.r_[np.arange(0, n_out, 61), n_out - 1]))
