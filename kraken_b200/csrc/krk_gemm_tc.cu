@@ -1348,7 +1348,12 @@ const int *cluster_counts(int sms) {
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&c[s], kernel, &cfg) != cudaSuccess) c[s] = 0;   // none: tiles are not shared
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;   // none: tiles are not shared
+            // Odd sizes do not pack that densely while the CTAs of the kernel before leave, and a cluster that comes late
+            // costs a wave (Q3_K 11008 x 4096, M = 300 behind the copy of f32 activations, 45 clusters of three: 66 us; 74 of
+            // two: 50).
+            c[s] = (s & 1) ? (n > 3 ? n - 3 : 0) : n;
         }
         (void)cudaGetLastError();
         c[1] = sms;
