@@ -115,7 +115,7 @@ int krk_cuda_gemv_group(void *const host_y[], const void *const host_x[],
                         int fuse_silu_pair, void *stream);
 
 /* Prefill GEMM on the tensor cores: y[rows][n_out] = x[rows][n_in] . W^T, W decoded to
- * f16 tiles in shared memory, f32 accumulation. Replaces Backend::gemm at rows > 8
+ * f16 tiles in tensor memory, f32 accumulation. Replaces Backend::gemm at rows > 8
  * (src/hip/backend_hip.hip:3284-3325 -> src/hip/kernels/gemm.hpp:621-970). x is f16
  * (KRK_CUDA_X_F16) or f32 (KRK_CUDA_X_F32, converted to f16 into the workspace first).
  * n_in must be a multiple of 256. */
@@ -191,11 +191,11 @@ struct krk_cuda_expert_bank {
  * elsewhere contribute nothing (a shard's partial sum). Replaces the per-expert loop /
  * moe_decode_batch / Backend::moe_dispatch (src/engine.cpp:12353-, 10896-11060;
  * include/krk/backend.hpp:1001-1009). ids/wts come from krk_cuda_route.
- * n_tok 1..8 (decode): the streaming GEMV over device-side matrix tables, ids never leave the device.
- * n_tok > 8 (prefill): expert-major, the reference's grouped form (src/engine.cpp:12353-12690; device twin
- * src/hip/kernels/moe_table.hpp:463-534): the plan is built on the device, its per-expert row counts are read
- * back once (this call synchronises the stream once), then per expert gather_rows -> gate / up / down as
- * tensor-core GEMMs (GEMVs for up to 8 rows) -> silu_mul -> scatter_axpy_rows in ascending expert id.
+ * ids never leave the device and nothing is read back. A few picks: the streaming GEMV over device-side matrix
+ * tables, an entry per pick. Decode batches and prefill: expert-major, the reference's grouped form
+ * (src/engine.cpp:12353-12690; device twin src/hip/kernels/moe_table.hpp:463-534), planned on the device: experts of
+ * few rows as streaming entries, experts of more rows as groups of one tensor-core launch per product, then the
+ * weighted sum in ascending expert id.
  * workspace: krk_cuda_moe_workspace_bytes() bytes of device memory, 256-byte aligned. */
 size_t krk_cuda_moe_workspace_bytes(const struct krk_cuda_expert_bank *bank, int k, int64_t n_tok);
 int krk_cuda_moe_ffn(void *y_f32, const void *x_f32, const void *ids_i32, const void *wts_f32,
