@@ -134,3 +134,17 @@ def test_topk_slice_edges(cuda, oracle, n, k):
     lg[2::97] = 0.0
     check_topk(cuda, oracle, lg, k)
     check_topk(cuda, oracle, np.minimum(lg, np.float32(0.25)), k)   # the top is one run of equals
+
+
+@pytest.mark.parametrize("n", [1, 31, 2048, 2049, 70000])
+def test_topk_of_one(cuda, oracle, n):
+    """k = 1 selects by a maximum: equal greatest keys go to the lowest id, within a slice and across slices; rows of
+    nothing but -infinity; the last key of the row."""
+    rng = np.random.default_rng(SEED + n)
+    lg = rng.standard_normal(n).astype(np.float32)
+    check_topk(cuda, oracle, lg, 1)
+    lg[rng.integers(0, n, 9)] = 7.0
+    check_topk(cuda, oracle, lg, 1)
+    lg[:] = -np.inf
+    lg[-1] = -1e30
+    check_topk(cuda, oracle, lg, 1)
