@@ -7,6 +7,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <string>
 
 #include "krk_cuda.h"
 
@@ -43,24 +46,39 @@ CudaBackend *CudaBackend::make(int device_index, std::string *err) {
         if (err) *err = e != cudaSuccess ? cudaGetErrorString(e) : "device index out of range";
         return nullptr;
     }
-    cudaDeviceProp prop;
-    if ((e = cudaSetDevice(device_index)) != cudaSuccess ||
-        (e = cudaGetDeviceProperties(&prop, device_index)) != cudaSuccess) {
+    if ((e = cudaSetDevice(device_index)) != cudaSuccess) {
         if (err) *err = cudaGetErrorString(e);
         return nullptr;
     }
-    if (prop.major != 10) {
-        if (err) *err = std::string("device is sm_") + std::to_string(prop.major * 10 + prop.minor) +
-                        "; this backend is built for sm_100a only";
+    // The device's properties take 3 to 11 ms to ask for: once per device.
+    struct Facts {
+        int sm = 0;
+        std::string describe;
+    };
+    static std::mutex mu;
+    static std::map<int, Facts> known;
+    std::lock_guard<std::mutex> lk(mu);
+    Facts &f = known[device_index];
+    if (f.sm == 0) {
+        cudaDeviceProp prop;
+        if ((e = cudaGetDeviceProperties(&prop, device_index)) != cudaSuccess) {
+            if (err) *err = cudaGetErrorString(e);
+            return nullptr;
+        }
+        char buf[256];
+        std::snprintf(buf, sizeof buf, "cuda:%d %s sm_%d%d %d SMs %.0f GiB", device_index, prop.name, prop.major,
+                      prop.minor, prop.multiProcessorCount, (double)prop.totalGlobalMem / (1 << 30));
+        f.describe = buf;
+        f.sm = prop.major * 10 + prop.minor;
+    }
+    if (f.sm / 10 != 10) {
+        if (err) *err = std::string("device is sm_") + std::to_string(f.sm) + "; this backend is built for sm_100a only";
         return nullptr;
     }
     CudaBackend *be = new CudaBackend();
     be->device_ = device_index;
     be->stream_ = nullptr;   // the default stream, like the reference (backend.hpp:775-779)
-    char buf[256];
-    std::snprintf(buf, sizeof buf, "cuda:%d %s sm_%d%d %d SMs %.0f GiB", device_index, prop.name, prop.major,
-                  prop.minor, prop.multiProcessorCount, (double)prop.totalGlobalMem / (1 << 30));
-    be->describe_ = buf;
+    be->describe_ = f.describe;
     return be;
 }
 
