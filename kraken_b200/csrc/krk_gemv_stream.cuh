@@ -542,16 +542,13 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
         load_slice<WT>(xr, at(u), f, mxb, live(u));
     }
     mxb = __reduce_max_sync(0xFFFFFFFFu, mxb);
-    // inv = kFixedOne / max and its counterpart s, each within a unit in the last place (|x * inv| <= 2^22 then); a maximum
-    // too small for that quotient is scaled by a power of two instead, and a non-finite activation makes the output NaN as
-    // it would in f32
+    // |x * inv| <= 2^22 over the whole f32 range: where the quotient would overflow, a power of two takes its place; a
+    // non-finite activation makes the output NaN
     const float mx = __uint_as_float(mxb);
-    float rcp;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp) : "f"(mx));
-    float inv = fmaf(rcp, fmaf(-mx, rcp, 1.0f), rcp) * kFixedOne, s = mx * (1.0f / kFixedOne);
-    if (mx < 1e-30f) {
-        inv = 2.658455991569832e36f;    // 2^121
-        s = 3.7615819226313200e-37f;    // 2^-121
+    float inv = __fdiv_rn(kFixedOne, mx), s = __fdiv_rn(mx, kFixedOne);
+    if (mx < 1.25e-32f) {
+        inv = 1.7014118346046923e38f;   // 2^127
+        s = 5.877471754111438e-39f;     // 2^-127
     }
     if (mxb > 0x7F7FFFFFu) {
         inv = 0.0f;

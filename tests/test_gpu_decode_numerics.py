@@ -1,0 +1,42 @@
+"""What the decode GEMV's fixed-point activations promise: the range of finite activations they cover."""
+import numpy as np
+import pytest
+
+from kraken_b200 import synth
+
+pytestmark = pytest.mark.gpu
+SEED = synth.BASE_SEED + 900
+FORMATS = [synth.Q8_0, synth.Q4_0, synth.Q4_K, synth.Q6_K, synth.Q5_0, synth.Q5_1, synth.Q5_K, synth.Q2_K, synth.Q3_K, synth.IQ4_NL]
+# bytes of a block, offsets of its f16 scales
+SCALES = {synth.Q8_0: (34, [0]), synth.Q4_0: (18, [0]), synth.Q5_0: (22, [0]), synth.Q5_1: (24, [0, 2]), synth.IQ4_NL: (18, [0]),
+          synth.Q2_K: (84, [80, 82]), synth.Q3_K: (110, [108]), synth.Q4_K: (144, [0, 2]), synth.Q5_K: (176, [0, 2]), synth.Q6_K: (210, [208])}
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("wt", FORMATS)
+def test_finite_activations_of_any_size(cuda, oracle, wt):
+    """The activation's scale is its largest magnitude over 2^22 - 1, from 1e38 (where a reciprocal of the maximum is a
+    subnormal number) down past 1.2e-32 (where 2^22 over the maximum is no f32 any more)."""
+    n_out, n_in = 48, 1024
+    w = synth.weights(wt, n_out, n_in, SEED, stream=wt)
+    size, fields = SCALES[wt]
+    blocks = w.reshape(-1, size)
+    for at in fields:   # small weights: the sums stay inside the f32 range
+        d = (1e-6 * (1.0 + np.arange(len(blocks)) % 7)).astype(np.float16)
+        blocks[:, at:at + 2] = d.view(np.uint8).reshape(-1, 2)
+    x1 = np.clip(synth.activations(2, n_in, SEED), -3.0, 3.0)
+    w64 = oracle.dequant_rows(w, wt, n_out, n_in).astype(np.float64)
+    for size in (1e38, 3e37, 1.0, 3e-30, 1e-31, 6e-32, 1e-32, 3e-33):
+        x = (x1 * np.float32(size)).astype(np.float32)
+        assert np.isfinite(x).all()
+        for rows in (1, 2):
+            want = x[:rows].astype(np.float64) @ w64.T
+            y = cuda.gemv(dev(x[:rows]), dev(w), wt, n_out, n_in).cpu().numpy()
+            assert np.abs(want).max() < 1e38
+            lim = 2e-6 * np.linalg.norm(w64, axis=1)[None] * np.linalg.norm(x[:rows].astype(np.float64), axis=1)[:, None]
+            err = np.abs(y.astype(np.float64) - want)
+            assert (err <= lim).all(), (size, rows, float((err / lim).max()))
