@@ -573,8 +573,8 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
 // A fragments of rows g and g+8, column g of the B fragment (limb g%3 of activation row g/3 of
 // the column group), and accumulator columns 2t, 2t+1.
 
-// Column groups that go through the MMAs (32-value block formats; the super-block formats multiply all NG, two rows of
-// four columns each). One or two groups carry two activation rows each in columns 0..5. The
+// Column groups that go through the MMAs (32-value block formats). One or two groups carry two activation rows each in
+// columns 0..5, and so does the one group of the super-block formats at one or two activation rows. The
 // form for five to eight rows has four groups of outputs but multiplies only three: rows 0..5 sit in columns 0..5
 // of groups 0..2 and rows 6 and 7 in the spare columns 6 and 7, limb mg of the row in group mg, so that 24 columns
 // carry 8 rows x 3 limbs with none to spare.
@@ -586,15 +586,18 @@ template <int NG>
 struct Accum {
     float f[NG][4];   // [group][(row g | g+8) x (col 2t | 2t+1)], already times the block scale d
 };
-// The super-block formats. A lane holds two neighbouring columns of every column group, and the columns are dealt so that
-// all it holds belongs to its own activation rows: a unit's integer sums, their limb weights and the minimum term then fold
-// into one number per weight row and activation row (a quarter of the registers of a sum per limb).
-//   Three and more rows: lane t looks after rows t and t + 4. Group 0 carries limbs 0 and 1 of row t in columns 2t and
-//   2t + 1, group 1 (five and more rows) the same of row t + 4, the last group limb 2 of both: 24 limb columns in
-//   three groups, and nothing is left to add between lanes at the end of a tile.
-//   One or two rows: one group, row 0 in columns 0..3 and row 1 in 4..7 (the fourth column of each unused).
-// The minimum term's chunk sums (four limbs) lie the same way: limbs 0, 1 then 2, 3 of row t, then of row t + 4; with one
-// or two rows the four limbs of a row in its four columns.
+// The super-block formats at one or two activation rows: the same, with a sum of its own for the minimum term.
+struct AccumPair {
+    float f[1][4];
+    float m[4];   // dmin * sum(min_c * sum_X_c), columns = 4 limbs x 2 activation rows
+};
+// The super-block formats at three and more rows, whose registers do not hold a sum per limb. A lane holds two neighbouring
+// columns of every column group, and the columns are dealt so that all it holds belongs to its own activation rows: a
+// unit's integer sums, their limb weights and the minimum term then fold into one number per weight row and activation row
+// (a quarter of the registers). Lane t looks after rows t and t + 4. Group 0 carries limbs 0 and 1 of row t in columns 2t
+// and 2t + 1, group 1 (five and more rows) the same of row t + 4, the last group limb 2 of both: 24 limb columns in
+// three groups, and nothing is left to add between lanes at the end of a tile. The minimum term's chunk sums (four limbs)
+// lie the same way: limbs 0, 1 then 2, 3 of row t, then of row t + 4.
 template <int NG>
 constexpr int kFoldGroups = NG == 4 ? 3 : NG;
 template <int NG>
@@ -603,26 +606,34 @@ template <int NG>
 struct AccumFold {
     float a[kFoldRows<NG>][2];   // [row t, t + 4][weight row g, g + 8]
 };
-// acc += d * (limb sums of a unit), dA and dB the scales of weight rows g and g + 8
 template <int NG>
-__device__ __forceinline__ void fold(AccumFold<NG> &acc, float dA, float dB, const int (&I)[NG][4], int t) {
-    if constexpr (NG == 1) {
-        const float w0 = t & 1 ? 1.0f : 65536.0f, w1 = t & 1 ? 0.0f : 256.0f;
-        acc.a[0][0] = fmaf(dA, fmaf(w0, (float)I[0][0], w1 * (float)I[0][1]), acc.a[0][0]);
-        acc.a[0][1] = fmaf(dB, fmaf(w0, (float)I[0][2], w1 * (float)I[0][3]), acc.a[0][1]);
-    } else {
+using AccumSuper = std::conditional_t<NG == 1, AccumPair, AccumFold<NG>>;
+// acc += d * (limb sums of a unit), dA and dB the scales of weight rows g and g + 8
+__device__ __forceinline__ void add_unit(AccumPair &acc, float dA, float dB, const int (&I)[1][4]) {
+    acc.f[0][0] = fmaf(dA, (float)I[0][0], acc.f[0][0]);
+    acc.f[0][1] = fmaf(dA, (float)I[0][1], acc.f[0][1]);
+    acc.f[0][2] = fmaf(dB, (float)I[0][2], acc.f[0][2]);
+    acc.f[0][3] = fmaf(dB, (float)I[0][3], acc.f[0][3]);
+}
+template <int NG>
+__device__ __forceinline__ void add_unit(AccumFold<NG> &acc, float dA, float dB, const int (&I)[NG][4]) {
 #pragma unroll
-        for (int h = 0; h < kFoldRows<NG>; h++) {
-            constexpr int L = kFoldGroups<NG> - 1;
-            acc.a[h][0] = fmaf(dA, fmaf(65536.0f, (float)I[h][0], fmaf(256.0f, (float)I[h][1], (float)I[L][h])), acc.a[h][0]);
-            acc.a[h][1] = fmaf(dB, fmaf(65536.0f, (float)I[h][2], fmaf(256.0f, (float)I[h][3], (float)I[L][2 + h])), acc.a[h][1]);
-        }
+    for (int h = 0; h < kFoldRows<NG>; h++) {
+        constexpr int L = kFoldGroups<NG> - 1;
+        acc.a[h][0] = fmaf(dA, fmaf(65536.0f, (float)I[h][0], fmaf(256.0f, (float)I[h][1], (float)I[L][h])), acc.a[h][0]);
+        acc.a[h][1] = fmaf(dB, fmaf(65536.0f, (float)I[h][2], fmaf(256.0f, (float)I[h][3], (float)I[L][2 + h])), acc.a[h][1]);
     }
 }
-// acc -= dmin * (minimums times group mg of the chunk sums)
+// the minimum term: dmin * (minimums times group mg of the chunk sums)
+__device__ __forceinline__ void add_min(AccumPair &acc, float nA, float nB, const int (&c)[4], int) {
+    acc.m[0] = fmaf(nA, (float)c[0], acc.m[0]);
+    acc.m[1] = fmaf(nA, (float)c[1], acc.m[1]);
+    acc.m[2] = fmaf(nB, (float)c[2], acc.m[2]);
+    acc.m[3] = fmaf(nB, (float)c[3], acc.m[3]);
+}
 template <int NG>
-__device__ __forceinline__ void fold_min(AccumFold<NG> &acc, float nA, float nB, const int (&c)[4], int mg, int t) {
-    const bool low = NG == 1 ? (t & 1) : (mg & 1);   // limbs 2 and 3 (weights 2^8, 1), else 0 and 1 (2^24, 2^16)
+__device__ __forceinline__ void add_min(AccumFold<NG> &acc, float nA, float nB, const int (&c)[4], int mg) {
+    const bool low = mg & 1;   // limbs 2 and 3 (weights 2^8, 1), else 0 and 1 (2^24, 2^16)
     const float w0 = low ? -256.0f : -16777216.0f, w1 = low ? -1.0f : -65536.0f;
     const int h = NG == 4 ? mg >> 1 : 0;
     acc.a[h][0] = fmaf(nA, fmaf(w0, (float)c[0], w1 * (float)c[1]), acc.a[h][0]);
@@ -634,6 +645,10 @@ __device__ __forceinline__ void accum_zero(Accum<NG> &a) {
     for (int i = 0; i < NG; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) a.f[i][j] = 0.0f;
+}
+__device__ __forceinline__ void accum_zero(AccumPair &a) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) a.f[0][j] = a.m[j] = 0.0f;
 }
 template <int NG>
 __device__ __forceinline__ void accum_zero(AccumFold<NG> &a) {
@@ -651,10 +666,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
     for (int mg = 0; mg < NG; mg++) {
         int r = 2 * mg + (g % 6) / 3, limb = g % 3;
         int rs = 2 * mg + g / 4, ls = g % 4;   // chunk sums
-        if (FOLD && NG == 1) {
-            r = g >> 2;
-            limb = min(g & 3, 2);
-        } else if (FOLD) {   // see AccumFold
+        if (FOLD) {   // see AccumFold
             const bool last = mg >= kFoldGroups<NG> - 1;
             r = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
             limb = last ? 2 : g & 1;
@@ -673,7 +685,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
 // same position; the nibbles follow them.
 template <int NG, bool FIFTH>
 __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, AccumFold<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, AccumSuper<NG> &acc) {
     constexpr int kQs = FIFTH ? 48 : 16;
     const uint4 hA = *reinterpret_cast<const uint4 *>(rowA);
     const uint4 hB = *reinterpret_cast<const uint4 *>(rowB);
@@ -721,7 +733,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
         }
     }
     const float dA = half_lo(hA.x), dB = half_lo(hB.x);
-    fold<NG>(acc, dA, dB, I, t);
+    add_unit(acc, dA, dB, I);
     // min term, also exact: one k16 MMA of the 8 mins of the super-block (k slots 0..7) against the
     // per-chunk sums of X, held as 4 limbs x 2 activation rows in the 8 columns
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
@@ -731,7 +743,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 5) + 4 * (t & 1));
         int cc[4];
         mma_s8_k16(cc, a0, a1, b0);
-        fold_min<NG>(acc, nA, nB, cc, mg, t);
+        add_min(acc, nA, nB, cc, mg);
     }
 }
 
@@ -1148,7 +1160,7 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
 
 template <int NG, int ODD>
 __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, AccumFold<NG> &acc) {
+                                          int t, AccumSuper<NG> &acc) {
     int I[NG][4];
 #pragma unroll
     for (int mg = 0; mg < kFoldGroups<NG>; mg++)
@@ -1197,7 +1209,7 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
     }
     const float dA = 0.25f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkA + 208)));
     const float dB = 0.25f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkB + 208)));
-    fold<NG>(acc, dA, dB, I, t);
+    add_unit(acc, dA, dB, I);
 }
 
 // A Q2_K super-block (src/quant.cpp:398-424): 16 bytes of (scale | min << 4), 64 bytes of 2-bit quants, d, dmin;
@@ -1207,7 +1219,7 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
 // sums of X (acc.m, as for Q4_K).
 template <int NG>
 __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, AccumFold<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, AccumSuper<NG> &acc) {
     const uint32_t *wa = reinterpret_cast<const uint32_t *>(blkA), *wb = reinterpret_cast<const uint32_t *>(blkB);
     uint32_t scA[4], scB[4];
 #pragma unroll
@@ -1243,13 +1255,13 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
     const uint32_t hA = wa[20], hB = wb[20];
     const float dA = half_lo(hA), dB = half_lo(hB), nA = half_hi(hA), nB = half_hi(hB);
     const uint32_t m0 = (wa[t] >> 4) & 0x0F0F0F0Fu, m1 = (wb[t] >> 4) & 0x0F0F0F0Fu;   // k slot j = group j: lane t brings 4t..4t+3
-    fold<NG>(acc, dA, dB, I, t);
+    add_unit(acc, dA, dB, I);
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 4) + 4 * t);
         int cc[4];
         mma_s8_k16(cc, m0, m1, b0);
-        fold_min<NG>(acc, nA, nB, cc, mg, t);
+        add_min(acc, nA, nB, cc, mg);
     }
 }
 
@@ -1260,7 +1272,7 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
 // 2 bytes off a word boundary (MODE as for Q6_K).
 template <int NG, int MODE>
 __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, AccumFold<NG> &acc) {
+                                          int t, AccumSuper<NG> &acc) {
     uint32_t SA[4], SB[4];
     {
         const uint32_t a0 = ld_q6<MODE>(blkA, 96), a1 = ld_q6<MODE>(blkA, 100), a2 = ld_q6<MODE>(blkA, 104);
@@ -1312,7 +1324,7 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
     }
     const float dA = 0.03125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkA + 108)));
     const float dB = 0.03125f * __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(blkB + 108)));
-    fold<NG>(acc, dA, dB, I, t);
+    add_unit(acc, dA, dB, I);
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------
@@ -1346,7 +1358,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     static_assert(!SINGLE || ((WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q4_0) && NG == 1), "the single-row forms are Q4_K and Q4_0");
     const int tps = STACK ? p.tps : 1;
     constexpr int kGroups = consumer_groups(NG), kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
-    constexpr bool kFold = block_size(WT) == 256 && !SINGLE;   // AccumFold
+    constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
     using F = Fmt<WT>;
     using SmemT = Smem<NG>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1557,7 +1569,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const int8_t *bp[NG], *sp[NG];
     const float *fe[NG], *fo[NG];   // Q5_1: per-block sums of the even / odd activation row of each column group
     float xs[2 * NG];   // this warp's scale of each activation row (kFold: of its own rows, xs[0] and xs[1])
-    std::conditional_t<kFold, AccumFold<NG>, Accum<NG>> acc;
+    std::conditional_t<kSuper, AccumSuper<NG>, Accum<NG>> acc;
     AccumSingle acs;
     accum_zero(acc);
     acs.f[0] = acs.f[1] = acs.m[0] = acs.m[1] = acs.m[2] = acs.m[3] = 0.0f;
@@ -1632,7 +1644,6 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     xs[r] = row < p.rows ? sm->scale[NG == 1 ? 0 : wid][row] : 0.0f;
                 }
             }
-            if (kFold && NG == 1) xs[0] = t < 2 ? xs[0] : xs[1];
             prepared = x;
             prepared_row = my_row;
             if (!SINGLE) lane_planes<NG, kFold>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
@@ -1747,26 +1758,23 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
 #pragma unroll
                      for (int b = 0; b < 2; b++) {
                          o[h][b] = acc.a[h][b] * xs[h];
-                         if (NG == 1) o[h][b] += __shfl_xor_sync(0xFFFFFFFFu, o[h][b], 1);   // lanes 0, 1: row 0; 2, 3: row 1
                      }
                  accum_zero(acc);
                  wait_phase(smem_u32(&sm->red_empty[rslot]), rphase ^ 1, gave_up, p.status);
-                 if (NG > 1 || (t & 1) == 0) {
 #pragma unroll
-                     for (int h = 0; h < kFoldRows<NG>; h++) {
-                         const int r = NG == 1 ? t >> 1 : t + 4 * h;
-                         float *dst = reinterpret_cast<float *>(&sm->red[rslot][wid][r >> 1][g]) + (r & 1);
-                         dst[0] = o[h][0];   // weight row g
-                         dst[2] = o[h][1];   // g + 8
-                     }
+                 for (int h = 0; h < kFoldRows<NG>; h++) {
+                     const int r = t + 4 * h;
+                     float *dst = reinterpret_cast<float *>(&sm->red[rslot][wid][r >> 1][g]) + (r & 1);
+                     dst[0] = o[h][0];   // weight row g
+                     dst[2] = o[h][1];   // g + 8
                  }
              } else {
+                 // minimum columns: limb c%4 (weights 2^24, 2^16, 2^8, 1) of activation row c/4
+                 const float me0 = t == 0 ? 16777216.0f : (t == 1 ? 256.0f : 0.0f), me1 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f);
                  float4 o[NG];
                  if constexpr (SINGLE != 0) {
                      // lane t holds limb t (weights 65536, 256, 1) of rows g and g+8, times 16
-                     // (Q4_0: lane t = 3 holds d * sum of X per block, the -8 of every quant); Q4_K's minimum columns: two
-                     // of four limbs (weights 2^24 .. 1) in lanes 0 and 1
-                     const float me0 = t == 0 ? 16777216.0f : (t == 1 ? 256.0f : 0.0f), me1 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f);
+                     // (Q4_0: lane t = 3 holds d * sum of X per block, the -8 of every quant)
                      const float wl = t == 0 ? 4096.0f : (t == 1 ? 16.0f : (t == 2 ? 0.0625f : (WT == KRK_CUDA_Q4_0 ? -8.0f : 0.0f)));
                      o[0].x = (wl * acs.f[0] - fmaf(me0, acs.m[0], me1 * acs.m[1])) * xs[0];
                      o[0].z = (wl * acs.f[1] - fmaf(me0, acs.m[2], me1 * acs.m[3])) * xs[0];
@@ -1775,7 +1783,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                  } else {
                      // Column c of a group carries limb c%3 (weights 65536, 256, 1) of activation row c/3; this lane
                      // holds columns 2t and 2t+1, so its accumulators enter the even activation row with (we0, we1)
-                     // and the odd one with (wo0, wo1).
+                     // and the odd one with (wo0, wo1). The minimum term is already a per-lane partial sum.
                      const float we0 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f), we1 = t == 0 ? 256.0f : 0.0f;
                      const float wo0 = t == 2 ? 256.0f : 0.0f, wo1 = t == 1 ? 65536.0f : (t == 2 ? 1.0f : 0.0f);
 #pragma unroll
@@ -1792,6 +1800,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                              o[mg].y = fmaf(wo0, acc.f[mg][0], wo1 * acc.f[mg][1]);   // row g,   odd
                              o[mg].z = fmaf(we0, acc.f[mg][2], we1 * acc.f[mg][3]);   // row g+8, even
                              o[mg].w = fmaf(wo0, acc.f[mg][2], wo1 * acc.f[mg][3]);   // row g+8, odd
+                         }
+                         if constexpr (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K) {
+                             const float mo0 = t == 2 ? 16777216.0f : (t == 3 ? 256.0f : 0.0f), mo1 = t == 2 ? 65536.0f : (t == 3 ? 1.0f : 0.0f);
+                             o[mg].x -= fmaf(me0, acc.m[0], me1 * acc.m[1]);
+                             o[mg].y -= fmaf(mo0, acc.m[0], mo1 * acc.m[1]);
+                             o[mg].z -= fmaf(me0, acc.m[2], me1 * acc.m[3]);
+                             o[mg].w -= fmaf(mo0, acc.m[2], mo1 * acc.m[3]);
                          }
                          o[mg].x *= xs[2 * mg];
                          o[mg].y *= xs[2 * mg + 1];

@@ -1,4 +1,7 @@
-"""What the decode GEMV's fixed-point activations promise: the range of finite activations they cover."""
+"""What the decode GEMV's fixed-point activations promise: the range of finite activations they cover, and results that do
+not change from one build to the next."""
+import zlib
+
 import numpy as np
 import pytest
 
@@ -40,3 +43,25 @@ def test_finite_activations_of_any_size(cuda, oracle, wt):
             lim = 2e-6 * np.linalg.norm(w64, axis=1)[None] * np.linalg.norm(x[:rows].astype(np.float64), axis=1)[:, None]
             err = np.abs(y.astype(np.float64) - want)
             assert (err <= lim).all(), (size, rows, float((err / lim).max()))
+
+
+# crc32 of the f32 results, per format: one row, two rows
+RESULTS = {synth.Q8_0: [3056184117, 3582628484], synth.Q4_0: [4275389815, 4277281545], synth.Q4_K: [3915479935, 2426236879],
+           synth.Q6_K: [607611225, 2896286947], synth.Q5_0: [4107378900, 2160153247], synth.Q5_1: [2911803218, 1148909278],
+           synth.Q5_K: [765817051, 716160757], synth.Q2_K: [2228023986, 3771803034], synth.Q3_K: [3856678096, 3514639972],
+           synth.IQ4_NL: [2476352332, 1264748544]}
+
+
+def results(cuda, wt):
+    n_out, n_in = 96, 4096
+    w = dev(synth.weights(wt, n_out, n_in, SEED + 1, stream=wt))
+    i = np.arange(2 * n_in, dtype=np.uint64)
+    x = dev(((i * 2654435761 % (1 << 32)).astype(np.float64) / (1 << 31) - 1.0).astype(np.float32).reshape(2, n_in))
+    return [zlib.crc32(cuda.gemv(x[:rows], w, wt, n_out, n_in).cpu().numpy().tobytes()) for rows in (1, 2)]
+
+
+@pytest.mark.parametrize("wt", FORMATS)
+def test_one_and_two_row_results_keep_their_bits(cuda, wt):
+    """A logit of 250 has steps of 1.5e-5, and the mass over a vocabulary takes exp() of such numbers: a different order of
+    the final f32 sums, each as good as the other, shows there as 2e-5. So the order stays."""
+    assert results(cuda, wt) == RESULTS[wt]
