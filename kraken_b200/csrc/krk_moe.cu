@@ -285,7 +285,7 @@ moe_combine_kernel(const __grid_constant__ MoeParams p) {
     // that grid is complete), and lets the one after it start the same way
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int t = blockIdx.y;
+    const int t = blockIdx.x;
     if (threadIdx.x < 32) {
         // lane s looks at slot s of this token: its place among the slots held here, by expert id
         const int s = threadIdx.x;
@@ -311,7 +311,7 @@ moe_combine_kernel(const __grid_constant__ MoeParams p) {
     __syncthreads();
     const int n = s_n;
     const int64_t n4 = p.n_embd >> 2;   // rows are whole 32-value blocks
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n4; j += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t j = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; j < n4; j += (int64_t)gridDim.y * blockDim.x) {
         // the loads of a batch of eight go out together; the additions keep their order
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         for (int i0 = 0; i0 < n; i0 += 8) {
@@ -684,9 +684,9 @@ size_t moe_workspace_bytes(const krk_cuda_expert_bank *bank, int k, int64_t n_to
 }
 
 static int launch_combine(const MoeParams &p, cudaStream_t st) {
-    const int64_t n4 = p.n_embd / 4;
-    return launched(launch_overlapped(moe_combine_kernel, dim3((unsigned)((n4 + kCombineThreads - 1) / kCombineThreads), (unsigned)p.n_tok),
-                                      dim3(kCombineThreads), st, p));
+    // tokens in x: a chunk of one pick each has 65,536 of them, and y ends at 65,535 (more columns than that are strided over)
+    const int64_t n4 = p.n_embd / 4, cols = (n4 + kCombineThreads - 1) / kCombineThreads;
+    return launched(launch_overlapped(moe_combine_kernel, dim3((unsigned)p.n_tok, (unsigned)(cols < 65535 ? cols : 65535)), dim3(kCombineThreads), st, p));
 }
 
 static MoeParams moe_params(float *y, const float *x, const int32_t *ids, const float *wts, const krk_cuda_expert_bank *bank, int k, int64_t n_tok) {

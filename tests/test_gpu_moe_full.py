@@ -194,3 +194,27 @@ def test_router_steps_and_plan_match_the_host(cuda, oracle):
                     want_wt.append(w_np[t, s])
         want_off.append(len(want_rows))
     assert off.tolist() == want_off and rows.tolist() == want_rows and wt.tolist() == want_wt
+
+
+@pytest.mark.parametrize("k, n_tok", [(1, 65536), (1, 65536 + 70), (2, 32768 + 5)])
+def test_calls_of_more_tokens_than_a_chunk(cuda, k, n_tok):
+    """65,536 picks go through the workspace at a time: a whole chunk of one pick each (more tokens than a grid's y extent
+    holds), and a short last chunk after it, down to one whose experts have too few rows for the tensor cores. f16
+    operands twice in a row: 2e-3, as for any prefill."""
+    import torch
+    n_embd, n_ff, n_exp = 256, 256, 4
+    gate, up, down = (dev(synth.weights(wt, n_exp * 256, 256, SEED + 60, stream=i)) for i, wt in enumerate((synth.Q4_K, synth.Q4_K, synth.Q6_K)))
+    bank = cuda.make_bank(gate, up, down, synth.Q4_K, synth.Q6_K, n_exp, 0, n_embd, n_ff)
+    gen = torch.Generator("cuda").manual_seed(7)
+    x, logits = (torch.randn((n_tok, n), device="cuda", generator=gen) for n in (n_embd, n_exp))
+    x *= 0.05   # (hidden values stay inside the f16 range)
+    y, ids, wts = cuda.moe_ffn_routed(x, logits, k, bank)
+    assert cuda.device_status() == 0
+    g, u, d = (cuda.dequant_rows(w, wt, n_exp * 256, 256).double().view(n_exp, 256, 256) for w, wt in ((gate, synth.Q4_K), (up, synth.Q4_K), (down, synth.Q6_K)))
+    ids, wts, xd = ids.long(), wts.double(), x.double()
+    want = torch.zeros((n_tok, n_embd), device="cuda", dtype=torch.double)
+    for e in range(n_exp):
+        w = (wts * (ids == e)).sum(dim=1, keepdim=True)
+        want += w * ((torch.nn.functional.silu(xd @ g[e].T) * (xd @ u[e].T)) @ d[e].T)
+    rel = ((y.double() - want).norm(dim=1) / want.norm(dim=1).clamp_min(1e-30))
+    assert rel.max().item() < 1e-2 and ((y.double() - want).norm() / want.norm()).item() < 2e-3, rel.topk(5)
