@@ -810,9 +810,9 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
                 else cur.template convert<0>(0, v);
                 // The stage is given back when its bytes ARE in registers: an arrival does not wait for loads in flight, and
                 // while the MMAs and the copies of X keep shared memory busy those took longer than a refill (Q8_0, tiles of
-                // 96 tokens and more: rows of a later stage in the first ones). Hence the address that needs them.
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]) + (cur.loaded() & p.zero));
+                // 96 tokens and more: rows of a later stage in the first ones). Hence the address that needs them, every lane's.
+                const int pending = __any_sync(0xFFFFFFFFu, (cur.loaded() & p.zero) != 0u);
+                if (lane == 0) mbar_arrive(smem_u32(&sm->raw_empty[sr]) + pending);
                 if (++sr == p.n_raw) {
                     sr = 0;
                     pr ^= 1;

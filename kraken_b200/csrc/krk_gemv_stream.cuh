@@ -156,6 +156,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// An arrival that cannot issue before `a` and `b` are there, whatever their values.
+__device__ __forceinline__ void mbar_arrive_after(uint32_t bar, uint32_t a, uint32_t b) {
+    asm volatile("{\n .reg .pred p;\n setp.gt.u32 p, %1, %2;\n @p mbarrier.arrive.shared::cta.b64 _, [%0];\n"
+                 " @!p mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(bar), "r"(a), "r"(b) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -655,6 +660,29 @@ __device__ __forceinline__ void accum_zero(AccumFold<NG> &a) {
 #pragma unroll
     for (int i = 0; i < kFoldRows<NG>; i++) a.a[i][0] = a.a[i][1] = 0.0f;
 }
+// All that a lane has summed, as one word (see the release of a stage).
+template <int N>
+__device__ __forceinline__ uint32_t bits_of(const float (&v)[N]) {
+    uint32_t b = 0u;
+#pragma unroll
+    for (int i = 0; i < N; i++) b ^= __float_as_uint(v[i]);
+    return b;
+}
+template <int NG>
+__device__ __forceinline__ uint32_t bits_of(const Accum<NG> &a) {
+    uint32_t b = 0u;
+#pragma unroll
+    for (int i = 0; i < kMmaGroups<NG>; i++) b ^= bits_of(a.f[i]);
+    return b;
+}
+__device__ __forceinline__ uint32_t bits_of(const AccumPair &a) { return bits_of(a.f[0]) ^ bits_of(a.m); }
+template <int NG>
+__device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
+    uint32_t b = 0u;
+#pragma unroll
+    for (int i = 0; i < kFoldRows<NG>; i++) b ^= bits_of(a.a[i]);
+    return b;
+}
 
 // Byte planes this lane reads its B fragments from, one per column group. A lane whose column
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
@@ -756,7 +784,7 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
 // two-MMA-per-chunk form; lane t keeps limb t of rows g and g+8 (t = 3 multiplies nothing).
 struct AccumSingle {
     float f[2];   // rows g, g+8: limb t of d * sum over sub-blocks, times 16
-    float m[4];   // the min term as in Accum::m of one column group
+    float m[4];   // the min term as in AccumPair
 };
 // The B fragments of a unit (x limbs, chunk sums) are the same for every row tile: a warp that always works
 // on the same K units keeps them in registers (BFrag) instead of reading them from shared memory per tile.
@@ -1731,8 +1759,15 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         }
                     }
                 }
+                // The stage is given back when its words HAVE arrived: an arrival does not wait for shared-memory loads in
+                // flight (see the decode warps of krk_gemm_tc.cu), and the copy of the next stage into this slot would meet
+                // them. All that was loaded is in the sums by now, so the arrival waits for those. Lane 0's do for the warp:
+                // what they were loaded by and multiplied by are instructions of the whole warp, which complete as one.
                 __syncwarp();
-                if (lane == 0) mbar_arrive(empty0 + 8 * slot);
+                if (lane == 0) {
+                    if constexpr (SINGLE != 0) mbar_arrive_after(empty0 + 8 * slot, __float_as_uint(acs.f[0]), __float_as_uint(acs.f[1]));
+                    else mbar_arrive_after(empty0 + 8 * slot, bits_of(acc), 0u);
+                }
                 if (++slot == p.n_stages) {
                     slot = 0;
                     phase ^= 1;

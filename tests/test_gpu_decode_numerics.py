@@ -65,3 +65,22 @@ def test_one_and_two_row_results_keep_their_bits(cuda, wt):
     """A logit of 250 has steps of 1.5e-5, and the mass over a vocabulary takes exp() of such numbers: a different order of
     the final f32 sums, each as good as the other, shows there as 2e-5. So the order stays."""
     assert results(cuda, wt) == RESULTS[wt]
+
+
+# (K = 11008 leaves a ring of few stages beside eight prepared rows; K = 2080 and 5120 are rows that start at any even address)
+@pytest.mark.parametrize("wt, n_out, n_in", [(synth.Q6_K, 3000, 11008), (synth.Q3_K, 3000, 5120), (synth.Q8_0, 3000, 2080), (synth.Q8_0, 5000, 4096),
+                                             (synth.Q4_K, 5000, 11008), (synth.Q4_0, 5000, 4096)])
+def test_stages_are_refilled_only_once_read(cuda, wt, n_out, n_in):
+    """The same call over and over, between calls that fill the ring with other bytes: same bits, and the right sums."""
+    import torch
+    w, other = (dev(synth.weights(wt, n_out, n_in, SEED + 2 + i, stream=wt)) for i in range(2))
+    w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+    for rows in (1, 2, 3, 5, 8):
+        x = dev(synth.activations(rows, n_in, SEED + rows))
+        first = cuda.gemv(x, w, wt, n_out, n_in)
+        lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None]
+        assert ((first.double() - x.double() @ w64.T).abs() <= lim).all()
+        for _ in range(40):
+            cuda.gemv(x, other, wt, n_out, n_in)
+            assert torch.equal(cuda.gemv(x, w, wt, n_out, n_in), first)
+    assert cuda.device_status() == 0
