@@ -41,6 +41,20 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
         if (mats[m].wt != wt) return 0;
     int rc = 0;
     KRK_DISPATCH_WT(wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, st));
+    // Rows whose four limbs (K not a multiple of 256) leave no room for a ring go in two launches: the weights twice through
+    // the ring are far quicker than the warp-per-row kernel once (8 rows of Q8_0 have room up to K of some 5600).
+    if (rc == 0 && rows > 1 && n_in % 256 != 0 && n_mat <= KRK_CUDA_MAX_GROUP) {
+        GemvMat part[KRK_CUDA_MAX_GROUP];
+        for (int m = 0; m < n_mat; m++) part[m] = mats[m];
+        const int first = (rows + 1) / 2;
+        rc = launch_gemv_stream(part, n_mat, n_in, first, accumulate, silu_pair, st);
+        if (rc != 1) return rc;
+        for (int m = 0; m < n_mat; m++) {
+            part[m].x += first * n_in;
+            part[m].y += first * mats[m].n_out;
+        }
+        rc = launch_gemv_stream(part, n_mat, n_in, rows - first, accumulate, silu_pair, st);
+    }
     return rc;
 }
 

@@ -291,8 +291,13 @@ struct Smem {
 __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
 __host__ __device__ inline int plane_stride(int n_in) { return n_in + kPlanePad; }
+// Limbs of an activation: three, or four where K is not a multiple of 256. Those shapes belong to the warp-per-row kernel
+// otherwise, which multiplies in f32; 22 bits against the largest magnitude of a warp's slices are 2 to 9 times as far off
+// (error against f64 of 2.3e-7 to 1.1e-6, f32: 1.2e-7), and the MMA's fourth column was unused.
 template <int WT>
-__host__ __device__ inline int plane_bytes(int n_in, int rows) { return align_up(rows * 3 * plane_stride(n_in), 128); }
+__host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
+template <int WT>
+__host__ __device__ inline int plane_bytes(int n_in, int rows) { return align_up(rows * (fine_limbs<WT>(n_in) ? 4 : 3) * plane_stride(n_in), 128); }
 // Sums of the quantised activation over the stretch of K that shares one minimum or offset: 32 values (2^5) for
 // Q4_K, Q5_K, Q4_0 and Q5_1, 16 for Q2_K.
 template <int WT>
@@ -405,11 +410,9 @@ __device__ __forceinline__ int sext8(int v) { return (v << 24) >> 24; }
 __device__ __forceinline__ uint32_t limbs3(int X) { return ((uint32_t)X + 0x00808080u) ^ 0x00808080u; }   // |X| < 2^23
 __device__ __forceinline__ uint32_t limbs4(int X) { return ((uint32_t)X + 0x80808080u) ^ 0x80808080u; }
 
-// NATURAL: limbs in value order everywhere (rows whose blocks start at any even address, see ld_q6); `live`: the lane's
-// values lie inside the row (the last unit of such a row may be short).
-template <int WT, bool NATURAL>
+template <int WT>
 __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p0,
-                                               int8_t *p1, int8_t *p2, int8_t *sums, int n_chunks, int lane, bool live) {
+                                               int8_t *p1, int8_t *p2, int8_t *sums, int n_chunks, int lane) {
     constexpr int PER = Fmt<WT>::unit_values / 32;
     int total = 0;
 #pragma unroll
@@ -427,13 +430,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
         const uint32_t w2 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u, w1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
         const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], 0x0062), __byte_perm(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
         const int i = k0 + j4;
-        if (NATURAL) {
-            if (live) {
-                *reinterpret_cast<uint32_t *>(p0 + i) = w0;
-                *reinterpret_cast<uint32_t *>(p1 + i) = w1;
-                *reinterpret_cast<uint32_t *>(p2 + i) = w2;
-            }
-        } else if (WT == KRK_CUDA_Q8_0 && ((i >> 5) & 1) == 0) {
+        if (WT == KRK_CUDA_Q8_0 && ((i >> 5) & 1) == 0) {
             // Even blocks start 2 bytes off a word boundary, so their lanes take the quants in the
             // order [0,1,30,31, 2..29]; the limbs follow: pair (e, e+1) lands at position pos(e).
             const int e = i & 31, base = i & ~31;
@@ -491,7 +488,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
         // (Q5_1: the block's offset m enters as m * sum)
         total += __shfl_xor_sync(0xFFFFFFFFu, total, 1);
         total += __shfl_xor_sync(0xFFFFFFFFu, total, 2);
-        if ((lane & 3) == 0 && live) reinterpret_cast<float *>(sums)[k0 >> 5] = (float)total;   // |sum| < 2^28
+        if ((lane & 3) == 0) reinterpret_cast<float *>(sums)[k0 >> 5] = (float)total;   // |sum| < 2^28
     }
     if (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K) {
         // a 32-value chunk is held by 4 consecutive lanes (Q2_K: a 16-value group by 2); |sum| <= 32 * 2^22
@@ -506,6 +503,46 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
             sums[2 * n_chunks + c] = (int8_t)(z >> 8);
             sums[3 * n_chunks + c] = (int8_t)z;
         }
+    }
+}
+
+// The same where K is not a multiple of 256: four limbs, in value order everywhere (rows whose blocks start at any even
+// address, see ld_q6). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
+// `live`: the lane's values lie inside the row (the last unit of such a row may be short).
+template <int WT>
+__device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p, int ps,
+                                                    int8_t *sums, int lane, bool live) {
+    constexpr int PER = Fmt<WT>::unit_values / 32;
+    int total = 0, rest = 0;
+#pragma unroll
+    for (int j4 = 0; j4 < PER; j4 += 4) {
+        uint32_t z[4];   // byte 3: limb 0 (weight 65536) ... byte 0: limb 3 (1/256)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float big = fmaf(f[j4 + j], inv, kMagic);
+            const int X = __float_as_int(big) - 0x4B400000;
+            const int r = __float_as_int(fmaf(fmaf(f[j4 + j], inv, kMagic - big), 256.0f, kMagic)) - 0x4B400000;   // |r| <= 128
+            total += X;
+            rest += r;
+            z[j] = limbs4(X * 256 + r);   // |X| <= 2^22
+        }
+        const uint32_t lo01 = __byte_perm(z[0], z[1], 0x5140), lo23 = __byte_perm(z[2], z[3], 0x5140);   // l3 l3 l2 l2
+        const uint32_t hi01 = __byte_perm(z[0], z[1], 0x7362), hi23 = __byte_perm(z[2], z[3], 0x7362);   // l1 l1 l0 l0
+        if (live) {
+            int8_t *at = p + k0 + j4;
+            *reinterpret_cast<uint32_t *>(at) = __byte_perm(hi01, hi23, 0x7632);
+            *reinterpret_cast<uint32_t *>(at + ps) = __byte_perm(hi01, hi23, 0x5410);
+            *reinterpret_cast<uint32_t *>(at + 2 * ps) = __byte_perm(lo01, lo23, 0x7632);
+            *reinterpret_cast<uint32_t *>(at + 3 * ps) = __byte_perm(lo01, lo23, 0x5410);
+        }
+    }
+    if (WT == KRK_CUDA_Q5_1) {   // the sum over each 32-value block, see quantize_slice
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
+            rest += __shfl_xor_sync(0xFFFFFFFFu, rest, o);
+        }
+        if ((lane & 3) == 0 && live) reinterpret_cast<float *>(sums)[k0 >> 5] = fmaf((float)rest, 0.00390625f, (float)total);
     }
 }
 
@@ -524,15 +561,19 @@ __device__ __forceinline__ void load_slice(const float *__restrict__ x, int k0, 
     for (int j = 0; j < PER; j++) mxb = max(mxb, __float_as_uint(f[j]) & 0x7FFFFFFFu);
 }
 
-// All slices this warp will read of one activation row; returns the row's scale for this warp. SHORT: the last unit may
-// hold fewer values than a full one.
-template <int WT, bool SHORT>
+// All slices this warp will read of one activation row; returns the row's scale for this warp. FINE: four limbs, and the
+// last unit may hold fewer values than a full one.
+template <int WT, bool FINE>
 __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, const StreamParams &p, int8_t *p0, int8_t *sums,
                                                int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 2;
     const int n_chunks = p.n_in >> kSumShift<WT>, ps = plane_stride(p.n_in);
     auto at = [&](int u) { return u * UV + lane * PER; };
-    auto live = [&](int u) { return !SHORT || at(u) < p.n_in; };
+    auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
+    auto quantize = [&](const float (&f)[PER], float inv, int u) {
+        if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
+        else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
+    };
     // the first two slices stay in registers between the max and the quantisation (K <= 4096 for
     // 256-value units); any further ones are read twice
     float held[kHeld][PER];
@@ -550,10 +591,18 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
     // |x * inv| <= 2^22 over the whole f32 range: where the quotient would overflow, a power of two takes its place; a
     // non-finite activation makes the output NaN
     const float mx = __uint_as_float(mxb);
-    float inv = __fdiv_rn(kFixedOne, mx), s = __fdiv_rn(mx, kFixedOne);
-    if (mx < 1.25e-32f) {
-        inv = 1.7014118346046923e38f;   // 2^127
-        s = 5.877471754111438e-39f;     // 2^-127
+    float inv, s;
+    if constexpr (FINE) {   // the power of two that takes the maximum to 2^21 .. 2^22, 2^127 at most
+        const uint32_t e = min(275u - (mxb >> 23), 254u);
+        inv = __uint_as_float(e << 23);
+        s = __uint_as_float(e < 254u ? (254u - e) << 23 : 0x00400000u);
+    } else {
+        inv = __fdiv_rn(kFixedOne, mx);
+        s = __fdiv_rn(mx, kFixedOne);
+        if (mx < 1.25e-32f) {
+            inv = 1.7014118346046923e38f;   // 2^127
+            s = 5.877471754111438e-39f;     // 2^-127
+        }
     }
     if (mxb > 0x7F7FFFFFu) {
         inv = 0.0f;
@@ -562,13 +611,13 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
 #pragma unroll
     for (int j = 0; j < kHeld; j++) {
         const int u = wid + j * kConsumerWarps;
-        if (u < p.units) quantize_slice<WT, SHORT>(held[j], inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane, live(u));
+        if (u < p.units) quantize(held[j], inv, u);
     }
     for (int u = wid + kHeld * kConsumerWarps; u < p.units; u += kConsumerWarps) {
         float f[PER];
         uint32_t m2 = 0u;
         load_slice<WT>(xr, at(u), f, m2, live(u));
-        quantize_slice<WT, SHORT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane, live(u));
+        quantize(f, inv, u);
     }
     return s;
 }
@@ -582,9 +631,9 @@ __device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, con
 // columns 0..5, and so does the one group of the super-block formats at one or two activation rows. The
 // form for five to eight rows has four groups of outputs but multiplies only three: rows 0..5 sit in columns 0..5
 // of groups 0..2 and rows 6 and 7 in the spare columns 6 and 7, limb mg of the row in group mg, so that 24 columns
-// carry 8 rows x 3 limbs with none to spare.
-template <int NG>
-constexpr int kMmaGroups = NG == 4 ? 3 : NG;
+// carry 8 rows x 3 limbs with none to spare. With four limbs (FINE) every group is multiplied, two rows in its eight columns.
+template <int NG, bool FINE>
+constexpr int kMmaGroups = NG == 4 && !FINE ? 3 : NG;
 
 // The 32-value block formats.
 template <int NG>
@@ -672,7 +721,7 @@ template <int NG>
 __device__ __forceinline__ uint32_t bits_of(const Accum<NG> &a) {
     uint32_t b = 0u;
 #pragma unroll
-    for (int i = 0; i < kMmaGroups<NG>; i++) b ^= bits_of(a.f[i]);
+    for (int i = 0; i < NG; i++) b ^= bits_of(a.f[i]);
     return b;
 }
 __device__ __forceinline__ uint32_t bits_of(const AccumPair &a) { return bits_of(a.f[0]) ^ bits_of(a.m); }
@@ -687,14 +736,17 @@ __device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
 // Byte planes this lane reads its B fragments from, one per column group. A lane whose column
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
 // accumulator columns are never looked at, so what it multiplies does not matter.
-template <int NG, bool FOLD>
+template <int NG, bool FOLD, bool FINE>
 __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int n_in, int n_sums, int rows, int g,
                                             const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         int r = 2 * mg + (g % 6) / 3, limb = g % 3;
         int rs = 2 * mg + g / 4, ls = g % 4;   // chunk sums
-        if (FOLD) {   // see AccumFold
+        if (FINE) {
+            r = 2 * mg + (g >> 2);
+            limb = g & 3;
+        } else if (FOLD) {   // see AccumFold
             const bool last = mg >= kFoldGroups<NG> - 1;
             r = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
             limb = last ? 2 : g & 1;
@@ -704,7 +756,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
             r = g;
             limb = mg % 3;
         }
-        bp[mg] = planes + (size_t)(min(r, rows - 1) * 3 + limb) * plane_stride(n_in);
+        bp[mg] = planes + (size_t)(min(r, rows - 1) * (FINE ? 4 : 3) + limb) * plane_stride(n_in);
         sp[mg] = chunk_sum + (size_t)(min(rs, rows - 1) * 4 + ls) * n_sums;
     }
 }
@@ -944,7 +996,7 @@ __device__ __forceinline__ void unit_q4_0_rows(const uint8_t *rowA, const uint8_
         dA *= 0.0625f;
         dB *= 0.0625f;
 #pragma unroll
-        for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+        for (int mg = 0; mg < kMmaGroups<NG, RAG>; mg++) {
             const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 4 * t);
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int c[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};
@@ -1011,7 +1063,7 @@ __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *
         grid(qa, la, ha);
         grid(qb, lb, hb);
 #pragma unroll
-        for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+        for (int mg = 0; mg < kMmaGroups<NG, RAG>; mg++) {
             const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 4 * t);
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int c[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // |sum| <= 32 * 127 * 128 < 2^19
@@ -1077,7 +1129,7 @@ __device__ __forceinline__ void unit_q5_0(const uint8_t *rowA, const uint8_t *ro
         dA *= 0.125f;
         dB *= 0.125f;
 #pragma unroll
-        for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+        for (int mg = 0; mg < kMmaGroups<NG, RAG>; mg++) {
             const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 4 * t);
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int c[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};
@@ -1094,7 +1146,8 @@ __device__ __forceinline__ void unit_q5_0(const uint8_t *rowA, const uint8_t *ro
 // Eight Q5_1 blocks (src/quant.cpp:366-379): scale d, offset m, the mask, the nibbles, all on word boundaries;
 // the value is d * q + m with q = 0..31. The A operand is 8 * q as an unsigned byte; the offset enters as
 // m * (sum of X over the block), which the activation pass leaves per block as a float: the lanes whose columns
-// carry the limb of weight 1 (column 2 of the even, column 5 of the odd activation row of a group) add it.
+// carry the limb of weight 1 (column 2 of the even, column 5 of the odd activation row of a group; of four limbs columns
+// 2 and 6) add it.
 template <int NG, bool RAG>
 __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           const float *const (&fe)[NG], const float *const (&fo)[NG], int t, Accum<NG> &acc, int nb) {
@@ -1110,7 +1163,7 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
         const uint32_t ha = ((qa >> 1) & 0x78787878u) | spread_top((ma >> (16 + 4 * t)) & 0xFu);
         const uint32_t hb = ((qb >> 1) & 0x78787878u) | spread_top((mb >> (16 + 4 * t)) & 0xFu);
 #pragma unroll
-        for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+        for (int mg = 0; mg < kMmaGroups<NG, RAG>; mg++) {
             const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 4 * t);
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int c[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // |sum| <= 32 * 248 * 128 < 2^20
@@ -1118,8 +1171,9 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
             mma_u8_k16_chain(c, ha, hb, b1);
             // (five to eight rows: the weight-1 limbs of rows 6 and 7 are columns 6 and 7 of group 2, in lane t = 3)
             const bool spare = NG == 4 && mg == 2 && t == 3;
-            const float se = t == 1 ? fe[mg][(kbase >> 5) + b] : (spare ? fe[NG - 1][(kbase >> 5) + b] : 0.0f);
-            const float so = t == 2 ? fo[mg][(kbase >> 5) + b] : (spare ? fo[NG - 1][(kbase >> 5) + b] : 0.0f);
+            const int at = (kbase >> 5) + b;
+            const float se = t == 1 ? fe[mg][at] : RAG ? (t == 3 ? fo[mg][at] : 0.0f) : spare ? fe[NG - 1][at] : 0.0f;
+            const float so = RAG ? 0.0f : t == 2 ? fo[mg][at] : spare ? fo[NG - 1][at] : 0.0f;
             acc.f[mg][0] = fmaf(dA, __int_as_float(c[0]) - kMagic, fmaf(oA, se, acc.f[mg][0]));
             acc.f[mg][1] = fmaf(dA, __int_as_float(c[1]) - kMagic, fmaf(oA, so, acc.f[mg][1]));
             acc.f[mg][2] = fmaf(dB, __int_as_float(c[2]) - kMagic, fmaf(oB, se, acc.f[mg][2]));
@@ -1167,7 +1221,7 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
             dB = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(rowB + 34 * b)));
         }
 #pragma unroll
-        for (int mg = 0; mg < kMmaGroups<NG>; mg++) {
+        for (int mg = 0; mg < kMmaGroups<NG, RAG>; mg++) {
             const uint32_t b0 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 4 * t);
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int cc[4];   // (presetting the accumulator to 1.5 * 2^23 to save the int-to-float step is 0.3-3 % slower here)
@@ -1387,6 +1441,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const int tps = STACK ? p.tps : 1;
     constexpr int kGroups = consumer_groups(NG), kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
+    constexpr bool kFine = RAG && !kSuper;   // fine_limbs
     using F = Fmt<WT>;
     using SmemT = Smem<NG>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1649,7 +1704,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             // (stacked tiles: every sub-tile prepares its own copy)
             auto prepare = [&](int r) {
-                return prepare_x_row<WT, RAG && block_size(WT) == 32>(x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in), p, planes + (size_t)(r * 3) * plane_stride(p.n_in),
+                return prepare_x_row<WT, kFine>(x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in), p, planes + (size_t)(r * (kFine ? 4 : 3)) * plane_stride(p.n_in),
                                                                       chunk_sum + (size_t)(r * 4) * (p.n_in >> kSumShift<WT>),
                                                                       stacked_idle ? p.units : my_unit, lane);
             };
@@ -1674,7 +1729,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<NG, kFold>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -1818,12 +1873,14 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                  } else {
                      // Column c of a group carries limb c%3 (weights 65536, 256, 1) of activation row c/3; this lane
                      // holds columns 2t and 2t+1, so its accumulators enter the even activation row with (we0, we1)
-                     // and the odd one with (wo0, wo1). The minimum term is already a per-lane partial sum.
-                     const float we0 = t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f), we1 = t == 0 ? 256.0f : 0.0f;
-                     const float wo0 = t == 2 ? 256.0f : 0.0f, wo1 = t == 1 ? 65536.0f : (t == 2 ? 1.0f : 0.0f);
+                     // and the odd one with (wo0, wo1). The minimum term is already a per-lane partial sum. Four limbs: limb c%4
+                     // (weights 65536, 256, 1, 1/256) of row c/4.
+                     const float w0 = t & 1 ? 1.0f : 65536.0f, w1 = t & 1 ? 0.00390625f : 256.0f;
+                     const float we0 = kFine ? (t < 2 ? w0 : 0.0f) : t == 0 ? 65536.0f : (t == 1 ? 1.0f : 0.0f), we1 = kFine ? (t < 2 ? w1 : 0.0f) : t == 0 ? 256.0f : 0.0f;
+                     const float wo0 = kFine ? (t < 2 ? 0.0f : w0) : t == 2 ? 256.0f : 0.0f, wo1 = kFine ? (t < 2 ? 0.0f : w1) : t == 1 ? 65536.0f : (t == 2 ? 1.0f : 0.0f);
 #pragma unroll
                      for (int mg = 0; mg < NG; mg++) {
-                         if (NG == 4 && mg == 3) {
+                         if (NG == 4 && mg == 3 && !kFine) {
                              // activation rows 6 and 7 rode in columns 6 and 7 (lane t = 3) of groups 0..2, limb mg in group mg
                              const float w0 = t == 3 ? 65536.0f : 0.0f, w1 = t == 3 ? 256.0f : 0.0f, w2 = t == 3 ? 1.0f : 0.0f;
                              o[mg].x = fmaf(w0, acc.f[0][0], fmaf(w1, acc.f[1 % NG][0], w2 * acc.f[2 % NG][0]));
