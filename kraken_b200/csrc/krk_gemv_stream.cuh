@@ -42,7 +42,7 @@
 #include <type_traits>
 #include <unordered_map>
 
-#include "krk_common.cuh"
+#include "krk_chunk.cuh"
 
 namespace krk_cuda {
 
@@ -1432,6 +1432,15 @@ template <int WT>
 constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_size(WT) == 32;
 template <int WT>
 constexpr bool kMayRag = kRagForm<WT> || WT == KRK_CUDA_Q2_K;
+// One result in f32 throughout, by one lane: what an infinity among the activations makes of a row (an infinity of either
+// sign, or a NaN against a zero weight) is not in the limbs, which give a NaN.
+template <int WT>
+__device__ __noinline__ float dot_f32(const uint8_t *w, const float *x, int n_in) {
+    float sum = 0.0f;
+    for (int c = 0; c < n_in >> 5; c++) sum += chunk_dot<WT>(w, c, x);
+    return sum;
+}
+
 template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false>
 __global__ void __launch_bounds__(cta_threads(consumer_groups(NG)), NG == 1 ? 2 : 1)
 gemv_stream_kernel(const __grid_constant__ StreamParams p) {
@@ -1580,6 +1589,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
 #pragma unroll
                     for (int w = 0; w < kConsumerWarps; w++) v += part[w];
                     const int srow = kTileRows * sub + row;   // row inside the stage
+                    if (kFine && v != v && r < p.rows && srow < s.n_rows) {
+                        const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
+                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)(s.row0 + srow) * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
+                    }
                     if (r < p.rows) {
                         if (p.step == 2 && s.which == 0) {
                             if (STACK) sm->gate[sub][i][lane] = v;   // kept for the silu fold with the `up` tile

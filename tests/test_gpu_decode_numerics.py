@@ -106,3 +106,31 @@ def test_rows_of_odd_block_counts_are_as_exact_as_f32(cuda, wt, outliers):
             worst = max(worst, ((y.double() - want).norm() / want.norm()).item())
     assert worst <= (1.7e-7 if wt == synth.Q5_1 else 1.4e-7)
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("wt", [synth.Q8_0, synth.Q4_0, synth.Q5_0, synth.Q5_1, synth.IQ4_NL])
+def test_rows_of_odd_block_counts_keep_infinities(cuda, wt):
+    """K not a multiple of 256: an infinite activation gives what f32 arithmetic gives, and only in its own row."""
+    import torch
+    n_out, n_in = 100, 2080
+    w = dev(synth.weights(wt, n_out, n_in, SEED + 5, stream=wt))
+    w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+    for rows in (1, 2, 4, 8, 11):
+        x = dev(synth.activations(rows, n_in, SEED + rows))
+        x[rows // 2, 777] = float("-inf")
+        if rows > 2:
+            x[0, 2079] = float("nan")
+        want = x.double() @ w64.T
+        got = cuda.gemv(x, w, wt, n_out, n_in) if rows <= 8 else cuda.gemm(x, w, wt, n_out, n_in)
+        assert torch.isinf(want[rows // 2]).any()
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+        assert torch.equal(torch.sign(got[torch.isinf(got)]).double(), torch.sign(want[torch.isinf(want)]))
+        fine = torch.isfinite(want)
+        assert (got[fine].double() - want[fine]).norm() <= 2e-7 * want[fine].norm()
+    # the gate/up fold: silu(gate) of an infinite gate
+    x = dev(synth.activations(1, n_in, SEED))[0]
+    x[777] = float("inf")
+    got = cuda.gemv_group([x, x], [w, w], [wt, wt], [n_out, n_out], n_in, fuse_silu_pair=True)[0]
+    gate = x.double() @ w64.T
+    want = gate / (1.0 + torch.exp(-gate)) * gate
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
