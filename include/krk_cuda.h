@@ -248,7 +248,7 @@ int krk_cuda_sum_parts(void *out_f32, const void *parts_f32, int n_parts, int64_
  *     raised) until every peer's epoch has arrived here, so the end of the kernel is the end of the
  *     all-gather on this GPU. With 0 the host enqueues krk_cuda_wait_flags where it wants the row.
  * Use two output buffers alternately so that a fast GPU's next step cannot overwrite a row a slow GPU
- * is still reading. Shapes the streaming kernel does not address return KRK_CUDA_ESHAPE. */
+ * is still reading. n_in is a multiple of 256; that and shapes the streaming kernel has no room for return KRK_CUDA_ESHAPE. */
 int krk_cuda_gemv_allgather(void *const host_y_peers[], void *const host_flag_peers[], int n_peers, int my_rank,
                             int epoch, int wait_in_kernel, int64_t slice_offset, int64_t n_out_total,
                             const void *x_f32, const void *w, int wt, int64_t n_out_local, int64_t n_in,

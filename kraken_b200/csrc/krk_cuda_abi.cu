@@ -354,7 +354,7 @@ int krk_cuda_gemv_allgather(void *const host_y_peers[], void *const host_flag_pe
     if (slice_offset < 0 || n_out_total < slice_offset + n_out_local) return KRK_CUDA_ESHAPE;
     const int rc = check_matmul_args(host_y_peers[my_rank], x_f32, w, wt, n_out_local, n_in, rows);
     if (rc != KRK_CUDA_OK) return rc;
-    if (rows < 1 || rows > KRK_CUDA_MAX_ROWS || n_out_local < 1) return KRK_CUDA_ESHAPE;
+    if (rows < 1 || rows > KRK_CUDA_MAX_ROWS || n_out_local < 1 || n_in % 256 != 0) return KRK_CUDA_ESHAPE;
     PeerScatter ps;
     for (int q = 0; q < n_peers; q++) {
         if (!host_y_peers[q] || !host_flag_peers[q]) return KRK_CUDA_ENULL;

@@ -66,6 +66,8 @@ def test_preflight_refusals_launch_nothing():
     assert L.krk_cuda_gemm(a, a, capi.X_F16, a, capi.Q8_0, 8, 96, 16, None, 0, None) == -2
     assert L.krk_cuda_gemv_group(None, None, None, None, None, 256, 17, 0, None) == -8
     assert L.krk_cuda_gemv_group(None, None, None, None, None, 256, 2, 0, None) == -3
+    peers = (C.c_void_p * 1)(0x1000)
+    assert L.krk_cuda_gemv_allgather(peers, peers, 1, 0, 1, 0, 0, 8, a, a, capi.Q8_0, 8, 288, 1, None) == -2   # whole blocks, but not of 256
     # empty problems are a no-op success (the reference walks zero outputs without complaint)
     assert L.krk_cuda_gemv(None, None, None, capi.Q4_K, 0, 256, 1, 0, None) == 0
     assert L.krk_cuda_dequant_rows(None, None, capi.Q8_0, 0, 256, None) == 0
