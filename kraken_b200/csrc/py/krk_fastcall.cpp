@@ -7,6 +7,7 @@
 #include <Python.h>
 
 #include <ATen/ops/empty.h>
+#include <ATen/ops/empty_like.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -248,7 +249,7 @@ PyObject *silu_mul(PyObject *, PyObject *const *a, Py_ssize_t n) {   // gate, up
     if (!g.ok) return nullptr;
     at::Tensor made;
     if (!out) {
-        made = empty_like_device(*gate, gate->sizes(), gate->scalar_type());
+        made = at::empty_like(*gate, gate->options().requires_grad(false));   // with its strides: the kernel goes through the memory as it lies
         out = &made;
     }
     const int rc = krk_cuda_silu_mul(Args::ptr(out), Args::ptr(gate), up, gate->numel(), st);
