@@ -158,6 +158,7 @@ def _raise(rc: int, where: str) -> None:
 
 
 _fc.set_raise(_raise)
+_fc.set_address(lambda p: C.cast(p, _vp).value or 0)
 
 
 def _stream_ptr(stream=None):

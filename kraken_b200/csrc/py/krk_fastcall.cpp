@@ -17,7 +17,8 @@
 
 namespace {
 
-PyObject *g_raise = nullptr;   // capi's (rc, where) -> raises
+PyObject *g_raise = nullptr;     // capi's (rc, where) -> raises
+PyObject *g_address = nullptr;   // capi's ctypes pointer -> int
 
 PyObject *fail(int rc, const char *where) {
     PyObject *r = PyObject_CallFunction(g_raise, "is", rc, where);
@@ -35,10 +36,26 @@ struct Args {
         if (v == -1 && PyErr_Occurred()) ok = false;
         return v;
     }
+    // An address: an integer, None, or whatever ctypes takes for a void pointer.
     uintptr_t addr(int k) {
-        const unsigned long long v = PyLong_AsUnsignedLongLong(a[k]);
-        if (v == ~0ull && PyErr_Occurred()) ok = false;
-        return (uintptr_t)v;
+        if (a[k] == Py_None) return 0;
+        PyObject *o = PyLong_Check(a[k]) ? nullptr : PyObject_CallOneArg(g_address, a[k]);
+        if (!o && !PyLong_Check(a[k])) {
+            ok = false;
+            return 0;
+        }
+        const uintptr_t v = (uintptr_t)PyLong_AsUnsignedLongLongMask(o ? o : a[k]);
+        Py_XDECREF(o);
+        if (PyErr_Occurred()) ok = false;
+        return v;
+    }
+    void *backend(int k) {
+        if (!PyLong_Check(a[k])) {
+            if (ok) PyErr_SetString(PyExc_TypeError, "the backend is closed");
+            ok = false;
+            return nullptr;
+        }
+        return (void *)addr(k);
     }
     float f(int k) {
         const double v = PyFloat_AsDouble(a[k]);
@@ -96,6 +113,11 @@ at::Tensor empty_like_device(const at::Tensor &like, at::IntArrayRef sizes, at::
 PyObject *set_raise(PyObject *, PyObject *f) {
     Py_INCREF(f);
     Py_XSETREF(g_raise, f);
+    Py_RETURN_NONE;
+}
+PyObject *set_address(PyObject *, PyObject *f) {
+    Py_INCREF(f);
+    Py_XSETREF(g_address, f);
     Py_RETURN_NONE;
 }
 
@@ -415,7 +437,7 @@ PyObject *moe_ffn_routed(PyObject *, PyObject *const *a, Py_ssize_t n) {   // x,
 PyObject *backend_upload(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be, dst, host_src, bytes, off
     KRK_NARGS(5, "backend_upload")
     Args g{a};
-    void *be = (void *)g.addr(0), *dst = (void *)g.addr(1);
+    void *be = g.backend(0), *dst = (void *)g.addr(1);
     const void *src = (const void *)g.addr(2);
     const size_t bytes = (size_t)g.i(3), off = (size_t)g.i(4);
     if (!g.ok) return nullptr;
@@ -425,7 +447,7 @@ PyObject *backend_upload(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be
 PyObject *backend_download(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be, host_dst, src, bytes, off
     KRK_NARGS(5, "backend_download")
     Args g{a};
-    void *be = (void *)g.addr(0), *dst = (void *)g.addr(1);
+    void *be = g.backend(0), *dst = (void *)g.addr(1);
     const void *src = (const void *)g.addr(2);
     const size_t bytes = (size_t)g.i(3), off = (size_t)g.i(4);
     if (!g.ok) return nullptr;
@@ -435,7 +457,7 @@ PyObject *backend_download(PyObject *, PyObject *const *a, Py_ssize_t n) {   // 
 PyObject *backend_gemm(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be, out, x, w, wt, n_out, n_in, rows
     KRK_NARGS(8, "backend_gemm")
     Args g{a};
-    void *be = (void *)g.addr(0), *out = (void *)g.addr(1);
+    void *be = g.backend(0), *out = (void *)g.addr(1);
     const void *x = (const void *)g.addr(2), *w = (const void *)g.addr(3);
     const int wt = (int)g.i(4);
     const int64_t n_out = g.i(5), n_in = g.i(6), rows = g.i(7);
@@ -446,7 +468,7 @@ PyObject *backend_gemm(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be, 
 PyObject *backend_gemm_accumulate(PyObject *, PyObject *const *a, Py_ssize_t n) {   // be, dst, x, w, wt, n_out, n_in, rows
     KRK_NARGS(8, "backend_gemm_accumulate")
     Args g{a};
-    void *be = (void *)g.addr(0), *dst = (void *)g.addr(1);
+    void *be = g.backend(0), *dst = (void *)g.addr(1);
     const void *x = (const void *)g.addr(2), *w = (const void *)g.addr(3);
     const int wt = (int)g.i(4);
     const int64_t n_out = g.i(5), n_in = g.i(6), rows = g.i(7);
@@ -485,7 +507,7 @@ PyObject *backend_gemm_group(PyObject *, PyObject *const *a, Py_ssize_t n) {
         if (a[9] != Py_None) wt[i] = (int)ft.i((int)i);
         if (a[10] != Py_None) x[i] = (const void *)fx.addr((int)i);
     }
-    void *be = (void *)g.addr(0);
+    void *be = g.backend(0);
     const void *x0 = (const void *)g.addr(2);
     const int wt0 = (int)g.i(4);
     const int64_t n_in = g.i(6), rows = g.i(7);
@@ -501,6 +523,7 @@ PyObject *backend_gemm_group(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 #define KRK_FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"set_raise", set_raise, METH_O, nullptr},
+                         {"set_address", set_address, METH_O, nullptr},
                          KRK_FAST(gemv),
                          KRK_FAST(gemv_group),
                          KRK_FAST(gemm),

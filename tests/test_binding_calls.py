@@ -1,4 +1,7 @@
 """The Python binding's calls: what they accept and refuse, and what they allocate."""
+import ctypes as C
+
+import numpy as np
 import pytest
 
 from kraken_b200 import capi
@@ -13,3 +16,34 @@ def test_silu_mul_keeps_the_layout_of_its_inputs(cuda):
         assert y.stride() == gate.stride() and not y.requires_grad
         want = torch.nn.functional.silu(gate.double()) * up.double()
         assert (y - want).abs().max().item() < 1e-5
+
+
+@pytest.mark.gpu
+def test_backend_takes_every_form_of_pointer(cuda):
+    """Integers, None where no pointer is needed, and what ctypes takes for a void pointer."""
+    import torch
+    be = cuda.Backend(0)
+    w = torch.zeros(64 * 34, dtype=torch.uint8, device="cuda")
+    w[0::34], w[1::34] = 0, 0x3C                      # Q8_0 blocks of scale 1.0
+    w.view(64, 34)[:, 2:] = 1
+    src = np.full(32, 2.0, np.float32)
+    x, y = torch.zeros(32, device="cuda"), torch.zeros((2, 64), device="cuda")
+    be.upload(C.c_void_p(x.data_ptr()), src.ctypes.data_as(C.POINTER(C.c_float)), src.nbytes)
+    outs, ws = [y[0].data_ptr(), y[1].data_ptr()], [C.c_void_p(w.data_ptr()), w.data_ptr()]
+    ran, fused = be.gemm_group(outs, None, ws, cuda.Q8_0, [64, 64], 32, xs=[x.data_ptr()] * 2)
+    assert ran and not fused
+    be.sync()
+    assert (y == 64.0).all()
+    be.upload(x.data_ptr(), src.tobytes(), src.nbytes)
+    be.gemm(C.c_void_p(y.data_ptr()), x.data_ptr(), w.data_ptr(), cuda.Q8_0, 64, 32, 1)
+    got = (C.c_float * 128)()
+    be.download(got, y.data_ptr(), 512)
+    assert list(got) == [64.0] * 128
+    be.close()
+    with pytest.raises(TypeError):
+        be.upload(x.data_ptr(), src.ctypes.data, src.nbytes)
+
+
+def test_addresses_are_checked_before_the_call():
+    with pytest.raises((TypeError, C.ArgumentError)):
+        capi._fc.backend_upload(1, 2.5, 0, 0, 0)
