@@ -274,7 +274,11 @@ PyObject *silu_mul(PyObject *, PyObject *const *a, Py_ssize_t n) {   // gate, up
         made = at::empty_like(*gate, gate->options().requires_grad(false));   // with its strides: the kernel goes through the memory as it lies
         out = &made;
     }
-    const int rc = krk_cuda_silu_mul(Args::ptr(out), Args::ptr(gate), up, gate->numel(), st);
+    void *y = Args::ptr(out), *gp = Args::ptr(gate);
+    const int64_t count = gate->numel();
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = krk_cuda_silu_mul(y, gp, up, count, st);
+    Py_END_ALLOW_THREADS
     if (rc != 0) return fail(rc, "silu_mul");
     if (made.defined()) return THPVariable_Wrap(made);
     Py_INCREF(a[2]);
@@ -296,7 +300,11 @@ PyObject *embed(PyObject *, PyObject *const *a, Py_ssize_t n) {   // table, wt, 
         made = empty_like_device(*table, {tokens->numel(), n_embd}, at::kFloat);
         out = &made;
     }
-    const int rc = krk_cuda_embed(Args::ptr(out), Args::ptr(table), wt, n_vocab, n_embd, Args::ptr(tokens), tokens->numel(), st);
+    void *y = Args::ptr(out), *tp = Args::ptr(table), *ip = Args::ptr(tokens);
+    const int64_t n_tok = tokens->numel();
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = krk_cuda_embed(y, tp, wt, n_vocab, n_embd, ip, n_tok, st);
+    Py_END_ALLOW_THREADS
     if (rc != 0) return fail(rc, "embed");
     if (made.defined()) return THPVariable_Wrap(made);
     Py_INCREF(a[5]);
@@ -323,8 +331,10 @@ PyObject *logits_topk(PyObject *, PyObject *const *a, Py_ssize_t n) {
     }
     at::Tensor ids = empty_like_device(*logits, {k}, at::kInt), vals = empty_like_device(*logits, {k}, at::kFloat);
     if (want_mass) mass = empty_like_device(*logits, {1}, at::kFloat);
-    const int rc = krk_cuda_logits_topk(Args::ptr(logits), logits->numel(), (int)k, Args::ptr(pen), rep_pen, softcap, temp, Args::ptr(&ids),
-                                        Args::ptr(&vals), want_mass ? Args::ptr(&mass) : nullptr, Args::ptr(ws), (size_t)ws->numel(), st);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS rc = krk_cuda_logits_topk(Args::ptr(logits), logits->numel(), (int)k, Args::ptr(pen), rep_pen, softcap, temp, Args::ptr(&ids),
+                                                     Args::ptr(&vals), want_mass ? Args::ptr(&mass) : nullptr, Args::ptr(ws), (size_t)ws->numel(), st);
+    Py_END_ALLOW_THREADS
     if (rc != 0) return fail(rc, "logits_topk");
     PyObject *r = PyTuple_New(3);
     if (!r) return nullptr;

@@ -1,5 +1,7 @@
 """The Python binding's calls: what they accept and refuse, and what they allocate."""
 import ctypes as C
+import os
+import re
 
 import numpy as np
 import pytest
@@ -47,3 +49,14 @@ def test_backend_takes_every_form_of_pointer(cuda):
 def test_addresses_are_checked_before_the_call():
     with pytest.raises((TypeError, C.ArgumentError)):
         capi._fc.backend_upload(1, 2.5, 0, 0, 0)
+
+
+def test_every_launching_call_releases_the_interpreter_lock():
+    """A launch can wait for room in the device's queue, and what empties it may be a host callback that needs the lock."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    text = open(os.path.join(root, "kraken_b200", "csrc", "py", "krk_fastcall.cpp")).read()
+    calls = [m for m in re.finditer(r"\bkrk_cuda_\w+\(", text) if "workspace_bytes" not in m.group()]
+    assert len(calls) >= 13
+    for m in calls:
+        line = text[text.rfind("\n", 0, m.start()) + 1:m.start()]
+        assert "Py_BEGIN_ALLOW_THREADS" in line, m.group()
