@@ -173,7 +173,7 @@ PyObject *gemv_group(PyObject *, PyObject *const *a, Py_ssize_t n) {   // xs, ws
     if (!xs.s || !ws.s || !wts.s || !nos.s) return nullptr;
     const Py_ssize_t m = ws.n;
     if (m > KRK_CUDA_MAX_GROUP) return fail(KRK_CUDA_EARG, "gemv_group");
-    if (xs.n < m || wts.n < m || nos.n < m) {
+    if (xs.n != m || wts.n != m || nos.n != m) {
         PyErr_SetString(PyExc_ValueError, "gemv_group: argument lists of unequal length");
         return nullptr;
     }
@@ -203,8 +203,8 @@ PyObject *gemv_group(PyObject *, PyObject *const *a, Py_ssize_t n) {   // xs, ws
     void *st = g.stream(7);
     if (g.ok) {
         Seq ys(outs);
-        if (!ys.s || ys.n < m) {
-            if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "gemv_group: too few outputs");
+        if (!ys.s || ys.n != m) {
+            if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "gemv_group: as many outputs as matrices are needed");
             g.ok = false;
         }
         for (Py_ssize_t i = 0; i < m && g.ok; i++) y[i] = Args::ptr(g.tensor(ys[i]));
@@ -500,7 +500,7 @@ PyObject *backend_gemm_group(PyObject *, PyObject *const *a, Py_ssize_t n) {
     Seq wts(a[9] == Py_None ? empty : a[9]), xs(a[10] == Py_None ? empty : a[10]);
     Py_DECREF(empty);
     if (!wts.s || !xs.s) return nullptr;
-    if ((size_t)outs.n < m || (size_t)nos.n < m || (a[9] != Py_None && (size_t)wts.n < m) || (a[10] != Py_None && (size_t)xs.n < m)) {
+    if ((size_t)outs.n != m || (size_t)nos.n != m || (a[9] != Py_None && (size_t)wts.n != m) || (a[10] != Py_None && (size_t)xs.n != m)) {
         PyErr_SetString(PyExc_ValueError, "gemm_group: argument lists of unequal length");
         return nullptr;
     }

@@ -60,3 +60,24 @@ def test_every_launching_call_releases_the_interpreter_lock():
     for m in calls:
         line = text[text.rfind("\n", 0, m.start()) + 1:m.start()]
         assert "Py_BEGIN_ALLOW_THREADS" in line, m.group()
+
+
+@pytest.mark.parametrize("longer", range(5))
+def test_group_lists_of_unequal_length_are_refused(longer):
+    import torch
+    t = torch.zeros(64)
+    lists = [[t, t], [t, t], [capi.Q8_0] * 2, [1, 1], [t, t]]   # xs, ws, wts, n_outs, outs
+    if longer != 1:
+        lists[longer] = lists[longer] + lists[longer][:1]
+    else:
+        lists = [l if i == 1 else l + l[:1] for i, l in enumerate(lists)]
+    xs, ws, wts, n_outs, outs = lists
+    with pytest.raises(ValueError):
+        capi._fc.gemv_group(xs, ws, wts, n_outs, 32, outs, False, NoStream)
+    addresses = lambda l: [0x1000] * len(l)   # noqa: E731
+    with pytest.raises(ValueError):
+        capi._fc.backend_gemm_group(0, addresses(outs), 0, addresses(ws), capi.Q8_0, n_outs, 32, 1, False, wts, addresses(xs))
+
+
+class NoStream:
+    cuda_stream = 0
