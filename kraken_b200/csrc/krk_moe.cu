@@ -740,8 +740,10 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
     p.n_tok = (int)n_tok;
     // From the rows an expert can expect: the token tile (an expert's rows should fit one, since every further tile
     // decodes its weights again; up to 64 tokens two accumulators alternate), and the rows per entry of the few-row experts.
+    // Over five banks of 8 to 128 experts, tiles of 128 take 1.03 of the time of tiles of 64 at 60 mean rows and 0.89 at 72;
+    // tiles of 256 take 1.12 of the time of tiles of 128 at 112, 1.01 at 128 and 0.96 at 160.
     const int64_t picks = n_tok * k, mean = picks / n_expert;
-    p.tile_m = mean <= 44 ? 64 : mean <= 100 ? 128 : 256;
+    p.tile_m = mean <= 60 ? 64 : mean <= 120 ? 128 : 256;
     p.cap_log2 = entry_rows_log2(picks, n_expert);
     p.cap = 1 << p.cap_log2;
     p.n_groups = many ? reinterpret_cast<int *>(ws + L.head) : nullptr;
