@@ -100,6 +100,7 @@ struct StreamParams {
     int n_entries;        // matrices, or gate/up pairs when silu_pair
     int step;             // matrices per entry (2 for gate/up pairs)
     int rows;             // activation rows
+    int groups;           // consumer groups of a CTA
     int accumulate;
     int n_in;
     int units;            // n_in / unit_values
@@ -274,7 +275,7 @@ __device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volati
 
 // ---- shared-memory map ---------------------------------------------------------------------------
 
-template <int NG>
+template <int NG, int GROUPS = consumer_groups(NG)>
 struct Smem {
     unsigned long long full[kMaxStages];     // weights of a stage have landed
     unsigned long long empty[kMaxStages];    // every consumer warp is done with the stage
@@ -284,7 +285,7 @@ struct Smem {
     int touched[11];   // where the parameter fetches of the first instructions end (never read)
     float gate[kMaxStack][NG][32];   // epilogue warp: the gate tile(s) of a gate/up pair, until the up tile arrives
     // per consumer warp, column group and row pair (g, g+8): {row g x even activation row, g x odd, g+8 x even, g+8 x odd}
-    float4 red[consumer_groups(NG) * red_slots(NG)][kConsumerWarps][NG][8];
+    float4 red[GROUPS * red_slots(NG)][kConsumerWarps][NG][8];
     float scale[NG == 1 ? 1 : kConsumerWarps][2 * NG];   // two groups: each prepared half of the activation rows, these are the scales
 };
 
@@ -1441,18 +1442,18 @@ __device__ __noinline__ float dot_f32(const uint8_t *w, const float *x, int n_in
     return sum;
 }
 
-template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false>
-__global__ void __launch_bounds__(cta_threads(consumer_groups(NG)), NG == 1 ? 2 : 1)
+template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG)>
+__global__ void __launch_bounds__(cta_threads(GROUPS), GROUPS == 1 ? 2 : 1)
 gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // STACK: several 16-row tiles per stage (p.tps of them); compiled apart so that the usual one-tile
     // form carries none of its index arithmetic.
     static_assert(!SINGLE || ((WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q4_0) && NG == 1), "the single-row forms are Q4_K and Q4_0");
     const int tps = STACK ? p.tps : 1;
-    constexpr int kGroups = consumer_groups(NG), kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
+    constexpr int kGroups = GROUPS, kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
     constexpr bool kFine = RAG && !kSuper;   // fine_limbs
     using F = Fmt<WT>;
-    using SmemT = Smem<NG>;
+    using SmemT = Smem<NG, GROUPS>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     SmemT *sm = reinterpret_cast<SmemT *>(smem_raw);
     int8_t *planes = reinterpret_cast<int8_t *>(smem_raw + align_up((int)sizeof(SmemT), 128));
@@ -1945,10 +1946,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     }
 }
 
-template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false>
+template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG)>
 int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     static bool configured[64] = {};   // per instantiation and device: the opt-in is sticky
-    auto kernel = gemv_stream_kernel<WT, NG, STACK, SINGLE, RAG>;
+    auto kernel = gemv_stream_kernel<WT, NG, STACK, SINGLE, RAG, GROUPS>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
@@ -1963,7 +1964,7 @@ int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(cta_threads(consumer_groups(NG)));
+    cfg.blockDim = dim3(cta_threads(GROUPS));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1984,7 +1985,7 @@ int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
 // Fills the fields that depend only on the format, the width and the activation row count.
 // Returns false when the streaming kernel does not address the shape.
 template <int WT>
-bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t *smem_out, bool want_tma = false) {
+bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t *smem_out, bool want_tma = false, bool one_group = false) {
     using F = Fmt<WT>;
     // K not a multiple of 256: whole 32-value blocks, rows copied the ragged way, the last unit short. (Below 256 values
     // there is little to stream, and the warp-per-row kernel serves.)
@@ -1994,6 +1995,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.units = (int)((n_in + F::unit_values - 1) / F::unit_values);
     p.row_bytes = (int)row_bytes(WT, n_in);
     p.rows = rows;
+    p.groups = rows <= 2 || one_group ? 1 : 2;
     p.accumulate = 0;
     p.step = silu_pair ? 2 : 1;
     p.whole_tiles = 0;
@@ -2054,11 +2056,11 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.row_stride = raw + ((F::stride_mod - raw % 128) + 128) % 128;
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
-    const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
+    const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
     const int fixed = align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows));
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
-    const bool halves = rows <= 2;
+    const bool halves = p.groups == 1;
     int max_fit = halves ? (kSmemLimit - fixed) / p.stage_bytes : 0;
     if (max_fit < 3) max_fit = (kSmemWhole - fixed) / p.stage_bytes;
     const int most = halves ? kMaxHalfStages : kMaxStages;
@@ -2098,6 +2100,8 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
         if (kQ4K && p.rows == 1 && !p.whole_tiles && p.units <= 2 * kConsumerWarps) return launch_one<WT, 1, false, kQ4K ? 2 : 0>(p, grid, smem, st);
         if (kQ4K && p.rows == 1) return launch_one<WT, 1, false, kQ4K ? 1 : 0>(p, grid, smem, st);
         if (p.rows <= 2) return launch_one<WT, 1, false, 0>(p, grid, smem, st);
+        if constexpr (WT == KRK_CUDA_Q8_0)
+            if (p.rows <= 4 && p.groups == 1) return launch_one<WT, 2, false, 0, false, 1>(p, grid, smem, st);
         if (p.rows <= 4) return launch_one<WT, 2, false, 0>(p, grid, smem, st);
         return launch_one<WT, 4, false, 0>(p, grid, smem, st);
     }
@@ -2110,13 +2114,13 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
 // matrices of a decode step the slower streaming of eight warps costs more than the overlap saves.
 // The forms of two consumer groups get one whatever their shared memory.
 template <int WT>
-int ctas_per_sm(size_t smem, int rows) {
+int ctas_per_sm(size_t smem, int groups) {
     static const int want = [] {
         const char *e = std::getenv("KRK_CUDA_GEMV_CTAS_PER_SM");
         const int v = e ? std::atoi(e) : 0;
         return v == 1 ? 1 : 2;
     }();
-    return rows <= 2 && smem <= (size_t)kSmemLimit ? want : 1;
+    return groups == 1 && smem <= (size_t)kSmemLimit ? want : 1;
 }
 
 // Tensor maps are encoded on the host (a driver call of a microsecond or two) and kept per (matrix, box):
@@ -2214,6 +2218,18 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
             if (!encode_maps<WT>(p, n_mat)) tma = false;   // a map cannot be encoded: set up again for row copies
         }
     }
+    if constexpr (WT == KRK_CUDA_Q8_0) {
+        // Three and four rows of Q8_0: a tile is four stages of 128-value units where the other formats have two, so two
+        // groups hold the whole ring and the next tiles are not under way while these are multiplied. Where there are
+        // tiles for two one-group CTAs per SM, and a half has room for them, those stream (one group against two, four rows:
+        // 49152 x 4096 52.8 against 76.0 us, 11008 x 4096 18.2 against 20.6; 4096 x 4096 10.7 against 10.2, and 512 x 1024 5.8
+        // against 4.5).
+        int64_t tiles = 0;
+        for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
+        if ((rows == 3 || rows == 4) && n_in % 256 == 0 && tiles > 2 * sm_count() && setup_format<WT>(p, n_in, rows, silu_pair, smem, false, true) &&
+            p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit)
+            return true;
+    }
     return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem);
 }
 
@@ -2241,7 +2257,7 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     // A launch whose tiles fit one to an SM takes one CTA per SM: a second would only cut tiles in two (both halves still
     // cost a whole tile of MMAs), and the other half of the SM lets the next launch start early (Q8_0 2048x2048 3.92 ->
     // 3.42 us, Q6_K 2048x6656 10.5 -> 8.1 us).
-    const int per_sm = tiles <= sm_count() ? 1 : ctas_per_sm<WT>(smem, p.rows);
+    const int per_sm = tiles <= sm_count() ? 1 : ctas_per_sm<WT>(smem, p.groups);
     const int sms = sm_count() * per_sm;
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
@@ -2275,7 +2291,7 @@ int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_
     p.entry_gran = (int)((n_out + p.gran - 1) / p.gran);
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
-    const int rc = launch_rows<WT>(p, sm_count() * ctas_per_sm<WT>(smem, p.rows), smem, st);
+    const int rc = launch_rows<WT>(p, sm_count() * ctas_per_sm<WT>(smem, p.groups), smem, st);
     return rc == KRK_CUDA_OK ? 1 : rc;
 }
 
@@ -2303,7 +2319,7 @@ int launch_peers_fmt(const GemvMat &mat, int64_t n_in, int rows, const PeerScatt
     p.wait_peers = ps.wait_peers;
     p.peer_row_stride = ps.row_stride;
     p.peer_offset = ps.offset;
-    const int sms = sm_count() * ctas_per_sm<WT>(smem, p.rows);
+    const int sms = sm_count() * ctas_per_sm<WT>(smem, p.groups);
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
     p.gran_r = total % grid;

@@ -134,3 +134,19 @@ def test_rows_of_odd_block_counts_keep_infinities(cuda, wt):
     gate = x.double() @ w64.T
     want = gate / (1.0 + torch.exp(-gate)) * gate
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+
+
+@pytest.mark.parametrize("n_out", [4736, 4737, 5003])
+def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
+    """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
+    import torch
+    for n_in in (1024, 4096):
+        w = dev(synth.weights(synth.Q8_0, n_out, n_in, SEED + 6, stream=1))
+        w64 = cuda.dequant_rows(w, synth.Q8_0, n_out, n_in).double()
+        for rows in (2, 3, 4, 5):
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            base = torch.randn((rows, n_out), device="cuda")
+            y = cuda.gemv(x, w, synth.Q8_0, n_out, n_in, out=base.clone(), accumulate=True)
+            lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
+            assert ((y.double() - base.double() - x.double() @ w64.T).abs() <= lim).all()
+    assert cuda.device_status() == 0
