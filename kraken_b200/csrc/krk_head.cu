@@ -70,14 +70,18 @@ constexpr int kNone = 0x7FFFFFFF;
 
 // By a whole block: the k-th largest of the keys that `each(f)` hands to f (each thread its own; zeros are ignored), and
 // how many of its equals belong to the k largest. Fewer than k keys: threshold 0, nothing taken from its equals.
-// ONE (k = 1): the greatest, one pass and one barrier in place of four passes of three; compiled apart, since the
-// other form loses 1.2 us beside the extra code (42,146 logits and their head: 34.2 -> 29.2 us at k = 1).
-template <bool ONE, class Each>
+// k = 1 (kGreatest): one pass and one barrier in place of four passes of three; compiled apart, since the other form
+// loses 1.2 us beside the extra code (42,146 logits and their head: 34.2 -> 29.2 us at k = 1). A few (kFew): the distinct
+// keys from the greatest down, each with its number, a pass and a barrier each (32,000 logits, few against radix: k = 2 7.3
+// against 11.4 us, k = 6 10.4 against 11.7, k = 8 12.0 against 11.7).
+enum SelectMode { kRadix, kGreatest, kFew };
+constexpr int kFewK = 7;
+template <SelectMode MODE, class Each>
 __device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &threshold, int &of_equals) {
     __shared__ int hist[256];
     __shared__ uint32_t s_prefix;
     __shared__ int s_left;
-    if constexpr (ONE) {
+    if constexpr (MODE == kGreatest) {
         uint32_t most = 0u;
         each([&](uint32_t u) { most = max(most, u); });
         most = __reduce_max_sync(0xFFFFFFFFu, most);
@@ -87,6 +91,35 @@ __device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &thres
         threshold = __reduce_max_sync(0xFFFFFFFFu, lane < (int)blockDim.x / 32 ? (uint32_t)hist[lane] : 0u);
         of_equals = threshold != 0u ? 1 : 0;
         return;
+    }
+    if constexpr (MODE == kFew) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x / 32;
+        uint32_t below = 0xFFFFFFFFu;   // (no key has this value: it would be a NaN's)
+        int want = k;
+        for (int pass = 0;; pass ^= 1) {
+            uint32_t most = 0u;
+            each([&](uint32_t u) { most = max(most, u < below ? u : 0u); });
+            most = __reduce_max_sync(0xFFFFFFFFu, most);
+            int same = 0;
+            each([&](uint32_t u) { same += u == most; });
+            same = __reduce_add_sync(0xFFFFFFFFu, same);
+            // (two halves in turn: a warp may be a pass ahead of the last reader, never two)
+            if (lane == 0) {
+                hist[128 * pass + 2 * warp] = (int)most;
+                hist[128 * pass + 2 * warp + 1] = same;
+            }
+            __syncthreads();
+            const uint32_t m = lane < n_warps ? (uint32_t)hist[128 * pass + 2 * lane] : 0u;
+            const int c = lane < n_warps ? hist[128 * pass + 2 * lane + 1] : 0;
+            below = __reduce_max_sync(0xFFFFFFFFu, m);
+            const int n = __reduce_add_sync(0xFFFFFFFFu, m == below ? c : 0);
+            if (below == 0u || n >= want) {   // fewer than k keys, or the k-th is among these
+                threshold = below;
+                of_equals = below == 0u ? 0 : want;
+                return;
+            }
+            want -= n;
+        }
     }
     uint32_t prefix = 0u, mask = 0u;
     int left = k;
@@ -147,7 +180,7 @@ struct Selected {
 };
 
 // cand_u / cand_i: [blocks][k] in no order; part: [blocks][2] = (slice max, slice sum of exp((key - slice max) * inv_temp))
-template <bool ONE>
+template <SelectMode MODE>
 __global__ void __launch_bounds__(kTopkThreads)
 topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ cand_u, int *__restrict__ cand_i,
                    float *__restrict__ part) {
@@ -177,7 +210,7 @@ topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ 
     if (lane == 0) red[warp] = mx;
     uint32_t threshold;
     int of_equals;
-    radix_select<ONE>([&](auto &&f) {
+    radix_select<MODE>([&](auto &&f) {
 #pragma unroll
         for (int j = 0; j < kTopkPer; j++) f(u[j]);
     }, p.k, threshold, of_equals);   // (its barriers publish red[])
@@ -230,7 +263,7 @@ topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ 
     }
 }
 
-template <bool ONE>
+template <SelectMode MODE>
 __global__ void __launch_bounds__(kMergeThreads)
 topk_merge_kernel(const __grid_constant__ TopkParams p, const uint32_t *__restrict__ cand_u, const int *__restrict__ cand_i,
                   const float *__restrict__ part, int n_blocks, int32_t *__restrict__ ids, float *__restrict__ vals,
@@ -263,7 +296,7 @@ topk_merge_kernel(const __grid_constant__ TopkParams p, const uint32_t *__restri
     };
     uint32_t threshold;
     int of_equals;
-    radix_select<ONE>([&](auto &&f) { each_at([&](uint32_t u, int64_t) { f(u); }); }, k, threshold, of_equals);
+    radix_select<MODE>([&](auto &&f) { each_at([&](uint32_t u, int64_t) { f(u); }); }, k, threshold, of_equals);
     each_at([&](uint32_t u, int64_t i) {
         if (u > threshold) {
             const int at = atomicAdd(&sel.n, 1);
@@ -339,6 +372,7 @@ int launch_logits_topk(const float *logits, int64_t n, int k, const uint32_t *pe
     if (k < 1 || k > kTopkMaxK || n < 1) return KRK_CUDA_EARG;
     if (n > INT32_MAX) return KRK_CUDA_ESHAPE;   // ids are 32-bit
     const int blocks = topk_blocks(n);
+    const SelectMode mode = k == 1 ? kGreatest : k <= kFewK ? kFew : kRadix;
     uint32_t *cand_u = static_cast<uint32_t *>(workspace);
     int *cand_i = reinterpret_cast<int *>(cand_u + (size_t)blocks * k);
     float *part = reinterpret_cast<float *>(cand_i + (size_t)blocks * k);
@@ -350,9 +384,9 @@ int launch_logits_topk(const float *logits, int64_t n, int k, const uint32_t *pe
     p.inv_temp = temp > 0.0f ? 1.0f / temp : 1.0f;
     p.n = n;
     p.k = k;
-    int rc = launched(launch_overlapped(k == 1 ? topk_slices_kernel<true> : topk_slices_kernel<false>, dim3((unsigned)blocks), dim3(kTopkThreads), st, p, cand_u, cand_i, part));
+    int rc = launched(launch_overlapped(mode == kGreatest ? topk_slices_kernel<kGreatest> : mode == kFew ? topk_slices_kernel<kFew> : topk_slices_kernel<kRadix>, dim3((unsigned)blocks), dim3(kTopkThreads), st, p, cand_u, cand_i, part));
     if (rc != KRK_CUDA_OK) return rc;
-    return launched(launch_overlapped(k == 1 ? topk_merge_kernel<true> : topk_merge_kernel<false>, dim3(1), dim3(kMergeThreads), st, p, cand_u, cand_i, part, blocks, ids, vals, mass_out));
+    return launched(launch_overlapped(mode == kGreatest ? topk_merge_kernel<kGreatest> : mode == kFew ? topk_merge_kernel<kFew> : topk_merge_kernel<kRadix>, dim3(1), dim3(kMergeThreads), st, p, cand_u, cand_i, part, blocks, ids, vals, mass_out));
 }
 
 } // namespace krk_cuda

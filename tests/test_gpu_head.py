@@ -148,3 +148,27 @@ def test_topk_of_one(cuda, oracle, n):
     lg[:] = -np.inf
     lg[-1] = -1e30
     check_topk(cuda, oracle, lg, 1)
+
+
+@pytest.mark.parametrize("n", [3, 2048, 2049, 70001])
+def test_topk_of_a_few(cuda, n):
+    """k around the change from one greatest key after the other to the radix select: ties beyond k, infinities and NaN keys."""
+    for case in range(4):
+        lg = synth.normal(n, SEED + 90 + case, 3)
+        if case == 1:
+            lg = np.round(lg)                                  # few distinct values: ties across slices
+        elif case == 2:
+            lg[:] = 1.0
+            lg[n // 2] = np.nan
+        elif case == 3:
+            lg[::2] = -np.inf
+            lg[1::3] = np.nan
+        key = np.where(np.isnan(lg), np.float32(-np.inf), lg)
+        order = np.lexsort((np.arange(n), -key))
+        for k in (1, 2, 3, 6, 7, 8, 9):
+            ids, vals, _ = cuda.logits_topk(dev(lg), k)
+            m = min(k, n)
+            assert ids.cpu().numpy()[:m].tolist() == order[:m].tolist(), (case, k)
+            assert np.array_equal(vals.cpu().numpy()[:m], key[order[:m]])
+            assert (ids.cpu().numpy()[m:] == -1).all()
+    assert cuda.device_status() == 0
