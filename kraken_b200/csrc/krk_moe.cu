@@ -710,10 +710,18 @@ static MoeParams moe_params(float *y, const float *x, const int32_t *ids, const 
     return p;
 }
 
+// Few weight bytes over all picks: reading an expert again costs less than the longer preparation of four and eight rows (two
+// against four, 18 MB 27.2 against 32.3 us, 28 MB 23.8 against 30.6), or than the longer plan (an entry per pick).
+constexpr double kFewBytes = 64e6, kByPickBytes = 25e6;
 // Rows per entry of the few-row experts, from the rows an expert can expect: two cost what one does, four and eight 1.5
 // and 2.2 times.
 static int entry_rows_log2(int64_t picks, int n_expert) {
     return 5 * picks < 2 * n_expert ? 0 : picks < 2 * n_expert ? 1 : picks < 5 * n_expert ? 2 : 3;
+}
+
+// Weight bytes of all picks' experts.
+static double pick_bytes(const krk_cuda_expert_bank *bank, int64_t picks) {
+    return (double)picks * (2.0 * bank->n_ff * row_bytes(bank->wt_gate_up, bank->n_embd) + (double)bank->n_embd * row_bytes(bank->wt_down, bank->n_ff));
 }
 
 static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const float *x, const int32_t *ids, const float *wts,
@@ -745,6 +753,7 @@ static int moe_ffn_chunk(const GroupedLayout &L, uint8_t *ws, float *y, const fl
     const int64_t picks = n_tok * k, mean = picks / n_expert;
     p.tile_m = mean <= 60 ? 64 : mean <= 120 ? 128 : 256;
     p.cap_log2 = entry_rows_log2(picks, n_expert);
+    if (!many && p.cap_log2 > 1 && pick_bytes(bank, picks) < kFewBytes) p.cap_log2 = 1;
     p.cap = 1 << p.cap_log2;
     p.n_groups = many ? reinterpret_cast<int *>(ws + L.head) : nullptr;
     p.groups = reinterpret_cast<GemmGroup *>(ws + L.groups);
@@ -889,6 +898,9 @@ static int launch_moe_ffn_loop(float *y, const float *x, const int32_t *ids, con
     return KRK_CUDA_OK;
 }
 
+// Widths that are not whole super-blocks and few weight bytes: the warp-per-row kernels (4 MB 13.1 us against 18.7 streaming,
+// 8 MB 22.6 against 25.7, 11.6 MB 29.5 against 34.6; 14.6 MB 33.5 against 25.6).
+constexpr double kOddBytes = 12e6;
 int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const float *wts,
                            const krk_cuda_expert_bank *bank, int k, int64_t n_tok, void *workspace,
                            cudaStream_t st, const float *logits, int n_expert) {
@@ -896,8 +908,9 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
     // kernel; every other path runs the routing kernel on its own.
     // (few picks, or so thinly spread that entries would hold one row each: an entry per pick, and the shorter plan)
     const int last = bank->expert_base + bank->n_local;
-    const bool by_pick = n_tok <= KRK_CUDA_MAX_ROWS && (n_tok * k <= 8 || entry_rows_log2(n_tok * k, n_expert > last ? n_expert : last) == 0);
-    if (!by_pick && grouped_takes(bank, n_tok)) return launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, logits, n_expert, workspace, st);
+    const bool by_pick = n_tok <= KRK_CUDA_MAX_ROWS && (n_tok * k <= 8 || entry_rows_log2(n_tok * k, n_expert > last ? n_expert : last) == 0 || pick_bytes(bank, n_tok * k) < kByPickBytes);
+    const bool small_odd = n_tok <= KRK_CUDA_MAX_ROWS && (bank->n_embd % 256 != 0 || bank->n_ff % 256 != 0) && pick_bytes(bank, n_tok * k) < kOddBytes;
+    if (!by_pick && !small_odd && grouped_takes(bank, n_tok)) return launch_moe_ffn_grouped(y, x, ids, wts, bank, k, n_tok, logits, n_expert, workspace, st);
     bool routed = logits == nullptr;
     if (n_tok > KRK_CUDA_MAX_ROWS) {
         if (!routed) {
@@ -916,7 +929,7 @@ int launch_moe_ffn_generic(float *y, const float *x, const int32_t *ids, const f
     gu_banks.base[0] = p.gate;
     gu_banks.base[1] = p.up;
     gu_banks.rows = (int64_t)bank->n_local * bank->n_ff;
-    if (picks <= kPlanThreads && stream_takes(bank->wt_gate_up, bank->n_embd, 1) && stream_takes(bank->wt_down, bank->n_ff, 1)) {
+    if (!small_odd && picks <= kPlanThreads && stream_takes(bank->wt_gate_up, bank->n_embd, 1) && stream_takes(bank->wt_down, bank->n_ff, 1)) {
         const bool fuse_route = !routed && n_expert <= kPlanRouteExperts && n_tok * 32 <= kPlanThreads;
         if (!routed && !fuse_route) {
             const int rc = launch_route(const_cast<int32_t *>(ids), const_cast<float *>(wts), logits, n_tok, n_expert, k, st);

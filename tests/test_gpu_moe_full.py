@@ -218,3 +218,28 @@ def test_calls_of_more_tokens_than_a_chunk(cuda, k, n_tok):
         want += w * ((torch.nn.functional.silu(xd @ g[e].T) * (xd @ u[e].T)) @ d[e].T)
     rel = ((y.double() - want).norm(dim=1) / want.norm(dim=1).clamp_min(1e-30))
     assert rel.max().item() < 1e-2 and ((y.double() - want).norm() / want.norm()).item() < 2e-3, rel.topk(5)
+
+
+@pytest.mark.parametrize("n_exp, k, n_embd, n_ff, wt_gu, wt_dn", [(8, 2, 1024, 512, synth.Q5_K, synth.Q6_K), (8, 4, 1056, 544, synth.Q8_0, synth.Q8_0),
+                                                                  (8, 2, 2048, 1024, synth.Q4_K, synth.Q4_K)])
+def test_small_banks_on_every_path(cuda, n_exp, k, n_embd, n_ff, wt_gu, wt_dn):
+    """Decode batches of banks with few weight bytes: an entry per pick, two rows per entry, four, and (widths that are not
+    whole super-blocks) the warp-per-row kernels; the lines between lie at 12, 25 and 64 MB over all picks."""
+    import torch
+    gate, up = (dev(synth.weights(wt_gu, n_exp * n_ff, n_embd, SEED + 70, stream=i)) for i in range(2))
+    down = dev(synth.weights(wt_dn, n_exp * n_embd, n_ff, SEED + 70, stream=2))
+    bank = cuda.make_bank(gate, up, down, wt_gu, wt_dn, n_exp, 0, n_embd, n_ff)
+    g, u = (cuda.dequant_rows(w, wt_gu, n_exp * n_ff, n_embd).double().view(n_exp, n_ff, n_embd) for w in (gate, up))
+    d = cuda.dequant_rows(down, wt_dn, n_exp * n_embd, n_ff).double().view(n_exp, n_embd, n_ff)
+    gen = torch.Generator("cuda").manual_seed(3)
+    for n_tok in (1, 2, 3, 4, 6, 8):
+        x, logits = (torch.randn((n_tok, n), device="cuda", generator=gen) for n in (n_embd, n_exp))
+        y, ids, wts = cuda.moe_ffn_routed(x * 0.05, logits, k, bank)
+        want = torch.zeros((n_tok, n_embd), device="cuda", dtype=torch.double)
+        xd = (x * 0.05).double()
+        for t in range(n_tok):
+            for s in range(k):
+                e = ids[t, s].item()
+                want[t] += wts[t, s].double() * (d[e] @ (torch.nn.functional.silu(g[e] @ xd[t]) * (u[e] @ xd[t])))
+        assert ((y.double() - want).norm() / want.norm()).item() < 2e-5, n_tok
+    assert cuda.device_status() == 0
