@@ -39,11 +39,23 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
     const int wt = mats[0].wt;
     for (int m = 1; m < n_mat; m++)
         if (mats[m].wt != wt) return 0;
+    int64_t out = 0;
+    for (int m = 0; m < n_mat; m++) out += mats[m].n_out;
+    // K not a multiple of 256. Short rows leave little to stream beside the preparation of the activation, and matrices that
+    // fill few SMs with rows little to gain: the warp-per-row kernel (one row, 1024 weight rows, streaming against it: K = 288
+    // Q8_0 4.0 against 2.6 us, Q5_0 5.7 against 2.5; K = 544 3.3 against 2.8 and 5.1 against 2.7; K = 1056 3.9 against 4.2 and
+    // 4.1 against 3.8, Q5_1 at three rows 7.6 against 5.9; K = 2080 4.9 against 5.7 and 4.8 against 5.2). Below 512
+    // weight rows either is a matter of a few microseconds.
+    const bool odd_k = n_in % 256 != 0, few_rows = out < 8 * sm_count();
+    if (odd_k && out >= 512 && (n_in < 1024 || (wt == KRK_CUDA_Q5_1 && n_in < 2048 && few_rows))) return 0;
     int rc = 0;
     KRK_DISPATCH_WT(wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, st));
-    // Rows whose four limbs (K not a multiple of 256) leave no room for a ring go in two launches: the weights twice through
-    // the ring are far quicker than the warp-per-row kernel once (8 rows of Q8_0 have room up to K of some 5600).
-    if (rc == 0 && rows > 1 && n_in % 256 != 0 && n_mat <= KRK_CUDA_MAX_GROUP) {
+    // Activation rows whose four limbs leave no room for a ring go in two launches: the weights twice through the ring are
+    // quicker than the warp-per-row kernel once (8 rows of K = 11232, 2048 weight rows: Q8_0 50 against 81 us, Q5_1 70 against
+    // 75), but for matrices that do not fill the SMs with rows in the formats with the longer units (512 weight rows: Q4_0
+    // 57 against 52, Q5_1 70 against 53; Q8_0 48 against 55; six rows of Q4_0 37 against 42).
+    const bool halve = !few_rows || wt == KRK_CUDA_Q8_0 || wt == KRK_CUDA_IQ4_NL || (wt != KRK_CUDA_Q5_1 && rows <= 6);
+    if (rc == 0 && rows > 1 && odd_k && halve && n_mat <= KRK_CUDA_MAX_GROUP) {
         GemvMat part[KRK_CUDA_MAX_GROUP];
         for (int m = 0; m < n_mat; m++) part[m] = mats[m];
         const int first = (rows + 1) / 2;

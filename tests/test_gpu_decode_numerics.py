@@ -150,3 +150,21 @@ def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
             lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
             assert ((y.double() - base.double() - x.double() @ w64.T).abs() <= lim).all()
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("wt", [synth.Q8_0, synth.Q4_0, synth.Q5_1])
+def test_rows_of_odd_block_counts_on_either_kernel(cuda, wt):
+    """The lines between the streaming and the warp-per-row kernel, K not a multiple of 256: K = 1024 from 512 weight rows on
+    (Q5_1: 2048 below eight rows per SM), and wide activations of many rows, in two launches or not."""
+    for n_out, n_in, row_counts in ((511, 992, (1, 3, 8)), (512, 992, (1, 3, 8)), (512, 1056, (1, 8)), (1183, 2016, (2, 5)), (1184, 2016, (2, 5)),
+                                    (100, 11232, (5, 6, 7, 8)), (1200, 11232, (5, 8))):
+        w = dev(synth.weights(wt, n_out, n_in, SEED + 7, stream=wt))
+        w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+        for rows in row_counts:
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            want = x.double() @ w64.T
+            for _ in range(2):
+                y = cuda.gemv(x, w, wt, n_out, n_in)
+                # (the bound of the f32 kernel's distance above, for its longer rows too)
+                assert ((y.double() - want).norm() / want.norm()).item() <= 3e-7, (n_out, n_in, rows)
+    assert cuda.device_status() == 0
