@@ -35,7 +35,7 @@ extern "C" {
 #define KRK_CUDA_Q4_K 12
 #define KRK_CUDA_Q6_K 14
 /* further GGUF formats a Q4_K_M / Q5_K_M file mixes in: decoded bit-exactly and served by the prefill GEMM and,
- * for decode, by the streaming GEMV (the shape-agnostic GEMV when K is not a multiple of 256) */
+ * for decode, by the streaming GEMV (the warp-per-row GEMV for short rows when K is not a multiple of 256) */
 #define KRK_CUDA_Q5_0 6
 #define KRK_CUDA_Q5_1 7
 #define KRK_CUDA_Q5_K 13
@@ -196,7 +196,10 @@ struct krk_cuda_expert_bank {
  * (src/engine.cpp:12353-12690; device twin src/hip/kernels/moe_table.hpp:463-534), planned on the device: experts of
  * few rows as streaming entries, experts of more rows as groups of one tensor-core launch per product, then the
  * weighted sum in ascending expert id.
- * workspace: krk_cuda_moe_workspace_bytes() bytes of device memory, 256-byte aligned. */
+ * workspace: krk_cuda_moe_workspace_bytes() bytes of device memory, 256-byte aligned. Above eight tokens it holds f16
+ * copies of x and of the hidden rows and f32 output rows for every pick, of at most 65,536 picks at a time: for 128 experts
+ * of 4096 x 1536 and top-8 12 MB at 8 tokens, 136 MB at 512, 476 MB at 2048 and 1.84 GB from 8192 tokens on, however
+ * many. A host with less room calls with fewer tokens at a time. */
 size_t krk_cuda_moe_workspace_bytes(const struct krk_cuda_expert_bank *bank, int k, int64_t n_tok);
 int krk_cuda_moe_ffn(void *y_f32, const void *x_f32, const void *ids_i32, const void *wts_f32,
                      const struct krk_cuda_expert_bank *bank, int k, int64_t n_tok,
