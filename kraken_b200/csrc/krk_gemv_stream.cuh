@@ -1,5 +1,6 @@
 // Streaming decode GEMV for sm_100a: weights in any of the ten block formats (Q4_K, Q6_K, Q8_0, Q4_0, Q5_K, Q5_0,
-// Q5_1, IQ4_NL, Q2_K, Q3_K), K a multiple of 256, 1..8 activation rows, up to 16 matrices per launch.
+// Q5_1, IQ4_NL, Q2_K, Q3_K), K a multiple of 256 (of 32 for the formats of 32-value blocks), 1..8 activation rows, up to 16
+// matrices per launch.
 //
 // Design (B200-first, not the reference's one-warp-per-row walk of src/hip/kernels/gemm.hpp:76):
 //
@@ -20,7 +21,8 @@
 //    tensor cores as EXACT integer arithmetic: the quants are fed as s8 fragments straight from
 //    the packed bytes (one AND per four nibbles) to mma.sync m16n8k32 / m16n8k16 (s8 x s8 -> s32),
 //    16 output rows at a time, and the activation is held as three signed 8-bit limbs of a
-//    23-bit fixed-point number (x ~ s * (l0*65536 + l1*256 + l2), |X| < 2^22), one limb per MMA column.
+//    23-bit fixed-point number (x ~ s * (l0*65536 + l1*256 + l2), |X| < 2^22), one limb per MMA column
+//    (four limbs where K is not a multiple of 256, see fine_limbs).
 //    The products and sums are exact; the only rounding is the 23-bit quantisation of x
 //    (relative to max|x|, i.e. f32-mantissa sized) and the final f32 scale arithmetic, so the
 //    result sits well inside the 1e-4 * ||w_row|| * ||x|| bound. Sub-block scales are applied
@@ -2222,7 +2224,7 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
         // Three and four rows of Q8_0: a tile is four stages of 128-value units where the other formats have two, so two
         // groups hold the whole ring and the next tiles are not under way while these are multiplied. Where there are
         // tiles for two one-group CTAs per SM, and a half has room for them, those stream (one group against two, four rows:
-        // 49152 x 4096 52.8 against 76.0 us, 11008 x 4096 18.2 against 20.6; 4096 x 4096 10.7 against 10.2, and 512 x 1024 5.8
+        // 49152 x 4096 55.5 against 76.0 us, 11008 x 4096 18.8 against 20.6; 4096 x 4096 10.7 against 10.2, and 512 x 1024 5.8
         // against 4.5).
         int64_t tiles = 0;
         for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
