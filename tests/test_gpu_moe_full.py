@@ -221,10 +221,12 @@ def test_calls_of_more_tokens_than_a_chunk(cuda, k, n_tok):
 
 
 @pytest.mark.parametrize("n_exp, k, n_embd, n_ff, wt_gu, wt_dn", [(8, 2, 1024, 512, synth.Q5_K, synth.Q6_K), (8, 4, 1056, 544, synth.Q8_0, synth.Q8_0),
-                                                                  (8, 2, 2048, 1024, synth.Q4_K, synth.Q4_K)])
+                                                                  (8, 2, 2048, 1024, synth.Q4_K, synth.Q4_K), (4, 4, 2048, 1536, synth.Q8_0, synth.Q5_0),
+                                                                  (4, 4, 1536, 2048, synth.Q4_K, synth.Q6_K)])
 def test_small_banks_on_every_path(cuda, n_exp, k, n_embd, n_ff, wt_gu, wt_dn):
-    """Decode batches of banks with few weight bytes: an entry per pick, two rows per entry, four, and (widths that are not
-    whole super-blocks) the warp-per-row kernels; the lines between lie at 12, 25 and 64 MB over all picks."""
+    """Decode batches of banks with few weight bytes: an entry per pick, two rows per entry, and (widths that are not whole
+    super-blocks) the warp-per-row kernels; the lines between lie at 12, 25 and 64 MB over all picks. The last two banks
+    lie beyond them: four and eight rows per entry."""
     import torch
     gate, up = (dev(synth.weights(wt_gu, n_exp * n_ff, n_embd, SEED + 70, stream=i)) for i in range(2))
     down = dev(synth.weights(wt_dn, n_exp * n_embd, n_ff, SEED + 70, stream=2))
