@@ -97,39 +97,40 @@ template <> struct Fmt<KRK_CUDA_Q3_K> { static constexpr int unit_values = 256, 
 template <> struct Fmt<KRK_CUDA_IQ4_NL> { static constexpr int unit_values = 256, unit_bytes = 144, stride_mod = 16, tma = 1; };
 template <> struct Fmt<KRK_CUDA_Q5_1> { static constexpr int unit_values = 256, unit_bytes = 192, stride_mod = 16, tma = 0; };
 
-// What every warp reads before its first load stands first: parameters arrive cold in every launch, a cache line at a time.
+// Parameters arrive cold in every launch, a 64-byte line at a time (some 700 clocks each): what every warp reads before its
+// first load stands in the first line, what a launch of one matrix needs besides in the second.
 struct StreamParams {
     int n_entries;        // matrices, or gate/up pairs when silu_pair
     int step;             // matrices per entry (2 for gate/up pairs)
     int rows;             // activation rows
-    int groups;           // consumer groups of a CTA
-    int accumulate;
-    int n_in;
     int units;            // n_in / unit_values
-    int row_bytes;
+    int n_in;
+    int total_gran;
+    int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
+    const StreamTable *dev_table;   // when set, the matrices come from device memory
+    const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
     int gran;             // rows per granule: 1, or 8 when rows are not 16-byte multiples
-    int whole_tiles;      // 1: a stage is one contiguous copy of whole rows (unaligned row size)
-    int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
-                          // copied from the 16-byte boundary below its first byte, and its bytes sit that far
-                          // (0..15 bytes, a multiple of 2) into the row's slot
     int tps;              // 16-row tiles stacked in one stage (> 1 when a row has so few K units that one
                           // tile would leave most consumer warps idle: warp w takes unit w % units of
                           // sub-tile w / units)
+    int whole_tiles;      // 1: a stage is one contiguous copy of whole rows (unaligned row size)
+    int n_stages;
+    GemvMat mat[KRK_CUDA_MAX_GROUP];
+    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
+    int *status;
+    int entry_gran;       // table launches: granules of every entry (all have one shape)
+    int groups;           // consumer groups of a CTA
+    int accumulate;
+    int row_bytes;
+    int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
+                          // copied from the 16-byte boundary below its first byte, and its bytes sit that far
+                          // (0..15 bytes, a multiple of 2) into the row's slot
     int row_stride;       // bytes between rows inside a stage
     int unit_stride;      // bytes between the K units of one row group inside a stage
     int use_tma;          // 1: a stage arrives as one tiled tensor copy, laid out [unit][row][unit_bytes]; 2: [row][units]
     int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this
     int box_bytes;        // bytes one tensor copy signals (the whole box, also where the matrix clips it)
     int stage_bytes;
-    int n_stages;
-    int total_gran;
-    int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
-    const StreamTable *dev_table;   // when set, the matrices come from device memory
-    const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
-    int entry_gran;       // table launches: granules of every entry (all have one shape)
-    int *status;
-    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
-    GemvMat mat[KRK_CUDA_MAX_GROUP];
     // Table launches with tensor copies: every matrix of the table lies inside one of two stacked banks (the gate
     // and the up bank of an expert set), each described by ONE tensor map (wmap[0], wmap[1]) over all of its
     // rows; a matrix is then a row offset into its bank.
@@ -433,52 +434,32 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
         const uint32_t w2 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u, w1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
         const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], 0x0062), __byte_perm(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
         const int i = k0 + j4;
-        if (WT == KRK_CUDA_Q8_0 && ((i >> 5) & 1) == 0) {
-            // Even blocks start 2 bytes off a word boundary, so their lanes take the quants in the
-            // order [0,1,30,31, 2..29]; the limbs follow: pair (e, e+1) lands at position pos(e).
-            const int e = i & 31, base = i & ~31;
-            const int ka = e < 2 ? e : (e >= 30 ? e - 28 : e + 2);
-            const int e2 = e + 2;
-            const int kb = e2 < 2 ? e2 : (e2 >= 30 ? e2 - 28 : e2 + 2);
-            *reinterpret_cast<uint16_t *>(p0 + base + ka) = (uint16_t)(w0 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p0 + base + kb) = (uint16_t)(w0 >> 16);
-            *reinterpret_cast<uint16_t *>(p1 + base + ka) = (uint16_t)(w1 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p1 + base + kb) = (uint16_t)(w1 >> 16);
-            *reinterpret_cast<uint16_t *>(p2 + base + ka) = (uint16_t)(w2 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p2 + base + kb) = (uint16_t)(w2 >> 16);
-        } else if (WT == KRK_CUDA_Q5_0 && ((i >> 5) & 1) == 0) {
-            // As Q4_0, [16 of the low half][16 of the high half], but the quants of an even block start 6 bytes
-            // into it: its lanes take them rotated by two, [14,15, 0..13], so that lane t holds values 4t-2..4t+1
-            // of a half and their fifth bits are four neighbours of the rotated mask.
-            const int e = i & 15, base = (i & ~31) + (i & 16);
-            const int ka = (e + 2) & 15, kb = (e + 4) & 15;
-            *reinterpret_cast<uint16_t *>(p0 + base + ka) = (uint16_t)(w0 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p0 + base + kb) = (uint16_t)(w0 >> 16);
-            *reinterpret_cast<uint16_t *>(p1 + base + ka) = (uint16_t)(w1 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p1 + base + kb) = (uint16_t)(w1 >> 16);
-            *reinterpret_cast<uint16_t *>(p2 + base + ka) = (uint16_t)(w2 & 0xFFFF);
-            *reinterpret_cast<uint16_t *>(p2 + base + kb) = (uint16_t)(w2 >> 16);
-        } else if (WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_IQ4_NL) {
-            // A block's 16 quant bytes hold value j in their low and value 16 + j in their high nibbles, so the
-            // limbs of a block lie as [16 of the low half][16 of the high half], each in the order the lanes take
-            // the quant bytes: as they are in odd blocks; [0,1,14,15, 2..13] in even blocks, whose quants start
-            // 2 bytes off a word boundary (pairs stay together, as for Q8_0).
-            const int e = i & 15, base = (i & ~31) + (i & 16);
-            if (((i >> 5) & 1) == 0) {
-                const int e2 = e + 2;
-                const int ka = e < 2 ? e : (e >= 14 ? e - 12 : e + 2);
-                const int kb = e2 < 2 ? e2 : (e2 >= 14 ? e2 - 12 : e2 + 2);
-                *reinterpret_cast<uint16_t *>(p0 + base + ka) = (uint16_t)(w0 & 0xFFFF);
-                *reinterpret_cast<uint16_t *>(p0 + base + kb) = (uint16_t)(w0 >> 16);
-                *reinterpret_cast<uint16_t *>(p1 + base + ka) = (uint16_t)(w1 & 0xFFFF);
-                *reinterpret_cast<uint16_t *>(p1 + base + kb) = (uint16_t)(w1 >> 16);
-                *reinterpret_cast<uint16_t *>(p2 + base + ka) = (uint16_t)(w2 & 0xFFFF);
-                *reinterpret_cast<uint16_t *>(p2 + base + kb) = (uint16_t)(w2 >> 16);
+        if (WT == KRK_CUDA_Q8_0 || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_IQ4_NL) {
+            // The blocks of these formats are an odd number of half words long: the quants of every other (even) block start 2
+            // bytes off a word boundary, and their lanes take them in another order, which the limbs follow in pairs: pair
+            // (e, e + 1) lands at ka, (e + 2, e + 3) at kb. (Odd blocks go the same way, e and e + 2: no lane branches.)
+            //   Q8_0: [0,1,30,31, 2..29].
+            //   Q4_0, IQ4_NL: a block's 16 quant bytes hold value j in their low and value 16 + j in their high nibbles, so its
+            //   limbs lie as [16 of the low half][16 of the high half], each as [0,1,14,15, 2..13].
+            //   Q5_0: halves alike, but the quants start 6 bytes into the block: rotated by two, [14,15, 0..13], so that lane t
+            //   holds values 4t-2..4t+1 of a half and their fifth bits are four neighbours of the rotated mask.
+            constexpr int kRun = WT == KRK_CUDA_Q8_0 ? 32 : 16;
+            const int e = i & (kRun - 1), base = i & ~(kRun - 1);
+            int ka, kb;
+            if (WT == KRK_CUDA_Q5_0) {
+                ka = (e + 2) & 15;
+                kb = (e + 4) & 15;
             } else {
-                *reinterpret_cast<uint32_t *>(p0 + base + e) = w0;
-                *reinterpret_cast<uint32_t *>(p1 + base + e) = w1;
-                *reinterpret_cast<uint32_t *>(p2 + base + e) = w2;
+                ka = e < 2 ? e : e + 2;
+                kb = e + 2 >= kRun - 2 ? e + 6 - kRun : e + 4;
             }
+            if ((i >> 5) & 1) ka = e, kb = e + 2;
+            *reinterpret_cast<uint16_t *>(p0 + base + ka) = (uint16_t)(w0 & 0xFFFF);
+            *reinterpret_cast<uint16_t *>(p0 + base + kb) = (uint16_t)(w0 >> 16);
+            *reinterpret_cast<uint16_t *>(p1 + base + ka) = (uint16_t)(w1 & 0xFFFF);
+            *reinterpret_cast<uint16_t *>(p1 + base + kb) = (uint16_t)(w1 >> 16);
+            *reinterpret_cast<uint16_t *>(p2 + base + ka) = (uint16_t)(w2 & 0xFFFF);
+            *reinterpret_cast<uint16_t *>(p2 + base + kb) = (uint16_t)(w2 >> 16);
         } else {
             *reinterpret_cast<uint32_t *>(p0 + i) = w0;
             *reinterpret_cast<uint32_t *>(p1 + i) = w1;
@@ -549,80 +530,112 @@ __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::un
     }
 }
 
-// (the running maximum is kept on the bit patterns of |x|: they order like the values, and anything above the
-// largest finite pattern is an infinity or a NaN)
-template <int WT>
-__device__ __forceinline__ void load_slice(const float *__restrict__ x, int k0, float (&f)[Fmt<WT>::unit_values / 32],
-                                           uint32_t &mxb, bool live) {
-    constexpr int PER = Fmt<WT>::unit_values / 32;
+template <int N>
+__device__ __forceinline__ void load_values(const float *__restrict__ x, float (&f)[N]) {
 #pragma unroll
-    for (int j = 0; j < PER; j += 4) {
-        const float4 v = live ? *reinterpret_cast<const float4 *>(x + k0 + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int j = 0; j < N; j += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(x + j);
         f[j] = v.x; f[j + 1] = v.y; f[j + 2] = v.z; f[j + 3] = v.w;
     }
+}
+// max(mx, |f|), a NaN if there is one
+template <int N>
+__device__ __forceinline__ void max_abs(float &mx, const float (&f)[N]) {
 #pragma unroll
-    for (int j = 0; j < PER; j++) mxb = max(mxb, __float_as_uint(f[j]) & 0x7FFFFFFFu);
+    for (int j = 0; j < N; j += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(f[j]), "f"(f[j + 1]));
 }
 
-// All slices this warp will read of one activation row; returns the row's scale for this warp. FINE: four limbs, and the
-// last unit may hold fewer values than a full one.
-template <int WT, bool FINE>
-__device__ __forceinline__ float prepare_x_row(const float *__restrict__ xr, const StreamParams &p, int8_t *p0, int8_t *sums,
-                                               int wid, int lane) {
-    constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 2;
-    const int n_chunks = p.n_in >> kSumShift<WT>, ps = plane_stride(p.n_in);
+// All slices that a warp will read of activation rows r0, r0 + step, ... < rows (row(r) is where row r lies); scale(r, s) gets
+// the row's scale for this warp. FINE: four limbs, and the last unit may hold fewer values than a full one.
+// Every CTA prepares all of x, so this is bound by issue slots and by the latency of x: a maximum takes half an instruction a
+// value, a row's loads go out together (kHeld slices stay in registers between the maximum and the quantisation, K <= 4096;
+// further ones are read twice, kBatch at a time for the maximum), and the next row's go out before a row is quantised.
+template <int WT, bool FINE, class RowFn, class ScaleFn>
+__device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
+                                          int8_t *chunk_sum, int wid, int lane) {
+    constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
+    const int n_chunks = p.n_in >> kSumShift<WT>, ps = plane_stride(p.n_in), units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
-    auto quantize = [&](const float (&f)[PER], float inv, int u) {
-        if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
-        else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
+    // (where a warp has no such slice, or a lane no such value, it reads another of its own: the maximum is none the worse)
+    auto from = [&](int u) {
+        const int v = u < units ? u : wid;
+        return live(v) ? at(v) : v * UV;
     };
-    // the first two slices stay in registers between the max and the quantisation (K <= 4096 for
-    // 256-value units); any further ones are read twice
-    float held[kHeld][PER];
-    uint32_t mxb = 0u;
+    float held[kHeld][PER], next[kHeld][PER];
+    auto load = [&](const float *xr, float (&f)[kHeld][PER]) {
 #pragma unroll
-    for (int j = 0; j < kHeld; j++) {
-        const int u = wid + j * kConsumerWarps;
-        if (u < p.units) load_slice<WT>(xr, at(u), held[j], mxb, live(u));
-    }
-    for (int u = wid + kHeld * kConsumerWarps; u < p.units; u += kConsumerWarps) {
-        float f[PER];
-        load_slice<WT>(xr, at(u), f, mxb, live(u));
-    }
-    mxb = __reduce_max_sync(0xFFFFFFFFu, mxb);
-    // |x * inv| <= 2^22 over the whole f32 range: where the quotient would overflow, a power of two takes its place; a
-    // non-finite activation makes the output NaN
-    const float mx = __uint_as_float(mxb);
-    float inv, s;
-    if constexpr (FINE) {   // the power of two that takes the maximum to 2^21 .. 2^22, 2^127 at most
-        const uint32_t e = min(275u - (mxb >> 23), 254u);
-        inv = __uint_as_float(e << 23);
-        s = __uint_as_float(e < 254u ? (254u - e) << 23 : 0x00400000u);
-    } else {
-        inv = __fdiv_rn(kFixedOne, mx);
-        s = __fdiv_rn(mx, kFixedOne);
-        if (mx < 1.25e-32f) {
-            inv = 1.7014118346046923e38f;   // 2^127
-            s = 5.877471754111438e-39f;     // 2^-127
+        for (int j = 0; j < kHeld; j++) load_values(xr + from(wid + j * kConsumerWarps), f[j]);
+    };
+    if (r0 >= rows || wid >= units) return;
+    const float *xr = row(r0);
+    load(xr, held);
+#pragma unroll 1
+    for (int r = r0; r < rows; r += step) {
+        float mx = 0.0f;
+#pragma unroll 1
+        for (int u0 = wid + kHeld * kConsumerWarps; u0 < units; u0 += kBatch * kConsumerWarps) {
+            float f[kBatch][PER];
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) load_values(xr + from(u0 + j * kConsumerWarps), f[j]);
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) max_abs(mx, f[j]);
         }
-    }
-    if (mxb > 0x7F7FFFFFu) {
-        inv = 0.0f;
-        s = __int_as_float(0x7FC00000);
-    }
 #pragma unroll
-    for (int j = 0; j < kHeld; j++) {
-        const int u = wid + j * kConsumerWarps;
-        if (u < p.units) quantize(held[j], inv, u);
+        for (int j = 0; j < kHeld; j++) max_abs(mx, held[j]);
+        const float *const xr1 = r + step < rows ? row(r + step) : xr;
+        if (r + step < rows) load(xr1, next);
+        // (bit patterns of magnitudes order like the values, infinities and NaNs above them)
+        const uint32_t mxb = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(mx));
+        // |x * inv| <= 2^22 over the whole f32 range: where the quotient would overflow, a power of two takes its place; a
+        // non-finite activation makes the output NaN
+        mx = __uint_as_float(mxb);
+        float inv, s;
+        if constexpr (FINE) {   // the power of two that takes the maximum to 2^21 .. 2^22, 2^127 at most
+            const uint32_t e = min(275u - (mxb >> 23), 254u);
+            inv = __uint_as_float(e << 23);
+            s = __uint_as_float(e < 254u ? (254u - e) << 23 : 0x00400000u);
+        } else {
+            inv = __fdiv_rn(kFixedOne, mx);
+            s = __fdiv_rn(mx, kFixedOne);
+            if (mx < 1.25e-32f) {
+                inv = 1.7014118346046923e38f;   // 2^127
+                s = 5.877471754111438e-39f;     // 2^-127
+            }
+        }
+        if (mxb > 0x7F7FFFFFu) {
+            inv = 0.0f;
+            s = __int_as_float(0x7FC00000);
+        }
+        int8_t *p0 = planes + (size_t)(r * (FINE ? 4 : 3)) * ps, *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
+        auto quantize = [&](const float (&f)[PER], int u) {
+            if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
+            else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
+        };
+#pragma unroll
+        for (int j = 0; j < kHeld; j++) {
+            const int u = wid + j * kConsumerWarps;
+            if (u < units) quantize(held[j], u);
+        }
+        int u = wid + kHeld * kConsumerWarps;
+        if (u < units) {
+            float f[PER], g[PER];
+            load_values(xr + from(u), f);
+#pragma unroll 1
+            for (; u < units; u += kConsumerWarps) {
+                load_values(xr + from(u + kConsumerWarps), g);
+                quantize(f, u);
+#pragma unroll
+                for (int j = 0; j < PER; j++) f[j] = g[j];
+            }
+        }
+        scale(r, s);
+        xr = xr1;
+#pragma unroll
+        for (int j = 0; j < kHeld; j++)
+#pragma unroll
+            for (int i = 0; i < PER; i++) held[j][i] = next[j][i];
     }
-    for (int u = wid + kHeld * kConsumerWarps; u < p.units; u += kConsumerWarps) {
-        float f[PER];
-        uint32_t m2 = 0u;
-        load_slice<WT>(xr, at(u), f, m2, live(u));
-        quantize(f, inv, u);
-    }
-    return s;
 }
 
 // ---- per-format unit kernels -------------------------------------------------------------------------
@@ -1482,22 +1495,18 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
 
     if (warp == 0) {
         // ===== producer warp: weights only, so it can run ahead of everything else =====
-        if (lane == 0) {
-            for (int s = 0; s < p.n_stages; s++) {
-                mbar_init(smem_u32(&sm->full[s]), 1);
-                mbar_init(smem_u32(&sm->empty[s]), kGroups * kConsumerWarps);
-            }
-            for (int s = 0; s < kGroups * red_slots(NG); s++) {
-                mbar_init(smem_u32(&sm->red_full[s]), n_warps);
-                mbar_init(smem_u32(&sm->red_empty[s]), 1);
-            }
-            sm->gave_up = 0;
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __threadfence_block();
-        }
+        // (a lane per barrier)
+        static_assert(kMaxStages == 8 && kGroups * red_slots(NG) <= kMaxRedSlots && kMaxRedSlots == 4, "24 lanes");
+        if (lane < 8) mbar_init(smem_u32(&sm->full[lane]), 1);
+        else if (lane < 16) mbar_init(smem_u32(&sm->empty[lane - 8]), kGroups * kConsumerWarps);
+        else if (lane < 20) mbar_init(smem_u32(&sm->red_empty[lane - 16]), 1);
+        else if (lane < 24) mbar_init(smem_u32(&sm->red_full[lane - 20]), n_warps);
+        else if (lane == 24) sm->gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __threadfence_block();
         __syncwarp();
-        // the other warps wait here for the barriers (they arrive as they start); this warp does not wait
+        // the other warps wait for the barriers here before they first look at one; this warp does not wait
         asm volatile("bar.arrive 1, %0;" ::"r"(kThreads) : "memory");
         // A device-side table is the output of the kernel before this one: wait for that grid.
         if (p.dev_table) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1560,12 +1569,17 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         });
         return;
     }
-    asm volatile("bar.sync 1, %0;" ::"r"(kThreads) : "memory");
     if (p.dev_table) asm volatile("griddepcontrol.wait;" ::: "memory");
     const TableView tv(p);
+    bool synced = false;   // the barriers are known to be there
+    auto sync_start = [&] {
+        asm volatile("bar.sync 1, %0;" ::"r"(kThreads) : "memory");
+        synced = true;
+    };
 
     if (warp == kEpilogueWarp) {
         // ===== epilogue warp =====
+        sync_start();
         // Output (row, activation row) of a tile is the sum, over the consumer warps in warp order, of the
         // share each warp left in `red` (already added up over the four lanes of a row group).
         constexpr int kSlots = red_slots(NG);
@@ -1712,31 +1726,36 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             // x may be the output of the kernel before this one (and y its input): wait for that grid to
             // complete. Weights are never written by a kernel in flight, so the producer warp does not wait.
             if (prepared == nullptr) {
-                // (x to level 2 meanwhile, where it is coherent whoever still writes it)
-                for (int u = my_unit; u < p.units; u += kConsumerWarps)
-                    if (u * F::unit_values + lane * (F::unit_values / 32) < p.n_in)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(x + u * F::unit_values + lane * (F::unit_values / 32)));
+                // (x to level 2 meanwhile, where it is coherent whoever still writes it: a lane per 128-byte line of the warp's slices)
+                constexpr int kLines = F::unit_values / 32;
+                if (!p.dev_table)   // (a table's launch has waited)
+                    for (int r = grp; r < (SINGLE ? 1 : p.rows); r += kGroups)
+                        for (int l = lane; my_unit + l / kLines * kConsumerWarps < p.units; l += 32) {
+                            const int k = (my_unit + l / kLines * kConsumerWarps) * F::unit_values + l % kLines * 32;
+                            if (!kFine || k < p.n_in) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (size_t)r * p.n_in + k));
+                        }
                 asm volatile("griddepcontrol.wait;" ::: "memory");
             }
             // (stacked tiles: every sub-tile prepares its own copy)
-            auto prepare = [&](int r) {
-                return prepare_x_row<WT, kFine>(x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in), p, planes + (size_t)(r * (kFine ? 4 : 3)) * plane_stride(p.n_in),
-                                                                      chunk_sum + (size_t)(r * 4) * (p.n_in >> kSumShift<WT>),
-                                                                      stacked_idle ? p.units : my_unit, lane);
-            };
+            auto row = [&](int r) { return x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in); };
+            const int first_unit = stacked_idle ? p.units : my_unit;
             if (kGroups == 1) {
 #pragma unroll
-                for (int r = 0; r < 2 * NG; r++) xs[r] = r < p.rows ? prepare(r) : 0.0f;
+                for (int r = 0; r < 2 * NG; r++) xs[r] = 0.0f;
+                prepare_x<WT, kFine>(row, [&](int r, float v) {
+#pragma unroll
+                    for (int q = 0; q < 2 * NG; q++) xs[q] = q == r ? v : xs[q];
+                }, 0, 1, SINGLE ? 1 : p.rows, p, planes, chunk_sum, first_unit, lane);
                 __syncwarp();
+                if (!synced) sync_start();
             } else {
                 // each group prepares every other row; nobody may still read the activation before this one
                 if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
-#pragma unroll 1
-                for (int r = grp; r < p.rows; r += kGroups) {
-                    const float sc = prepare(r);
-                    if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = sc;
-                }
-                asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
+                prepare_x<WT, kFine>(row, [&](int r, float v) {
+                    if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = v;
+                }, grp, kGroups, p.rows, p, planes, chunk_sum, first_unit, lane);
+                if (!synced) sync_start();
+                else asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
 #pragma unroll
                 for (int r = 0; r < (kFold ? kFoldRows<NG> : 2 * NG); r++) {
                     const int row = kFold ? t + 4 * r : r;
@@ -1946,6 +1965,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
         }
     }
+    if (!synced) sync_start();   // (a CTA without work)
 }
 
 template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG)>
