@@ -73,6 +73,7 @@ constexpr int kPlanePad = 32;                     // bytes between limb planes b
 constexpr float kFixedOne = 4194303.0f;           // 2^22 - 1: every limb stays in s8 and X = rint(x / s) is one FMA against
                                                   // the bits of 1.5 * 2^23 (no conversion instruction)
 constexpr long long kWaitCycles = 4000000000LL;   // ~2 s at boost clock, then give up
+constexpr uint32_t kWaitHalfMs = (uint32_t)(kWaitCycles >> 20);
 
 template <int WT> struct Fmt;
 // tma: how a stage can arrive as ONE tiled tensor copy. 1: a unit is a whole number of 16-byte granules (Q4_K's
@@ -255,25 +256,19 @@ __device__ __forceinline__ float half_hi(uint32_t w) { return __half2float(__ush
 // Bounded wait on an mbarrier phase. Once any wait in the CTA has given up, every later wait
 // returns at once, so the CTA runs to its end (on stale data, inside its own buffers) instead
 // of hanging.
-static __device__ __noinline__ void wait_phase_slow(uint32_t bar, uint32_t parity, volatile int *gave_up, int *status) {
-    const long long t0 = clock64();
-    for (;;) {
-        for (int i = 0; i < 32; i++) {
-            if (mbar_try_wait(bar, parity)) return;
-            __nanosleep(20);   // leave the issue slots to the warps that have work
-        }
+// (Inline: around a call the kernels kept a frame of local memory, whose first accesses miss level 1 in every launch.)
+__device__ __forceinline__ uint32_t half_milliseconds() { return (uint32_t)(clock64() >> 20); }   // about
+__device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volatile int *gave_up, int *status) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint32_t t0 = half_milliseconds();
+    while (!mbar_try_wait(bar, parity)) {   // (the hardware suspends the warp for a while in each)
         if (*gave_up) return;
-        if (clock64() - t0 > kWaitCycles) {
+        if (half_milliseconds() - t0 > kWaitHalfMs) {
             *gave_up = 1;
             atomicExch(status, KRK_CUDA_ETIMEOUT);
             return;
         }
     }
-}
-__device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volatile int *gave_up, int *status) {
-    if (mbar_try_wait(bar, parity)) return;
-    if (*gave_up) return;
-    wait_phase_slow(bar, parity, gave_up, status);
 }
 
 // ---- shared-memory map ---------------------------------------------------------------------------
@@ -534,8 +529,9 @@ template <int N>
 __device__ __forceinline__ void load_values(const float *__restrict__ x, float (&f)[N]) {
 #pragma unroll
     for (int j = 0; j < N; j += 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(x + j);
-        f[j] = v.x; f[j + 1] = v.y; f[j + 2] = v.z; f[j + 3] = v.w;
+        // (in this order, all before their first use: left to itself the compiler put some behind the others' arithmetic, a round trip
+        // to level 2 more: Q4_K 4096 x 4096 at four rows 8.55 against 7.79 us)
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[j]), "=f"(f[j + 1]), "=f"(f[j + 2]), "=f"(f[j + 3]) : "l"(x + j) : "memory");
     }
 }
 // max(mx, |f|), a NaN if there is one
@@ -833,7 +829,8 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
     // min term, also exact: one k16 MMA of the 8 mins of the super-block (k slots 0..7) against the
     // per-chunk sums of X, held as 4 limbs x 2 activation rows in the 8 columns
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
-    const uint32_t a0 = t < 2 ? mnA[t & 1] : 0u, a1 = t < 2 ? mnB[t & 1] : 0u;
+    // (no index that depends on the lane: that would put the words in local memory)
+    const uint32_t a0 = t == 0 ? mnA[0] : t == 1 ? mnA[1] : 0u, a1 = t == 0 ? mnB[0] : t == 1 ? mnB[1] : 0u;
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 5) + 4 * (t & 1));
@@ -899,7 +896,8 @@ __device__ __forceinline__ void unit_q4_k_single(const uint8_t *rowA, const uint
     acc.f[0] = fmaf(dA, (float)(16 * loA + hrA - hlA), acc.f[0]);
     acc.f[1] = fmaf(dB, (float)(16 * loB + hrB - hlB), acc.f[1]);
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
-    const uint32_t a0 = t < 2 ? mnA[t & 1] : 0u, a1 = t < 2 ? mnB[t & 1] : 0u;
+    // (no index that depends on the lane: that would put the words in local memory)
+    const uint32_t a0 = t == 0 ? mnA[0] : t == 1 ? mnA[1] : 0u, a1 = t == 0 ? mnB[0] : t == 1 ? mnB[1] : 0u;
     float cm[4];
     mma_s8_k16_biased(cm, a0, a1, bf.m);   // |sum| <= 8 x 63 x 128 < 2^22
     acc.m[0] = fmaf(nA, cm[0], acc.m[0]);
@@ -1583,9 +1581,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         // Output (row, activation row) of a tile is the sum, over the consumer warps in warp order, of the
         // share each warp left in `red` (already added up over the four lanes of a row group).
         constexpr int kSlots = red_slots(NG);
-        float gate_reg[NG];   // gate tile kept for the silu fold (stacked tiles keep theirs in shared memory)
-        int tile_it = 0;
-        walk(p, tv, tps, [](int) {}, [&](const StageInfo &s) {
+        float gate_reg[NG];   // silu of the gate tile (stacked tiles keep theirs in shared memory)
+        int tile_it = 0, n_out = 0;
+        float *y0 = nullptr;
+        walk(p, tv, tps, [&](int m) {
+            y0 = tv.y(m);
+            n_out = tv.n_out(m);
+        }, [&](const StageInfo &s) {
             if (!s.last) return;
             // (two groups take the tiles in turn, each through slots of its own)
             const int nth = tile_it / kGroups, slot = (tile_it % kGroups) * kSlots + nth % kSlots;
@@ -1612,7 +1614,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     }
                     if (r < p.rows) {
                         if (p.step == 2 && s.which == 0) {
-                            if (STACK) sm->gate[sub][i][lane] = v;   // kept for the silu fold with the `up` tile
+                            v = __fdiv_rn(v, __fadd_rn(1.0f, exp_as_host(-v)));   // kept for the `up` tile
+                            if (STACK) sm->gate[sub][i][lane] = v;
                             else gate_reg[i] = v;
                         } else if (srow < s.n_rows) {
                             if (p.n_peers > 0) {
@@ -1620,10 +1623,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                                 const long long at = (long long)r * p.peer_row_stride + p.peer_offset + s.row0 + srow;
                                 for (int q = 0; q < p.n_peers; q++) p.peer_y[q][at] = v;
                             } else {
-                                const int om = p.step == 2 ? s.mat - 1 : s.mat;
-                                float *y = tv.y(om) + (size_t)r * tv.n_out(om) + s.row0 + srow;
-                                const float gt = STACK ? sm->gate[sub][i][lane] : gate_reg[i];
-                                if (p.step == 2) v = __fmul_rn(__fdiv_rn(gt, __fadd_rn(1.0f, exp_as_host(-gt))), v);
+                                float *y = y0 + (size_t)r * n_out + s.row0 + srow;
+                                if (p.step == 2) v = __fmul_rn(STACK ? sm->gate[sub][i][lane] : gate_reg[i], v);
                                 *y = p.accumulate ? __fadd_rn(*y, v) : v;
                             }
                         }
@@ -1704,16 +1705,21 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
 
     // The same walk as walk() above, written flat: per stage a consumer warp only needs the ring
     // slot and its K units, not which matrix or rows the tile belongs to.
-    const int cta = (int)blockIdx.x;
-    const int g0 = cta * tv.gran_q + min(cta, tv.gran_r);
-    const int g1 = g0 + tv.gran_q + (cta < tv.gran_r ? 1 : 0);
     const int n_chunks = p.whole_tiles ? 1 : (p.units + kConsumerWarps - 1) / kConsumerWarps;
     const uint32_t full0 = smem_u32(&sm->full[0]), empty0 = smem_u32(&sm->empty[0]);
     int slot = 0;
     uint32_t phase = 0;
-    for (int e = tv.first(g0); e < tv.n_entries; e++) {
+    // (What only the step from one entry to the next needs is worked out there again: registers are short in the tile loop, and
+    // spilled ones miss level 1 at their first use in a launch.)
+    for (int e = -1;;) {
+        int cta;
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
+        const TableView tv(p);
+        const int g0 = cta * tv.gran_q + min(cta, tv.gran_r);
+        const int g1 = g0 + tv.gran_q + (cta < tv.gran_r ? 1 : 0);
+        e = e < 0 ? tv.first(g0) : e + 1;
+        if (e >= tv.n_entries || tv.begin(e) >= g1) break;
         const int lo = max(g0, tv.begin(e)), hi = min(g1, tv.begin(e + 1));
-        if (tv.begin(e) >= g1) break;
         if (lo >= hi) continue;
         const int m = e * p.step;
         const int r0 = (lo - tv.begin(e)) * p.gran;
