@@ -121,6 +121,7 @@ struct StreamParams {
     int *status;
     int entry_gran;       // table launches: granules of every entry (all have one shape)
     int groups;           // consumer groups of a CTA
+    int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
     int accumulate;
     int row_bytes;
     int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
@@ -830,10 +831,10 @@ __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *ro
     // per-chunk sums of X, held as 4 limbs x 2 activation rows in the 8 columns
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
     // (no index that depends on the lane: that would put the words in local memory)
-    const uint32_t a0 = t == 0 ? mnA[0] : t == 1 ? mnA[1] : 0u, a1 = t == 0 ? mnB[0] : t == 1 ? mnB[1] : 0u;
+    const uint32_t a0 = t & 1 ? mnA[1] : mnA[0], a1 = t & 1 ? mnB[1] : mnB[0];   // (k slots 8..15, lanes 2 and 3, meet zeros)
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 5) + 4 * (t & 1));
+        const uint32_t b0 = t < 2 ? *reinterpret_cast<const uint32_t *>(sp[mg] + (kbase >> 5) + 4 * t) : 0u;
         int cc[4];
         mma_s8_k16(cc, a0, a1, b0);
         add_min(acc, nA, nB, cc, mg);
@@ -861,7 +862,7 @@ __device__ __forceinline__ BFrag load_bfrag(const int8_t *bq, const int8_t *sq, 
     BFrag f;
 #pragma unroll
     for (int p = 0; p < 4; p++) f.b[p] = *reinterpret_cast<const uint2 *>(bq + 64 * p + 8 * t);
-    f.m = *reinterpret_cast<const uint32_t *>(sq + 4 * (t & 1));
+    f.m = t < 2 ? *reinterpret_cast<const uint32_t *>(sq + 4 * t) : 0u;
     return f;
 }
 __device__ __forceinline__ void unit_q4_k_single(const uint8_t *rowA, const uint8_t *rowB, const BFrag &bf, int t,
@@ -897,7 +898,7 @@ __device__ __forceinline__ void unit_q4_k_single(const uint8_t *rowA, const uint
     acc.f[1] = fmaf(dB, (float)(16 * loB + hrB - hlB), acc.f[1]);
     const float nA = half_hi(hA.x), nB = half_hi(hB.x);
     // (no index that depends on the lane: that would put the words in local memory)
-    const uint32_t a0 = t == 0 ? mnA[0] : t == 1 ? mnA[1] : 0u, a1 = t == 0 ? mnB[0] : t == 1 ? mnB[1] : 0u;
+    const uint32_t a0 = t & 1 ? mnA[1] : mnA[0], a1 = t & 1 ? mnB[1] : mnB[0];   // (k slots 8..15, lanes 2 and 3, meet zeros)
     float cm[4];
     mma_s8_k16_biased(cm, a0, a1, bf.m);   // |sum| <= 8 x 63 x 128 < 2^22
     acc.m[0] = fmaf(nA, cm[0], acc.m[0]);
@@ -1446,6 +1447,9 @@ template <int WT>
 constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_size(WT) == 32;
 template <int WT>
 constexpr bool kMayRag = kRagForm<WT> || WT == KRK_CUDA_Q2_K;
+// Forms whose two groups may take a tile's stages in turn (StreamParams::by_stage).
+template <int WT>
+__host__ __device__ constexpr bool may_by_stage(bool ragged, int groups) { return kRagForm<WT> && block_size(WT) == 256 && ragged && groups == 2; }
 // One result in f32 throughout, by one lane: what an infinity among the activations makes of a row (an infinity of either
 // sign, or a NaN against a zero weight) is not in the limbs, which give a NaN.
 template <int WT>
@@ -1465,6 +1469,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kGroups = GROUPS, kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
     constexpr bool kFine = RAG && !kSuper;   // fine_limbs
+    constexpr bool kMayByStage = may_by_stage<WT>(RAG, kGroups);
     using F = Fmt<WT>;
     using SmemT = Smem<NG, GROUPS>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1590,8 +1595,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         }, [&](const StageInfo &s) {
             if (!s.last) return;
             // (two groups take the tiles in turn, each through slots of its own)
-            const int nth = tile_it / kGroups, slot = (tile_it % kGroups) * kSlots + nth % kSlots;
+            const bool both = kMayByStage && p.by_stage;   // (a tile's sums come from both, through a slot of each)
+            const int nth = both ? tile_it : tile_it / kGroups, slot = (both ? 0 : (tile_it % kGroups) * kSlots) + nth % kSlots;
             wait_phase(smem_u32(&sm->red_full[slot]), (nth / kSlots) & 1, gave_up, p.status);
+            if (both) wait_phase(smem_u32(&sm->red_full[slot + kSlots]), (nth / kSlots) & 1, gave_up, p.status);
             tile_it++;
 #pragma unroll
             for (int sub = 0; sub < (STACK ? kMaxStack : 1); sub++) {
@@ -1607,6 +1614,13 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     float v = 0.0f;
 #pragma unroll
                     for (int w = 0; w < kConsumerWarps; w++) v += part[w];
+                    if (both) {
+                        const float *src1 = src + (size_t)kSlots * (kConsumerWarps * NG * 8 * 4);
+#pragma unroll
+                        for (int w = 0; w < kConsumerWarps; w++) part[w] = src1[(size_t)w * (NG * 8 * 4)];
+#pragma unroll
+                        for (int w = 0; w < kConsumerWarps; w++) v += part[w];
+                    }
                     const int srow = kTileRows * sub + row;   // row inside the stage
                     if (kFine && v != v && r < p.rows && srow < s.n_rows) {
                         const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
@@ -1632,7 +1646,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm->red_empty[slot]));
+            if (lane == 0) {
+                mbar_arrive(smem_u32(&sm->red_empty[slot]));
+                if (both) mbar_arrive(smem_u32(&sm->red_empty[slot + kSlots]));
+            }
         });
         if (p.n_peers > 0) {
             // This CTA's stores are out. The CTA that reports last publishes the epoch to every peer and
@@ -1789,19 +1806,21 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         const int stage_rows = kTileRows * tps;
         const int n_tiles = ((r1 - r0 + stage_rows - 1) / stage_rows) * p.step;
         for (int tile = 0; tile < n_tiles; tile++) {
-            if (kGroups > 1 && tile_it % kGroups != grp) {
-                // the other group's tile: its stages are seen to land (a ring slot's parity only tells two laps apart for a
-                // warp that looks at every lap) and given back
-                tile_it++;
-                for (int ck = 0; ck < n_chunks; ck++) {
-                    wait_phase(full0 + 8 * slot, phase, gave_up, p.status);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(empty0 + 8 * slot);
-                    if (++slot == p.n_stages) {
-                        slot = 0;
-                        phase ^= 1;
-                    }
+            // the other group's stage: it is seen to land (a ring slot's parity only tells two laps apart for a warp that looks at
+            // every lap) and given back
+            auto pass = [&] {
+                wait_phase(full0 + 8 * slot, phase, gave_up, p.status);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty0 + 8 * slot);
+                if (++slot == p.n_stages) {
+                    slot = 0;
+                    phase ^= 1;
                 }
+            };
+            const bool by_stage = kMayByStage && p.by_stage;
+            if (kGroups == 2 && !by_stage && tile_it % 2 != grp) {
+                tile_it++;
+                for (int ck = 0; ck < n_chunks; ck++) pass();
                 continue;
             }
             // ragged rows: how far this lane's two rows sit into their slots of a stage
@@ -1873,12 +1892,15 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                 stage(0, held[0]);
                 if (n_chunks > 1) stage(1, held[1]);
             } else {
-                for (int ck = 0; ck < n_chunks; ck++) stage(ck, held[0]);
+                for (int ck = 0; ck < n_chunks; ck++) {
+                    if (by_stage && (ck & 1) != grp) pass();
+                    else stage(ck, held[0]);
+                }
             }
             {
              // ---- end of the tile: the lanes of a row group add their weighted shares ----
              constexpr int kSlots = red_slots(NG);
-             const int nth = tile_it / kGroups, rslot = grp * kSlots + nth % kSlots;
+             const int nth = by_stage ? tile_it : tile_it / kGroups, rslot = grp * kSlots + nth % kSlots;
              const uint32_t rphase = (nth / kSlots) & 1;
              tile_it++;
              if (wid >= n_warps) continue;
@@ -2094,6 +2116,13 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     const int most = halves ? kMaxHalfStages : kMaxStages;
     p.n_stages = max_fit < most ? max_fit : most;
     if (p.n_stages < 2) return false;
+    // Two groups that take tiles in turn want a ring that holds a tile of each: a stage of the second tile only lands when one of
+    // the first is done with. Where it does not, they take a tile's stages in turn (Q6_K 4096 x 11008 at four rows, six stages to
+    // a tile and a ring of three: 25.8 -> 24.4 us; three stages to a tile leave one group twice the other's: 14.9 -> 15.3). Only in
+    // the forms for ragged rows of the super-block formats, which such rows mostly are: the others would lose 2 to 4 % to the code
+    // and gain nothing (Q4_K 4096 x 11008 17.5 -> 18.7 us).
+    p.by_stage = may_by_stage<WT>(p.ragged != 0, p.groups) && p.units > 3 * kConsumerWarps &&
+                 p.n_stages < 2 * ((p.units + kConsumerWarps - 1) / kConsumerWarps);
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
     return true;
 }

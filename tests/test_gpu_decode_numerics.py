@@ -168,3 +168,21 @@ def test_rows_of_odd_block_counts_on_either_kernel(cuda, wt):
                 # (the bound of the f32 kernel's distance above, for its longer rows too)
                 assert ((y.double() - want).norm() / want.norm()).item() <= 3e-7, (n_out, n_in, rows)
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("wt", FORMATS)
+@pytest.mark.parametrize("n_in", [2304, 4352, 6656, 11008, 12544])
+def test_rows_of_many_slices(cuda, oracle, wt, n_in):
+    """A warp prepares one to seven slices of every activation row (held, in one batch of loads, in a second), and two groups
+    of warps share a tile's stages where the ring does not hold two tiles. 22 bits of the largest activation of a warp's slices
+    (about four sigma here) leave 4 * 2^-22 / sqrt(12) a value, 2.8e-7 of the norms' product for a result; seven times that."""
+    n_out = 80
+    w = synth.weights(wt, n_out, n_in, SEED + 2, stream=wt)
+    w64 = oracle.dequant_rows(w, wt, n_out, n_in).astype(np.float64)
+    x = synth.activations(6, n_in, SEED + 3)
+    x[1] *= 1e-3
+    for rows in (1, 2, 3, 4, 6):
+        y = cuda.gemv(dev(x[:rows]), dev(w), wt, n_out, n_in).cpu().numpy()
+        x64 = x[:rows].astype(np.float64)
+        lim = 2e-6 * np.linalg.norm(w64, axis=1)[None] * np.linalg.norm(x64, axis=1)[:, None]
+        assert (np.abs(y.reshape(rows, n_out) - x64 @ w64.T) <= lim).all(), rows
