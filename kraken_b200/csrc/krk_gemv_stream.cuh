@@ -69,7 +69,6 @@ constexpr int kMaxHalfStages = 4;                // of a half-SM one. Measured: 
                                                  // 0.89 of the copy bandwidth, five (all that fit) at 0.86, three at 0.86
 constexpr int kSmemLimit = 113 * 1024;           // two CTAs per SM (228 KB, 1 KB reserved per CTA)
 constexpr int kSmemWhole = 227 * 1024;
-constexpr int kPlanePad = 32;                     // bytes between limb planes beyond n_in: spreads the B-fragment loads over the banks
 constexpr float kFixedOne = 4194303.0f;           // 2^22 - 1: every limb stays in s8 and X = rint(x / s) is one FMA against
                                                   // the bits of 1.5 * 2^23 (no conversion instruction)
 constexpr long long kWaitCycles = 4000000000LL;   // ~2 s at boost clock, then give up
@@ -106,8 +105,8 @@ struct StreamParams {
     int rows;             // activation rows
     int units;            // n_in / unit_values
     int n_in;
-    int total_gran;
-    int gran_q, gran_r;   // total_gran = grid * gran_q + gran_r
+    int plane_pitch;      // bytes from a limb plane of the prepared activation to the next, see plane_pitch()
+    int gran_q, gran_r;   // granules in all = grid * gran_q + gran_r
     const StreamTable *dev_table;   // when set, the matrices come from device memory
     const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
     int gran;             // rows per granule: 1, or 8 when rows are not 16-byte multiples
@@ -119,6 +118,8 @@ struct StreamParams {
     GemvMat mat[KRK_CUDA_MAX_GROUP];
     int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
     int *status;
+    int row_pitch;        // bytes from an activation row's planes to the next row's
+    int plane_bytes;      // of all rows
     int entry_gran;       // table launches: granules of every entry (all have one shape)
     int groups;           // consumer groups of a CTA
     int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
@@ -290,22 +291,41 @@ struct Smem {
 
 __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
-__host__ __device__ inline int plane_stride(int n_in) { return n_in + kPlanePad; }
 // Limbs of an activation: three, or four where K is not a multiple of 256. Those shapes belong to the warp-per-row kernel
 // otherwise, which multiplies in f32; 22 bits against the largest magnitude of a warp's slices are 2 to 9 times as far off
 // (error against f64 of 2.3e-7 to 1.1e-6, f32: 1.2e-7), and the MMA's fourth column was unused.
 template <int WT>
 __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
+// Where the planes lie, so that the eight columns of a B fragment (rows and limbs as lane_planes deals them) are read from
+// different banks. Q4_K and Q5_K load 8 bytes a lane, 32 a column: limbs lie 32 bytes on, rows 64 (modulo 128). The others load 4,
+// 16 a column: limbs 16 on; rows 32 in the folded form of the super-block formats, else next to each other. (The one-row form of
+// Q4_0 takes a limb in two columns; Q5_0 loses 3 % at eight rows with limbs 16 on.) Limbs 32 on in all and rows next to each
+// other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows 33.9 -> 32.1 us, Q6_K at four 32.9 -> 31.2, Q5_K at
+// four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.6.
 template <int WT>
-__host__ __device__ inline int plane_bytes(int n_in, int rows) { return align_up(rows * (fine_limbs<WT>(n_in) ? 4 : 3) * plane_stride(n_in), 128); }
+inline int plane_pitch(int n_in, int rows) {
+    const bool wide = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1);
+    return align_up(n_in, 128) + (wide ? 32 : 16);
+}
+template <int WT>
+inline int plane_row_pitch(int n_in, int rows) {
+    const int planes = (fine_limbs<WT>(n_in) ? 4 : 3) * plane_pitch<WT>(n_in, rows);
+    return planes + (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K ? 96 : block_size(WT) == 256 && rows > 2 ? 112 : 0);
+}
 // Sums of the quantised activation over the stretch of K that shares one minimum or offset: 32 values (2^5) for
 // Q4_K, Q5_K, Q4_0 and Q5_1, 16 for Q2_K.
 template <int WT>
 constexpr int kSumShift = WT == KRK_CUDA_Q2_K ? 4 : 5;
+// Elements from a plane of sums to the next: signed-byte limbs (four planes a row, 16 bytes apart modulo 128: eight columns are
+// read at a time), or one plane of floats a row (Q4_0, Q5_1).
 template <int WT>
-__host__ __device__ inline int chunk_sum_bytes(int n_in, int rows) {   // [row][4 limbs][n_in >> kSumShift] s8
+__host__ __device__ inline int sum_pitch(int n_in) {
+    return WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K ? align_up(n_in >> kSumShift<WT>, 128) + 16 : n_in >> 5;
+}
+template <int WT>
+__host__ __device__ inline int chunk_sum_bytes(int n_in, int rows) {   // four planes of bytes or one of floats
     return (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_Q5_1 || WT == KRK_CUDA_Q2_K)
-               ? align_up(rows * (n_in >> kSumShift<WT>) * 4, 128) : 0;   // Q4_0, Q5_1: [row][n_in / 32] f32
+               ? align_up(rows * 4 * sum_pitch<WT>(n_in), 128) : 0;
 }
 
 // ---- the walk over this CTA's stages: identical in the producer and in the consumers -------------
@@ -551,7 +571,7 @@ template <int WT, bool FINE, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
-    const int n_chunks = p.n_in >> kSumShift<WT>, ps = plane_stride(p.n_in), units = p.units;
+    const int n_chunks = sum_pitch<WT>(p.n_in), ps = p.plane_pitch, units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
     // (where a warp has no such slice, or a lane no such value, it reads another of its own: the maximum is none the worse)
@@ -604,7 +624,7 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
             inv = 0.0f;
             s = __int_as_float(0x7FC00000);
         }
-        int8_t *p0 = planes + (size_t)(r * (FINE ? 4 : 3)) * ps, *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
+        int8_t *p0 = planes + (size_t)r * p.row_pitch, *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
         auto quantize = [&](const float (&f)[PER], int u) {
             if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
             else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
@@ -750,7 +770,7 @@ __device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
 // accumulator columns are never looked at, so what it multiplies does not matter.
 template <int NG, bool FOLD, bool FINE>
-__device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int n_in, int n_sums, int rows, int g,
+__device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int plane_pitch, int row_pitch, int n_sums, int rows, int g,
                                             const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
@@ -769,7 +789,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
             r = g;
             limb = mg % 3;
         }
-        bp[mg] = planes + (size_t)(min(r, rows - 1) * (FINE ? 4 : 3) + limb) * plane_stride(n_in);
+        bp[mg] = planes + (size_t)min(r, rows - 1) * row_pitch + limb * plane_pitch;
         sp[mg] = chunk_sum + (size_t)(min(rs, rows - 1) * 4 + ls) * n_sums;
     }
 }
@@ -1477,7 +1497,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     int8_t *planes = reinterpret_cast<int8_t *>(smem_raw + align_up((int)sizeof(SmemT), 128));
     // one copy of the prepared activation per stacked sub-tile: the warps of a sub-tile move on to the next
     // matrix (and its activation) on their own, so they must not share planes with another sub-tile
-    int8_t *chunk_sum = planes + tps * plane_bytes<WT>(p.n_in, p.rows);
+    int8_t *chunk_sum = planes + tps * p.plane_bytes;
     uint8_t *stages = reinterpret_cast<uint8_t *>(chunk_sum) + tps * chunk_sum_bytes<WT>(p.n_in, p.rows);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1712,12 +1732,12 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const bool stacked_idle = STACK && my_sub >= tps;
     const uint32_t lane_off = (uint32_t)(kTileRows * my_sub + g) * p.row_stride;
     if (!stacked_idle) {
-        planes += my_sub * plane_bytes<WT>(p.n_in, p.rows);
+        planes += my_sub * p.plane_bytes;
         chunk_sum += my_sub * chunk_sum_bytes<WT>(p.n_in, p.rows);
     }
     // single-row form: column g = limb g/2 of the low (g even) or high (g odd) chunk of a group
-    const int8_t *bq = planes + (g < 6 ? (g >> 1) * plane_stride(p.n_in) + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
-    const int8_t *sq = chunk_sum + (g & 3) * (p.n_in >> 5);
+    const int8_t *bq = planes + (g < 6 ? (g >> 1) * p.plane_pitch + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
+    const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in);
     BFrag held[2];
 
     // The same walk as walk() above, written flat: per stage a consumer warp only needs the ring
@@ -1787,7 +1807,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, p.n_in, p.n_in >> kSumShift<WT>, p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, p.plane_pitch, p.row_pitch, sum_pitch<WT>(p.n_in), p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -2107,7 +2127,10 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
-    const int fixed = align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows));
+    p.plane_pitch = plane_pitch<WT>(p.n_in, rows);
+    p.row_pitch = plane_row_pitch<WT>(p.n_in, rows);
+    p.plane_bytes = align_up(rows * p.row_pitch, 128);
+    const int fixed = align_up(smem_struct, 128) + p.tps * (p.plane_bytes + chunk_sum_bytes<WT>(p.n_in, rows));
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
     const bool halves = p.groups == 1;
@@ -2307,7 +2330,6 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
         p.n_entries++;
     }
     p.gran_begin[p.n_entries] = total;
-    p.total_gran = total;
     if (total == 0) return 1;
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
@@ -2341,7 +2363,6 @@ int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_
     }
     if (!tma && !setup_format<WT>(p, n_in, rows, silu_pair, &smem)) return 0;
     p.n_entries = 0;
-    p.total_gran = 0;
     p.gran_q = p.gran_r = 0;
     p.dev_table = table;
     p.table_rows = x_rows;
@@ -2363,7 +2384,6 @@ int launch_peers_fmt(const GemvMat &mat, int64_t n_in, int rows, const PeerScatt
     p.gran_begin[0] = 0;
     const int total = (int)((mat.n_out + p.gran - 1) / p.gran);
     p.gran_begin[1] = total;
-    p.total_gran = total;
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
     p.n_peers = ps.n_peers;
