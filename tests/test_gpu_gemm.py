@@ -178,3 +178,13 @@ def test_gemm_left_over_tiles_are_shared(cuda, oracle, wt):
     unequal length, clusters without a tile, a last weight tile of one row and outputs that float4 stores cannot describe."""
     for n_out, n_in, rows in ((19200, 2304, 40), (19201, 1280, 40), (11008, 1024, 300), (128 * 149, 2048, 256)):
         run_gemm(cuda, oracle, wt, n_out, n_in, rows, SEED + 140 + rows, check_rows=np.unique(np.r_[np.arange(0, n_out, 61), n_out - 1]))
+
+
+@pytest.mark.parametrize("rows,n_in", [(9, 256), (16, 4096), (17, 4096), (65, 1280), (257, 768), (2050, 1024)])
+def test_f32_activations_are_the_f16_ones(cuda, rows, n_in):
+    """The f16 copy of f32 activations, of one and of four quads a thread (more than 64 blocks of one), with and without a
+    remainder: the product is the same bits as that of activations converted before."""
+    import torch
+    w = torch.from_numpy(synth.weights(synth.Q4_K, 130, n_in, synth.BASE_SEED + 77, stream=3)).cuda()
+    x = torch.randn((rows, n_in), device="cuda", generator=torch.Generator("cuda").manual_seed(rows))
+    assert torch.equal(cuda.gemm(x, w, synth.Q4_K, 130, n_in), cuda.gemm(x.half(), w, synth.Q4_K, 130, n_in))
