@@ -105,7 +105,6 @@ struct StreamParams {
     int rows;             // activation rows
     int units;            // n_in / unit_values
     int n_in;
-    int plane_pitch;      // bytes from a limb plane of the prepared activation to the next, see plane_pitch()
     int gran_q, gran_r;   // granules in all = grid * gran_q + gran_r
     const StreamTable *dev_table;   // when set, the matrices come from device memory
     const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
@@ -118,8 +117,6 @@ struct StreamParams {
     GemvMat mat[KRK_CUDA_MAX_GROUP];
     int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
     int *status;
-    int row_pitch;        // bytes from an activation row's planes to the next row's
-    int plane_bytes;      // of all rows
     int entry_gran;       // table launches: granules of every entry (all have one shape)
     int groups;           // consumer groups of a CTA
     int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
@@ -297,21 +294,23 @@ __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / 
 template <int WT>
 __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
 // Where the planes lie, so that the eight columns of a B fragment (rows and limbs as lane_planes deals them) are read from
-// different banks. Q4_K and Q5_K load 8 bytes a lane, 32 a column: limbs lie 32 bytes on, rows 64 (modulo 128). The others load 4,
+// different banks. (Worked out on the device too: as parameters they cost the Q6_K head 2 %.) Q4_K and Q5_K load 8 bytes a lane, 32 a column: limbs lie 32 bytes on, rows 64 (modulo 128). The others load 4,
 // 16 a column: limbs 16 on; rows 32 in the folded form of the super-block formats, else next to each other. (The one-row form of
 // Q4_0 takes a limb in two columns; Q5_0 loses 3 % at eight rows with limbs 16 on.) Limbs 32 on in all and rows next to each
 // other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows 33.9 -> 32.1 us, Q6_K at four 32.9 -> 31.2, Q5_K at
 // four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.6.
 template <int WT>
-inline int plane_pitch(int n_in, int rows) {
+__host__ __device__ inline int plane_pitch(int n_in, int rows) {
     const bool wide = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1);
     return align_up(n_in, 128) + (wide ? 32 : 16);
 }
 template <int WT>
-inline int plane_row_pitch(int n_in, int rows) {
+__host__ __device__ inline int plane_row_pitch(int n_in, int rows) {
     const int planes = (fine_limbs<WT>(n_in) ? 4 : 3) * plane_pitch<WT>(n_in, rows);
     return planes + (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K ? 96 : block_size(WT) == 256 && rows > 2 ? 112 : 0);
 }
+template <int WT>
+__host__ __device__ inline int plane_bytes(int n_in, int rows) { return align_up(rows * plane_row_pitch<WT>(n_in, rows), 128); }
 // Sums of the quantised activation over the stretch of K that shares one minimum or offset: 32 values (2^5) for
 // Q4_K, Q5_K, Q4_0 and Q5_1, 16 for Q2_K.
 template <int WT>
@@ -571,7 +570,7 @@ template <int WT, bool FINE, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
-    const int n_chunks = sum_pitch<WT>(p.n_in), ps = p.plane_pitch, units = p.units;
+    const int n_chunks = sum_pitch<WT>(p.n_in), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
     // (where a warp has no such slice, or a lane no such value, it reads another of its own: the maximum is none the worse)
@@ -624,7 +623,7 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
             inv = 0.0f;
             s = __int_as_float(0x7FC00000);
         }
-        int8_t *p0 = planes + (size_t)r * p.row_pitch, *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
+        int8_t *p0 = planes + (size_t)r * plane_row_pitch<WT>(p.n_in, p.rows), *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
         auto quantize = [&](const float (&f)[PER], int u) {
             if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
             else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
@@ -1497,7 +1496,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     int8_t *planes = reinterpret_cast<int8_t *>(smem_raw + align_up((int)sizeof(SmemT), 128));
     // one copy of the prepared activation per stacked sub-tile: the warps of a sub-tile move on to the next
     // matrix (and its activation) on their own, so they must not share planes with another sub-tile
-    int8_t *chunk_sum = planes + tps * p.plane_bytes;
+    int8_t *chunk_sum = planes + tps * plane_bytes<WT>(p.n_in, p.rows);
     uint8_t *stages = reinterpret_cast<uint8_t *>(chunk_sum) + tps * chunk_sum_bytes<WT>(p.n_in, p.rows);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1732,11 +1731,11 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const bool stacked_idle = STACK && my_sub >= tps;
     const uint32_t lane_off = (uint32_t)(kTileRows * my_sub + g) * p.row_stride;
     if (!stacked_idle) {
-        planes += my_sub * p.plane_bytes;
+        planes += my_sub * plane_bytes<WT>(p.n_in, p.rows);
         chunk_sum += my_sub * chunk_sum_bytes<WT>(p.n_in, p.rows);
     }
     // single-row form: column g = limb g/2 of the low (g even) or high (g odd) chunk of a group
-    const int8_t *bq = planes + (g < 6 ? (g >> 1) * p.plane_pitch + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
+    const int8_t *bq = planes + (g < 6 ? (g >> 1) * plane_pitch<WT>(p.n_in, p.rows) + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
     const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in);
     BFrag held[2];
 
@@ -1807,7 +1806,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, p.plane_pitch, p.row_pitch, sum_pitch<WT>(p.n_in), p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, plane_pitch<WT>(p.n_in, p.rows), plane_row_pitch<WT>(p.n_in, p.rows), sum_pitch<WT>(p.n_in), p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -2127,10 +2126,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
-    p.plane_pitch = plane_pitch<WT>(p.n_in, rows);
-    p.row_pitch = plane_row_pitch<WT>(p.n_in, rows);
-    p.plane_bytes = align_up(rows * p.row_pitch, 128);
-    const int fixed = align_up(smem_struct, 128) + p.tps * (p.plane_bytes + chunk_sum_bytes<WT>(p.n_in, rows));
+    const int fixed = align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows));
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
     const bool halves = p.groups == 1;
