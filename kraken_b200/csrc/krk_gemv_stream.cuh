@@ -294,37 +294,45 @@ __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / 
 template <int WT>
 __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
 // Where the planes lie, so that the eight columns of a B fragment (rows and limbs as lane_planes deals them) are read from
-// different banks. (Worked out on the device too: as parameters they cost the Q6_K head 2 %.) Q4_K and Q5_K load 8 bytes a lane, 32 a column: limbs lie 32 bytes on, rows 64 (modulo 128). The others load 4,
-// 16 a column: limbs 16 on; rows 32 in the folded form of the super-block formats, else next to each other. (The one-row form of
-// Q4_0 takes a limb in two columns; Q5_0 loses 3 % at eight rows with limbs 16 on.) Limbs 32 on in all and rows next to each
-// other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows 33.9 -> 32.1 us, Q6_K at four 32.9 -> 31.2, Q5_K at
-// four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.6.
+// different banks, in no more room than next to each other at n_in + 32. (Worked out on the device too: as parameters they cost
+// the Q6_K head 2 %.) Most formats load 4 bytes a lane, 16 a column: planes lie an odd multiple of 16 bytes apart, rows of the
+// super-block formats 96 (modulo 128). Q4_K and Q5_K load 8, 32 a column: planes lie 32 on (modulo 128), and limbs 0 and 1 of all rows
+// before all limbs 2, so that rows lie 64 on. (The one-row form of Q4_0 takes a limb in two columns; Q5_0 loses 3 % at eight rows
+// with limbs 16 on.) All 32 on and rows next to each other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows
+// 33.9 -> 31.2 us, Q6_K at four 32.9 -> 30.4, Q5_K at four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.4.
+template <int WT>
+constexpr bool kWidePlanes = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K;
 template <int WT>
 __host__ __device__ inline int plane_pitch(int n_in, int rows) {
-    const bool wide = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1);
-    return align_up(n_in, 128) + (wide ? 32 : 16);
+    return n_in + (kWidePlanes<WT> || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1) ? 32 : 16);
+}
+// Byte offset of a limb plane of activation row r of `rows`.
+template <int WT>
+__host__ __device__ inline int plane_at(int n_in, int rows, int r, int limb) {
+    const int pitch = plane_pitch<WT>(n_in, rows);
+    if (kWidePlanes<WT>) return (limb < 2 ? 2 * r + limb : 2 * rows + r) * pitch;
+    return r * ((fine_limbs<WT>(n_in) ? 4 : 3) * pitch + (block_size(WT) == 256 ? 48 : 0)) + limb * pitch;
 }
 template <int WT>
-__host__ __device__ inline int plane_row_pitch(int n_in, int rows) {
-    const int planes = (fine_limbs<WT>(n_in) ? 4 : 3) * plane_pitch<WT>(n_in, rows);
-    return planes + (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K ? 96 : block_size(WT) == 256 && rows > 2 ? 112 : 0);
+__host__ __device__ inline int plane_bytes(int n_in, int rows) {
+    return align_up(kWidePlanes<WT> ? 3 * rows * plane_pitch<WT>(n_in, rows) : plane_at<WT>(n_in, rows, rows, 0), 128);
 }
-template <int WT>
-__host__ __device__ inline int plane_bytes(int n_in, int rows) { return align_up(rows * plane_row_pitch<WT>(n_in, rows), 128); }
 // Sums of the quantised activation over the stretch of K that shares one minimum or offset: 32 values (2^5) for
 // Q4_K, Q5_K, Q4_0 and Q5_1, 16 for Q2_K.
 template <int WT>
 constexpr int kSumShift = WT == KRK_CUDA_Q2_K ? 4 : 5;
-// Elements from a plane of sums to the next: signed-byte limbs (four planes a row, 16 bytes apart modulo 128: eight columns are
-// read at a time), or one plane of floats a row (Q4_0, Q5_1).
+// Elements from a plane of sums to the next: signed-byte limbs (four planes a row; eight columns are read at a time, 8 bytes each,
+// or 16 for Q2_K, so the pitch is an odd multiple of that where shared memory is not short), or one plane of floats a row (Q4_0,
+// Q5_1).
 template <int WT>
-__host__ __device__ inline int sum_pitch(int n_in) {
-    return WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K ? align_up(n_in >> kSumShift<WT>, 128) + 16 : n_in >> 5;
+__host__ __device__ inline int sum_pitch(int n_in, int rows) {
+    const int runs = (n_in >> 8) | (rows * n_in <= 40960 ? 1 : 0);
+    return kWidePlanes<WT> ? 8 * runs : WT == KRK_CUDA_Q2_K ? 16 * runs : n_in >> 5;
 }
 template <int WT>
 __host__ __device__ inline int chunk_sum_bytes(int n_in, int rows) {   // four planes of bytes or one of floats
     return (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_Q5_1 || WT == KRK_CUDA_Q2_K)
-               ? align_up(rows * 4 * sum_pitch<WT>(n_in), 128) : 0;
+               ? align_up(rows * 4 * sum_pitch<WT>(n_in, rows), 128) : 0;
 }
 
 // ---- the walk over this CTA's stages: identical in the producer and in the consumers -------------
@@ -570,7 +578,7 @@ template <int WT, bool FINE, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
-    const int n_chunks = sum_pitch<WT>(p.n_in), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
+    const int n_chunks = sum_pitch<WT>(p.n_in, p.rows), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
     // (where a warp has no such slice, or a lane no such value, it reads another of its own: the maximum is none the worse)
@@ -623,10 +631,10 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
             inv = 0.0f;
             s = __int_as_float(0x7FC00000);
         }
-        int8_t *p0 = planes + (size_t)r * plane_row_pitch<WT>(p.n_in, p.rows), *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
+        int8_t *p0 = planes + plane_at<WT>(p.n_in, p.rows, r, 0), *p2 = planes + plane_at<WT>(p.n_in, p.rows, r, 2), *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
         auto quantize = [&](const float (&f)[PER], int u) {
             if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
-            else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p0 + 2 * ps, sums, n_chunks, lane);
+            else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p2, sums, n_chunks, lane);
         };
 #pragma unroll
         for (int j = 0; j < kHeld; j++) {
@@ -768,8 +776,8 @@ __device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
 // Byte planes this lane reads its B fragments from, one per column group. A lane whose column
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
 // accumulator columns are never looked at, so what it multiplies does not matter.
-template <int NG, bool FOLD, bool FINE>
-__device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int plane_pitch, int row_pitch, int n_sums, int rows, int g,
+template <int WT, int NG, bool FOLD, bool FINE>
+__device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int n_in, int n_sums, int rows, int g,
                                             const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
@@ -788,7 +796,7 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
             r = g;
             limb = mg % 3;
         }
-        bp[mg] = planes + (size_t)min(r, rows - 1) * row_pitch + limb * plane_pitch;
+        bp[mg] = planes + plane_at<WT>(n_in, rows, min(r, rows - 1), limb);
         sp[mg] = chunk_sum + (size_t)(min(rs, rows - 1) * 4 + ls) * n_sums;
     }
 }
@@ -1508,9 +1516,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     volatile int *gave_up = &sm->gave_up;
     // Parameters arrive cold in every launch, and a miss holds its warp for some 700 clocks, one line after the other:
-    // warps 1..8 fetch a 64-byte line each, side by side (the scalars and the first seven entries). Q4_K 4096 x 4096
-    // 5.09 -> 4.95 us in a chain of launches, 1536 x 1536 3.37 -> 3.25. Only the single-row forms: the others have the
-    // longer start anyway and gain nothing (Q6_K 5.22 -> 5.18, Q8_0 5.94 -> 6.03, Q3_K 5.49 -> 5.65).
+    // warps 1..8 fetch a 64-byte line each, side by side (the scalars and the first entries). Q4_K 4096 x 4096 4.61 -> 4.55 us
+    // in a chain of launches. Only the single-row forms: the others have the longer start anyway and gain nothing.
     static_assert(kGroups * kConsumerWarps >= 8 && sizeof(StreamParams) >= 8 * 64, "a warp for each of eight lines");
     if (SINGLE && warp >= 1 && warp <= 8 && lane == 0)
         sm->touched[warp] = reinterpret_cast<const int *>(&p)[16 * (warp - 1)];
@@ -1736,7 +1743,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     }
     // single-row form: column g = limb g/2 of the low (g even) or high (g odd) chunk of a group
     const int8_t *bq = planes + (g < 6 ? (g >> 1) * plane_pitch<WT>(p.n_in, p.rows) + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
-    const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in);
+    const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in, p.rows);
     BFrag held[2];
 
     // The same walk as walk() above, written flat: per stage a consumer warp only needs the ring
@@ -1806,7 +1813,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<NG, kFold, kFine>(planes, chunk_sum, plane_pitch<WT>(p.n_in, p.rows), plane_row_pitch<WT>(p.n_in, p.rows), sum_pitch<WT>(p.n_in), p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<WT, NG, kFold, kFine>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.rows), p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -2134,7 +2141,9 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     if (max_fit < 3) max_fit = (kSmemWhole - fixed) / p.stage_bytes;
     const int most = halves ? kMaxHalfStages : kMaxStages;
     p.n_stages = max_fit < most ? max_fit : most;
-    if (p.n_stages < 2) return false;
+    // (a shape is taken if it would be with limb planes of n_in + 32 bytes: beyond, the warp-per-row kernel multiplies in f32)
+    const int spread = align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
+    if (p.n_stages < 2 || kSmemWhole - fixed - p.tps * spread < 2 * p.stage_bytes) return false;
     // Two groups that take tiles in turn want a ring that holds a tile of each: a stage of the second tile only lands when one of
     // the first is done with. Where it does not, they take a tile's stages in turn (Q6_K 4096 x 11008 at four rows, six stages to
     // a tile and a ring of three: 25.8 -> 24.4 us; three stages to a tile leave one group twice the other's: 14.9 -> 15.3). Only in
