@@ -1474,9 +1474,10 @@ template <int WT>
 constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_size(WT) == 32;
 template <int WT>
 constexpr bool kMayRag = kRagForm<WT> || WT == KRK_CUDA_Q2_K;
-// Forms whose two groups may take a tile's stages in turn (StreamParams::by_stage).
+// Forms whose two groups may take a tile's stages in turn (StreamParams::by_stage): ragged Q6_K. (Q3_K 4096 x 8960 at four rows
+// 19.1 -> 20.0 us with it.)
 template <int WT>
-__host__ __device__ constexpr bool may_by_stage(bool ragged, int groups) { return kRagForm<WT> && block_size(WT) == 256 && ragged && groups == 2; }
+__host__ __device__ constexpr bool may_by_stage(bool ragged, int groups) { return WT == KRK_CUDA_Q6_K && ragged && groups == 2; }
 // One result in f32 throughout, by one lane: what an infinity among the activations makes of a row (an infinity of either
 // sign, or a NaN against a zero weight) is not in the limbs, which give a NaN.
 template <int WT>
@@ -2058,6 +2059,20 @@ int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     return KRK_CUDA_OK;
 }
 
+// StreamParams::by_stage. Two groups that take tiles in turn want a ring that holds a tile of each: a stage of the second tile only
+// lands when one of the first is done with. Where it does not, they take a tile's stages in turn (Q6_K at four rows, stages to a
+// tile and in the ring: 16384 x 6656, 4 and 4, 39.8 -> 37.9 us; x 8960, 5 and 3, 51.6 -> 50.1; x 11008, 6 and 3, 62.3 -> 58.0;
+// three rows of x 14592, 8 and 3, 83.2 -> 75.6). Not of three stages, which leave one group twice the other's (14.9 -> 15.3), and
+// not in a ring of two, where each group holds one stage and none is on its way (four rows of 4096 x 12544 29.1 -> 31.2, six of
+// 16384 x 8960 69.3 -> 71.8), unless no CTA has a second tile, so that one group would have nothing to do (five rows of
+// 1024 x 10496 20.1 -> 18.7, eight of x 6656 16.6 -> 15.6). Only in the forms for ragged rows: the others would lose 2 to 4 % to the
+// code and gain nothing (Q4_K 4096 x 11008 17.5 -> 18.7 us).
+template <int WT>
+bool stages_in_turn(const StreamParams &p, bool one_tile) {
+    const int tile_stages = (p.units + kConsumerWarps - 1) / kConsumerWarps;
+    return may_by_stage<WT>(p.ragged != 0, p.groups) && tile_stages > 3 && p.n_stages < 2 * tile_stages && (p.n_stages >= 3 || one_tile);
+}
+
 // Fills the fields that depend only on the format, the width and the activation row count.
 // Returns false when the streaming kernel does not address the shape.
 template <int WT>
@@ -2144,13 +2159,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     // (a shape is taken if it would be with limb planes of n_in + 32 bytes: beyond, the warp-per-row kernel multiplies in f32)
     const int spread = align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
     if (p.n_stages < 2 || kSmemWhole - fixed - p.tps * spread < 2 * p.stage_bytes) return false;
-    // Two groups that take tiles in turn want a ring that holds a tile of each: a stage of the second tile only lands when one of
-    // the first is done with. Where it does not, they take a tile's stages in turn (Q6_K 4096 x 11008 at four rows, six stages to
-    // a tile and a ring of three: 25.8 -> 24.4 us; three stages to a tile leave one group twice the other's: 14.9 -> 15.3). Only in
-    // the forms for ragged rows of the super-block formats, which such rows mostly are: the others would lose 2 to 4 % to the code
-    // and gain nothing (Q4_K 4096 x 11008 17.5 -> 18.7 us).
-    p.by_stage = may_by_stage<WT>(p.ragged != 0, p.groups) && p.units > 3 * kConsumerWarps &&
-                 p.n_stages < 2 * ((p.units + kConsumerWarps - 1) / kConsumerWarps);
+    p.by_stage = stages_in_turn<WT>(p, false);
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
     return true;
 }
@@ -2342,6 +2351,7 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     // cost a whole tile of MMAs), and the other half of the SM lets the next launch start early (Q8_0 2048x2048 3.92 ->
     // 3.42 us, Q6_K 2048x6656 10.5 -> 8.1 us).
     const int per_sm = tiles <= sm_count() ? 1 : ctas_per_sm<WT>(smem, p.groups);
+    if (tiles <= sm_count()) p.by_stage = stages_in_turn<WT>(p, true);
     const int sms = sm_count() * per_sm;
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
