@@ -553,14 +553,16 @@ __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::un
     }
 }
 
+// N values of x, or zeros. Predicated, not branched around (arrays that are filled in branches were spilled, 130 bytes and more a
+// thread) and not read from elsewhere instead (that is as much traffic as the real thing). And in this order, all before their
+// first use: left to itself the compiler put some behind the others' arithmetic, a round trip to level 2 more.
 template <int N>
-__device__ __forceinline__ void load_values(const float *__restrict__ x, float (&f)[N]) {
+__device__ __forceinline__ void load_values(const float *__restrict__ x, float (&f)[N], bool there) {
 #pragma unroll
-    for (int j = 0; j < N; j += 4) {
-        // (in this order, all before their first use: left to itself the compiler put some behind the others' arithmetic, a round trip
-        // to level 2 more: Q4_K 4096 x 4096 at four rows 8.55 against 7.79 us)
-        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[j]), "=f"(f[j + 1]), "=f"(f[j + 2]), "=f"(f[j + 3]) : "l"(x + j) : "memory");
-    }
+    for (int j = 0; j < N; j += 4)
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n mov.f32 %2, 0f00000000;\n"
+                     " mov.f32 %3, 0f00000000;\n @p ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+                     : "=&f"(f[j]), "=&f"(f[j + 1]), "=&f"(f[j + 2]), "=&f"(f[j + 3]) : "l"(x + j), "r"((uint32_t)there) : "memory");
 }
 // max(mx, |f|), a NaN if there is one
 template <int N>
@@ -569,27 +571,29 @@ __device__ __forceinline__ void max_abs(float &mx, const float (&f)[N]) {
     for (int j = 0; j < N; j += 2) asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(f[j]), "f"(f[j + 1]));
 }
 
+// Forms that load the next activation row before they quantise one. The others have no registers for it: spilled, they read local
+// memory that misses level 1 in every launch (five to eight rows of 2048 to 6656 values 5 to 16 % longer), or their loop over the
+// tiles came out slower (ragged Q6_K 16384 x 11008 at one row 50.5 us without, 54.2 with it; the other way round Q5_1 16384 x 14336
+// 78.4 and 75.3, Q6_K 16384 x 4096 15.5 and 15.0, Q8_0 1024 x 2304 at three rows 6.0 and 5.5).
+template <int WT, int NG, bool RAG>
+constexpr bool kLoadsAhead = NG == 1 ? WT == KRK_CUDA_Q5_1 || ((WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K) && !RAG) : NG == 2 && WT == KRK_CUDA_Q8_0;
 // All slices that a warp will read of activation rows r0, r0 + step, ... < rows (row(r) is where row r lies); scale(r, s) gets
 // the row's scale for this warp. FINE: four limbs, and the last unit may hold fewer values than a full one.
 // Every CTA prepares all of x, so this is bound by issue slots and by the latency of x: a maximum takes half an instruction a
 // value, a row's loads go out together (kHeld slices stay in registers between the maximum and the quantisation, K <= 4096;
-// further ones are read twice, kBatch at a time for the maximum), and the next row's go out before a row is quantised.
-template <int WT, bool FINE, class RowFn, class ScaleFn>
+// further ones are read twice, kBatch at a time for the maximum).
+template <int WT, bool FINE, bool AHEAD, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
     const int n_chunks = sum_pitch<WT>(p.n_in, p.rows), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
-    // (where a warp has no such slice, or a lane no such value, it reads another of its own: the maximum is none the worse)
-    auto from = [&](int u) {
-        const int v = u < units ? u : wid;
-        return live(v) ? at(v) : v * UV;
-    };
-    float held[kHeld][PER], next[kHeld][PER];
-    auto load = [&](const float *xr, float (&f)[kHeld][PER]) {
+    auto load_slice = [&](const float *xr, int u, float (&f)[PER]) { load_values(xr + at(u), f, u < units && live(u)); };
+    float held[kHeld][PER], next[AHEAD ? kHeld : 1][PER];
+    auto load = [&](const float *xr, auto &f) {
 #pragma unroll
-        for (int j = 0; j < kHeld; j++) load_values(xr + from(wid + j * kConsumerWarps), f[j]);
+        for (int j = 0; j < kHeld; j++) load_slice(xr, wid + j * kConsumerWarps, f[j]);
     };
     if (r0 >= rows || wid >= units) return;
     const float *xr = row(r0);
@@ -601,14 +605,15 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         for (int u0 = wid + kHeld * kConsumerWarps; u0 < units; u0 += kBatch * kConsumerWarps) {
             float f[kBatch][PER];
 #pragma unroll
-            for (int j = 0; j < kBatch; j++) load_values(xr + from(u0 + j * kConsumerWarps), f[j]);
+            for (int j = 0; j < kBatch; j++) load_slice(xr, u0 + j * kConsumerWarps, f[j]);
 #pragma unroll
             for (int j = 0; j < kBatch; j++) max_abs(mx, f[j]);
         }
 #pragma unroll
         for (int j = 0; j < kHeld; j++) max_abs(mx, held[j]);
         const float *const xr1 = r + step < rows ? row(r + step) : xr;
-        if (r + step < rows) load(xr1, next);
+        if constexpr (AHEAD)
+            if (r + step < rows) load(xr1, next);
         // (bit patterns of magnitudes order like the values, infinities and NaNs above them)
         const uint32_t mxb = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(mx));
         // |x * inv| <= 2^22 over the whole f32 range: where the quotient would overflow, a power of two takes its place; a
@@ -644,10 +649,10 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         int u = wid + kHeld * kConsumerWarps;
         if (u < units) {
             float f[PER], g[PER];
-            load_values(xr + from(u), f);
+            load_slice(xr, u, f);
 #pragma unroll 1
             for (; u < units; u += kConsumerWarps) {
-                load_values(xr + from(u + kConsumerWarps), g);
+                load_slice(xr, u + kConsumerWarps, g);
                 quantize(f, u);
 #pragma unroll
                 for (int j = 0; j < PER; j++) f[j] = g[j];
@@ -655,10 +660,14 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         }
         scale(r, s);
         xr = xr1;
+        if constexpr (AHEAD) {
 #pragma unroll
-        for (int j = 0; j < kHeld; j++)
+            for (int j = 0; j < kHeld; j++)
 #pragma unroll
-            for (int i = 0; i < PER; i++) held[j][i] = next[j][i];
+                for (int i = 0; i < PER; i++) held[j][i] = next[j][i];
+        } else if (r + step < rows) {
+            load(xr, held);
+        }
     }
 }
 
@@ -1792,7 +1801,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             if (kGroups == 1) {
 #pragma unroll
                 for (int r = 0; r < 2 * NG; r++) xs[r] = 0.0f;
-                prepare_x<WT, kFine>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>>(row, [&](int r, float v) {
 #pragma unroll
                     for (int q = 0; q < 2 * NG; q++) xs[q] = q == r ? v : xs[q];
                 }, 0, 1, SINGLE ? 1 : p.rows, p, planes, chunk_sum, first_unit, lane);
@@ -1801,7 +1810,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             } else {
                 // each group prepares every other row; nobody may still read the activation before this one
                 if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
-                prepare_x<WT, kFine>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>>(row, [&](int r, float v) {
                     if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = v;
                 }, grp, kGroups, p.rows, p, planes, chunk_sum, first_unit, lane);
                 if (!synced) sync_start();
@@ -1812,6 +1821,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     xs[r] = row < p.rows ? sm->scale[NG == 1 ? 0 : wid][row] : 0.0f;
                 }
             }
+            // (zero already, but not held over the preparation, where registers are short: ragged Q6_K 4096 x 2304 at four rows 9 % less)
+            if (NG == 4 || (RAG && kSuper && kGroups == 2)) accum_zero(acc);
             prepared = x;
             prepared_row = my_row;
             if (!SINGLE) lane_planes<WT, NG, kFold, kFine>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.rows), p.rows, g, bp, sp);
