@@ -293,25 +293,27 @@ __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / 
 // (error against f64 of 2.3e-7 to 1.1e-6, f32: 1.2e-7), and the MMA's fourth column was unused.
 template <int WT>
 __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
-// Where the planes lie, so that the eight columns of a B fragment (rows and limbs as lane_planes deals them) are read from
-// different banks, in no more room than next to each other at n_in + 32. (Worked out on the device too: as parameters they cost
-// the Q6_K head 2 %.) Most formats load 4 bytes a lane, 16 a column: planes lie an odd multiple of 16 bytes apart, rows of the
-// super-block formats 96 (modulo 128). Q4_K and Q5_K load 8, 32 a column: planes lie 32 on (modulo 128), and limbs 0 and 1 of all rows
-// before all limbs 2, so that rows lie 64 on. (The one-row form of Q4_0 takes a limb in two columns; Q5_0 loses 3 % at eight rows
-// with limbs 16 on.) All 32 on and rows next to each other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows
-// 33.9 -> 31.2 us, Q6_K at four 32.9 -> 30.4, Q5_K at four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.4.
+// Where the planes lie, so that at up to four rows the eight columns of a B fragment (column_of) are read from different banks, in
+// no more room than next to each other at n_in + 32. (Worked out on the device too: as parameters they cost the Q6_K head 2 %.) Most
+// formats load 4 bytes a lane, 16 a column: planes lie an odd multiple of 16 bytes apart, rows of the super-block formats 96
+// (modulo 128) from three rows on. Q4_K and Q5_K load 8, 32 a column, four columns at a time: planes lie 32 on (modulo 128), and from
+// three rows on limbs 0 and 1 of all rows before all limbs 2, so that rows lie 64 on. (The one-row form of Q4_0 takes a limb in two
+// columns. Q5_0 loses 3 % at eight rows with limbs 16 on, and it and Q5_1 keep 32: two and more columns to a bank.) All 32 on and
+// rows next to each other were two- to four-fold conflicts: 32768 x 4096, Q4_K at eight rows 33.9 -> 31.2 us, Q6_K at four 32.9 -> 30.4, Q5_K
+// at four 26.4 -> 25.4; Q4_0 2080 x 5600 at four rows 12.1 -> 10.4. At five to eight rows the group of all limbs 2 (32-value
+// blocks: the columns of rows 6 and 7) still meets two columns to a bank.
 template <int WT>
 constexpr bool kWidePlanes = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K;
 template <int WT>
 __host__ __device__ inline int plane_pitch(int n_in, int rows) {
-    return n_in + (kWidePlanes<WT> || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1) ? 32 : 16);
+    return n_in + (kWidePlanes<WT> || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1 && !fine_limbs<WT>(n_in)) ? 32 : 16);
 }
 // Byte offset of a limb plane of activation row r of `rows`.
 template <int WT>
 __host__ __device__ inline int plane_at(int n_in, int rows, int r, int limb) {
     const int pitch = plane_pitch<WT>(n_in, rows);
-    if (kWidePlanes<WT>) return (limb < 2 ? 2 * r + limb : 2 * rows + r) * pitch;
-    return r * ((fine_limbs<WT>(n_in) ? 4 : 3) * pitch + (block_size(WT) == 256 ? 48 : 0)) + limb * pitch;
+    if (kWidePlanes<WT> && rows > 2) return (limb < 2 ? 2 * r + limb : 2 * rows + r) * pitch;
+    return r * ((fine_limbs<WT>(n_in) ? 4 : 3) * pitch + (block_size(WT) == 256 && !kWidePlanes<WT> && rows > 2 ? 48 : 0)) + limb * pitch;
 }
 template <int WT>
 __host__ __device__ inline int plane_bytes(int n_in, int rows) {
@@ -782,6 +784,29 @@ __device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
     return b;
 }
 
+// What column g of column group mg carries: a limb of an activation row, and of its chunk sums.
+struct Column {
+    int row, limb, sum_row, sum_limb;
+};
+template <int NG, bool FOLD, bool FINE>
+__host__ __device__ __forceinline__ Column column_of(int mg, int g) {
+    // (columns 6 and 7, which carry nothing, read what columns 4 and 5 do)
+    Column c{2 * mg + (g >= 6 ? 1 : g / 3), g >= 6 ? g - 5 : g % 3, 2 * mg + g / 4, g % 4};
+    if (FINE) {
+        c.row = 2 * mg + (g >> 2);
+        c.limb = g & 3;
+    } else if (FOLD) {   // see AccumFold
+        const bool last = mg >= kFoldGroups<NG> - 1;
+        c.row = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
+        c.limb = last ? 2 : g & 1;
+        c.sum_row = (g >> 1) + 4 * (mg >> 1);
+        c.sum_limb = 2 * (mg & 1) + (g & 1);
+    } else if (NG == 4 && g >= 6) {   // the spare columns: limb mg of activation row 6 or 7 (group 3 multiplies nothing)
+        c.row = g;
+        c.limb = mg % 3;
+    }
+    return c;
+}
 // Byte planes this lane reads its B fragments from, one per column group. A lane whose column
 // carries no limb (columns 6, 7, or an activation row past `rows`) reads some valid plane: its
 // accumulator columns are never looked at, so what it multiplies does not matter.
@@ -790,23 +815,9 @@ __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *
                                             const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
-        int r = 2 * mg + (g % 6) / 3, limb = g % 3;
-        int rs = 2 * mg + g / 4, ls = g % 4;   // chunk sums
-        if (FINE) {
-            r = 2 * mg + (g >> 2);
-            limb = g & 3;
-        } else if (FOLD) {   // see AccumFold
-            const bool last = mg >= kFoldGroups<NG> - 1;
-            r = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
-            limb = last ? 2 : g & 1;
-            rs = (g >> 1) + 4 * (mg >> 1);
-            ls = 2 * (mg & 1) + (g & 1);
-        } else if (NG == 4 && g >= 6) {   // the spare columns: limb mg of activation row 6 or 7 (group 3 multiplies nothing)
-            r = g;
-            limb = mg % 3;
-        }
-        bp[mg] = planes + plane_at<WT>(n_in, rows, min(r, rows - 1), limb);
-        sp[mg] = chunk_sum + (size_t)(min(rs, rows - 1) * 4 + ls) * n_sums;
+        const Column c = column_of<NG, FOLD, FINE>(mg, g);
+        bp[mg] = planes + plane_at<WT>(n_in, rows, min(c.row, rows - 1), c.limb);
+        sp[mg] = chunk_sum + (size_t)(min(c.sum_row, rows - 1) * 4 + c.sum_limb) * n_sums;
     }
 }
 

@@ -1,5 +1,7 @@
 // The decode GEMV's plan and shared-memory layout (setup_format and what it counts with), on the host: no device is needed.
+#include <algorithm>
 #include <cstdio>
+#include <vector>
 
 #include "krk_gemv_stream.cuh"
 
@@ -31,17 +33,84 @@ static void check_format() {
             }
 }
 
+// How often the fullest bank of shared memory is met when the columns of a B fragment are read: `bytes` a lane, four lanes a
+// column, 128 bytes at a time; equal addresses count once.
+template <int WT, int NG, bool FOLD, bool FINE>
+static int wavefronts(int n_in, int rows, int mg, int bytes) {
+    const int per_pass = 128 / (4 * bytes);
+    int worst = 0;
+    for (int g0 = 0; g0 < 8; g0 += per_pass) {
+        int words[32][8], count[32] = {};
+        for (int g = g0; g < g0 + per_pass; g++) {
+            const Column c = column_of<NG, FOLD, FINE>(mg, g);
+            const int at = plane_at<WT>(n_in, rows, c.row < rows ? c.row : rows - 1, c.limb);
+            for (int w = at / 4; w < at / 4 + bytes; w++) {
+                int i = 0;
+                while (i < count[w % 32] && words[w % 32][i] != w) i++;
+                if (i == count[w % 32]) words[w % 32][count[w % 32]++] = w;
+            }
+        }
+        for (int b = 0; b < 32; b++) worst = count[b] > worst ? count[b] : worst;
+    }
+    return worst;
+}
+
+template <int WT, int NG, bool FINE>
+static void check_banks(int n_in, int rows) {
+    constexpr bool kFold = block_size(WT) == 256 && NG > 1;
+    if (WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1) return;   // (32 bytes between planes, see plane_at)
+    for (int mg = 0; mg < (kFold ? kFoldGroups<NG> : kMmaGroups<NG, FINE>); mg++) {
+        const int n = wavefronts<WT, NG, kFold, FINE>(n_in, rows, mg, kWidePlanes<WT> ? 8 : 4);
+        check(n <= (rows <= 4 ? 1 : 2), "bank conflicts", WT, n_in, rows, mg, n);
+    }
+}
+
+template <int WT>
+static void check_planes() {
+    for (int rows = 1; rows <= KRK_CUDA_MAX_ROWS; rows++)
+        for (int n_in = 256; n_in <= 20480; n_in += block_size(WT)) {
+            const bool fine = fine_limbs<WT>(n_in);
+            // planes lie apart, 16-byte aligned (32 in the formats that load 8 bytes), inside their room, which is that of planes of n_in + 32
+            std::vector<int> at;
+            for (int r = 0; r < rows; r++)
+                for (int l = 0; l < (fine ? 4 : 3); l++) at.push_back(plane_at<WT>(n_in, rows, r, l));
+            std::sort(at.begin(), at.end());
+            for (size_t i = 0; i < at.size(); i++)
+                check(at[i] % 16 == 0 && at[i] >= 0 && at[i] + n_in <= (i + 1 < at.size() ? at[i + 1] : plane_bytes<WT>(n_in, rows)), "planes", WT, n_in,
+                      rows, (int)i, at[i]);
+            check(plane_bytes<WT>(n_in, rows) <= align_up((int)at.size() * (n_in + 32), 128), "planes' room", WT, n_in, rows, plane_bytes<WT>(n_in, rows), 0);
+            if constexpr (block_size(WT) == 32) {
+                if (fine && rows <= 2) check_banks<WT, 1, true>(n_in, rows);
+                else if (fine && rows <= 4) check_banks<WT, 2, true>(n_in, rows);
+                else if (fine) check_banks<WT, 4, true>(n_in, rows);
+            }
+            if (!fine && rows <= 2) check_banks<WT, 1, false>(n_in, rows);
+            else if (!fine && rows <= 4) check_banks<WT, 2, false>(n_in, rows);
+            else if (!fine) check_banks<WT, 4, false>(n_in, rows);
+        }
+}
+
 int main() {
     check_format<KRK_CUDA_Q4_0>();
+    check_planes<KRK_CUDA_Q4_0>();
     check_format<KRK_CUDA_Q5_0>();
+    check_planes<KRK_CUDA_Q5_0>();
     check_format<KRK_CUDA_Q5_1>();
+    check_planes<KRK_CUDA_Q5_1>();
     check_format<KRK_CUDA_Q8_0>();
+    check_planes<KRK_CUDA_Q8_0>();
     check_format<KRK_CUDA_IQ4_NL>();
+    check_planes<KRK_CUDA_IQ4_NL>();
     check_format<KRK_CUDA_Q2_K>();
+    check_planes<KRK_CUDA_Q2_K>();
     check_format<KRK_CUDA_Q3_K>();
+    check_planes<KRK_CUDA_Q3_K>();
     check_format<KRK_CUDA_Q4_K>();
+    check_planes<KRK_CUDA_Q4_K>();
     check_format<KRK_CUDA_Q5_K>();
+    check_planes<KRK_CUDA_Q5_K>();
     check_format<KRK_CUDA_Q6_K>();
+    check_planes<KRK_CUDA_Q6_K>();
     std::printf("%d of %d checks failed\n", bad, checked);
     return bad != 0;
 }
