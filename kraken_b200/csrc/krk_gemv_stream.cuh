@@ -108,7 +108,8 @@ struct StreamParams {
     int gran_q, gran_r;   // granules in all = grid * gran_q + gran_r
     const StreamTable *dev_table;   // when set, the matrices come from device memory
     const int32_t *table_rows;      // table launches: [entries][rows], see launch_gemv_stream_table
-    int gran;             // rows per granule: 1, or 8 when rows are not 16-byte multiples
+    short gran;           // rows per granule: 1, or 8 when rows are not 16-byte multiples
+    short spread_sums;    // 1: planes of chunk sums lie an odd multiple of their load apart, see sum_pitch
     int tps;              // 16-row tiles stacked in one stage (> 1 when a row has so few K units that one
                           // tile would leave most consumer warps idle: warp w takes unit w % units of
                           // sub-tile w / units)
@@ -324,17 +325,17 @@ __host__ __device__ inline int plane_bytes(int n_in, int rows) {
 template <int WT>
 constexpr int kSumShift = WT == KRK_CUDA_Q2_K ? 4 : 5;
 // Elements from a plane of sums to the next: signed-byte limbs (four planes a row; eight columns are read at a time, 8 bytes each,
-// or 16 for Q2_K, so the pitch is an odd multiple of that where shared memory is not short), or one plane of floats a row (Q4_0,
-// Q5_1).
+// or 16 for Q2_K, so the pitch is an odd multiple of that where the ring is none the smaller for it: spread, see setup_format), or
+// one plane of floats a row (Q4_0, Q5_1).
 template <int WT>
-__host__ __device__ inline int sum_pitch(int n_in, int rows) {
-    const int runs = (n_in >> 8) | (rows * n_in <= 40960 ? 1 : 0);
+__host__ __device__ inline int sum_pitch(int n_in, int spread) {
+    const int runs = (n_in >> 8) | spread;
     return kWidePlanes<WT> ? 8 * runs : WT == KRK_CUDA_Q2_K ? 16 * runs : n_in >> 5;
 }
 template <int WT>
-__host__ __device__ inline int chunk_sum_bytes(int n_in, int rows) {   // four planes of bytes or one of floats
+__host__ __device__ inline int chunk_sum_bytes(int n_in, int rows, int spread) {   // four planes of bytes or one of floats
     return (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_Q5_1 || WT == KRK_CUDA_Q2_K)
-               ? align_up(rows * 4 * sum_pitch<WT>(n_in, rows), 128) : 0;
+               ? align_up(rows * 4 * sum_pitch<WT>(n_in, spread), 128) : 0;
 }
 
 // ---- the walk over this CTA's stages: identical in the producer and in the consumers -------------
@@ -588,7 +589,7 @@ template <int WT, bool FINE, bool AHEAD, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
-    const int n_chunks = sum_pitch<WT>(p.n_in, p.rows), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
+    const int n_chunks = sum_pitch<WT>(p.n_in, p.spread_sums), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
     auto load_slice = [&](const float *xr, int u, float (&f)[PER]) { load_values(xr + at(u), f, u < units && live(u)); };
@@ -1526,7 +1527,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // one copy of the prepared activation per stacked sub-tile: the warps of a sub-tile move on to the next
     // matrix (and its activation) on their own, so they must not share planes with another sub-tile
     int8_t *chunk_sum = planes + tps * plane_bytes<WT>(p.n_in, p.rows);
-    uint8_t *stages = reinterpret_cast<uint8_t *>(chunk_sum) + tps * chunk_sum_bytes<WT>(p.n_in, p.rows);
+    uint8_t *stages = reinterpret_cast<uint8_t *>(chunk_sum) + tps * chunk_sum_bytes<WT>(p.n_in, p.rows, p.spread_sums);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n_warps = min(kConsumerWarps, p.units * tps);   // consumer warps that ever hold a unit
@@ -1760,11 +1761,11 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const uint32_t lane_off = (uint32_t)(kTileRows * my_sub + g) * p.row_stride;
     if (!stacked_idle) {
         planes += my_sub * plane_bytes<WT>(p.n_in, p.rows);
-        chunk_sum += my_sub * chunk_sum_bytes<WT>(p.n_in, p.rows);
+        chunk_sum += my_sub * chunk_sum_bytes<WT>(p.n_in, p.rows, p.spread_sums);
     }
     // single-row form: column g = limb g/2 of the low (g even) or high (g odd) chunk of a group
     const int8_t *bq = planes + (g < 6 ? (g >> 1) * plane_pitch<WT>(p.n_in, p.rows) + (WT == KRK_CUDA_Q4_0 ? 16 : 32) * (g & 1) : 0);
-    const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in, p.rows);
+    const int8_t *sq = chunk_sum + (g & 3) * sum_pitch<WT>(p.n_in, p.spread_sums);
     BFrag held[2];
 
     // The same walk as walk() above, written flat: per stage a consumer warp only needs the ring
@@ -1836,7 +1837,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             if (NG == 4 || (RAG && kSuper && kGroups == 2)) accum_zero(acc);
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<WT, NG, kFold, kFine>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.rows), p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<WT, NG, kFold, kFine>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.spread_sums), p.rows, g, bp, sp);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -2170,17 +2171,27 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
-    const int fixed = align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows));
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
     const bool halves = p.groups == 1;
-    int max_fit = halves ? (kSmemLimit - fixed) / p.stage_bytes : 0;
-    if (max_fit < 3) max_fit = (kSmemWhole - fixed) / p.stage_bytes;
     const int most = halves ? kMaxHalfStages : kMaxStages;
-    p.n_stages = max_fit < most ? max_fit : most;
+    auto fixed_bytes = [&](int spread) {
+        return align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows, spread));
+    };
+    auto depth = [&](int fixed, bool half) {
+        const int fit = ((half ? kSmemLimit : kSmemWhole) - fixed) / p.stage_bytes;
+        return fit < most ? fit : most;
+    };
+    auto fits_half = [&](int fixed) { return halves && depth(fixed, true) >= 3; };
+    // Chunk sums without bank conflicts take 128 bytes and more; a stage, or the half SM, is worth more than they are (Q2_K at five
+    // rows of 8192: 41.5 us with seven stages, 41.7 with six).
+    const int close = fixed_bytes(0), apart = fixed_bytes(1);
+    p.spread_sums = fits_half(apart) == fits_half(close) && depth(apart, fits_half(apart)) == depth(close, fits_half(close));
+    const int fixed = p.spread_sums ? apart : close;
+    p.n_stages = depth(fixed, fits_half(fixed));
     // (a shape is taken if it would be with limb planes of n_in + 32 bytes: beyond, the warp-per-row kernel multiplies in f32)
     const int spread = align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
-    if (p.n_stages < 2 || kSmemWhole - fixed - p.tps * spread < 2 * p.stage_bytes) return false;
+    if (p.n_stages < 2 || kSmemWhole - close - p.tps * spread < 2 * p.stage_bytes) return false;
     p.by_stage = stages_in_turn<WT>(p, false);
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
     return true;

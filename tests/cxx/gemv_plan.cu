@@ -25,6 +25,14 @@ static void check_format() {
                 if (!setup_format<WT>(p, n_in, rows, 0, &smem, tma != 0)) continue;
                 const int tile_stages = (p.units + kConsumerWarps - 1) / kConsumerWarps;
                 check(smem <= (size_t)kSmemWhole && p.n_stages >= 2, "room", WT, n_in, rows, (int)smem, p.n_stages);
+                // the ring is as deep, and as much of the SM left, as beside chunk sums that lie next to each other
+                const int held = (int)smem - p.n_stages * p.stage_bytes;
+                const int close = held - p.tps * (chunk_sum_bytes<WT>(p.n_in, rows, p.spread_sums) - chunk_sum_bytes<WT>(p.n_in, rows, 0));
+                int fit = p.groups == 1 ? (kSmemLimit - close) / p.stage_bytes : 0;
+                const bool half = fit >= 3;
+                if (!half) fit = (kSmemWhole - close) / p.stage_bytes;
+                const int most = p.groups == 1 ? kMaxHalfStages : kMaxStages;
+                check(p.n_stages == (fit < most ? fit : most) && (!half || smem <= (size_t)kSmemLimit), "ring", WT, n_in, rows, p.n_stages, fit);
                 // a tile's stages in turn: where the ring is short of two tiles, but a stage is on its way beside the two in use or
                 // there is one tile only
                 const bool short_ring = WT == KRK_CUDA_Q6_K && p.ragged && p.groups == 2 && tile_stages > 3 && p.n_stages < 2 * tile_stages;
