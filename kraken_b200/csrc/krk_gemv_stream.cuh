@@ -254,21 +254,21 @@ __device__ __forceinline__ float half_lo(uint32_t w) { return __half2float(__ush
 __device__ __forceinline__ float half_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
 
 // Bounded wait on an mbarrier phase. Once any wait in the CTA has given up, every later wait
-// returns at once, so the CTA runs to its end (on stale data, inside its own buffers) instead
-// of hanging.
+// returns after its first try (which the hardware bounds), so the CTA runs to its end (on stale data, inside its own buffers)
+// instead of hanging.
 // (Inline: around a call the kernels kept a frame of local memory, whose first accesses miss level 1 in every launch.)
 __device__ __forceinline__ uint32_t half_milliseconds() { return (uint32_t)(clock64() >> 20); }   // about
 __device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volatile int *gave_up, int *status) {
     if (mbar_try_wait(bar, parity)) return;
     const uint32_t t0 = half_milliseconds();
-    while (!mbar_try_wait(bar, parity)) {   // (the hardware suspends the warp for a while in each)
+    do {
         if (*gave_up) return;
         if (half_milliseconds() - t0 > kWaitHalfMs) {
             *gave_up = 1;
             atomicExch(status, KRK_CUDA_ETIMEOUT);
             return;
         }
-    }
+    } while (!mbar_try_wait(bar, parity));   // (the hardware suspends the warp for a while in each)
 }
 
 // ---- shared-memory map ---------------------------------------------------------------------------
