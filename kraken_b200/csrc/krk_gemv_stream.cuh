@@ -98,7 +98,8 @@ template <> struct Fmt<KRK_CUDA_IQ4_NL> { static constexpr int unit_values = 256
 template <> struct Fmt<KRK_CUDA_Q5_1> { static constexpr int unit_values = 256, unit_bytes = 192, stride_mod = 16, tma = 0; };
 
 // Parameters arrive cold in every launch, a 64-byte line at a time (some 700 clocks each): what every warp reads before its
-// first load stands in the first line, what a launch of one matrix needs besides in the second.
+// first load stands in the first line, the rest of what a launch of one matrix needs in the second, and the first matrices from
+// the fourth on.
 struct StreamParams {
     int n_entries;        // matrices, or gate/up pairs when silu_pair
     int step;             // matrices per entry (2 for gate/up pairs)
@@ -115,23 +116,23 @@ struct StreamParams {
                           // sub-tile w / units)
     int whole_tiles;      // 1: a stage is one contiguous copy of whole rows (unaligned row size)
     int n_stages;
-    GemvMat mat[KRK_CUDA_MAX_GROUP];
-    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
     int *status;
-    int entry_gran;       // table launches: granules of every entry (all have one shape)
-    int groups;           // consumer groups of a CTA
-    int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
-    int accumulate;
     int row_bytes;
-    int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
-                          // copied from the 16-byte boundary below its first byte, and its bytes sit that far
-                          // (0..15 bytes, a multiple of 2) into the row's slot
     int row_stride;       // bytes between rows inside a stage
     int unit_stride;      // bytes between the K units of one row group inside a stage
+    int stage_bytes;
     int use_tma;          // 1: a stage arrives as one tiled tensor copy, laid out [unit][row][unit_bytes]; 2: [row][units]
     int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this
     int box_bytes;        // bytes one tensor copy signals (the whole box, also where the matrix clips it)
-    int stage_bytes;
+    int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
+                          // copied from the 16-byte boundary below its first byte, and its bytes sit that far
+                          // (0..15 bytes, a multiple of 2) into the row's slot
+    int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
+    int accumulate;
+    int entry_gran;       // table launches: granules of every entry (all have one shape)
+    int groups;           // consumer groups of a CTA
+    int gran_begin[KRK_CUDA_MAX_GROUP + 1];   // first row granule of each entry
+    GemvMat mat[KRK_CUDA_MAX_GROUP];
     // Table launches with tensor copies: every matrix of the table lies inside one of two stacked banks (the gate
     // and the up bank of an expert set), each described by ONE tensor map (wmap[0], wmap[1]) over all of its
     // rows; a matrix is then a row offset into its bank.
@@ -146,6 +147,7 @@ struct StreamParams {
     // rows of a stage, units of a stage}
     CUtensorMap wmap[KRK_CUDA_MAX_GROUP];
 };
+static_assert(offsetof(StreamParams, status) == 64 && offsetof(StreamParams, gran_begin) == 120 && offsetof(StreamParams, mat) == 192, "the lines above");
 
 
 // ---- PTX wrappers ----------------------------------------------------------------------------
