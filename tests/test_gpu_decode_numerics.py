@@ -173,8 +173,8 @@ def test_rows_of_odd_block_counts_on_either_kernel(cuda, wt):
 @pytest.mark.parametrize("wt", FORMATS)
 @pytest.mark.parametrize("n_in", [2304, 4352, 6656, 11008, 12544])
 def test_rows_of_many_slices(cuda, oracle, wt, n_in):
-    """A warp prepares one to seven slices of every activation row (held, in one batch of loads, in a second), and two groups
-    of warps share a tile's stages where the ring does not hold two tiles. 22 bits of the largest activation of a warp's slices
+    """A warp prepares one to seven slices of every activation row (held, in one batch of loads, in a second; six of the widest rows go
+    to the warp-per-row kernel in most formats). 22 bits of the largest activation of a warp's slices
     (about four sigma here) leave 4 * 2^-22 / sqrt(12) a value, 2.8e-7 of the norms' product for a result; seven times that."""
     n_out = 80
     w = synth.weights(wt, n_out, n_in, SEED + 2, stream=wt)
@@ -186,3 +186,48 @@ def test_rows_of_many_slices(cuda, oracle, wt, n_in):
         x64 = x[:rows].astype(np.float64)
         lim = 2e-6 * np.linalg.norm(w64, axis=1)[None] * np.linalg.norm(x64, axis=1)[:, None]
         assert (np.abs(y.reshape(rows, n_out) - x64 @ w64.T) <= lim).all(), rows
+
+
+@pytest.mark.parametrize("n_in, n_out, row_counts", [(11008, 7201, (3, 4)), (6656, 7201, (4, 5, 6)), (8960, 4801, (3, 5)), (12544, 100, (4,)), (10496, 1000, (5,))])
+def test_stages_of_a_tile_in_turn(cuda, n_in, n_out, row_counts):
+    """Ragged Q6_K rows whose ring does not hold two tiles: both consumer groups multiply every tile, each through slots of its own
+    (two at three and four rows, one beyond), which a CTA's third and fourth tile meet again, an odd number of stages later too;
+    the last two shapes are one tile a CTA in a ring of two stages. The bound is that of test_rows_of_many_slices; silu has a slope
+    of 1.1 at most."""
+    import torch
+    wt = synth.Q6_K
+    w, other = (dev(synth.weights(wt, n_out, n_in, SEED + 8, stream=20 + i)) for i in range(2))
+    w64, other64 = (cuda.dequant_rows(m, wt, n_out, n_in).double() for m in (w, other))
+    be = cuda.Backend(0)
+    for rows in row_counts:
+        x = dev(synth.activations(rows, n_in, SEED + rows))
+        norms = x.double().norm(dim=1)[:, None]
+        want, lim = x.double() @ w64.T, 2e-6 * w64.norm(dim=1)[None] * norms
+        before = cuda.family_count(cuda.FAMILY_GEMV_STREAM)
+        first = cuda.gemv(x, w, wt, n_out, n_in)
+        assert cuda.family_count(cuda.FAMILY_GEMV_STREAM) == before + 1
+        assert ((first.double() - want).abs() <= lim).all(), rows
+        for _ in range(10):
+            cuda.gemv(x, other, wt, n_out, n_in)
+            assert torch.equal(cuda.gemv(x, w, wt, n_out, n_in), first)
+        base = torch.randn((rows, n_out), device="cuda")
+        got = cuda.gemv(x, w, wt, n_out, n_in, out=base.clone(), accumulate=True)
+        assert torch.equal(got, base + first)
+        # several matrices in one launch, and the gate/up fold
+        outs = [torch.empty((rows, n_out), device="cuda") for _ in range(3)]
+        torch.cuda.synchronize()
+        before = cuda.family_count(cuda.FAMILY_GEMV_STREAM)
+        ran, _ = be.gemm_group([o.data_ptr() for o in outs], x.data_ptr(), [m.data_ptr() for m in (w, other, w)], wt, [n_out] * 3, n_in, rows=rows)
+        torch.cuda.synchronize()
+        assert ran and cuda.family_count(cuda.FAMILY_GEMV_STREAM) == before + 1
+        up, up_lim = x.double() @ other64.T, 2e-6 * other64.norm(dim=1)[None] * norms
+        assert ((outs[0].double() - want).abs() <= lim).all() and torch.equal(outs[2], outs[0])
+        assert ((outs[1].double() - up).abs() <= up_lim).all()
+        ran, fused = be.gemm_group([o.data_ptr() for o in outs[:2]], x.data_ptr(), [m.data_ptr() for m in (w, other)], wt, [n_out] * 2, n_in, rows=rows,
+                                   silu=True)
+        torch.cuda.synchronize()
+        assert ran and fused
+        silu = want / (1.0 + torch.exp(-want))
+        assert ((outs[0].double() - silu * up).abs() <= 1.1 * lim * (up.abs() + up_lim) + silu.abs() * up_lim + 1e-6 * (silu * up).abs()).all()
+    be.close()
+    assert cuda.device_status() == 0

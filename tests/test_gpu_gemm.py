@@ -188,3 +188,15 @@ def test_f32_activations_are_the_f16_ones(cuda, rows, n_in):
     w = torch.from_numpy(synth.weights(synth.Q4_K, 130, n_in, synth.BASE_SEED + 77, stream=3)).cuda()
     x = torch.randn((rows, n_in), device="cuda", generator=torch.Generator("cuda").manual_seed(rows))
     assert torch.equal(cuda.gemm(x, w, synth.Q4_K, 130, n_in), cuda.gemm(x.half(), w, synth.Q4_K, 130, n_in))
+
+
+def test_f32_activations_of_several_laps(cuda):
+    """8.9 million values, where 1184 blocks of 4096 are a lap, and a remainder; finite values beyond the f16 range saturate."""
+    import torch
+    rows, n_in = 2049, 4352
+    w = torch.from_numpy(synth.weights(synth.Q4_K, 130, n_in, synth.BASE_SEED + 78, stream=3)).cuda()
+    x = torch.randn((rows, n_in), device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    x[::97, 11::501] = 1e5
+    x[5::97, 7::499] = -7e4
+    want = cuda.gemm(x.clamp(-65504.0, 65504.0).half(), w, synth.Q4_K, 130, n_in)
+    assert torch.isfinite(want).all() and torch.equal(cuda.gemm(x, w, synth.Q4_K, 130, n_in), want)
