@@ -1169,7 +1169,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUt
 }
 
 // A thread takes QUADS quads, a block's width apart and all in flight together. Four, where one each is more than 64 blocks: fewer
-// blocks leave more SMs to the GEMM's CTAs, which start beside them, and fit at a time (behind a product: Q6_K 4096 x 11008 at 37
+// blocks leave more SMs to the GEMM's CTAs, which start beside them, and fit at a time (passes back to back; alone it gives nothing: Q6_K 4096 x 11008 at 37
 // tokens 20.8 -> 19.1 us, Q8_0 4096 x 4096 at 64 tokens 12.4 -> 11.2, Q3_K 11008 x 4096 at 300 tokens 50.4 -> 48.3). Below, the
 // longer thread only takes longer (16 tokens of 4096 values 8.7 against 9.05).
 constexpr int kConvertThreads = 256, kConvertFewBlocks = 64;

@@ -426,13 +426,12 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
 }
 
 // ---- activation preparation -------------------------------------------------------------------------
-// Consumer warp w only ever multiplies K units w, w+16, ... so it prepares exactly those slices
-// of x itself: no other warp reads them and no CTA-wide barrier is involved. Per activation row:
-// s = max|x| / (127 * 2^16) over the warp's slices, X = rint(x / s) as three balanced s8 limbs
-// written as byte planes [row][limb][k] in the order the B fragments are read, and (Q4_K) the
-// integer sum of X over every 32-value chunk as four balanced s8 limbs [row][limb][chunk] for
-// the `min` term. s is returned (NaN when a slice holds a non-finite activation, so the output
-// becomes NaN as it would in f32) and multiplies the warp's partial sums at the end of each tile.
+// Consumer warp w only ever multiplies K units w, w + 8, ... so it (of two groups, the warp w of one of them: each prepares every
+// other activation row) prepares exactly those slices of x. Per activation row: s = max|x| / (2^22 - 1) over the warp's slices,
+// X = rint(x / s) as three balanced s8 limbs (four where K is not a multiple of 256) written as byte planes (plane_at) in the
+// order the B fragments are read, and (formats with a minimum or an offset) the integer sum of X over every stretch of K that shares
+// one, as four planes of s8 limbs or one of floats (sum_pitch). s is NaN when a slice holds a non-finite activation, so the output
+// becomes NaN as it would in f32; it multiplies the warp's partial sums at the end of each tile.
 
 __device__ __forceinline__ int sext8(int v) { return (v << 24) >> 24; }
 
@@ -1743,7 +1742,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     }
 
     // ===== consumer warps =====
-    const int grp = kGroups == 1 ? 0 : (warp - 1) / kConsumerWarps;   // consumer group: takes tiles grp, grp + 2, ...
+    const int grp = kGroups == 1 ? 0 : (warp - 1) / kConsumerWarps;   // consumer group: takes every other tile, or every other stage (by_stage)
     const int wid = warp - 1 - grp * kConsumerWarps, g = lane >> 2, t = lane & 3;
     const float *prepared = nullptr;
     int prepared_row = 0;
