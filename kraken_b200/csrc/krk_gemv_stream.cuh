@@ -518,7 +518,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
 }
 
 // The same where K is not a multiple of 256: four limbs, in value order everywhere (rows whose blocks start at any even
-// address, see ld_q6). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
+// address, see Words). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
 // `live`: the lane's values lie inside the row (the last unit of such a row may be short).
 template <int WT>
 __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p, int ps,
@@ -956,27 +956,36 @@ __device__ __forceinline__ void unit_q4_k_single(const uint8_t *rowA, const uint
     acc.m[3] = fmaf(nB, cm[3], acc.m[3]);
 }
 
-// 32-bit load at a 4-byte-multiple offset of a Q6_K block that itself starts 0 or 2 bytes off
-// a word boundary (blocks are 210 bytes, so odd blocks of a row are misaligned).
-// MODE 0: the block starts on a word boundary; 1: 2 bytes off; 2: either, found from the address (ragged rows:
-// the two rows of a lane may differ).
+// 32-bit words at constant even offsets of a block or row in shared memory. MODE 0: it starts on a word boundary; 1: 2 bytes off
+// (blocks of 210 and 110 bytes: every other one of a row); 2: either, found from the address (ragged rows: the two rows of a lane
+// may differ). There every word is glued from two aligned ones by a shift, and both are found once for all words of an offset's
+// parity: worked out per word, through an integer that hides from the compiler that the loads are from shared memory, they were
+// most of a unit (Q6_K 4096 x 11008 731 -> 555 instructions a unit, 17.4 -> 14.5 us; Q8_0 11200 x 2080 502 -> 386, 12.4 -> 10.9).
 template <int MODE>
-__device__ __forceinline__ uint32_t ld_q6(const uint8_t *blk, int off) {
-    if (MODE == 2) {
-        const uintptr_t a = reinterpret_cast<uintptr_t>(blk + off);
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-        return __funnelshift_r(w[0], w[1], (uint32_t)(a & 2) * 8u);
+struct Words {
+    const uint8_t *p0, *p2;   // offsets that are multiples of 4, and the others
+    uint32_t s0, s2;
+    __device__ __forceinline__ explicit Words(const uint8_t *at) : p0(at), p2(at), s0(0), s2(0) {
+        if (MODE == 2) {
+            const uint32_t by = smem_u32(at) & 2u;
+            p0 = at - by;
+            p2 = at + by - 2;
+            s0 = 8u * by;
+            s2 = 16u - s0;
+        }
     }
-    if (MODE == 1) {
-        const uint32_t lo = *reinterpret_cast<const uint32_t *>(blk + off - 2);
-        const uint32_t hi = *reinterpret_cast<const uint32_t *>(blk + off + 2);
-        return __byte_perm(lo, hi, 0x5432);
+    __device__ __forceinline__ uint32_t operator()(int off) const {
+        if (MODE == 2) {
+            const uint32_t *w = reinterpret_cast<const uint32_t *>((off & 2 ? p2 : p0) + off);
+            return __funnelshift_r(w[0], w[1], off & 2 ? s2 : s0);
+        }
+        if (MODE == 1) return __byte_perm(*reinterpret_cast<const uint32_t *>(p0 + off - 2), *reinterpret_cast<const uint32_t *>(p0 + off + 2), 0x5432);
+        return *reinterpret_cast<const uint32_t *>(p0 + off);
     }
-    return *reinterpret_cast<const uint32_t *>(blk + off);
-}
+};
 
 // The 32-value blocks of rows that start at any even address (K not a multiple of 256): every word is glued from two
-// aligned loads, the limbs lie in value order, and only the first `nb` blocks of a unit exist (the last unit of a row may be
+// aligned loads, the limbs lie in value order (see Words), and only the first `nb` blocks of a unit exist (the last unit of a row may be
 // short; what its slot holds past the row is never looked at).
 __device__ __forceinline__ float half_at(const uint8_t *p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(p))); }
 
@@ -1027,14 +1036,15 @@ __device__ __forceinline__ void unit_q4_0(const uint8_t *rowA, const uint8_t *ro
 template <int NG, bool RAG>
 __device__ __forceinline__ void unit_q4_0_rows(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                                int t, Accum<NG> &acc, int nb) {
+    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
         uint32_t qa, qb;
         float dA, dB;
         if (RAG) {
-            qa = ld_q6<2>(rowA + 18 * b, 2 + 4 * t);
-            qb = ld_q6<2>(rowB + 18 * b, 2 + 4 * t);
+            qa = wA(18 * b + 2);
+            qb = wB(18 * b + 2);
             dA = half_at(rowA + 18 * b);
             dB = half_at(rowB + 18 * b);
         } else if ((b & 1) == 0) {
@@ -1099,14 +1109,15 @@ __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *
         lo4 = prmt(r01, r23, 0x6420u);
         hi4 = prmt(r01, r23, 0x7531u);
     };
+    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
         uint32_t qa, qb;
         float dA, dB;
         if (RAG) {
-            qa = ld_q6<2>(rowA + 18 * b, 2 + 4 * t);
-            qb = ld_q6<2>(rowB + 18 * b, 2 + 4 * t);
+            qa = wA(18 * b + 2);
+            qb = wB(18 * b + 2);
             dA = half_at(rowA + 18 * b);
             dB = half_at(rowB + 18 * b);
         } else if ((b & 1) == 0) {
@@ -1155,16 +1166,17 @@ __device__ __forceinline__ uint32_t spread_top(uint32_t n) { return (n * 0x10204
 template <int NG, bool RAG>
 __device__ __forceinline__ void unit_q5_0(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, Accum<NG> &acc, int nb) {
+    const Words<RAG ? 2 : 0> wA(rowA), wB(rowB);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
         uint32_t qa, qb, ma, mb;
         float dA, dB;
         if (RAG) {
-            qa = ld_q6<2>(rowA + 22 * b, 6 + 4 * t);
-            qb = ld_q6<2>(rowB + 22 * b, 6 + 4 * t);
-            ma = ~ld_q6<2>(rowA + 22 * b, 2);
-            mb = ~ld_q6<2>(rowB + 22 * b, 2);
+            qa = wA(22 * b + 6 + 4 * t);
+            qb = wB(22 * b + 6 + 4 * t);
+            ma = ~wA(22 * b + 2);
+            mb = ~wB(22 * b + 2);
             dA = half_at(rowA + 22 * b);
             dB = half_at(rowB + 22 * b);
         } else if ((b & 1) == 0) {
@@ -1252,16 +1264,17 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
 template <int NG, bool RAG>
 __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, Accum<NG> &acc, int nb) {
+    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 4; b++) {
         if (RAG && b >= nb) break;
         uint32_t a0, a1, a2, a3;
         float dA, dB;
         if (RAG) {
-            a0 = ld_q6<2>(rowA + 34 * b, 2 + 4 * t);
-            a1 = ld_q6<2>(rowB + 34 * b, 2 + 4 * t);
-            a2 = ld_q6<2>(rowA + 34 * b, 18 + 4 * t);
-            a3 = ld_q6<2>(rowB + 34 * b, 18 + 4 * t);
+            a0 = wA(34 * b + 2);
+            a1 = wB(34 * b + 2);
+            a2 = wA(34 * b + 18);
+            a3 = wB(34 * b + 18);
             dA = half_at(rowA + 34 * b);
             dB = half_at(rowB + 34 * b);
         } else if ((b & 1) == 0) {
@@ -1307,6 +1320,7 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
 template <int NG, int ODD>
 __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, AccumSuper<NG> &acc) {
+    const Words<ODD> wA(blkA), wB(blkB);
     int I[NG][4];
 #pragma unroll
     for (int mg = 0; mg < kFoldGroups<NG>; mg++)
@@ -1317,15 +1331,15 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
         uint32_t qlA[4], qlB[4], qhA[2], qhB[2], scA[2], scB[2];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            qlA[i] = ld_q6<ODD>(blkA, 64 * h + 16 * i + 4 * t);
-            qlB[i] = ld_q6<ODD>(blkB, 64 * h + 16 * i + 4 * t);
+            qlA[i] = wA(64 * h + 16 * i + 4 * t);
+            qlB[i] = wB(64 * h + 16 * i + 4 * t);
         }
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            qhA[i] = ld_q6<ODD>(blkA, 128 + 32 * h + 16 * i + 4 * t) ^ 0xAAAAAAAAu;
-            qhB[i] = ld_q6<ODD>(blkB, 128 + 32 * h + 16 * i + 4 * t) ^ 0xAAAAAAAAu;
-            scA[i] = ld_q6<ODD>(blkA, 192 + 8 * h + 4 * i);
-            scB[i] = ld_q6<ODD>(blkB, 192 + 8 * h + 4 * i);
+            qhA[i] = wA(128 + 32 * h + 16 * i + 4 * t) ^ 0xAAAAAAAAu;
+            qhB[i] = wB(128 + 32 * h + 16 * i + 4 * t) ^ 0xAAAAAAAAu;
+            scA[i] = wA(192 + 8 * h + 4 * i);
+            scB[i] = wB(192 + 8 * h + 4 * i);
         }
         // group G = 2*quad + s covers values 16G..16G+15 of the half (src/quant.cpp:491-512):
         // low 4 bits from ql[32*(quad&1) + 16s ...] (high nibble when quad >= 2), bits 4-5 from
@@ -1419,10 +1433,11 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
 template <int NG, int MODE>
 __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, AccumSuper<NG> &acc) {
+    const Words<MODE> wA(blkA), wB(blkB);
     uint32_t SA[4], SB[4];
     {
-        const uint32_t a0 = ld_q6<MODE>(blkA, 96), a1 = ld_q6<MODE>(blkA, 100), a2 = ld_q6<MODE>(blkA, 104);
-        const uint32_t b0 = ld_q6<MODE>(blkB, 96), b1 = ld_q6<MODE>(blkB, 100), b2 = ld_q6<MODE>(blkB, 104);
+        const uint32_t a0 = wA(96), a1 = wA(100), a2 = wA(104);
+        const uint32_t b0 = wB(96), b1 = wB(100), b2 = wB(104);
         // scale i: low four bits in the nibbles of bytes 0..7, high two in byte 8 + i % 4 at bits 2 * (i / 4)
         SA[0] = (a0 & 0x0F0F0F0Fu) | ((a2 << 4) & 0x30303030u);
         SA[1] = (a1 & 0x0F0F0F0Fu) | ((a2 << 2) & 0x30303030u);
@@ -1438,8 +1453,8 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
             SB[k] = (SB[k] + 0x60606060u) ^ 0x80808080u;
         }
     }
-    const uint32_t hmA[2] = {~ld_q6<MODE>(blkA, 4 * t), ~ld_q6<MODE>(blkA, 16 + 4 * t)};
-    const uint32_t hmB[2] = {~ld_q6<MODE>(blkB, 4 * t), ~ld_q6<MODE>(blkB, 16 + 4 * t)};
+    const uint32_t hmA[2] = {~wA(4 * t), ~wA(16 + 4 * t)};
+    const uint32_t hmB[2] = {~wB(4 * t), ~wB(16 + 4 * t)};
     int I[NG][4];
 #pragma unroll
     for (int mg = 0; mg < kFoldGroups<NG>; mg++)
@@ -1447,8 +1462,8 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
         for (int j = 0; j < 4; j++) I[mg][j] = 0;
 #pragma unroll
     for (int n = 0; n < 2; n++) {
-        const uint32_t qA[2] = {ld_q6<MODE>(blkA, 32 + 32 * n + 4 * t), ld_q6<MODE>(blkA, 48 + 32 * n + 4 * t)};
-        const uint32_t qB[2] = {ld_q6<MODE>(blkB, 32 + 32 * n + 4 * t), ld_q6<MODE>(blkB, 48 + 32 * n + 4 * t)};
+        const uint32_t qA[2] = {wA(32 + 32 * n + 4 * t), wA(48 + 32 * n + 4 * t)};
+        const uint32_t qB[2] = {wB(32 + 32 * n + 4 * t), wB(48 + 32 * n + 4 * t)};
 #pragma unroll
         for (int js = 0; js < 8; js++) {
             const int j = js >> 1, s = js & 1, G = 8 * n + js, hb = 4 * n + j;
