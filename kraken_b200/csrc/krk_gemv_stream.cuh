@@ -78,10 +78,11 @@ template <int WT> struct Fmt;
 // tma: how a stage can arrive as ONE tiled tensor copy. 1: a unit is a whole number of 16-byte granules (Q4_K's
 // 144 bytes): box {unit bytes, rows, units}, laid out [unit][row][unit bytes]. 2: eight units of a row are (Q6_K:
 // 8 x 210 = 1680 bytes, as 210 64-bit elements): box {8 units, rows}, laid out [row][8 units], which is the
-// layout of the per-row copies with a 1680-byte pitch. 0: per-row bulk copies only.
+// layout of the per-row copies with a 1680-byte pitch. 3: a stage's part of a row is, but rows at that pitch would meet on the same
+// banks (see box_pitch): box {that and up to 16 bytes more, rows} over the row bytes as 64-bit elements.
 template <> struct Fmt<KRK_CUDA_Q4_K> { static constexpr int unit_values = 256, unit_bytes = 144, stride_mod = 32, tma = 1; };
 template <> struct Fmt<KRK_CUDA_Q6_K> { static constexpr int unit_values = 256, unit_bytes = 210, stride_mod = 16, tma = 2; };
-template <> struct Fmt<KRK_CUDA_Q8_0> { static constexpr int unit_values = 128, unit_bytes = 136, stride_mod = 16, tma = 0; };
+template <> struct Fmt<KRK_CUDA_Q8_0> { static constexpr int unit_values = 128, unit_bytes = 136, stride_mod = 16, tma = 3; };
 // Q5_K: Q4_K's header and nibbles with 32 bytes of fifth bits between them (src/quant.cpp:462-489).
 template <> struct Fmt<KRK_CUDA_Q5_K> { static constexpr int unit_values = 256, unit_bytes = 176, stride_mod = 32, tma = 1; };
 // Q4_0: eight 18-byte blocks are 144 bytes, the size of a Q4_K unit, so the stages are laid out the same way.
@@ -91,11 +92,11 @@ template <> struct Fmt<KRK_CUDA_Q4_0> { static constexpr int unit_values = 256, 
 // same banks, so its stages arrive as per-row copies with a padded pitch.
 template <> struct Fmt<KRK_CUDA_Q5_0> { static constexpr int unit_values = 256, unit_bytes = 176, stride_mod = 16, tma = 1; };
 // Q2_K (84 bytes) and Q3_K (110 bytes): per-row copies; rows that are not 16-byte multiples go the ragged way.
-template <> struct Fmt<KRK_CUDA_Q2_K> { static constexpr int unit_values = 256, unit_bytes = 84, stride_mod = 16, tma = 0; };
-template <> struct Fmt<KRK_CUDA_Q3_K> { static constexpr int unit_values = 256, unit_bytes = 110, stride_mod = 16, tma = 0; };
+template <> struct Fmt<KRK_CUDA_Q2_K> { static constexpr int unit_values = 256, unit_bytes = 84, stride_mod = 16, tma = 3; };
+template <> struct Fmt<KRK_CUDA_Q3_K> { static constexpr int unit_values = 256, unit_bytes = 110, stride_mod = 16, tma = 3; };
 // IQ4_NL: Q4_0's block with grid indices in place of quants.
 template <> struct Fmt<KRK_CUDA_IQ4_NL> { static constexpr int unit_values = 256, unit_bytes = 144, stride_mod = 16, tma = 1; };
-template <> struct Fmt<KRK_CUDA_Q5_1> { static constexpr int unit_values = 256, unit_bytes = 192, stride_mod = 16, tma = 0; };
+template <> struct Fmt<KRK_CUDA_Q5_1> { static constexpr int unit_values = 256, unit_bytes = 192, stride_mod = 16, tma = 3; };
 
 // Parameters arrive cold in every launch, a 64-byte line at a time (some 700 clocks each): what every warp reads before its
 // first load stands in the first line, the rest of what a launch of one matrix needs in the second, and the first matrices from
@@ -121,8 +122,9 @@ struct StreamParams {
     int row_stride;       // bytes between rows inside a stage
     int unit_stride;      // bytes between the K units of one row group inside a stage
     int stage_bytes;
-    int use_tma;          // 1: a stage arrives as one tiled tensor copy, laid out [unit][row][unit_bytes]; 2: [row][units]
-    int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this
+    int use_tma;          // 1: a stage arrives as one tiled tensor copy, laid out [unit][row][unit_bytes]; 2, 3: [row][units]
+    int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this (use_tma == 3: 0, and its first coordinate
+                          // the unit's place in the row in 64-bit elements)
     int box_bytes;        // bytes one tensor copy signals (the whole box, also where the matrix clips it)
     int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
                           // copied from the 16-byte boundary below its first byte, and its bytes sit that far
@@ -178,10 +180,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// One tiled tensor copy global -> shared (no multicast): box origin (0, row, unit).
-__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int row, int unit, uint32_t bar) {
+// One tiled tensor copy global -> shared (no multicast): box origin (at, row, unit).
+__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int at, int row, int unit, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(unit), "r"(bar) : "memory");
+                 ::"r"(dst), "l"(map), "r"(at), "r"(row), "r"(unit), "r"(bar) : "memory");
 }
 // c = A x B with a zero accumulator input (the sub-block scale is applied to c afterwards).
 __device__ __forceinline__ void mma_s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -1593,9 +1595,11 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         // (a 64-bit division per stage, by the one lane that issues a copy per stage)
                         const int bank = s.mat % p.step;
                         const int row_off = (int)((size_t)(tv.w(s.mat) - p.bank_base[bank]) / (size_t)p.row_bytes);
-                        tma_box(smem_u32(dst), &p.wmap[bank], row_off + s.row0, s.unit0 / p.tma_unit_div, full);
+                        if constexpr (F::tma == 3) tma_box(smem_u32(dst), &p.wmap[bank], s.unit0 * F::unit_bytes / 8, row_off + s.row0, 0, full);
+                        else tma_box(smem_u32(dst), &p.wmap[bank], 0, row_off + s.row0, s.unit0 / p.tma_unit_div, full);
                     } else {
-                        tma_box(smem_u32(dst), &p.wmap[s.mat], s.row0, s.unit0 / p.tma_unit_div, full);
+                        if constexpr (F::tma == 3) tma_box(smem_u32(dst), &p.wmap[s.mat], s.unit0 * F::unit_bytes / 8, s.row0, 0, full);
+                        else tma_box(smem_u32(dst), &p.wmap[s.mat], 0, s.row0, s.unit0 / p.tma_unit_div, full);
                     }
                 }
             } else if (kMayRag<WT> && p.ragged) {
@@ -2112,6 +2116,13 @@ bool stages_in_turn(const StreamParams &p, bool one_tile) {
     return may_by_stage<WT>(p.ragged != 0, p.groups) && tile_stages > 3 && p.n_stages < 2 * tile_stages && (p.n_stages >= 3 || one_tile);
 }
 
+// Bytes from row to row of a box that brings `bytes` of each (a multiple of 8): the eight rows of a fragment load meet on different
+// banks where it is an odd multiple of 16, and what a box brings beyond a row's part is never looked at. One copy a stage in
+// place of one a row: from a lane per row a copy takes 82 clocks to issue whatever its size, 13 bytes a clock and SM at Q8_0's 1088
+// (128256 x 4096 101.5 -> 84.2 us, 1.0 of the copy bandwidth; 22016 x 4096 at one, four and eight rows 21.2, 26.7, 40.2 -> 18.5, 23.1, 29.5;
+// Q3_K 22016 x 4096 18.4 -> 17.1, Q2_K 16.2 -> 14.8).
+__host__ __device__ constexpr int box_pitch(int bytes) { return align_up(bytes, 16) + (align_up(bytes, 16) / 16 % 2 == 0 ? 16 : 0); }
+
 // Fills the fields that depend only on the format, the width and the activation row count.
 // Returns false when the streaming kernel does not address the shape.
 template <int WT>
@@ -2173,6 +2184,12 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.use_tma = 2;
         p.tma_unit_div = kConsumerWarps;
         p.row_stride = ku_max * F::unit_bytes;
+        p.box_bytes = kTileRows * p.tps * p.row_stride;
+        p.stage_bytes = align_up(p.box_bytes, 128);
+        p.gran = kTileRows * p.tps;
+    } else if (want_tma && F::tma == 3 && !p.ragged && p.row_bytes % 16 == 0) {
+        p.use_tma = 3;
+        p.row_stride = box_pitch(ku_max * F::unit_bytes);
         p.box_bytes = kTileRows * p.tps * p.row_stride;
         p.stage_bytes = align_up(p.box_bytes, 128);
         p.gran = kTileRows * p.tps;
@@ -2308,7 +2325,7 @@ inline bool weight_map(CUtensorMap *out, const uint8_t *w, int64_t n_out, int ro
     if (!encode) return false;
     static std::mutex mu;
     static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-    const MapKey key{w, n_out, row_bytes, unit_bytes, box_rows, mode == 2 ? -box_units : box_units};
+    const MapKey key{w, n_out, row_bytes, unit_bytes, box_rows, mode == 1 ? box_units : -box_units};
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
@@ -2316,16 +2333,16 @@ inline bool weight_map(CUtensorMap *out, const uint8_t *w, int64_t n_out, int ro
         return true;
     }
     // mode 1: {unit bytes, rows, units of a row} in bytes; mode 2: {box_units units as 64-bit elements, rows, groups of
-    // box_units units of a row}
-    const int inner_bytes = mode == 2 ? box_units * unit_bytes : unit_bytes;
-    if (mode == 2 && (inner_bytes % 16 != 0 || inner_bytes / 8 > 256 || row_bytes % inner_bytes != 0)) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)(mode == 2 ? inner_bytes / 8 : inner_bytes), (cuuint64_t)n_out,
-                                (cuuint64_t)(row_bytes / inner_bytes)};
+    // box_units units of a row}; mode 3: {the row as 64-bit elements, rows, 1}
+    const int inner_bytes = mode == 3 ? row_bytes : mode == 2 ? box_units * unit_bytes : unit_bytes, size = mode == 1 ? 1 : 8;
+    const int box_inner = mode == 3 ? box_pitch(box_units * unit_bytes) : inner_bytes;
+    if (mode != 1 && (inner_bytes % 16 != 0 || box_inner / 8 > 256 || row_bytes % inner_bytes != 0)) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)(inner_bytes / size), (cuuint64_t)n_out, (cuuint64_t)(row_bytes / inner_bytes)};
     const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)inner_bytes};
-    const cuuint32_t box[3] = {(cuuint32_t)dims[0], (cuuint32_t)box_rows, (cuuint32_t)(mode == 2 ? 1 : box_units)};
+    const cuuint32_t box[3] = {(cuuint32_t)(box_inner / size), (cuuint32_t)box_rows, (cuuint32_t)(mode == 1 ? box_units : 1)};
     const cuuint32_t elem[3] = {1, 1, 1};
     CUtensorMap m;
-    if (encode(&m, mode == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t *>(w), dims, strides, box, elem,
+    if (encode(&m, mode != 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t *>(w), dims, strides, box, elem,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2_promotion(),
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
@@ -2348,15 +2365,35 @@ bool encode_maps(StreamParams &p, int n) {
     return true;
 }
 
+// Launches of a format whose stages could be one box each (use_tma == 3) that copy row by row all the same, at one and two
+// activation rows and up to two tiles an SM. Row copies let any number of rows go to a CTA, a box brings whole tiles. Fewer tiles
+// than half of the SMs: all SMs at work on parts of tiles beat a tile each on some (box against rows, us: Q2_K 1024 x 4096 4.7
+// against 4.2, Q8_0 1024 x 8192 7.5 against 6.8). Two activation rows: boxes fill the ring sooner, which the loads of x then wait
+// behind, and only just over a tile an SM is that worth it (Q8_0 4096 x 4096 7.4 against 6.7, 4700 x 4096 8.2 against 7.0, 2048 x 4096 4.8
+// against 4.7; 3200 x 4096 5.9 against 6.1). Q5_1's rows of 1536 bytes stream as well by themselves (4700 x 5632 10.6 against 9.8,
+// 4096 x 1024 at two rows 5.3 against 4.9; beyond, 6000 x 5632, 12.1 against 12.7).
+template <int WT>
+bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
+    const int sms = sm_count();
+    if (p.rows > 2 || tiles > 2 * sms) return false;
+    if (WT == KRK_CUDA_Q5_1) return true;
+    if (p.units < kConsumerWarps) return false;
+    if (tiles <= sms / 2) return true;
+    return p.rows == 2 && p.units > kConsumerWarps && smem <= (size_t)kSmemLimit && (tiles <= sms || tiles > 3 * sms / 2);
+}
+
 // setup_format with the tensor-copy layout where the format and the matrices allow it (the maps are encoded here),
 // else with per-row copies. False when the streaming kernel does not address the shape.
 template <int WT>
 bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in, int rows, int silu_pair, size_t *smem) {
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
+    int64_t tiles = 0;
+    for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
     if (tma) {
         if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
-        if (p.use_tma) {
+        if (p.use_tma == 3 && rows_apart<WT>(p, tiles, *smem)) tma = false;
+        if (tma && p.use_tma) {
             for (int m = 0; m < n_mat; m++) p.mat[m] = mats[m];
             if (!encode_maps<WT>(p, n_mat)) tma = false;   // a map cannot be encoded: set up again for row copies
         }
@@ -2367,11 +2404,10 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
         // tiles for two one-group CTAs per SM, and a half has room for them, those stream (one group against two, four rows:
         // 49152 x 4096 55.5 against 76.0 us, 11008 x 4096 18.8 against 20.6; 4096 x 4096 10.7 against 10.2, and 512 x 1024 5.8
         // against 4.5).
-        int64_t tiles = 0;
-        for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
-        if ((rows == 3 || rows == 4) && n_in % 256 == 0 && tiles > 2 * sm_count() && setup_format<WT>(p, n_in, rows, silu_pair, smem, false, true) &&
-            p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit)
-            return true;
+        if ((rows == 3 || rows == 4) && n_in % 256 == 0 && tiles > 2 * sm_count()) {
+            if (setup_format<WT>(p, n_in, rows, silu_pair, smem, tma, true) && p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit) return true;
+            if (tma && !setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
+        }
     }
     return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem);
 }
@@ -2424,13 +2460,14 @@ int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_
     // With the banks known, a stage arrives as one tensor copy out of the bank's map.
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     bool tma = false;
-    if (banks && Fmt<WT>::tma == 1 && !no_tma && setup_format<WT>(p, n_in, rows, silu_pair, &smem, true) && p.use_tma == 1) {
+    if (banks && (Fmt<WT>::tma == 1 || Fmt<WT>::tma == 3) && !no_tma && setup_format<WT>(p, n_in, rows, silu_pair, &smem, true) &&
+        (p.use_tma == 1 || p.use_tma == 3)) {
         tma = true;
         const int ku_max = p.units < kConsumerWarps ? p.units : kConsumerWarps;
         for (int b = 0; b < p.step && tma; b++) {
             p.bank_base[b] = banks->base[b];
             tma = banks->base[b] && (reinterpret_cast<uintptr_t>(banks->base[b]) & 15) == 0 && banks->rows > 0 &&
-                  weight_map(&p.wmap[b], banks->base[b], banks->rows, p.row_bytes, Fmt<WT>::unit_bytes, kTileRows * p.tps, ku_max, 1);
+                  weight_map(&p.wmap[b], banks->base[b], banks->rows, p.row_bytes, Fmt<WT>::unit_bytes, kTileRows * p.tps, ku_max, p.use_tma);
         }
     }
     if (!tma && !setup_format<WT>(p, n_in, rows, silu_pair, &smem)) return 0;

@@ -136,6 +136,25 @@ def test_rows_of_odd_block_counts_keep_infinities(cuda, wt):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
 
 
+# (a box holds a stage's part of 16 rows and up to 16 bytes more of each: one stage and several, whole and clipped by the row's end,
+# stacked tiles; rows clipped by the matrix's end; launches on either side of the rules by tiles, of 74, 148, 222 and 296)
+@pytest.mark.parametrize("wt, widths", [(synth.Q8_0, (256, 512, 1024, 2304, 4096, 11008)), (synth.Q2_K, (1024, 3072, 8192)),
+                                        (synth.Q3_K, (2048, 6144)), (synth.Q5_1, (256, 768, 2304, 4096))])
+def test_stages_in_one_box_of_padded_rows(cuda, wt, widths):
+    import torch
+    for n_in in widths:
+        for n_out in (1, 15, 33, 1185, 2367, 2369, 3553, 4737):
+            w = dev(synth.weights(wt, n_out, n_in, SEED + 7, stream=wt))
+            w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+            for rows in (1, 2, 4, 7):
+                x = dev(synth.activations(rows, n_in, SEED + rows))
+                y = cuda.gemv(x, w, wt, n_out, n_in)
+                # the bound of test_finite_activations_of_any_size: 22 bits of x against its largest value, twice over
+                lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None]
+                assert ((y.double() - x.double() @ w64.T).abs() <= lim).all(), (n_in, n_out, rows)
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out", [4736, 4737, 5003])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
     """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
