@@ -43,6 +43,7 @@
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
+#include <vector>
 
 #include "krk_chunk.cuh"
 
@@ -62,6 +63,7 @@ __host__ __device__ constexpr int cta_threads(int groups) { return groups * kCon
 // Tiles whose partial sums may wait for the epilogue warp (fewer when more activation rows make a slot larger).
 __host__ __device__ constexpr int red_slots(int ng) { return ng == 1 ? 4 : ng == 2 ? 2 : 1; }   // of each consumer group
 constexpr int kMaxRedSlots = 4;
+constexpr int kMaxMaps = 24;      // of a launch: three matrices of ragged rows
 constexpr int kMaxStack = 4;      // 16-row tiles per stage at most
 constexpr int kTileRows = 16;                     // the M of the MMA
 constexpr int kMaxStages = 8;                    // of a whole-SM CTA
@@ -126,9 +128,8 @@ struct StreamParams {
     int tma_unit_div;     // the copy's third coordinate is the stage's first unit / this (use_tma == 3: 0, and its first coordinate
                           // the unit's place in the row in 64-bit elements)
     int box_bytes;        // bytes one tensor copy signals (the whole box, also where the matrix clips it)
-    int ragged;           // 1: rows are not 16-byte multiples and too long for whole tiles: every row of a stage is
-                          // copied from the 16-byte boundary below its first byte, and its bytes sit that far
-                          // (0..15 bytes, a multiple of 2) into the row's slot
+    int ragged;           // rows are not 16-byte multiples and too long for whole tiles: how many rows on (2, 4 or 8) a row lies
+                          // equally far off a 16-byte boundary, see TilePlace; else 0
     int by_stage;         // 1: the two groups take a tile's stages in turn, each with sums of its own; 0: they take tiles in turn
     int accumulate;
     int entry_gran;       // table launches: granules of every entry (all have one shape)
@@ -145,10 +146,10 @@ struct StreamParams {
     int *peer_flag[KRK_CUDA_MAX_PEERS];   // peer_flag[q][my_rank] <- epoch once every CTA here has stored
     int n_peers, my_rank, epoch, wait_peers;
     long long peer_row_stride, peer_offset;
-    // per matrix: the weights as a 3-d tensor {unit_bytes, n_out rows, units per row}; box = {unit_bytes,
-    // rows of a stage, units of a stage}
-    CUtensorMap wmap[KRK_CUDA_MAX_GROUP];
+    // per matrix (ragged rows: per matrix and phase, see TilePlace): the weights as a 3-d tensor, see weight_maps
+    CUtensorMap wmap[kMaxMaps];
 };
+static_assert(sizeof(StreamParams) <= 4096, "what every launch may pass");
 static_assert(offsetof(StreamParams, status) == 64 && offsetof(StreamParams, gran_begin) == 120 && offsetof(StreamParams, mat) == 192, "the lines above");
 
 
@@ -284,7 +285,10 @@ struct Smem {
     unsigned long long red_full[kMaxRedSlots];  // every consumer warp has written its partial sums of a tile
     unsigned long long red_empty[kMaxRedSlots]; // the epilogue warp has consumed them
     int gave_up;
-    int touched[11];   // where the parameter fetches of the first instructions end (never read)
+    union {
+        int touched[11];            // where the parameter fetches of the first instructions end (never read)
+        uint32_t lead[kMaxStages];  // ragged rows: how far the rows of a stage lie into their slots (0..15 bytes)
+    };
     float gate[kMaxStack][NG][32];   // epilogue warp: the gate tile(s) of a gate/up pair, until the up tile arrives
     // per consumer warp, column group and row pair (g, g+8): {row g x even activation row, g x odd, g+8 x even, g+8 x odd}
     float4 red[GROUPS * red_slots(NG)][kConsumerWarps][NG][8];
@@ -348,7 +352,8 @@ struct StageInfo {
     int mat;        // matrix index
     int which;      // 0, or 1 for the `up` half of a gate/up pair
     int row0;       // first output row of the tile
-    int n_rows;     // valid rows in the stage (1..16 * tps)
+    int n_rows;     // valid rows in the stage (1..16 * tps); ragged rows: every p.ragged-th from row0 on
+    int of, k;      // ragged rows: the tile's phase, and its first row among those of the phase (TilePlace)
     int unit0;      // first K unit of this stage
     int n_units;    // units in this stage (1..16)
     int last;       // last stage of the tile
@@ -386,7 +391,38 @@ struct TableView {
     __device__ __forceinline__ int n_out(int m) const { return (int)(dev ? dev->mat[m].n_out : p.mat[m].n_out); }
 };
 
-template <class SegmentFn, class StageFn>
+// Ragged rows: rows `ragged` apart lie equally far off a 16-byte boundary, so a tile takes such rows, of one phase (row modulo
+// `ragged`): they are a matrix of 16-byte-multiple pitch, of which a stage arrives as one tensor copy, and every word of the tile lies
+// alike. An entry's granules are tiles, phase by phase: all phases have as many, or the first ones one more, and a phase's rows are
+// dealt to its tiles evenly (16 * tps at most). A phase without rows, in matrices of fewer than eight, has tiles of none, whose sums
+// go nowhere.
+struct TilePlace {
+    int phase, left;   // the tile's phase, and how many of its tiles are left, this one included
+    __device__ __forceinline__ static int tiles(const StreamParams &p, int granules, int phase) {
+        const int shift = __ffs(p.ragged) - 1, each = granules >> shift;
+        return max(each + (phase < granules - (each << shift) ? 1 : 0), 1);
+    }
+    __device__ __forceinline__ TilePlace(const StreamParams &p, int at, int granules) {   // granule `at` of an entry's
+        const int more = tiles(p, granules, 0), most = tiles(p, granules, p.ragged - 1), n_more = more == most ? 0 : granules - (most * p.ragged);
+        const bool first = at < n_more * more;
+        const int n = first ? more : most, rel = first ? at : at - n_more * more, of = rel / n;
+        phase = of + (first ? 0 : n_more);
+        left = n - (rel - of * n);
+    }
+    __device__ __forceinline__ void next(const StreamParams &p, int granules) {
+        if (--left == 0) left = tiles(p, granules, ++phase);
+    }
+    // the tile's rows: `count` from the phase's k-th on
+    __device__ __forceinline__ void rows(const StreamParams &p, int granules, int n_out, int &k, int &count) const {
+        const int n = tiles(p, granules, phase), i = n - left, all = (n_out - phase + p.ragged - 1) / p.ragged;
+        const int each = all / n, more = all - each * n;   // the first `more` tiles have a row more
+        k = i * each + min(i, more);
+        count = each + (i < more ? 1 : 0);
+    }
+};
+template <int WT>
+constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_size(WT) == 32;
+template <bool RAGGED, class SegmentFn, class StageFn>
 __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv, int tps, SegmentFn &&on_segment, StageFn &&on_stage) {
     // balanced split of the granules over the CTAs: the first gran_r CTAs take one more
     const int c = (int)blockIdx.x;
@@ -403,14 +439,16 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
         const int r1 = min(n_out, (hi - tv.begin(e)) * p.gran);
         on_segment(e * p.step);
         const int stage_rows = kTileRows * tps;
-        for (int tr = r0; tr < r1; tr += stage_rows) {
+        auto tile = [&](int row0, int n_rows, int of, int k) {
             for (int which = 0; which < p.step; which++) {
                 for (int u0 = 0; u0 < p.units; u0 += ku_max) {
                     StageInfo s;
                     s.mat = e * p.step + which;
                     s.which = which;
-                    s.row0 = tr;
-                    s.n_rows = min(stage_rows, r1 - tr);
+                    s.row0 = row0;
+                    s.n_rows = n_rows;
+                    s.of = of;
+                    s.k = k;
                     s.unit0 = u0;
                     s.n_units = min(ku_max, p.units - u0);
                     s.last = u0 + ku_max >= p.units;
@@ -423,7 +461,18 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
                     on_stage(s);
                 }
             }
+        };
+        if (RAGGED && p.ragged) {
+            const int granules = tv.begin(e + 1) - tv.begin(e);
+            TilePlace at(p, lo - tv.begin(e), granules);
+            for (int i = lo; i < hi; i++, at.next(p, granules)) {
+                int k, n;
+                at.rows(p, granules, n_out, k, n);
+                tile(at.phase + p.ragged * k, n, at.phase, k);
+            }
+            continue;
         }
+        for (int tr = r0; tr < r1; tr += stage_rows) tile(tr, min(stage_rows, r1 - tr), 0, 0);
     }
 }
 
@@ -520,7 +569,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
 }
 
 // The same where K is not a multiple of 256: four limbs, in value order everywhere (rows whose blocks start at any even
-// address, see Words). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
+// address). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
 // `live`: the lane's values lie inside the row (the last unit of such a row may be short).
 template <int WT>
 __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p, int ps,
@@ -958,17 +1007,15 @@ __device__ __forceinline__ void unit_q4_k_single(const uint8_t *rowA, const uint
     acc.m[3] = fmaf(nB, cm[3], acc.m[3]);
 }
 
-// 32-bit words at constant even offsets of a block or row in shared memory. MODE 0: it starts on a word boundary; 1: 2 bytes off
-// (blocks of 210 and 110 bytes: every other one of a row); 2: either, found from the address (ragged rows: the two rows of a lane
-// may differ). There every word is glued from two aligned ones by a shift, and both are found once for all words of an offset's
-// parity: worked out per word, through an integer that hides from the compiler that the loads are from shared memory, they were
-// most of a unit (Q6_K 4096 x 11008 731 -> 555 instructions a unit, 17.4 -> 14.5 us; Q8_0 11200 x 2080 502 -> 386, 12.4 -> 10.9).
-template <int MODE>
+// 32-bit words at constant even offsets of a block or row in shared memory that starts on a word boundary (BY2 0), 2 bytes off one
+// (1: blocks of 210 and 110 bytes, every other one of a row; ragged rows, those of every other phase), or either (2: both starts that a
+// word may have and both shifts are found once for all words). A word off the boundary is glued from two.
+template <int BY2>
 struct Words {
-    const uint8_t *p0, *p2;   // offsets that are multiples of 4, and the others
+    const uint8_t *p0, *p2;   // 2: for offsets that are multiples of 4, and for the others
     uint32_t s0, s2;
     __device__ __forceinline__ explicit Words(const uint8_t *at) : p0(at), p2(at), s0(0), s2(0) {
-        if (MODE == 2) {
+        if (BY2 == 2) {
             const uint32_t by = smem_u32(at) & 2u;
             p0 = at - by;
             p2 = at + by - 2;
@@ -977,17 +1024,17 @@ struct Words {
         }
     }
     __device__ __forceinline__ uint32_t operator()(int off) const {
-        if (MODE == 2) {
+        if (BY2 == 2) {
             const uint32_t *w = reinterpret_cast<const uint32_t *>((off & 2 ? p2 : p0) + off);
             return __funnelshift_r(w[0], w[1], off & 2 ? s2 : s0);
         }
-        if (MODE == 1) return __byte_perm(*reinterpret_cast<const uint32_t *>(p0 + off - 2), *reinterpret_cast<const uint32_t *>(p0 + off + 2), 0x5432);
-        return *reinterpret_cast<const uint32_t *>(p0 + off);
+        if (((off >> 1) & 1) == BY2) return *reinterpret_cast<const uint32_t *>(p0 + off);
+        return __byte_perm(*reinterpret_cast<const uint32_t *>(p0 + off - 2), *reinterpret_cast<const uint32_t *>(p0 + off + 2), 0x5432);
     }
 };
 
-// The 32-value blocks of rows that start at any even address (K not a multiple of 256): every word is glued from two
-// aligned loads, the limbs lie in value order (see Words), and only the first `nb` blocks of a unit exist (the last unit of a row may be
+// The 32-value blocks of rows that start at any even address (K not a multiple of 256): the limbs lie in value order, words are
+// read as they lie or glued (see Words; BY2: the tile's rows start 2 bytes off a word boundary), and only the first `nb` blocks of a unit exist (the last unit of a row may be
 // short; what its slot holds past the row is never looked at).
 __device__ __forceinline__ float half_at(const uint8_t *p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(p))); }
 
@@ -1035,10 +1082,10 @@ __device__ __forceinline__ void unit_q4_0(const uint8_t *rowA, const uint8_t *ro
 // The same eight blocks for 2..8 activation rows: the quants are centred first ((q + 0x78) ^ 0x80 is q - 8 as a
 // signed byte, no carry since q <= 15), low and high nibbles go to one k16 MMA each per column group, and the
 // columns carry the limbs of two activation rows as in the other general forms.
-template <int NG, bool RAG>
+template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_q4_0_rows(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                                int t, Accum<NG> &acc, int nb) {
-    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
+    const Words<BY2> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
@@ -1099,7 +1146,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 // Nibbles 0..3 of a quant word are [low 0, high 0, low 1, high 1], so two last permutes regroup the results into
 // the four low-nibble and the four high-nibble values. 13 integer instructions per eight values. The limbs lie
 // as for Q4_0.
-template <int NG, bool RAG>
+template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                             int t, Accum<NG> &acc, int nb) {
     constexpr uint32_t kG0 = 0xBFAD9881u, kG1 = 0xF6EADDCFu, kG2 = 0x26190D01u, kG3 = 0x71594535u;
@@ -1111,7 +1158,7 @@ __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *
         lo4 = prmt(r01, r23, 0x6420u);
         hi4 = prmt(r01, r23, 0x7531u);
     };
-    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
+    const Words<BY2> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
@@ -1165,10 +1212,10 @@ __device__ __forceinline__ uint32_t spread_top(uint32_t n) { return (n * 0x10204
 // group, chained on one accumulator preset to the bits of 1.5 * 2^23 (|sum| <= 32 * 128 * 128 = 2^19). Blocks at
 // an even index have mask and quants 2 bytes off a word boundary: the mask is glued from two words, lane t takes
 // quant bytes 4t-2..4t+1 (lane 0: 14, 15, 0, 1) and the mask is rotated to match.
-template <int NG, bool RAG>
+template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_q5_0(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, Accum<NG> &acc, int nb) {
-    const Words<RAG ? 2 : 0> wA(rowA), wB(rowB);
+    const Words<BY2> wA(rowA), wB(rowB);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;
@@ -1263,10 +1310,10 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
 // Four Q8_0 blocks. A block is a 2-byte scale then 32 quants, so blocks at an even index have
 // their quants 2 bytes off a word boundary: their lanes read the aligned words and lane t = 0
 // glues the two half words at the ends into one (the activation limbs are permuted to match).
-template <int NG, bool RAG>
+template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, Accum<NG> &acc, int nb) {
-    const Words<RAG ? 2 : 0> wA(rowA + 4 * t), wB(rowB + 4 * t);
+    const Words<BY2> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 4; b++) {
         if (RAG && b >= nb) break;
@@ -1319,10 +1366,10 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
 // Four integer instructions per four quants against six for assembling q and then centring it; the factor 4
 // leaves with the block scale.
 
-template <int NG, int ODD>
+template <int NG, int BY2>
 __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, AccumSuper<NG> &acc) {
-    const Words<ODD> wA(blkA), wB(blkB);
+    const Words<BY2> wA(blkA), wB(blkB);
     int I[NG][4];
 #pragma unroll
     for (int mg = 0; mg < kFoldGroups<NG>; mg++)
@@ -1431,11 +1478,11 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
 // bytes, d; value = d * (scale - 32) * (q2 - (mask bit ? 0 : 4)). The A operand is 32 * (q3 - 4) with q3 = q2 + 4 *
 // mask bit: q2 at bits 5-6 and the inverted mask bit at bit 7 (a 3-bit two's complement at the top of the byte),
 // two shifts, an AND and an AND-OR per four quants; the 32 leaves with d. Blocks are 110 bytes: every other one is
-// 2 bytes off a word boundary (MODE as for Q6_K).
-template <int NG, int MODE>
+// 2 bytes off a word boundary.
+template <int NG, int BY2>
 __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, AccumSuper<NG> &acc) {
-    const Words<MODE> wA(blkA), wB(blkB);
+    const Words<BY2> wA(blkA), wB(blkB);
     uint32_t SA[4], SB[4];
     {
         const uint32_t a0 = wA(96), a1 = wA(100), a2 = wA(104);
@@ -1509,10 +1556,6 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
 // RAG: the form for ragged rows of Q6_K and Q3_K and of the 32-value block formats (K not a multiple of 256), whose units
 // find each word's alignment from its address; compiled apart so that the usual form does not carry another copy of
 // the unit. (Q2_K's words are aligned at every row start: its usual form serves ragged rows too.)
-template <int WT>
-constexpr bool kRagForm = WT == KRK_CUDA_Q6_K || WT == KRK_CUDA_Q3_K || block_size(WT) == 32;
-template <int WT>
-constexpr bool kMayRag = kRagForm<WT> || WT == KRK_CUDA_Q2_K;
 // Forms whose two groups may take a tile's stages in turn (StreamParams::by_stage): ragged Q6_K. (Q3_K 4096 x 8960 at four rows
 // 19.1 -> 20.0 us with it.)
 template <int WT>
@@ -1537,6 +1580,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
     constexpr bool kFine = RAG && !kSuper;   // fine_limbs
     constexpr bool kMayByStage = may_by_stage<WT>(RAG, kGroups);
+    constexpr bool kRagged = RAG || WT == KRK_CUDA_Q2_K;   // p.ragged may be set
     using F = Fmt<WT>;
     using SmemT = Smem<NG, GROUPS>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -1580,13 +1624,31 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         // A device-side table is the output of the kernel before this one: wait for that grid.
         if (p.dev_table) asm volatile("griddepcontrol.wait;" ::: "memory");
         const TableView tv(p);
-        walk(p, tv, tps, [](int) {}, [&](const StageInfo &s) {
+        walk<kRagged>(p, tv, tps, [](int) {}, [&](const StageInfo &s) {
             const int slot = s.slot;
             const uint32_t full = smem_u32(&sm->full[slot]), empty = smem_u32(&sm->empty[slot]);
             wait_phase(empty, s.phase ^ 1, gave_up, p.status);
             uint8_t *dst = stages + (size_t)slot * p.stage_bytes;
             const uint8_t *src = tv.w(s.mat) + (size_t)s.row0 * p.row_bytes;
-            if (p.use_tma) {
+            if (kRagged && !RAG && lane == 0) sm->lead[slot] = 0u;
+            if (kRagged && p.ragged) {
+                // from the 16-byte boundary below each row's part on; a stage starts a multiple of 8 units (a multiple of 16 bytes in
+                // every format) into its rows, so a row lies equally far off in every stage
+                const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15);
+                if (lane == 0) sm->lead[slot] = a;   // (and the arrival below, which the consumers wait for, comes after it)
+                if (p.use_tma) {
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(full, (uint32_t)p.box_bytes);
+                        tma_box(smem_u32(dst), &p.wmap[s.mat * p.ragged + s.of], s.unit0 * F::unit_bytes / 8, s.k, 0, full);
+                    }
+                } else {
+                    const uint32_t bytes = (a + min((uint32_t)s.n_units * F::unit_bytes, (uint32_t)(p.row_bytes - s.unit0 * F::unit_bytes)) + 15u) & ~15u;
+                    if (lane == 0) mbar_arrive_expect_tx(full, bytes * s.n_rows);
+                    __syncwarp();
+                    for (int r = lane; r < s.n_rows; r += 32)
+                        bulk_g2s(smem_u32(dst + r * p.row_stride), src + (size_t)r * p.ragged * p.row_bytes + (size_t)s.unit0 * F::unit_bytes - a, bytes, full);
+                }
+            } else if (p.use_tma) {
                 // the box is clipped where the matrix ends (rows past n_out, units past the row) and
                 // still signals its full size
                 if (lane == 0) {
@@ -1601,23 +1663,6 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         if constexpr (F::tma == 3) tma_box(smem_u32(dst), &p.wmap[s.mat], s.unit0 * F::unit_bytes / 8, s.row0, 0, full);
                         else tma_box(smem_u32(dst), &p.wmap[s.mat], 0, s.row0, s.unit0 / p.tma_unit_div, full);
                     }
-                }
-            } else if (kMayRag<WT> && p.ragged) {
-                // a stage starts a multiple of 8 units (a multiple of 16 bytes in every format) into its rows, so a row lies equally far off
-                // a 16-byte boundary in every stage
-                const uint32_t bytes = min((uint32_t)s.n_units * F::unit_bytes, (uint32_t)(p.row_bytes - s.unit0 * F::unit_bytes));
-                uint32_t total = 0;
-                for (int r = lane; r < s.n_rows; r += 32) {
-                    const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(src + (size_t)r * p.row_bytes) & 15);
-                    total += (a + bytes + 15u) & ~15u;
-                }
-                total = __reduce_add_sync(0xFFFFFFFFu, total);
-                if (lane == 0) mbar_arrive_expect_tx(full, total);
-                __syncwarp();
-                for (int r = lane; r < s.n_rows; r += 32) {
-                    const uint8_t *row = src + (size_t)r * p.row_bytes + (size_t)s.unit0 * F::unit_bytes;
-                    const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15);
-                    bulk_g2s(smem_u32(dst + r * p.row_stride), row - a, (a + bytes + 15u) & ~15u, full);
                 }
             } else if (!p.whole_tiles) {
                 const uint32_t bytes = (uint32_t)s.n_units * F::unit_bytes;
@@ -1657,7 +1702,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         float gate_reg[NG];   // silu of the gate tile (stacked tiles keep theirs in shared memory)
         int tile_it = 0, n_out = 0;
         float *y0 = nullptr;
-        walk(p, tv, tps, [&](int m) {
+        walk<kRagged>(p, tv, tps, [&](int m) {
             y0 = tv.y(m);
             n_out = tv.n_out(m);
         }, [&](const StageInfo &s) {
@@ -1690,9 +1735,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         for (int w = 0; w < kConsumerWarps; w++) v += part[w];
                     }
                     const int srow = kTileRows * sub + row;   // row inside the stage
+                    const int yrow = s.row0 + (kRagged && p.ragged ? srow * p.ragged : srow);
                     if (kFine && v != v && r < p.rows && srow < s.n_rows) {
                         const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
-                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)(s.row0 + srow) * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
+                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)(s.row0 + srow * p.ragged) * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
                     }
                     if (r < p.rows) {
                         if (p.step == 2 && s.which == 0) {
@@ -1702,10 +1748,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         } else if (srow < s.n_rows) {
                             if (p.n_peers > 0) {
                                 // plain stores into every GPU's copy of the full row (NVLink peer stores)
-                                const long long at = (long long)r * p.peer_row_stride + p.peer_offset + s.row0 + srow;
+                                const long long at = (long long)r * p.peer_row_stride + p.peer_offset + yrow;
                                 for (int q = 0; q < p.n_peers; q++) p.peer_y[q][at] = v;
                             } else {
-                                float *y = y0 + (size_t)r * n_out + s.row0 + srow;
+                                float *y = y0 + (size_t)r * n_out + yrow;
                                 if (p.step == 2) v = __fmul_rn(STACK ? sm->gate[sub][i][lane] : gate_reg[i], v);
                                 *y = p.accumulate ? __fadd_rn(*y, v) : v;
                             }
@@ -1874,7 +1920,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
         }
         const int stage_rows = kTileRows * tps;
-        const int n_tiles = ((r1 - r0 + stage_rows - 1) / stage_rows) * p.step;
+        const int n_tiles = (RAG || (kRagged && p.ragged) ? hi - lo : (r1 - r0 + stage_rows - 1) / stage_rows) * p.step;
         for (int tile = 0; tile < n_tiles; tile++) {
             // the other group's stage: it is seen to land (a ring slot's parity only tells two laps apart for a warp that looks at
             // every lap) and given back
@@ -1893,28 +1939,23 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                 for (int ck = 0; ck < n_chunks; ck++) pass();
                 continue;
             }
-            // ragged rows: how far this lane's two rows sit into their slots of a stage
-            uint32_t ragA = 0, ragB = 0;
-            if (RAG || (WT == KRK_CUDA_Q2_K && p.ragged)) {
-                const int row = r0 + (tile / p.step) * stage_rows + kTileRows * my_sub + g;
-                const uintptr_t base = reinterpret_cast<uintptr_t>(tv.w(m + tile % p.step));
-                ragA = (uint32_t)((base + (size_t)row * p.row_bytes) & 15);
-                ragB = (uint32_t)((base + (size_t)(row + 8) * p.row_bytes) & 15);
-            }
             // one stage of the tile: `bf` are the warp's held B fragments for it (SINGLE == 2), else unused
             auto stage = [&](const int ck, const BFrag &bf) {
                 wait_phase(full0 + 8 * slot, phase, gave_up, p.status);
                 const int stage_units = p.whole_tiles ? p.units : min(kConsumerWarps, p.units - ck * kConsumerWarps);
                 if (!stacked_idle) {
-                    const uint8_t *tile0 = stages + (size_t)slot * p.stage_bytes + lane_off;
+                    const uint32_t lead = kRagged ? sm->lead[slot] : 0u;   // (0 where rows are not ragged)
+                    const bool by2 = kFine && (lead & 2u);   // rows start 2 bytes off a word boundary
+                    const uint8_t *tile0 = stages + (size_t)slot * p.stage_bytes + lane_off + lead;
                     for (int su = my_unit; su < stage_units; su += kConsumerWarps) {
-                        const uint8_t *rowA = tile0 + (size_t)su * p.unit_stride + ragA;
-                        const uint8_t *rowB = tile0 + (size_t)su * p.unit_stride + (size_t)8 * p.row_stride + ragB;
+                        const uint8_t *rowA = tile0 + (size_t)su * p.unit_stride;
+                        const uint8_t *rowB = tile0 + (size_t)su * p.unit_stride + (size_t)8 * p.row_stride;
                         const int unit = ck * kConsumerWarps + su;
                         const int kbase = unit * F::unit_values;
                         const int nb = (p.n_in - kbase) >> 5;   // 32-value blocks of the unit (short rows: fewer than a full unit's)
                         if constexpr (WT == KRK_CUDA_Q4_0 && !SINGLE) {
-                            unit_q4_0_rows<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
+                            if (by2) unit_q4_0_rows<NG, RAG, 1>(rowA, rowB, kbase, bp, t, acc, nb);
+                            else unit_q4_0_rows<NG, RAG, 0>(rowA, rowB, kbase, bp, t, acc, nb);
                         } else if constexpr (WT == KRK_CUDA_Q4_0) {
                             unit_q4_0(rowA, rowB, bq + kbase, reinterpret_cast<const float *>(chunk_sum) + (kbase >> 5), t, acs);
                         } else if constexpr (SINGLE == 2) {
@@ -1924,11 +1965,14 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                         } else if constexpr (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K) {
                             unit_q4_k<NG, WT == KRK_CUDA_Q5_K>(rowA, rowB, kbase, bp, sp, t, acc);
                         } else if constexpr (WT == KRK_CUDA_Q8_0) {
-                            unit_q8_0<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
+                            if (by2) unit_q8_0<NG, RAG, 1>(rowA, rowB, kbase, bp, t, acc, nb);
+                            else unit_q8_0<NG, RAG, 0>(rowA, rowB, kbase, bp, t, acc, nb);
                         } else if constexpr (WT == KRK_CUDA_Q5_0) {
-                            unit_q5_0<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
+                            if (by2) unit_q5_0<NG, RAG, 1>(rowA, rowB, kbase, bp, t, acc, nb);
+                            else unit_q5_0<NG, RAG, 0>(rowA, rowB, kbase, bp, t, acc, nb);
                         } else if constexpr (WT == KRK_CUDA_IQ4_NL) {
-                            unit_iq4_nl<NG, RAG>(rowA, rowB, kbase, bp, t, acc, nb);
+                            if (by2) unit_iq4_nl<NG, RAG, 1>(rowA, rowB, kbase, bp, t, acc, nb);
+                            else unit_iq4_nl<NG, RAG, 0>(rowA, rowB, kbase, bp, t, acc, nb);
                         } else if constexpr (WT == KRK_CUDA_Q2_K) {
                             unit_q2_k<NG>(rowA, rowB, kbase, bp, sp, t, acc);
                         } else if constexpr (WT == KRK_CUDA_Q3_K) {
@@ -2162,9 +2206,12 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     // Q2_K rows are 16-byte multiples for K % 1024 == 0, Q3_K rows for K % 2048 == 0
     if ((WT == KRK_CUDA_Q2_K || WT == KRK_CUDA_Q3_K) && (p.row_bytes & 15) != 0) p.ragged = 1;
     if (odd_k) p.ragged = 1;
+    if (p.ragged) p.ragged = p.row_bytes & 2 ? 8 : p.row_bytes & 4 ? 4 : 2;
     const int ku_max = p.whole_tiles ? p.units : (p.units < kConsumerWarps ? p.units : kConsumerWarps);
     p.tps = kConsumerWarps / p.units;   // 0 when a tile has more units than there are consumer warps
     p.tps = p.tps < 1 ? 1 : (p.tps > kMaxStack ? kMaxStack : p.tps);
+    // (what decides whether a shape is taken, see below, and is the pitch of row copies of 16-byte multiples)
+    const int raw = ku_max * F::unit_bytes + (p.ragged ? 48 : 0), rows_stride = raw + ((F::stride_mod - raw % 128) + 128) % 128;
     p.use_tma = 0;
     p.box_bytes = 0;
     p.unit_stride = F::unit_bytes;
@@ -2187,9 +2234,9 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.box_bytes = kTileRows * p.tps * p.row_stride;
         p.stage_bytes = align_up(p.box_bytes, 128);
         p.gran = kTileRows * p.tps;
-    } else if (want_tma && F::tma == 3 && !p.ragged && p.row_bytes % 16 == 0) {
-        p.use_tma = 3;
-        p.row_stride = box_pitch(ku_max * F::unit_bytes);
+    } else if (p.ragged || (want_tma && F::tma == 3)) {
+        p.use_tma = want_tma ? 3 : 0;
+        p.row_stride = box_pitch(ku_max * F::unit_bytes + (p.ragged ? 14 : 0));
         p.box_bytes = kTileRows * p.tps * p.row_stride;
         p.stage_bytes = align_up(p.box_bytes, 128);
         p.gran = kTileRows * p.tps;
@@ -2197,10 +2244,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.row_stride = p.row_bytes;
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_bytes, 128);
     } else {
-        // (ragged rows: up to 15 bytes before and 15 after the row's own, and a word of slack for the loads that
-        // glue a value from two words)
-        const int raw = ku_max * F::unit_bytes + (p.ragged ? 48 : 0);
-        p.row_stride = raw + ((F::stride_mod - raw % 128) + 128) % 128;
+        p.row_stride = rows_stride;
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
@@ -2222,9 +2266,10 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.spread_sums = fits_half(apart) == fits_half(close) && depth(apart, fits_half(apart)) == depth(close, fits_half(close));
     const int fixed = p.spread_sums ? apart : close;
     p.n_stages = depth(fixed, fits_half(fixed));
-    // (a shape is taken if it would be with limb planes of n_in + 32 bytes: beyond, the warp-per-row kernel multiplies in f32)
+    // (a shape is taken if it would be with limb planes of n_in + 32 bytes and stages of row copies: beyond, the warp-per-row kernel multiplies in f32)
     const int spread = align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
-    if (p.n_stages < 2 || kSmemWhole - close - p.tps * spread < 2 * p.stage_bytes) return false;
+    const int stage = p.ragged || F::tma == 3 ? align_up(kTileRows * p.tps * rows_stride, 128) : p.stage_bytes;
+    if (p.n_stages < 2 || kSmemWhole - close - p.tps * spread < 2 * stage) return false;
     p.by_stage = stages_in_turn<WT>(p, false);
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
     return true;
@@ -2312,8 +2357,11 @@ inline CUtensorMapL2promotion l2_promotion() {
     return v == 0 ? CU_TENSOR_MAP_L2_PROMOTION_NONE : v == 1 ? CU_TENSOR_MAP_L2_PROMOTION_L2_64B
            : v == 2 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
 }
-inline bool weight_map(CUtensorMap *out, const uint8_t *w, int64_t n_out, int row_bytes, int unit_bytes, int box_rows, int box_units,
-                int mode) {
+// The tensor maps of a matrix, one, or one per phase of its rows (`ragged`, see TilePlace): mode 1: {unit bytes, rows, units of a row} in
+// bytes; mode 2: {box_units units as 64-bit elements, rows, groups of box_units units of a row}; mode 3: {the row as 64-bit elements, rows,
+// 1}; ragged: {that from the 16-byte boundary below the phase's first row on, its rows, 1}.
+inline bool weight_maps(CUtensorMap *out, const uint8_t *w, int64_t n_out, int row_bytes, int unit_bytes, int box_rows, int box_units,
+                int mode, int ragged) {
     static EncodeTiledFn encode = [] {
         void *ptr = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -2323,32 +2371,35 @@ inline bool weight_map(CUtensorMap *out, const uint8_t *w, int64_t n_out, int ro
         return reinterpret_cast<EncodeTiledFn>(ptr);
     }();
     if (!encode) return false;
+    const int n = ragged ? ragged : 1;
     static std::mutex mu;
-    static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
+    static std::unordered_map<MapKey, std::vector<CUtensorMap>, MapKeyHash> cache;
     const MapKey key{w, n_out, row_bytes, unit_bytes, box_rows, mode == 1 ? box_units : -box_units};
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
-        *out = it->second;
+        for (int c = 0; c < n; c++) out[c] = it->second[c];
         return true;
     }
-    // mode 1: {unit bytes, rows, units of a row} in bytes; mode 2: {box_units units as 64-bit elements, rows, groups of
-    // box_units units of a row}; mode 3: {the row as 64-bit elements, rows, 1}
-    const int inner_bytes = mode == 3 ? row_bytes : mode == 2 ? box_units * unit_bytes : unit_bytes, size = mode == 1 ? 1 : 8;
-    const int box_inner = mode == 3 ? box_pitch(box_units * unit_bytes) : inner_bytes;
-    if (mode != 1 && (inner_bytes % 16 != 0 || box_inner / 8 > 256 || row_bytes % inner_bytes != 0)) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)(inner_bytes / size), (cuuint64_t)n_out, (cuuint64_t)(row_bytes / inner_bytes)};
-    const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)inner_bytes};
-    const cuuint32_t box[3] = {(cuuint32_t)(box_inner / size), (cuuint32_t)box_rows, (cuuint32_t)(mode == 1 ? box_units : 1)};
-    const cuuint32_t elem[3] = {1, 1, 1};
-    CUtensorMap m;
-    if (encode(&m, mode != 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t *>(w), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2_promotion(),
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    for (int c = 0; c < n; c++) {
+        const int64_t first = c < n_out ? c : 0;   // (a phase without rows: never copied)
+        const int lead = ragged ? (int)((size_t)first * row_bytes & 15) : 0;
+        const int inner_bytes = ragged ? align_up(lead + row_bytes, 8) : mode == 3 ? row_bytes : mode == 2 ? box_units * unit_bytes : unit_bytes;
+        const int box_inner = mode == 3 ? box_pitch(box_units * unit_bytes + (ragged ? 14 : 0)) : inner_bytes, size = mode == 1 ? 1 : 8;
+        if (mode != 1 && (box_inner / 8 > 256 || (!ragged && (inner_bytes % 16 != 0 || row_bytes % inner_bytes != 0)))) return false;
+        const cuuint64_t dims[3] = {(cuuint64_t)(inner_bytes / size), (cuuint64_t)(ragged ? (n_out - first + ragged - 1) / ragged : n_out),
+                                    (cuuint64_t)(ragged ? 1 : row_bytes / inner_bytes)};
+        const cuuint64_t strides[2] = {(cuuint64_t)row_bytes * n, (cuuint64_t)(ragged ? (size_t)row_bytes * n : (size_t)inner_bytes)};
+        const cuuint32_t box[3] = {(cuuint32_t)(box_inner / size), (cuuint32_t)box_rows, (cuuint32_t)(mode == 1 ? box_units : 1)};
+        const cuuint32_t elem[3] = {1, 1, 1};
+        const uint8_t *base = w + (size_t)first * row_bytes - lead;
+        if (encode(&out[c], mode != 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t *>(base), dims, strides, box, elem,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2_promotion(),
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
     if (cache.size() > 65536) cache.clear();   // bounded: a host that keeps re-uploading weights starts over
-    cache.emplace(key, m);
-    *out = m;
+    cache.emplace(key, std::vector<CUtensorMap>(out, out + n));
     return true;
 }
 
@@ -2356,13 +2407,20 @@ inline bool weight_map(CUtensorMap *out, const uint8_t *w, int64_t n_out, int ro
 template <int WT>
 bool encode_maps(StreamParams &p, int n) {
     using F = Fmt<WT>;
-    const int ku_max = p.units < kConsumerWarps ? p.units : kConsumerWarps;
+    const int ku_max = p.units < kConsumerWarps ? p.units : kConsumerWarps, each = p.ragged ? p.ragged : 1;
+    if (n * each > kMaxMaps) return false;
     for (int m = 0; m < n; m++) {
         if (p.mat[m].n_out <= 0) continue;
         if ((reinterpret_cast<uintptr_t>(p.mat[m].w) & 15) != 0) return false;
-        if (!weight_map(&p.wmap[m], p.mat[m].w, p.mat[m].n_out, p.row_bytes, F::unit_bytes, kTileRows * p.tps, ku_max, p.use_tma)) return false;
+        if (!weight_maps(&p.wmap[m * each], p.mat[m].w, p.mat[m].n_out, p.row_bytes, F::unit_bytes, kTileRows * p.tps, ku_max, p.use_tma, p.ragged)) return false;
     }
     return true;
+}
+
+// Granules of a matrix. (Ragged rows: every phase has as many, some of the last phases' maybe without a row.)
+inline int64_t granules(const StreamParams &p, int64_t n_out) {
+    if (p.ragged) return p.ragged * (((n_out + p.ragged - 1) / p.ragged + p.gran - 1) / p.gran);
+    return (n_out + p.gran - 1) / p.gran;
 }
 
 // Launches of a format whose stages could be one box each (use_tma == 3) that copy row by row all the same, at one and two
@@ -2392,7 +2450,7 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
     if (tma) {
         if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
-        if (p.use_tma == 3 && rows_apart<WT>(p, tiles, *smem)) tma = false;
+        if (p.use_tma == 3 && !p.ragged && rows_apart<WT>(p, tiles, *smem)) tma = false;
         if (tma && p.use_tma) {
             for (int m = 0; m < n_mat; m++) p.mat[m] = mats[m];
             if (!encode_maps<WT>(p, n_mat)) tma = false;   // a map cannot be encoded: set up again for row copies
@@ -2424,8 +2482,8 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
         if (mats[m].n_out > (1 << 30)) return 0;
         for (int j = 0; j < p.step; j++) p.mat[p.n_entries * p.step + j] = mats[m + j];
         p.gran_begin[p.n_entries] = total;
-        total += (int)((mats[m].n_out + p.gran - 1) / p.gran);
-        tiles += (int)((mats[m].n_out + kTileRows * p.tps - 1) / (kTileRows * p.tps));
+        total += (int)granules(p, mats[m].n_out);
+        tiles += p.ragged ? (int)granules(p, mats[m].n_out) : (int)((mats[m].n_out + kTileRows * p.tps - 1) / (kTileRows * p.tps));
         p.n_entries++;
     }
     p.gran_begin[p.n_entries] = total;
@@ -2442,9 +2500,15 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     // that belong to the next CTA). Else the CTAs of the next launch, which find room beside these, go to the idle SMs two at a
     // time and take twice as long there (Q6_K 2048 x 8192 8.5 -> 6.6 us, Q5_K 2048 x 8192 8.0 -> 6.4, Q4_K 2048 x 5632 4.8 -> 4.4). Not the
     // forms that take a whole SM: there the idle SMs let the next launch start (four rows of 2048 x 5632 7.4 and 7.7).
-    if (p.use_tma && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count() && tiles > sm_count() / 2) {
-        p.gran = 1;
-        p.gran_begin[1] = total = (int)mats[0].n_out;
+    if ((p.use_tma || p.ragged) && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
+        if (p.ragged) {   // (of four rows at least)
+            const int least = (int)(mats[0].n_out / (4 * p.ragged)) * p.ragged;
+            if (least >= sm_count()) p.gran_begin[1] = total = sm_count();
+            else if (least > total) p.gran_begin[1] = total = least;
+        } else if (tiles > sm_count() / 2) {
+            p.gran = 1;
+            p.gran_begin[1] = total = (int)mats[0].n_out;
+        }
     }
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
@@ -2461,13 +2525,13 @@ int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     bool tma = false;
     if (banks && (Fmt<WT>::tma == 1 || Fmt<WT>::tma == 3) && !no_tma && setup_format<WT>(p, n_in, rows, silu_pair, &smem, true) &&
-        (p.use_tma == 1 || p.use_tma == 3)) {
+        (p.use_tma == 1 || p.use_tma == 3) && !p.ragged) {
         tma = true;
         const int ku_max = p.units < kConsumerWarps ? p.units : kConsumerWarps;
         for (int b = 0; b < p.step && tma; b++) {
             p.bank_base[b] = banks->base[b];
             tma = banks->base[b] && (reinterpret_cast<uintptr_t>(banks->base[b]) & 15) == 0 && banks->rows > 0 &&
-                  weight_map(&p.wmap[b], banks->base[b], banks->rows, p.row_bytes, Fmt<WT>::unit_bytes, kTileRows * p.tps, ku_max, p.use_tma);
+                  weight_maps(&p.wmap[b], banks->base[b], banks->rows, p.row_bytes, Fmt<WT>::unit_bytes, kTileRows * p.tps, ku_max, p.use_tma, 0);
         }
     }
     if (!tma && !setup_format<WT>(p, n_in, rows, silu_pair, &smem)) return 0;
@@ -2475,7 +2539,7 @@ int launch_table_fmt(const StreamTable *table, const int32_t *x_rows, int64_t n_
     p.gran_q = p.gran_r = 0;
     p.dev_table = table;
     p.table_rows = x_rows;
-    p.entry_gran = (int)((n_out + p.gran - 1) / p.gran);
+    p.entry_gran = (int)granules(p, n_out);
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;
     const int rc = launch_rows<WT>(p, sm_count() * ctas_per_sm<WT>(smem, p.groups), smem, st);
@@ -2491,7 +2555,7 @@ int launch_peers_fmt(const GemvMat &mat, int64_t n_in, int rows, const PeerScatt
     p.mat[0] = mat;
     p.n_entries = 1;
     p.gran_begin[0] = 0;
-    const int total = (int)((mat.n_out + p.gran - 1) / p.gran);
+    const int total = (int)granules(p, mat.n_out);
     p.gran_begin[1] = total;
     p.status = device_status_word();
     if (!p.status) return KRK_CUDA_EDEVICE;

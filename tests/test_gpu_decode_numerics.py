@@ -155,6 +155,48 @@ def test_stages_in_one_box_of_padded_rows(cuda, wt, widths):
     assert cuda.device_status() == 0
 
 
+# Rows that are not 16-byte multiples go in tiles of rows 2, 4 or 8 apart: K = 32, 64 and 128 times odd numbers (Q8_0, Q4_0, IQ4_NL, Q5_0),
+# any K off a multiple of 2048 (Q6_K that long or that odd, Q3_K) or 1024 (Q2_K); matrices of fewer rows than that, of parts of
+# tiles, and on either side of a tile for every SM
+@pytest.mark.parametrize("wt, widths", [(synth.Q8_0, (288, 544, 1056, 2112, 2176)), (synth.Q4_0, (2080, 2112, 2176)), (synth.Q5_0, (2080, 2176)),
+                                        (synth.Q5_1, (2080, 2112)), (synth.IQ4_NL, (2080,)), (synth.Q6_K, (4352, 4864, 5120, 11008)), (synth.Q3_K, (256, 512, 1024, 2304)),
+                                        (synth.Q2_K, (256, 512, 2304))])
+def test_ragged_rows_in_tiles_of_a_phase(cuda, wt, widths):
+    import torch
+    for n_in in widths:
+        for n_out in (1, 7, 9, 129, 600, 2367, 2500, 4739):
+            w = dev(synth.weights(wt, n_out, n_in, SEED + 8, stream=wt))
+            w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+            for rows in (1, 2, 3, 8):
+                x = dev(synth.activations(rows, n_in, SEED + rows))
+                base = torch.randn((rows, n_out), device="cuda")
+                y = cuda.gemv(x, w, wt, n_out, n_in, out=base.clone(), accumulate=True)
+                # as in test_stages_in_one_box_of_padded_rows, and the rounding of the sum with the old value
+                lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
+                assert ((y.double() - base - x.double() @ w64.T).abs() <= lim).all(), (n_in, n_out, rows)
+    assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("wt, n_in", [(synth.Q8_0, 2080), (synth.Q6_K, 5120), (synth.Q3_K, 2304)])
+def test_ragged_rows_of_groups(cuda, wt, n_in):
+    """Three matrices of eight phases still have a tensor map each, four are copied row by row; pairs; a group as Backend sends it."""
+    import torch
+    x = dev(synth.activations(1, n_in, SEED))[0]
+    for sizes in ((2080, 416, 417), (300, 5, 33, 1000), (9,)):
+        ws = [dev(synth.weights(wt, n, n_in, SEED + 9 + i, stream=wt)) for i, n in enumerate(sizes)]
+        got = cuda.gemv_group([x] * len(sizes), ws, [wt] * len(sizes), list(sizes), n_in)
+        for n, w, y in zip(sizes, ws, got):
+            w64 = cuda.dequant_rows(w, wt, n, n_in).double()
+            assert ((y.double() - w64 @ x.double()).abs() <= 2e-6 * w64.norm(dim=1) * x.double().norm()).all()
+    for n in (33, 3000):
+        w, v = (dev(synth.weights(wt, n, n_in, SEED + 20 + i, stream=wt)) for i in range(2))
+        got = cuda.gemv_group([x, x], [w, v], [wt, wt], [n, n], n_in, fuse_silu_pair=True)[0].double()
+        g, u = (cuda.dequant_rows(m, wt, n, n_in).double() @ x.double() for m in (w, v))
+        want = g / (1.0 + torch.exp(-g)) * u
+        assert (got - want).norm() <= 2e-6 * want.norm()
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out", [4736, 4737, 5003])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
     """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
