@@ -61,7 +61,7 @@ constexpr int kConsumerThreads = kConsumerWarps * 32;
 __host__ __device__ constexpr int consumer_groups(int ng) { return ng == 1 ? 1 : 2; }
 __host__ __device__ constexpr int cta_threads(int groups) { return groups * kConsumerThreads + 64; }   // warp 0: producer, then the consumers, then the epilogue
 // Tiles whose partial sums may wait for the epilogue warp (fewer when more activation rows make a slot larger).
-__host__ __device__ constexpr int red_slots(int ng) { return ng == 1 ? 4 : ng == 2 ? 2 : 1; }   // of each consumer group
+__host__ __device__ constexpr int red_slots(int ng, int groups = 2) { return ng == 1 ? 4 / groups : ng == 2 ? 2 : 1; }   // of each consumer group
 constexpr int kMaxRedSlots = 4;
 constexpr int kMaxMaps = 24;      // of a launch: three matrices of ragged rows
 constexpr int kMaxStack = 4;      // 16-row tiles per stage at most
@@ -291,7 +291,7 @@ struct Smem {
     };
     float gate[kMaxStack][NG][32];   // epilogue warp: the gate tile(s) of a gate/up pair, until the up tile arrives
     // per consumer warp, column group and row pair (g, g+8): {row g x even activation row, g x odd, g+8 x even, g+8 x odd}
-    float4 red[GROUPS * red_slots(NG)][kConsumerWarps][NG][8];
+    float4 red[GROUPS * red_slots(NG, GROUPS)][kConsumerWarps][NG][8];
     float scale[NG == 1 ? 1 : kConsumerWarps][2 * NG];   // two groups: each prepared half of the activation rows, these are the scales
 };
 
@@ -477,7 +477,7 @@ __device__ __forceinline__ void walk(const StreamParams &p, const TableView &tv,
 }
 
 // ---- activation preparation -------------------------------------------------------------------------
-// Consumer warp w only ever multiplies K units w, w + 8, ... so it (of two groups, the warp w of one of them: each prepares every
+// Consumer warp w only ever multiplies K units w, w + WARPS, ... so it (of two groups, the warp w of one of them: each prepares every
 // other activation row) prepares exactly those slices of x. Per activation row: s = max|x| / (2^22 - 1) over the warp's slices,
 // X = rint(x / s) as three balanced s8 limbs (four where K is not a multiple of 256) written as byte planes (plane_at) in the
 // order the B fragments are read, and (formats with a minimum or an offset) the integer sum of X over every stretch of K that shares
@@ -637,7 +637,7 @@ constexpr bool kLoadsAhead = NG == 1 ? WT == KRK_CUDA_Q5_1 || ((WT == KRK_CUDA_Q
 // Every CTA prepares all of x, so this is bound by issue slots and by the latency of x: a maximum takes half an instruction a
 // value, a row's loads go out together (kHeld slices stay in registers between the maximum and the quantisation, K <= 4096;
 // further ones are read twice, kBatch at a time for the maximum).
-template <int WT, bool FINE, bool AHEAD, class RowFn, class ScaleFn>
+template <int WT, bool FINE, bool AHEAD, int WARPS, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
@@ -648,7 +648,7 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
     float held[kHeld][PER], next[AHEAD ? kHeld : 1][PER];
     auto load = [&](const float *xr, auto &f) {
 #pragma unroll
-        for (int j = 0; j < kHeld; j++) load_slice(xr, wid + j * kConsumerWarps, f[j]);
+        for (int j = 0; j < kHeld; j++) load_slice(xr, wid + j * WARPS, f[j]);
     };
     if (r0 >= rows || wid >= units) return;
     const float *xr = row(r0);
@@ -657,10 +657,10 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
     for (int r = r0; r < rows; r += step) {
         float mx = 0.0f;
 #pragma unroll 1
-        for (int u0 = wid + kHeld * kConsumerWarps; u0 < units; u0 += kBatch * kConsumerWarps) {
+        for (int u0 = wid + kHeld * WARPS; u0 < units; u0 += kBatch * WARPS) {
             float f[kBatch][PER];
 #pragma unroll
-            for (int j = 0; j < kBatch; j++) load_slice(xr, u0 + j * kConsumerWarps, f[j]);
+            for (int j = 0; j < kBatch; j++) load_slice(xr, u0 + j * WARPS, f[j]);
 #pragma unroll
             for (int j = 0; j < kBatch; j++) max_abs(mx, f[j]);
         }
@@ -698,16 +698,16 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         };
 #pragma unroll
         for (int j = 0; j < kHeld; j++) {
-            const int u = wid + j * kConsumerWarps;
+            const int u = wid + j * WARPS;
             if (u < units) quantize(held[j], u);
         }
-        int u = wid + kHeld * kConsumerWarps;
+        int u = wid + kHeld * WARPS;
         if (u < units) {
             float f[PER], g[PER];
             load_slice(xr, u, f);
 #pragma unroll 1
-            for (; u < units; u += kConsumerWarps) {
-                load_slice(xr, u + kConsumerWarps, g);
+            for (; u < units; u += WARPS) {
+                load_slice(xr, u + WARPS, g);
                 quantize(f, u);
 #pragma unroll
                 for (int j = 0; j < PER; j++) f[j] = g[j];
@@ -1560,6 +1560,9 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
 // 19.1 -> 20.0 us with it.)
 template <int WT>
 __host__ __device__ constexpr bool may_by_stage(bool ragged, int groups) { return WT == KRK_CUDA_Q6_K && ragged && groups == 2; }
+// The form of two groups for one and two activation rows: they always take a tile's stages in turn, and a warp prepares the units
+// that it multiplies, so no two warps share anything but a tile's sums.
+__host__ __device__ constexpr bool in_turn(int ng, int groups) { return ng == 1 && groups == 2; }
 // One result in f32 throughout, by one lane: what an infinity among the activations makes of a row (an infinity of either
 // sign, or a NaN against a zero weight) is not in the limbs, which give a NaN.
 template <int WT>
@@ -1579,7 +1582,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kGroups = GROUPS, kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
     constexpr bool kFine = RAG && !kSuper;   // fine_limbs
-    constexpr bool kMayByStage = may_by_stage<WT>(RAG, kGroups);
+    constexpr bool kInTurn = in_turn(NG, kGroups), kMayByStage = kInTurn || may_by_stage<WT>(RAG, kGroups);
+    constexpr int kUnitStep = kInTurn ? 2 * kConsumerWarps : kConsumerWarps;   // from a warp's K unit to its next
     constexpr bool kRagged = RAG || WT == KRK_CUDA_Q2_K;   // p.ragged may be set
     using F = Fmt<WT>;
     using SmemT = Smem<NG, GROUPS>;
@@ -1609,7 +1613,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     if (warp == 0) {
         // ===== producer warp: weights only, so it can run ahead of everything else =====
         // (a lane per barrier)
-        static_assert(kMaxStages == 8 && kGroups * red_slots(NG) <= kMaxRedSlots && kMaxRedSlots == 4, "24 lanes");
+        static_assert(kMaxStages == 8 && kGroups * red_slots(NG, kGroups) <= kMaxRedSlots && kMaxRedSlots == 4, "24 lanes");
         if (lane < 8) mbar_init(smem_u32(&sm->full[lane]), 1);
         else if (lane < 16) mbar_init(smem_u32(&sm->empty[lane - 8]), kGroups * kConsumerWarps);
         else if (lane < 20) mbar_init(smem_u32(&sm->red_empty[lane - 16]), 1);
@@ -1698,7 +1702,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         sync_start();
         // Output (row, activation row) of a tile is the sum, over the consumer warps in warp order, of the
         // share each warp left in `red` (already added up over the four lanes of a row group).
-        constexpr int kSlots = red_slots(NG);
+        constexpr int kSlots = red_slots(NG, kGroups);
         float gate_reg[NG];   // silu of the gate tile (stacked tiles keep theirs in shared memory)
         int tile_it = 0, n_out = 0;
         float *y0 = nullptr;
@@ -1708,7 +1712,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         }, [&](const StageInfo &s) {
             if (!s.last) return;
             // (two groups take the tiles in turn, each through slots of its own)
-            const bool both = kMayByStage && p.by_stage;   // (a tile's sums come from both, through a slot of each)
+            const bool both = kMayByStage && (kInTurn || p.by_stage);   // (a tile's sums come from both, through a slot of each)
             const int nth = both ? tile_it : tile_it / kGroups, slot = (both ? 0 : (tile_it % kGroups) * kSlots) + nth % kSlots;
             wait_phase(smem_u32(&sm->red_full[slot]), (nth / kSlots) & 1, gave_up, p.status);
             if (both) wait_phase(smem_u32(&sm->red_full[slot + kSlots]), (nth / kSlots) & 1, gave_up, p.status);
@@ -1860,26 +1864,26 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
         const bool picked = !SINGLE && p.table_rows;
         const int my_row = picked && lane < p.rows ? p.table_rows[e * p.rows + lane] : lane;
         if (x != prepared || (picked && __any_sync(0xFFFFFFFFu, my_row != prepared_row))) {
+            const int first_unit = stacked_idle ? p.units : my_unit + (kInTurn ? kConsumerWarps * grp : 0);
             // x may be the output of the kernel before this one (and y its input): wait for that grid to
             // complete. Weights are never written by a kernel in flight, so the producer warp does not wait.
             if (prepared == nullptr) {
                 // (x to level 2 meanwhile, where it is coherent whoever still writes it: a lane per 128-byte line of the warp's slices)
                 constexpr int kLines = F::unit_values / 32;
                 if (!p.dev_table)   // (a table's launch has waited)
-                    for (int r = grp; r < (SINGLE ? 1 : p.rows); r += kGroups)
-                        for (int l = lane; my_unit + l / kLines * kConsumerWarps < p.units; l += 32) {
-                            const int k = (my_unit + l / kLines * kConsumerWarps) * F::unit_values + l % kLines * 32;
+                    for (int r = kInTurn ? 0 : grp; r < (SINGLE ? 1 : p.rows); r += kInTurn ? 1 : kGroups)
+                        for (int l = lane; first_unit + l / kLines * kUnitStep < p.units; l += 32) {
+                            const int k = (first_unit + l / kLines * kUnitStep) * F::unit_values + l % kLines * 32;
                             if (!kFine || k < p.n_in) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (size_t)r * p.n_in + k));
                         }
                 asm volatile("griddepcontrol.wait;" ::: "memory");
             }
             // (stacked tiles: every sub-tile prepares its own copy)
             auto row = [&](int r) { return x + (SINGLE ? (size_t)0 : (size_t)__shfl_sync(0xFFFFFFFFu, my_row, r) * p.n_in); };
-            const int first_unit = stacked_idle ? p.units : my_unit;
-            if (kGroups == 1) {
+            if (kGroups == 1 || kInTurn) {   // every warp prepares what it reads itself
 #pragma unroll
                 for (int r = 0; r < 2 * NG; r++) xs[r] = 0.0f;
-                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>, kUnitStep>(row, [&](int r, float v) {
 #pragma unroll
                     for (int q = 0; q < 2 * NG; q++) xs[q] = q == r ? v : xs[q];
                 }, 0, 1, SINGLE ? 1 : p.rows, p, planes, chunk_sum, first_unit, lane);
@@ -1888,7 +1892,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             } else {
                 // each group prepares every other row; nobody may still read the activation before this one
                 if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
-                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>, kConsumerWarps>(row, [&](int r, float v) {
                     if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = v;
                 }, grp, kGroups, p.rows, p, planes, chunk_sum, first_unit, lane);
                 if (!synced) sync_start();
@@ -1933,7 +1937,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     phase ^= 1;
                 }
             };
-            const bool by_stage = kMayByStage && p.by_stage;
+            const bool by_stage = kMayByStage && (kInTurn || p.by_stage);
             if (kGroups == 2 && !by_stage && tile_it % 2 != grp) {
                 tile_it++;
                 for (int ck = 0; ck < n_chunks; ck++) pass();
@@ -2013,7 +2017,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             }
             {
              // ---- end of the tile: the lanes of a row group add their weighted shares ----
-             constexpr int kSlots = red_slots(NG);
+             constexpr int kSlots = red_slots(NG, kGroups);
              const int nth = by_stage ? tile_it : tile_it / kGroups, rslot = grp * kSlots + nth % kSlots;
              const uint32_t rphase = (nth / kSlots) & 1;
              tile_it++;
@@ -2167,10 +2171,22 @@ bool stages_in_turn(const StreamParams &p, bool one_tile) {
 // Q3_K 22016 x 4096 18.4 -> 17.1, Q2_K 16.2 -> 14.8).
 __host__ __device__ constexpr int box_pitch(int bytes) { return align_up(bytes, 16) + (align_up(bytes, 16) / 16 % 2 == 0 ? 16 : 0); }
 
+// Whether one or two activation rows may go to two groups of consumer warps that take a tile's stages in turn (in_turn), one CTA
+// to an SM. They do where a half SM has no room for the ring (one group left an SM with eight warps: Q6_K 4096 x 11008 13.9 -> 12.8 us, Q8_0 at
+// two rows 15.6 -> 13.2), and where no CTA has a second tile and a tile has many stages (Q4_K 1024 x 8192 5.4 -> 4.1, 2048 x 11008 5.7 -> 4.9;
+// at 4608 values, two stages and a part of a third, 0.85 to 1.16 of the time, so from beyond 5120 on; up to 8192 not where tiles for
+// nearly all SMs would give up the next launch's early start, 2368 x 5632 1.00 to 1.06). Up to 4096 values, which the
+// vocabulary heads have, results keep the order of their sums, in which eight warps add their units one after the other.
+template <int WT>
+bool stages_halve(const StreamParams &p) {
+    return p.tps == 1 && !p.whole_tiles && p.units > kConsumerWarps && (p.n_in > 4096 || fine_limbs<WT>(p.n_in));
+}
+
 // Fills the fields that depend only on the format, the width and the activation row count.
 // Returns false when the streaming kernel does not address the shape.
 template <int WT>
-bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t *smem_out, bool want_tma = false, bool one_group = false) {
+bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t *smem_out, bool want_tma = false, bool one_group = false,
+                  bool whole_sm = false) {
     using F = Fmt<WT>;
     // K not a multiple of 256: whole 32-value blocks, rows copied the ragged way, the last unit short. (Below 256 values
     // there is little to stream, and the warp-per-row kernel serves.)
@@ -2250,8 +2266,8 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
-    const bool halves = p.groups == 1;
-    const int most = halves ? kMaxHalfStages : kMaxStages;
+    bool halves = p.groups == 1;
+    int most = halves ? kMaxHalfStages : kMaxStages;
     auto fixed_bytes = [&](int spread) {
         return align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows, spread));
     };
@@ -2263,6 +2279,11 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     // Chunk sums without bank conflicts take 128 bytes and more; a stage, or the half SM, is worth more than they are (Q2_K at five
     // rows of 8192: 41.5 us with seven stages, 41.7 with six).
     const int close = fixed_bytes(0), apart = fixed_bytes(1);
+    if (rows <= 2 && (whole_sm || !fits_half(close)) && stages_halve<WT>(p)) {
+        p.groups = 2;
+        halves = false;
+        most = kMaxStages;
+    }
     p.spread_sums = fits_half(apart) == fits_half(close) && depth(apart, fits_half(apart)) == depth(close, fits_half(close));
     const int fixed = p.spread_sums ? apart : close;
     p.n_stages = depth(fixed, fits_half(fixed));
@@ -2285,12 +2306,15 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
                 if (p.rows <= 4) return launch_one<WT, 2, true, 0, true>(p, grid, smem, st);
                 return launch_one<WT, 4, true, 0, true>(p, grid, smem, st);
             }
+            if (p.rows <= 2 && p.groups == 2) return launch_one<WT, 1, false, 0, true, 2>(p, grid, smem, st);
             if (p.rows <= 2) return launch_one<WT, 1, false, 0, true>(p, grid, smem, st);
             if (p.rows <= 4) return launch_one<WT, 2, false, 0, true>(p, grid, smem, st);
             return launch_one<WT, 4, false, 0, true>(p, grid, smem, st);
         }
     }
     if constexpr (WT == KRK_CUDA_Q4_0) {
+        if (p.rows <= 2 && p.groups == 2)
+            return p.rows == 1 ? launch_one<WT, 1, false, 1, false, 2>(p, grid, smem, st) : launch_one<WT, 1, false, 0, false, 2>(p, grid, smem, st);
         if (p.rows == 1) return p.tps > 1 ? launch_one<WT, 1, true, 1>(p, grid, smem, st) : launch_one<WT, 1, false, 1>(p, grid, smem, st);
         if (p.rows <= 2) return p.tps > 1 ? launch_one<WT, 1, true, 0>(p, grid, smem, st) : launch_one<WT, 1, false, 0>(p, grid, smem, st);
         if (p.rows <= 4) return p.tps > 1 ? launch_one<WT, 2, true, 0>(p, grid, smem, st) : launch_one<WT, 2, false, 0>(p, grid, smem, st);
@@ -2302,6 +2326,8 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
             if (p.rows <= 4) return launch_one<WT, 2, true, 0>(p, grid, smem, st);
             return launch_one<WT, 4, true, 0>(p, grid, smem, st);
         }
+        if (p.rows <= 2 && p.groups == 2)
+            return kQ4K && p.rows == 1 ? launch_one<WT, 1, false, kQ4K ? 1 : 0, false, 2>(p, grid, smem, st) : launch_one<WT, 1, false, 0, false, 2>(p, grid, smem, st);
         if (kQ4K && p.rows == 1 && !p.whole_tiles && p.units <= 2 * kConsumerWarps) return launch_one<WT, 1, false, kQ4K ? 2 : 0>(p, grid, smem, st);
         if (kQ4K && p.rows == 1) return launch_one<WT, 1, false, kQ4K ? 1 : 0>(p, grid, smem, st);
         if (p.rows <= 2) return launch_one<WT, 1, false, 0>(p, grid, smem, st);
@@ -2447,10 +2473,12 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     int64_t tiles = 0;
     for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
+    // A tile for an SM at most, of many stages: two groups, see stages_halve.
+    const bool whole_sm = rows <= 2 && n_in > 5120 && tiles <= (n_in >= 8192 ? sm_count() : sm_count() * 7 / 8);
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
     if (tma) {
-        if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
-        if (p.use_tma == 3 && !p.ragged && rows_apart<WT>(p, tiles, *smem)) tma = false;
+        if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true, false, whole_sm)) return false;
+        if (p.use_tma == 3 && !p.ragged && p.groups == 1 && rows_apart<WT>(p, tiles, *smem)) tma = false;
         if (tma && p.use_tma) {
             for (int m = 0; m < n_mat; m++) p.mat[m] = mats[m];
             if (!encode_maps<WT>(p, n_mat)) tma = false;   // a map cannot be encoded: set up again for row copies
@@ -2467,7 +2495,7 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
             if (tma && !setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
         }
     }
-    return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem);
+    return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem, false, false, whole_sm);
 }
 
 template <int WT>

@@ -197,6 +197,60 @@ def test_ragged_rows_of_groups(cuda, wt, n_in):
     assert cuda.device_status() == 0
 
 
+# One and two rows of many stages go to two groups of warps that take a tile's stages in turn: a tile for an SM at most beyond 5120
+# values (129 tiles up to 8192), and any number where half an SM has no room for the ring
+@pytest.mark.parametrize("wt", FORMATS)
+def test_one_and_two_rows_with_stages_in_turn(cuda, wt):
+    import torch
+    widths = (5152, 5376, 8192, 11008, 14336) if SCALES[wt][0] < 84 else (5376, 8192, 11008, 14336)
+    for n_in in widths:
+        for n_out in (5, 600, 2064, 2065, 2368, 2369, 4739):
+            w = dev(synth.weights(wt, n_out, n_in, SEED + 10, stream=wt))
+            w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+            for rows in (1, 2):
+                x = dev(synth.activations(rows, n_in, SEED + rows))
+                base = torch.randn((rows, n_out), device="cuda")
+                y = cuda.gemv(x, w, wt, n_out, n_in, out=base.clone(), accumulate=True)
+                lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
+                assert ((y.double() - base - x.double() @ w64.T).abs() <= lim).all(), (n_in, n_out, rows)
+    # groups of two activations, and gate/up pairs
+    n_in, sizes = 11008, (700, 33)
+    x, z = dev(synth.activations(2, n_in, SEED))
+    ws = [dev(synth.weights(wt, n, n_in, SEED + 11 + i, stream=wt)) for i, n in enumerate(sizes)]
+    for v, n, w, y in zip((x, z), sizes, ws, cuda.gemv_group([x, z], ws, [wt] * 2, list(sizes), n_in)):
+        w64 = cuda.dequant_rows(w, wt, n, n_in).double()
+        assert ((y.double() - w64 @ v.double()).abs() <= 2e-6 * w64.norm(dim=1) * v.double().norm()).all()
+    pair = [dev(synth.weights(wt, 900, n_in, SEED + 13 + i, stream=wt)) for i in range(2)]
+    got = cuda.gemv_group([x, x], pair, [wt, wt], [900, 900], n_in, fuse_silu_pair=True)[0].double()
+    g, u = (cuda.dequant_rows(m, wt, 900, n_in).double() @ x.double() for m in pair)
+    want = g / (1.0 + torch.exp(-g)) * u
+    assert (got - want).norm() <= 2e-6 * want.norm()
+    assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("wt", [synth.Q4_K, synth.Q6_K, synth.Q8_0])
+def test_routed_experts_of_wide_activations(cuda, wt):
+    """The same two groups behind a device-side table of matrices."""
+    import torch
+    n_embd, n_ff, n_exp = 14336, 256, 4
+    gate, up = (dev(synth.weights(wt, n_exp * n_ff, n_embd, SEED + 30 + i, stream=wt)) for i in range(2))
+    down = dev(synth.weights(wt, n_exp * n_embd, n_ff, SEED + 32, stream=wt))
+    bank = cuda.make_bank(gate, up, down, wt, wt, n_exp, 0, n_embd, n_ff)
+    G, U = (cuda.dequant_rows(m, wt, n_exp * n_ff, n_embd).double().view(n_exp, n_ff, n_embd) for m in (gate, up))
+    D = cuda.dequant_rows(down, wt, n_exp * n_embd, n_ff).double().view(n_exp, n_embd, n_ff)
+    for rows in (1, 2, 5):
+        x = dev(synth.activations(rows, n_embd, SEED + rows))
+        ids, wts = cuda.route(dev(synth.activations(rows, n_exp, SEED, stream=7)), 2)
+        y = cuda.moe_ffn(x, ids, wts, bank).double()
+        want = torch.zeros_like(y)
+        for r in range(rows):
+            for e, c in zip(ids[r].tolist(), wts[r].double()):
+                g, u = G[e] @ x[r].double(), U[e] @ x[r].double()
+                want[r] += c * (D[e] @ (g / (1.0 + torch.exp(-g)) * u))
+        assert (y - want).norm() <= 4e-6 * want.norm(), rows
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out", [4736, 4737, 5003])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
     """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
