@@ -33,6 +33,26 @@ static __global__ void __launch_bounds__(32) flag_wait_kernel(const int *flags, 
     __threadfence_system();
 }
 
+// Activation rows whose limbs leave no room for a ring, K a multiple of 256: half of them at a time, or half of those, with four
+// limbs, so that results are as exact as those of the warp-per-row kernel, which multiplies in f32 and had these shapes (error against f64
+// sums at 8 rows, K of 7424 to 14336: 0.9e-7 to 1.4e-7 here, 1.4e-7 to 1.6e-7 there; 22 bits 2.6e-7, and eight times that with outliers).
+// 4096 x 11264: Q4_K at six and eight rows 97 -> 30, 117 -> 51 us, Q6_K 101 -> 35, 122 -> 61; 16384 x 9984 at eight rows 404 -> 77, 425 -> 109.
+static int launch_parts(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, cudaStream_t st) {
+    int rc = 0;
+    if (rows <= 4) KRK_DISPATCH_WT(mats[0].wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, true, st));
+    if (rc != 0 || rows == 1) return rc;
+    GemvMat part[KRK_CUDA_MAX_GROUP];
+    for (int m = 0; m < n_mat; m++) part[m] = mats[m];
+    const int first = (rows + 1) / 2;
+    rc = launch_parts(part, n_mat, n_in, first, accumulate, silu_pair, st);
+    if (rc != 1) return rc;
+    for (int m = 0; m < n_mat; m++) {
+        part[m].x += first * n_in;
+        part[m].y += first * mats[m].n_out;
+    }
+    return launch_parts(part, n_mat, n_in, rows - first, accumulate, silu_pair, st);
+}
+
 int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair,
                        cudaStream_t st) {
     if (n_mat < 1 || rows < 1 || rows > KRK_CUDA_MAX_ROWS) return 0;
@@ -49,7 +69,9 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
     const bool odd_k = n_in % 256 != 0, few_rows = out < 8 * sm_count();
     if (odd_k && out >= 512 && (n_in < 1024 || (wt == KRK_CUDA_Q5_1 && n_in < 2048 && few_rows))) return 0;
     int rc = 0;
-    KRK_DISPATCH_WT(wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, st));
+    KRK_DISPATCH_WT(wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, false, st));
+    // (few rows of Q5_1, whose units are the longest: 256 x 11264 at six rows 43.8 and 45.9 us)
+    if (rc == 0 && rows > 1 && !odd_k && n_mat <= KRK_CUDA_MAX_GROUP && (wt != KRK_CUDA_Q5_1 || out >= 512)) return launch_parts(mats, n_mat, n_in, rows, accumulate, silu_pair, st);
     // Activation rows whose four limbs leave no room for a ring go in two launches: the weights twice through the ring are
     // quicker than the warp-per-row kernel once (8 rows of K = 11232, 2048 weight rows: Q8_0 50 against 81 us, Q5_1 70 against
     // 75), but for matrices that do not fill the SMs with rows in the formats with the longer units (512 weight rows: Q4_0

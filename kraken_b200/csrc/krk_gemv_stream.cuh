@@ -299,7 +299,8 @@ __host__ __device__ constexpr int align_up(int v, int a) { return (v + a - 1) / 
 
 // Limbs of an activation: three, or four where K is not a multiple of 256. Those shapes belong to the warp-per-row kernel
 // otherwise, which multiplies in f32; 22 bits against the largest magnitude of a warp's slices are 2 to 9 times as far off
-// (error against f64 of 2.3e-7 to 1.1e-6, f32: 1.2e-7), and the MMA's fourth column was unused.
+// (error against f64 of 2.3e-7 to 1.1e-6, f32: 1.2e-7), and the MMA's fourth column was unused. (`wide` below: shapes with K a
+// multiple of 256 that would belong to that kernel too, see launch_parts.)
 template <int WT>
 __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) == 32 && n_in % 256 != 0; }
 // Where the planes lie, so that at up to four rows the eight columns of a B fragment (column_of) are read from different banks, in
@@ -314,19 +315,19 @@ __host__ __device__ constexpr bool fine_limbs(int n_in) { return block_size(WT) 
 template <int WT>
 constexpr bool kWidePlanes = WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K;
 template <int WT>
-__host__ __device__ inline int plane_pitch(int n_in, int rows) {
-    return n_in + (kWidePlanes<WT> || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1 && !fine_limbs<WT>(n_in)) ? 32 : 16);
+__host__ __device__ inline int plane_pitch(int n_in, int rows, bool wide = false) {
+    return n_in + (kWidePlanes<WT> || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q5_1 || (WT == KRK_CUDA_Q4_0 && rows == 1 && !wide && !fine_limbs<WT>(n_in)) ? 32 : 16);
 }
 // Byte offset of a limb plane of activation row r of `rows`.
 template <int WT>
-__host__ __device__ inline int plane_at(int n_in, int rows, int r, int limb) {
-    const int pitch = plane_pitch<WT>(n_in, rows);
-    if (kWidePlanes<WT> && rows > 2) return (limb < 2 ? 2 * r + limb : 2 * rows + r) * pitch;
-    return r * ((fine_limbs<WT>(n_in) ? 4 : 3) * pitch + (block_size(WT) == 256 && !kWidePlanes<WT> && rows > 2 ? 48 : 0)) + limb * pitch;
+__host__ __device__ inline int plane_at(int n_in, int rows, int r, int limb, bool wide = false) {
+    const int pitch = plane_pitch<WT>(n_in, rows, wide);
+    if (kWidePlanes<WT> && rows > 2) return (limb < 2 ? 2 * r + limb : limb * rows + r) * pitch;
+    return r * ((wide || fine_limbs<WT>(n_in) ? 4 : 3) * pitch + (block_size(WT) == 256 && !kWidePlanes<WT> && rows > 2 ? 48 : 0)) + limb * pitch;
 }
 template <int WT>
-__host__ __device__ inline int plane_bytes(int n_in, int rows) {
-    return align_up(kWidePlanes<WT> ? 3 * rows * plane_pitch<WT>(n_in, rows) : plane_at<WT>(n_in, rows, rows, 0), 128);
+__host__ __device__ inline int plane_bytes(int n_in, int rows, bool wide = false) {
+    return align_up(kWidePlanes<WT> ? (wide ? 4 : 3) * rows * plane_pitch<WT>(n_in, rows, wide) : plane_at<WT>(n_in, rows, rows, 0, wide), 128);
 }
 // Sums of the quantised activation over the stretch of K that shares one minimum or offset: 32 values (2^5) for
 // Q4_K, Q5_K, Q4_0 and Q5_1, 16 for Q2_K.
@@ -572,8 +573,8 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
 // address). x * inv is exact (inv is a power of two): 22 bits and, in units of 2^-8, what they leave.
 // `live`: the lane's values lie inside the row (the last unit of such a row may be short).
 template <int WT>
-__device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p, int ps,
-                                                    int8_t *sums, int lane, bool live) {
+__device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p01, int8_t *p23, int ps0, int ps2,
+                                                    int8_t *sums, int n_chunks, int lane, bool live) {
     constexpr int PER = Fmt<WT>::unit_values / 32;
     int total = 0, rest = 0;
 #pragma unroll
@@ -591,11 +592,11 @@ __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::un
         const uint32_t lo01 = __byte_perm(z[0], z[1], 0x5140), lo23 = __byte_perm(z[2], z[3], 0x5140);   // l3 l3 l2 l2
         const uint32_t hi01 = __byte_perm(z[0], z[1], 0x7362), hi23 = __byte_perm(z[2], z[3], 0x7362);   // l1 l1 l0 l0
         if (live) {
-            int8_t *at = p + k0 + j4;
-            *reinterpret_cast<uint32_t *>(at) = __byte_perm(hi01, hi23, 0x7632);
-            *reinterpret_cast<uint32_t *>(at + ps) = __byte_perm(hi01, hi23, 0x5410);
-            *reinterpret_cast<uint32_t *>(at + 2 * ps) = __byte_perm(lo01, lo23, 0x7632);
-            *reinterpret_cast<uint32_t *>(at + 3 * ps) = __byte_perm(lo01, lo23, 0x5410);
+            const int at = k0 + j4;
+            *reinterpret_cast<uint32_t *>(p01 + at) = __byte_perm(hi01, hi23, 0x7632);
+            *reinterpret_cast<uint32_t *>(p01 + ps0 + at) = __byte_perm(hi01, hi23, 0x5410);
+            *reinterpret_cast<uint32_t *>(p23 + at) = __byte_perm(lo01, lo23, 0x7632);
+            *reinterpret_cast<uint32_t *>(p23 + ps2 + at) = __byte_perm(lo01, lo23, 0x5410);
         }
     }
     if (WT == KRK_CUDA_Q5_1) {   // the sum over each 32-value block, see quantize_slice
@@ -605,6 +606,17 @@ __device__ __forceinline__ void quantize_slice_fine(const float (&f)[Fmt<WT>::un
             rest += __shfl_xor_sync(0xFFFFFFFFu, rest, o);
         }
         if ((lane & 3) == 0 && live) reinterpret_cast<float *>(sums)[k0 >> 5] = fmaf((float)rest, 0.00390625f, (float)total);
+    }
+    if (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q5_K || WT == KRK_CUDA_Q2_K) {   // see quantize_slice; in eighths (see add_min), |sum| <= 2^30
+        total = 8 * total + ((rest + 16) >> 5);
+        total += __shfl_xor_sync(0xFFFFFFFFu, total, 1);
+        if (WT != KRK_CUDA_Q2_K) total += __shfl_xor_sync(0xFFFFFFFFu, total, 2);
+        if ((lane & (WT == KRK_CUDA_Q2_K ? 1 : 3)) == 0) {
+            const int c = k0 >> kSumShift<WT>;
+            const uint32_t z = limbs4(total);
+#pragma unroll
+            for (int l = 0; l < 4; l++) sums[l * n_chunks + c] = (int8_t)(z >> (24 - 8 * l));
+        }
     }
 }
 
@@ -637,11 +649,13 @@ constexpr bool kLoadsAhead = NG == 1 ? WT == KRK_CUDA_Q5_1 || ((WT == KRK_CUDA_Q
 // Every CTA prepares all of x, so this is bound by issue slots and by the latency of x: a maximum takes half an instruction a
 // value, a row's loads go out together (kHeld slices stay in registers between the maximum and the quantisation, K <= 4096;
 // further ones are read twice, kBatch at a time for the maximum).
-template <int WT, bool FINE, bool AHEAD, int WARPS, class RowFn, class ScaleFn>
+template <int WT, bool FINE, bool WIDE, bool AHEAD, int WARPS, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
-    const int n_chunks = sum_pitch<WT>(p.n_in, p.spread_sums), ps = plane_pitch<WT>(p.n_in, p.rows), units = p.units;
+    const int n_chunks = sum_pitch<WT>(p.n_in, p.spread_sums), units = p.units;
+    constexpr bool wide = FINE || WIDE;
+    const int ps = plane_pitch<WT>(p.n_in, p.rows, wide);
     auto at = [&](int u) { return u * UV + lane * PER; };
     auto live = [&](int u) { return !FINE || at(u) < p.n_in; };
     auto load_slice = [&](const float *xr, int u, float (&f)[PER]) { load_values(xr + at(u), f, u < units && live(u)); };
@@ -675,7 +689,7 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         // non-finite activation makes the output NaN
         mx = __uint_as_float(mxb);
         float inv, s;
-        if constexpr (FINE) {   // the power of two that takes the maximum to 2^21 .. 2^22, 2^127 at most
+        if constexpr (FINE || WIDE) {   // the power of two that takes the maximum to 2^21 .. 2^22, 2^127 at most
             const uint32_t e = min(275u - (mxb >> 23), 254u);
             inv = __uint_as_float(e << 23);
             s = __uint_as_float(e < 254u ? (254u - e) << 23 : 0x00400000u);
@@ -691,9 +705,10 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
             inv = 0.0f;
             s = __int_as_float(0x7FC00000);
         }
-        int8_t *p0 = planes + plane_at<WT>(p.n_in, p.rows, r, 0), *p2 = planes + plane_at<WT>(p.n_in, p.rows, r, 2), *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
+        int8_t *p0 = planes + plane_at<WT>(p.n_in, p.rows, r, 0, wide), *p2 = planes + plane_at<WT>(p.n_in, p.rows, r, 2, wide), *sums = chunk_sum + (size_t)(r * 4) * n_chunks;
         auto quantize = [&](const float (&f)[PER], int u) {
-            if constexpr (FINE) quantize_slice_fine<WT>(f, inv, at(u), p0, ps, sums, lane, live(u));
+            if constexpr (FINE || WIDE)
+                quantize_slice_fine<WT>(f, inv, at(u), p0, p2, ps, plane_at<WT>(p.n_in, p.rows, r, 3, wide) - plane_at<WT>(p.n_in, p.rows, r, 2, wide), sums, n_chunks, lane, live(u));
             else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p2, sums, n_chunks, lane);
         };
 #pragma unroll
@@ -760,12 +775,14 @@ template <int NG>
 constexpr int kFoldGroups = NG == 4 ? 3 : NG;
 template <int NG>
 constexpr int kFoldRows = NG == 4 ? 2 : 1;   // activation rows a lane looks after
-template <int NG>
+// WIDE: four limbs, limb 3 (weight 1/256) in the column beside limb 2's, which nothing else uses up to four rows.
+template <int NG, bool WIDE = false>
 struct AccumFold {
+    static_assert(!WIDE || NG == 2, "limb 3 has a column at up to four rows");
     float a[kFoldRows<NG>][2];   // [row t, t + 4][weight row g, g + 8]
 };
-template <int NG>
-using AccumSuper = std::conditional_t<NG == 1, AccumPair, AccumFold<NG>>;
+template <int NG, bool WIDE = false>
+using AccumSuper = std::conditional_t<NG == 1, AccumPair, AccumFold<NG, WIDE>>;
 // acc += d * (limb sums of a unit), dA and dB the scales of weight rows g and g + 8
 __device__ __forceinline__ void add_unit(AccumPair &acc, float dA, float dB, const int (&I)[1][4]) {
     acc.f[0][0] = fmaf(dA, (float)I[0][0], acc.f[0][0]);
@@ -773,13 +790,13 @@ __device__ __forceinline__ void add_unit(AccumPair &acc, float dA, float dB, con
     acc.f[0][2] = fmaf(dB, (float)I[0][2], acc.f[0][2]);
     acc.f[0][3] = fmaf(dB, (float)I[0][3], acc.f[0][3]);
 }
-template <int NG>
-__device__ __forceinline__ void add_unit(AccumFold<NG> &acc, float dA, float dB, const int (&I)[NG][4]) {
+template <int NG, bool WIDE>
+__device__ __forceinline__ void add_unit(AccumFold<NG, WIDE> &acc, float dA, float dB, const int (&I)[NG][4]) {
 #pragma unroll
     for (int h = 0; h < kFoldRows<NG>; h++) {
         constexpr int L = kFoldGroups<NG> - 1;
-        acc.a[h][0] = fmaf(dA, fmaf(65536.0f, (float)I[h][0], fmaf(256.0f, (float)I[h][1], (float)I[L][h])), acc.a[h][0]);
-        acc.a[h][1] = fmaf(dB, fmaf(65536.0f, (float)I[h][2], fmaf(256.0f, (float)I[h][3], (float)I[L][2 + h])), acc.a[h][1]);
+        acc.a[h][0] = fmaf(dA, fmaf(65536.0f, (float)I[h][0], fmaf(256.0f, (float)I[h][1], WIDE ? fmaf(0.00390625f, (float)I[L][1], (float)I[L][0]) : (float)I[L][h])), acc.a[h][0]);
+        acc.a[h][1] = fmaf(dB, fmaf(65536.0f, (float)I[h][2], fmaf(256.0f, (float)I[h][3], WIDE ? fmaf(0.00390625f, (float)I[L][3], (float)I[L][2]) : (float)I[L][2 + h])), acc.a[h][1]);
     }
 }
 // the minimum term: dmin * (minimums times group mg of the chunk sums)
@@ -789,10 +806,11 @@ __device__ __forceinline__ void add_min(AccumPair &acc, float nA, float nB, cons
     acc.m[2] = fmaf(nB, (float)c[2], acc.m[2]);
     acc.m[3] = fmaf(nB, (float)c[3], acc.m[3]);
 }
-template <int NG>
-__device__ __forceinline__ void add_min(AccumFold<NG> &acc, float nA, float nB, const int (&c)[4], int mg) {
+template <int NG, bool WIDE>
+__device__ __forceinline__ void add_min(AccumFold<NG, WIDE> &acc, float nA, float nB, const int (&c)[4], int mg) {
     const bool low = mg & 1;   // limbs 2 and 3 (weights 2^8, 1), else 0 and 1 (2^24, 2^16)
-    const float w0 = low ? -256.0f : -16777216.0f, w1 = low ? -1.0f : -65536.0f;
+    constexpr float kUnit = WIDE ? 0.125f : 1.0f;
+    const float w0 = kUnit * (low ? -256.0f : -16777216.0f), w1 = kUnit * (low ? -1.0f : -65536.0f);
     const int h = NG == 4 ? mg >> 1 : 0;
     acc.a[h][0] = fmaf(nA, fmaf(w0, (float)c[0], w1 * (float)c[1]), acc.a[h][0]);
     acc.a[h][1] = fmaf(nB, fmaf(w0, (float)c[2], w1 * (float)c[3]), acc.a[h][1]);
@@ -808,8 +826,8 @@ __device__ __forceinline__ void accum_zero(AccumPair &a) {
 #pragma unroll
     for (int j = 0; j < 4; j++) a.f[0][j] = a.m[j] = 0.0f;
 }
-template <int NG>
-__device__ __forceinline__ void accum_zero(AccumFold<NG> &a) {
+template <int NG, bool WIDE>
+__device__ __forceinline__ void accum_zero(AccumFold<NG, WIDE> &a) {
 #pragma unroll
     for (int i = 0; i < kFoldRows<NG>; i++) a.a[i][0] = a.a[i][1] = 0.0f;
 }
@@ -829,8 +847,8 @@ __device__ __forceinline__ uint32_t bits_of(const Accum<NG> &a) {
     return b;
 }
 __device__ __forceinline__ uint32_t bits_of(const AccumPair &a) { return bits_of(a.f[0]) ^ bits_of(a.m); }
-template <int NG>
-__device__ __forceinline__ uint32_t bits_of(const AccumFold<NG> &a) {
+template <int NG, bool WIDE>
+__device__ __forceinline__ uint32_t bits_of(const AccumFold<NG, WIDE> &a) {
     uint32_t b = 0u;
 #pragma unroll
     for (int i = 0; i < kFoldRows<NG>; i++) b ^= bits_of(a.a[i]);
@@ -845,13 +863,13 @@ template <int NG, bool FOLD, bool FINE>
 __host__ __device__ __forceinline__ Column column_of(int mg, int g) {
     // (columns 6 and 7, which carry nothing, read what columns 4 and 5 do)
     Column c{2 * mg + (g >= 6 ? 1 : g / 3), g >= 6 ? g - 5 : g % 3, 2 * mg + g / 4, g % 4};
-    if (FINE) {
+    if (FINE && !FOLD) {
         c.row = 2 * mg + (g >> 2);
         c.limb = g & 3;
     } else if (FOLD) {   // see AccumFold
         const bool last = mg >= kFoldGroups<NG> - 1;
         c.row = (g >> 1) + (last ? (NG == 4 ? 4 * (g & 1) : 0) : 4 * mg);
-        c.limb = last ? 2 : g & 1;
+        c.limb = last ? (FINE ? 2 + (g & 1) : 2) : g & 1;
         c.sum_row = (g >> 1) + 4 * (mg >> 1);
         c.sum_limb = 2 * (mg & 1) + (g & 1);
     } else if (NG == 4 && g >= 6) {   // the spare columns: limb mg of activation row 6 or 7 (group 3 multiplies nothing)
@@ -865,20 +883,20 @@ __host__ __device__ __forceinline__ Column column_of(int mg, int g) {
 // accumulator columns are never looked at, so what it multiplies does not matter.
 template <int WT, int NG, bool FOLD, bool FINE>
 __device__ __forceinline__ void lane_planes(const int8_t *planes, const int8_t *chunk_sum, int n_in, int n_sums, int rows, int g,
-                                            const int8_t *(&bp)[NG], const int8_t *(&sp)[NG]) {
+                                            const int8_t *(&bp)[NG], const int8_t *(&sp)[NG], bool wide) {
 #pragma unroll
     for (int mg = 0; mg < NG; mg++) {
         const Column c = column_of<NG, FOLD, FINE>(mg, g);
-        bp[mg] = planes + plane_at<WT>(n_in, rows, min(c.row, rows - 1), c.limb);
+        bp[mg] = planes + plane_at<WT>(n_in, rows, min(c.row, rows - 1), c.limb, wide);
         sp[mg] = chunk_sum + (size_t)(min(c.sum_row, rows - 1) * 4 + c.sum_limb) * n_sums;
     }
 }
 
 // FIFTH: the Q5_K super-block: 32 bytes after the header whose bit c is the fifth quant bit of chunk c's value at the
 // same position; the nibbles follow them.
-template <int NG, bool FIFTH>
+template <int NG, bool FIFTH, class Acc>
 __device__ __forceinline__ void unit_q4_k(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, AccumSuper<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, Acc &acc) {
     constexpr int kQs = FIFTH ? 48 : 16;
     const uint4 hA = *reinterpret_cast<const uint4 *>(rowA);
     const uint4 hB = *reinterpret_cast<const uint4 *>(rowB);
@@ -1366,9 +1384,9 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
 // Four integer instructions per four quants against six for assembling q and then centring it; the factor 4
 // leaves with the block scale.
 
-template <int NG, int BY2>
+template <int NG, int BY2, class Acc>
 __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, AccumSuper<NG> &acc) {
+                                          int t, Acc &acc) {
     const Words<BY2> wA(blkA), wB(blkB);
     int I[NG][4];
 #pragma unroll
@@ -1426,9 +1444,9 @@ __device__ __forceinline__ void unit_q6_k(const uint8_t *blkA, const uint8_t *bl
 // G = 8n + 2j + s takes bits 2j, 2j+1 of quant bytes 32n + 16s ..+15: one shift and one AND per four quants, one
 // k16 MMA per group. The minimums go through one more MMA per super-block, the 16 of them against the group
 // sums of X (acc.m, as for Q4_K).
-template <int NG>
+template <int NG, class Acc>
 __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          const int8_t *const (&sp)[NG], int t, AccumSuper<NG> &acc) {
+                                          const int8_t *const (&sp)[NG], int t, Acc &acc) {
     const uint32_t *wa = reinterpret_cast<const uint32_t *>(blkA), *wb = reinterpret_cast<const uint32_t *>(blkB);
     uint32_t scA[4], scB[4];
 #pragma unroll
@@ -1479,9 +1497,9 @@ __device__ __forceinline__ void unit_q2_k(const uint8_t *blkA, const uint8_t *bl
 // mask bit: q2 at bits 5-6 and the inverted mask bit at bit 7 (a 3-bit two's complement at the top of the byte),
 // two shifts, an AND and an AND-OR per four quants; the 32 leaves with d. Blocks are 110 bytes: every other one is
 // 2 bytes off a word boundary.
-template <int NG, int BY2>
+template <int NG, int BY2, class Acc>
 __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *blkB, int kbase, const int8_t *const (&bp)[NG],
-                                          int t, AccumSuper<NG> &acc) {
+                                          int t, Acc &acc) {
     const Words<BY2> wA(blkA), wB(blkB);
     uint32_t SA[4], SB[4];
     {
@@ -1572,7 +1590,7 @@ __device__ __noinline__ float dot_f32(const uint8_t *w, const float *x, int n_in
     return sum;
 }
 
-template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG)>
+template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG), bool WIDE = false>
 __global__ void __launch_bounds__(cta_threads(GROUPS), GROUPS == 1 ? 2 : 1)
 gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     // STACK: several 16-row tiles per stage (p.tps of them); compiled apart so that the usual one-tile
@@ -1581,7 +1599,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const int tps = STACK ? p.tps : 1;
     constexpr int kGroups = GROUPS, kThreads = cta_threads(kGroups), kEpilogueWarp = kGroups * kConsumerWarps + 1;
     constexpr bool kSuper = block_size(WT) == 256, kFold = kSuper && NG > 1;   // AccumSuper, AccumFold
-    constexpr bool kFine = RAG && !kSuper;   // fine_limbs
+    constexpr bool kFine = RAG && !kSuper;   // four limbs; in the super-block formats: WIDE
+    static_assert(!WIDE || kFold, "four limbs of a super-block format: the folded form");
     constexpr bool kInTurn = in_turn(NG, kGroups), kMayByStage = kInTurn || may_by_stage<WT>(RAG, kGroups);
     constexpr int kUnitStep = kInTurn ? 2 * kConsumerWarps : kConsumerWarps;   // from a warp's K unit to its next
     constexpr bool kRagged = RAG || WT == KRK_CUDA_Q2_K;   // p.ragged may be set
@@ -1592,7 +1611,8 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     int8_t *planes = reinterpret_cast<int8_t *>(smem_raw + align_up((int)sizeof(SmemT), 128));
     // one copy of the prepared activation per stacked sub-tile: the warps of a sub-tile move on to the next
     // matrix (and its activation) on their own, so they must not share planes with another sub-tile
-    int8_t *chunk_sum = planes + tps * plane_bytes<WT>(p.n_in, p.rows);
+    constexpr bool wide = kFine || WIDE;
+    int8_t *chunk_sum = planes + tps * plane_bytes<WT>(p.n_in, p.rows, wide);
     uint8_t *stages = reinterpret_cast<uint8_t *>(chunk_sum) + tps * chunk_sum_bytes<WT>(p.n_in, p.rows, p.spread_sums);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1740,9 +1760,9 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     }
                     const int srow = kTileRows * sub + row;   // row inside the stage
                     const int yrow = s.row0 + (kRagged && p.ragged ? srow * p.ragged : srow);
-                    if (kFine && v != v && r < p.rows && srow < s.n_rows) {
+                    if ((kFine || WIDE) && v != v && r < p.rows && srow < s.n_rows) {
                         const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
-                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)(s.row0 + srow * p.ragged) * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
+                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)yrow * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
                     }
                     if (r < p.rows) {
                         if (p.step == 2 && s.which == 0) {
@@ -1818,7 +1838,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const int8_t *bp[NG], *sp[NG];
     const float *fe[NG], *fo[NG];   // Q5_1: per-block sums of the even / odd activation row of each column group
     float xs[2 * NG];   // this warp's scale of each activation row (kFold: of its own rows, xs[0] and xs[1])
-    std::conditional_t<kSuper, AccumSuper<NG>, Accum<NG>> acc;
+    std::conditional_t<kSuper, AccumSuper<NG, WIDE>, Accum<NG>> acc;
     AccumSingle acs;
     accum_zero(acc);
     acs.f[0] = acs.f[1] = acs.m[0] = acs.m[1] = acs.m[2] = acs.m[3] = 0.0f;
@@ -1830,7 +1850,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     const bool stacked_idle = STACK && my_sub >= tps;
     const uint32_t lane_off = (uint32_t)(kTileRows * my_sub + g) * p.row_stride;
     if (!stacked_idle) {
-        planes += my_sub * plane_bytes<WT>(p.n_in, p.rows);
+        planes += my_sub * plane_bytes<WT>(p.n_in, p.rows, wide);
         chunk_sum += my_sub * chunk_sum_bytes<WT>(p.n_in, p.rows, p.spread_sums);
     }
     // single-row form: column g = limb g/2 of the low (g even) or high (g odd) chunk of a group
@@ -1883,7 +1903,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             if (kGroups == 1 || kInTurn) {   // every warp prepares what it reads itself
 #pragma unroll
                 for (int r = 0; r < 2 * NG; r++) xs[r] = 0.0f;
-                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>, kUnitStep>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, kUnitStep>(row, [&](int r, float v) {
 #pragma unroll
                     for (int q = 0; q < 2 * NG; q++) xs[q] = q == r ? v : xs[q];
                 }, 0, 1, SINGLE ? 1 : p.rows, p, planes, chunk_sum, first_unit, lane);
@@ -1892,7 +1912,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             } else {
                 // each group prepares every other row; nobody may still read the activation before this one
                 if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
-                prepare_x<WT, kFine, kLoadsAhead<WT, NG, RAG>, kConsumerWarps>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, kConsumerWarps>(row, [&](int r, float v) {
                     if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = v;
                 }, grp, kGroups, p.rows, p, planes, chunk_sum, first_unit, lane);
                 if (!synced) sync_start();
@@ -1907,7 +1927,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             if (NG == 4 || (RAG && kSuper && kGroups == 2)) accum_zero(acc);
             prepared = x;
             prepared_row = my_row;
-            if (!SINGLE) lane_planes<WT, NG, kFold, kFine>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.spread_sums), p.rows, g, bp, sp);
+            if (!SINGLE) lane_planes<WT, NG, kFold, kFine || WIDE>(planes, chunk_sum, p.n_in, sum_pitch<WT>(p.n_in, p.spread_sums), p.rows, g, bp, sp, wide);
             if (WT == KRK_CUDA_Q5_1) {
 #pragma unroll
                 for (int mg = 0; mg < NG; mg++) {   // per-block sums of the group's even and odd activation rows
@@ -2114,10 +2134,10 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     if (!synced) sync_start();   // (a CTA without work)
 }
 
-template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG)>
+template <int WT, int NG, bool STACK, int SINGLE, bool RAG = false, int GROUPS = consumer_groups(NG), bool WIDE = false>
 int launch_one(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     static bool configured[64] = {};   // per instantiation and device: the opt-in is sticky
-    auto kernel = gemv_stream_kernel<WT, NG, STACK, SINGLE, RAG, GROUPS>;
+    auto kernel = gemv_stream_kernel<WT, NG, STACK, SINGLE, RAG, GROUPS, WIDE>;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
@@ -2186,7 +2206,7 @@ bool stages_halve(const StreamParams &p) {
 // Returns false when the streaming kernel does not address the shape.
 template <int WT>
 bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t *smem_out, bool want_tma = false, bool one_group = false,
-                  bool whole_sm = false) {
+                  bool whole_sm = false, bool wide = false) {
     using F = Fmt<WT>;
     // K not a multiple of 256: whole 32-value blocks, rows copied the ragged way, the last unit short. (Below 256 values
     // there is little to stream, and the warp-per-row kernel serves.)
@@ -2196,7 +2216,8 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     p.units = (int)((n_in + F::unit_values - 1) / F::unit_values);
     p.row_bytes = (int)row_bytes(WT, n_in);
     p.rows = rows;
-    p.groups = rows <= 2 || one_group ? 1 : 2;
+    const bool pair = rows <= 2 && !(wide && block_size(WT) == 256);   // the form for two rows, not that for three and four
+    p.groups = pair || one_group ? 1 : 2;
     p.accumulate = 0;
     p.step = silu_pair ? 2 : 1;
     p.whole_tiles = 0;
@@ -2221,7 +2242,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     }
     // Q2_K rows are 16-byte multiples for K % 1024 == 0, Q3_K rows for K % 2048 == 0
     if ((WT == KRK_CUDA_Q2_K || WT == KRK_CUDA_Q3_K) && (p.row_bytes & 15) != 0) p.ragged = 1;
-    if (odd_k) p.ragged = 1;
+    if (odd_k || (wide && block_size(WT) == 32)) p.ragged = 1;   // (wide: for the form of four limbs, whose rows may be 16-byte multiples too)
     if (p.ragged) p.ragged = p.row_bytes & 2 ? 8 : p.row_bytes & 4 ? 4 : 2;
     const int ku_max = p.whole_tiles ? p.units : (p.units < kConsumerWarps ? p.units : kConsumerWarps);
     p.tps = kConsumerWarps / p.units;   // 0 when a tile has more units than there are consumer warps
@@ -2263,13 +2284,13 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
         p.row_stride = rows_stride;
         p.stage_bytes = align_up(kTileRows * p.tps * p.row_stride, 128);
     }
-    const int smem_struct = rows <= 2 ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
+    const int smem_struct = pair ? (int)sizeof(Smem<1>) : one_group ? (int)sizeof(Smem<2, 1>) : rows <= 4 ? (int)sizeof(Smem<2>) : (int)sizeof(Smem<4>);
     // Depth of the ring: as many stages as fit beside the prepared activation in half an SM, at most kMaxHalfStages. Wide
     // activations (large K) leave too little of a half; they, and the forms of two consumer groups, take the whole SM.
     bool halves = p.groups == 1;
     int most = halves ? kMaxHalfStages : kMaxStages;
     auto fixed_bytes = [&](int spread) {
-        return align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows) + chunk_sum_bytes<WT>(p.n_in, rows, spread));
+        return align_up(smem_struct, 128) + p.tps * (plane_bytes<WT>(p.n_in, rows, wide) + chunk_sum_bytes<WT>(p.n_in, rows, spread));
     };
     auto depth = [&](int fixed, bool half) {
         const int fit = ((half ? kSmemLimit : kSmemWhole) - fixed) / p.stage_bytes;
@@ -2279,7 +2300,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     // Chunk sums without bank conflicts take 128 bytes and more; a stage, or the half SM, is worth more than they are (Q2_K at five
     // rows of 8192: 41.5 us with seven stages, 41.7 with six).
     const int close = fixed_bytes(0), apart = fixed_bytes(1);
-    if (rows <= 2 && (whole_sm || !fits_half(close)) && stages_halve<WT>(p)) {
+    if (pair && (whole_sm || !fits_half(close)) && stages_halve<WT>(p)) {
         p.groups = 2;
         halves = false;
         most = kMaxStages;
@@ -2288,8 +2309,8 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     const int fixed = p.spread_sums ? apart : close;
     p.n_stages = depth(fixed, fits_half(fixed));
     // (a shape is taken if it would be with limb planes of n_in + 32 bytes and stages of row copies: beyond, the warp-per-row kernel multiplies in f32)
-    const int spread = align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
-    const int stage = p.ragged || F::tma == 3 ? align_up(kTileRows * p.tps * rows_stride, 128) : p.stage_bytes;
+    const int spread = wide ? 0 : align_up(rows * (fine_limbs<WT>(p.n_in) ? 4 : 3) * (p.n_in + 32), 128) - plane_bytes<WT>(p.n_in, rows);
+    const int stage = !wide && (p.ragged || F::tma == 3) ? align_up(kTileRows * p.tps * rows_stride, 128) : p.stage_bytes;
     if (p.n_stages < 2 || kSmemWhole - close - p.tps * spread < 2 * stage) return false;
     p.by_stage = stages_in_turn<WT>(p, false);
     *smem_out = (size_t)fixed + (size_t)p.n_stages * p.stage_bytes;
@@ -2338,6 +2359,20 @@ int launch_rows(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
     }
 }
 
+// Up to four rows of a super-block format with four limbs. 0: no such form.
+template <int WT>
+int launch_rows_wide(const StreamParams &p, int grid, size_t smem, cudaStream_t st) {
+    if (p.tps > 1 || p.rows > 4) return 0;
+    if constexpr (kRagForm<WT>) {
+        if (p.ragged) {
+            const int rc = launch_one<WT, 2, false, 0, true, 2, true>(p, grid, smem, st);
+            return rc == KRK_CUDA_OK ? 1 : rc;
+        }
+    }
+    const int rc = launch_one<WT, 2, false, 0, false, 2, true>(p, grid, smem, st);
+    return rc == KRK_CUDA_OK ? 1 : rc;
+}
+
 // CTAs of one launch per SM. 2 (default): both halves of an SM work on this launch (16 consumer warps per SM:
 // 0.80-0.83 of the copy bandwidth on large Q4_K / Q8_0 matrices against 0.5-0.7 with one). 1
 // (KRK_CUDA_GEMV_CTAS_PER_SM=1): the other half is left to the next launch in the stream, which becomes
@@ -2362,16 +2397,16 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
 struct MapKey {
     const void *w;
     int64_t n_out;
-    int row_bytes, unit_bytes, box_rows, box_units;
+    int row_bytes, unit_bytes, box_rows, box_units, ragged;
     bool operator==(const MapKey &o) const {
         return w == o.w && n_out == o.n_out && row_bytes == o.row_bytes && unit_bytes == o.unit_bytes &&
-               box_rows == o.box_rows && box_units == o.box_units;
+               box_rows == o.box_rows && box_units == o.box_units && ragged == o.ragged;
     }
 };
 struct MapKeyHash {
     size_t operator()(const MapKey &k) const {
         size_t h = reinterpret_cast<size_t>(k.w) * 0x9E3779B97F4A7C15ull;
-        h ^= (size_t)k.n_out * 0xC2B2AE3D27D4EB4Full + (size_t)k.row_bytes * 31 + (size_t)k.box_rows * 7 + (size_t)k.box_units;
+        h ^= (size_t)k.n_out * 0xC2B2AE3D27D4EB4Full + (size_t)k.row_bytes * 31 + (size_t)k.box_rows * 7 + (size_t)k.box_units + (size_t)k.ragged * 131;
         return h;
     }
 };
@@ -2400,7 +2435,7 @@ inline bool weight_maps(CUtensorMap *out, const uint8_t *w, int64_t n_out, int r
     const int n = ragged ? ragged : 1;
     static std::mutex mu;
     static std::unordered_map<MapKey, std::vector<CUtensorMap>, MapKeyHash> cache;
-    const MapKey key{w, n_out, row_bytes, unit_bytes, box_rows, mode == 1 ? box_units : -box_units};
+    const MapKey key{w, n_out, row_bytes, unit_bytes, box_rows, mode == 1 ? box_units : -box_units, ragged};
     std::lock_guard<std::mutex> lk(mu);
     auto it = cache.find(key);
     if (it != cache.end()) {
@@ -2469,7 +2504,7 @@ bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
 // setup_format with the tensor-copy layout where the format and the matrices allow it (the maps are encoded here),
 // else with per-row copies. False when the streaming kernel does not address the shape.
 template <int WT>
-bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in, int rows, int silu_pair, size_t *smem) {
+bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in, int rows, int silu_pair, size_t *smem, bool wide = false) {
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     int64_t tiles = 0;
     for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
@@ -2477,14 +2512,14 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     const bool whole_sm = rows <= 2 && n_in > 5120 && tiles <= (n_in >= 8192 ? sm_count() : sm_count() * 7 / 8);
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
     if (tma) {
-        if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true, false, whole_sm)) return false;
+        if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true, false, whole_sm, wide)) return false;
         if (p.use_tma == 3 && !p.ragged && p.groups == 1 && rows_apart<WT>(p, tiles, *smem)) tma = false;
         if (tma && p.use_tma) {
             for (int m = 0; m < n_mat; m++) p.mat[m] = mats[m];
             if (!encode_maps<WT>(p, n_mat)) tma = false;   // a map cannot be encoded: set up again for row copies
         }
     }
-    if constexpr (WT == KRK_CUDA_Q8_0) {
+    if (WT == KRK_CUDA_Q8_0 && !wide) {
         // Three and four rows of Q8_0: a tile is four stages of 128-value units where the other formats have two, so two
         // groups hold the whole ring and the next tiles are not under way while these are multiplied. Where there are
         // tiles for two one-group CTAs per SM, and a half has room for them, those stream (one group against two, four rows:
@@ -2495,14 +2530,14 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
             if (tma && !setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
         }
     }
-    return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem, false, false, whole_sm);
+    return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem, false, false, whole_sm, wide);
 }
 
 template <int WT>
-int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, cudaStream_t st) {
+int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, bool wide, cudaStream_t st) {
     StreamParams p;
     size_t smem = 0;
-    if (!setup_launch<WT>(p, mats, n_mat, n_in, rows, silu_pair, &smem)) return 0;
+    if (!setup_launch<WT>(p, mats, n_mat, n_in, rows, silu_pair, &smem, wide)) return 0;
     p.accumulate = accumulate;
     p.n_entries = 0;
     int total = 0, tiles = 0;
@@ -2541,6 +2576,8 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     const int grid = total < sms ? total : sms;
     p.gran_q = total / grid;
     p.gran_r = total % grid;
+    if constexpr (block_size(WT) == 256)
+        if (wide) return launch_rows_wide<WT>(p, grid, smem, st);
     const int rc = launch_rows<WT>(p, grid, smem, st);
     return rc == KRK_CUDA_OK ? 1 : rc;
 }
@@ -2614,7 +2651,7 @@ bool takes_fmt(int64_t n_in, int rows) {
 }
 
 #define KRK_STREAM_FORMAT(LINKAGE, WT)                                                                                                  \
-    LINKAGE template int launch_fmt<WT>(const GemvMat *, int, int64_t, int, int, int, cudaStream_t);                                    \
+    LINKAGE template int launch_fmt<WT>(const GemvMat *, int, int64_t, int, int, int, bool, cudaStream_t);                                    \
     LINKAGE template int launch_table_fmt<WT>(const StreamTable *, const int32_t *, int64_t, int64_t, int, int, const StreamBanks *, cudaStream_t); \
     LINKAGE template int launch_peers_fmt<WT>(const GemvMat &, int64_t, int, const PeerScatter &, cudaStream_t);                        \
     LINKAGE template bool takes_fmt<WT>(int64_t, int);

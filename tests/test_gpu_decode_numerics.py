@@ -251,6 +251,39 @@ def test_routed_experts_of_wide_activations(cuda, wt):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("outliers", [False, True])
+@pytest.mark.parametrize("wt", FORMATS)
+def test_rows_without_room_are_as_exact_as_f32(cuda, wt, outliers):
+    """K a multiple of 256 and so many activation rows that their limbs leave no room for a ring: parts of them, with four limbs. The
+    warp-per-row kernel, which such shapes took before, is 1.4e-7 to 1.64e-7 from the f64 sums over such inputs."""
+    import torch
+    for n_out, n_in in ((700, 14592), (33, 14336), (513, 16640), (530, 20480)):   # (no format has room for five rows)
+        w = dev(synth.weights(wt, n_out, n_in, SEED + 14, stream=wt))
+        w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+        for rows in (5, 6, 7, 8):
+            x = synth.activations(rows, n_in, SEED + rows)
+            if outliers:
+                x[:, 5::97] *= 300.0
+            x = dev(x)
+            base = torch.zeros((rows, n_out), device="cuda")
+            y = cuda.gemv(x, w, wt, n_out, n_in, out=base, accumulate=True)
+            want = x.double() @ w64.T
+            err = ((y.double() - want).norm() / want.norm()).item()
+            assert err <= 1.64e-7, (n_in, rows, err)
+    # an infinite activation gives what f32 arithmetic gives, and only in its own row
+    n_out, n_in, rows = 40, 14336, 7
+    w = dev(synth.weights(wt, n_out, n_in, SEED + 15, stream=wt))
+    w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+    x = dev(synth.activations(rows, n_in, SEED))
+    x[3, 777], x[0, 5] = float("-inf"), float("nan")
+    want, got = x.double() @ w64.T, cuda.gemv(x, w, wt, n_out, n_in)
+    assert torch.isinf(want[3]).any()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert (got[fine].double() - want[fine]).norm() <= 2e-7 * want[fine].norm()
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n_out", [4736, 4737, 5003])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
     """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
