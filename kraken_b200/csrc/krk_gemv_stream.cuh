@@ -493,10 +493,14 @@ __device__ __forceinline__ int sext8(int v) { return (v << 24) >> 24; }
 __device__ __forceinline__ uint32_t limbs3(int X) { return ((uint32_t)X + 0x00808080u) ^ 0x00808080u; }   // |X| < 2^23
 __device__ __forceinline__ uint32_t limbs4(int X) { return ((uint32_t)X + 0x80808080u) ^ 0x80808080u; }
 
-template <int WT>
+// OCTETS: a lane's eight values' limbs are stored together: 8 bytes a lane meet no bank twice, 4 do. Three and more rows (Q6_K 4096 x
+// 11008 at four rows 18.4 -> 18.0 us, Q4_K 15.2 -> 14.9); one row holds the first four longer and gains nothing (a Q4_K model's pass 1089 and 1093).
+template <int WT, bool OCTETS>
 __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_values / 32], float inv, int k0, int8_t *p0,
                                                int8_t *p1, int8_t *p2, int8_t *sums, int n_chunks, int lane) {
     constexpr int PER = Fmt<WT>::unit_values / 32;
+    constexpr bool kInOrder = !(WT == KRK_CUDA_Q8_0 || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_IQ4_NL);
+    uint32_t low[3];
     int total = 0;
 #pragma unroll
     for (int j4 = 0; j4 < PER; j4 += 4) {
@@ -513,7 +517,7 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
         const uint32_t w2 = __byte_perm(lo01, lo23, 0x5410) ^ 0x80808080u, w1 = __byte_perm(lo01, lo23, 0x7632) ^ 0x80808080u;
         const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], 0x0062), __byte_perm(z[2], z[3], 0x0062), 0x5410) ^ 0x80808080u;
         const int i = k0 + j4;
-        if (WT == KRK_CUDA_Q8_0 || WT == KRK_CUDA_Q5_0 || WT == KRK_CUDA_Q4_0 || WT == KRK_CUDA_IQ4_NL) {
+        if (!kInOrder) {
             // The blocks of these formats are an odd number of half words long: the quants of every other (even) block start 2
             // bytes off a word boundary, and their lanes take them in another order, which the limbs follow in pairs: pair
             // (e, e + 1) lands at ka, (e + 2, e + 3) at kb. (Odd blocks go the same way, e and e + 2: no lane branches.)
@@ -540,9 +544,18 @@ __device__ __forceinline__ void quantize_slice(const float (&f)[Fmt<WT>::unit_va
             *reinterpret_cast<uint16_t *>(p2 + base + ka) = (uint16_t)(w2 & 0xFFFF);
             *reinterpret_cast<uint16_t *>(p2 + base + kb) = (uint16_t)(w2 >> 16);
         } else {
-            *reinterpret_cast<uint32_t *>(p0 + i) = w0;
-            *reinterpret_cast<uint32_t *>(p1 + i) = w1;
-            *reinterpret_cast<uint32_t *>(p2 + i) = w2;
+            static_assert(!kInOrder || PER == 8, "two quads a lane");
+            if (!OCTETS) {
+                *reinterpret_cast<uint32_t *>(p0 + i) = w0;
+                *reinterpret_cast<uint32_t *>(p1 + i) = w1;
+                *reinterpret_cast<uint32_t *>(p2 + i) = w2;
+            } else if (j4 == 0) {
+                low[0] = w0, low[1] = w1, low[2] = w2;
+            } else {
+                *reinterpret_cast<uint2 *>(p0 + k0) = make_uint2(low[0], w0);
+                *reinterpret_cast<uint2 *>(p1 + k0) = make_uint2(low[1], w1);
+                *reinterpret_cast<uint2 *>(p2 + k0) = make_uint2(low[2], w2);
+            }
         }
     }
     total -= (int)((unsigned)PER * 0x4B400000u);   // the sum of X
@@ -649,7 +662,7 @@ constexpr bool kLoadsAhead = NG == 1 ? WT == KRK_CUDA_Q5_1 || ((WT == KRK_CUDA_Q
 // Every CTA prepares all of x, so this is bound by issue slots and by the latency of x: a maximum takes half an instruction a
 // value, a row's loads go out together (kHeld slices stay in registers between the maximum and the quantisation, K <= 4096;
 // further ones are read twice, kBatch at a time for the maximum).
-template <int WT, bool FINE, bool WIDE, bool AHEAD, int WARPS, class RowFn, class ScaleFn>
+template <int WT, bool FINE, bool WIDE, bool AHEAD, bool OCTETS, int WARPS, class RowFn, class ScaleFn>
 __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, int step, int rows, const StreamParams &p, int8_t *planes,
                                           int8_t *chunk_sum, int wid, int lane) {
     constexpr int UV = Fmt<WT>::unit_values, PER = UV / 32, kHeld = 16 / PER, kBatch = 32 / PER;
@@ -709,7 +722,7 @@ __device__ __forceinline__ void prepare_x(RowFn &&row, ScaleFn &&scale, int r0, 
         auto quantize = [&](const float (&f)[PER], int u) {
             if constexpr (FINE || WIDE)
                 quantize_slice_fine<WT>(f, inv, at(u), p0, p2, ps, plane_at<WT>(p.n_in, p.rows, r, 3, wide) - plane_at<WT>(p.n_in, p.rows, r, 2, wide), sums, n_chunks, lane, live(u));
-            else quantize_slice<WT>(f, inv, at(u), p0, p0 + ps, p2, sums, n_chunks, lane);
+            else quantize_slice<WT, OCTETS>(f, inv, at(u), p0, p0 + ps, p2, sums, n_chunks, lane);
         };
 #pragma unroll
         for (int j = 0; j < kHeld; j++) {
@@ -1903,7 +1916,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             if (kGroups == 1 || kInTurn) {   // every warp prepares what it reads itself
 #pragma unroll
                 for (int r = 0; r < 2 * NG; r++) xs[r] = 0.0f;
-                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, kUnitStep>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, (NG > 1), kUnitStep>(row, [&](int r, float v) {
 #pragma unroll
                     for (int q = 0; q < 2 * NG; q++) xs[q] = q == r ? v : xs[q];
                 }, 0, 1, SINGLE ? 1 : p.rows, p, planes, chunk_sum, first_unit, lane);
@@ -1912,7 +1925,7 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             } else {
                 // each group prepares every other row; nobody may still read the activation before this one
                 if (prepared != nullptr) asm volatile("bar.sync 2, %0;" ::"n"(kGroups * kConsumerThreads) : "memory");
-                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, kConsumerWarps>(row, [&](int r, float v) {
+                prepare_x<WT, kFine, WIDE, kLoadsAhead<WT, NG, RAG>, (NG > 1), kConsumerWarps>(row, [&](int r, float v) {
                     if (lane == 0) sm->scale[NG == 1 ? 0 : wid][r] = v;
                 }, grp, kGroups, p.rows, p, planes, chunk_sum, first_unit, lane);
                 if (!synced) sync_start();
