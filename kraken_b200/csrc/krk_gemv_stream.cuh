@@ -2574,14 +2574,16 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     const int sms = sm_count() * per_sm;
     // Tiles for more than half of the SMs but not for all: the rows are dealt to all of them, up to 16 each (a box brings some
     // that belong to the next CTA). Else the CTAs of the next launch, which find room beside these, go to the idle SMs two at a
-    // time and take twice as long there (Q6_K 2048 x 8192 8.5 -> 6.6 us, Q5_K 2048 x 8192 8.0 -> 6.4, Q4_K 2048 x 5632 4.8 -> 4.4). Not the
-    // forms that take a whole SM: there the idle SMs let the next launch start (four rows of 2048 x 5632 7.4 and 7.7).
+    // time and take twice as long there (Q6_K 2048 x 8192 8.5 -> 6.6 us, Q5_K 2048 x 8192 8.0 -> 6.4, Q4_K 2048 x 5632 4.8 -> 4.4). With several
+    // stages to a tile from two fifths on (1024 x 4096: Q4_K 0.94 of the time, Q5_K 0.89, Q6_K 0.91; 768 x 4096 1.03, 1.02, 1.08; of one
+    // stage, 1024 x 2048, 1.02, 0.95, 1.07). Not the forms that take a whole SM: there the idle SMs let the next launch start (four rows of
+    // 2048 x 5632 7.4 and 7.7).
     if ((p.use_tma || p.ragged) && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
         if (p.ragged) {   // (of four rows at least)
             const int least = (int)(mats[0].n_out / (4 * p.ragged)) * p.ragged;
             if (least >= sm_count()) p.gran_begin[1] = total = sm_count();
             else if (least > total) p.gran_begin[1] = total = least;
-        } else if (tiles > sm_count() / 2) {
+        } else if (tiles > sm_count() / 2 || (tiles > sm_count() * 2 / 5 && p.units > kConsumerWarps)) {
             p.gran = 1;
             p.gran_begin[1] = total = (int)mats[0].n_out;
         }
