@@ -42,6 +42,7 @@ constexpr int kTopkMaxK = 64;
 constexpr int kTopkSlice = 2048;        // keys of a block of the first kernel
 constexpr int kTopkPer = kTopkSlice / kTopkThreads;
 constexpr int kMergeThreads = 1024;
+constexpr int kRankBlocks = 512;         // lists up to which the second kernel ranks, see rank_select
 constexpr int kMergeHeld = 8192;        // candidates the second kernel keeps in shared memory
 
 struct TopkParams {
@@ -263,6 +264,77 @@ topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ 
     }
 }
 
+// By a whole block: the k best of n_blocks lists of k keys each, without radix passes. The best few of every list, k in all at
+// least, have a k-th largest, and k keys are not below that: what is below is out, and what is left, about twice k, is ranked key
+// against key (ties to the lower id). False, in every thread, where more are left than the block has threads: many equal keys.
+// (Candidates are all near the top, so that the radix select's first digits put them in one bin: 128,256 logits, k = 40, 16.0 -> 11.8
+// us with the first kernel, k = 64 18.0 -> 12.8, 32,000 logits k = 5 10.1 -> 7.4.)
+// Ranks of n distinct keys among each other, eight threads to a key: f(key, rank).
+template <class F>
+__device__ __forceinline__ void rank_keys(const unsigned long long *keys, int n, F &&f) {
+    const int part = threadIdx.x & 7;
+    for (int base = 0; base < n; base += kMergeThreads / 8) {
+        const int i = base + (int)(threadIdx.x >> 3);
+        const unsigned long long mine = keys[min(i, n - 1)];
+        int rank = 0;
+#pragma unroll 4
+        for (int q = part; q < n; q += 8) rank += keys[q] > mine;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) rank += __shfl_xor_sync(0xFFFFFFFFu, rank, o);
+        if (part == 0 && i < n) f(mine, rank);
+    }
+}
+template <class EachAt>
+__device__ __forceinline__ bool rank_select(EachAt &&each_at, const TopkParams &p, const uint32_t *__restrict__ cand_u, const int *__restrict__ cand_i,
+                                            int n_blocks, int32_t *__restrict__ ids, float *__restrict__ vals) {
+    static_assert(kTopkMaxK <= 64 && kRankBlocks + kTopkMaxK <= kMergeThreads, "two keys of a list a lane");
+    __shared__ unsigned long long keys[kMergeThreads];   // a key's order, then what is the greater the lower the index or the id
+    __shared__ uint32_t s_bound;
+    __shared__ int s_left;
+    const int tid = threadIdx.x, lane = tid & 31, k = p.k, each = (k + n_blocks - 1) / n_blocks;
+    if (tid == 0) s_left = 0;
+    for (int b = tid >> 5; b < n_blocks; b += kMergeThreads / 32) {
+        const uint32_t *list = cand_u + (size_t)b * k;
+        uint32_t u0 = lane < k ? list[lane] : 0u, u1 = lane + 32 < k ? list[lane + 32] : 0u;
+        for (int r = 0; r < each; r++) {
+            const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, max(u0, u1));
+            const bool first = lane == __ffs(__ballot_sync(0xFFFFFFFFu, u0 == most || u1 == most)) - 1;   // one of equals
+            const int at = b * each + r;
+            if (lane == 0) keys[at] = (unsigned long long)most << 32 | (uint32_t)~at;
+            if (first && u0 == most) u0 = 0u;
+            else if (first) u1 = 0u;
+        }
+    }
+    __syncthreads();
+    // (k of them at least, k + n_blocks - 1 at most)
+    rank_keys(keys, n_blocks * each, [&](unsigned long long key, int rank) {
+        if (rank == k - 1) s_bound = max((uint32_t)(key >> 32), 1u);   // (a zero is no key)
+    });
+    __syncthreads();
+    const uint32_t bound = s_bound;
+    each_at([&](uint32_t u, int64_t i) {
+        if (u >= bound) {
+            const int at = atomicAdd(&s_left, 1);
+            if (at < kMergeThreads) keys[at] = (unsigned long long)u << 32 | (uint32_t)~cand_i[i];
+        }
+    });
+    __syncthreads();
+    const int n = s_left;
+    if (n > kMergeThreads) return false;
+    rank_keys(keys, n, [&](unsigned long long key, int rank) {
+        if (rank < k) {
+            const int id = (int)~(uint32_t)key;
+            ids[rank] = id;
+            vals[rank] = topk_key(p, id);
+        }
+    });
+    if (tid >= n && tid < k) {   // fewer than k keys
+        ids[tid] = -1;
+        vals[tid] = -FLT_MAX;
+    }
+    return true;
+}
+
 template <SelectMode MODE>
 __global__ void __launch_bounds__(kMergeThreads)
 topk_merge_kernel(const __grid_constant__ TopkParams p, const uint32_t *__restrict__ cand_u, const int *__restrict__ cand_i,
@@ -294,6 +366,8 @@ topk_merge_kernel(const __grid_constant__ TopkParams p, const uint32_t *__restri
     auto each_at = [&](auto &&f) {
         for (int64_t i = tid; i < total; i += kMergeThreads) f(in_smem ? held[i] : cand_u[i], i);
     };
+    if constexpr (MODE != kGreatest)
+        if (n_blocks <= kRankBlocks && rank_select(each_at, p, cand_u, cand_i, n_blocks, ids, vals)) return;
     uint32_t threshold;
     int of_equals;
     radix_select<MODE>([&](auto &&f) { each_at([&](uint32_t u, int64_t) { f(u); }); }, k, threshold, of_equals);
