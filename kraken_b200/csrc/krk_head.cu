@@ -81,7 +81,7 @@ template <SelectMode MODE, class Each>
 __device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &threshold, int &of_equals) {
     __shared__ int hist[256];
     __shared__ uint32_t s_prefix;
-    __shared__ int s_left;
+    __shared__ int s_left, s_all;
     if constexpr (MODE == kGreatest) {
         uint32_t most = 0u;
         each([&](uint32_t u) { most = max(most, u); });
@@ -155,8 +155,13 @@ __device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &thres
                         above += c[q];
                         j++;
                     }
+                int in_bin = c[7];
+#pragma unroll
+                for (int q = 0; q < 7; q++)
+                    if (j == q) in_bin = c[q];
                 s_prefix = prefix | ((uint32_t)(255 - 8 * lane - j) << shift);
                 s_left = left - above;
+                s_all = in_bin == left - above;
             }
         }
         __syncthreads();
@@ -168,6 +173,13 @@ __device__ __forceinline__ void radix_select(Each &&each, int k, uint32_t &thres
         }
         prefix = s_prefix;
         mask |= 255u << shift;
+        // all of the bin belong to the k largest: the later digits do not matter (most slices, after two digits: 128,256 logits at
+        // k = 40 11.8 -> 11.1 us)
+        if (s_all && prefix != 0u && shift != 0) {
+            threshold = prefix - 1u;
+            of_equals = 0;
+            return;
+        }
     }
     threshold = prefix;
     of_equals = left;

@@ -172,3 +172,24 @@ def test_topk_of_a_few(cuda, n):
             assert np.array_equal(vals.cpu().numpy()[:m], key[order[:m]])
             assert (ids.cpu().numpy()[m:] == -1).all()
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 39, 2048, 2049, 6000, 128256, 1_100_000])
+def test_topk_of_lists_and_ties(cuda, n):
+    """The second kernel ranks what is left above a bound, and goes back to radix passes where more is left than it has threads
+    (many equal keys) or there are more lists than it takes (beyond 1,048,576 logits); a slice stops at the digit that decides."""
+    import torch
+    rng = np.random.default_rng(n)
+    normal = (rng.standard_normal(n) * 8).astype(np.float32)
+    few = rng.integers(0, 5, n).astype(np.float32)
+    rare = np.full(n, -np.inf, np.float32)
+    rare[rng.integers(0, n, 11)] = 3.0
+    near = (100.0 + np.arange(n) % 97 * 2.0 ** -17).astype(np.float32)   # keys that differ in their last digits only
+    for x in (normal, np.zeros(n, np.float32), few, rare, near, -np.abs(normal)):
+        order = np.lexsort((np.arange(n), -x.astype(np.float64)))
+        for k in (2, 7, 8, 40, 64):
+            got = cuda.logits_topk(torch.from_numpy(x[None]).cuda(), k, temp=0.8)
+            ids, vals = got[0].cpu().numpy().reshape(-1), got[1].cpu().numpy().reshape(-1)
+            m = min(n, k)
+            assert np.array_equal(ids[:m], order[:m]), (k, ids[:8], order[:8])
+            assert np.array_equal(vals[:m], x[order[:m]]) and (ids[m:] == -1).all()
