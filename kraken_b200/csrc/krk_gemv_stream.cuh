@@ -5,8 +5,8 @@
 // Design (B200-first, not the reference's one-warp-per-row walk of src/hip/kernels/gemm.hpp:76):
 //
 //  * One persistent CTA per SM owns a contiguous range of output rows. A producer warp streams
-//    that range through a ring of shared-memory stages with bulk-async copies (cp.async.bulk,
-//    one copy per weight row so that rows land on a padded, bank-conflict-free stride) signalled
+//    that range through a ring of shared-memory stages, one tensor copy a stage wherever a map can describe it (a copy takes 82
+//    clocks to issue whatever its size; else one bulk copy per weight row), laid out without bank conflicts and signalled
 //    on mbarriers; 8 consumer warps never touch global memory for weights. The ring keeps
 //    50-90 KB of HBM reads in flight per SM without spending registers on it.
 //
@@ -22,7 +22,7 @@
 //    the packed bytes (one AND per four nibbles) to mma.sync m16n8k32 / m16n8k16 (s8 x s8 -> s32),
 //    16 output rows at a time, and the activation is held as three signed 8-bit limbs of a
 //    23-bit fixed-point number (x ~ s * (l0*65536 + l1*256 + l2), |X| < 2^22), one limb per MMA column
-//    (four limbs where K is not a multiple of 256, see fine_limbs).
+//    (four limbs where K is not a multiple of 256, see fine_limbs, and where rows go in parts, see launch_parts).
 //    The products and sums are exact; the only rounding is the 23-bit quantisation of x
 //    (relative to max|x|, i.e. f32-mantissa sized) and the final f32 scale arithmetic, so the
 //    result sits well inside the 1e-4 * ||w_row|| * ||x|| bound. Sub-block scales are applied
@@ -91,9 +91,9 @@ template <> struct Fmt<KRK_CUDA_Q5_K> { static constexpr int unit_values = 256, 
 template <> struct Fmt<KRK_CUDA_Q4_0> { static constexpr int unit_values = 256, unit_bytes = 144, stride_mod = 16, tma = 1; };
 // Q5_0: eight 22-byte blocks are 176 bytes, the size of a Q5_K unit (rows of a fragment load 44 words apart: no
 // bank is met twice). Q5_1: eight 24-byte blocks are 192 bytes, a pitch that would put rows g and g + 2 on the
-// same banks, so its stages arrive as per-row copies with a padded pitch.
+// same banks, so its stages have a padded pitch.
 template <> struct Fmt<KRK_CUDA_Q5_0> { static constexpr int unit_values = 256, unit_bytes = 176, stride_mod = 16, tma = 1; };
-// Q2_K (84 bytes) and Q3_K (110 bytes): per-row copies; rows that are not 16-byte multiples go the ragged way.
+// Q2_K (84 bytes) and Q3_K (110 bytes): rows that are not 16-byte multiples go the ragged way.
 template <> struct Fmt<KRK_CUDA_Q2_K> { static constexpr int unit_values = 256, unit_bytes = 84, stride_mod = 16, tma = 3; };
 template <> struct Fmt<KRK_CUDA_Q3_K> { static constexpr int unit_values = 256, unit_bytes = 110, stride_mod = 16, tma = 3; };
 // IQ4_NL: Q4_0's block with grid indices in place of quants.
@@ -2245,7 +2245,7 @@ bool setup_format(StreamParams &p, int64_t n_in, int rows, int silu_pair, size_t
     if (WT == KRK_CUDA_Q6_K && (n_in % 2048) != 0) {
         // 210-byte blocks: rows are 16-byte multiples only for K % 2048 == 0. Otherwise whole 16-row
         // tiles are copied contiguously (needs 4-byte-multiple rows and the tile in one stage), or, for longer
-        // or odd rows (K = 11008: 9030 bytes), row by row from the 16-byte boundary below each row.
+        // or odd rows (K = 11008: 9030 bytes), rows that lie alike together, see TilePlace.
         if ((p.row_bytes & 3) == 0 && p.units <= 2 * kConsumerWarps) {
             p.whole_tiles = 1;
             p.gran = 8;
