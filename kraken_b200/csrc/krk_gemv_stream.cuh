@@ -2533,12 +2533,11 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
         }
     }
     if (WT == KRK_CUDA_Q8_0 && !wide) {
-        // Three and four rows of Q8_0: a tile is four stages of 128-value units where the other formats have two, so two
-        // groups hold the whole ring and the next tiles are not under way while these are multiplied. Where there are
-        // tiles for two one-group CTAs per SM, and a half has room for them, those stream (one group against two, four rows:
-        // 49152 x 4096 55.5 against 76.0 us, 11008 x 4096 18.8 against 20.6; 4096 x 4096 10.7 against 10.2, and 512 x 1024 5.8
-        // against 4.5).
-        if ((rows == 3 || rows == 4) && n_in % 256 == 0 && tiles > 2 * sm_count()) {
+        // Many tiles at three rows, or at three and four of one stage each (1024 values): one group and two CTAs per SM (three rows of 22016 x
+        // 4096 22.2 us against 22.9 with two groups; four of 32768 x 1024 12.6 against 14.4). Else two groups: 6144 x 4096 10.6 against 9.8,
+        // at four rows 11.6 against 10.0, 11008 x 4096 15.3 against 14.0, 22016 x 4096 23.4 against 23.0 (since a stage is one copy they no longer wait
+        // for the ring, of which a tile is four stages there).
+        if (n_in % 256 == 0 && ((rows == 3 && tiles > 6 * sm_count()) || ((rows == 3 || rows == 4) && n_in <= 1024 && tiles > 5 * sm_count()))) {
             if (setup_format<WT>(p, n_in, rows, silu_pair, smem, tma, true) && p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit) return true;
             if (tma && !setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
         }
