@@ -2515,12 +2515,14 @@ bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
 }
 
 // setup_format with the tensor-copy layout where the format and the matrices allow it (the maps are encoded here),
-// else with per-row copies. False when the streaming kernel does not address the shape.
+// else with per-row copies. False when the streaming kernel does not address the shape. `whole_rows`: the rows of the matrix that
+// the one here is a slice of, which then decide in place of its own: the forms add up in orders of their own.
 template <int WT>
-bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in, int rows, int silu_pair, size_t *smem, bool wide = false) {
+bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in, int rows, int silu_pair, size_t *smem, bool wide = false,
+                  int64_t whole_rows = 0) {
     static const bool no_tma = std::getenv("KRK_CUDA_GEMV_NO_TMA") != nullptr;
     int64_t tiles = 0;
-    for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += (mats[m].n_out + kTileRows - 1) / kTileRows;
+    for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += ((whole_rows ? whole_rows : mats[m].n_out) + kTileRows - 1) / kTileRows;
     // A tile for an SM at most, of many stages: two groups, see stages_halve.
     const bool whole_sm = rows <= 2 && n_in > 5120 && tiles <= (n_in >= 8192 ? sm_count() : sm_count() * 7 / 8);
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
@@ -2630,7 +2632,9 @@ int launch_peers_fmt(const GemvMat &mat, int64_t n_in, int rows, const PeerScatt
     StreamParams p;
     size_t smem = 0;
     if (mat.n_out > (1 << 30) || mat.n_out <= 0) return 0;
-    if (!setup_launch<WT>(p, &mat, 1, n_in, rows, 0, &smem)) return 0;
+    if (!setup_launch<WT>(p, &mat, 1, n_in, rows, 0, &smem, false, ps.row_stride)) return 0;
+    // (as launch_fmt has it for the whole row)
+    if ((p.ragged ? granules(p, ps.row_stride) : (ps.row_stride + kTileRows * p.tps - 1) / (kTileRows * p.tps)) <= sm_count()) p.by_stage = stages_in_turn<WT>(p, true);
     p.mat[0] = mat;
     p.n_entries = 1;
     p.gran_begin[0] = 0;

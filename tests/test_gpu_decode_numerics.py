@@ -228,6 +228,24 @@ def test_one_and_two_rows_with_stages_in_turn(cuda, wt):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("wt", FORMATS)
+def test_slices_of_a_sharded_head_keep_the_bits_of_the_whole(cuda, wt):
+    """krk_cuda_gemv_allgather, a slice at a time into one row: the form, and with it the order of sums, goes by the rows of the whole head
+    (of 296 tiles, where a slice has 148 or fewer, and of one tile for an SM)."""
+    import torch
+    for n_in in (5376, 8192, 8960):
+        for n_out, cuts in ((4736, (0, 2368, 3000, 4736)), (2000, (0, 1000, 2000))):
+            w = dev(synth.weights(wt, n_out, n_in, SEED + 16, stream=wt))
+            per_row = w.numel() // n_out
+            for rows in (1, 2, 3):
+                x = dev(synth.activations(rows, n_in, SEED + rows))
+                full, flags = torch.zeros((rows, n_out), device="cuda"), torch.zeros(3, dtype=torch.int32, device="cuda")
+                for step, (lo, hi) in enumerate(zip(cuts, cuts[1:])):
+                    cuda.gemv_allgather([full.data_ptr()], [flags.data_ptr()], 0, step + 1, lo, n_out, x, w.view(-1)[lo * per_row:hi * per_row], wt, hi - lo, n_in)
+                assert torch.equal(full, cuda.gemv(x, w, wt, n_out, n_in)), (n_in, n_out, rows)
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("wt", [synth.Q4_K, synth.Q6_K, synth.Q8_0])
 def test_routed_experts_of_wide_activations(cuda, wt):
     """The same two groups behind a device-side table of matrices."""
