@@ -1750,50 +1750,62 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
             wait_phase(smem_u32(&sm->red_full[slot]), (nth / kSlots) & 1, gave_up, p.status);
             if (both) wait_phase(smem_u32(&sm->red_full[slot + kSlots]), (nth / kSlots) & 1, gave_up, p.status);
             tile_it++;
+            auto sums = [&](const int sub, const int i) {   // of 16 weight rows and activation rows 2i and 2i + 1
+                const int idx = lane + 32 * i, row = idx & (kTileRows - 1), r = idx >> 4;   // r = 2*i + (lane >> 4)
+                const float *src = reinterpret_cast<const float *>(&sm->red[slot][sub * sub_warps][i][row & 7]) +
+                                   2 * (row >> 3) + (r & 1);
+                float part[kConsumerWarps];
 #pragma unroll
-            for (int sub = 0; sub < (STACK ? kMaxStack : 1); sub++) {
-                if (sub >= tps) break;
+                for (int w = 0; w < kConsumerWarps; w++) part[w] = w < sub_warps ? src[(size_t)w * (NG * 8 * 4)] : 0.0f;
+                float v = 0.0f;
 #pragma unroll
-                for (int i = 0; i < NG; i++) {
-                    const int idx = lane + 32 * i, row = idx & (kTileRows - 1), r = idx >> 4;   // r = 2*i + (lane >> 4)
-                    const float *src = reinterpret_cast<const float *>(&sm->red[slot][sub * sub_warps][i][row & 7]) +
-                                       2 * (row >> 3) + (r & 1);
-                    float part[kConsumerWarps];
+                for (int w = 0; w < kConsumerWarps; w++) v += part[w];
+                if (both) {
+                    const float *src1 = src + (size_t)kSlots * (kConsumerWarps * NG * 8 * 4);
 #pragma unroll
-                    for (int w = 0; w < kConsumerWarps; w++) part[w] = w < sub_warps ? src[(size_t)w * (NG * 8 * 4)] : 0.0f;
-                    float v = 0.0f;
+                    for (int w = 0; w < kConsumerWarps; w++) part[w] = src1[(size_t)w * (NG * 8 * 4)];
 #pragma unroll
                     for (int w = 0; w < kConsumerWarps; w++) v += part[w];
-                    if (both) {
-                        const float *src1 = src + (size_t)kSlots * (kConsumerWarps * NG * 8 * 4);
-#pragma unroll
-                        for (int w = 0; w < kConsumerWarps; w++) part[w] = src1[(size_t)w * (NG * 8 * 4)];
-#pragma unroll
-                        for (int w = 0; w < kConsumerWarps; w++) v += part[w];
-                    }
-                    const int srow = kTileRows * sub + row;   // row inside the stage
-                    const int yrow = s.row0 + (kRagged && p.ragged ? srow * p.ragged : srow);
-                    if ((kFine || WIDE) && v != v && r < p.rows && srow < s.n_rows) {
-                        const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
-                        v = dot_f32<WT>(tv.w(s.mat) + (size_t)yrow * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
-                    }
-                    if (r < p.rows) {
-                        if (p.step == 2 && s.which == 0) {
-                            v = __fdiv_rn(v, __fadd_rn(1.0f, exp_as_host(-v)));   // kept for the `up` tile
-                            if (STACK) sm->gate[sub][i][lane] = v;
-                            else gate_reg[i] = v;
-                        } else if (srow < s.n_rows) {
-                            if (p.n_peers > 0) {
-                                // plain stores into every GPU's copy of the full row (NVLink peer stores)
-                                const long long at = (long long)r * p.peer_row_stride + p.peer_offset + yrow;
-                                for (int q = 0; q < p.n_peers; q++) p.peer_y[q][at] = v;
-                            } else {
-                                float *y = y0 + (size_t)r * n_out + yrow;
-                                if (p.step == 2) v = __fmul_rn(STACK ? sm->gate[sub][i][lane] : gate_reg[i], v);
-                                *y = p.accumulate ? __fadd_rn(*y, v) : v;
-                            }
+                }
+                const int srow = kTileRows * sub + row;   // row inside the stage
+                const int yrow = s.row0 + (kRagged && p.ragged ? srow * p.ragged : srow);
+                if ((kFine || WIDE) && v != v && r < p.rows && srow < s.n_rows) {
+                    const int xr = p.table_rows ? p.table_rows[s.mat / p.step * p.rows + r] : r;
+                    v = dot_f32<WT>(tv.w(s.mat) + (size_t)yrow * p.row_bytes, tv.x(s.mat) + (size_t)xr * p.n_in, p.n_in);
+                }
+                if (r < p.rows) {
+                    if (p.step == 2 && s.which == 0) {
+                        v = __fdiv_rn(v, __fadd_rn(1.0f, exp_as_host(-v)));   // kept for the `up` tile
+                        if (STACK) sm->gate[sub][i][lane] = v;
+                        else gate_reg[i] = v;
+                    } else if (srow < s.n_rows) {
+                        if (p.n_peers > 0) {
+                            // plain stores into every GPU's copy of the full row (NVLink peer stores)
+                            const long long at = (long long)r * p.peer_row_stride + p.peer_offset + yrow;
+                            for (int q = 0; q < p.n_peers; q++) p.peer_y[q][at] = v;
+                        } else {
+                            float *y = y0 + (size_t)r * n_out + yrow;
+                            if (p.step == 2) v = __fmul_rn(STACK ? sm->gate[sub][i][lane] : gate_reg[i], v);
+                            *y = p.accumulate ? __fadd_rn(*y, v) : v;
                         }
                     }
+                }
+            };
+            if constexpr (STACK && NG > 1) {
+                // This code runs once or a few times in a launch, from a cold instruction cache: where it would be long, it is a loop
+                // (Q2_K 4096 x 512 at five rows 10.0 -> 7.3 us, 4096 x 256 9.7 -> 6.9; with one column group 1.00, with one tile to a
+                // stage 0.98 to 1.03).
+#pragma unroll 1
+                for (int sub = 0; sub < tps; sub++) {
+#pragma unroll (NG == 4 ? 1 : NG)
+                    for (int i = 0; i < NG; i++) sums(sub, i);
+                }
+            } else {
+#pragma unroll
+                for (int sub = 0; sub < (STACK ? kMaxStack : 1); sub++) {
+                    if (sub >= tps) break;
+#pragma unroll
+                    for (int i = 0; i < NG; i++) sums(sub, i);
                 }
             }
             __syncwarp();
