@@ -98,7 +98,44 @@ static void check_planes() {
         }
 }
 
+// Tiles of ragged rows (TilePlace): every row in one tile, none of more rows than a stage holds, and the same tiles from whichever
+// granule a CTA starts; as many granules as the rows fill, and rows dealt to more.
+static void check_phases() {
+    StreamParams p = {};
+    for (p.ragged = 2; p.ragged <= 8; p.ragged *= 2)
+        for (int gran = kTileRows; gran <= kTileRows * kMaxStack; gran *= 2)
+            for (int n_out = 1; n_out <= 2600; n_out += n_out < 160 ? 1 : 53) {
+                p.gran = (short)gran;
+                const int fill = (int)granules(p, n_out);
+                for (int all : {fill, n_out / (4 * p.ragged) * p.ragged, 148}) {
+                    if (all < fill || (all > fill && all > n_out)) continue;
+                    std::vector<int> at(all), count(all), seen(n_out, 0);
+                    TilePlace tile(p, 0, all);
+                    for (int i = 0; i < all; i++, tile.next()) {
+                        tile.look(p, all, n_out);
+                        at[i] = tile.phase + p.ragged * tile.first_row();
+                        count[i] = tile.count();
+                        check(tile.phase < p.ragged && count[i] >= 0 && count[i] <= gran, "rows of a tile", p.ragged, n_out, all, i, count[i]);
+                        for (int r = 0; r < count[i]; r++) {
+                            const int row = at[i] + p.ragged * r;
+                            check(row < n_out, "row", p.ragged, n_out, all, i, row);
+                            if (row < n_out) seen[row]++;
+                        }
+                    }
+                    for (int r = 0; r < n_out; r++) check(seen[r] == 1, "a row's tiles", p.ragged, n_out, all, r, seen[r]);
+                    for (int first = 1; first < all; first += 1 + all / 7) {
+                        TilePlace from(p, first, all);
+                        for (int i = first; i < all && i < first + 3; i++, from.next()) {
+                            from.look(p, all, n_out);
+                            check(from.phase + p.ragged * from.first_row() == at[i] && from.count() == count[i], "start", p.ragged, n_out, all, first, i);
+                        }
+                    }
+                }
+            }
+}
+
 int main() {
+    check_phases();
     check_format<KRK_CUDA_Q4_0>();
     check_planes<KRK_CUDA_Q4_0>();
     check_format<KRK_CUDA_Q5_0>();
