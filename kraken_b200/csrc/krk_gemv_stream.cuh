@@ -2599,9 +2599,12 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     // stage, 1024 x 2048, 1.02, 0.95, 1.07). Not the forms that take a whole SM: there the idle SMs let the next launch start (four rows of
     // 2048 x 5632 7.4 and 7.7).
     if ((p.use_tma || p.ragged) && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
-        if (p.ragged) {   // (of four rows at least)
+        if (p.ragged) {
+            // Of four rows where that keeps to two fifths of the SMs, else of whatever all of them get: between the two the next launch's CTAs
+            // go to the idle SMs (one row, 200, 256 and 416 weight rows on 48, 64 and 104 SMs against 148: Q3_K x 5120 5.0, 5.7 and 6.7
+            // us against 5.1; Q6_K x 2304 4.1, 4.5 and 4.7 against 4.1).
             const int least = (int)(mats[0].n_out / (4 * p.ragged)) * p.ragged;
-            if (least >= sm_count()) p.gran_begin[1] = total = sm_count();
+            if (least > sm_count() * 2 / 5) p.gran_begin[1] = total = sm_count();
             else if (least > total) p.gran_begin[1] = total = least;
         } else if (tiles > sm_count() / 2 || (tiles > sm_count() * 2 / 5 && p.units > kConsumerWarps)) {
             p.gran = 1;

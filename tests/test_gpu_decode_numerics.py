@@ -177,6 +177,23 @@ def test_ragged_rows_in_tiles_of_a_phase(cuda, wt, widths):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("wt, n_in", [(synth.Q8_0, 2080), (synth.Q5_1, 2080), (synth.Q6_K, 2304), (synth.Q3_K, 5120), (synth.Q2_K, 2304)])
+def test_few_ragged_rows_on_either_side_of_the_dealing(cuda, wt, n_in):
+    """Tiles of four rows (of 8, 4 or 2 phases) up to two fifths of 148 SMs, one to three rows on every SM beyond."""
+    import torch
+    for n_out in (232, 236, 240, 256, 263, 416, 591):
+        w = dev(synth.weights(wt, n_out, n_in, SEED + 17, stream=wt))
+        w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+        for rows in (1, 2):
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            base = torch.randn((rows, n_out), device="cuda")
+            y = cuda.gemv(x, w, wt, n_out, n_in, out=base.clone(), accumulate=True)
+            # as in test_ragged_rows_in_tiles_of_a_phase
+            lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
+            assert ((y.double() - base - x.double() @ w64.T).abs() <= lim).all(), (n_out, rows)
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("wt, n_in", [(synth.Q8_0, 2080), (synth.Q6_K, 5120), (synth.Q3_K, 2304)])
 def test_ragged_rows_of_groups(cuda, wt, n_in):
     """Three matrices of eight phases still have a tensor map each, four are copied row by row; pairs; a group as Backend sends it."""
