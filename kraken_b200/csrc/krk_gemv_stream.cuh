@@ -2566,6 +2566,15 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem, false, false, whole_sm, wide);
 }
 
+// Tiles of one stage that stay whole, at most, where a launch could deal their rows to all SMs (see launch_fmt): half of the SMs have
+// one, four fifths in the one-row forms of Q4_K and Q4_0 with warps to spare (1280 to 1792 x 1280 and x 1536 dealt 1.02 to 1.05 of the
+// time; x 2048 0.94 to 1.02) and of Q6_K (1200 to 1792 x 2048 1.00 to 1.07; two rows 0.94 to 1.04).
+template <int WT>
+int whole_up_to(const StreamParams &p) {
+    const bool spare = (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q4_0) && p.units < kConsumerWarps;
+    return p.rows == 1 && (spare || WT == KRK_CUDA_Q6_K) ? sm_count() * 4 / 5 : sm_count() / 2;
+}
+
 template <int WT>
 int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, bool wide, cudaStream_t st) {
     StreamParams p;
@@ -2596,8 +2605,9 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     // that belong to the next CTA). Else the CTAs of the next launch, which find room beside these, go to the idle SMs two at a
     // time and take twice as long there (Q6_K 2048 x 8192 8.5 -> 6.6 us, Q5_K 2048 x 8192 8.0 -> 6.4, Q4_K 2048 x 5632 4.8 -> 4.4). With several
     // stages to a tile from two fifths on (1024 x 4096: Q4_K 0.94 of the time, Q5_K 0.89, Q6_K 0.91; 768 x 4096 1.03, 1.02, 1.08; of one
-    // stage, 1024 x 2048, 1.02, 0.95, 1.07). Not the forms that take a whole SM: there the idle SMs let the next launch start (four rows of
+    // stage, 1024 x 2048, 1.02, 0.95, 1.07, and see whole_up_to). Not the forms that take a whole SM: there the idle SMs let the next launch start (four rows of
     // 2048 x 5632 7.4 and 7.7).
+    const bool one_stage = p.units <= kConsumerWarps;
     if ((p.use_tma || p.ragged) && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
         if (p.ragged) {
             // Of four rows where that keeps to two fifths of the SMs, else of whatever all of them get: between the two the next launch's CTAs
@@ -2606,7 +2616,7 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
             const int least = (int)(mats[0].n_out / (4 * p.ragged)) * p.ragged;
             if (least > sm_count() * 2 / 5) p.gran_begin[1] = total = sm_count();
             else if (least > total) p.gran_begin[1] = total = least;
-        } else if (tiles > sm_count() / 2 || (tiles > sm_count() * 2 / 5 && p.units > kConsumerWarps)) {
+        } else if (tiles > (one_stage ? whole_up_to<WT>(p) : sm_count() * 2 / 5)) {
             p.gran = 1;
             p.gran_begin[1] = total = (int)mats[0].n_out;
         }
