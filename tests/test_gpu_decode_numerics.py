@@ -155,6 +155,25 @@ def test_stages_in_one_box_of_padded_rows(cuda, wt, widths):
     assert cuda.device_status() == 0
 
 
+# Row copies again where CTAs have as many tiles (74 SMs' and 148's worth of 16 rows, twice and thrice that and more), on either side
+@pytest.mark.parametrize("wt, n_in, n_outs, row_counts", [
+    (synth.Q5_1, 1280, (8500, 9216), (1, 2)), (synth.Q5_1, 4096, (4600, 4736, 9216, 14208), (1, 2, 3, 5, 6)), (synth.Q5_1, 5632, (4736, 18432), (2, 4)),
+    (synth.Q8_0, 1024, (4800, 8192, 9472, 14224), (2,)), (synth.Q8_0, 2048, (5632, 8192, 14000, 14224), (2,)), (synth.Q8_0, 4096, (4144, 4145, 4700), (1,)),
+    (synth.Q2_K, 2048, (1200, 2368, 2369), (1, 2)), (synth.Q3_K, 2048, (1200, 2368, 2369), (1, 2))])
+def test_row_copies_where_tiles_come_out_even(cuda, wt, n_in, n_outs, row_counts):
+    import torch
+    for n_out in n_outs:
+        w = dev(synth.weights(wt, n_out, n_in, SEED + 19, stream=wt))
+        w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
+        for rows in row_counts:
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            y = cuda.gemv(x, w, wt, n_out, n_in)
+            # as in test_stages_in_one_box_of_padded_rows
+            lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None]
+            assert ((y.double() - x.double() @ w64.T).abs() <= lim).all(), (n_out, rows)
+    assert cuda.device_status() == 0
+
+
 # Rows that are not 16-byte multiples go in tiles of rows 2, 4 or 8 apart: K = 32, 64 and 128 times odd numbers (Q8_0, Q4_0, IQ4_NL, Q5_0),
 # any K off a multiple of 2048 (Q6_K that long or that odd, Q3_K) or 1024 (Q2_K); matrices of fewer rows than that, of parts of
 # tiles, and on either side of a tile for every SM
@@ -319,11 +338,14 @@ def test_rows_without_room_are_as_exact_as_f32(cuda, wt, outliers):
     assert cuda.device_status() == 0
 
 
-@pytest.mark.parametrize("n_out", [4736, 4737, 5003])
-def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
-    """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
+@pytest.mark.parametrize("n_in, tiles", [(768, (3, 5)), (1024, (2, 3, 5)), (4096, (2, 6))])
+def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_in, tiles):
+    """Two consumer groups share a CTA up to six tiles of 16 weight rows per SM at three rows and everywhere at four; up to 1024 values
+    up to three at three rows, five at four (three below 1024). Beyond, every CTA has one group, and two share an SM; up to 1024 values
+    stages come as row copies beyond five tiles per SM."""
     import torch
-    for n_in in (1024, 4096):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n_out in sorted({16 * sms * t + more for t in tiles for more in (0, 1, 267)}):
         w = dev(synth.weights(synth.Q8_0, n_out, n_in, SEED + 6, stream=1))
         w64 = cuda.dequant_rows(w, synth.Q8_0, n_out, n_in).double()
         for rows in (2, 3, 4, 5):
@@ -331,7 +353,24 @@ def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
             base = torch.randn((rows, n_out), device="cuda")
             y = cuda.gemv(x, w, synth.Q8_0, n_out, n_in, out=base.clone(), accumulate=True)
             lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
-            assert ((y.double() - base.double() - x.double() @ w64.T).abs() <= lim).all()
+            assert ((y.double() - base.double() - x.double() @ w64.T).abs() <= lim).all(), (n_out, rows)
+    assert cuda.device_status() == 0
+
+
+def test_q8_0_three_rows_of_one_group_in_a_launch_of_two_matrices(cuda):
+    import torch
+    n_in, rows, sizes = 4096, 3, (9000, 6001)   # 938 tiles: beyond six per SM together
+    x = dev(synth.activations(rows, n_in, SEED))
+    ws = [dev(synth.weights(synth.Q8_0, n, n_in, SEED + 18 + i, stream=i)) for i, n in enumerate(sizes)]
+    ys = [torch.zeros((rows, n), device="cuda") for n in sizes]
+    be = cuda.Backend(0)
+    torch.cuda.synchronize()
+    ran, _ = be.gemm_group([y.data_ptr() for y in ys], x.data_ptr(), [w.data_ptr() for w in ws], synth.Q8_0, list(sizes), n_in, rows=rows)
+    be.sync()
+    assert ran
+    for n, w, y in zip(sizes, ws, ys):
+        w64 = cuda.dequant_rows(w, synth.Q8_0, n, n_in).double()
+        assert ((y.double() - x.double() @ w64.T).abs() <= 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None]).all()
     assert cuda.device_status() == 0
 
 
