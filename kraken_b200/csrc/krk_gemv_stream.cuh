@@ -779,6 +779,33 @@ template <int NG>
 struct Accum {
     float f[NG][4];   // [group][(row g | g+8) x (col 2t | 2t+1)], already times the block scale d
 };
+// Where rows are to be as exact as f32 (FINE: four limbs) a unit's blocks are added up by themselves, at up to four activation rows, and
+// then added as one: a warp adds K / 256 blocks one after the other, and the error grows with the root of that (12544 values, against
+// f64: Q8_0 1.45e-7 -> 1.05e-7, IQ4_NL 1.49e-7 -> 0.99e-7, Q5_1 1.76e-7 -> 1.16e-7; the warp-per-row kernel 1.42e-7, 1.42e-7, 1.70e-7. 1.004 of
+// the time). Q4_0 and Q5_0 are below that kernel's without it.
+template <bool FINE, int NG>
+constexpr bool kUnitSums = FINE && NG <= 2;
+template <bool FINE, int NG>
+__device__ __forceinline__ float (&unit_sums(Accum<NG> &acc, float (&own)[NG][4]))[NG][4] {
+    if constexpr (kUnitSums<FINE, NG>) {
+#pragma unroll
+        for (int mg = 0; mg < NG; mg++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) own[mg][j] = 0.0f;
+        return own;
+    } else {
+        return acc.f;
+    }
+}
+template <bool FINE, int NG>
+__device__ __forceinline__ void add_unit_sums(Accum<NG> &acc, const float (&own)[NG][4]) {
+    if constexpr (kUnitSums<FINE, NG>) {
+#pragma unroll
+        for (int mg = 0; mg < NG; mg++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc.f[mg][j] += own[mg][j];
+    }
+}
 // The super-block formats at one or two activation rows: the same, with a sum of its own for the minimum term.
 struct AccumPair {
     float f[1][4];
@@ -1187,6 +1214,8 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                             int t, Accum<NG> &acc, int nb) {
+    float own[NG][4];
+    float (&sum)[NG][4] = unit_sums<RAG>(acc, own);
     constexpr uint32_t kG0 = 0xBFAD9881u, kG1 = 0xF6EADDCFu, kG2 = 0x26190D01u, kG3 = 0x71594535u;
     auto grid = [&](uint32_t q, uint32_t &lo4, uint32_t &hi4) {
         const uint32_t s = q & 0x77777777u, s2 = s >> 16, y = q << 4;
@@ -1231,12 +1260,13 @@ __device__ __forceinline__ void unit_iq4_nl(const uint8_t *rowA, const uint8_t *
             int c[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};   // |sum| <= 32 * 127 * 128 < 2^19
             mma_s8_k16_chain(c, la, lb, b0);
             mma_s8_k16_chain(c, ha, hb, b1);
-            acc.f[mg][0] = fmaf(dA, __int_as_float(c[0]) - kMagic, acc.f[mg][0]);
-            acc.f[mg][1] = fmaf(dA, __int_as_float(c[1]) - kMagic, acc.f[mg][1]);
-            acc.f[mg][2] = fmaf(dB, __int_as_float(c[2]) - kMagic, acc.f[mg][2]);
-            acc.f[mg][3] = fmaf(dB, __int_as_float(c[3]) - kMagic, acc.f[mg][3]);
+            sum[mg][0] = fmaf(dA, __int_as_float(c[0]) - kMagic, sum[mg][0]);
+            sum[mg][1] = fmaf(dA, __int_as_float(c[1]) - kMagic, sum[mg][1]);
+            sum[mg][2] = fmaf(dB, __int_as_float(c[2]) - kMagic, sum[mg][2]);
+            sum[mg][3] = fmaf(dB, __int_as_float(c[3]) - kMagic, sum[mg][3]);
         }
     }
+    add_unit_sums<RAG>(acc, own);
 }
 
 // Bits 0..3 of n to bit 7 of bytes 0..3: bit i times 2^(7j + 7) lands at 8k + 7 only for i = j = k, and no two
@@ -1314,6 +1344,8 @@ __device__ __forceinline__ void unit_q5_0(const uint8_t *rowA, const uint8_t *ro
 template <int NG, bool RAG>
 __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           const float *const (&fe)[NG], const float *const (&fo)[NG], int t, Accum<NG> &acc, int nb) {
+    float own[NG][4];
+    float (&sum)[NG][4] = unit_sums<RAG>(acc, own);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
         if (RAG && b >= nb) break;   // (rows start on 8-byte boundaries: words stay aligned)
@@ -1337,12 +1369,13 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
             const int at = (kbase >> 5) + b;
             const float se = t == 1 ? fe[mg][at] : RAG ? (t == 3 ? fo[mg][at] : 0.0f) : spare ? fe[NG - 1][at] : 0.0f;
             const float so = RAG ? 0.0f : t == 2 ? fo[mg][at] : spare ? fo[NG - 1][at] : 0.0f;
-            acc.f[mg][0] = fmaf(dA, __int_as_float(c[0]) - kMagic, fmaf(oA, se, acc.f[mg][0]));
-            acc.f[mg][1] = fmaf(dA, __int_as_float(c[1]) - kMagic, fmaf(oA, so, acc.f[mg][1]));
-            acc.f[mg][2] = fmaf(dB, __int_as_float(c[2]) - kMagic, fmaf(oB, se, acc.f[mg][2]));
-            acc.f[mg][3] = fmaf(dB, __int_as_float(c[3]) - kMagic, fmaf(oB, so, acc.f[mg][3]));
+            sum[mg][0] = fmaf(dA, __int_as_float(c[0]) - kMagic, fmaf(oA, se, sum[mg][0]));
+            sum[mg][1] = fmaf(dA, __int_as_float(c[1]) - kMagic, fmaf(oA, so, sum[mg][1]));
+            sum[mg][2] = fmaf(dB, __int_as_float(c[2]) - kMagic, fmaf(oB, se, sum[mg][2]));
+            sum[mg][3] = fmaf(dB, __int_as_float(c[3]) - kMagic, fmaf(oB, so, sum[mg][3]));
         }
     }
+    add_unit_sums<RAG>(acc, own);
 }
 
 // Four Q8_0 blocks. A block is a 2-byte scale then 32 quants, so blocks at an even index have
@@ -1351,6 +1384,8 @@ __device__ __forceinline__ void unit_q5_1(const uint8_t *rowA, const uint8_t *ro
 template <int NG, bool RAG, int BY2>
 __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *rowB, int kbase, const int8_t *const (&bp)[NG],
                                           int t, Accum<NG> &acc, int nb) {
+    float own[NG][4];
+    float (&sum)[NG][4] = unit_sums<RAG>(acc, own);
     const Words<BY2> wA(rowA + 4 * t), wB(rowB + 4 * t);
 #pragma unroll
     for (int b = 0; b < 4; b++) {
@@ -1390,12 +1425,13 @@ __device__ __forceinline__ void unit_q8_0(const uint8_t *rowA, const uint8_t *ro
             const uint32_t b1 = *reinterpret_cast<const uint32_t *>(bp[mg] + kbase + 32 * b + 16 + 4 * t);
             int cc[4];   // (presetting the accumulator to 1.5 * 2^23 to save the int-to-float step is 0.3-3 % slower here)
             mma_s8_k32(cc, a0, a1, a2, a3, b0, b1);
-            acc.f[mg][0] = fmaf(dA, (float)cc[0], acc.f[mg][0]);
-            acc.f[mg][1] = fmaf(dA, (float)cc[1], acc.f[mg][1]);
-            acc.f[mg][2] = fmaf(dB, (float)cc[2], acc.f[mg][2]);
-            acc.f[mg][3] = fmaf(dB, (float)cc[3], acc.f[mg][3]);
+            sum[mg][0] = fmaf(dA, (float)cc[0], sum[mg][0]);
+            sum[mg][1] = fmaf(dA, (float)cc[1], sum[mg][1]);
+            sum[mg][2] = fmaf(dB, (float)cc[2], sum[mg][2]);
+            sum[mg][3] = fmaf(dB, (float)cc[3], sum[mg][3]);
         }
     }
+    add_unit_sums<RAG>(acc, own);
 }
 
 // The A operand is 4 * (q - 32) as a signed byte: the low four quant bits at bits 2-5, the high two at bits 6-7

@@ -338,6 +338,20 @@ def test_rows_without_room_are_as_exact_as_f32(cuda, wt, outliers):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("wt", [synth.Q8_0, synth.IQ4_NL, synth.Q5_1])
+def test_rows_without_room_add_no_error_block_by_block(cuda, wt):
+    """The 32-value formats at the widths where a warp adds the most blocks: the mean of eight errors is that of sums by unit (1.0e-7 to
+    1.1e-7 here), below what adding block by block gives (1.38e-7 to 1.45e-7; the warp-per-row kernel 1.33e-7 to 1.42e-7)."""
+    errs = []
+    for i in range(8):
+        n_out, n_in, rows = 530, 12544, 6
+        w = dev(synth.weights(wt, n_out, n_in, 900 + i, stream=wt))
+        x = dev(synth.activations(rows, n_in, 77 + i))
+        want = x.double() @ cuda.dequant_rows(w, wt, n_out, n_in).double().T
+        errs.append(((cuda.gemv(x, w, wt, n_out, n_in).double() - want).norm() / want.norm()).item())
+    assert np.mean(errs) <= 1.25e-7, errs
+
+
 @pytest.mark.parametrize("n_in, tiles", [(768, (3, 5)), (1024, (2, 3, 5)), (4096, (2, 6))])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_in, tiles):
     """Two consumer groups share a CTA up to six tiles of 16 weight rows per SM at three rows and everywhere at four; up to 1024 values
