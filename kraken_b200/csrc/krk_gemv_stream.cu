@@ -34,9 +34,14 @@ static __global__ void __launch_bounds__(32) flag_wait_kernel(const int *flags, 
 }
 
 // Activation rows whose limbs leave no room for a ring, K a multiple of 256: half of them at a time, or half of those, with four
-// limbs, so that results are as exact as those of the warp-per-row kernel, which multiplies in f32 and had these shapes (error against f64
-// sums at 8 rows, K of 7424 to 14336: 0.9e-7 to 1.4e-7 here, 1.4e-7 to 1.6e-7 there; 22 bits 2.6e-7, and eight times that with outliers).
+// limbs: 30 bits below the largest activation of a warp's slices, sums of activations (formats with a minimum) in eighths of the
+// 22nd. The warp-per-row kernel, which had these shapes, multiplies in f32: it keeps 24 bits of every activation, however small, but
+// adds up in more steps, and its results are no nearer the f64 sums (530 weight rows, normal activations and with every 97th 300
+// times as large, worst of twelve: 12544 values, six rows 0.7e-7 to 1.2e-7 here, 1.4e-7 to 1.7e-7 there; 21504, three rows 0.9e-7 to
+// 1.4e-7, 1.5e-7 to 1.9e-7; 22 bits 2.6e-7 and eight times that. Q2_K, whose sums are of 16 values, up to 24576 values: beyond, 40960 with
+// two rows 2.3e-7 against 1.9e-7).
 // 4096 x 11264: Q4_K at six and eight rows 97 -> 30, 117 -> 51 us, Q6_K 101 -> 35, 122 -> 61; 16384 x 9984 at eight rows 404 -> 77, 425 -> 109.
+// A shape that has room for some rows has it for fewer: no part is refused after one that was launched.
 static int launch_parts(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, cudaStream_t st) {
     int rc = 0;
     if (rows <= 4) KRK_DISPATCH_WT(mats[0].wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, true, st));
@@ -71,7 +76,8 @@ int launch_gemv_stream(const GemvMat *mats, int n_mat, int64_t n_in, int rows, i
     int rc = 0;
     KRK_DISPATCH_WT(wt, rc = stream::launch_fmt<WT>(mats, n_mat, n_in, rows, accumulate, silu_pair, false, st));
     // (few rows of Q5_1, whose units are the longest: 256 x 11264 at six rows 43.8 and 45.9 us)
-    if (rc == 0 && rows > 1 && !odd_k && n_mat <= KRK_CUDA_MAX_GROUP && (wt != KRK_CUDA_Q5_1 || out >= 512)) return launch_parts(mats, n_mat, n_in, rows, accumulate, silu_pair, st);
+    if (rc == 0 && rows > 1 && !odd_k && n_mat <= KRK_CUDA_MAX_GROUP && (wt != KRK_CUDA_Q5_1 || out >= 512) && (wt != KRK_CUDA_Q2_K || n_in <= 24576))
+        return launch_parts(mats, n_mat, n_in, rows, accumulate, silu_pair, st);
     // Activation rows whose four limbs leave no room for a ring go in two launches: the weights twice through the ring are
     // quicker than the warp-per-row kernel once (8 rows of K = 11232, 2048 weight rows: Q8_0 50 against 81 us, Q5_1 70 against
     // 75), but for matrices that do not fill the SMs with rows in the formats with the longer units (512 weight rows: Q4_0
