@@ -338,6 +338,27 @@ def test_rows_without_room_are_as_exact_as_f32(cuda, wt, outliers):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("outliers", [False, True])
+@pytest.mark.parametrize("wt", FORMATS)
+def test_two_to_four_rows_without_room(cuda, wt, outliers):
+    """The widest rows: two, three and four of them in parts of two and one, added onto what is there. The warp-per-row kernel, which
+    such shapes took before, is at worst this far from the f64 sums over such inputs (16128, 21504 and 32512 values; the fewest weight
+    rows leave the most to chance); and the rounding of the last sum."""
+    import torch
+    for n_in, rows, bound in ((16128, 4, 1.71e-7), (21504, 3, 1.88e-7), (32512, 2, 2.11e-7)):   # (beyond what any format has room for)
+        for n_out, worst in ((33, 2.46e-7), (530, bound)):
+            w = dev(synth.weights(wt, n_out, n_in, SEED + 21, stream=wt))
+            x = synth.activations(rows, n_in, SEED + rows)
+            if outliers:
+                x[:, 5::97] *= 300.0
+            x = dev(x)
+            base = torch.randn((rows, n_out), device="cuda")
+            got = cuda.gemv(x, w, wt, n_out, n_in, out=base.clone(), accumulate=True).double()
+            want = x.double() @ cuda.dequant_rows(w, wt, n_out, n_in).double().T
+            assert (got - base - want).norm() <= worst * want.norm() + 2.0 ** -24 * got.norm(), (n_in, rows, n_out)
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("wt", [synth.Q8_0, synth.IQ4_NL, synth.Q5_1])
 def test_rows_without_room_add_no_error_block_by_block(cuda, wt):
     """The 32-value formats at the widths where a warp adds the most blocks: the mean of eight errors is that of sums by unit (1.0e-7 to
@@ -350,6 +371,43 @@ def test_rows_without_room_add_no_error_block_by_block(cuda, wt):
         want = x.double() @ cuda.dequant_rows(w, wt, n_out, n_in).double().T
         errs.append(((cuda.gemv(x, w, wt, n_out, n_in).double() - want).norm() / want.norm()).item())
     assert np.mean(errs) <= 1.25e-7, errs
+
+
+@pytest.mark.parametrize("wt", [synth.Q4_K, synth.Q2_K, synth.Q6_K, synth.Q8_0, synth.Q5_1])
+def test_rows_without_room_in_groups_pairs_and_residuals(cuda, wt):
+    """As a model's layer sends them: two matrices of one activation, a gate/up pair (silu has a slope of 1.1 at most), a projection
+    onto the residual."""
+    import torch
+    be = cuda.Backend(0)
+    for n_in in (12544, 14336):   # (no format has room for five rows)
+        ws = [dev(synth.weights(wt, n, n_in, SEED + 22 + i, stream=wt)) for i, n in enumerate((700, 1033, 1033))]
+        w64 = [cuda.dequant_rows(w, wt, n, n_in).double() for w, n in zip(ws, (700, 1033, 1033))]
+        for rows in (5, 6, 8):
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            want = [x.double() @ m.T for m in w64]
+            ys = [torch.full((rows, n), 7.0, device="cuda") for n in (700, 1033)]
+            torch.cuda.synchronize()
+            ran, _ = be.gemm_group([y.data_ptr() for y in ys], x.data_ptr(), [w.data_ptr() for w in ws[:2]], wt, [700, 1033], n_in, rows=rows)
+            be.sync()
+            assert ran
+            for y, v in zip(ys, want):
+                assert (y.double() - v).norm() <= 1.64e-7 * v.norm(), (n_in, rows)
+            ys = [torch.full((rows, 1033), 7.0, device="cuda") for _ in range(2)]
+            torch.cuda.synchronize()
+            ran, fused = be.gemm_group([y.data_ptr() for y in ys], x.data_ptr(), [w.data_ptr() for w in ws[1:]], wt, [1033] * 2, n_in, rows=rows, silu=True)
+            be.sync()
+            assert ran
+            if fused:
+                v = want[1] / (1.0 + torch.exp(-want[1])) * want[2]
+                lim = 2e-6 * x.double().norm(dim=1)[:, None] * (1.1 * w64[1].norm(dim=1)[None] * want[2].abs() + w64[2].norm(dim=1)[None] * want[1].abs()) + 1e-6 * v.abs()
+                assert ((ys[0].double() - v).abs() <= lim).all(), (n_in, rows)
+            base = torch.randn((rows, 700), device="cuda")
+            y = base.clone()
+            torch.cuda.synchronize()
+            assert be.gemm_accumulate(y.data_ptr(), x.data_ptr(), ws[0].data_ptr(), wt, 700, n_in, rows)
+            be.sync()
+            assert (y.double() - base - want[0]).norm() <= 1.64e-7 * want[0].norm() + 2.0 ** -24 * y.double().norm(), (n_in, rows)
+    assert cuda.device_status() == 0
 
 
 @pytest.mark.parametrize("n_in, tiles", [(768, (3, 5)), (1024, (2, 3, 5)), (4096, (2, 6))])
@@ -410,7 +468,7 @@ def test_rows_of_odd_block_counts_on_either_kernel(cuda, wt):
 @pytest.mark.parametrize("n_in", [2304, 4352, 6656, 11008, 12544])
 def test_rows_of_many_slices(cuda, oracle, wt, n_in):
     """A warp prepares one to seven slices of every activation row (held, in one batch of loads, in a second; six of the widest rows go
-    to the warp-per-row kernel in most formats). 22 bits of the largest activation of a warp's slices
+    in parts, with four limbs). 22 bits of the largest activation of a warp's slices
     (about four sigma here) leave 4 * 2^-22 / sqrt(12) a value, 2.8e-7 of the norms' product for a result; seven times that."""
     n_out = 80
     w = synth.weights(wt, n_out, n_in, SEED + 2, stream=wt)
