@@ -2527,8 +2527,14 @@ inline bool weight_maps(CUtensorMap *out, const uint8_t *w, int64_t n_out, int r
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }
-    if (cache.size() > 65536) cache.clear();   // bounded: a host that keeps re-uploading weights starts over
+    // bounded, at 8 MB of maps: a host that keeps re-uploading weights starts over
+    static size_t held = 0;
+    if (held + n > 65536) {
+        cache.clear();
+        held = 0;
+    }
     cache.emplace(key, std::vector<CUtensorMap>(out, out + n));
+    held += n;
     return true;
 }
 
