@@ -55,15 +55,16 @@ namespace stream {
 
 constexpr int kConsumerWarps = 8;
 constexpr int kConsumerThreads = kConsumerWarps * 32;
-// One or two groups of consumer warps per CTA. One or two activation rows: one group in half an SM. More rows: two
-// groups in a whole SM that share one prepared activation and take tiles in turn (one group per SM, all that its
-// registers allowed before the accumulators were folded, left the schedulers waiting half of the time).
+// One or two groups of consumer warps per CTA. One or two activation rows: one group in half an SM, or, of many stages, two groups in a
+// whole SM that take a tile's stages in turn (see stages_halve). More rows: two groups in a whole SM that share one prepared activation
+// and take tiles in turn (one group per SM, all that its registers allowed before the accumulators were folded, left the schedulers
+// waiting half of the time); one group and two CTAs per SM in some launches of Q8_0 (see setup_launch).
 __host__ __device__ constexpr int consumer_groups(int ng) { return ng == 1 ? 1 : 2; }
 __host__ __device__ constexpr int cta_threads(int groups) { return groups * kConsumerThreads + 64; }   // warp 0: producer, then the consumers, then the epilogue
 // Tiles whose partial sums may wait for the epilogue warp (fewer when more activation rows make a slot larger).
 __host__ __device__ constexpr int red_slots(int ng, int groups = 2) { return ng == 1 ? 4 / groups : ng == 2 ? 2 : 1; }   // of each consumer group
 constexpr int kMaxRedSlots = 4;
-constexpr int kMaxMaps = 24;      // of a launch: three matrices of ragged rows
+constexpr int kMaxMaps = 24;      // of a launch: three matrices of ragged rows (with 16, a kilobyte of parameters less, every other launch takes as long)
 constexpr int kMaxStack = 4;      // 16-row tiles per stage at most
 constexpr int kTileRows = 16;                     // the M of the MMA
 constexpr int kMaxStages = 8;                    // of a whole-SM CTA
@@ -395,8 +396,8 @@ struct TableView {
 // Ragged rows: rows `ragged` apart lie equally far off a 16-byte boundary, so a tile takes such rows, of one phase (row modulo
 // `ragged`): they are a matrix of 16-byte-multiple pitch, of which a stage arrives as one tensor copy, and every word of the tile lies
 // alike. An entry's granules are tiles, phase by phase: all phases have as many, or the first ones one more, and a phase's rows are
-// dealt to its tiles evenly (16 * tps at most). A phase without rows, in matrices of fewer than eight, has tiles of none, whose sums
-// go nowhere.
+// dealt to its tiles evenly (16 * tps at most). A phase without rows, in matrices of fewer than eight, has tiles of none: their stages are
+// copied like any other (by a map of the first phase's rows, see weight_maps) and their sums go nowhere.
 struct TilePlace {
     int phase, n, i;   // the tile's phase, how many tiles that has (0: not looked up yet), and which of them it is
     int each, more;    // rows of a tile of the phase: the first `more` have one more than `each`
@@ -1627,9 +1628,9 @@ __device__ __forceinline__ void unit_q3_k(const uint8_t *blkA, const uint8_t *bl
 // Either way an SM runs sixteen consumer warps of up to 96 registers: two half-SM CTAs for one or two activation rows,
 // one CTA of two consumer groups for more (see consumer_groups).
 
-// RAG: the form for ragged rows of Q6_K and Q3_K and of the 32-value block formats (K not a multiple of 256), whose units
-// find each word's alignment from its address; compiled apart so that the usual form does not carry another copy of
-// the unit. (Q2_K's words are aligned at every row start: its usual form serves ragged rows too.)
+// RAG: the form for ragged rows of Q6_K and Q3_K, whose units find each word's alignment from its address, and of the 32-value block
+// formats (K not a multiple of 256), whose tiles lie on a word boundary or off it as one; compiled apart so that the usual form does not
+// carry another copy of the unit. (Q2_K's words are aligned at every row start: its usual form serves ragged rows too.)
 // Forms whose two groups may take a tile's stages in turn (StreamParams::by_stage): ragged Q6_K. (Q3_K 4096 x 8960 at four rows
 // 19.1 -> 20.0 us with it.)
 template <int WT>
@@ -2511,7 +2512,7 @@ inline bool weight_maps(CUtensorMap *out, const uint8_t *w, int64_t n_out, int r
         return true;
     }
     for (int c = 0; c < n; c++) {
-        const int64_t first = c < n_out ? c : 0;   // (a phase without rows: never copied)
+        const int64_t first = c < n_out ? c : 0;   // (a phase without rows: its empty tiles are copied all the same, from these)
         const int lead = ragged ? (int)((size_t)first * row_bytes & 15) : 0;
         const int inner_bytes = ragged ? align_up(lead + row_bytes, 8) : mode == 3 ? row_bytes : mode == 2 ? box_units * unit_bytes : unit_bytes;
         const int box_inner = mode == 3 ? box_pitch(box_units * unit_bytes + (ragged ? 14 : 0)) : inner_bytes, size = mode == 1 ? 1 : 8;

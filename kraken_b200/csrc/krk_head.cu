@@ -9,11 +9,11 @@
 // key(i) = logits[i], clamped to +-softcap when softcap > 0, then divided (positive) or multiplied
 // (negative) by rep_pen where the token's bit is set in pen_mask; the k largest keys in descending order,
 // ties toward the lower id; ids past the row's length are -1 / -FLT_MAX; mass = sum over the whole row of
-// exp((key - max) / temp). Two kernels, both a radix select: four passes over 8-bit digits of the order-preserving
-// integer form of the keys find the k-th largest, everything above it (and the lowest ids among its equals) is
-// collected. Every block of the first kernel selects from its 2048-key slice of the row and leaves the slice's (max, sum
-// of exp); the one block of the second selects from the slices' candidates, ranks the k of them against each other and
-// folds the sums. What bounds it is latency: about a dozen barriers and two passes through level 2. (Pulling the k best
+// exp((key - max) / temp). Two kernels. The first is a radix select: up to four passes over 8-bit digits of the
+// order-preserving integer form of the keys find the k-th largest (as soon as a digit decides, no further), everything above it (and the
+// lowest ids among its equals) is collected. Every block selects from its 2048-key slice of the row and leaves the slice's (max, sum
+// of exp). The one block of the second kernel ranks what of the slices' candidates is above a bound (see rank_select; the radix select
+// again where many keys are equal or there are more than 512 slices) and folds the sums. What bounds it is latency: about a dozen barriers and two passes through level 2. (Pulling the k best
 // out one at a time, by warp arg-max and list merges, took 52 us at k = 40 on 128,256 logits.)
 #include "krk_common.cuh"
 
@@ -276,11 +276,6 @@ topk_slices_kernel(const __grid_constant__ TopkParams p, uint32_t *__restrict__ 
     }
 }
 
-// By a whole block: the k best of n_blocks lists of k keys each, without radix passes. The best few of every list, k in all at
-// least, have a k-th largest, and k keys are not below that: what is below is out, and what is left, about twice k, is ranked key
-// against key (ties to the lower id). False, in every thread, where more are left than the block has threads: many equal keys.
-// (Candidates are all near the top, so that the radix select's first digits put them in one bin: 128,256 logits, k = 40, 16.0 -> 11.8
-// us with the first kernel, k = 64 18.0 -> 12.8, 32,000 logits k = 5 10.1 -> 7.4.)
 // Ranks of n distinct keys among each other, eight threads to a key: f(key, rank).
 template <class F>
 __device__ __forceinline__ void rank_keys(const unsigned long long *keys, int n, F &&f) {
@@ -296,6 +291,11 @@ __device__ __forceinline__ void rank_keys(const unsigned long long *keys, int n,
         if (part == 0 && i < n) f(mine, rank);
     }
 }
+// By a whole block: the k best of n_blocks lists of k keys each, without radix passes. The best few of every list, k in all at
+// least, have a k-th largest, and k keys are not below that: what is below is out, and what is left, about twice k, is ranked key
+// against key (ties to the lower id). False, in every thread, where more are left than the block has threads: many equal keys.
+// (Candidates are all near the top, so that the radix select's first digits put them in one bin: 128,256 logits, k = 40, 16.0 -> 11.8
+// us with the first kernel, k = 64 18.0 -> 12.8, 32,000 logits k = 5 10.1 -> 7.4.)
 template <class EachAt>
 __device__ __forceinline__ bool rank_select(EachAt &&each_at, const TopkParams &p, const uint32_t *__restrict__ cand_u, const int *__restrict__ cand_i,
                                             int n_blocks, int32_t *__restrict__ ids, float *__restrict__ vals) {
