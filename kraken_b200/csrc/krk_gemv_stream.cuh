@@ -2627,15 +2627,6 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     return tma || setup_format<WT>(p, n_in, rows, silu_pair, smem, false, false, whole_sm, wide);
 }
 
-// Tiles of one stage that stay whole, at most, where a launch could deal their rows to all SMs (see launch_fmt): half of the SMs have
-// one, four fifths in the one-row forms of Q4_K and Q4_0 with warps to spare (1280 to 1792 x 1280 and x 1536 dealt 1.02 to 1.05 of the
-// time; x 2048 0.94 to 1.02) and of Q6_K (1200 to 1792 x 2048 1.00 to 1.07; two rows 0.94 to 1.04).
-template <int WT>
-int whole_up_to(const StreamParams &p) {
-    const bool spare = (WT == KRK_CUDA_Q4_K || WT == KRK_CUDA_Q4_0) && p.units < kConsumerWarps;
-    return p.rows == 1 && (spare || WT == KRK_CUDA_Q6_K) ? sm_count() * 4 / 5 : sm_count() / 2;
-}
-
 template <int WT>
 int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accumulate, int silu_pair, bool wide, cudaStream_t st) {
     StreamParams p;
@@ -2662,22 +2653,21 @@ int launch_fmt(const GemvMat *mats, int n_mat, int64_t n_in, int rows, int accum
     const int per_sm = tiles <= sm_count() ? 1 : ctas_per_sm<WT>(smem, p.groups);
     if (tiles <= sm_count()) p.by_stage = stages_in_turn<WT>(p, true);
     const int sms = sm_count() * per_sm;
-    // Tiles for more than half of the SMs but not for all: the rows are dealt to all of them, up to 16 each (a box brings some
-    // that belong to the next CTA). Else the CTAs of the next launch, which find room beside these, go to the idle SMs two at a
-    // time and take twice as long there (Q6_K 2048 x 8192 8.5 -> 6.6 us, Q5_K 2048 x 8192 8.0 -> 6.4, Q4_K 2048 x 5632 4.8 -> 4.4). With several
-    // stages to a tile from two fifths on (1024 x 4096: Q4_K 0.94 of the time, Q5_K 0.89, Q6_K 0.91; 768 x 4096 1.03, 1.02, 1.08; of one
-    // stage, 1024 x 2048, 1.02, 0.95, 1.07, and see whole_up_to). Not the forms that take a whole SM: there the idle SMs let the next launch start (four rows of
-    // 2048 x 5632 7.4 and 7.7).
-    const bool one_stage = p.units <= kConsumerWarps;
-    if ((p.use_tma || p.ragged) && p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
+    // Tiles for fewer SMs than there are. The CTAs of the next launch, which find room beside these, go to the idle SMs two at a time and
+    // take twice as long there: a chain of launches of one shape is quicker if the rows are dealt to all SMs, up to 16 each (a
+    // box brings some that belong to the next CTA; 1280 to 2304 x 4096 0.7 to 0.9 of the time). In a model's pass the CTAs of several launches
+    // to come find room beside fewer, and whole tiles are quicker: rows dealt cost the formats with tensor copies of packed units 1 to 10 %
+    // there (one row, 1792 / 4864 values, Q5_0 1.11 of the time, Q4_0 1.06, Q5_K 1.05; two rows, 1024 / 3584, Q4_K 1.08, Q5_K 1.07), so
+    // their tiles stay whole, but at two rows, of one stage, for over seven tenths of the SMs (q, k and v of one size one after the other,
+    // 1792 and 2048 values 0.95 to 0.97 of the time, where k and v are smaller 0.99 to 1.02). Where a box takes the place of row copies, which went to all SMs by themselves, rows are dealt above half of the
+    // SMs (Q8_0 2304 x 5120 5.3 us, whole tiles 6.5, row copies 6.0; a pass, 2048 / 4096, 0.92, 0.88 and 1), ragged ones above nine
+    // twentieths (one row, tiles on 48, 64, 80 and 104 SMs and on all: Q3_K x 5120 5.0, 5.7, 6.3, 6.7 and 5.1 us, row copies 6.0; a pass,
+    // 1024 / 2816, 64 tiles on as many 1.03 and on all 1.12 of the time that row copies took, Q2_K 1.06 and 1.11). Not the forms that
+    // take a whole SM: there the idle SMs let the next launch start (four rows of 2048 x 5632 7.4 and 7.7; ragged ones 1.02 to 1.17 of the time).
+    if (p.groups == 1 && smem <= (size_t)kSmemLimit && p.tps == 1 && p.n_entries == 1 && tiles <= sm_count()) {
         if (p.ragged) {
-            // Of four rows where that keeps to two fifths of the SMs, else of whatever all of them get: between the two the next launch's CTAs
-            // go to the idle SMs (one row, 200, 256 and 416 weight rows on 48, 64 and 104 SMs against 148: Q3_K x 5120 5.0, 5.7 and 6.7
-            // us against 5.1; Q6_K x 2304 4.1, 4.5 and 4.7 against 4.1).
-            const int least = (int)(mats[0].n_out / (4 * p.ragged)) * p.ragged;
-            if (least > sm_count() * 2 / 5) p.gran_begin[1] = total = sm_count();
-            else if (least > total) p.gran_begin[1] = total = least;
-        } else if (tiles > (one_stage ? whole_up_to<WT>(p) : sm_count() * 2 / 5)) {
+            if (total > sm_count() * 9 / 20) p.gran_begin[1] = total = sm_count();
+        } else if ((p.use_tma == 3 && tiles > sm_count() / 2) || (p.use_tma && rows == 2 && p.units <= kConsumerWarps && tiles > sm_count() * 7 / 10)) {
             p.gran = 1;
             p.gran_begin[1] = total = (int)mats[0].n_out;
         }

@@ -149,7 +149,7 @@ static void check_phases() {
             for (int n_out = 1; n_out <= 2600; n_out += n_out < 160 ? 1 : 53) {
                 p.gran = (short)gran;
                 const int fill = (int)granules(p, n_out);
-                for (int all : {fill, n_out / (4 * p.ragged) * p.ragged, 148}) {
+                for (int all : {fill, 148}) {
                     if (all < fill || (all > fill && all > n_out)) continue;
                     std::vector<int> at(all), count(all), seen(n_out, 0);
                     TilePlace tile(p, 0, all);

@@ -198,9 +198,9 @@ def test_ragged_rows_in_tiles_of_a_phase(cuda, wt, widths):
 
 @pytest.mark.parametrize("wt, n_in", [(synth.Q8_0, 2080), (synth.Q5_1, 2080), (synth.Q6_K, 2304), (synth.Q3_K, 5120), (synth.Q2_K, 2304)])
 def test_few_ragged_rows_on_either_side_of_the_dealing(cuda, wt, n_in):
-    """Tiles of four rows (of 8, 4 or 2 phases) up to two fifths of 148 SMs, one to three rows on every SM beyond."""
+    """Whole tiles (of 8, 4 or 2 phases) up to nine twentieths of 148 SMs, ten to fourteen rows on every SM beyond."""
     import torch
-    for n_out in (232, 236, 240, 256, 263, 416, 591):
+    for n_out in (232, 263, 416, 591, 1024, 1025, 1056, 1057, 1153):
         w = dev(synth.weights(wt, n_out, n_in, SEED + 17, stream=wt))
         w64 = cuda.dequant_rows(w, wt, n_out, n_in).double()
         for rows in (1, 2):
