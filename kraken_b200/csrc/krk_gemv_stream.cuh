@@ -2570,11 +2570,11 @@ inline int64_t granules(const StreamParams &p, int64_t n_out) {
 // which the loads of x then wait behind, and only just over a tile an SM is that worth it (Q8_0 4096 x 4096 7.4 against 6.7, 4700 x 4096
 // 8.2 against 7.0, 2048 x 4096 4.8 against 4.7; 3200 x 4096 5.9 against 6.1).
 // Further on, CTAs that all have as many tiles gain nothing by whole ones. Two rows of Q8_0 in one stage or two (8192 and 14000 x 1024
-// 1.03 and 1.10, x 2048 1.07 and 1.04; 5632 x 1024 0.95, 22016 x 2048 0.94, and 0.80 to 1.00 at 2304 values), one row of it in four
+// 1.03 and 1.10, x 2048 1.07 and 1.04; 5632 x 1024 0.95, 65536 x 1024 0.94, 22016 x 2048 0.94, and 0.80 to 1.00 at 2304 values), one row of it in four
 // (4200 to 4736 x 4096 1.02 to 1.07; x 3072 and x 5120 0.96 to 1.01).
 // Q5_1's rows of 1536 bytes stream as well by themselves: up to two tiles an SM (4700 x 5632 10.6 against 9.8, 4096 x 1024 at two
 // rows 5.3 against 4.9; beyond, 6000 x 5632, 12.1 against 12.7) and where CTAs have as many tiles (14208 x 2048 at one and two rows 1.05
-// and 1.09, x 1024 0.91 and 0.95, 32768 x 5632 0.98; 4736 x 4096 at three to five rows 1.04 to 1.07, 6144 x 4096 0.95 to 0.99, 14000 x
+// and 1.09, x 1024 0.91 and 0.95, 32768 x 5632 0.98; two rows of 8192 x 2048 and x 4096 1.03 and 1.05, one of x 2048 0.98; 4736 x 4096 at three to five rows 1.04 to 1.07, 6144 x 4096 0.95 to 0.99, 14000 x
 // 5120 at eight 0.97).
 template <int WT>
 bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
@@ -2583,7 +2583,7 @@ bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
     const int64_t ctas = few && smem <= (size_t)kSmemLimit ? 2 * sms : sms, last = tiles % ctas;
     auto even = [&](int tenths) { return tiles >= ctas && (last == 0 || 10 * last >= tenths * ctas); };
     if (WT == KRK_CUDA_Q5_1) {
-        if (few) return tiles <= 2 * sms || (even(9) && p.n_in >= 1280 && (p.n_in <= 3072 || (p.n_in <= 5632 && tiles <= 3 * ctas)));
+        if (few) return tiles <= 2 * sms || (even(p.rows == 2 || p.n_in >= 4096 ? 7 : 9) && p.n_in >= 1280 && p.n_in <= 5632 && tiles <= (p.n_in <= 3072 ? 7 : 3) * ctas);
         return p.rows <= 5 && even(9) && p.n_in >= 2048 && p.n_in <= 5632;
     }
     if (!few || p.units < kConsumerWarps) return false;
@@ -2591,7 +2591,7 @@ bool rows_apart(const StreamParams &p, int64_t tiles, size_t smem) {
     if (tiles <= 2 * sms)
         return p.rows == 2 ? p.units > kConsumerWarps && smem <= (size_t)kSmemLimit && (tiles <= sms || tiles > 3 * sms / 2)
                            : WT == KRK_CUDA_Q8_0 && p.units == 4 * kConsumerWarps && tiles > 7 * sms / 4;
-    if (WT != KRK_CUDA_Q8_0 || p.rows != 2) return false;
+    if (WT != KRK_CUDA_Q8_0 || p.rows != 2 || tiles > 7 * ctas) return false;
     return p.units == kConsumerWarps ? even(7) || tiles > 3 * ctas : p.units == 2 * kConsumerWarps && even(7) && tiles < 3 * ctas;
 }
 
@@ -2620,11 +2620,12 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
         // Many tiles at three rows, or at three and four of one stage each (1024 values and fewer): one group and two CTAs per SM (three rows of
         // 22016 x 4096 22.2 us against 22.9 with two groups, 8192 x 768 5.6 against 6.0; four of 32768 x 1024 12.6 against 14.4). Else two groups:
         // 6144 x 4096 10.6 against 9.8, at four rows 11.6 against 10.0, 11008 x 4096 15.3 against 14.0, 22016 x 4096 23.4 against 23.0 (since a
-        // stage is one copy they no longer wait for the ring, of which a tile is four stages there). Many tiles of one stage come faster
-        // as row copies (14000 x 1024 at three rows 7.9 against 7.3, 32768 x 1024 at four 13.2 against 12.3; 8192 x 1024 5.9 against 6.1).
+        // stage is one copy they no longer wait for the ring, of which a tile is four stages there). Tiles of one stage come faster as
+        // row copies from five to fourteen an SM (14000 x 1024 at three rows 7.9 against 7.3, 32768 x 1024 at four 13.2 against 12.3; 8192 x 1024 5.9
+        // against 6.1, 49152 x 768 14.5 against 15.5, 128256 x 1024 33.2 against 36.8).
         const int64_t least = rows == 3 ? (n_in <= 1024 ? 3 : 6) : n_in < 1024 ? 3 : 5;
         if (n_in % 256 == 0 && (rows == 3 || (rows == 4 && n_in <= 1024)) && tiles > least * sm_count()) {
-            if (setup_format<WT>(p, n_in, rows, silu_pair, smem, tma && (n_in > 1024 || tiles <= 5 * sm_count()), true) && p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit) return true;
+            if (setup_format<WT>(p, n_in, rows, silu_pair, smem, tma && (n_in > 1024 || tiles <= 5 * sm_count() || tiles > 14 * sm_count()), true) && p.tps == 1 && p.n_stages >= 3 && *smem <= (size_t)kSmemLimit) return true;
             if (tma && !setup_format<WT>(p, n_in, rows, silu_pair, smem, true)) return false;
         }
     }

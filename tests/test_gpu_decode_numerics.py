@@ -410,11 +410,11 @@ def test_rows_without_room_in_groups_pairs_and_residuals(cuda, wt):
     assert cuda.device_status() == 0
 
 
-@pytest.mark.parametrize("n_in, tiles", [(768, (3, 5)), (1024, (2, 3, 5)), (4096, (2, 6))])
+@pytest.mark.parametrize("n_in, tiles", [(768, (3, 5, 14)), (1024, (2, 3, 5, 14)), (4096, (2, 6))])
 def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_in, tiles):
     """Two consumer groups share a CTA up to six tiles of 16 weight rows per SM at three rows and everywhere at four; up to 1024 values
     up to three at three rows, five at four (three below 1024). Beyond, every CTA has one group, and two share an SM; up to 1024 values
-    stages come as row copies beyond five tiles per SM."""
+    stages come as row copies from five to fourteen tiles per SM."""
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     for n_out in sorted({16 * sms * t + more for t in tiles for more in (0, 1, 267)}):
