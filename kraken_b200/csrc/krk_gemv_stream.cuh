@@ -2262,7 +2262,7 @@ __host__ __device__ constexpr int box_pitch(int bytes) { return align_up(bytes, 
 
 // Whether one or two activation rows may go to two groups of consumer warps that take a tile's stages in turn (in_turn), one CTA
 // to an SM. They do where a half SM has no room for the ring (one group left an SM with eight warps: Q6_K 4096 x 11008 13.9 -> 12.8 us, Q8_0 at
-// two rows 15.6 -> 13.2), and where no CTA has a second tile and a tile has many stages (Q4_K 1024 x 8192 5.4 -> 4.1, 2048 x 11008 5.7 -> 4.9;
+// two rows 15.6 -> 13.2), and where no CTA has a second tile and a tile has many stages (Q4_K 1024 x 8192 6.2 -> 4.7, 2080 x 11008 8.7 -> 6.3;
 // at 4608 values, two stages and a part of a third, 0.85 to 1.16 of the time, so from beyond 5120 on; up to 8192 not where tiles for
 // nearly all SMs would give up the next launch's early start, 2368 x 5632 1.00 to 1.06). A model's pass shows the same at one row (2048 /
 // 8192 values 0.80 to 0.93 of the time, 1792 / 6912 0.82 to 0.95, 2048 / 5632 0.85 to 1.03) and a gain at two only while tiles leave SMs
