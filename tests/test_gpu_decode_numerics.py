@@ -410,8 +410,24 @@ def test_rows_without_room_in_groups_pairs_and_residuals(cuda, wt):
     assert cuda.device_status() == 0
 
 
+@pytest.mark.parametrize("n_out", [4736, 4737, 5003])
+def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_out):
+    """Up to two tiles of 16 weight rows per SM (148: 4736 rows) two consumer groups share a CTA, beyond that every CTA has one."""
+    import torch
+    for n_in in (1024, 4096):
+        w = dev(synth.weights(synth.Q8_0, n_out, n_in, SEED + 6, stream=1))
+        w64 = cuda.dequant_rows(w, synth.Q8_0, n_out, n_in).double()
+        for rows in (2, 3, 4, 5):
+            x = dev(synth.activations(rows, n_in, SEED + rows))
+            base = torch.randn((rows, n_out), device="cuda")
+            y = cuda.gemv(x, w, synth.Q8_0, n_out, n_in, out=base.clone(), accumulate=True)
+            lim = 2e-6 * w64.norm(dim=1)[None] * x.double().norm(dim=1)[:, None] + 1e-6 * base.abs()
+            assert ((y.double() - base.double() - x.double() @ w64.T).abs() <= lim).all()
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n_in, tiles", [(768, (3, 5, 14)), (1024, (2, 3, 5, 14)), (4096, (2, 6))])
-def test_q8_0_three_and_four_rows_across_the_change_of_form(cuda, n_in, tiles):
+def test_q8_0_three_and_four_rows_of_one_group(cuda, n_in, tiles):
     """Two consumer groups share a CTA up to six tiles of 16 weight rows per SM at three rows and everywhere at four; up to 1024 values
     up to three at three rows, five at four (three below 1024). Beyond, every CTA has one group, and two share an SM; up to 1024 values
     stages come as row copies from five to fourteen tiles per SM."""
@@ -468,7 +484,7 @@ def test_rows_of_odd_block_counts_on_either_kernel(cuda, wt):
 @pytest.mark.parametrize("n_in", [2304, 4352, 6656, 11008, 12544])
 def test_rows_of_many_slices(cuda, oracle, wt, n_in):
     """A warp prepares one to seven slices of every activation row (held, in one batch of loads, in a second; six of the widest rows go
-    in parts, with four limbs). 22 bits of the largest activation of a warp's slices
+    to the warp-per-row kernel in most formats). 22 bits of the largest activation of a warp's slices
     (about four sigma here) leave 4 * 2^-22 / sqrt(12) a value, 2.8e-7 of the norms' product for a result; seven times that."""
     n_out = 80
     w = synth.weights(wt, n_out, n_in, SEED + 2, stream=wt)
