@@ -1835,10 +1835,11 @@ gemv_stream_kernel(const __grid_constant__ StreamParams p) {
                     }
                 }
             };
-            if constexpr (STACK && NG > 1) {
+            if constexpr (STACK && NG > 1 && !(WT == KRK_CUDA_Q5_K && NG == 4)) {
                 // This code runs once or a few times in a launch, from a cold instruction cache: where it would be long, it is a loop
                 // (Q2_K 4096 x 512 at five rows 10.0 -> 7.3 us, 4096 x 256 9.7 -> 6.9; with one column group 1.00, with one tile to a
-                // stage 0.98 to 1.03).
+                // stage 0.98 to 1.03). Not Q5_K's, which is no longer than it was before rows in phases: at five and more rows of 1024
+                // values the consumers lose by it (4736 x 1024 at eight 8.5 -> 8.9; of 512 values 0.95 to 0.99 of the time).
 #pragma unroll 1
                 for (int sub = 0; sub < tps; sub++) {
 #pragma unroll (NG == 4 ? 1 : NG)
