@@ -2266,9 +2266,9 @@ __host__ __device__ constexpr int box_pitch(int bytes) { return align_up(bytes, 
 // two rows 15.6 -> 13.2), and where no CTA has a second tile and a tile has many stages (Q4_K 1024 x 8192 6.2 -> 4.7, 2080 x 11008 8.7 -> 6.3;
 // at 4608 values, two stages and a part of a third, 0.85 to 1.16 of the time, so from beyond 5120 on; up to 8192 not where tiles for
 // nearly all SMs would give up the next launch's early start, 2368 x 5632 1.00 to 1.06). A model's pass shows the same at one row (2048 /
-// 8192 values 0.80 to 0.93 of the time, 1792 / 6912 0.82 to 0.95, 2048 / 5632 0.85 to 1.03) and a gain at two only while tiles leave SMs
-// idle (1536 / 5632 0.97 to 1.00; 2048 / 5632 1.02 to 1.10, 2048 / 8192 0.99 to 1.04, 2304 / 9216 1.00 to 1.03), so up to four fifths of
-// them. Up to 4096 values results keep the order of their sums, in which eight warps add their units one after the other; beyond 5120 it
+// 8192 values 0.80 to 0.93 of the time, 1792 / 6912 0.82 to 0.95, 2048 / 5632 0.85 to 1.03), and at two through the backend (against one
+// group from four fifths of the SMs on: 2048 / 8192 Q8_0 0.90 of the time, IQ4_NL 0.91, Q4_K 0.94; 2048 / 5632 0.95 to 0.99, 2304 / 8704 0.92 to
+// 1.01; called matrix by matrix 0.96 to 1.08, most 1.00). Up to 4096 values results keep the order of their sums, in which eight warps add their units one after the other; beyond 5120 it
 // goes by the rows of a launch's matrices (of a slice of a head, by those of the whole, see setup_launch).
 template <int WT>
 bool stages_halve(const StreamParams &p) {
@@ -2606,8 +2606,7 @@ bool setup_launch(StreamParams &p, const GemvMat *mats, int n_mat, int64_t n_in,
     int64_t tiles = 0;
     for (int m = 0; m < n_mat; m += silu_pair ? 2 : 1) tiles += ((whole_rows ? whole_rows : mats[m].n_out) + kTileRows - 1) / kTileRows;
     // A tile for an SM at most, of many stages: two groups, see stages_halve.
-    const int most = rows == 2 ? sm_count() * 4 / 5 : n_in >= 8192 ? sm_count() : sm_count() * 7 / 8;
-    const bool whole_sm = rows <= 2 && n_in > 5120 && tiles <= most;
+    const bool whole_sm = rows <= 2 && n_in > 5120 && tiles <= (n_in >= 8192 ? sm_count() : sm_count() * 7 / 8);
     bool tma = Fmt<WT>::tma != 0 && !no_tma;
     if (tma) {
         if (!setup_format<WT>(p, n_in, rows, silu_pair, smem, true, false, whole_sm, wide)) return false;
